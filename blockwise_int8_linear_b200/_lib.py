@@ -1,4 +1,5 @@
-"""ctypes binding of libbi8.so (declared in include/bi8.h).
+"""Loading of libbi8.so (declared in include/bi8.h), through ctypes, and of the extension that calls it for the functional
+operations.
 
 There is no fallback: if the library cannot be loaded, or a call returns an error status, an
 exception is raised.  Tensors are passed as raw device pointers plus sizes; the current torch
@@ -32,6 +33,7 @@ ADDEND_FULL = 0x100
 PRE_NONE, PRE_RMSNORM, PRE_SILU_MUL = 0, 1, 2
 
 _lib = None
+_native = None
 
 
 class Bi8Error(RuntimeError):
@@ -92,6 +94,21 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+def native():
+    """The extension module that runs the functional operations (``csrc/torch_ops.cpp``)."""
+    global _native
+    if _native is None:
+        lib()
+        if not os.path.exists(os.path.join(_HERE, "_native.so")):
+            raise ImportError(
+                f"{os.path.join(_HERE, '_native.so')} is missing: build it with `python -m blockwise_int8_linear_b200.build` "
+                "(there is no non-CUDA fallback)")
+        from . import _native as module
+        module.set_error_class(Bi8Error)
+        _native = module
+    return _native
+
+
 def check(status: int, what: str) -> None:
     if status != 0:
         msg = lib().bi8_last_error_string().decode(errors="replace")
@@ -113,38 +130,13 @@ def stream_ptr() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-_workspaces: dict = {}       # (device, stream handle) -> buffer, eager launches
-_capture_ws: dict = {}       # (device, capture id) -> buffer, launches recorded into the CUDA graph being captured
-
-
-def _capture_id(stream) -> int:
-    cid = ctypes.c_ulonglong(0)
-    check(lib().bi8_stream_capture_id(ctypes.c_void_p(stream.cuda_stream), ctypes.byref(cid)), "bi8_stream_capture_id")
-    return int(cid.value)
-
-
 def workspace(device: torch.device, nbytes: int):
-    """GEMM workspace of at least ``nbytes`` for (device, current stream), or None for 0 bytes.
-
-    The workspace is scratch for split-K partial results.  Eager launches: one buffer per stream is reused by all GEMMs
-    queued on that stream (they run one after the other), which saves an allocator round trip per call; a larger request
-    replaces the buffer.  While the stream is being captured, the buffer's address is baked into the CUDA graph, so every
-    capture gets a buffer of its own (keyed by the capture's sequence number): two graphs never share scratch and may be
-    replayed on different streams.  All GEMMs of one graph share its buffer, which is correct because a graph's kernels
-    run in capture order.  The buffer is allocated from the capture's memory pool, which keeps it reserved for the graph's
-    lifetime; this module drops its own reference when it sees the next capture (or an eager call)."""
+    """GEMM workspace of at least ``nbytes`` for (device, current stream), or None for 0 bytes: scratch for the partial
+    results of divided tiles, one buffer per stream for eager launches, one per CUDA graph while a stream is captured (the
+    table is the one of ``csrc/torch_ops.cpp``, which the functional operations use)."""
     if nbytes <= 0:
         return None
-    stream = torch.cuda.current_stream(device)
-    cid = _capture_id(stream) if torch.cuda.is_current_stream_capturing() else 0
-    for k in [k for k in _capture_ws if k != (device.index, cid)]:
-        del _capture_ws[k]
-    table, key = (_capture_ws, (device.index, cid)) if cid else (_workspaces, (device.index, stream.cuda_stream))
-    ws = table.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(max(nbytes, 2 * ws.numel() if ws is not None else 0), dtype=torch.uint8, device=device)
-        table[key] = ws
-    return ws
+    return native().workspace(device.index if device.index is not None else torch.cuda.current_device(), nbytes)
 
 
 def device_status() -> int:

@@ -9,16 +9,16 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from . import _lib
 from . import block_linear_config
 from .triton_functions import (
     dequantize_block_rowwise,
     int8_matmul_block64_rowwise_dequantize,
     quantize_block_colwise,
-    pre_quantize_matmul_block_rowwise_dequantize,
     quantize_block_dual,
     quantize_block_rowwise,
-    quantize_matmul_block_rowwise_dequantize,
 )
+from .triton_functions import _block, _pre_code
 
 __all__ = [
     "replace_linear_with_blockwise_int8", "fast_matmul", "blockwise_int8_linear", "BlockInt8Linear", "BlockLinear",
@@ -191,17 +191,19 @@ class BlockInt8Linear(nn.Linear):
         W_int8, state_W = quantize_block_rowwise(self.weight.detach())
         return dequantize_block_rowwise(W_int8, state_W)
 
+    def _quantized_weight(self):
+        """``(W_int8, state_W)``, quantized on first use."""
+        W_int8 = self._buffers.get("W_int8")           # nn.Module's own attribute look-up searches three dicts first
+        if W_int8 is None:
+            if not hasattr(self, "W_int8"):
+                self.prepare_for_eval()
+            return self.W_int8, self.state_W
+        return W_int8, self._buffers["state_W"]
+
     def infer(self, x):
-        if not hasattr(self, "W_int8"):
-            self.prepare_for_eval()
-        X = x.reshape(-1, x.size(-1))
-        if X.size(0) <= 64:
-            # decode-sized batches: the same two steps in one library call whose kernels overlap
-            return quantize_matmul_block_rowwise_dequantize(X, self.W_int8.t(), self.state_W, self.bias).view(*x.size()[:-1], -1)
-        X_int8, state_X = quantize_block_rowwise(X)
-        return int8_matmul_block64_rowwise_dequantize(
-            X_int8, self.W_int8.t(), state_X, self.state_W, self.bias
-        ).view(*x.size()[:-1], -1)
+        W_int8, state_W = self._quantized_weight()
+        return _lib.native().linear(_lib.PRE_NONE, x, W_int8, state_W, self._parameters["bias"], None, None, 0.0, None, _block(),
+                                    block_linear_config.INPUT_OUTPUT_TORCH_TYPE)
 
     def infer_pre(self, x, op="none", x2=None, norm_weight=None, eps=1e-5, residual=None):
         """``infer`` with the elementwise step that produces this projection's input fused into the quantizer, and the
@@ -211,14 +213,9 @@ class BlockInt8Linear(nn.Linear):
         ``op='rmsnorm'``   ``infer(rms_norm(x, eps) [* norm_weight])``
         ``op='silu_mul'``  ``infer(F.silu(x) * x2)``
         ``residual``       ``residual + infer(...)`` in the activation type; ``residual`` has the output's shape."""
-        if not hasattr(self, "W_int8"):
-            self.prepare_for_eval()
-        X = x.reshape(-1, x.size(-1))
-        X2 = x2.reshape(-1, x2.size(-1)) if x2 is not None else None
-        R = residual.reshape(-1, residual.size(-1)) if residual is not None else None
-        out = pre_quantize_matmul_block_rowwise_dequantize(op, X, self.W_int8.t(), self.state_W, self.bias, x2=X2,
-                                                           norm_weight=norm_weight, eps=eps, residual=R)
-        return out.view(*x.size()[:-1], -1)
+        W_int8, state_W = self._quantized_weight()
+        return _lib.native().linear(_pre_code(op), x, W_int8, state_W, self._parameters["bias"], x2, norm_weight, eps, residual, _block(),
+                                    block_linear_config.INPUT_OUTPUT_TORCH_TYPE)
 
     def forward(self, x):
         if not self.training:

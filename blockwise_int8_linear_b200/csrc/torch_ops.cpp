@@ -1,0 +1,631 @@
+// Python extension `_native`: the host path between the Python functions and libbi8.so.
+//
+// Every public operation is one call into this module: it validates its operands, allocates the results and the scratch from
+// torch's caching allocator, and enqueues the kernels through the C ABI of include/bi8.h on torch's current stream.  Written
+// against the CPython call protocol (METH_FASTCALL) without a binding layer, because a decode-sized layer is 9 us of device
+// time: the same steps in Python (tensor views, torch.empty, attribute look-ups, one ctypes call with twenty converted
+// arguments) took 40 us per call and were what bounded every call below about 50 us.
+//
+// Nothing here computes: the operations' meaning, shapes and layouts are described in triton_functions.py, and there is no
+// path for tensors that are not on a CUDA device.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/core/LegacyTypeDispatch.h>
+#include <ATen/ops/empty.h>
+#include <ATen/ops/empty_strided.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <algorithm>
+#include <mutex>
+#include <string>
+#include <unordered_map>
+
+#include "../../include/bi8.h"
+
+namespace {
+
+using at::Tensor;
+
+// ---- errors: the Python exception types that the functions have always raised ------------------------------------------
+struct PyFail {
+    PyObject* type;          // borrowed: a builtin exception class or g_error_class
+    std::string text;
+};
+PyObject* g_error_class = nullptr;       // blockwise_int8_linear_b200._lib.Bi8Error, set once when the module is loaded
+
+[[noreturn]] void value_error(std::string text) { throw PyFail{PyExc_ValueError, std::move(text)}; }
+[[noreturn]] void assertion(const char* text) { throw PyFail{PyExc_AssertionError, text}; }
+
+void check(int status, const char* what) {
+    if (status != BI8_OK)
+        throw PyFail{g_error_class ? g_error_class : PyExc_RuntimeError,
+                     std::string(what) + " failed with status " + std::to_string(status) + ": " + bi8_last_error_string()};
+}
+
+std::string shape_of(const Tensor& t) {
+    std::string s = "[";
+    for (int64_t i = 0; i < t.dim(); ++i) s += (i ? ", " : "") + std::to_string(t.size(i));
+    return s + "]";
+}
+std::string shape_of(int64_t a, int64_t b) { return "[" + std::to_string(a) + ", " + std::to_string(b) + "]"; }
+
+int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+int dtype_code(at::ScalarType t) {
+    switch (t) {
+        case at::kBFloat16: return BI8_BF16;
+        case at::kHalf: return BI8_F16;
+        case at::kFloat: return BI8_F32;
+        default: value_error(std::string("unsupported dtype ") + c10::toString(t) + ": expected bfloat16, float16 or float32");
+    }
+}
+
+// ---- allocation and streams ---------------------------------------------------------------------------------------------
+Tensor empty_on(const Tensor& like, at::IntArrayRef sizes, at::ScalarType type) {
+    return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device()));
+}
+
+// Scratch of the GEMMs (partial results of divided tiles), one buffer per (device, stream) for eager launches: GEMMs queued on a
+// stream run one after the other, so they share it, which saves an allocator round trip per call; a larger request replaces the
+// buffer.  While a stream is being captured the buffer's address is baked into the CUDA graph, so every capture gets
+// a buffer of its own, keyed by the capture's sequence number and allocated from the capture's memory pool, which keeps it
+// reserved for the graph's lifetime; the table drops its own reference when it sees the next capture or an eager call.  At
+// most kMostStreams streams are remembered: one more empties the table (the allocator takes the buffers back in
+// stream order).
+constexpr size_t kMostStreams = 64;
+struct WsKey {
+    int device;
+    uint64_t id;
+    bool operator==(const WsKey& o) const { return device == o.device && id == o.id; }
+};
+struct WsHash {
+    size_t operator()(const WsKey& k) const { return std::hash<uint64_t>()(k.id * 0x9E3779B97F4A7C15ull + (uint64_t)k.device); }
+};
+std::mutex g_ws_mutex;
+std::unordered_map<WsKey, Tensor, WsHash>& eager_table() {
+    static auto* t = new std::unordered_map<WsKey, Tensor, WsHash>();      // never destroyed: the allocator may be gone at exit
+    return *t;
+}
+std::unordered_map<WsKey, Tensor, WsHash>& capture_table() {
+    static auto* t = new std::unordered_map<WsKey, Tensor, WsHash>();
+    return *t;
+}
+
+// The returned tensor keeps the buffer alive while the caller enqueues its kernels (another thread may replace the entry).
+Tensor workspace(c10::Device device, c10::cuda::CUDAStream stream, int64_t bytes) {
+    if (bytes <= 0) return Tensor();
+    unsigned long long capture = 0;
+    check(bi8_stream_capture_id(stream.stream(), &capture), "bi8_stream_capture_id");
+    const WsKey key{device.index(), capture ? (uint64_t)capture : (uint64_t)reinterpret_cast<uintptr_t>(stream.stream())};
+    std::lock_guard<std::mutex> lock(g_ws_mutex);
+    auto& captures = capture_table();
+    for (auto it = captures.begin(); it != captures.end();) it = (capture && it->first == key) ? std::next(it) : captures.erase(it);
+    auto& table = capture ? captures : eager_table();
+    auto it = table.find(key);
+    if (it != table.end() && it->second.numel() >= bytes) return it->second;
+    const int64_t want = std::max<int64_t>(bytes, it != table.end() ? 2 * it->second.numel() : 0);
+    if (it == table.end() && table.size() >= kMostStreams) table.clear();
+    Tensor t = at::empty({want}, at::TensorOptions().dtype(at::kByte).device(device));
+    table[key] = t;
+    return t;
+}
+
+// Makes the operand's device current for a call and names its current stream.
+struct OnDevice {
+    c10::cuda::CUDAGuard guard;
+    c10::cuda::CUDAStream stream;
+    explicit OnDevice(const Tensor& t) : guard(t.device()), stream(c10::cuda::getCurrentCUDAStream(t.device().index())) {}
+    void* raw() const { return stream.stream(); }
+};
+
+// ---- matrices -----------------------------------------------------------------------------------------------------------
+// A matrix with contiguous rows: where it lies, its row pitch in elements, and the tensor that owns it.
+struct Mat {
+    Tensor owner;
+    const void* ptr = nullptr;
+    int64_t rows = 0, cols = 0, ld = 0;
+};
+
+bool rows_contiguous(int64_t rows, int64_t cols, int64_t s0, int64_t s1) {
+    return (cols == 1 || s1 == 1) && (rows <= 1 || s0 >= cols);
+}
+
+Mat mat(const Tensor& t, int64_t rows, int64_t cols, int64_t s0, int64_t s1, bool transposed) {
+    Mat m;
+    m.rows = rows;
+    m.cols = cols;
+    if (rows_contiguous(rows, cols, s0, s1)) {
+        m.owner = t;
+        m.ld = rows > 1 ? s0 : std::max<int64_t>(cols, 1);
+    } else {
+        m.owner = (transposed ? t.t() : t).contiguous();
+        m.ld = std::max<int64_t>(cols, 1);
+    }
+    m.ptr = m.owner.data_ptr();
+    return m;
+}
+
+Mat mat2d(const Tensor& t) {
+    if (t.dim() != 2) value_error("expected a 2-D tensor, got " + shape_of(t));
+    return mat(t, t.size(0), t.size(1), t.stride(0), t.stride(1), false);
+}
+
+Mat mat2d_t(const Tensor& t) {          // the transpose of a 2-D tensor
+    return mat(t, t.size(1), t.size(0), t.stride(1), t.stride(0), true);
+}
+
+// [..., K] as [rows, K]
+Mat mat_rows(const Tensor& t) {
+    if (t.dim() == 2) return mat2d(t);
+    if (t.dim() == 0) value_error("expected a tensor with a feature dimension, got a scalar");
+    const int64_t k = t.size(-1), rows = k ? t.numel() / k : t.numel();
+    if (t.is_contiguous()) return mat(t, rows, k, k, 1, false);
+    return mat2d(t.reshape({-1, k}));
+}
+
+void need_cuda(const Tensor& t) {
+    if (!t.is_cuda()) assertion("x.is_cuda");
+}
+
+// Zero-padded copy of a large 16-bit matrix whose row or column count is not a multiple of 16, or an undefined tensor when no
+// padding is called for.  The fast quantizers and the tensor-core GEMM want 16-byte aligned rows.  Padding with zeros
+// changes no result: the pad stays inside the last block (block sizes here are multiples of 16), and zeros change
+// neither a block's absmax nor the quantized values of its other elements.
+Tensor pad16(const Tensor& x, int64_t block, bool rows, bool cols) {
+    const int64_t r = x.size(0), c = x.size(1);
+    if ((x.scalar_type() != at::kBFloat16 && x.scalar_type() != at::kHalf) || block % 16 != 0 || r * c < (1 << 22)) return Tensor();
+    const int64_t rp = rows ? ceil_div(r, 16) * 16 : r, cp = cols ? ceil_div(c, 16) * 16 : c;
+    if ((rp == r && cp == c) || std::min(r, c) < 256) return Tensor();
+    Tensor buf = empty_on(x, {rp, cp}, x.scalar_type());
+    if (rp != r) buf.zero_();
+    else buf.narrow(1, c, cp - c).zero_();
+    buf.narrow(0, 0, r).narrow(1, 0, c).copy_(x);
+    return buf;
+}
+
+// Copy with a 16-byte aligned row pitch of an int8 operand that has none; the bytes between K and the pitch are never read.
+Mat repitch(const Mat& m, const Tensor& like) {
+    if (m.ld % 16 == 0 && reinterpret_cast<uintptr_t>(m.ptr) % 16 == 0) return m;
+    Mat out = m;
+    out.ld = ceil_div(m.cols, 16) * 16;
+    out.owner = empty_on(like, {m.rows, out.ld}, at::kChar);
+    out.owner.narrow(1, 0, m.cols).copy_(m.owner.dim() == 2 && m.owner.size(0) == m.rows && m.owner.size(1) == m.cols ? m.owner : m.owner.t());
+    out.ptr = out.owner.data_ptr();
+    return out;
+}
+
+// ---- quantizers ---------------------------------------------------------------------------------------------------------
+struct Quantized {
+    Tensor q, s;
+};
+
+Quantized quantize_rowwise(const Tensor& x, int64_t block) {
+    need_cuda(x);
+    if (x.dim() == 2) {
+        const Tensor padded = pad16(x, block, false, true);
+        if (padded.defined()) {
+            Quantized r = quantize_rowwise(padded, block);
+            return {r.q.narrow(1, 0, x.size(1)), r.s};       // a view with an aligned row pitch, which the GEMM takes as it is
+        }
+    }
+    OnDevice on(x);
+    const Mat m = mat2d(x);
+    const int code = dtype_code(x.scalar_type());
+    Quantized r{empty_on(x, {m.rows, m.cols}, at::kChar), empty_on(x, {ceil_div(m.cols, block), m.rows}, at::kFloat)};
+    check(bi8_quantize_rowwise(m.ptr, code, m.ld, r.q.mutable_data_ptr<int8_t>(), r.s.mutable_data_ptr<float>(), m.rows, m.cols, (int)block, on.raw()),
+          "bi8_quantize_rowwise");
+    return r;
+}
+
+Quantized quantize_colwise(const Tensor& x, int64_t block) {
+    need_cuda(x);
+    if (x.dim() == 2) {
+        const Tensor padded = pad16(x, block, true, true);
+        if (padded.defined()) {
+            Quantized r = quantize_colwise(padded, block);
+            return {r.q.narrow(0, 0, x.size(1)).narrow(1, 0, x.size(0)), r.s.narrow(1, 0, x.size(1))};
+        }
+    }
+    OnDevice on(x);
+    const Mat m = mat2d(x);
+    const int code = dtype_code(x.scalar_type());
+    Quantized r{empty_on(x, {m.cols, m.rows}, at::kChar), empty_on(x, {ceil_div(m.rows, block), m.cols}, at::kFloat)};
+    check(bi8_quantize_colwise(m.ptr, code, m.ld, r.q.mutable_data_ptr<int8_t>(), r.s.mutable_data_ptr<float>(), m.rows, m.cols, (int)block, on.raw()),
+          "bi8_quantize_colwise");
+    return r;
+}
+
+struct Dual {
+    Quantized row, col;
+};
+
+Dual quantize_dual(const Tensor& x, int64_t block) {
+    need_cuda(x);
+    if (x.dim() == 2) {
+        const Tensor padded = pad16(x, block, true, true);
+        if (padded.defined()) {
+            Dual d = quantize_dual(padded, block);
+            const int64_t r = x.size(0), c = x.size(1);
+            return {{d.row.q.narrow(0, 0, r).narrow(1, 0, c), d.row.s.narrow(1, 0, r)}, {d.col.q.narrow(0, 0, c).narrow(1, 0, r), d.col.s.narrow(1, 0, c)}};
+        }
+    }
+    OnDevice on(x);
+    const Mat m = mat2d(x);
+    const int code = dtype_code(x.scalar_type());
+    Dual d{{empty_on(x, {m.rows, m.cols}, at::kChar), empty_on(x, {ceil_div(m.cols, block), m.rows}, at::kFloat)},
+           {empty_on(x, {m.cols, m.rows}, at::kChar), empty_on(x, {ceil_div(m.rows, block), m.cols}, at::kFloat)}};
+    check(bi8_quantize_dual(m.ptr, code, m.ld, d.row.q.mutable_data_ptr<int8_t>(), d.row.s.mutable_data_ptr<float>(),
+                            d.col.q.mutable_data_ptr<int8_t>(), d.col.s.mutable_data_ptr<float>(), m.rows, m.cols, (int)block, on.raw()),
+          "bi8_quantize_dual");
+    return d;
+}
+
+void check_scales(const Tensor& s, int64_t nb, int64_t rows, int64_t block, const char* name) {
+    if (s.dim() != 2 || s.size(0) != nb || s.size(1) != rows || s.scalar_type() != at::kFloat)
+        value_error(std::string(name) + " must be float32 " + shape_of(nb, rows) + " for block " + std::to_string(block) + ", got " +
+                    c10::toString(s.scalar_type()) + " " + shape_of(s));
+}
+
+Tensor dequantize(const Tensor& q, const Tensor& state, int64_t block, at::ScalarType out_type) {
+    need_cuda(q);
+    if (q.dim() != 2) value_error("expected a 2-D tensor, got " + shape_of(q));
+    if (q.scalar_type() != at::kChar) value_error(std::string("expected an int8 tensor, got ") + c10::toString(q.scalar_type()));
+    const int64_t m = q.size(0), k = q.size(1);
+    check_scales(state, ceil_div(k, block), m, block, "state");
+    OnDevice on(q);
+    const Tensor x = q.contiguous(), s = state.contiguous();
+    Tensor out = empty_on(q, {m, k}, out_type);
+    check(bi8_dequantize_rowwise(x.const_data_ptr<int8_t>(), s.const_data_ptr<float>(), out.data_ptr(), dtype_code(out_type), m, k, (int)block, on.raw()),
+          "bi8_dequantize_rowwise");
+    return out;
+}
+
+// ---- GEMM ---------------------------------------------------------------------------------------------------------------
+// Bias operand: a contiguous vector of a type the kernels read, or nothing.
+struct Bias {
+    Tensor owner;
+    const void* ptr = nullptr;
+    int code = 0;
+    Bias(const Tensor& b, int64_t n) {
+        if (!b.defined()) return;
+        if (b.numel() != n) value_error("bias must have " + std::to_string(n) + " elements, got " + std::to_string(b.numel()));
+        owner = (b.dim() == 1 ? b : b.reshape({n})).contiguous();
+        const at::ScalarType t = owner.scalar_type();
+        if (t != at::kBFloat16 && t != at::kHalf && t != at::kFloat) owner = owner.to(at::kFloat);
+        ptr = owner.data_ptr();
+        code = dtype_code(owner.scalar_type());
+    }
+};
+
+struct Operands {
+    Mat a, bt;
+};
+
+// Brings both int8 operands to the form the library takes: a [M, K] and b^T [N, K] with contiguous rows.
+Operands gemm_operands(const Tensor& a, const Tensor& b) {
+    need_cuda(a);
+    if (a.dim() != 2 || b.dim() != 2) value_error("expected 2-D operands, got " + shape_of(a) + " and " + shape_of(b));
+    if (a.size(1) != b.size(0)) assertion("incompatible dimensions");
+    if (a.scalar_type() != at::kChar || b.scalar_type() != at::kChar)
+        value_error(std::string("operands must be int8, got ") + c10::toString(a.scalar_type()) + " and " + c10::toString(b.scalar_type()));
+    Operands o{mat2d(a), mat2d_t(b)};
+    // The tensor-core kernel needs 16-byte aligned operand rows: for a long contraction that is not a multiple of 16 both
+    // operands are re-pitched once.
+    const int64_t k = a.size(1);
+    if (k % 16 != 0 && k >= 256 && o.a.rows * o.bt.rows >= 128 * 128) {
+        o.a = repitch(o.a, a);
+        o.bt = repitch(o.bt, a);
+    }
+    return o;
+}
+
+Tensor gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& state_x, const Tensor& state_w, const Tensor& bias_in, int64_t block,
+            at::ScalarType out_type, int flags) {
+    need_cuda(a_in);
+    OnDevice on(a_in);
+    const Operands o = gemm_operands(a_in, b_in);
+    const int64_t m = o.a.rows, n = o.bt.rows, k = o.a.cols, nb = ceil_div(k, block);
+    check_scales(state_x, nb, m, block, "state_x");
+    check_scales(state_w, nb, n, block, "state_w");
+    const Tensor sx = state_x.contiguous(), sw = state_w.contiguous();
+    Tensor c = empty_on(a_in, {m, n}, out_type);
+    const Bias bias(bias_in, n);
+    const size_t ws_bytes = bi8_gemm_workspace_bytes(m, n, k, (int)block);
+    const Tensor ws = workspace(a_in.device(), on.stream, (int64_t)ws_bytes);
+    check(bi8_gemm_dequant(static_cast<const int8_t*>(o.a.ptr), o.a.ld, static_cast<const int8_t*>(o.bt.ptr), o.bt.ld, sx.const_data_ptr<float>(),
+                           sw.const_data_ptr<float>(), bias.ptr, bias.code, c.data_ptr(), n, dtype_code(out_type), m, n, k, (int)block,
+                           ws.defined() ? ws.data_ptr() : nullptr, ws_bytes, flags, on.raw()),
+          "bi8_gemm_dequant");
+    return c;
+}
+
+Tensor block_partials(const Tensor& a, const Tensor& b, int64_t block, int flags) {
+    need_cuda(a);
+    OnDevice on(a);
+    const Operands o = gemm_operands(a, b);
+    const int64_t m = o.a.rows, n = o.bt.rows, k = o.a.cols;
+    Tensor out = at::zeros({ceil_div(k, block), m, n}, at::TensorOptions().dtype(at::kInt).device(a.device()));
+    check(bi8_gemm_block_partials(static_cast<const int8_t*>(o.a.ptr), o.a.ld, static_cast<const int8_t*>(o.bt.ptr), o.bt.ld,
+                                  out.mutable_data_ptr<int32_t>(), m, n, k, (int)block, flags, on.raw()),
+          "bi8_gemm_block_partials");
+    return out;
+}
+
+// ---- producer step + quantizer + GEMM + residual ------------------------------------------------------------------------
+// Operands of a fused producer step with a shared row pitch.
+struct Pre {
+    int op;
+    Mat x, x2;
+    Tensor weight;
+    Pre(int op_, const Tensor& x_in, const Tensor& x2_in, const Tensor& w_in) : op(op_), x(mat_rows(x_in)) {
+        if (op == BI8_PRE_SILU_MUL) {
+            if (!x2_in.defined() || x2_in.sizes() != x_in.sizes() || x2_in.scalar_type() != x_in.scalar_type() || x2_in.device() != x_in.device())
+                value_error("silu_mul needs a second operand with x's shape, dtype and device");
+            x2 = mat_rows(x2_in);
+            if (x2.ld != x.ld) {           // e.g. one of the two was copied: give both the same row pitch
+                x = mat_rows(x_in.contiguous());
+                x2 = mat_rows(x2_in.contiguous());
+            }
+        }
+        if (op == BI8_PRE_RMSNORM && w_in.defined()) {
+            if (w_in.numel() != x.cols) value_error("norm weight must have " + std::to_string(x.cols) + " elements, got " + std::to_string(w_in.numel()));
+            weight = (w_in.dim() == 1 ? w_in : w_in.reshape({-1})).to(x_in.scalar_type()).contiguous();
+        }
+    }
+    const void* weight_ptr() const { return weight.defined() ? weight.data_ptr() : nullptr; }
+};
+
+Quantized quantize_pre(int op, const Tensor& x_in, const Tensor& x2, const Tensor& weight, double eps, int64_t block) {
+    need_cuda(x_in);
+    if (x_in.dim() != 2) value_error("expected a 2-D tensor, got " + shape_of(x_in));
+    OnDevice on(x_in);
+    const Pre pre(op, x_in, x2, weight);
+    const int64_t m = pre.x.rows, k = pre.x.cols;
+    Quantized r{empty_on(x_in, {m, k}, at::kChar), empty_on(x_in, {ceil_div(k, block), m}, at::kFloat)};
+    check(bi8_quantize_rowwise_pre(op, pre.x.ptr, pre.x2.ptr, dtype_code(x_in.scalar_type()), pre.x.ld, pre.weight_ptr(), (float)eps,
+                                   r.q.mutable_data_ptr<int8_t>(), r.s.mutable_data_ptr<float>(), m, k, (int)block, on.raw()),
+          "bi8_quantize_rowwise_pre");
+    return r;
+}
+
+// y = pre(x) W^T (+ bias) (+ residual) for x [..., K] and the int8 weights as `w` = [N, K] (or, with `w_transposed`, its [K, N] view)
+Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, const Tensor& state_w, const Tensor& bias_in, const Tensor& x2,
+              const Tensor& norm_weight, double eps, const Tensor& residual, const Tensor& out_in, int64_t block, at::ScalarType out_type, int flags) {
+    need_cuda(x_in);
+    if (w.dim() != 2) value_error("expected 2-D weights, got " + shape_of(w));
+    if (x_in.dim() == 0 || x_in.size(-1) != w.size(w_transposed ? 0 : 1)) assertion("incompatible dimensions");
+    if (w.scalar_type() != at::kChar) value_error(std::string("weights must be int8, got ") + c10::toString(w.scalar_type()));
+    OnDevice on(x_in);
+    const Pre pre(op, x_in, x2, norm_weight);
+    const Mat bt = w_transposed ? mat2d_t(w) : mat2d(w);
+    const int64_t m = pre.x.rows, k = pre.x.cols, n = bt.rows, nb = ceil_div(k, block);
+    check_scales(state_w, nb, n, block, "state_w");
+    const Tensor sw = state_w.contiguous();
+    c10::SmallVector<int64_t, 6> shape(x_in.sizes().begin(), x_in.sizes().end());
+    shape.back() = n;
+    Tensor out = out_in, res = residual;
+    int64_t ldc = n, ldr = 0;
+    auto check_2d = [&](const Tensor& t, const char* name) {
+        if (t.dim() != 2 || t.size(0) != m || t.size(1) != n || t.scalar_type() != out_type || t.stride(1) != 1 || t.device() != x_in.device())
+            value_error(std::string(name) + " must be " + c10::toString(out_type) + " " + shape_of(m, n) + " with contiguous rows on " + x_in.device().str());
+        return m > 1 ? t.stride(0) : std::max<int64_t>(n, 1);
+    };
+    if (out.defined()) ldc = check_2d(out, "out");
+    else out = empty_on(x_in, shape, out_type);
+    if (res.defined()) {
+        if (res.dim() != 2 && n > 0) res = res.reshape({-1, n});
+        ldr = check_2d(res, "residual");
+    }
+    const Bias bias(bias_in, n);
+    Tensor target = out;
+    if (res.defined() && out.data_ptr() == res.data_ptr() && !(m <= 64 && bias.ptr == nullptr && n % 4 == 0 && k % 16 == 0 && ldc == ldr)) {
+        target = empty_on(x_in, {m, n}, out_type);          // not the path that may update in place
+        ldc = n;
+    }
+    const int x_code = dtype_code(x_in.scalar_type());
+    const size_t ws_bytes = bi8_gemm_workspace_bytes(m, n, k, (int)block);
+    const Tensor ws = workspace(x_in.device(), on.stream, (int64_t)ws_bytes);
+    void* ws_ptr = ws.defined() ? ws.data_ptr() : nullptr;
+    if (k % 16 != 0 && op == BI8_PRE_NONE && !res.defined() && m > 64 && target.is_same(out) && !out_in.defined() && flags == 0) {
+        // rows that are not 16-byte aligned: the quantizer and the GEMM re-pitch their operands
+        const Quantized r = quantize_rowwise(pre.x.owner.dim() == 2 ? pre.x.owner : pre.x.owner.reshape({m, k}), block);
+        return gemm(r.q, w_transposed ? w : w.t(), r.s, sw, bias_in, block, out_type, 0).view(shape);
+    }
+    const Tensor xq = empty_on(x_in, {m, k}, at::kChar), sx = empty_on(x_in, {nb, m}, at::kFloat);
+    check(bi8_gemm_dequant_fused_pre(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps, xq.mutable_data_ptr<int8_t>(),
+                                     sx.mutable_data_ptr<float>(), static_cast<const int8_t*>(bt.ptr), bt.ld, sw.const_data_ptr<float>(), bias.ptr,
+                                     bias.code, res.defined() ? res.data_ptr() : nullptr, ldr, target.data_ptr(), ldc, dtype_code(out_type), m, n,
+                                     k, (int)block, ws_ptr, ws_bytes, flags, on.raw()),
+          "bi8_gemm_dequant_fused_pre");
+    if (!target.is_same(out)) out.copy_(target);
+    return out;
+}
+
+// ---- decode step: rotary embedding and cache append ---------------------------------------------------------------------
+Tensor rope_cache_append(const Tensor& qkv_in, const Tensor& cis_in, const Tensor& pos, const Tensor& kcache, const Tensor& vcache) {
+    need_cuda(qkv_in);
+    if (qkv_in.dim() != 4 || qkv_in.size(1) != 3 || qkv_in.size(3) % 2 != 0) value_error("expected [B, 3, H, D] with even D, got " + shape_of(qkv_in));
+    const int64_t b = qkv_in.size(0), h = qkv_in.size(2), d = qkv_in.size(3);
+    OnDevice on(qkv_in);
+    const Tensor qkv = qkv_in.contiguous();
+    // complex64 [D/2] or float32 (cos, sin) pairs: the same bytes
+    const bool cplx = cis_in.scalar_type() == at::kComplexFloat;
+    if ((!cplx && cis_in.scalar_type() != at::kFloat) || cis_in.numel() * (cplx ? 2 : 1) != d || !cis_in.is_contiguous())
+        value_error("cis must hold " + std::to_string(d / 2) + " contiguous (cos, sin) float32 pairs");
+    if (pos.scalar_type() != at::kLong || pos.numel() != 1 || pos.device() != qkv.device())
+        value_error("pos must be an int64 tensor with one element on the activations' device");
+    if (kcache.dim() != 4) value_error("caches must be 4-D, got " + shape_of(kcache));
+    const int64_t max_len = kcache.size(2);
+    for (const Tensor* c : {&kcache, &vcache})
+        if (c->dim() != 4 || c->size(0) != b || c->size(1) != h || c->size(2) != max_len || c->size(3) != d || c->scalar_type() != qkv.scalar_type() ||
+            !c->is_contiguous() || c->device() != qkv.device())
+            value_error(std::string("caches must be contiguous ") + c10::toString(qkv.scalar_type()) + " [" + std::to_string(b) + ", " + std::to_string(h) +
+                        ", max_len, " + std::to_string(d) + "] on " + qkv.device().str());
+    Tensor q = empty_on(qkv, {b, h, 1, d}, qkv.scalar_type());
+    check(bi8_rope_cache_append(qkv.data_ptr(), dtype_code(qkv.scalar_type()), static_cast<const float*>(cis_in.data_ptr()),
+                                static_cast<const long long*>(pos.data_ptr()), q.data_ptr(), kcache.data_ptr(), vcache.data_ptr(), b, h, d, max_len, on.raw()),
+          "bi8_rope_cache_append");
+    return q;
+}
+
+// ---- bindings -----------------------------------------------------------------------------------------------------------
+struct Args {
+    PyObject* const* a;
+    Py_ssize_t n;
+    const Tensor& tensor(int i) const {
+        if (!THPVariable_Check(a[i])) throw PyFail{PyExc_TypeError, std::string("expected a tensor, got ") + Py_TYPE(a[i])->tp_name};
+        return THPVariable_Unpack(a[i]);
+    }
+    Tensor optional(int i) const { return a[i] == Py_None ? Tensor() : tensor(i); }
+    int64_t integer(int i) const {
+        const long long v = PyLong_AsLongLong(a[i]);
+        if (v == -1 && PyErr_Occurred()) throw python_error();
+        return v;
+    }
+    double number(int i) const {
+        const double v = PyFloat_AsDouble(a[i]);
+        if (v == -1.0 && PyErr_Occurred()) throw python_error();
+        return v;
+    }
+    at::ScalarType dtype(int i) const {
+        if (!THPDtype_Check(a[i])) throw PyFail{PyExc_TypeError, "expected a torch.dtype"};
+        const at::ScalarType t = reinterpret_cast<THPDtype*>(a[i])->scalar_type;
+        (void)dtype_code(t);
+        return t;
+    }
+    int64_t block(int i) const {
+        const int64_t b = integer(i);
+        if (b < 1 || b > 0x7fffffff) value_error("block size must be positive, got " + std::to_string(b));
+        return b;
+    }
+};
+
+PyObject* wrap(const Tensor& t) { return THPVariable_Wrap(t); }
+PyObject* wrap(const Quantized& r) {
+    PyObject* t = PyTuple_New(2);
+    PyTuple_SET_ITEM(t, 0, wrap(r.q));
+    PyTuple_SET_ITEM(t, 1, wrap(r.s));
+    return t;
+}
+PyObject* wrap(const Dual& d) {
+    PyObject* t = PyTuple_New(4);
+    PyTuple_SET_ITEM(t, 0, wrap(d.row.q));
+    PyTuple_SET_ITEM(t, 1, wrap(d.row.s));
+    PyTuple_SET_ITEM(t, 2, wrap(d.col.q));
+    PyTuple_SET_ITEM(t, 3, wrap(d.col.s));
+    return t;
+}
+
+// Runs `body` without the interpreter lock (kernel launches can block when the launch queue is full) and without recording
+// autograd history, and turns its exceptions into Python's.
+template <typename Body>
+PyObject* call(const char* name, const Args& args, Py_ssize_t want, Body body) {
+    try {
+        if (args.n != want) throw PyFail{PyExc_TypeError, std::string(name) + " takes " + std::to_string(want) + " arguments, got " + std::to_string(args.n)};
+        auto result = [&] {
+            auto work = body(args);            // reads the arguments with the lock held
+            pybind11::gil_scoped_release no_gil;
+            at::AutoDispatchBelowADInplaceOrView below_autograd;
+            return work();
+        }();
+        return wrap(result);
+    } catch (const PyFail& e) {
+        PyErr_SetString(e.type, e.text.c_str());
+        return nullptr;
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());
+        return nullptr;
+    }
+}
+
+#define BI8_METHOD(name) PyObject* name##_py(PyObject*, PyObject* const* a, Py_ssize_t n)
+
+BI8_METHOD(quantize_rowwise) {
+    return call("quantize_rowwise", {a, n}, 2, [](const Args& g) { return [x = g.tensor(0), b = g.block(1)] { return quantize_rowwise(x, b); }; });
+}
+BI8_METHOD(quantize_colwise) {
+    return call("quantize_colwise", {a, n}, 2, [](const Args& g) { return [x = g.tensor(0), b = g.block(1)] { return quantize_colwise(x, b); }; });
+}
+BI8_METHOD(quantize_dual) {
+    return call("quantize_dual", {a, n}, 2, [](const Args& g) { return [x = g.tensor(0), b = g.block(1)] { return quantize_dual(x, b); }; });
+}
+BI8_METHOD(quantize_pre) {       // op, x, x2, weight, eps, block
+    return call("quantize_pre", {a, n}, 6, [](const Args& g) {
+        return [op = (int)g.integer(0), x = g.tensor(1), x2 = g.optional(2), w = g.optional(3), eps = g.number(4), b = g.block(5)] {
+            return quantize_pre(op, x, x2, w, eps, b);
+        };
+    });
+}
+BI8_METHOD(dequantize) {         // q, state, block, dtype
+    return call("dequantize", {a, n}, 4, [](const Args& g) {
+        return [q = g.tensor(0), s = g.tensor(1), b = g.block(2), t = g.dtype(3)] { return dequantize(q, s, b, t); };
+    });
+}
+BI8_METHOD(gemm) {               // a, b, state_x, state_w, bias, block, dtype, flags
+    return call("gemm", {a, n}, 8, [](const Args& g) {
+        return [x = g.tensor(0), y = g.tensor(1), sx = g.tensor(2), sw = g.tensor(3), bias = g.optional(4), b = g.block(5), t = g.dtype(6),
+                f = (int)g.integer(7)] { return gemm(x, y, sx, sw, bias, b, t, f); };
+    });
+}
+BI8_METHOD(block_partials) {     // a, b, block, flags
+    return call("block_partials", {a, n}, 4, [](const Args& g) {
+        return [x = g.tensor(0), y = g.tensor(1), b = g.block(2), f = (int)g.integer(3)] { return block_partials(x, y, b, f); };
+    });
+}
+BI8_METHOD(matmul) {             // op, x [M, K], b [K, N], state_w, bias, x2, norm_weight, eps, residual, out, block, dtype, flags
+    return call("matmul", {a, n}, 13, [](const Args& g) {
+        if (g.tensor(1).dim() != 2) {
+            need_cuda(g.tensor(1));
+            value_error("expected a 2-D tensor, got " + shape_of(g.tensor(1)));
+        }
+        return [op = (int)g.integer(0), x = g.tensor(1), w = g.tensor(2), sw = g.tensor(3), bias = g.optional(4), x2 = g.optional(5), nw = g.optional(6),
+                eps = g.number(7), res = g.optional(8), out = g.optional(9), b = g.block(10), t = g.dtype(11), f = (int)g.integer(12)] {
+            return linear(op, x, w, true, sw, bias, x2, nw, eps, res, out, b, t, f);
+        };
+    });
+}
+BI8_METHOD(linear) {             // op, x [..., K], W int8 [N, K], state_w, bias, x2, norm_weight, eps, residual, block, dtype
+    return call("linear", {a, n}, 11, [](const Args& g) {
+        return [op = (int)g.integer(0), x = g.tensor(1), w = g.tensor(2), sw = g.tensor(3), bias = g.optional(4), x2 = g.optional(5), nw = g.optional(6),
+                eps = g.number(7), res = g.optional(8), b = g.block(9), t = g.dtype(10)] {
+            return linear(op, x, w, false, sw, bias, x2, nw, eps, res, Tensor(), b, t, 0);
+        };
+    });
+}
+BI8_METHOD(rope_cache_append) {  // qkv, cis, pos, kcache, vcache
+    return call("rope_cache_append", {a, n}, 5, [](const Args& g) {
+        return [q = g.tensor(0), c = g.tensor(1), p = g.tensor(2), k = g.tensor(3), v = g.tensor(4)] { return rope_cache_append(q, c, p, k, v); };
+    });
+}
+BI8_METHOD(workspace) {          // device index, bytes (> 0)
+    return call("workspace", {a, n}, 2, [](const Args& g) {
+        return [d = (int)g.integer(0), bytes = g.integer(1)] {
+            const c10::Device device(c10::kCUDA, (c10::DeviceIndex)d);
+            c10::cuda::CUDAGuard guard(device);
+            return workspace(device, c10::cuda::getCurrentCUDAStream(device.index()), bytes);
+        };
+    });
+}
+PyObject* set_error_class_py(PyObject*, PyObject* cls) {
+    Py_XINCREF(cls);
+    Py_XSETREF(g_error_class, cls);
+    Py_RETURN_NONE;
+}
+
+#define BI8_ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name##_py)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {BI8_ENTRY(quantize_rowwise), BI8_ENTRY(quantize_colwise), BI8_ENTRY(quantize_dual), BI8_ENTRY(quantize_pre),
+                         BI8_ENTRY(dequantize), BI8_ENTRY(gemm), BI8_ENTRY(block_partials), BI8_ENTRY(matmul), BI8_ENTRY(linear),
+                         BI8_ENTRY(rope_cache_append), BI8_ENTRY(workspace),
+                         {"set_error_class", set_error_class_py, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Host path of the blockwise-int8 operations.", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module); }

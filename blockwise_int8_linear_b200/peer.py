@@ -53,6 +53,44 @@ def _exchange_buffers(nbytes: int, device, world: int, group, local: bool):
     return bufs, handle, (ctypes.c_void_p * 8)(*(ptrs + [ptrs[0]] * (8 - len(ptrs))))
 
 
+def _rows_contiguous(t: torch.Tensor) -> torch.Tensor:
+    """2-D tensor whose last dimension is contiguous and whose row pitch covers a row."""
+    if t.shape[1] != 1 and t.stride(1) != 1:
+        return t.contiguous()
+    if t.shape[0] > 1 and t.stride(0) < t.shape[1]:
+        return t.contiguous()
+    return t
+
+
+def _pitch(t: torch.Tensor) -> int:
+    return t.stride(0) if t.shape[0] > 1 else max(t.shape[1], 1)
+
+
+def _pre_operands(op: str, x, x2, norm_weight):
+    """Checks the operands of a fused producer step: returns (code, x, x2, weight) with shared row pitch and dtype."""
+    if op not in ("none", "rmsnorm", "silu_mul"):
+        raise ValueError(f"unknown producer step {op!r}: expected 'none', 'rmsnorm' or 'silu_mul'")
+    assert x.is_cuda
+    if x.dim() != 2:
+        raise ValueError(f"expected a 2-D tensor, got {tuple(x.shape)}")
+    x = _rows_contiguous(x)
+    if op == "silu_mul":
+        if x2 is None or tuple(x2.shape) != tuple(x.shape) or x2.dtype != x.dtype or x2.device != x.device:
+            raise ValueError("silu_mul needs a second operand with x's shape, dtype and device")
+        x2 = _rows_contiguous(x2)
+        if _pitch(x2) != _pitch(x):         # e.g. one of the two was copied: give both the same row pitch
+            x, x2 = x.contiguous(), x2.contiguous()
+    else:
+        x2 = None
+    if op == "rmsnorm" and norm_weight is not None:
+        if norm_weight.numel() != x.shape[1]:
+            raise ValueError(f"norm weight must have {x.shape[1]} elements, got {norm_weight.numel()}")
+        norm_weight = norm_weight.reshape(-1).to(x.dtype).contiguous()
+    else:
+        norm_weight = None
+    return {"none": _lib.PRE_NONE, "rmsnorm": _lib.PRE_RMSNORM, "silu_mul": _lib.PRE_SILU_MUL}[op], x, x2, norm_weight
+
+
 class PeerAllReduce:
     """``PeerAllReduce(capacity, device, group)(partial, bias)`` -> ``cast(sum over ranks of partial) + bias``.
 
@@ -126,7 +164,7 @@ class PeerAllReduce:
         normalise over this rank's slice only and is rejected).  For decode-sized batches (at most 64 rows) the kernel that
         finishes the weight-streaming GEMM exchanges its sums with the other ranks itself; the result equals
         ``self(partial)`` on the fp32 output of ``quantize_matmul_block_rowwise_dequantize``."""
-        from .triton_functions import _block, _pitch, _pre_operands, ceil_div
+        from .triton_functions import _block, ceil_div
         if op == "rmsnorm" and self.world > 1:
             raise ValueError("a row-parallel layer holds a slice of the features: normalise before the slice is taken")
         block = _block()
