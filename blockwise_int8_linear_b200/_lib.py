@@ -104,7 +104,8 @@ def native():
                 f"{os.path.join(_HERE, '_native.so')} is missing: build it with `python -m blockwise_int8_linear_b200.build` "
                 "(there is no non-CUDA fallback)")
         from . import _native as module
-        module.set_error_class(Bi8Error)
+        from . import block_linear_config
+        module.bind(Bi8Error, block_linear_config)
         _native = module
     return _native
 

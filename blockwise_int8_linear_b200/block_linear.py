@@ -15,7 +15,6 @@ from .triton_functions import (
     dequantize_block_rowwise,
     int8_matmul_block64_rowwise_dequantize,
     quantize_block_colwise,
-    quantize_block_dual,
     quantize_block_rowwise,
 )
 from .triton_functions import _block, _pre_code
@@ -79,70 +78,14 @@ class blockwise_int8_linear(torch.autograd.Function):
     ``CACHE_QUANTIZED_WEIGHTS`` is set); the transposed operands of the backward GEMMs are quantized straight from
     the row-major tensors by the fused column-wise quantizer, which is bit-identical to ``t().contiguous()`` +
     row-wise quantize.  With ``FUSE_DUAL_QUANTIZE`` (default) X and G are each read once for both of their
-    quantizations, and the backward pass keeps X as its transposed int8 copy; every result is unchanged."""
+    quantizations, and the backward pass keeps X as its transposed int8 copy; every result is unchanged.
+
+    Both passes run in the extension as a native autograd node (``csrc/torch_ops.cpp``, ``LinearBackward``): a Python
+    ``Function`` costs the engine two interpreter calls per layer, which is more than a small layer's kernels take."""
 
     @staticmethod
-    def forward(ctx, X_3D, W, bias):
-        X = X_3D.reshape(-1, X_3D.size(-1))
-        ctx.has_bias = bias is not None
-        ctx.wcache = cache = _weight_cache(W)
-        if ctx.needs_input_grad[1] and getattr(block_linear_config, "FUSE_DUAL_QUANTIZE", True):
-            # the weight gradient needs X blocked along the tokens (block_linear.py:100-101): both quantizations come
-            # from one read of X, and the backward pass keeps the int8 transposed copy instead of X itself
-            X_int8, state_X, Xt_int8, state_Xt = quantize_block_dual(X)
-            ctx.save_for_backward(Xt_int8, state_Xt, W)
-            ctx.x_quantized = True
-            ctx.block = block_linear_config.GROUP_SIZE
-        else:
-            X_int8, state_X = quantize_block_rowwise(X)
-            ctx.save_for_backward(X, W)
-            ctx.x_quantized = False
-        if cache is not None and "row" in cache:
-            W_int8, state_W = cache["row"]
-        else:
-            W_int8, state_W = quantize_block_rowwise(W)
-            if cache is not None:
-                cache["row"] = (W_int8, state_W)
-        out = int8_matmul_block64_rowwise_dequantize(X_int8, W_int8.t(), state_X, state_W, bias)
-        return out.view(*X_3D.size()[:-1], -1)
-
-    @staticmethod
-    def backward(ctx, G_3D):
-        G = G_3D.reshape(-1, G_3D.size(-1))
-        if ctx.x_quantized:
-            if ctx.block != block_linear_config.GROUP_SIZE:
-                raise RuntimeError("GROUP_SIZE changed between the forward and the backward pass of a BlockInt8Linear")
-            x_int8, x_state, W = ctx.saved_tensors
-        else:
-            X, W = ctx.saved_tensors
-        grad_X = grad_W = grad_bias = None
-        gt_int8 = None
-        if ctx.needs_input_grad[0] and ctx.needs_input_grad[1] and getattr(block_linear_config, "FUSE_DUAL_QUANTIZE", True):
-            # G is needed blocked along N (for dX) and along the tokens (for dW): one read
-            g_int8, g_state, gt_int8, gt_state = quantize_block_dual(G)
-        elif ctx.needs_input_grad[0]:
-            g_int8, g_state = quantize_block_rowwise(G)
-        if ctx.needs_input_grad[0]:
-            # contraction over N: both operands blocked along N (block_linear.py:92-95)
-            cache = ctx.wcache         # still valid: autograd refuses to run backward on a weight modified since forward
-            if cache is not None and "col" in cache:
-                Wt_int8, w_state = cache["col"]
-            else:
-                Wt_int8, w_state = quantize_block_colwise(W)                 # [K, N], state [N/B, K]
-                if cache is not None:
-                    cache["col"] = (Wt_int8, w_state)
-            grad_X = int8_matmul_block64_rowwise_dequantize(g_int8, Wt_int8.t(), g_state, w_state)
-            grad_X = grad_X.view(*G_3D.size()[:-1], -1)
-        if ctx.needs_input_grad[1]:
-            # contraction over the tokens: both operands blocked along M (block_linear.py:100-104)
-            if not ctx.x_quantized:
-                x_int8, x_state = quantize_block_colwise(X)                  # [K, M], state [M/B, K]
-            if gt_int8 is None:
-                gt_int8, gt_state = quantize_block_colwise(G)                # [N, M], state [M/B, N]
-            grad_W = int8_matmul_block64_rowwise_dequantize(gt_int8, x_int8.t(), gt_state, x_state)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            grad_bias = G.sum(dim=0)
-        return grad_X, grad_W, grad_bias
+    def apply(X_3D, W, bias):
+        return _lib.native().train_linear(X_3D, W, bias, getattr(block_linear_config, "FUSE_DUAL_QUANTIZE", True), _weight_cache(W))
 
 
 class BlockInt8Linear(nn.Linear):
@@ -202,7 +145,7 @@ class BlockInt8Linear(nn.Linear):
 
     def infer(self, x):
         W_int8, state_W = self._quantized_weight()
-        return _lib.native().linear(_lib.PRE_NONE, x, W_int8, state_W, self._parameters["bias"], None, None, 0.0, None, _block(),
+        return _lib.native().linear(_lib.PRE_NONE, x, W_int8, state_W, self.bias, None, None, 0.0, None, _block(),
                                     block_linear_config.INPUT_OUTPUT_TORCH_TYPE)
 
     def infer_pre(self, x, op="none", x2=None, norm_weight=None, eps=1e-5, residual=None):
@@ -214,15 +157,16 @@ class BlockInt8Linear(nn.Linear):
         ``op='silu_mul'``  ``infer(F.silu(x) * x2)``
         ``residual``       ``residual + infer(...)`` in the activation type; ``residual`` has the output's shape."""
         W_int8, state_W = self._quantized_weight()
-        return _lib.native().linear(_pre_code(op), x, W_int8, state_W, self._parameters["bias"], x2, norm_weight, eps, residual, _block(),
+        return _lib.native().linear(_pre_code(op), x, W_int8, state_W, self.bias, x2, norm_weight, eps, residual, _block(),
                                     block_linear_config.INPUT_OUTPUT_TORCH_TYPE)
 
     def forward(self, x):
         if not self.training:
             return self.infer(x)
-        if self.weight.numel() == 0:
+        weight = self.weight
+        if weight.numel() == 0:
             raise RuntimeError("this BlockInt8Linear dropped its floating-point weight for inference; training needs it")
-        return blockwise_int8_linear.apply(x, self.weight, self.bias)
+        return blockwise_int8_linear.apply(x, weight, self.bias)
 
     def _load_from_state_dict(self, state_dict, prefix, local_metadata, strict, missing_keys, unexpected_keys, error_msgs):
         # a checkpoint saved after the first eval forward carries W_int8/state_W: make room for them

@@ -11,19 +11,22 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <ATen/core/LegacyTypeDispatch.h>
-#include <ATen/ops/empty.h>
-#include <ATen/ops/empty_strided.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <algorithm>
 #include <mutex>
+#include <optional>
 #include <string>
 #include <unordered_map>
 
@@ -38,7 +41,7 @@ struct PyFail {
     PyObject* type;          // borrowed: a builtin exception class or g_error_class
     std::string text;
 };
-PyObject* g_error_class = nullptr;       // blockwise_int8_linear_b200._lib.Bi8Error, set once when the module is loaded
+PyObject* g_error_class = nullptr;       // blockwise_int8_linear_b200._lib.Bi8Error, set when the module is loaded
 
 [[noreturn]] void value_error(std::string text) { throw PyFail{PyExc_ValueError, std::move(text)}; }
 [[noreturn]] void assertion(const char* text) { throw PyFail{PyExc_AssertionError, text}; }
@@ -68,18 +71,31 @@ int dtype_code(at::ScalarType t) {
 }
 
 // ---- allocation and streams ---------------------------------------------------------------------------------------------
+// the allocator behind torch.empty, without the dispatcher in front of it
 Tensor empty_on(const Tensor& like, at::IntArrayRef sizes, at::ScalarType type) {
-    return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device()));
+    return at::detail::empty_cuda(sizes, type, like.device(), std::nullopt);
 }
 
-// Scratch of the GEMMs (partial results of divided tiles), one buffer per (device, stream) for eager launches: GEMMs queued on a
+// Sizes of the buffers that one call carves out of a single allocation.
+struct Carve {
+    int64_t bytes = 0;
+    int64_t take(int64_t n) {
+        const int64_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    }
+};
+
+// Scratch of the GEMMs (partial results of divided tiles, quantized activations that no caller sees), one buffer per (device, stream) for eager launches: GEMMs queued on a
 // stream run one after the other, so they share it, which saves an allocator round trip per call; a larger request replaces the
 // buffer.  While a stream is being captured the buffer's address is baked into the CUDA graph, so every capture gets
 // a buffer of its own, keyed by the capture's sequence number and allocated from the capture's memory pool, which keeps it
 // reserved for the graph's lifetime; the table drops its own reference when it sees the next capture or an eager call.  At
 // most kMostStreams streams are remembered: one more empties the table (the allocator takes the buffers back in
-// stream order).
+// stream order).  A request above kMostKept is not remembered: it is allocated for its call, which then runs for
+// far longer than the allocation takes.
 constexpr size_t kMostStreams = 64;
+constexpr int64_t kMostKept = 32 << 20;
 struct WsKey {
     int device;
     uint64_t id;
@@ -101,6 +117,7 @@ std::unordered_map<WsKey, Tensor, WsHash>& capture_table() {
 // The returned tensor keeps the buffer alive while the caller enqueues its kernels (another thread may replace the entry).
 Tensor workspace(c10::Device device, c10::cuda::CUDAStream stream, int64_t bytes) {
     if (bytes <= 0) return Tensor();
+    if (bytes > kMostKept) return at::detail::empty_cuda({bytes}, at::kByte, device, std::nullopt);
     unsigned long long capture = 0;
     check(bi8_stream_capture_id(stream.stream(), &capture), "bi8_stream_capture_id");
     const WsKey key{device.index(), capture ? (uint64_t)capture : (uint64_t)reinterpret_cast<uintptr_t>(stream.stream())};
@@ -110,9 +127,9 @@ Tensor workspace(c10::Device device, c10::cuda::CUDAStream stream, int64_t bytes
     auto& table = capture ? captures : eager_table();
     auto it = table.find(key);
     if (it != table.end() && it->second.numel() >= bytes) return it->second;
-    const int64_t want = std::max<int64_t>(bytes, it != table.end() ? 2 * it->second.numel() : 0);
+    const int64_t want = std::min(std::max<int64_t>(bytes, it != table.end() ? 2 * it->second.numel() : 0), kMostKept);
     if (it == table.end() && table.size() >= kMostStreams) table.clear();
-    Tensor t = at::empty({want}, at::TensorOptions().dtype(at::kByte).device(device));
+    Tensor t = at::detail::empty_cuda({want}, at::kByte, device, std::nullopt);
     table[key] = t;
     return t;
 }
@@ -431,20 +448,200 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
     }
     const int x_code = dtype_code(x_in.scalar_type());
     const size_t ws_bytes = bi8_gemm_workspace_bytes(m, n, k, (int)block);
-    const Tensor ws = workspace(x_in.device(), on.stream, (int64_t)ws_bytes);
-    void* ws_ptr = ws.defined() ? ws.data_ptr() : nullptr;
+    // the quantized activations live in the stream's scratch behind the GEMM's workspace
+    Carve carve;
+    carve.take((int64_t)ws_bytes);
+    const int64_t xq_at = carve.take(m * k), sx_at = carve.take(nb * m * 4);
+    const Tensor ws = workspace(x_in.device(), on.stream, carve.bytes);
+    char* ws_ptr = ws.defined() ? static_cast<char*>(ws.data_ptr()) : nullptr;
     if (k % 16 != 0 && op == BI8_PRE_NONE && !res.defined() && m > 64 && target.is_same(out) && !out_in.defined() && flags == 0) {
         // rows that are not 16-byte aligned: the quantizer and the GEMM re-pitch their operands
         const Quantized r = quantize_rowwise(pre.x.owner.dim() == 2 ? pre.x.owner : pre.x.owner.reshape({m, k}), block);
         return gemm(r.q, w_transposed ? w : w.t(), r.s, sw, bias_in, block, out_type, 0).view(shape);
     }
-    const Tensor xq = empty_on(x_in, {m, k}, at::kChar), sx = empty_on(x_in, {nb, m}, at::kFloat);
-    check(bi8_gemm_dequant_fused_pre(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps, xq.mutable_data_ptr<int8_t>(),
-                                     sx.mutable_data_ptr<float>(), static_cast<const int8_t*>(bt.ptr), bt.ld, sw.const_data_ptr<float>(), bias.ptr,
-                                     bias.code, res.defined() ? res.data_ptr() : nullptr, ldr, target.data_ptr(), ldc, dtype_code(out_type), m, n,
-                                     k, (int)block, ws_ptr, ws_bytes, flags, on.raw()),
+    check(bi8_gemm_dequant_fused_pre(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps,
+                                     reinterpret_cast<int8_t*>(ws_ptr + xq_at), reinterpret_cast<float*>(ws_ptr + sx_at),
+                                     static_cast<const int8_t*>(bt.ptr), bt.ld, sw.const_data_ptr<float>(), bias.ptr, bias.code,
+                                     res.defined() ? res.data_ptr() : nullptr, ldr, target.data_ptr(), ldc, dtype_code(out_type), m, n, k,
+                                     (int)block, ws_bytes ? ws_ptr : nullptr, ws_bytes, flags, on.raw()),
           "bi8_gemm_dequant_fused_pre");
     if (!target.is_same(out)) out.copy_(target);
+    return out;
+}
+
+// ---- training: forward and backward as one autograd node ----------------------------------------------------------------
+// What the Python side knows at call time; the backward pass looks it up again (block size and result type are module-level
+// knobs, and the cache of quantized weights is a dict on the weight).
+PyObject* g_config = nullptr;            // the module blockwise_int8_linear_b200.block_linear_config
+
+int64_t config_block() {                 // with the interpreter lock
+    PyObject* v = PyObject_GetAttrString(g_config, "GROUP_SIZE");
+    if (!v) throw python_error();
+    const long long b = PyLong_AsLongLong(v);
+    Py_DECREF(v);
+    if (b == -1 && PyErr_Occurred()) throw python_error();
+    if (b < 1 || b > 0x7fffffff) value_error("block size must be positive, got " + std::to_string(b));
+    return b;
+}
+at::ScalarType config_dtype() {          // with the interpreter lock
+    PyObject* v = PyObject_GetAttrString(g_config, "INPUT_OUTPUT_TORCH_TYPE");
+    if (!v) throw python_error();
+    const bool is_dtype = THPDtype_Check(v);
+    const at::ScalarType t = is_dtype ? reinterpret_cast<THPDtype*>(v)->scalar_type : at::kFloat;
+    Py_DECREF(v);
+    if (!is_dtype) throw PyFail{PyExc_TypeError, "INPUT_OUTPUT_TORCH_TYPE must be a torch.dtype"};
+    (void)dtype_code(t);
+    return t;
+}
+
+// One blocking of a weight, from the cache dict under `key` or by `make` (then put into the cache, if there is one).
+template <typename Make>
+Quantized cached_weight(PyObject* cache, const char* key, Make make) {
+    if (!cache) return make();
+    {
+        pybind11::gil_scoped_acquire gil;
+        PyObject* hit = PyDict_GetItemString(cache, key);
+        if (hit && PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 2)
+            return {THPVariable_Unpack(PyTuple_GET_ITEM(hit, 0)), THPVariable_Unpack(PyTuple_GET_ITEM(hit, 1))};
+    }
+    const Quantized r = make();
+    pybind11::gil_scoped_acquire gil;
+    PyObject* pair = PyTuple_Pack(2, THPVariable_Wrap(r.q), THPVariable_Wrap(r.s));
+    if (!pair) throw python_error();
+    Py_DECREF(PyTuple_GET_ITEM(pair, 0));        // the tuple holds the only references
+    Py_DECREF(PyTuple_GET_ITEM(pair, 1));
+    const int rc = PyDict_SetItemString(cache, key, pair);
+    Py_DECREF(pair);
+    if (rc != 0) throw python_error();
+    return r;
+}
+
+Tensor rows_2d(const Tensor& t) { return t.dim() == 2 ? t : t.reshape({-1, t.size(-1)}); }
+
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+// Backward of y = x W^T + bias with both GEMMs in blockwise int8 (block_linear.py:85-112 in the reference).
+struct LinearBackward : public Node {
+    SavedVariable x, x_state;            // x as its column-wise int8 copy and scales, or x itself (x_state then empty)
+    SavedVariable weight;
+    bool x_quantized = false, has_bias = false, fuse_dual = true;
+    int64_t block = 0;
+    std::vector<int64_t> x_sizes;
+    PyObject* cache = nullptr;           // owned reference to the weight's cache dict, or null
+
+    ~LinearBackward() override {
+        if (cache && Py_IsInitialized()) {
+            pybind11::gil_scoped_acquire gil;
+            Py_DECREF(cache);
+        }
+    }
+    std::string name() const override { return "blockwise_int8_linearBackward"; }
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        x.reset_data();
+        x_state.reset_data();
+        weight.reset_data();
+    }
+    variable_list apply(variable_list&& grads) override;
+};
+
+variable_list LinearBackward::apply(variable_list&& grads) {
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    int64_t b = 0;
+    at::ScalarType type;
+    try {
+        {
+            pybind11::gil_scoped_acquire gil;
+            b = config_block();
+            type = config_dtype();
+        }
+        if (x_quantized && b != block)
+            throw std::runtime_error("GROUP_SIZE changed between the forward and the backward pass of a BlockInt8Linear");
+        std::lock_guard<std::mutex> lock(mutex_);
+        auto self = getptr();
+        const Tensor saved_x = x.unpack(self), w = weight.unpack(self);
+        at::AutoDispatchBelowADInplaceOrView below_autograd;
+        const Tensor g = rows_2d(grads[0]);
+        const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1);
+        Quantized g_row, g_col;
+        if (need_x && need_w && fuse_dual) {
+            // G is needed blocked along N (for dX) and along the tokens (for dW): one read
+            Dual d = quantize_dual(g, b);
+            g_row = d.row;
+            g_col = d.col;
+        } else if (need_x) {
+            g_row = quantize_rowwise(g, b);
+        }
+        if (need_x) {
+            // contraction over N, both operands blocked along N (block_linear.py:92-95).  A cached blocking is still valid:
+            // unpacking the weight raised if it was modified since the forward pass.
+            const Quantized wt = cached_weight(cache, "col", [&] { return quantize_colwise(w, b); });
+            out[0] = gemm(g_row.q, wt.q.t(), g_row.s, wt.s, Tensor(), b, type, 0).view(x_sizes);
+        }
+        if (need_w) {
+            // contraction over the tokens, both operands blocked along M (block_linear.py:100-104)
+            const Quantized xt = x_quantized ? Quantized{saved_x, x_state.unpack(self)} : quantize_colwise(rows_2d(saved_x), b);
+            if (!g_col.q.defined()) g_col = quantize_colwise(g, b);
+            out[1] = gemm(g_col.q, xt.q.t(), g_col.s, xt.s, Tensor(), b, type, 0);
+        }
+        if (has_bias && task_should_compute_output(2)) out[2] = g.sum(0);
+    } catch (const PyFail& e) {
+        pybind11::gil_scoped_acquire gil;
+        PyErr_SetString(e.type, e.text.c_str());
+        python_error err;
+        err.persist();
+        throw err;
+    }
+    return out;
+}
+
+// y = x W^T (+ bias), every operand quantized on the fly, recorded for backward when a gradient is wanted.  With `fuse_dual`
+// a layer whose weight is trained reads x once for both of its blockings and keeps the int8 transposed copy instead of x.
+Tensor train_linear(const Tensor& x_in, const Tensor& w, const Tensor& bias, int64_t block, at::ScalarType type, bool fuse_dual, PyObject* cache) {
+    need_cuda(x_in);
+    if (x_in.dim() == 0 || w.dim() != 2 || x_in.size(-1) != w.size(1)) assertion("incompatible dimensions");
+    const bool grad = at::GradMode::is_enabled() && (x_in.requires_grad() || w.requires_grad() || (bias.defined() && bias.requires_grad()));
+    std::shared_ptr<LinearBackward> node;
+    if (grad) {
+        node = std::shared_ptr<LinearBackward>(new LinearBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(x_in, w, bias));
+    }
+    Tensor out;
+    {
+        at::AutoDispatchBelowADInplaceOrView below_autograd;
+        const Tensor x = rows_2d(x_in);
+        Quantized xq;
+        if (node && w.requires_grad() && fuse_dual) {
+            Dual d = quantize_dual(x, block);
+            xq = d.row;
+            node->x = SavedVariable(d.col.q, false);
+            node->x_state = SavedVariable(d.col.s, false);
+            node->x_quantized = true;
+        } else {
+            xq = quantize_rowwise(x, block);
+        }
+        const Quantized wq = cached_weight(cache, "row", [&] { return quantize_rowwise(w, block); });
+        c10::SmallVector<int64_t, 6> shape(x_in.sizes().begin(), x_in.sizes().end());
+        shape.back() = w.size(0);
+        out = gemm(xq.q, wq.q.t(), xq.s, wq.s, bias, block, type, 0).view(shape);
+    }
+    if (node) {
+        if (!node->x_quantized) node->x = SavedVariable(x_in, false);
+        node->weight = SavedVariable(w, false);
+        node->has_bias = bias.defined();
+        node->fuse_dual = fuse_dual;
+        node->block = block;
+        node->x_sizes = x_in.sizes().vec();
+        if (cache) {
+            pybind11::gil_scoped_acquire gil;
+            Py_INCREF(cache);
+            node->cache = cache;
+        }
+        torch::autograd::set_history(out, node);
+    }
     return out;
 }
 
@@ -523,16 +720,16 @@ PyObject* wrap(const Dual& d) {
     return t;
 }
 
-// Runs `body` without the interpreter lock (kernel launches can block when the launch queue is full) and without recording
-// autograd history, and turns its exceptions into Python's.
+// Runs `body` without the interpreter lock (kernel launches can block when the launch queue is full) and turns its exceptions into Python's.
 template <typename Body>
-PyObject* call(const char* name, const Args& args, Py_ssize_t want, Body body) {
+PyObject* call(const char* name, const Args& args, Py_ssize_t want, Body body, bool records_history = false) {
     try {
         if (args.n != want) throw PyFail{PyExc_TypeError, std::string(name) + " takes " + std::to_string(want) + " arguments, got " + std::to_string(args.n)};
         auto result = [&] {
             auto work = body(args);            // reads the arguments with the lock held
             pybind11::gil_scoped_release no_gil;
-            at::AutoDispatchBelowADInplaceOrView below_autograd;
+            std::optional<at::AutoDispatchBelowADInplaceOrView> below_autograd;
+            if (!records_history) below_autograd.emplace();
             return work();
         }();
         return wrap(result);
@@ -599,6 +796,15 @@ BI8_METHOD(linear) {             // op, x [..., K], W int8 [N, K], state_w, bias
         };
     });
 }
+BI8_METHOD(train_linear) {       // x [..., K], W [N, K], bias, fuse_dual, cache dict or None: block size and type from the config module
+    return call("train_linear", {a, n}, 5, [](const Args& g) {
+        PyObject* cache = g.a[4] == Py_None ? nullptr : g.a[4];
+        if (cache && !PyDict_Check(cache)) throw PyFail{PyExc_TypeError, "the weight cache must be a dict"};
+        return [x = g.tensor(0), w = g.tensor(1), bias = g.optional(2), fuse = PyObject_IsTrue(g.a[3]) == 1, b = config_block(), t = config_dtype(), cache] {
+            return train_linear(x, w, bias, b, t, fuse, cache);
+        };
+    }, true);
+}
 BI8_METHOD(rope_cache_append) {  // qkv, cis, pos, kcache, vcache
     return call("rope_cache_append", {a, n}, 5, [](const Args& g) {
         return [q = g.tensor(0), c = g.tensor(1), p = g.tensor(2), k = g.tensor(3), v = g.tensor(4)] { return rope_cache_append(q, c, p, k, v); };
@@ -613,17 +819,21 @@ BI8_METHOD(workspace) {          // device index, bytes (> 0)
         };
     });
 }
-PyObject* set_error_class_py(PyObject*, PyObject* cls) {
-    Py_XINCREF(cls);
-    Py_XSETREF(g_error_class, cls);
+BI8_METHOD(bind) {               // the exception class of failed library calls, the configuration module
+    if (n != 2) {
+        PyErr_SetString(PyExc_TypeError, "bind takes 2 arguments");
+        return nullptr;
+    }
+    g_error_class = Py_NewRef(a[0]);
+    g_config = Py_NewRef(a[1]);
     Py_RETURN_NONE;
 }
 
 #define BI8_ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name##_py)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {BI8_ENTRY(quantize_rowwise), BI8_ENTRY(quantize_colwise), BI8_ENTRY(quantize_dual), BI8_ENTRY(quantize_pre),
                          BI8_ENTRY(dequantize), BI8_ENTRY(gemm), BI8_ENTRY(block_partials), BI8_ENTRY(matmul), BI8_ENTRY(linear),
-                         BI8_ENTRY(rope_cache_append), BI8_ENTRY(workspace),
-                         {"set_error_class", set_error_class_py, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
+                         BI8_ENTRY(train_linear), BI8_ENTRY(rope_cache_append), BI8_ENTRY(workspace), BI8_ENTRY(bind),
+                         {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Host path of the blockwise-int8 operations.", -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
