@@ -68,30 +68,36 @@ int check_gemm(const GemmArgs& g, bool partials) {
     return BI8_OK;
 }
 
+// The kernels that do not add GemmArgs::residual themselves are followed by one that does.
+int then_residual(int rc, const GemmArgs& g, cudaStream_t st) {
+    if (rc != BI8_OK || g.residual == nullptr) return rc;
+    return launch_residual_add(g.C, g.ldc, g.residual, g.ldr, g.out_dtype, g.M, g.N, st);
+}
+
 int dispatch_gemm(const GemmArgs& g, cudaStream_t st) {
     const char* why = "";
     const bool tc_ok = g.K > 0 && gemm_tc_applicable(g, &why);
     if (g.flags & BI8_GEMM_FORCE_SMALLM) {
         if (!gemm_smallm_applicable(g)) return fail(BI8_ERR_ALIGN, "small-M GEMM not applicable (needs M <= 16, block 32/64/128, K %% 16 == 0, 32-byte aligned weight rows)");
-        return launch_gemm_smallm(g, st);
+        return then_residual(launch_gemm_smallm(g, st), g, st);
     }
     if (g.flags & BI8_GEMM_FORCE_SKINNY) {
         if (!gemm_skinny_applicable(g))
             return fail(BI8_ERR_ALIGN, "skinny tensor-core GEMM not applicable (needs M <= 64, block 32/64/128, N %% 4 == 0, 16-byte aligned "
                                        "operand rows and weight scales, and the workspace bi8_gemm_workspace_bytes() asks for)");
-        return launch_gemm_skinny(g, st);
+        return then_residual(launch_gemm_skinny(g, st), g, st);
     }
     const bool free_choice = !(g.flags & (BI8_GEMM_FORCE_TC | BI8_GEMM_FORCE_GENERIC)) && g.K > 0;
     // M <= 64: one pass over the weights on the tensor cores with exchanged operand roles (needs the workspace)
-    if (free_choice && gemm_skinny_applicable(g)) return launch_gemm_skinny(g, st);
+    if (free_choice && gemm_skinny_applicable(g)) return then_residual(launch_gemm_skinny(g, st), g, st);
     // otherwise M <= 8 streams the weights on the CUDA cores; 9..16 would stream them twice and is faster on the
     // general tensor-core kernel
-    if (free_choice && g.M <= 8 && gemm_smallm_applicable(g)) return launch_gemm_smallm(g, st);
+    if (free_choice && g.M <= 8 && gemm_smallm_applicable(g)) return then_residual(launch_gemm_smallm(g, st), g, st);
     if (g.flags & BI8_GEMM_FORCE_TC) {
         if (!tc_ok) return fail(BI8_ERR_ALIGN, "tensor-core GEMM not applicable: %s", why);
         return launch_gemm_tc(g, st);
     }
-    if ((g.flags & BI8_GEMM_FORCE_GENERIC) || !tc_ok || g.K == 0) return launch_gemm_generic(g, st);
+    if ((g.flags & BI8_GEMM_FORCE_GENERIC) || !tc_ok || g.K == 0) return then_residual(launch_gemm_generic(g, st), g, st);
     return launch_gemm_tc(g, st);
 }
 
@@ -322,10 +328,13 @@ int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtyp
                                    "K %% 16 == 0, workspace given, no bias)");
     int rc = bi8_quantize_rowwise_pre(op, x, x2, x_dtype, ldx, norm_weight, eps, xq, sx, M, K, block, stream);
     if (rc != BI8_OK) return rc;
-    rc = bi8_gemm_dequant(xq, K, Wq, ldw, sx, sW, bias, bias_dtype, C, ldc, out_dtype, M, N, K, block, workspace, workspace_bytes,
-                          flags & ~BI8_GEMM_QUANT_IN_KERNEL, stream);
-    if (rc != BI8_OK || !residual) return rc;
-    return launch_residual_add(C, ldc, residual, ldr, out_dtype, M, N, st);
+    g.flags = flags & ~BI8_GEMM_QUANT_IN_KERNEL;
+    g.bias = bias;
+    g.bias_dtype = bias_dtype;
+    g.residual = residual;
+    g.ldr = ldr;
+    rc = check_gemm(g, false);
+    return rc != BI8_OK ? rc : dispatch_gemm(g, st);
 }
 
 size_t bi8_peer_allreduce_large_buffer_bytes(int world, int64_t capacity) {

@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <mutex>
+#include <utility>
 
 #include "../../include/bi8.h"
 
@@ -44,6 +45,33 @@ struct SmemOptIn {
         return BI8_OK;
     }
 };
+
+// Launch that may start before its predecessor in the stream has completed (programmatic stream serialisation).  Every kernel
+// launched this way executes after_predecessor() in every thread, before it touches memory that an earlier kernel reads or
+// writes; dependents are released only there, so that "the predecessor has completed" always means that everything before
+// it has completed too.  What it saves is the launch latency and the kernel's set-up, 1-2 us per kernel of a chain.
+template <typename... P, typename... A>
+int launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+    return BI8_OK;
+}
+
+#if defined(__CUDACC__)
+__device__ __forceinline__ void after_predecessor() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
 
 // ---- launchers implemented in the other translation units -------------------------------------
 int launch_quantize_rowwise(const void* x, int dt, int64_t ldx, int8_t* q, float* s, int64_t M, int64_t K,
@@ -111,6 +139,8 @@ struct GemmArgs {
     unsigned wait_limit_us = 0;         // diagnostic: limit of the general kernel's bounded waits (0 = default, about 2 s)
     int skip_stage = -1;                // diagnostic: the general kernel's producer leaves this stage of its first item out
     const PeerEpilogue* peer = nullptr; // decode kernel only: reduce over the ranks inside its reduction kernel
+    const void* residual = nullptr;     // general tensor-core kernel only: [M, N] addend of the output type, added after the bias
+    int64_t ldr = 0;                    // its row pitch in elements
     int64_t bias_ld = 0;                // decode kernel only: row pitch of `bias` in elements; non-zero makes it an [M, N] addend
 };
 

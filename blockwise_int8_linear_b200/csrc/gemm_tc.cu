@@ -108,7 +108,11 @@ struct TcParams {
     int tma_scales;     // bit 0: sA is described by the tensor map tmSA, bit 1: sB by tmSB
     int ksplit;         // > 1: the K stages are divided over ksplit work items per tile (split-K)
     int stages_per_split;
-    float* ws;          // split-K: fp32 partial results [ksplit, M, N]
+    float* ws;          // split-K: fp32 partial results, one slot of slot_floats values per work item (ws_index)
+    int slot_floats;    // BN x the tile rows that exist in any tile, rounded up to the 32 of a warp
+    const void* residual;     // [M, N] addend of the output type with row pitch ldr, or null
+    int64_t ldr;
+    int res_vec;        // its base and row pitch allow 16-byte loads
     unsigned wait_limit_us;   // 0: default limit of the bounded waits (about two seconds)
     int skip_stage;     // >= 0: diagnostic, the producer leaves this stage of its first work item out
 };
@@ -133,15 +137,21 @@ struct Geo {
     static_assert((SC_FLOATS * 4) % 128 == 0 && (SB_OFF * 4) % 128 == 0 && C::scale_off % 1024 == 0, "TMA destinations of the scale boxes are 128-byte aligned");
 };
 
-// Work item -> tile and K-stage range.  Items of one split are consecutive, so CTAs that run together work on
-// different tiles of the same K range.
-__device__ __forceinline__ void item_range(int item, int num_tiles, int nks, int stages_per_split, int& tile, int& split,
-                                           int& ks0, int& ks1) {
-    tile = item % num_tiles;
-    split = item / num_tiles;
-    ks0 = split * stages_per_split;
-    ks1 = ks0 + stages_per_split;
-    if (ks1 > nks) ks1 = nks;
+// Work item -> tile and K-stage range.  Items of one split are consecutive, so CTAs that run together work on different
+// tiles of the same K range.  `slot` is the item's place in the workspace, -1 where tiles are not divided.
+__device__ __forceinline__ void item_range(int item, const TcParams& p, int nks, int& tile, int& slot, int& ks0, int& ks1) {
+    if (p.ksplit == 1) {
+        tile = item;
+        slot = -1;
+        ks0 = 0;
+        ks1 = nks;
+    } else {
+        const int tiles = p.tiles_m * p.tiles_n, split = item / tiles;
+        tile = item - split * tiles;
+        slot = tile * p.ksplit + split;
+        ks0 = split * p.stages_per_split;
+        ks1 = ks0 + p.stages_per_split < nks ? ks0 + p.stages_per_split : nks;
+    }
 }
 
 template <int BN>
@@ -223,6 +233,95 @@ __device__ __forceinline__ void fold_columns(const uint32_t (&S)[NC], uint32_t s
     }
 }
 
+// Place of (lane quarter, column slice, group of eight columns, row of the quarter) in a workspace slot: a warp stores 1 KiB
+// runs, a thread 32 bytes of its row, and the reduction kernel reads a row's eight columns as one sector.
+template <int PW, int COLS>
+__host__ __device__ constexpr int ws_index(int quarter, int slice, int group, int row) {
+    return (((quarter * PW + slice) * (COLS / 8) + group) * 32 + row) * 8;
+}
+
+// element n of a vector of type `dt`
+__device__ __forceinline__ float load_as_f32(const void* v, int dt, int64_t n) {
+    if (dt == BI8_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(v)[n]);
+    if (dt == BI8_F16) return __half2float(static_cast<const __half*>(v)[n]);
+    return static_cast<const float*>(v)[n];
+}
+// elements n .. n + live - 1 (at most eight), all requested before the first is used; the rest reads as zero
+__device__ __forceinline__ void load8_as_f32(float (&f)[8], const void* v, int dt, int64_t n, int live) {
+    if (dt == BI8_F32) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) f[u] = u < live ? __ldcg(static_cast<const float*>(v) + n + u) : 0.0f;
+    } else {
+        uint16_t h[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) h[u] = u < live ? __ldcg(static_cast<const unsigned short*>(v) + n + u) : (unsigned short)0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) f[u] = dt == BI8_BF16 ? bf16lo(h[u]) : __half2float(__ushort_as_half(h[u]));
+    }
+}
+// a + b where both have (a) or are first rounded to (b) the 16-bit type: the sum rounded once more (reference lines 127-131)
+__device__ __forceinline__ uint32_t add_rounded(uint32_t a16, float b, bool bf) {
+    if (bf) return pack_bf16x2(__fadd_rn(bf16lo(a16), __bfloat162float(__float2bfloat16_rn(b))), 0.0f) & 0xffffu;
+    const float a = __half2float(__ushort_as_half((unsigned short)a16));
+    return (uint32_t)__half_as_ushort(__float2half_rn(__fadd_rn(a, __half2float(__float2half_rn(b)))));
+}
+
+// One staged 16-byte piece (8 values of a 16-bit type or 4 of fp32) plus a vector of addends, value by value.
+template <typename Addend>
+__device__ __forceinline__ void add_piece(uint32_t addr, bool wide, bool bf, Addend addend) {
+    uint32_t w[4];
+    lds_v4(addr, w[0], w[1], w[2], w[3]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        if (wide) w[u] = __float_as_uint(__fadd_rn(__uint_as_float(w[u]), addend(u)));
+        else w[u] = add_rounded(w[u] & 0xffffu, addend(2 * u), bf) | (add_rounded(w[u] >> 16, addend(2 * u + 1), bf) << 16);
+    }
+    sts_v4(addr, w[0], w[1], w[2], w[3]);
+}
+
+// Adds bias[n] and then residual[m, n], each in the output type, to a thread's staged row (COLS 16-bit or COLS/2 fp32 values at
+// shared address `row_addr`, columns from col0).  Columns and rows outside the output get no addend; they are not stored.
+template <int COLS>
+__device__ __forceinline__ void add_staged(const TcParams& p, uint32_t row_addr, int m, int col0, bool wide) {
+    const bool bf = p.out_dtype == BI8_BF16;
+    const int per = wide ? 4 : 8;                       // elements of a 16-byte piece
+    const int left = p.N - col0;
+    if (p.bias != nullptr) {
+#pragma unroll 1
+        for (int g = 0; g < COLS / 8; ++g)
+            add_piece(row_addr + (uint32_t)(g * 16), wide, bf, [&](int e) {
+                const int n = g * per + e;
+                return n < left ? load_as_f32(p.bias, p.bias_dtype, col0 + n) : 0.0f;
+            });
+    }
+    if (p.residual != nullptr && m < p.M) {
+        const int64_t r0 = (int64_t)m * p.ldr + col0;
+        if (p.res_vec && COLS / 8 * per <= left) {
+            // the row's pieces are all requested before the first is added
+            uint4 res[COLS / 8];
+#pragma unroll
+            for (int g = 0; g < COLS / 8; ++g)
+                res[g] = __ldcg(reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(p.residual) + (r0 + g * per) * (wide ? 4 : 2)));
+#pragma unroll
+            for (int g = 0; g < COLS / 8; ++g) {
+                const uint32_t rw[4] = {res[g].x, res[g].y, res[g].z, res[g].w};
+                add_piece(row_addr + (uint32_t)(g * 16), wide, bf, [&](int e) {
+                    if (wide) return __uint_as_float(rw[e & 3]);
+                    const uint32_t h = (rw[(e >> 1) & 3] >> (16 * (e & 1))) & 0xffffu;
+                    return bf ? bf16lo(h) : __half2float(__ushort_as_half((unsigned short)h));
+                });
+            }
+        } else {
+#pragma unroll 1
+            for (int g = 0; g < COLS / 8; ++g)
+                add_piece(row_addr + (uint32_t)(g * 16), wide, bf, [&](int e) {
+                    const int n = g * per + e;
+                    return n < left ? load_as_f32(p.residual, p.out_dtype, r0 + n) : 0.0f;
+                });
+        }
+    }
+}
+
 template <int QB, int MODE, bool SEED, int PW>
 __global__ void __launch_bounds__(Cfg<PW>::THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -279,6 +378,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    // Launched so that all of the above may run while the preceding kernel finishes; no global memory is touched before this
+    // wait.  Dependents become resident as this kernel's CTAs leave.
+    after_predecessor();
 
     if (warp < kRoleWarps) {
         setmaxnreg_dec<C::ROLE_REGS>();
@@ -296,8 +398,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             constexpr uint32_t kSaBytes = (uint32_t)(G::BPS * kBM * 4), kSbBytes = (uint32_t)(G::BPS * BN * 4);
             const bool tma_sa = kScales && (p.tma_scales & 1), tma_sb = kScales && (p.tma_scales & 2);
             for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-                int tile, split, ks0, ks1, m0, n0;
-                item_range(item, num_tiles, nks, p.stages_per_split, tile, split, ks0, ks1);
+                int tile, slot, ks0, ks1, m0, n0;
+                item_range(item, p, nks, tile, slot, ks0, ks1);
                 tile_coords<BN>(tile, p.tiles_m, m0, n0);
                 for (int ks = ks0; ks < ks1; ++ks) {
                     ok = warp_wait(bar(G::EMPTY_AB + stage), phase ^ 1u, abort_flag, wait_limit);
@@ -406,8 +508,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (++stage == kStages) { stage = 0; phase ^= 1u; }
             };
             for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-                int tile, split, ks0, ks1;
-                item_range(item, num_tiles, nks, p.stages_per_split, tile, split, ks0, ks1);
+                int tile, slot, ks0, ks1;
+                item_range(item, p, nks, tile, slot, ks0, ks1);
                 for (int ks = ks0; ks < ks1 && ok; ks += 3) {
                     issue_stage(std::integral_constant<int, 0>{});
                     if (ks + 1 < ks1 && ok) issue_stage(std::integral_constant<int, 1>{});
@@ -535,8 +637,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         };
 
         for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-            int tile, split, ks0, ks1, m0, n0;
-            item_range(item, num_tiles, nks, p.stages_per_split, tile, split, ks0, ks1);
+            int tile, slot, ks0, ks1, m0, n0;
+            item_range(item, p, nks, tile, slot, ks0, ks1);
             tile_coords<BN>(tile, p.tiles_m, m0, n0);
             m = m0 + row;
             nbase = n0 + slice * COLS;
@@ -551,29 +653,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             if (!ok) break;
 
-            if (MODE == 0) {
+            if (MODE == 0 && slot >= 0) {
+                // Part of a divided tile: straight from the registers to the item's workspace slot, in the order in which
+                // the reduction kernel reads it (ws_index: 32 bytes of one row per thread and step).
+                float* dst = p.ws + (int64_t)slot * p.slot_floats + ws_index<PW, COLS>(quarter, slice, 0, lane);
+                const bool live = quarter * 32 * BN < p.slot_floats;
+#pragma unroll
+                for (int g = 0; g < COLS / 8; ++g) {
+                    if (!live) break;
+                    float v[8];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) unpack_f32x2(acc2[4 * g + u], v[2 * u], v[2 * u + 1]);
+                    float4* d4 = reinterpret_cast<float4*>(dst + g * 256);
+                    d4[0] = make_float4(v[0], v[1], v[2], v[3]);
+                    d4[1] = make_float4(v[4], v[5], v[6], v[7]);
+                }
+            } else if (MODE == 0) {
                 // The tile leaves through the warp's staging area in shared memory: every lane writes its row's share
                 // (ROWB bytes), then either one TMA store or a loop of coalesced stores moves the 32 x ROWB bytes out.
-                // 2-byte outputs take one pass of COLS columns, 4-byte outputs (fp32, split-K partial sums) two passes of
-                // COLS / 2.  Addresses are derived here from the thread index rather than kept in registers through the
-                // K loop, whose register budget is full.
+                // 2-byte outputs take one pass of COLS columns, 4-byte outputs two passes of COLS / 2.  Addresses are
+                // derived here from the thread index rather than kept in registers through the K loop, whose register
+                // budget is full.  Bias and residual are added to the staged row by a loop of its own: with their code
+                // unrolled between the casts the epilogue was 1.1 us per tile (instruction fetch), a third of a K = 512 tile.
                 constexpr uint32_t ROWB = (uint32_t)(COLS * 2);
                 uint32_t tid_now;
                 asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid_now));
                 const uint32_t ln = tid_now & 31u;
                 const uint32_t out_stage = base + G::out_off + ((tid_now >> 5) - (uint32_t)kRoleWarps) * G::OUT_WARP_BYTES;
                 const uint32_t my_row = out_stage + ln * ROWB;
-                const bool partial = p.ksplit > 1;
-                const bool wide = partial || p.out_dtype == BI8_F32;
-                const bool bf = p.out_dtype == BI8_BF16;
-                const bool has_bias = p.bias != nullptr && !partial;   // split-K: cast and bias happen in the reduction
+                const bool wide = p.out_dtype == BI8_F32;
                 const int row0 = m - (int)ln;                         // first row of the warp's part
-                auto bias_at = [&](int n) -> float {
-                    if (n >= p.N) return 0.0f;
-                    if (p.bias_dtype == BI8_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n]);
-                    if (p.bias_dtype == BI8_F16) return __half2float(static_cast<const __half*>(p.bias)[n]);
-                    return static_cast<const float*>(p.bias)[n];
-                };
                 const int passes = wide ? 2 : 1;
 #pragma unroll 1
                 for (int ps = 0; ps < passes; ++ps) {
@@ -587,16 +696,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             float v[4];
                             unpack_f32x2(acc2[2 * g], v[0], v[1]);
                             unpack_f32x2(acc2[2 * g + 1], v[2], v[3]);
-                            if (has_bias) {
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) v[u] = __fadd_rn(v[u], bias_at(col0 + g * 4 + u));
-                            }
                             sts_v4(my_row + (uint32_t)(g * 16), __float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]),
                                    __float_as_uint(v[3]));
                         }
                         // the second pass finds its columns where the first found its own
 #pragma unroll
                         for (int i = 0; i < COLS / 4; ++i) acc2[i] = acc2[i + COLS / 4];
+                    } else if (p.out_dtype == BI8_BF16) {
+#pragma unroll
+                        for (int g = 0; g < COLS / 8; ++g) {
+                            uint32_t w[4];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                float lo, hi;
+                                unpack_f32x2(acc2[g * 4 + u], lo, hi);
+                                w[u] = pack_bf16x2(lo, hi);
+                            }
+                            sts_v4(my_row + (uint32_t)(g * 16), w[0], w[1], w[2], w[3]);
+                        }
                     } else {
 #pragma unroll
                         for (int g = 0; g < COLS / 8; ++g) {
@@ -605,26 +722,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             for (int u = 0; u < 4; ++u) {
                                 float lo, hi;
                                 unpack_f32x2(acc2[g * 4 + u], lo, hi);
-                                uint32_t pk = bf ? pack_bf16x2(lo, hi) : pack_f16x2(lo, hi);
-                                if (has_bias) {
-                                    // the reference adds the bias after the cast, in the output type (lines 127-131)
-                                    const int n = col0 + g * 8 + 2 * u;
-                                    const float blo = bias_at(n), bhi = bias_at(n + 1);
-                                    if (bf) {
-                                        uint32_t bb = pack_bf16x2(blo, bhi);
-                                        pk = pack_bf16x2(__fadd_rn(bf16lo(pk), bf16lo(bb)), __fadd_rn(bf16hi(pk), bf16hi(bb)));
-                                    } else {
-                                        __half2 a2 = *reinterpret_cast<__half2*>(&pk);
-                                        __half2 b2 = __floats2half2_rn(blo, bhi);
-                                        float2 af = __half22float2(a2), bfv = __half22float2(b2);
-                                        pk = pack_f16x2(__fadd_rn(af.x, bfv.x), __fadd_rn(af.y, bfv.y));
-                                    }
-                                }
-                                w[u] = pk;
+                                w[u] = pack_f16x2(lo, hi);
                             }
                             sts_v4(my_row + (uint32_t)(g * 16), w[0], w[1], w[2], w[3]);
                         }
                     }
+                    if (p.bias != nullptr || p.residual != nullptr) add_staged<COLS>(p, my_row, m, col0, wide);
                     if (p.tma_store) {
                         // rows and columns of the box that lie outside the tensor are not written
                         fence_proxy_async_smem();
@@ -634,20 +737,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             tma_store_commit();
                         }
                     } else {
-                        // Destinations that a tensor map cannot describe (base or row pitch not 16-byte aligned) and
-                        // split-K partial sums: consecutive lanes store consecutive 4-byte words of a row, or 2-byte
-                        // elements where the rows of a 16-bit output are not all 4-byte aligned.
+                        // Destinations that a tensor map cannot describe (base or row pitch not 16-byte aligned):
+                        // consecutive lanes store consecutive 4-byte words of a row, or 2-byte elements where the rows of
+                        // a 16-bit output are not all 4-byte aligned.
                         __syncwarp();
                         const int esz = wide ? 4 : 2;
-                        unsigned char* dst;
-                        int64_t pitch;
-                        if (partial) {
-                            pitch = (int64_t)p.N * 4;
-                            dst = reinterpret_cast<unsigned char*>(p.ws) + ((int64_t)split * p.M + row0) * pitch + (int64_t)col0 * 4;
-                        } else {
-                            pitch = p.ldc * esz;
-                            dst = static_cast<unsigned char*>(p.C) + (int64_t)row0 * pitch + (int64_t)col0 * esz;
-                        }
+                        const int64_t pitch = p.ldc * esz;
+                        unsigned char* dst = static_cast<unsigned char*>(p.C) + (int64_t)row0 * pitch + (int64_t)col0 * esz;
                         const int rows_valid = p.M - row0;                         // may exceed 32 or be negative
                         const int cols_left = p.N - col0;
                         const int cols_pass = wide ? COLS / 2 : COLS;
@@ -695,62 +791,81 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
 }
 
-// Split-K reduction: C[m,n] = cast(sum_s ws[s,m,n]) (+ cast(bias[n]) in the output type).  The splits are added in
-// ascending order, so the result does not depend on scheduling.  VEC = 4: a thread takes four consecutive columns of a row
-// (16-byte loads of every split, all in flight before the first addition); VEC = 1 for N not a multiple of 4.
-template <int VEC>
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ ws, int ksplit, const void* __restrict__ bias,
-                                                            int bias_dtype, void* __restrict__ C, int64_t ldc, int out_dtype,
-                                                            int M, int N) {
-    const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * VEC;
-    const int64_t total = (int64_t)M * N;
-    if (i >= total) return;
-    const int m = (int)(i / N), n = (int)(i % N);
-    float acc[VEC];
+// Reduction of the divided tiles: C[m,n] = cast(sum over the tile's parts) (+ cast(bias[n])) (+ residual[m,n]), the parts added
+// in ascending order, so that the result does not depend on scheduling.  A thread takes eight consecutive columns of
+// a row: one 32-byte sector of every part (four parts in flight), one 16-byte store (two for fp32) where C allows it.
+// The parts are at most one slot per SM (12 MB) and come from L2.  Launched as a programmatic dependent of the GEMM:
+// its CTAs are resident as the GEMM's leave.
+template <int BN, int COLS>
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const TcParams p) {
+    after_predecessor();
+    constexpr int GROUPS = BN / 8;                       // groups of eight columns in a tile row
+    const int item = blockIdx.x * 256 + threadIdx.x;
+    const int t = item / (kBM * GROUPS), rem = item - t * (kBM * GROUPS);
+    const int r = rem / GROUPS, cg = rem - r * GROUPS;   // consecutive threads: consecutive columns of a row
+    if (t >= p.tiles_m * p.tiles_n) return;
+    int m0, n0;
+    tile_coords<BN>(t, p.tiles_m, m0, n0);
+    const int m = m0 + r, n = n0 + cg * 8;
+    if (m >= p.M || n >= p.N) return;
+    const int slice = cg / (COLS / 8), group = cg - slice * (COLS / 8);
+    const float* src = p.ws + (int64_t)t * p.ksplit * p.slot_floats + ws_index<BN / COLS, COLS>(r / 32, slice, group, r & 31);
+    const int live = p.N - n < 8 ? p.N - n : 8;
+    const int64_t o = (int64_t)m * p.ldc + n, ro = (int64_t)m * p.ldr + n;
+    float acc[8], bias[8], res[8];
 #pragma unroll
-    for (int u = 0; u < VEC; ++u) acc[u] = 0.0f;
-    for (int s0 = 0; s0 < ksplit; s0 += 4) {
-        float v[4][VEC];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (s0 + q < ksplit) {
-                const float* src = ws + (int64_t)(s0 + q) * total + i;
-                if (VEC == 4) {
-                    const float4 f = __ldcg(reinterpret_cast<const float4*>(src));
-                    v[q][0] = f.x;
-                    if (VEC > 1) { v[q][1 % VEC] = f.y; v[q][2 % VEC] = f.z; v[q][3 % VEC] = f.w; }
-                } else {
-                    v[q][0] = __ldcg(src);
-                }
-            }
-        }
+    for (int u = 0; u < 8; ++u) acc[u] = bias[u] = res[u] = 0.0f;
+    const bool has_bias = p.bias != nullptr, has_res = p.residual != nullptr;
+    if (has_bias) load8_as_f32(bias, p.bias, p.bias_dtype, n, live);
+    if (has_res) load8_as_f32(res, p.residual, p.out_dtype, ro, live);
+    for (int s0 = 0; s0 < p.ksplit; s0 += 4) {
+        float4 v[4][2];
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-            if (s0 + q < ksplit) {
+            if (s0 + q < p.ksplit) {
+                const float4* s4 = reinterpret_cast<const float4*>(src + (int64_t)(s0 + q) * p.slot_floats);
+                v[q][0] = __ldcg(s4);
+                v[q][1] = __ldcg(s4 + 1);
+            }
 #pragma unroll
-                for (int u = 0; u < VEC; ++u) acc[u] = __fadd_rn(acc[u], v[q][u]);
+        for (int q = 0; q < 4; ++q)
+            if (s0 + q < p.ksplit) {
+                const float f[8] = {v[q][0].x, v[q][0].y, v[q][0].z, v[q][0].w, v[q][1].x, v[q][1].y, v[q][1].z, v[q][1].w};
+#pragma unroll
+                for (int u = 0; u < 8; ++u) acc[u] = __fadd_rn(acc[u], f[u]);
             }
     }
-    const bool hb = bias != nullptr;
+    if (p.out_dtype == BI8_F32) {
 #pragma unroll
-    for (int u = 0; u < VEC; ++u) {
-        float bv = 0.0f;
-        if (hb) {
-            if (bias_dtype == BI8_BF16) bv = __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[n + u]);
-            else if (bias_dtype == BI8_F16) bv = __half2float(static_cast<const __half*>(bias)[n + u]);
-            else bv = static_cast<const float*>(bias)[n + u];
+        for (int u = 0; u < 8; ++u) {
+            if (has_bias) acc[u] = __fadd_rn(acc[u], bias[u]);
+            if (has_res) acc[u] = __fadd_rn(acc[u], res[u]);
         }
-        const int64_t o = (int64_t)m * ldc + n + u;
-        if (out_dtype == BI8_F32) {
-            static_cast<float*>(C)[o] = hb ? __fadd_rn(acc[u], bv) : acc[u];
-        } else if (out_dtype == BI8_BF16) {
-            __nv_bfloat16 c = __float2bfloat16_rn(acc[u]);
-            if (hb) c = __float2bfloat16_rn(__fadd_rn(__bfloat162float(c), __bfloat162float(__float2bfloat16_rn(bv))));
-            static_cast<__nv_bfloat16*>(C)[o] = c;
+        float* c = static_cast<float*>(p.C) + o;
+        if (live == 8 && p.vec_store) {
+            reinterpret_cast<float4*>(c)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            reinterpret_cast<float4*>(c)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
         } else {
-            __half c = __float2half_rn(acc[u]);
-            if (hb) c = __float2half_rn(__fadd_rn(__half2float(c), __half2float(__float2half_rn(bv))));
-            static_cast<__half*>(C)[o] = c;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (u < live) c[u] = acc[u];
+        }
+    } else {
+        const bool bf = p.out_dtype == BI8_BF16;
+        uint32_t h[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            h[u] = (bf ? pack_bf16x2(acc[u], 0.0f) : pack_f16x2(acc[u], 0.0f)) & 0xffffu;
+            if (has_bias) h[u] = add_rounded(h[u], bias[u], bf);
+            if (has_res) h[u] = add_rounded(h[u], res[u], bf);
+        }
+        uint16_t* c = static_cast<uint16_t*>(p.C) + o;
+        if (live == 8 && p.vec_store) {
+            *reinterpret_cast<uint4*>(c) = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
+        } else {
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (u < live) c[u] = (uint16_t)h[u];
         }
     }
 }
@@ -819,9 +934,7 @@ int launch_one(const TcMaps& tm, const TcParams& p, int grid, cudaStream_t st) {
         regs_ok = ((1 + PW) * fa.numRegs >= C::ROLE_REGS + PW * C::EPI_REGS && (1 + PW) * 32 * fa.numRegs <= 16384) ? 1 : -1;
     }
     if (regs_ok < 0) return fail(BI8_ERR_CUDA, "tensor-core GEMM: the kernel was compiled with a register count its register moves do not fit");
-    gemm_tc_kernel<QB, MODE, SEED, PW><<<grid, C::THREADS, smem, st>>>(tm.a, tm.b, tm.sa, tm.sb, tm.c, p);
-    BI8_CUDA_TRY(cudaGetLastError());
-    return BI8_OK;
+    return launch_chained(gemm_tc_kernel<QB, MODE, SEED, PW>, grid, C::THREADS, smem, st, tm.a, tm.b, tm.sa, tm.sb, tm.c, p);
 }
 
 // Promotion warps per lane quarter (and with it the tile width) of the kernel that runs.
@@ -836,15 +949,21 @@ int launch_qb(const TcMaps& tm, const TcParams& p, int grid, bool partials, bool
 
 }  // namespace
 
-// Split-K plan: when the output has fewer tiles than the device has SMs (small M), the K stages of every tile are
-// divided over `ksplit` work items so that all SMs stream weights; partial results go to an fp32 workspace
-// [ksplit, M, N] and a second kernel adds them in a fixed order.
+// Split-K plan: when the output has at most half as many tiles as the device has SMs (small M), the K stages of every tile
+// are divided over `ksplit` work items so that all SMs work; partial results go to an fp32 workspace, one slot per
+// item, and a second kernel adds them in a fixed order.  (Dividing the tiles left over after the last full round of a larger
+// output as well would make equal rows of A give unequal bits, depending on the tile they lie in.)
 namespace {
 struct SplitPlan {
     int ksplit = 1;
     int stages_per_split = 0;
+    int slot_floats = 0;
     size_t bytes = 0;
 };
+// A stage (128 K-bytes of a tile) takes about 0.8 us; dividing costs the second kernel and the workspace's round trip,
+// 2.5-4 us: tiles are divided only where each gets at least this many stages shorter.
+constexpr int kSplitGain = 4;
+
 SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int sms) {
     SplitPlan pl;
     const int bn = tc_bn();
@@ -855,12 +974,13 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int sms) {
     int s = (int)(sms / tiles);
     if (s > nks) s = nks;
     if (s > 32) s = 32;
-    while (s > 1 && (size_t)s * (size_t)M * (size_t)N * 4 > (size_t)256 << 20) --s;
-    if (s <= 1) return pl;
     const int spp = (nks + s - 1) / s;
-    pl.ksplit = (nks + spp - 1) / spp;
+    s = (nks + spp - 1) / spp;
+    if (s <= 1 || nks - spp < kSplitGain) return pl;
+    pl.ksplit = s;
     pl.stages_per_split = spp;
-    pl.bytes = pl.ksplit > 1 ? (size_t)pl.ksplit * (size_t)M * (size_t)N * 4 : 0;
+    pl.slot_floats = (int)((M < kBM ? (M + 31) / 32 * 32 : kBM) * bn);
+    pl.bytes = (size_t)tiles * (size_t)s * (size_t)pl.slot_floats * 4;
     return pl;
 }
 }  // namespace
@@ -946,6 +1066,10 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     }
     p.ksplit = pl.ksplit;
     p.stages_per_split = pl.stages_per_split;
+    p.slot_floats = pl.slot_floats;
+    p.residual = g.residual;
+    p.ldr = g.ldr;
+    p.res_vec = (g.residual != nullptr && aligned(g.residual, 16) && (g.ldr * esz) % 16 == 0) ? 1 : 0;
     if (!partials && pl.ksplit == 1 && p.vec_store) {
         // one box = what a promotion warp stages per pass: 32 rows x (its columns, or half of them for 4-byte elements)
         const int cols = bn / kPW;
@@ -964,15 +1088,8 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
         default: return fail(BI8_ERR_BLOCK, "tensor-core GEMM supports block 32, 64, 128 (got %d)", g.block);
     }
     if (rc != BI8_OK || pl.ksplit == 1) return rc;
-    const int64_t total = g.M * g.N;
-    if (g.N % 4 == 0)
-        splitk_reduce_kernel<4><<<(unsigned)((total / 4 + 255) / 256), 256, 0, st>>>(p.ws, pl.ksplit, g.bias, g.bias_dtype, g.C, g.ldc,
-                                                                                 g.out_dtype, (int)g.M, (int)g.N);
-    else
-        splitk_reduce_kernel<1><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(p.ws, pl.ksplit, g.bias, g.bias_dtype, g.C, g.ldc,
-                                                                             g.out_dtype, (int)g.M, (int)g.N);
-    BI8_CUDA_TRY(cudaGetLastError());
-    return BI8_OK;
+    constexpr int kTileItems = kBM * (Cfg<kPW>::BN / 8);
+    return launch_chained(splitk_reduce_kernel<Cfg<kPW>::BN, Cfg<kPW>::COLS>, (unsigned)((tiles * kTileItems + 255) / 256), 256, 0, st, p);
 }
 
 int run_mma_peak_probe(int iters, float* ms, int* sm_count) {

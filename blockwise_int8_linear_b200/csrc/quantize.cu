@@ -65,6 +65,7 @@ template <typename T, int B, int VEC>
 __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
     const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int M, int K, int nb,
     int col_tiles) {
+    after_predecessor();
     constexpr int WCOLS = 32 * VEC;         // columns per warp pass
     constexpr int LPB = B / VEC;            // lanes sharing one block
     constexpr int BPT = WCOLS / B;          // blocks per tile row
@@ -166,6 +167,7 @@ template <typename T, int B>
 __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
     const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int M, int K, int nb,
     int col_units, int64_t total_units) {
+    after_predecessor();
     constexpr int LPB = B / 16;             // lanes sharing one block
     const int lane = threadIdx.x & 31;
     const int64_t gw = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
@@ -289,6 +291,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_rowwise_ragged_kernel(
     const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int64_t K, int B,
     int64_t nb, int64_t groups_per_row) {
+    after_predecessor();
     const int lane = threadIdx.x & 31;
     const int64_t task = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     if (task >= M * groups_per_row) return;
@@ -326,6 +329,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_rowwise_generic_kernel(
     const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int64_t K, int B,
     int64_t nb) {
+    after_predecessor();
     const int lane = threadIdx.x & 31;
     const int64_t task = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     if (task >= M * nb) return;
@@ -352,6 +356,7 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_generic_kernel(
 template <typename T, int B>
 __global__ void __launch_bounds__(kThreads) quantize_colwise_vec_kernel(
     const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int R, int C, int col_tiles) {
+    after_predecessor();
     constexpr int TC = 128;
     constexpr int NBLK = kThreads / TC;     // blocks (along rows of x) per tile
     constexpr int TR = NBLK * B;
@@ -443,6 +448,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_colwise_ragged_kernel(
     const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int64_t R, int64_t C, int B,
     int64_t col_tiles) {
+    after_predecessor();
     extern __shared__ unsigned char tile[];                 // [kThreads][B + 4]
     const int pitch = B + 4;
     const int64_t j = blockIdx.x / col_tiles, c0 = (blockIdx.x % col_tiles) * kThreads;
@@ -475,6 +481,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_colwise_generic_kernel(
     const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int64_t R, int64_t C, int B,
     int64_t nb) {
+    after_predecessor();
     const int64_t task = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (task >= nb * C) return;
     const int64_t j = task / C, c = task % C;
@@ -517,6 +524,7 @@ template <typename TO, int B>
 __global__ void __launch_bounds__(kThreads) dequantize_rowwise_vec_kernel(
     const int8_t* __restrict__ q, const float* __restrict__ s, TO* __restrict__ out, int M, int K, int nb,
     int col_tiles) {
+    after_predecessor();
     constexpr int WCOLS = 512;
     constexpr int BPT = WCOLS / B;
     constexpr int LPB = B / 16;
@@ -567,6 +575,7 @@ __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <typename TO>
 __global__ void __launch_bounds__(kThreads) dequantize_rowwise_generic_kernel(
     const int8_t* __restrict__ q, const float* __restrict__ s, TO* __restrict__ out, int64_t M, int64_t K, int B) {
+    after_predecessor();
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (i >= M * K) return;
     const int64_t m = i / K, k = i % K;
@@ -590,10 +599,7 @@ int quantize_rowwise_t(const T* x, int64_t ldx, int8_t* q, float* s, int64_t M, 
     do {                                                                                                   \
         const int64_t ctiles = (K + 32 * VV - 1) / (32 * VV);                                              \
         if (row_tiles * ctiles >= (1ll << 31)) break;                                                      \
-        quantize_rowwise_vec_kernel<T, BB, VV><<<(unsigned)(row_tiles * ctiles), kThreads, 0, st>>>(        \
-            x, ldx, q, s, (int)M, (int)K, (int)nb, (int)ctiles);                                           \
-        BI8_CUDA_TRY(cudaGetLastError());                                                                  \
-        return BI8_OK;                                                                                     \
+        return launch_chained(quantize_rowwise_vec_kernel<T, BB, VV>, (unsigned)(row_tiles * ctiles), kThreads, 0, st, x, ldx, q, s, (int)M, (int)K, (int)nb, (int)ctiles);                                                                                     \
     } while (0)
     if constexpr (sizeof(T) == 2) {
         if (v16 && aligned(s, 16) && (block == 32 || block == 64 || block == 128 || block == 256)) {
@@ -607,10 +613,7 @@ int quantize_rowwise_t(const T* x, int64_t ldx, int8_t* q, float* s, int64_t M, 
             if (ctas > 2ll * sms) ctas = 2ll * sms;                  // two resident CTAs per SM, persistent beyond that
 #define BI8_QSTREAM(BB)                                                                                          \
     if (block == BB) {                                                                                           \
-        quantize_rowwise_stream_kernel<T, BB><<<(unsigned)ctas, kThreads, 0, st>>>(x, ldx, q, s, (int)M, (int)K,  \
-                                                                                   (int)nb, col_units, total);   \
-        BI8_CUDA_TRY(cudaGetLastError());                                                                        \
-        return BI8_OK;                                                                                           \
+        return launch_chained(quantize_rowwise_stream_kernel<T, BB>, (unsigned)ctas, kThreads, 0, st, x, ldx, q, s, (int)M, (int)K, (int)nb, col_units, total);                                                                                           \
     }
             BI8_QSTREAM(32) BI8_QSTREAM(64) BI8_QSTREAM(128) BI8_QSTREAM(256)
 #undef BI8_QSTREAM
@@ -633,17 +636,13 @@ int quantize_rowwise_t(const T* x, int64_t ldx, int8_t* q, float* s, int64_t M, 
         const int64_t gpr = (nb + kRagGroup - 1) / kRagGroup;
         const int64_t rgrid = (M * gpr + kThreads / 32 - 1) / (kThreads / 32);
         if (rgrid < (1ll << 31)) {
-            quantize_rowwise_ragged_kernel<T><<<(unsigned)rgrid, kThreads, 0, st>>>(x, ldx, q, s, M, K, block, nb, gpr);
-            BI8_CUDA_TRY(cudaGetLastError());
-            return BI8_OK;
+            return launch_chained(quantize_rowwise_ragged_kernel<T>, (unsigned)rgrid, kThreads, 0, st, x, ldx, q, s, M, K, block, nb, gpr);
         }
     }
     const int64_t tasks = M * nb;
     const int64_t grid = (tasks + kThreads / 32 - 1) / (kThreads / 32);
     if (grid >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "quantize_rowwise: %lld blocks exceed the grid limit", (long long)tasks);
-    quantize_rowwise_generic_kernel<T><<<(unsigned)grid, kThreads, 0, st>>>(x, ldx, q, s, M, K, block, nb);
-    BI8_CUDA_TRY(cudaGetLastError());
-    return BI8_OK;
+    return launch_chained(quantize_rowwise_generic_kernel<T>, (unsigned)grid, kThreads, 0, st, x, ldx, q, s, M, K, block, nb);
 }
 
 template <typename T, int B>
@@ -655,9 +654,7 @@ int colwise_vec(const T* x, int64_t ldx, int8_t* q, float* s, int64_t R, int64_t
     static SmemOptIn opt_in;                // per kernel instance; set once per device
     const int rc = opt_in.ensure(quantize_colwise_vec_kernel<T, B>, smem);
     if (rc != BI8_OK) return rc;
-    quantize_colwise_vec_kernel<T, B><<<(unsigned)(ctiles * rtiles), kThreads, smem, st>>>(x, ldx, q, s, (int)R, (int)C, (int)ctiles);
-    BI8_CUDA_TRY(cudaGetLastError());
-    return BI8_OK;
+    return launch_chained(quantize_colwise_vec_kernel<T, B>, (unsigned)(ctiles * rtiles), kThreads, smem, st, x, ldx, q, s, (int)R, (int)C, (int)ctiles);
 }
 
 template <typename T>
@@ -680,16 +677,12 @@ int quantize_colwise_t(const T* x, int64_t ldx, int8_t* q, float* s, int64_t R, 
                 const int rc = opt_in.ensure(quantize_colwise_ragged_kernel<T>, smem);
                 if (rc != BI8_OK) return rc;
             }
-            quantize_colwise_ragged_kernel<T><<<(unsigned)(nb * col_tiles), kThreads, smem, st>>>(x, ldx, q, s, R, C, block, col_tiles);
-            BI8_CUDA_TRY(cudaGetLastError());
-            return BI8_OK;
+            return launch_chained(quantize_colwise_ragged_kernel<T>, (unsigned)(nb * col_tiles), kThreads, smem, st, x, ldx, q, s, R, C, block, col_tiles);
         }
     }
     const int64_t grid = (nb * C + kThreads - 1) / kThreads;
     if (grid >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "quantize_colwise: grid too large");
-    quantize_colwise_generic_kernel<T><<<(unsigned)grid, kThreads, 0, st>>>(x, ldx, q, s, R, C, block, nb);
-    BI8_CUDA_TRY(cudaGetLastError());
-    return BI8_OK;
+    return launch_chained(quantize_colwise_generic_kernel<T>, (unsigned)grid, kThreads, 0, st, x, ldx, q, s, R, C, block, nb);
 }
 
 template <typename TO>
@@ -700,19 +693,14 @@ int dequantize_t(const int8_t* q, const float* s, TO* out, int64_t M, int64_t K,
     if (vec && row_tiles * ctiles < (1ll << 31)) {
 #define BI8_DEQ(BB)                                                                                         \
     if (block == BB) {                                                                                      \
-        dequantize_rowwise_vec_kernel<TO, BB><<<(unsigned)(row_tiles * ctiles), kThreads, 0, st>>>(           \
-            q, s, out, (int)M, (int)K, (int)nb, (int)ctiles);                                               \
-        BI8_CUDA_TRY(cudaGetLastError());                                                                   \
-        return BI8_OK;                                                                                      \
+        return launch_chained(dequantize_rowwise_vec_kernel<TO, BB>, (unsigned)(row_tiles * ctiles), kThreads, 0, st, q, s, out, (int)M, (int)K, (int)nb, (int)ctiles);                                                                                      \
     }
         BI8_DEQ(32) BI8_DEQ(64) BI8_DEQ(128) BI8_DEQ(256)
 #undef BI8_DEQ
     }
     const int64_t grid = (M * K + kThreads - 1) / kThreads;
     if (grid >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "dequantize: grid too large");
-    dequantize_rowwise_generic_kernel<TO><<<(unsigned)grid, kThreads, 0, st>>>(q, s, out, M, K, block);
-    BI8_CUDA_TRY(cudaGetLastError());
-    return BI8_OK;
+    return launch_chained(dequantize_rowwise_generic_kernel<TO>, (unsigned)grid, kThreads, 0, st, q, s, out, M, K, block);
 }
 
 }  // namespace

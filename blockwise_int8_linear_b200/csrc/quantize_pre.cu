@@ -158,8 +158,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quan
                                                                        const void* __restrict__ weight, float eps,
                                                                        int8_t* __restrict__ q, float* __restrict__ sx, int M, int K,
                                                                        int nb, int vec_in, int vec_out) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");           // a no-op unless launched as a programmatic dependent
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    after_predecessor();
     constexpr int LPB = QB / 8;
     constexpr int dt = DT;                                        // the element type is a template parameter: no per-element tests
     __shared__ float warp_sum[THREADS / 32];
@@ -249,8 +248,7 @@ __global__ void __launch_bounds__(kPreThreads) silu_mul_quantize_kernel(const vo
                                                                         int64_t ldx, int8_t* __restrict__ q,
                                                                         float* __restrict__ sx, int M, int K, int nb, int vec_in,
                                                                         int vec_out) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");           // a no-op unless launched as a programmatic dependent
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    after_predecessor();
     constexpr int LPB = QB / 8;
     constexpr int dt = DT;
     const int upr = nb * LPB;
@@ -276,6 +274,7 @@ __global__ void __launch_bounds__(kPreThreads) silu_mul_quantize_kernel(const vo
 // C[m, n] = cast(C[m, n] + R[m, n]): the addition a layer's `x + proj(...)` performs in the activation type
 __global__ void __launch_bounds__(kPreThreads) residual_add_kernel(void* C, int64_t ldc, const void* R, int64_t ldr, int dt, int64_t M,
                                                                    int64_t N) {
+    after_predecessor();
     const int64_t i = (int64_t)blockIdx.x * kPreThreads + threadIdx.x;
     if (i >= M * N) return;
     const int64_t m = i / N, n = i % N, c = m * ldc + n, r = m * ldr + n;
@@ -296,9 +295,7 @@ int launch_residual_add(void* C, int64_t ldc, const void* R, int64_t ldr, int dt
     if (M <= 0 || N <= 0) return BI8_OK;
     const int64_t blocks = (M * N + kPreThreads - 1) / kPreThreads;
     if (blocks > 0x7fffffff) return fail(BI8_ERR_LIMIT, "residual add: more than 2^31 blocks");
-    residual_add_kernel<<<(unsigned)blocks, kPreThreads, 0, st>>>(C, ldc, R, ldr, dt, M, N);
-    BI8_CUDA_TRY(cudaGetLastError());
-    return BI8_OK;
+    return launch_chained(residual_add_kernel, (unsigned)blocks, kPreThreads, 0, st, C, ldc, R, ldr, dt, M, N);
 }
 
 int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t ldx, const void* weight, float eps, int8_t* q, float* sx,
@@ -311,26 +308,16 @@ int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t l
     const int vec_in = rows16 && aligned(x, 16) && (!x2 || aligned(x2, 16)) && (!weight || aligned(weight, 16));
     const int vec_out = K % 8 == 0 && aligned(q, 8);
     if (op == BI8_PRE_NONE) return launch_quantize_rowwise(x, dt, ldx, q, sx, M, K, block, st);
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = M <= 64 ? 1 : 0;       // decode: resident while the predecessor finishes (the kernels wait for it themselves)
     const int Mi = (int)M, Ki = (int)K;
     if (op == BI8_PRE_RMSNORM) {
         // 128 threads per row where the row fits their registers and there are rows enough to fill the SMs ten deep; a
         // handful of decode rows finish sooner with 256 threads each
         const bool narrow = (int64_t)nb * (block / 8) <= kPreHold * 128 && M > 1024;
-        cfg.gridDim = dim3((unsigned)M);
-        cfg.blockDim = dim3(narrow ? 128 : 256);
 #define BI8_PRE_RMS_T(QB, T)                                                                                                          \
     do {                                                                                                                             \
-        if (dt == BI8_BF16) BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, rmsnorm_quantize_kernel<QB, T, BI8_BF16>, x, ldx, weight, eps, q, sx, Mi, Ki, nb, vec_in, vec_out)); \
-        else if (dt == BI8_F16) BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, rmsnorm_quantize_kernel<QB, T, BI8_F16>, x, ldx, weight, eps, q, sx, Mi, Ki, nb, vec_in, vec_out)); \
-        else BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, rmsnorm_quantize_kernel<QB, T, BI8_F32>, x, ldx, weight, eps, q, sx, Mi, Ki, nb, vec_in, vec_out)); \
+        if (dt == BI8_BF16) return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_BF16>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, sx, Mi, Ki, nb, vec_in, vec_out); \
+        else if (dt == BI8_F16) return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_F16>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, sx, Mi, Ki, nb, vec_in, vec_out); \
+        else return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_F32>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, sx, Mi, Ki, nb, vec_in, vec_out); \
     } while (0)
 #define BI8_PRE_RMS(QB)                                                                                                              \
     if (narrow) BI8_PRE_RMS_T(QB, 128);                                                                                              \
@@ -346,13 +333,12 @@ int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t l
     } else if (op == BI8_PRE_SILU_MUL) {
         if (!x2) return fail(BI8_ERR_NULL, "quantize_pre: the gated activation needs its second operand");
         const int64_t units = M * nb * (block / 8);
-        cfg.gridDim = dim3((unsigned)((units + kPreThreads - 1) / kPreThreads));
-        cfg.blockDim = dim3(kPreThreads);
+        const unsigned grid = (unsigned)((units + kPreThreads - 1) / kPreThreads);
 #define BI8_PRE_SILU(QB)                                                                                                             \
     do {                                                                                                                             \
-        if (dt == BI8_BF16) BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, silu_mul_quantize_kernel<QB, BI8_BF16>, x, x2, ldx, q, sx, Mi, Ki, nb, vec_in, vec_out)); \
-        else if (dt == BI8_F16) BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, silu_mul_quantize_kernel<QB, BI8_F16>, x, x2, ldx, q, sx, Mi, Ki, nb, vec_in, vec_out)); \
-        else BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, silu_mul_quantize_kernel<QB, BI8_F32>, x, x2, ldx, q, sx, Mi, Ki, nb, vec_in, vec_out)); \
+        if (dt == BI8_BF16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_BF16>, grid, kPreThreads, 0, st, x, x2, ldx, q, sx, Mi, Ki, nb, vec_in, vec_out); \
+        else if (dt == BI8_F16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_F16>, grid, kPreThreads, 0, st, x, x2, ldx, q, sx, Mi, Ki, nb, vec_in, vec_out); \
+        else return launch_chained(silu_mul_quantize_kernel<QB, BI8_F32>, grid, kPreThreads, 0, st, x, x2, ldx, q, sx, Mi, Ki, nb, vec_in, vec_out); \
     } while (0)
         switch (block) {
             case 32: BI8_PRE_SILU(32); break;

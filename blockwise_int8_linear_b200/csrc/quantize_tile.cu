@@ -165,6 +165,9 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
         sts_u32(abort_flag, 0u);
         mbar_fence_init();
         fence_proxy_async_smem();
+    }
+    after_predecessor();
+    if (tid == 0) {
         for (int s = 0; s < NST - 1; ++s) {
             const int64_t t0 = (int64_t)blockIdx.x + (int64_t)s * gridDim.x;
             if (t0 < num_tiles) issue((int)t0, s);
@@ -418,10 +421,7 @@ int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap
     const int64_t tiles = ctiles * rtiles;
     const int64_t resident = (int64_t)(DUAL ? 1 : 2) * di.sms;                 // CTAs that fit at once
     const int grid = (int)(tiles < resident ? tiles : resident);
-    quantize_tile_kernel<T, B, DUAL><<<grid, DUAL ? 2 * kQThreads : kQThreads, smem, st>>>(tx, tqc, tqr, s_col, s_row, (int)R, (int)C,
-                                                                                        (int)ctiles, (int)tiles, status);
-    BI8_CUDA_TRY(cudaGetLastError());
-    return BI8_OK;
+    return launch_chained(quantize_tile_kernel<T, B, DUAL>, grid, DUAL ? 2 * kQThreads : kQThreads, smem, st, tx, tqc, tqr, s_col, s_row, (int)R, (int)C, (int)ctiles, (int)tiles, status);
 }
 
 template <typename T>

@@ -9,6 +9,8 @@
 // device memory, so the launch can be captured in a CUDA graph and replayed while the position advances.
 #include "bi8_common.cuh"
 
+#include <type_traits>
+
 namespace bi8 {
 namespace {
 
@@ -39,6 +41,7 @@ __global__ void __launch_bounds__(256) rope_cache_append_kernel(const T* __restr
                                                                 const long long* __restrict__ pos, T* __restrict__ q_out,
                                                                 T* __restrict__ kcache, T* __restrict__ vcache, int B, int H, int D,
                                                                 int max_len) {
+    after_predecessor();
     const int half = D / 2;
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= (int64_t)B * H * half) return;
@@ -64,16 +67,12 @@ int launch_rope_cache_append(const void* qkv, int dt, const float* cis, const lo
     const int64_t n = B * H * (D / 2);
     if (n == 0) return BI8_OK;
     const unsigned grid = (unsigned)((n + 255) / 256);
-    if (dt == BI8_BF16)
-        rope_cache_append_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-            static_cast<const __nv_bfloat16*>(qkv), reinterpret_cast<const float2*>(cis), pos, static_cast<__nv_bfloat16*>(q_out),
-            static_cast<__nv_bfloat16*>(kcache), static_cast<__nv_bfloat16*>(vcache), (int)B, (int)H, (int)D, (int)max_len);
-    else
-        rope_cache_append_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(qkv), reinterpret_cast<const float2*>(cis), pos,
-                                                              static_cast<__half*>(q_out), static_cast<__half*>(kcache),
-                                                              static_cast<__half*>(vcache), (int)B, (int)H, (int)D, (int)max_len);
-    BI8_CUDA_TRY(cudaGetLastError());
-    return BI8_OK;
+    auto launch = [&](auto* type_tag) {
+        using T = std::remove_pointer_t<decltype(type_tag)>;
+        return launch_chained(rope_cache_append_kernel<T>, grid, 256, 0, st, static_cast<const T*>(qkv), reinterpret_cast<const float2*>(cis), pos,
+                              static_cast<T*>(q_out), static_cast<T*>(kcache), static_cast<T*>(vcache), (int)B, (int)H, (int)D, (int)max_len);
+    };
+    return dt == BI8_BF16 ? launch(static_cast<__nv_bfloat16*>(nullptr)) : launch(static_cast<__half*>(nullptr));
 }
 
 }  // namespace bi8
