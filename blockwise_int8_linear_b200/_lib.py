@@ -28,6 +28,8 @@ EXPORTS = [
     "bi8_gemm_wait_selftest", "bi8_stream_capture_id", "bi8_quantize_rowwise_pre", "bi8_gemm_dequant_fused_pre",
     "bi8_row_parallel_linear_pre", "bi8_peer_allreduce_large", "bi8_peer_allreduce_large_buffer_bytes",
     "bi8_peer_allreduce_large_partial_offset", "bi8_peer_allreduce_large_out_offset", "bi8_rope_cache_append",
+    "bi8_gemm_dequant_residual", "bi8_quantize_rowwise_pitched", "bi8_quantize_colwise_pitched", "bi8_quantize_dual_pitched",
+    "bi8_quantize_rowwise_pre_pitched", "bi8_dequantize_rowwise_pitched",
 ]
 ADDEND_FULL = 0x100
 PRE_NONE, PRE_RMSNORM, PRE_SILU_MUL = 0, 1, 2
@@ -57,6 +59,12 @@ def lib() -> ctypes.CDLL:
         L.bi8_quantize_colwise.argtypes = [vp, i32, i64, vp, vp, i64, i64, i32, vp]
         L.bi8_quantize_dual.argtypes = [vp, i32, i64, vp, vp, vp, vp, i64, i64, i32, vp]
         L.bi8_dequantize_rowwise.argtypes = [vp, vp, vp, i32, i64, i64, i32, vp]
+        L.bi8_gemm_dequant_residual.argtypes = [vp, i64, vp, i64, vp, vp, vp, i32, vp, i64, vp, i64, i32, i64, i64, i64, i32, vp, sz, i32, vp]
+        L.bi8_quantize_rowwise_pitched.argtypes = [vp, i32, i64, vp, i64, vp, i64, i64, i32, vp]
+        L.bi8_quantize_colwise_pitched.argtypes = [vp, i32, i64, vp, i64, vp, i64, i64, i32, vp]
+        L.bi8_quantize_dual_pitched.argtypes = [vp, i32, i64, vp, i64, vp, vp, i64, vp, i64, i64, i32, vp]
+        L.bi8_quantize_rowwise_pre_pitched.argtypes = [i32, vp, vp, i32, i64, vp, c.c_float, vp, i64, vp, i64, i64, i32, vp]
+        L.bi8_dequantize_rowwise_pitched.argtypes = [vp, i64, vp, vp, i32, i64, i64, i32, vp]
         L.bi8_peer_allreduce_buffer_bytes.argtypes = [i32, i64]
         L.bi8_peer_allreduce_buffer_bytes.restype = sz
         L.bi8_row_parallel_linear.argtypes = [vp, i32, i64, vp, vp, vp, i64, vp, vp, i64, i64, i64, i32, vp, sz, c.POINTER(vp), i32, i32,

@@ -128,43 +128,59 @@ int bi8_device_status(int* detail) {
     return BI8_OK;
 }
 
-int bi8_quantize_rowwise(const void* x, int x_dtype, int64_t ldx, int8_t* q, float* s, int64_t M, int64_t K, int block,
-                         void* stream) {
+int bi8_quantize_rowwise_pitched(const void* x, int x_dtype, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t M, int64_t K, int block,
+                                 void* stream) {
     if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "quantize_rowwise: unknown dtype code %d", x_dtype);
     if (block < 1) return fail(BI8_ERR_BLOCK, "quantize_rowwise: block size %d", block);
-    if (M < 0 || K < 0 || ldx < K) return fail(BI8_ERR_SHAPE, "quantize_rowwise: bad shape M=%lld K=%lld ldx=%lld", (long long)M, (long long)K, (long long)ldx);
+    if (M < 0 || K < 0 || ldx < K || ldq < K) return fail(BI8_ERR_SHAPE, "quantize_rowwise: bad shape M=%lld K=%lld ldx=%lld ldq=%lld", (long long)M, (long long)K, (long long)ldx, (long long)ldq);
     if (M == 0 || K == 0) return BI8_OK;
     if (!x || !q || !s) return fail(BI8_ERR_NULL, "quantize_rowwise: null pointer");
     if (!aligned(x, dtype_size(x_dtype)) || !aligned(s, 4)) return fail(BI8_ERR_ALIGN, "quantize_rowwise: pointer not element aligned");
-    return launch_quantize_rowwise(x, x_dtype, ldx, q, s, M, K, block, static_cast<cudaStream_t>(stream));
+    return launch_quantize_rowwise(x, x_dtype, ldx, q, ldq, s, M, K, block, static_cast<cudaStream_t>(stream));
+}
+
+int bi8_quantize_rowwise(const void* x, int x_dtype, int64_t ldx, int8_t* q, float* s, int64_t M, int64_t K, int block,
+                         void* stream) {
+    return bi8_quantize_rowwise_pitched(x, x_dtype, ldx, q, K, s, M, K, block, stream);
+}
+
+int bi8_quantize_colwise_pitched(const void* x, int x_dtype, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t R, int64_t C, int block,
+                                 void* stream) {
+    if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "quantize_colwise: unknown dtype code %d", x_dtype);
+    if (block < 1) return fail(BI8_ERR_BLOCK, "quantize_colwise: block size %d", block);
+    if (R < 0 || C < 0 || ldx < C || ldq < R) return fail(BI8_ERR_SHAPE, "quantize_colwise: bad shape R=%lld C=%lld ldx=%lld ldq=%lld", (long long)R, (long long)C, (long long)ldx, (long long)ldq);
+    if (R == 0 || C == 0) return BI8_OK;
+    if (!x || !q || !s) return fail(BI8_ERR_NULL, "quantize_colwise: null pointer");
+    if (!aligned(x, dtype_size(x_dtype)) || !aligned(s, 4)) return fail(BI8_ERR_ALIGN, "quantize_colwise: pointer not element aligned");
+    return launch_quantize_colwise(x, x_dtype, ldx, q, ldq, s, R, C, block, static_cast<cudaStream_t>(stream));
 }
 
 int bi8_quantize_colwise(const void* x, int x_dtype, int64_t ldx, int8_t* q, float* s, int64_t R, int64_t C, int block,
                          void* stream) {
-    if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "quantize_colwise: unknown dtype code %d", x_dtype);
-    if (block < 1) return fail(BI8_ERR_BLOCK, "quantize_colwise: block size %d", block);
-    if (R < 0 || C < 0 || ldx < C) return fail(BI8_ERR_SHAPE, "quantize_colwise: bad shape R=%lld C=%lld ldx=%lld", (long long)R, (long long)C, (long long)ldx);
-    if (R == 0 || C == 0) return BI8_OK;
-    if (!x || !q || !s) return fail(BI8_ERR_NULL, "quantize_colwise: null pointer");
-    if (!aligned(x, dtype_size(x_dtype)) || !aligned(s, 4)) return fail(BI8_ERR_ALIGN, "quantize_colwise: pointer not element aligned");
-    return launch_quantize_colwise(x, x_dtype, ldx, q, s, R, C, block, static_cast<cudaStream_t>(stream));
+    return bi8_quantize_colwise_pitched(x, x_dtype, ldx, q, R, s, R, C, block, stream);
 }
 
-int bi8_quantize_dual(const void* x, int x_dtype, int64_t ldx, int8_t* q_row, float* s_row, int8_t* q_col, float* s_col, int64_t R,
-                      int64_t C, int block, void* stream) {
+int bi8_quantize_dual_pitched(const void* x, int x_dtype, int64_t ldx, int8_t* q_row, int64_t ldq_row, float* s_row, int8_t* q_col, int64_t ldq_col,
+                              float* s_col, int64_t R, int64_t C, int block, void* stream) {
     if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "quantize_dual: unknown dtype code %d", x_dtype);
     if (block < 1) return fail(BI8_ERR_BLOCK, "quantize_dual: block size %d", block);
-    if (R < 0 || C < 0 || ldx < C) return fail(BI8_ERR_SHAPE, "quantize_dual: bad shape R=%lld C=%lld ldx=%lld", (long long)R, (long long)C, (long long)ldx);
+    if (R < 0 || C < 0 || ldx < C || ldq_row < C || ldq_col < R)
+        return fail(BI8_ERR_SHAPE, "quantize_dual: bad shape R=%lld C=%lld ldx=%lld ldq=%lld, %lld", (long long)R, (long long)C, (long long)ldx, (long long)ldq_row, (long long)ldq_col);
     if (R == 0 || C == 0) return BI8_OK;
     if (!x || !q_row || !s_row || !q_col || !s_col) return fail(BI8_ERR_NULL, "quantize_dual: null pointer");
     if (!aligned(x, dtype_size(x_dtype)) || !aligned(s_row, 4) || !aligned(s_col, 4)) return fail(BI8_ERR_ALIGN, "quantize_dual: pointer not element aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (quantize_tile_applicable(x, x_dtype, ldx, q_col, q_row, R, C, block))
-        return launch_quantize_tile(x, x_dtype, ldx, q_col, s_col, q_row, s_row, R, C, block, st);
-    // shapes the one-pass kernel does not take: the two single-purpose quantizers, same results
-    const int rc = launch_quantize_rowwise(x, x_dtype, ldx, q_row, s_row, R, C, block, st);
+    if (quantize_tile_applicable(x_dtype, q_col, ldq_col, q_row, ldq_row, R, C, block))
+        return launch_quantize_tile(x, x_dtype, ldx, q_col, ldq_col, s_col, q_row, ldq_row, s_row, R, C, block, st);
+    // what the one-pass kernel does not take: the two single-purpose quantizers, same results
+    const int rc = launch_quantize_rowwise(x, x_dtype, ldx, q_row, ldq_row, s_row, R, C, block, st);
     if (rc != BI8_OK) return rc;
-    return launch_quantize_colwise(x, x_dtype, ldx, q_col, s_col, R, C, block, st);
+    return launch_quantize_colwise(x, x_dtype, ldx, q_col, ldq_col, s_col, R, C, block, st);
+}
+
+int bi8_quantize_dual(const void* x, int x_dtype, int64_t ldx, int8_t* q_row, float* s_row, int8_t* q_col, float* s_col, int64_t R,
+                      int64_t C, int block, void* stream) {
+    return bi8_quantize_dual_pitched(x, x_dtype, ldx, q_row, C, s_row, q_col, R, s_col, R, C, block, stream);
 }
 
 size_t bi8_peer_allreduce_buffer_bytes(int world, int64_t capacity) {
@@ -180,15 +196,20 @@ int bi8_peer_allreduce(void* const* peer_bufs, int rank, int world, int64_t capa
                                  static_cast<cudaStream_t>(stream));
 }
 
-int bi8_dequantize_rowwise(const int8_t* q, const float* s, void* out, int out_dtype, int64_t M, int64_t K, int block,
-                           void* stream) {
+int bi8_dequantize_rowwise_pitched(const int8_t* q, int64_t ldq, const float* s, void* out, int out_dtype, int64_t M, int64_t K, int block,
+                                   void* stream) {
     if (!dtype_ok(out_dtype)) return fail(BI8_ERR_DTYPE, "dequantize: unknown dtype code %d", out_dtype);
     if (block < 1) return fail(BI8_ERR_BLOCK, "dequantize: block size %d", block);
-    if (M < 0 || K < 0) return fail(BI8_ERR_SHAPE, "dequantize: bad shape M=%lld K=%lld", (long long)M, (long long)K);
+    if (M < 0 || K < 0 || ldq < K) return fail(BI8_ERR_SHAPE, "dequantize: bad shape M=%lld K=%lld ldq=%lld", (long long)M, (long long)K, (long long)ldq);
     if (M == 0 || K == 0) return BI8_OK;
     if (!q || !s || !out) return fail(BI8_ERR_NULL, "dequantize: null pointer");
     if (!aligned(out, dtype_size(out_dtype)) || !aligned(s, 4)) return fail(BI8_ERR_ALIGN, "dequantize: pointer not element aligned");
-    return launch_dequantize_rowwise(q, s, out, out_dtype, M, K, block, static_cast<cudaStream_t>(stream));
+    return launch_dequantize_rowwise(q, ldq, s, out, out_dtype, M, K, block, static_cast<cudaStream_t>(stream));
+}
+
+int bi8_dequantize_rowwise(const int8_t* q, const float* s, void* out, int out_dtype, int64_t M, int64_t K, int block,
+                           void* stream) {
+    return bi8_dequantize_rowwise_pitched(q, K, s, out, out_dtype, M, K, block, stream);
 }
 
 size_t bi8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int block) {
@@ -208,6 +229,19 @@ int bi8_gemm_dequant(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb
     GemmArgs g{A, lda, Bt, ldb, sA, sB, bias, bias_dtype, C, ldc, out_dtype, nullptr, M, N, K, block, flags, workspace, workspace_bytes};
     int rc = check_gemm(g, false);
     if (rc != BI8_OK || M == 0 || N == 0) return rc;
+    return dispatch_gemm(g, static_cast<cudaStream_t>(stream));
+}
+
+int bi8_gemm_dequant_residual(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb, const float* sA, const float* sB, const void* bias,
+                              int bias_dtype, const void* residual, int64_t ldr, void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N,
+                              int64_t K, int block, void* workspace, size_t workspace_bytes, int flags, void* stream) {
+    GemmArgs g{A, lda, Bt, ldb, sA, sB, bias, bias_dtype, C, ldc, out_dtype, nullptr, M, N, K, block, flags, workspace, workspace_bytes};
+    int rc = check_gemm(g, false);
+    if (rc != BI8_OK || M == 0 || N == 0) return rc;
+    if (residual && ldr < N) return fail(BI8_ERR_SHAPE, "gemm_dequant_residual: residual row pitch smaller than the row");
+    if (residual && !aligned(residual, dtype_size(out_dtype))) return fail(BI8_ERR_ALIGN, "gemm_dequant_residual: residual not element aligned");
+    g.residual = residual;
+    g.ldr = ldr;
     return dispatch_gemm(g, static_cast<cudaStream_t>(stream));
 }
 
@@ -263,18 +297,23 @@ int bi8_gemm_dequant_fused_quant(const void* x, int x_dtype, int64_t ldx, int8_t
                             workspace_bytes, flags & ~BI8_GEMM_FORCE_SKINNY, stream);
 }
 
-int bi8_quantize_rowwise_pre(int op, const void* x, const void* x2, int x_dtype, int64_t ldx, const void* weight, float eps, int8_t* q,
-                             float* scales, int64_t M, int64_t K, int block, void* stream) {
+int bi8_quantize_rowwise_pre_pitched(int op, const void* x, const void* x2, int x_dtype, int64_t ldx, const void* weight, float eps, int8_t* q,
+                                     int64_t ldq, float* scales, int64_t M, int64_t K, int block, void* stream) {
     if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "quantize_rowwise_pre: unknown dtype code %d", x_dtype);
     if (op != BI8_PRE_NONE && op != BI8_PRE_RMSNORM && op != BI8_PRE_SILU_MUL)
         return fail(BI8_ERR_SHAPE, "quantize_rowwise_pre: unknown operation code %d", op);
-    if (M < 0 || K < 0 || ldx < K) return fail(BI8_ERR_SHAPE, "quantize_rowwise_pre: bad shape M %lld K %lld ldx %lld", (long long)M, (long long)K, (long long)ldx);
+    if (M < 0 || K < 0 || ldx < K || ldq < K) return fail(BI8_ERR_SHAPE, "quantize_rowwise_pre: bad shape M %lld K %lld ldx %lld", (long long)M, (long long)K, (long long)ldx);
     if (M == 0 || K == 0) return BI8_OK;
     if (!x || !q || !scales || (op == BI8_PRE_SILU_MUL && !x2)) return fail(BI8_ERR_NULL, "quantize_rowwise_pre: null pointer");
     const size_t esz = dtype_size(x_dtype);
     if (!aligned(x, esz) || (x2 && !aligned(x2, esz)) || (weight && !aligned(weight, esz)) || !aligned(scales, 4))
         return fail(BI8_ERR_ALIGN, "quantize_rowwise_pre: pointer not element aligned");
-    return launch_quantize_pre(op, x, x2, x_dtype, ldx, weight, eps, q, scales, M, K, block, static_cast<cudaStream_t>(stream));
+    return launch_quantize_pre(op, x, x2, x_dtype, ldx, weight, eps, q, ldq, scales, M, K, block, static_cast<cudaStream_t>(stream));
+}
+
+int bi8_quantize_rowwise_pre(int op, const void* x, const void* x2, int x_dtype, int64_t ldx, const void* weight, float eps, int8_t* q,
+                             float* scales, int64_t M, int64_t K, int block, void* stream) {
+    return bi8_quantize_rowwise_pre_pitched(op, x, x2, x_dtype, ldx, weight, eps, q, K, scales, M, K, block, stream);
 }
 
 int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtype, int64_t ldx, const void* norm_weight, float eps,

@@ -74,21 +74,22 @@ __device__ __forceinline__ void after_predecessor() {
 #endif
 
 // ---- launchers implemented in the other translation units -------------------------------------
-int launch_quantize_rowwise(const void* x, int dt, int64_t ldx, int8_t* q, float* s, int64_t M, int64_t K,
+// (ldq: row pitch of the int8 result in bytes)
+int launch_quantize_rowwise(const void* x, int dt, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t M, int64_t K,
                             int block, cudaStream_t st);
-int launch_quantize_colwise(const void* x, int dt, int64_t ldx, int8_t* q, float* s, int64_t R, int64_t C,
+int launch_quantize_colwise(const void* x, int dt, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t R, int64_t C,
                             int block, cudaStream_t st);
 // tile quantizer (quantize_tile.cu): column-wise result, and with q_row != nullptr the row-wise result of the same input
-bool quantize_tile_applicable(const void* x, int dt, int64_t ldx, const void* q_col, const void* q_row, int64_t R, int64_t C, int block);
-int launch_quantize_tile(const void* x, int dt, int64_t ldx, int8_t* q_col, float* s_col, int8_t* q_row, float* s_row, int64_t R,
-                         int64_t C, int block, cudaStream_t st);
+bool quantize_tile_applicable(int dt, const void* q_col, int64_t ldqc, const void* q_row, int64_t ldqr, int64_t R, int64_t C, int block);
+int launch_quantize_tile(const void* x, int dt, int64_t ldx, int8_t* q_col, int64_t ldqc, float* s_col, int8_t* q_row, int64_t ldqr,
+                         float* s_row, int64_t R, int64_t C, int block, cudaStream_t st);
 // sum of the ranks' fp32 partial results over peer memory (peer_reduce.cu)
 size_t peer_allreduce_buffer_bytes(int world, int64_t capacity);
 int launch_peer_allreduce(void* const* peer_bufs, int rank, int world, int64_t capacity, const float* partial, int64_t M, int64_t N,
                           const void* bias, int bias_dtype, void* out, int out_dtype, unsigned wait_limit_us, cudaStream_t st);
-// quantizers with the producing elementwise step in front (quantize_pre.cu); q has row pitch K
-int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t ldx, const void* weight, float eps, int8_t* q, float* sx,
-                        int64_t M, int64_t K, int block, cudaStream_t st);
+// quantizers with the producing elementwise step in front (quantize_pre.cu)
+int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t ldx, const void* weight, float eps, int8_t* q, int64_t ldq,
+                        float* sx, int64_t M, int64_t K, int block, cudaStream_t st);
 // C[m, n] += R[m, n] in the type of C (C may be R)
 int launch_residual_add(void* C, int64_t ldc, const void* R, int64_t ldr, int dt, int64_t M, int64_t N, cudaStream_t st);
 // prefill-sized sum over ranks: reduce-scatter by peer loads, all-gather by peer stores (peer_reduce_large.cu)
@@ -100,7 +101,7 @@ int launch_peer_allreduce_large(void* const* peer_bufs, int rank, int world, int
 // rotary embedding of q and k and the append of k and v to the caches for one decode step (rope_cache.cu)
 int launch_rope_cache_append(const void* qkv, int dt, const float* cis, const long long* pos, void* q_out, void* kcache, void* vcache,
                              int64_t B, int64_t H, int64_t D, int64_t max_len, cudaStream_t st);
-int launch_dequantize_rowwise(const int8_t* q, const float* s, void* out, int dt, int64_t M, int64_t K,
+int launch_dequantize_rowwise(const int8_t* q, int64_t ldq, const float* s, void* out, int dt, int64_t M, int64_t K,
                               int block, cudaStream_t st);
 
 // Row-parallel layers: the fp32 result in C is this rank's partial result; where the kernel that finishes the GEMM can, it

@@ -793,7 +793,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 // Reduction of the divided tiles: C[m,n] = cast(sum over the tile's parts) (+ cast(bias[n])) (+ residual[m,n]), the parts added
 // in ascending order, so that the result does not depend on scheduling.  A thread takes eight consecutive columns of
-// a row: one 32-byte sector of every part (four parts in flight), one 16-byte store (two for fp32) where C allows it.
+// a row: one 32-byte sector of every part (eight parts in flight), one 16-byte store (two for fp32) where C allows it.
 // The parts are at most one slot per SM (12 MB) and come from L2.  Launched as a programmatic dependent of the GEMM:
 // its CTAs are resident as the GEMM's leave.
 template <int BN, int COLS>
@@ -818,17 +818,17 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const TcParams p) {
     const bool has_bias = p.bias != nullptr, has_res = p.residual != nullptr;
     if (has_bias) load8_as_f32(bias, p.bias, p.bias_dtype, n, live);
     if (has_res) load8_as_f32(res, p.residual, p.out_dtype, ro, live);
-    for (int s0 = 0; s0 < p.ksplit; s0 += 4) {
-        float4 v[4][2];
+    for (int s0 = 0; s0 < p.ksplit; s0 += 8) {
+        float4 v[8][2];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < 8; ++q)
             if (s0 + q < p.ksplit) {
                 const float4* s4 = reinterpret_cast<const float4*>(src + (int64_t)(s0 + q) * p.slot_floats);
                 v[q][0] = __ldcg(s4);
                 v[q][1] = __ldcg(s4 + 1);
             }
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < 8; ++q)
             if (s0 + q < p.ksplit) {
                 const float f[8] = {v[q][0].x, v[q][0].y, v[q][0].z, v[q][0].w, v[q][1].x, v[q][1].y, v[q][1].z, v[q][1].w};
 #pragma unroll

@@ -64,4 +64,27 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
     return d;
 }
 
+// Quantizes eight values of one block (scale amax) on packed pairs: the same operations, each rounded on its own, as BlockQ::q.
+// Returns the bytes of values 0-3 and 4-7.
+__device__ __forceinline__ void quantize8(const float (&v)[8], const BlockQ& bq, uint32_t& lo, uint32_t& hi) {
+    uint32_t b[8];
+    if (bq.fast) {
+        const uint64_t r2 = f2_pack(bq.rcp, bq.rcp), ns2 = f2_pack(-bq.scale, -bq.scale);
+        const uint64_t c127 = f2_pack(127.0f, 127.0f), cmagic = f2_pack(kMagic, kMagic), cone = f2_pack(1.0f, 1.0f);
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const uint64_t v2 = f2_pack(v[2 * h], v[2 * h + 1]);
+            const uint64_t q0 = f2_mul(v2, r2);
+            const uint64_t e = f2_fma(ns2, q0, v2);
+            const uint64_t y = f2_fma(e, r2, q0);
+            f2_bits(f2_fma(f2_mul(c127, y), cone, cmagic), b[2 * h], b[2 * h + 1]);
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) b[e] = bq.q(v[e]);
+    }
+    lo = pack4(b[0], b[1], b[2], b[3]);
+    hi = pack4(b[4], b[5], b[6], b[7]);
+}
+
 }  // namespace bi8

@@ -13,8 +13,10 @@
 // stores (and, for dequantize, its loads) are contiguous along the row index.
 #include "bi8_common.cuh"
 #include "quant_math.cuh"
+#include "tc_common.cuh"
 
 #include <cstdlib>
+#include <type_traits>
 
 namespace bi8 {
 namespace {
@@ -58,38 +60,83 @@ __device__ __forceinline__ void unpack2<__half>(uint32_t w, float& lo, float& hi
 }
 
 // ------------------------------------------------------------------------------------------------
-// Row-wise quantize, vector path.  T is a 16-bit float type.  VEC elements per lane (16: one 32-byte
-// load and one 16-byte store per lane; 8: 16-byte load, 8-byte store).  A CTA covers 32 rows x 32*VEC
-// columns; warp w handles rows w, w+8, w+16, w+24 and issues the four loads before any arithmetic.
-template <typename T, int B, int VEC>
+// Eight consecutive elements of a row as 4 or 8 words, from rows of any alignment.  The row is read in aligned 16-byte pieces:
+// the `NW / 4` pieces that begin at or before the lane's first byte and, with SHIFT, the one behind them, and the words are
+// funnel-shifted into place (the byte offset is the same in all lanes of a row, whose pieces are neighbours, so the
+// repeated piece comes from L1).  A piece is read only where it contains a byte of the row, so no access leaves the
+// tensor's 16-byte granules.  Elements from `valid` on read as zero.
+template <typename T, bool SHIFT>
+__device__ __forceinline__ void load_unit8(const T* p, const T* row_end, int valid, uint32_t (&w)[2 * sizeof(T)]) {
+    constexpr int NW = 2 * (int)sizeof(T), NV = NW / 4;
+    if constexpr (!SHIFT) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const uint4 d = ld_nc_v4(reinterpret_cast<const unsigned char*>(p) + 16 * v);
+            w[4 * v] = d.x; w[4 * v + 1] = d.y; w[4 * v + 2] = d.z; w[4 * v + 3] = d.w;
+        }
+    } else {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p), end = reinterpret_cast<uintptr_t>(row_end);
+        const uintptr_t base = a & ~(uintptr_t)15;
+        uint32_t r[NW + 4];
+#pragma unroll
+        for (int v = 0; v <= NV; ++v) {
+            uint4 d = make_uint4(0u, 0u, 0u, 0u);
+            if (base + 16 * v < end) d = __ldg(reinterpret_cast<const uint4*>(base + 16 * v));
+            r[4 * v] = d.x; r[4 * v + 1] = d.y; r[4 * v + 2] = d.z; r[4 * v + 3] = d.w;
+        }
+        // the offset is the same in all lanes: a branch per word offset instead of selects per word
+        const uint32_t off = (uint32_t)(a & 15u), bits = (off & 3u) * 8u;
+        auto shifted = [&](auto words) {
+            constexpr int WS = decltype(words)::value;
+#pragma unroll
+            for (int i = 0; i < NW; ++i) w[i] = __funnelshift_r(r[i + WS], r[i + WS + 1 < NW + 4 ? i + WS + 1 : NW + 3], bits);
+        };
+        if (off < 4u) shifted(std::integral_constant<int, 0>{});
+        else if (off < 8u) shifted(std::integral_constant<int, 1>{});
+        else if (off < 12u) shifted(std::integral_constant<int, 2>{});
+        else shifted(std::integral_constant<int, 3>{});
+    }
+    if (valid < 8) {
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            if constexpr (sizeof(T) == 4) {
+                if (i >= valid) w[i] = 0u;
+            } else {
+                if (2 * i >= valid) w[i] = 0u;
+                else if (2 * i + 1 >= valid) w[i] &= 0xffffu;
+            }
+        }
+    }
+}
+
+// Row-wise quantize, vector path: any float type and (SHIFT) any alignment of the input rows; the int8 rows begin on 8-byte
+// boundaries (pitch ldq).  A lane takes eight elements, a CTA covers 32 rows x 256 columns; warp w handles rows w, w+8,
+// w+16, w+24 and issues their loads before any arithmetic.  Bound by memory: for 16-bit inputs that the streaming kernel
+// below does not take (rows that are not 32-byte aligned) and for fp32.
+template <typename T, int B, bool SHIFT>
 __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
-    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int M, int K, int nb,
+    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int M, int K, int nb,
     int col_tiles) {
     after_predecessor();
-    constexpr int WCOLS = 32 * VEC;         // columns per warp pass
-    constexpr int LPB = B / VEC;            // lanes sharing one block
+    constexpr int WCOLS = 256;              // columns per warp pass
+    constexpr int LPB = B / 8;              // lanes sharing one block
     constexpr int BPT = WCOLS / B;          // blocks per tile row
-    constexpr int NW = VEC / 2;             // 32-bit words loaded per lane
-    static_assert(B % VEC == 0 && LPB >= 1 && LPB <= 32, "block must be a multiple of the lane vector");
+    constexpr int NW = 2 * (int)sizeof(T);  // 32-bit words of a lane's eight elements
+    static_assert(LPB >= 1 && LPB <= 32, "block must be a multiple of the lane vector");
     __shared__ float s_scale[BPT][kTileRows];
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ct = blockIdx.x % col_tiles, rt = blockIdx.x / col_tiles;
-    const int col = ct * WCOLS + lane * VEC;
-    const bool col_ok = col < K;            // K % VEC == 0 on this path: a lane is all in or all out
+    const int col = ct * WCOLS + lane * 8;
+    const int valid = K - col < 8 ? K - col : 8;          // elements of this lane inside the row; <= 0: none
 
     uint32_t raw[4][NW];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int row = rt * kTileRows + warp + 8 * i;
-        if (col_ok && row < M) {
-            const T* p = x + (int64_t)row * ldx + col;
-            if constexpr (VEC == 16) {
-                ld_nc_v8(p, raw[i]);
-            } else {
-                uint4 v = ld_nc_v4(p);
-                raw[i][0] = v.x; raw[i][1] = v.y; raw[i][2] = v.z; raw[i][3] = v.w;
-            }
+        if (valid > 0 && row < M) {
+            const T* xr = x + (int64_t)row * ldx;
+            load_unit8<T, SHIFT>(xr + col, xr + K, valid, raw[i]);
         } else {
 #pragma unroll
             for (int w = 0; w < NW; ++w) raw[i][w] = 0u;
@@ -98,29 +145,25 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int row = rt * kTileRows + warp + 8 * i;
-        float v[VEC];
+        float v[8];
         float amax = 0.0f;
+        if constexpr (sizeof(T) == 4) {
 #pragma unroll
-        for (int w = 0; w < NW; ++w) {
-            unpack2<T>(raw[i][w], v[2 * w], v[2 * w + 1]);
-            amax = fmaxf(amax, fmaxf(fabsf(v[2 * w]), fabsf(v[2 * w + 1])));
+            for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(raw[i][e]);
+        } else {
+#pragma unroll
+            for (int w = 0; w < NW; ++w) unpack2<T>(raw[i][w], v[2 * w], v[2 * w + 1]);
         }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
 #pragma unroll
         for (int off = 1; off < LPB; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
         BlockQ bq;
-        bq.set(amax, true);
-        uint32_t out[VEC / 4];
-#pragma unroll
-        for (int w = 0; w < VEC / 4; ++w)
-            out[w] = pack4(bq.q(v[4 * w]), bq.q(v[4 * w + 1]), bq.q(v[4 * w + 2]), bq.q(v[4 * w + 3]));
-        if (col_ok && row < M) {
-            int8_t* o = q + (int64_t)row * K + col;
-            if constexpr (VEC == 16) {
-                *reinterpret_cast<uint4*>(o) = make_uint4(out[0], out[1], out[2], out[3]);
-            } else {
-                *reinterpret_cast<uint2*>(o) = make_uint2(out[0], out[1]);
-            }
-        }
+        bq.set(amax, sizeof(T) == 2);
+        uint32_t lo, hi;
+        quantize8(v, bq, lo, hi);
+        // a lane with fewer than eight elements writes zeros into the row's padding (ldq covers it: see the launcher)
+        if (valid > 0 && row < M) *reinterpret_cast<uint2*>(q + (int64_t)row * ldq + col) = make_uint2(lo, hi);
         if ((lane % LPB) == 0) s_scale[lane / LPB][warp + 8 * i] = amax;
     }
     __syncthreads();
@@ -131,32 +174,6 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
     }
 }
 
-// Packed fp32 pairs (add/mul/fma.rn.f32x2): one instruction for two lanes of data, each lane rounded exactly
-// like the scalar instruction.
-__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void f2_unpack_bits(uint64_t v, uint32_t& lo, uint32_t& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
 // Row-wise quantize, streaming path (16-bit inputs, K % 16 == 0, 32-byte aligned rows).
 // Persistent warps: a warp owns units of 4 rows x 512 columns (lane = 16 consecutive elements of a row, one
 // 32-byte load and one 16-byte store per row) and keeps the loads of its NEXT unit in flight while it quantizes
@@ -165,7 +182,7 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
 // piece of the transposed scale tensor (s[j, m0..m0+3]).  The arithmetic is done on packed fp32 pairs.
 template <typename T, int B>
 __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
-    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int M, int K, int nb,
+    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int M, int K, int nb,
     int col_units, int64_t total_units) {
     after_predecessor();
     constexpr int LPB = B / 16;             // lanes sharing one block
@@ -179,7 +196,7 @@ __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
     const uint64_t c127 = f2_pack(127.0f, 127.0f), cmagic = f2_pack(kMagic, kMagic), cone = f2_pack(1.0f, 1.0f);
     auto round_pair = [&](uint64_t y2, uint32_t& b0, uint32_t& b1) {
         const uint64_t z = f2_mul(c127, y2);
-        f2_unpack_bits(f2_fma(z, cone, cmagic), b0, b1);
+        f2_bits(f2_fma(z, cone, cmagic), b0, b1);
     };
 
     auto load_unit = [&](int64_t u, uint32_t (&buf)[4][8]) {
@@ -241,14 +258,14 @@ __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
 #pragma unroll
                 for (int w = 0; w < 4; ++w) {
                     uint32_t a0, a1, a2, a3;
-                    f2_unpack_bits(v2[2 * w], a0, a1);
-                    f2_unpack_bits(v2[2 * w + 1], a2, a3);
+                    f2_bits(v2[2 * w], a0, a1);
+                    f2_bits(v2[2 * w + 1], a2, a3);
                     out[w] = pack4(bq.q(__uint_as_float(a0)), bq.q(__uint_as_float(a1)), bq.q(__uint_as_float(a2)),
                                    bq.q(__uint_as_float(a3)));
                 }
             }
             if (col < K && row < M)
-                *reinterpret_cast<uint4*>(q + (int64_t)row * K + col) = make_uint4(out[0], out[1], out[2], out[3]);
+                *reinterpret_cast<uint4*>(q + (int64_t)row * ldq + col) = make_uint4(out[0], out[1], out[2], out[3]);
         }
         if ((lane % LPB) == 0) {
             const int jb = (col / B);
@@ -289,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
 constexpr int kRagGroup = 8;
 template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_rowwise_ragged_kernel(
-    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int64_t K, int B,
+    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int64_t M, int64_t K, int B,
     int64_t nb, int64_t groups_per_row) {
     after_predecessor();
     const int lane = threadIdx.x & 31;
@@ -319,7 +336,7 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_ragged_kernel(
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int64_t k = j * B + lane + 32 * e;
-            if (lane + 32 * e < B && k < K) q[row * K + k] = (int8_t)(bq.q(v[b][e]) & 0xffu);
+            if (lane + 32 * e < B && k < K) q[row * ldq + k] = (int8_t)(bq.q(v[b][e]) & 0xffu);
         }
         if (lane == 0) s[j * M + row] = amax;
     }
@@ -327,7 +344,7 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_ragged_kernel(
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_rowwise_generic_kernel(
-    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int64_t K, int B,
+    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int64_t M, int64_t K, int B,
     int64_t nb) {
     after_predecessor();
     const int lane = threadIdx.x & 31;
@@ -342,111 +359,69 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_generic_kernel(
     for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
     BlockQ bq;
     bq.set(amax, sizeof(T) == 2);
-    for (int64_t k = lo + lane; k < hi; k += 32) q[row * K + k] = (int8_t)(bq.q(to_f32<T>(xr[k])) & 0xffu);
+    for (int64_t k = lo + lane; k < hi; k += 32) q[row * ldq + k] = (int8_t)(bq.q(to_f32<T>(xr[k])) & 0xffu);
     if (lane == 0) s[j * M + row] = amax;
 }
 
 // ------------------------------------------------------------------------------------------------
-// Column-wise quantize (fused transpose): x [R,C] -> q [C,R], s [ceil(R/B), C].  A CTA stages a tile of
-// NBLK*B rows x 128 columns in shared memory with 16-byte row-contiguous loads; then one thread owns one
-// (block, column): it reads the B values down the column once (bank-conflict free: lanes are consecutive columns),
-// keeps them packed in registers, takes the absmax and quantizes.  The int8 results go back to shared memory
-// transposed ([column][row], reusing the staging area), and the CTA writes them out as whole 128-byte (or longer)
-// runs of the output rows.
+// Column-wise quantize for fp32 inputs and for 16-bit ones that the tile quantizer does not take.  A CTA takes one block of B
+// rows x 64 columns: a thread has one column and B/4 consecutive rows, all of whose loads are in flight before the
+// first absmax; the four row groups of a column exchange their maxima through shared memory, the bytes go to a
+// transposed tile, and each column's B bytes leave as 16-byte pieces (bytes where the output is not aligned).  With one thread per column
+// and a loop down the block (the kernel below) a 300 x 256 matrix took 9 us of serial loads.
 template <typename T, int B>
-__global__ void __launch_bounds__(kThreads) quantize_colwise_vec_kernel(
-    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int R, int C, int col_tiles) {
+__global__ void __launch_bounds__(kThreads) quantize_colwise_cols_kernel(
+    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int R, int C, int col_tiles) {
     after_predecessor();
-    constexpr int TC = 128;
-    constexpr int NBLK = kThreads / TC;     // blocks (along rows of x) per tile
-    constexpr int TR = NBLK * B;
-    constexpr int PITCH = TC + 2;           // 16-bit elements; +2 keeps column reads conflict free
-    constexpr int OPITCH = TR + 16;         // bytes per output row in the transposed tile
-    static_assert(TC * OPITCH <= TR * PITCH * 2, "the transposed tile reuses the staging area");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint16_t* tile = reinterpret_cast<uint16_t*>(smem_raw);
-
-    const int ct = blockIdx.x % col_tiles, rt = blockIdx.x / col_tiles;
-    const int c0 = ct * TC, r0 = rt * TR;
-    // load: each row of the tile is 16 lanes x 16 bytes; all loads of a thread are issued before its first store
-    constexpr int VPR = TC / 8;
-    constexpr int PER_THREAD = TR * VPR / kThreads;
-    {
-        uint4 d[PER_THREAD];
-#pragma unroll
-        for (int u = 0; u < PER_THREAD; ++u) {
-            const int v = threadIdx.x + u * kThreads;
-            const int r = v / VPR, cv = (v % VPR) * 8;
-            d[u] = make_uint4(0u, 0u, 0u, 0u);
-            if (r0 + r < R && c0 + cv < C) d[u] = ld_nc_v4(x + (int64_t)(r0 + r) * ldx + c0 + cv);
-        }
-#pragma unroll
-        for (int u = 0; u < PER_THREAD; ++u) {
-            const int v = threadIdx.x + u * kThreads;
-            const int r = v / VPR, cv = (v % VPR) * 8;
-            uint32_t* dst = reinterpret_cast<uint32_t*>(tile + r * PITCH + cv);   // 4-byte aligned (PITCH even)
-            dst[0] = d[u].x; dst[1] = d[u].y; dst[2] = d[u].z; dst[3] = d[u].w;
-        }
-    }
-    __syncthreads();
-    const int c = threadIdx.x % TC, blk = threadIdx.x / TC;
-    const uint16_t* colp = tile + (blk * B) * PITCH + c;
-    uint32_t packed[B / 2];                 // the column's B values, two per register
+    constexpr int TC = 64, GROUPS = kThreads / TC, RPT = B / GROUPS;     // columns, row groups, rows per thread
+    constexpr int PITCH = B + 16;                                        // bytes; rows 16-byte aligned
+    __shared__ float s_max[GROUPS][TC];
+    __shared__ __align__(16) unsigned char tile[TC * PITCH];
+    const int j = blockIdx.x / col_tiles, c0 = (blockIdx.x % col_tiles) * TC;
+    const int c = threadIdx.x % TC, g = threadIdx.x / TC;
+    const int r0 = j * B + g * RPT;
+    const bool col_ok = c0 + c < C;
+    const T* xc = x + (int64_t)r0 * ldx + c0 + c;
+    float v[RPT];
     float amax = 0.0f;
 #pragma unroll
-    for (int r = 0; r < B; r += 2) {
-        const uint32_t lo = colp[r * PITCH], hi = colp[(r + 1) * PITCH];
-        packed[r / 2] = lo | (hi << 16);
-        float flo, fhi;
-        unpack2<T>(packed[r / 2], flo, fhi);
-        amax = fmaxf(amax, fmaxf(fabsf(flo), fabsf(fhi)));
-    }
-    BlockQ bq;
-    bq.set(amax, true);
-    uint32_t out[B / 4];
+    for (int r = 0; r < RPT; ++r) v[r] = (col_ok && r0 + r < R) ? to_f32<T>(xc[(int64_t)r * ldx]) : 0.0f;
 #pragma unroll
-    for (int g = 0; g < B / 4; ++g) {
-        float f0, f1, f2, f3;
-        unpack2<T>(packed[2 * g], f0, f1);
-        unpack2<T>(packed[2 * g + 1], f2, f3);
-        out[g] = pack4(bq.q(f0), bq.q(f1), bq.q(f2), bq.q(f3));
-    }
-    const int rb = r0 + blk * B;            // first row of this block
-    if (c0 + c < C && rb < R) s[(int64_t)(rb / B) * C + c0 + c] = amax;
-    __syncthreads();                        // every thread has read its column: the staging area can be reused
-    unsigned char* otile = smem_raw;        // [TC][OPITCH] int8, row = output row (column of x)
-#pragma unroll
-    for (int g = 0; g < B / 16; ++g)
-        *reinterpret_cast<uint4*>(otile + c * OPITCH + blk * B + g * 16) = make_uint4(out[4 * g], out[4 * g + 1], out[4 * g + 2], out[4 * g + 3]);
+    for (int r = 0; r < RPT; ++r) amax = fmaxf(amax, fabsf(v[r]));
+    s_max[g][c] = amax;
     __syncthreads();
-    // store: output row (c0 + cc) receives TR contiguous bytes starting at r0
-    constexpr int PIECES = TR / 16;         // 16-byte pieces per output row
-    const bool vec_ok = ((R & 15) == 0);
-    for (int v = threadIdx.x; v < TC * PIECES; v += kThreads) {
-        const int cc = v / PIECES, piece = v % PIECES;
-        const int rr = r0 + piece * 16;
-        if (c0 + cc >= C || rr >= R) continue;
-        const uint4 d = *reinterpret_cast<const uint4*>(otile + cc * OPITCH + piece * 16);
-        int8_t* o = q + (int64_t)(c0 + cc) * R + rr;
-        if (vec_ok && rr + 16 <= R) {
-            *reinterpret_cast<uint4*>(o) = d;
-        } else {
-            const uint32_t w[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
-            for (int u = 0; u < 16; ++u)
-                if (rr + u < R) o[u] = (int8_t)((w[u / 4] >> (8 * (u % 4))) & 0xffu);
+    for (int k = 0; k < GROUPS; ++k) amax = fmaxf(amax, s_max[k][c]);
+    BlockQ bq;
+    bq.set(amax, sizeof(T) == 2);
+    if (g == 0 && col_ok) s[(int64_t)j * C + c0 + c] = amax;
+#pragma unroll
+    for (int r = 0; r < RPT; r += 4)
+        *reinterpret_cast<uint32_t*>(tile + c * PITCH + g * RPT + r) = pack4(bq.q(v[r]), bq.q(v[r + 1]), bq.q(v[r + 2]), bq.q(v[r + 3]));
+    __syncthreads();
+    constexpr int PIECES = B / 16;
+    const bool vec = (ldq & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & 15u) == 0;
+    for (int t = threadIdx.x; t < TC * PIECES; t += kThreads) {
+        const int cc = t / PIECES, rr = (t % PIECES) * 16, left = R - (j * B + rr);
+        if (c0 + cc >= C || left <= 0) continue;
+        const unsigned char* src = tile + cc * PITCH + rr;
+        int8_t* dst = q + (int64_t)(c0 + cc) * ldq + j * B + rr;
+        if (vec && left >= 16) {
+            *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+        } else {
+            for (int b = 0; b < 16 && b < left; ++b) dst[b] = (int8_t)src[b];
         }
     }
 }
 
-// Column-wise quantize when rows of the input or of the output are not 16-byte aligned (e.g. 50257 columns).  A CTA takes
+// Column-wise quantize for the other block sizes, rows of any alignment.  A CTA takes
 // one block of B rows x kThreads columns: thread t reads its column down the block twice (absmax, then quantize; the
 // second pass hits L1/L2; consecutive threads read consecutive columns), parks the B bytes in shared memory, and the
 // warps then write each output row's B bytes as runs of 32 consecutive bytes.  (With one thread storing its column byte
 // by byte, every warp store touched 32 sectors.)  Dynamic shared memory: kThreads * (B + 4) bytes.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_colwise_ragged_kernel(
-    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int64_t R, int64_t C, int B,
+    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int64_t R, int64_t C, int B,
     int64_t col_tiles) {
     after_predecessor();
     extern __shared__ unsigned char tile[];                 // [kThreads][B + 4]
@@ -470,7 +445,7 @@ __global__ void __launch_bounds__(kThreads) quantize_colwise_ragged_kernel(
     for (int t = warp; t < kThreads; t += kThreads / 32) {
         const int64_t cc = c0 + t;
         if (cc >= C) break;
-        int8_t* dst = q + cc * R + lo;
+        int8_t* dst = q + cc * ldq + lo;
         const unsigned char* src = tile + (size_t)t * pitch;
         for (int r = lane; r < rows; r += 32) dst[r] = (int8_t)src[r];
     }
@@ -479,7 +454,7 @@ __global__ void __launch_bounds__(kThreads) quantize_colwise_ragged_kernel(
 // Column-wise quantize, any type / block / alignment: one thread per (block, column).
 template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_colwise_generic_kernel(
-    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, float* __restrict__ s, int64_t R, int64_t C, int B,
+    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int64_t R, int64_t C, int B,
     int64_t nb) {
     after_predecessor();
     const int64_t task = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -490,7 +465,7 @@ __global__ void __launch_bounds__(kThreads) quantize_colwise_generic_kernel(
     for (int64_t r = lo; r < hi; ++r) amax = fmaxf(amax, fabsf(to_f32<T>(x[r * ldx + c])));
     BlockQ bq;
     bq.set(amax, sizeof(T) == 2);
-    for (int64_t r = lo; r < hi; ++r) q[c * R + r] = (int8_t)(bq.q(to_f32<T>(x[r * ldx + c])) & 0xffu);
+    for (int64_t r = lo; r < hi; ++r) q[c * ldq + r] = (int8_t)(bq.q(to_f32<T>(x[r * ldx + c])) & 0xffu);
     s[j * C + c] = amax;
 }
 
@@ -522,7 +497,7 @@ __device__ __forceinline__ void store16<float>(float* o, const float (&f)[16]) {
 
 template <typename TO, int B>
 __global__ void __launch_bounds__(kThreads) dequantize_rowwise_vec_kernel(
-    const int8_t* __restrict__ q, const float* __restrict__ s, TO* __restrict__ out, int M, int K, int nb,
+    const int8_t* __restrict__ q, int64_t ldq, const float* __restrict__ s, TO* __restrict__ out, int M, int K, int nb,
     int col_tiles) {
     after_predecessor();
     constexpr int WCOLS = 512;
@@ -538,7 +513,7 @@ __global__ void __launch_bounds__(kThreads) dequantize_rowwise_vec_kernel(
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int row = rt * kTileRows + warp + 8 * i;
-        raw[i] = (col_ok && row < M) ? ld_nc_v4(q + (int64_t)row * K + col) : make_uint4(0u, 0u, 0u, 0u);
+        raw[i] = (col_ok && row < M) ? ld_nc_v4(q + (int64_t)row * ldq + col) : make_uint4(0u, 0u, 0u, 0u);
     }
     for (int t = threadIdx.x; t < BPT * kTileRows; t += kThreads) {
         const int j = t / kTileRows, r = t % kTileRows;
@@ -572,15 +547,53 @@ __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2hal
 template <>
 __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 
+// Dequantize to rows that are not 32-byte aligned (K not a multiple of 16), or any block size and alignment.  A warp takes a
+// run of 256 columns of a row; a lane's four stores are aligned 4-byte words (two 16-bit results, or one fp32), 32 lanes
+// next to each other, whatever the row's alignment: for a 16-bit row that begins between two words, the words hold elements
+// (2i - 1, 2i) and the row's first and last element are stored alone.
 template <typename TO>
-__global__ void __launch_bounds__(kThreads) dequantize_rowwise_generic_kernel(
-    const int8_t* __restrict__ q, const float* __restrict__ s, TO* __restrict__ out, int64_t M, int64_t K, int B) {
+__global__ void __launch_bounds__(kThreads) dequantize_rowwise_words_kernel(
+    const int8_t* __restrict__ q, int64_t ldq, const float* __restrict__ s, TO* __restrict__ out, int64_t M, int K, int B, int log2_b, int col_units) {
     after_predecessor();
-    const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (i >= M * K) return;
-    const int64_t m = i / K, k = i % K;
+    constexpr int EPW = 4 / (int)sizeof(TO), WORDS = 256 / (32 * EPW);   // elements per word, words per lane
+    const int lane = threadIdx.x & 31;
+    const int64_t unit = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    const int64_t m = unit / col_units;
+    if (m >= M) return;
+    TO* row = out + m * K;
+    const int odd = (int)((reinterpret_cast<uintptr_t>(row) & 3u) / sizeof(TO));    // elements past a word boundary: 0 or 1
+    const int first = (int)(unit % col_units) * 256 - odd;
+    const int8_t* qr = q + m * ldq;
     const float inv127 = 1.0f / 127.0f;
-    out[i] = from_f32<TO>(__fmul_rn(__fmul_rn(s[(k / B) * M + m], (float)q[i]), inv127));
+    int8_t b[WORDS][EPW];
+    float sc[WORDS][EPW];
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w)
+#pragma unroll
+        for (int e = 0; e < EPW; ++e) {
+            const int k = first + (w * 32 + lane) * EPW + e;
+            const bool in = k >= 0 && k < K;
+            b[w][e] = in ? qr[k] : (int8_t)0;
+            const int j = log2_b >= 0 ? k >> log2_b : k / B;
+            sc[w][e] = in ? __ldg(s + (int64_t)j * M + m) : 0.0f;
+        }
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) {
+        const int k = first + (w * 32 + lane) * EPW;
+        TO v[EPW];
+#pragma unroll
+        for (int e = 0; e < EPW; ++e) v[e] = from_f32<TO>(__fmul_rn(__fmul_rn(sc[w][e], (float)b[w][e]), inv127));
+        if (k >= 0 && k + EPW <= K) {
+            uint32_t word;
+            if constexpr (EPW == 1) word = __float_as_uint(v[0]);
+            else word = (uint32_t)*reinterpret_cast<const uint16_t*>(&v[0]) | ((uint32_t)*reinterpret_cast<const uint16_t*>(&v[EPW - 1]) << 16);
+            *reinterpret_cast<uint32_t*>(row + k) = word;
+        } else {
+#pragma unroll
+            for (int e = 0; e < EPW; ++e)
+                if (k + e >= 0 && k + e < K) row[k + e] = v[e];
+        }
+    }
 }
 
 bool use_v8() {
@@ -589,85 +602,59 @@ bool use_v8() {
 }
 
 template <typename T>
-int quantize_rowwise_t(const T* x, int64_t ldx, int8_t* q, float* s, int64_t M, int64_t K, int block, cudaStream_t st) {
+int quantize_rowwise_t(const T* x, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t M, int64_t K, int block, cudaStream_t st) {
     const int64_t nb = (K + block - 1) / block;
-    const bool small = sizeof(T) == 2 && M < (1ll << 31) && K < (1ll << 31);
-    const bool v16 = small && use_v8() && K % 16 == 0 && ldx % 16 == 0 && aligned(x, 32) && aligned(q, 16);
-    const bool v8 = small && K % 8 == 0 && ldx % 8 == 0 && aligned(x, 16) && aligned(q, 8);
-    const int64_t row_tiles = (M + kTileRows - 1) / kTileRows;
-#define BI8_QROW(BB, VV)                                                                                   \
-    do {                                                                                                   \
-        const int64_t ctiles = (K + 32 * VV - 1) / (32 * VV);                                              \
-        if (row_tiles * ctiles >= (1ll << 31)) break;                                                      \
-        return launch_chained(quantize_rowwise_vec_kernel<T, BB, VV>, (unsigned)(row_tiles * ctiles), kThreads, 0, st, x, ldx, q, s, (int)M, (int)K, (int)nb, (int)ctiles);                                                                                     \
-    } while (0)
+    const bool small = M < (1ll << 31) && K < (1ll << 30);
+    const bool block_ok = block == 32 || block == 64 || block == 128 || block == 256;
     if constexpr (sizeof(T) == 2) {
-        if (v16 && aligned(s, 16) && (block == 32 || block == 64 || block == 128 || block == 256)) {
-            int dev = 0, sms = 0;
-            BI8_CUDA_TRY(cudaGetDevice(&dev));
-            BI8_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        if (small && use_v8() && K % 16 == 0 && ldx % 16 == 0 && aligned(x, 32) && ldq % 16 == 0 && aligned(q, 16) && aligned(s, 16) && block_ok) {
+            const DeviceInfo di = device_info();
             const int col_units = (int)((K + 511) / 512);
             const int64_t total = ((M + 3) / 4) * col_units;
-            const int64_t warps_wanted = total;                      // one unit per warp at least
-            int64_t ctas = (warps_wanted + kThreads / 32 - 1) / (kThreads / 32);
-            if (ctas > 2ll * sms) ctas = 2ll * sms;                  // two resident CTAs per SM, persistent beyond that
-#define BI8_QSTREAM(BB)                                                                                          \
-    if (block == BB) {                                                                                           \
-        return launch_chained(quantize_rowwise_stream_kernel<T, BB>, (unsigned)ctas, kThreads, 0, st, x, ldx, q, s, (int)M, (int)K, (int)nb, col_units, total);                                                                                           \
-    }
+            int64_t ctas = (total + kThreads / 32 - 1) / (kThreads / 32);   // one unit per warp at least
+            if (ctas > 2ll * di.sms) ctas = 2ll * di.sms;                   // two resident CTAs per SM, persistent beyond that
+#define BI8_QSTREAM(BB) \
+    if (block == BB) return launch_chained(quantize_rowwise_stream_kernel<T, BB>, (unsigned)ctas, kThreads, 0, st, x, ldx, q, ldq, s, (int)M, (int)K, (int)nb, col_units, total);
             BI8_QSTREAM(32) BI8_QSTREAM(64) BI8_QSTREAM(128) BI8_QSTREAM(256)
 #undef BI8_QSTREAM
         }
-        if (v16) {
-            if (block == 32) BI8_QROW(32, 16);
-            if (block == 64) BI8_QROW(64, 16);
-            if (block == 128) BI8_QROW(128, 16);
-            if (block == 256) BI8_QROW(256, 16);
-        }
-        if (v8) {
-            if (block == 32) BI8_QROW(32, 8);
-            if (block == 64) BI8_QROW(64, 8);
-            if (block == 128) BI8_QROW(128, 8);
-            if (block == 256) BI8_QROW(256, 8);
-        }
     }
+    // Any input alignment, as long as the int8 rows are 8-byte aligned and their pitch covers a lane's last eight elements.
+    const int64_t row_tiles = (M + kTileRows - 1) / kTileRows, ctiles = (K + 255) / 256;
+    if (small && block_ok && ldq % 8 == 0 && aligned(q, 8) && row_tiles * ctiles < (1ll << 31)) {
+        const bool straight = K % 8 == 0 && aligned(x, 16) && (ldx * (int64_t)sizeof(T)) % 16 == 0;
+        const unsigned grid = (unsigned)(row_tiles * ctiles);
+#define BI8_QROW(BB)                                                                                                                                \
+    if (block == BB)                                                                                                                                \
+        return straight ? launch_chained(quantize_rowwise_vec_kernel<T, BB, false>, grid, kThreads, 0, st, x, ldx, q, ldq, s, (int)M, (int)K, (int)nb, (int)ctiles) \
+                        : launch_chained(quantize_rowwise_vec_kernel<T, BB, true>, grid, kThreads, 0, st, x, ldx, q, ldq, s, (int)M, (int)K, (int)nb, (int)ctiles);
+        BI8_QROW(32) BI8_QROW(64) BI8_QROW(128) BI8_QROW(256)
 #undef BI8_QROW
+    }
     if (block <= 64) {
         const int64_t gpr = (nb + kRagGroup - 1) / kRagGroup;
         const int64_t rgrid = (M * gpr + kThreads / 32 - 1) / (kThreads / 32);
-        if (rgrid < (1ll << 31)) {
-            return launch_chained(quantize_rowwise_ragged_kernel<T>, (unsigned)rgrid, kThreads, 0, st, x, ldx, q, s, M, K, block, nb, gpr);
-        }
+        if (rgrid < (1ll << 31))
+            return launch_chained(quantize_rowwise_ragged_kernel<T>, (unsigned)rgrid, kThreads, 0, st, x, ldx, q, ldq, s, M, K, block, nb, gpr);
     }
     const int64_t tasks = M * nb;
     const int64_t grid = (tasks + kThreads / 32 - 1) / (kThreads / 32);
     if (grid >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "quantize_rowwise: %lld blocks exceed the grid limit", (long long)tasks);
-    return launch_chained(quantize_rowwise_generic_kernel<T>, (unsigned)grid, kThreads, 0, st, x, ldx, q, s, M, K, block, nb);
-}
-
-template <typename T, int B>
-int colwise_vec(const T* x, int64_t ldx, int8_t* q, float* s, int64_t R, int64_t C, cudaStream_t st) {
-    constexpr int TC = 128, NBLK = kThreads / TC, TR = NBLK * B;
-    const int64_t ctiles = (C + TC - 1) / TC, rtiles = (R + TR - 1) / TR;
-    if (ctiles * rtiles >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "quantize_colwise: grid too large");
-    const size_t smem = (size_t)TR * (TC + 2) * 2;
-    static SmemOptIn opt_in;                // per kernel instance; set once per device
-    const int rc = opt_in.ensure(quantize_colwise_vec_kernel<T, B>, smem);
-    if (rc != BI8_OK) return rc;
-    return launch_chained(quantize_colwise_vec_kernel<T, B>, (unsigned)(ctiles * rtiles), kThreads, smem, st, x, ldx, q, s, (int)R, (int)C, (int)ctiles);
+    return launch_chained(quantize_rowwise_generic_kernel<T>, (unsigned)grid, kThreads, 0, st, x, ldx, q, ldq, s, M, K, block, nb);
 }
 
 template <typename T>
-int quantize_colwise_t(const T* x, int64_t ldx, int8_t* q, float* s, int64_t R, int64_t C, int block, cudaStream_t st) {
-    if constexpr (sizeof(T) == 2) {
-        const bool vec = R < (1ll << 31) && C < (1ll << 31) && C % 8 == 0 && ldx % 8 == 0 && aligned(x, 16) && aligned(q, 16);
-        if (vec) {
-            if (block == 32) return colwise_vec<T, 32>(x, ldx, q, s, R, C, st);
-            if (block == 64) return colwise_vec<T, 64>(x, ldx, q, s, R, C, st);
-            if (block == 128) return colwise_vec<T, 128>(x, ldx, q, s, R, C, st);
-        }
-    }
+int quantize_colwise_t(const T* x, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t R, int64_t C, int block, cudaStream_t st) {
+    const bool small = R < (1ll << 31) - 256 && C < (1ll << 31) - 256;
     const int64_t nb = (R + block - 1) / block;
+    const int64_t ctiles = (C + 63) / 64;
+    if (small && nb * ctiles < (1ll << 31)) {
+        const unsigned grid = (unsigned)(nb * ctiles);
+#define BI8_QCOLS(BB) \
+    if (block == BB) return launch_chained(quantize_colwise_cols_kernel<T, BB>, grid, kThreads, 0, st, x, ldx, q, ldq, s, (int)R, (int)C, (int)ctiles);
+        BI8_QCOLS(32) BI8_QCOLS(64) BI8_QCOLS(128)
+#undef BI8_QCOLS
+    }
     if (block <= 256) {
         const int64_t col_tiles = (C + kThreads - 1) / kThreads;
         const size_t smem = (size_t)kThreads * (block + 4);
@@ -677,62 +664,66 @@ int quantize_colwise_t(const T* x, int64_t ldx, int8_t* q, float* s, int64_t R, 
                 const int rc = opt_in.ensure(quantize_colwise_ragged_kernel<T>, smem);
                 if (rc != BI8_OK) return rc;
             }
-            return launch_chained(quantize_colwise_ragged_kernel<T>, (unsigned)(nb * col_tiles), kThreads, smem, st, x, ldx, q, s, R, C, block, col_tiles);
+            return launch_chained(quantize_colwise_ragged_kernel<T>, (unsigned)(nb * col_tiles), kThreads, smem, st, x, ldx, q, ldq, s, R, C, block, col_tiles);
         }
     }
     const int64_t grid = (nb * C + kThreads - 1) / kThreads;
     if (grid >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "quantize_colwise: grid too large");
-    return launch_chained(quantize_colwise_generic_kernel<T>, (unsigned)grid, kThreads, 0, st, x, ldx, q, s, R, C, block, nb);
+    return launch_chained(quantize_colwise_generic_kernel<T>, (unsigned)grid, kThreads, 0, st, x, ldx, q, ldq, s, R, C, block, nb);
 }
 
 template <typename TO>
-int dequantize_t(const int8_t* q, const float* s, TO* out, int64_t M, int64_t K, int block, cudaStream_t st) {
+int dequantize_t(const int8_t* q, int64_t ldq, const float* s, TO* out, int64_t M, int64_t K, int block, cudaStream_t st) {
     const int64_t nb = (K + block - 1) / block;
-    const bool vec = use_v8() && M < (1ll << 31) && K < (1ll << 31) && K % 16 == 0 && aligned(q, 16) && aligned(out, 32);
+    const bool small = M < (1ll << 31) && K < (1ll << 30);
     const int64_t row_tiles = (M + kTileRows - 1) / kTileRows, ctiles = (K + 511) / 512;
-    if (vec && row_tiles * ctiles < (1ll << 31)) {
-#define BI8_DEQ(BB)                                                                                         \
-    if (block == BB) {                                                                                      \
-        return launch_chained(dequantize_rowwise_vec_kernel<TO, BB>, (unsigned)(row_tiles * ctiles), kThreads, 0, st, q, s, out, (int)M, (int)K, (int)nb, (int)ctiles);                                                                                      \
-    }
+    if (small && use_v8() && K % 16 == 0 && ldq % 16 == 0 && aligned(q, 16) && aligned(out, 32) && row_tiles * ctiles < (1ll << 31)) {
+#define BI8_DEQ(BB)                                                                                                                    \
+    if (block == BB)                                                                                                                   \
+        return launch_chained(dequantize_rowwise_vec_kernel<TO, BB>, (unsigned)(row_tiles * ctiles), kThreads, 0, st, q, ldq, s, out,  \
+                              (int)M, (int)K, (int)nb, (int)ctiles);
         BI8_DEQ(32) BI8_DEQ(64) BI8_DEQ(128) BI8_DEQ(256)
 #undef BI8_DEQ
     }
-    const int64_t grid = (M * K + kThreads - 1) / kThreads;
-    if (grid >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "dequantize: grid too large");
-    return launch_chained(dequantize_rowwise_generic_kernel<TO>, (unsigned)grid, kThreads, 0, st, q, s, out, M, K, block);
+    const int64_t units = (K + 1 + 255) / 256;              // one element more: a row may begin between two words
+    const int64_t grid = (M * units + kThreads / 32 - 1) / (kThreads / 32);
+    if (grid >= (1ll << 31) || K >= (1ll << 30)) return fail(BI8_ERR_SHAPE, "dequantize: grid too large");
+    int log2_b = -1;
+    for (int i = 0; i < 31; ++i)
+        if (block == (1 << i)) log2_b = i;
+    return launch_chained(dequantize_rowwise_words_kernel<TO>, (unsigned)grid, kThreads, 0, st, q, ldq, s, out, M, (int)K, block, log2_b, (int)units);
 }
 
 }  // namespace
 
-int launch_quantize_rowwise(const void* x, int dt, int64_t ldx, int8_t* q, float* s, int64_t M, int64_t K, int block,
+int launch_quantize_rowwise(const void* x, int dt, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t M, int64_t K, int block,
                             cudaStream_t st) {
     switch (dt) {
-        case BI8_BF16: return quantize_rowwise_t(static_cast<const __nv_bfloat16*>(x), ldx, q, s, M, K, block, st);
-        case BI8_F16: return quantize_rowwise_t(static_cast<const __half*>(x), ldx, q, s, M, K, block, st);
-        case BI8_F32: return quantize_rowwise_t(static_cast<const float*>(x), ldx, q, s, M, K, block, st);
+        case BI8_BF16: return quantize_rowwise_t(static_cast<const __nv_bfloat16*>(x), ldx, q, ldq, s, M, K, block, st);
+        case BI8_F16: return quantize_rowwise_t(static_cast<const __half*>(x), ldx, q, ldq, s, M, K, block, st);
+        case BI8_F32: return quantize_rowwise_t(static_cast<const float*>(x), ldx, q, ldq, s, M, K, block, st);
     }
     return fail(BI8_ERR_DTYPE, "quantize_rowwise: unknown dtype code %d", dt);
 }
 
-int launch_quantize_colwise(const void* x, int dt, int64_t ldx, int8_t* q, float* s, int64_t R, int64_t C, int block,
+int launch_quantize_colwise(const void* x, int dt, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t R, int64_t C, int block,
                             cudaStream_t st) {
-    if (quantize_tile_applicable(x, dt, ldx, q, nullptr, R, C, block))
-        return launch_quantize_tile(x, dt, ldx, q, s, nullptr, nullptr, R, C, block, st);
+    if (quantize_tile_applicable(dt, q, ldq, nullptr, 0, R, C, block))
+        return launch_quantize_tile(x, dt, ldx, q, ldq, s, nullptr, 0, nullptr, R, C, block, st);
     switch (dt) {
-        case BI8_BF16: return quantize_colwise_t(static_cast<const __nv_bfloat16*>(x), ldx, q, s, R, C, block, st);
-        case BI8_F16: return quantize_colwise_t(static_cast<const __half*>(x), ldx, q, s, R, C, block, st);
-        case BI8_F32: return quantize_colwise_t(static_cast<const float*>(x), ldx, q, s, R, C, block, st);
+        case BI8_BF16: return quantize_colwise_t(static_cast<const __nv_bfloat16*>(x), ldx, q, ldq, s, R, C, block, st);
+        case BI8_F16: return quantize_colwise_t(static_cast<const __half*>(x), ldx, q, ldq, s, R, C, block, st);
+        case BI8_F32: return quantize_colwise_t(static_cast<const float*>(x), ldx, q, ldq, s, R, C, block, st);
     }
     return fail(BI8_ERR_DTYPE, "quantize_colwise: unknown dtype code %d", dt);
 }
 
-int launch_dequantize_rowwise(const int8_t* q, const float* s, void* out, int dt, int64_t M, int64_t K, int block,
+int launch_dequantize_rowwise(const int8_t* q, int64_t ldq, const float* s, void* out, int dt, int64_t M, int64_t K, int block,
                               cudaStream_t st) {
     switch (dt) {
-        case BI8_BF16: return dequantize_t(q, s, static_cast<__nv_bfloat16*>(out), M, K, block, st);
-        case BI8_F16: return dequantize_t(q, s, static_cast<__half*>(out), M, K, block, st);
-        case BI8_F32: return dequantize_t(q, s, static_cast<float*>(out), M, K, block, st);
+        case BI8_BF16: return dequantize_t(q, ldq, s, static_cast<__nv_bfloat16*>(out), M, K, block, st);
+        case BI8_F16: return dequantize_t(q, ldq, s, static_cast<__half*>(out), M, K, block, st);
+        case BI8_F32: return dequantize_t(q, ldq, s, static_cast<float*>(out), M, K, block, st);
     }
     return fail(BI8_ERR_DTYPE, "dequantize: unknown dtype code %d", dt);
 }

@@ -105,7 +105,7 @@ __device__ __forceinline__ float round_to(float v, int dt) {
 // Quantizes the eight values of a unit whose block's other units sit in the neighbouring lanes (LPB lanes per block)
 // and stores them; all 32 lanes of the warp must call it.
 template <int QB>
-__device__ __forceinline__ void quantize_unit(const float* y, bool valid, bool short_mantissa, int8_t* q, float* sx, int m, int k,
+__device__ __forceinline__ void quantize_unit(const float (&y)[8], bool valid, bool short_mantissa, int8_t* q, int64_t ldq, float* sx, int m, int k,
                                               int M, int K, bool vec) {
     constexpr int LPB = QB / 8;
     float amax = 0.0f;
@@ -115,30 +115,11 @@ __device__ __forceinline__ void quantize_unit(const float* y, bool valid, bool s
     for (int off = 1; off < LPB; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
     BlockQ bq;
     bq.set(amax, short_mantissa);
-    // the exact-division shortcut on packed pairs when every block of the warp qualifies (a lane without a unit does not
-    // count); else the scalar form with its per-block choice
-    const bool warp_fast = __all_sync(0xffffffffu, bq.fast || !valid);
     if (!valid) return;
-    uint32_t b[8];
-    if (warp_fast) {
-        const uint64_t r2 = f2_pack(bq.rcp, bq.rcp), ns2 = f2_pack(-amax, -amax);
-        const uint64_t c127 = f2_pack(127.0f, 127.0f), cmagic = f2_pack(kMagic, kMagic), cone = f2_pack(1.0f, 1.0f);
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            const uint64_t v2 = f2_pack(y[2 * h], y[2 * h + 1]);
-            const uint64_t q0 = f2_mul(v2, r2);
-            const uint64_t e = f2_fma(ns2, q0, v2);
-            const uint64_t yq = f2_fma(e, r2, q0);
-            f2_bits(f2_fma(f2_mul(c127, yq), cone, cmagic), b[2 * h], b[2 * h + 1]);
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) b[e] = bq.q(y[e]);
-    }
-    const uint32_t lo = pack4(b[0], b[1], b[2], b[3]);
-    const uint32_t hi = pack4(b[4], b[5], b[6], b[7]);
-    int8_t* dst = q + (int64_t)m * K + k;
-    if (vec && k + 8 <= K) {
+    uint32_t lo, hi;
+    quantize8(y, bq, lo, hi);
+    int8_t* dst = q + (int64_t)m * ldq + k;
+    if (vec) {                               // the row pitch covers the eight bytes of a row's last unit
         *reinterpret_cast<uint2*>(dst) = make_uint2(lo, hi);
     } else {
 #pragma unroll
@@ -156,7 +137,7 @@ __device__ __forceinline__ void quantize_unit(const float* y, bool valid, bool s
 template <int QB, int THREADS, int DT>
 __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quantize_kernel(const void* __restrict__ x, int64_t ldx,
                                                                        const void* __restrict__ weight, float eps,
-                                                                       int8_t* __restrict__ q, float* __restrict__ sx, int M, int K,
+                                                                       int8_t* __restrict__ q, int64_t ldq, float* __restrict__ sx, int M, int K,
                                                                        int nb, int vec_in, int vec_out) {
     after_predecessor();
     constexpr int LPB = QB / 8;
@@ -203,7 +184,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quan
     const float rstd = rsqrtf(__fadd_rn(__fdiv_rn(total, (float)K), eps));
     const bool short_mantissa = dt != BI8_F32;
     // normalises, rounds and quantizes the unit whose elements are in y (all lanes of a warp call it together)
-    auto finish_unit = [&](float* y, int k, bool valid) {
+    auto finish_unit = [&](float (&y)[8], int k, bool valid) {
         if (valid) {
             float w8[8];
             if (weight) load8(w8, weight, 0, k, K, dt, vec_in != 0);
@@ -214,7 +195,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quan
                 y[e] = round_to(v, dt);
             }
         }
-        quantize_unit<QB>(y, valid, short_mantissa, q, sx, m, k, M, K, vec_out != 0);
+        quantize_unit<QB>(y, valid, short_mantissa, q, ldq, sx, m, k, M, K, vec_out != 0);
     };
     if (hold) {
 #pragma unroll
@@ -245,7 +226,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quan
 // One thread per unit of eight elements, as in the decode quantizer.
 template <int QB, int DT>
 __global__ void __launch_bounds__(kPreThreads) silu_mul_quantize_kernel(const void* __restrict__ gate, const void* __restrict__ up,
-                                                                        int64_t ldx, int8_t* __restrict__ q,
+                                                                        int64_t ldx, int8_t* __restrict__ q, int64_t ldq,
                                                                         float* __restrict__ sx, int M, int K, int nb, int vec_in,
                                                                         int vec_out) {
     after_predecessor();
@@ -268,7 +249,7 @@ __global__ void __launch_bounds__(kPreThreads) silu_mul_quantize_kernel(const vo
             y[e] = round_to(__fmul_rn(s, v[e]), dt);
         }
     }
-    quantize_unit<QB>(y, valid, dt != BI8_F32, q, sx, m, k, M, K, vec_out != 0);
+    quantize_unit<QB>(y, valid, dt != BI8_F32, q, ldq, sx, m, k, M, K, vec_out != 0);
 }
 
 // C[m, n] = cast(C[m, n] + R[m, n]): the addition a layer's `x + proj(...)` performs in the activation type
@@ -298,7 +279,7 @@ int launch_residual_add(void* C, int64_t ldc, const void* R, int64_t ldr, int dt
     return launch_chained(residual_add_kernel, (unsigned)blocks, kPreThreads, 0, st, C, ldc, R, ldr, dt, M, N);
 }
 
-int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t ldx, const void* weight, float eps, int8_t* q, float* sx,
+int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t ldx, const void* weight, float eps, int8_t* q, int64_t ldq, float* sx,
                         int64_t M, int64_t K, int block, cudaStream_t st) {
     if (M == 0 || K == 0) return BI8_OK;
     if (M > 0x7fffffff || K > 0x3fffffff) return fail(BI8_ERR_LIMIT, "quantize_pre: M or K too large");
@@ -306,8 +287,8 @@ int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t l
     const int nb = (int)((K + block - 1) / block);
     const bool rows16 = (ldx * esz) % 16 == 0 && K % 8 == 0;
     const int vec_in = rows16 && aligned(x, 16) && (!x2 || aligned(x2, 16)) && (!weight || aligned(weight, 16));
-    const int vec_out = K % 8 == 0 && aligned(q, 8);
-    if (op == BI8_PRE_NONE) return launch_quantize_rowwise(x, dt, ldx, q, sx, M, K, block, st);
+    const int vec_out = ldq % 8 == 0 && aligned(q, 8);
+    if (op == BI8_PRE_NONE) return launch_quantize_rowwise(x, dt, ldx, q, ldq, sx, M, K, block, st);
     const int Mi = (int)M, Ki = (int)K;
     if (op == BI8_PRE_RMSNORM) {
         // 128 threads per row where the row fits their registers and there are rows enough to fill the SMs ten deep; a
@@ -315,9 +296,9 @@ int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t l
         const bool narrow = (int64_t)nb * (block / 8) <= kPreHold * 128 && M > 1024;
 #define BI8_PRE_RMS_T(QB, T)                                                                                                          \
     do {                                                                                                                             \
-        if (dt == BI8_BF16) return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_BF16>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, sx, Mi, Ki, nb, vec_in, vec_out); \
-        else if (dt == BI8_F16) return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_F16>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, sx, Mi, Ki, nb, vec_in, vec_out); \
-        else return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_F32>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, sx, Mi, Ki, nb, vec_in, vec_out); \
+        if (dt == BI8_BF16) return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_BF16>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
+        else if (dt == BI8_F16) return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_F16>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
+        else return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_F32>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
     } while (0)
 #define BI8_PRE_RMS(QB)                                                                                                              \
     if (narrow) BI8_PRE_RMS_T(QB, 128);                                                                                              \
@@ -336,9 +317,9 @@ int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t l
         const unsigned grid = (unsigned)((units + kPreThreads - 1) / kPreThreads);
 #define BI8_PRE_SILU(QB)                                                                                                             \
     do {                                                                                                                             \
-        if (dt == BI8_BF16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_BF16>, grid, kPreThreads, 0, st, x, x2, ldx, q, sx, Mi, Ki, nb, vec_in, vec_out); \
-        else if (dt == BI8_F16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_F16>, grid, kPreThreads, 0, st, x, x2, ldx, q, sx, Mi, Ki, nb, vec_in, vec_out); \
-        else return launch_chained(silu_mul_quantize_kernel<QB, BI8_F32>, grid, kPreThreads, 0, st, x, x2, ldx, q, sx, Mi, Ki, nb, vec_in, vec_out); \
+        if (dt == BI8_BF16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_BF16>, grid, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
+        else if (dt == BI8_F16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_F16>, grid, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
+        else return launch_chained(silu_mul_quantize_kernel<QB, BI8_F32>, grid, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
     } while (0)
         switch (block) {
             case 32: BI8_PRE_SILU(32); break;

@@ -8,7 +8,12 @@
 //
 // Persistent CTAs walk over tiles of 128 rows x 128 columns of a 16-bit input:
 //   * one elected thread fetches the tile with two TMA loads (64 columns = 128 bytes wide each, 128-byte swizzle) that
-//     complete on an mbarrier; rows and columns outside the tensor arrive as zeros;
+//     complete on an mbarrier; rows and columns outside the tensor arrive as zeros.  Inputs whose rows are not 16-byte
+//     aligned, which a tensor map cannot describe (a 50257-wide vocabulary), are fetched by all threads instead (SHIFT): a
+//     half-warp reads a tile row as aligned 16-byte pieces, shifts the bytes into place between neighbouring lanes and
+//     stores them where the TMA would have put them.  The loads of the next tile are in flight, in registers, while the
+//     current one is quantized.  (A zero-padded copy in front of the kernel cost one more pass: 0.9 ms for a
+//     8192 x 50257 matrix.);
 //   * column-wise: a thread owns a pair of adjacent columns and 32 rows.  It reads them as 32 four-byte words (all lanes
 //     of a warp read one row: conflict free under the swizzle), takes the absmax of both columns with packed 16-bit
 //     max instructions, exchanges it with the other row groups of its block through shared memory, and quantizes
@@ -131,11 +136,100 @@ __device__ __forceinline__ void role_barrier(int id, int n) { asm volatile("bar.
 // has its part of it in registers).  256 threads do the column-wise work; in the dual kernel 256 more do the row-wise work on the
 // same tile at the same time.  Each role has its own named barrier and its own elected thread for the TMA store of its
 // output tile, so neither waits for the other.
-template <typename T, int B, bool DUAL>
+// One tile of an input with unaligned rows, by NT threads: a half-warp has the 16 16-byte chunks of a row, the two half-warps have
+// rows r and r + 8, whose byte offset from a 16-byte boundary is the same (the row pitch is even), so that the shift is the
+// same in all lanes of a warp.  Per step, warp w of NT / 32 takes the row pairs w, w + NT / 32, ...
+template <int NT>
+struct ShiftLoader {
+    static constexpr int STEPS = kQT * 16 / NT;
+    uint4 piece[STEPS];           // the aligned 16 bytes at or before the chunk's first byte
+    uint4 last[STEPS];            // lane 15 of a half-warp: the 16 bytes behind its own
+    const unsigned char* x;
+    int64_t pitch;                // bytes
+    int R, C;
+
+    static __device__ __forceinline__ int tile_row(int tid, int step) {
+        const int g = (tid >> 5) + step * (NT / 32);
+        return (g >> 3) * 16 + (g & 7) + 8 * ((tid >> 4) & 1);
+    }
+    // Requests the pieces of the tile at (r0, c0).  A piece is read only where it contains a byte of the row's part inside the
+    // tile, so no access leaves the tensor's 16-byte granules.
+    __device__ __forceinline__ void request(int tid, int r0, int c0) {
+        const int i = tid & 15;
+        const unsigned char* tile = x + (int64_t)r0 * pitch + (int64_t)c0 * 2;
+        if (r0 + kQT <= R && c0 + kQT <= C) {
+#pragma unroll
+            for (int u = 0; u < STEPS; ++u) {
+                const uintptr_t a = reinterpret_cast<uintptr_t>(tile + (int64_t)tile_row(tid, u) * pitch);
+                const void* at = reinterpret_cast<const void*>((a & ~(uintptr_t)15) + 16 * i);
+                piece[u] = ld_nc_v4(at);
+                if (i == 15 && (a & 15u) != 0) last[u] = ld_nc_v4(static_cast<const unsigned char*>(at) + 16);
+            }
+        } else {
+            const int cols = C - c0 < kQT ? C - c0 : kQT;
+#pragma unroll
+            for (int u = 0; u < STEPS; ++u) {
+                piece[u] = last[u] = make_uint4(0u, 0u, 0u, 0u);
+                if (r0 + tile_row(tid, u) < R) {
+                    const uintptr_t a = reinterpret_cast<uintptr_t>(tile + (int64_t)tile_row(tid, u) * pitch);
+                    const uintptr_t end = a + (uintptr_t)cols * 2, at = (a & ~(uintptr_t)15) + 16 * i;
+                    if (at < end) piece[u] = ld_nc_v4(reinterpret_cast<const void*>(at));
+                    if (i == 15 && (a & 15u) != 0 && at + 16 < end) last[u] = ld_nc_v4(reinterpret_cast<const void*>(at + 16));
+                }
+            }
+        }
+    }
+    // Shifts the requested bytes into place and stores the tile at shared address `tile` (two swizzled 128 x 128-byte halves);
+    // elements outside the tensor become zero.  All lanes of a warp call it together.
+    __device__ __forceinline__ void store(int tid, int r0, int c0, uint32_t tile) {
+        const int i = tid & 15;
+        const bool edge = r0 + kQT > R || c0 + kQT > C;
+        const uint32_t dst = tile + (uint32_t)((i >> 3) * kQT * 128);
+        const uint32_t base_off = (uint32_t)(reinterpret_cast<uintptr_t>(x) + (uintptr_t)c0 * 2), p32 = (uint32_t)pitch;
+#pragma unroll
+        for (int u = 0; u < STEPS; ++u) {
+            const int tr = tile_row(tid, u);
+            const uint32_t off = (base_off + (uint32_t)(r0 + tr) * p32) & 15u, bits = (off & 2u) * 8u;
+            const uint32_t own[4] = {piece[u].x, piece[u].y, piece[u].z, piece[u].w};
+            const uint32_t tail[4] = {last[u].x, last[u].y, last[u].z, last[u].w};
+            uint32_t w[4];
+            auto shifted = [&](auto words) {              // the row's bytes begin `WS` words (and `bits` bits) into the piece
+                constexpr int WS = decltype(words)::value;
+                uint32_t r[5];
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    if (k + WS < 4) {
+                        r[k] = own[(k + WS) & 3];
+                    } else {
+                        const uint32_t next = __shfl_down_sync(0xffffffffu, own[(k + WS) & 3], 1);
+                        r[k] = i == 15 ? tail[(k + WS) & 3] : next;
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) w[k] = __funnelshift_r(r[k], r[k + 1], bits);
+            };
+            if (off < 4u) shifted(std::integral_constant<int, 0>{});
+            else if (off < 8u) shifted(std::integral_constant<int, 1>{});
+            else if (off < 12u) shifted(std::integral_constant<int, 2>{});
+            else shifted(std::integral_constant<int, 3>{});
+            if (edge) {
+                const int valid = r0 + tr < R ? C - (c0 + 8 * i) : 0;          // elements of the chunk inside the tensor
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (2 * k >= valid) w[k] = 0u;
+                    else if (2 * k + 1 >= valid) w[k] &= 0xffffu;
+                }
+            }
+            sts_v4(dst + swz(tr, i & 7), w[0], w[1], w[2], w[3]);
+        }
+    }
+};
+
+template <typename T, int B, bool DUAL, bool SHIFT>
 __global__ void __launch_bounds__(DUAL ? 2 * kQThreads : kQThreads, DUAL ? 1 : 2)
 quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmQc,
-                     const __grid_constant__ CUtensorMap tmQr, float* __restrict__ s_col, float* __restrict__ s_row, int R, int C,
-                     int col_tiles, int num_tiles, int* status) {
+                     const __grid_constant__ CUtensorMap tmQr, const void* __restrict__ x, int64_t ldx, float* __restrict__ s_col,
+                     float* __restrict__ s_row, int R, int C, int col_tiles, int num_tiles, int* status) {
     static_assert(B == 32 || B == 64 || B == 128, "block sizes of the tile quantizer");
     constexpr int NT = DUAL ? 2 * kQThreads : kQThreads;
     constexpr int NST = DUAL ? 3 : 2;                      // input stages: the loads of the next NST - 1 tiles are in flight
@@ -159,7 +253,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     };
     if (tid == 0) {
         for (int s = 0; s < NST; ++s) {
-            mbar_init(full(s), 1);
+            mbar_init(full(s), SHIFT ? NT : 1);
             mbar_init(empty(s), NT);
         }
         sts_u32(abort_flag, 0u);
@@ -167,13 +261,26 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
         fence_proxy_async_smem();
     }
     after_predecessor();
-    if (tid == 0) {
+    ShiftLoader<NT> loader;
+    if constexpr (SHIFT) {
+        loader.x = static_cast<const unsigned char*>(x);
+        loader.pitch = ldx * 2;
+        loader.R = R;
+        loader.C = C;
+        if ((int)blockIdx.x < num_tiles) loader.request(tid, ((int)blockIdx.x / col_tiles) * kQT, ((int)blockIdx.x % col_tiles) * kQT);
+    } else if (tid == 0) {
         for (int s = 0; s < NST - 1; ++s) {
             const int64_t t0 = (int64_t)blockIdx.x + (int64_t)s * gridDim.x;
             if (t0 < num_tiles) issue((int)t0, s);
         }
     }
     __syncthreads();
+    if constexpr (SHIFT) {
+        if ((int)blockIdx.x < num_tiles) {
+            loader.store(tid, ((int)blockIdx.x / col_tiles) * kQT, ((int)blockIdx.x % col_tiles) * kQT, base + L::in_off);
+            mbar_arrive(full(0));
+        }
+    }
 
     const bool col_role = tid < kQThreads;
     const int rt_id = col_role ? 1 : 2;                   // the role's named barrier
@@ -183,7 +290,10 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     int it = 0, cur = 0;
     uint32_t par = 0;                                      // parity of stage `cur`'s full barrier for this use
     for (int64_t t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
-        if (tid == 0) {
+        const int64_t tnext = t + gridDim.x;
+        if constexpr (SHIFT) {
+            if (tnext < num_tiles) loader.request(tid, (int)(tnext / col_tiles) * kQT, (int)(tnext % col_tiles) * kQT);
+        } else if (tid == 0) {
             // the tile NST - 1 iterations ahead goes into the stage that was read in the previous iteration
             const int64_t tn = t + (int64_t)(NST - 1) * gridDim.x;
             if (tn < num_tiles) {
@@ -201,6 +311,23 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
         const uint32_t in_tile = base + L::in_off + (uint32_t)cur * kInStage;
         const int this_stage = cur;
         if (++cur == NST) { cur = 0; par ^= 1u; }
+        // SHIFT: the next tile goes into stage `cur`, last read NST - 1 iterations ago
+        auto store_next = [&] {
+            if constexpr (SHIFT) {
+                if (tnext < num_tiles) {
+                    if (ok && it >= NST - 1) {
+                        ok = mbar_wait(empty(cur), (uint32_t)(((it + 1 - NST) / NST) & 1), abort_flag, kLimit);
+                        if (!ok) fail_code = QW_EMPTY;
+                    }
+                    // warp-aligned: the lanes exchange bytes; after a wait that ran out nothing is stored
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (ok) {
+                        loader.store(tid, (int)(tnext / col_tiles) * kQT, (int)(tnext % col_tiles) * kQT, base + L::in_off + (uint32_t)cur * kInStage);
+                        mbar_arrive(full(cur));
+                    }
+                }
+            }
+        };
 
         if (col_role) {
             // ---------------- column-wise ----------------
@@ -282,6 +409,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                 tma_store_2d(&tmQc, outc, r0, c0);
                 tma_store_commit();
             }
+            store_next();
         } else {
             // ---------------- row-wise ----------------
             const int rwarp = rtid >> 5;
@@ -351,6 +479,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                 tma_store_2d(&tmQr, outr, c0, r0);
                 tma_store_commit();
             }
+            store_next();
         }
     }
     // shared memory must stay valid until the last stores have read it
@@ -358,13 +487,13 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     if (!ok && rtid == 0 && fail_code != 0) report_timeout(status, abort_flag, fail_code);
 }
 
-// int8 [rows, cols] row-major, contiguous rows (cols a multiple of 16, 16-byte aligned base) -> boxes of 128 x 128 bytes, 128-byte swizzle
-int make_q_map(CUtensorMap* map, int8_t* ptr, int64_t rows, int64_t cols) {
+// int8 [rows, cols] row-major, row pitch ld bytes (a multiple of 16, 16-byte aligned base) -> boxes of 128 x 128 bytes, 128-byte swizzle
+int make_q_map(CUtensorMap* map, int8_t* ptr, int64_t rows, int64_t cols, int64_t ld) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fail(BI8_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     ensure_current_context();
     cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t gstride[1] = {(cuuint64_t)cols};
+    cuuint64_t gstride[1] = {(cuuint64_t)ld};
     cuuint32_t box[2] = {128, 128};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, ptr, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -398,22 +527,22 @@ int cached_x_map(CUtensorMap* map, int dev, const void* ptr, int64_t rows, int64
     if (rc == BI8_OK) map_cache().put(key, *map);
     return rc;
 }
-int cached_q_map(CUtensorMap* map, int dev, int8_t* ptr, int64_t rows, int64_t cols) {
-    const MapKey key{dev, 6, ptr, rows, cols, cols, 128, 128};
+int cached_q_map(CUtensorMap* map, int dev, int8_t* ptr, int64_t rows, int64_t cols, int64_t ld) {
+    const MapKey key{dev, 6, ptr, rows, cols, ld, 128, 128};
     if (map_cache().find(key, map)) return BI8_OK;
-    const int rc = make_q_map(map, ptr, rows, cols);
+    const int rc = make_q_map(map, ptr, rows, cols, ld);
     if (rc == BI8_OK) map_cache().put(key, *map);
     return rc;
 }
 
-template <typename T, int B, bool DUAL>
-int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap& tqr, float* s_col, float* s_row, int64_t R,
-                int64_t C, cudaStream_t st) {
+template <typename T, int B, bool DUAL, bool SHIFT>
+int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap& tqr, const void* x, int64_t ldx, float* s_col, float* s_row,
+                int64_t R, int64_t C, cudaStream_t st) {
     const int64_t ctiles = (C + kQT - 1) / kQT, rtiles = (R + kQT - 1) / kQT;
     if (ctiles * rtiles >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "quantize: grid too large");
     constexpr size_t smem = (DUAL ? QLayout<3>::bytes_dual : QLayout<2>::bytes_col) + 1024;
     static SmemOptIn opt_in;
-    const int rc = opt_in.ensure(quantize_tile_kernel<T, B, DUAL>, smem);
+    const int rc = opt_in.ensure(quantize_tile_kernel<T, B, DUAL, SHIFT>, smem);
     if (rc != BI8_OK) return rc;
     int* status = device_status_ptr();
     if (!status) return BI8_ERR_CUDA;
@@ -421,51 +550,56 @@ int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap
     const int64_t tiles = ctiles * rtiles;
     const int64_t resident = (int64_t)(DUAL ? 1 : 2) * di.sms;                 // CTAs that fit at once
     const int grid = (int)(tiles < resident ? tiles : resident);
-    return launch_chained(quantize_tile_kernel<T, B, DUAL>, grid, DUAL ? 2 * kQThreads : kQThreads, smem, st, tx, tqc, tqr, s_col, s_row, (int)R, (int)C, (int)ctiles, (int)tiles, status);
+    return launch_chained(quantize_tile_kernel<T, B, DUAL, SHIFT>, grid, DUAL ? 2 * kQThreads : kQThreads, smem, st, tx, tqc, tqr, x, ldx, s_col, s_row, (int)R, (int)C, (int)ctiles, (int)tiles, status);
 }
 
 template <typename T>
-int tile_dispatch(const void* x, int64_t ldx, int8_t* q_col, float* s_col, int8_t* q_row, float* s_row, int64_t R, int64_t C, int block,
-                  cudaStream_t st) {
+int tile_dispatch(const void* x, int64_t ldx, int8_t* q_col, int64_t ldqc, float* s_col, int8_t* q_row, int64_t ldqr, float* s_row, int64_t R,
+                  int64_t C, int block, cudaStream_t st) {
     CUtensorMap tx, tqc, tqr;
     int dev = 0;
     BI8_CUDA_TRY(cudaGetDevice(&dev));
-    int rc = cached_x_map(&tx, dev, x, R, C, ldx);
+    int rc = cached_q_map(&tqc, dev, q_col, C, R, ldqc);
     if (rc != BI8_OK) return rc;
-    rc = cached_q_map(&tqc, dev, q_col, C, R);
-    if (rc != BI8_OK) return rc;
-    tqr = tqc;
-    const bool dual = q_row != nullptr;
-    if (dual) {
-        rc = cached_q_map(&tqr, dev, q_row, R, C);
+    tx = tqr = tqc;
+    const bool shift = !aligned(x, 16) || (ldx * 2) % 16 != 0;        // no tensor map can describe the input
+    if (!shift) {
+        rc = cached_x_map(&tx, dev, x, R, C, ldx);
         if (rc != BI8_OK) return rc;
     }
-#define BI8_TILE(BB)                                                                                  \
-    if (block == BB)                                                                                  \
-        return dual ? launch_tile<T, BB, true>(tx, tqc, tqr, s_col, s_row, R, C, st)                  \
-                    : launch_tile<T, BB, false>(tx, tqc, tqr, s_col, s_row, R, C, st);
+    const bool dual = q_row != nullptr;
+    if (dual) {
+        rc = cached_q_map(&tqr, dev, q_row, R, C, ldqr);
+        if (rc != BI8_OK) return rc;
+    }
+#define BI8_TILE_D(BB, DUAL)                                                                                \
+    shift ? launch_tile<T, BB, DUAL, true>(tx, tqc, tqr, x, ldx, s_col, s_row, R, C, st)                    \
+          : launch_tile<T, BB, DUAL, false>(tx, tqc, tqr, x, ldx, s_col, s_row, R, C, st)
+#define BI8_TILE(BB) \
+    if (block == BB) return dual ? (BI8_TILE_D(BB, true)) : (BI8_TILE_D(BB, false));
     BI8_TILE(32) BI8_TILE(64) BI8_TILE(128)
 #undef BI8_TILE
+#undef BI8_TILE_D
     return fail(BI8_ERR_BLOCK, "tile quantizer supports block 32, 64, 128 (got %d)", block);
 }
 
 }  // namespace
 
-// The tile quantizer needs what its tensor maps need: a 16-bit input with 16-byte aligned base and row pitch, and int8
-// outputs whose rows (R bytes for the transposed one, C bytes for the row-wise one) are multiples of 16 bytes.
-bool quantize_tile_applicable(const void* x, int dt, int64_t ldx, const void* q_col, const void* q_row, int64_t R, int64_t C, int block) {
+// The tile quantizer takes 16-bit inputs of any alignment; its int8 outputs leave by TMA and need 16-byte aligned bases and row
+// pitches (ldqc for the transposed one, ldqr for the row-wise one).
+bool quantize_tile_applicable(int dt, const void* q_col, int64_t ldqc, const void* q_row, int64_t ldqr, int64_t R, int64_t C, int block) {
     if (dt != BI8_BF16 && dt != BI8_F16) return false;
     if (block != 32 && block != 64 && block != 128) return false;
-    if (R <= 0 || C <= 0 || R >= (1ll << 31) || C >= (1ll << 31)) return false;
-    if (!aligned(x, 16) || (ldx * 2) % 16 != 0 || !aligned(q_col, 16) || R % 16 != 0) return false;
-    if (q_row != nullptr && (!aligned(q_row, 16) || C % 16 != 0)) return false;
+    if (R <= 0 || C <= 0 || R >= (1ll << 31) - 256 || C >= (1ll << 31) - 256) return false;
+    if (!aligned(q_col, 16) || ldqc % 16 != 0) return false;
+    if (q_row != nullptr && (!aligned(q_row, 16) || ldqr % 16 != 0)) return false;
     return device_info().ok;
 }
 
-int launch_quantize_tile(const void* x, int dt, int64_t ldx, int8_t* q_col, float* s_col, int8_t* q_row, float* s_row, int64_t R,
-                         int64_t C, int block, cudaStream_t st) {
-    if (dt == BI8_BF16) return tile_dispatch<__nv_bfloat16>(x, ldx, q_col, s_col, q_row, s_row, R, C, block, st);
-    if (dt == BI8_F16) return tile_dispatch<__half>(x, ldx, q_col, s_col, q_row, s_row, R, C, block, st);
+int launch_quantize_tile(const void* x, int dt, int64_t ldx, int8_t* q_col, int64_t ldqc, float* s_col, int8_t* q_row, int64_t ldqr,
+                         float* s_row, int64_t R, int64_t C, int block, cudaStream_t st) {
+    if (dt == BI8_BF16) return tile_dispatch<__nv_bfloat16>(x, ldx, q_col, ldqc, s_col, q_row, ldqr, s_row, R, C, block, st);
+    if (dt == BI8_F16) return tile_dispatch<__half>(x, ldx, q_col, ldqc, s_col, q_row, ldqr, s_row, R, C, block, st);
     return fail(BI8_ERR_DTYPE, "tile quantizer takes bf16 or fp16 input");
 }
 

@@ -191,20 +191,14 @@ void need_cuda(const Tensor& t) {
     if (!t.is_cuda()) assertion("x.is_cuda");
 }
 
-// Zero-padded copy of a large 16-bit matrix whose row or column count is not a multiple of 16, or an undefined tensor when no
-// padding is called for.  The fast quantizers and the tensor-core GEMM want 16-byte aligned rows.  Padding with zeros
-// changes no result: the pad stays inside the last block (block sizes here are multiples of 16), and zeros change
-// neither a block's absmax nor the quantized values of its other elements.
-Tensor pad16(const Tensor& x, int64_t block, bool rows, bool cols) {
-    const int64_t r = x.size(0), c = x.size(1);
-    if ((x.scalar_type() != at::kBFloat16 && x.scalar_type() != at::kHalf) || block % 16 != 0 || r * c < (1 << 22)) return Tensor();
-    const int64_t rp = rows ? ceil_div(r, 16) * 16 : r, cp = cols ? ceil_div(c, 16) * 16 : c;
-    if ((rp == r && cp == c) || std::min(r, c) < 256) return Tensor();
-    Tensor buf = empty_on(x, {rp, cp}, x.scalar_type());
-    if (rp != r) buf.zero_();
-    else buf.narrow(1, c, cp - c).zero_();
-    buf.narrow(0, 0, r).narrow(1, 0, c).copy_(x);
-    return buf;
+// Row pitch of a quantized matrix: the next multiple of 16 bytes, which is what the wide kernels and the tensor-core GEMM take.
+int64_t pitch16(int64_t n) { return (n + 15) / 16 * 16; }
+
+// int8 [rows, cols] whose rows begin on 16-byte boundaries: dense where cols is a multiple of 16, else a view of a wider buffer
+Tensor empty_q(const Tensor& like, int64_t rows, int64_t cols) {
+    const int64_t ld = pitch16(cols);
+    Tensor t = empty_on(like, {rows, ld}, at::kChar);
+    return ld == cols ? t : t.narrow(1, 0, cols);
 }
 
 // Copy with a 16-byte aligned row pitch of an int8 operand that has none; the bytes between K and the pitch are never read.
@@ -225,36 +219,24 @@ struct Quantized {
 
 Quantized quantize_rowwise(const Tensor& x, int64_t block) {
     need_cuda(x);
-    if (x.dim() == 2) {
-        const Tensor padded = pad16(x, block, false, true);
-        if (padded.defined()) {
-            Quantized r = quantize_rowwise(padded, block);
-            return {r.q.narrow(1, 0, x.size(1)), r.s};       // a view with an aligned row pitch, which the GEMM takes as it is
-        }
-    }
     OnDevice on(x);
     const Mat m = mat2d(x);
     const int code = dtype_code(x.scalar_type());
-    Quantized r{empty_on(x, {m.rows, m.cols}, at::kChar), empty_on(x, {ceil_div(m.cols, block), m.rows}, at::kFloat)};
-    check(bi8_quantize_rowwise(m.ptr, code, m.ld, r.q.mutable_data_ptr<int8_t>(), r.s.mutable_data_ptr<float>(), m.rows, m.cols, (int)block, on.raw()),
+    Quantized r{empty_q(x, m.rows, m.cols), empty_on(x, {ceil_div(m.cols, block), m.rows}, at::kFloat)};
+    check(bi8_quantize_rowwise_pitched(m.ptr, code, m.ld, r.q.mutable_data_ptr<int8_t>(), pitch16(m.cols), r.s.mutable_data_ptr<float>(), m.rows,
+                                       m.cols, (int)block, on.raw()),
           "bi8_quantize_rowwise");
     return r;
 }
 
 Quantized quantize_colwise(const Tensor& x, int64_t block) {
     need_cuda(x);
-    if (x.dim() == 2) {
-        const Tensor padded = pad16(x, block, true, true);
-        if (padded.defined()) {
-            Quantized r = quantize_colwise(padded, block);
-            return {r.q.narrow(0, 0, x.size(1)).narrow(1, 0, x.size(0)), r.s.narrow(1, 0, x.size(1))};
-        }
-    }
     OnDevice on(x);
     const Mat m = mat2d(x);
     const int code = dtype_code(x.scalar_type());
-    Quantized r{empty_on(x, {m.cols, m.rows}, at::kChar), empty_on(x, {ceil_div(m.rows, block), m.cols}, at::kFloat)};
-    check(bi8_quantize_colwise(m.ptr, code, m.ld, r.q.mutable_data_ptr<int8_t>(), r.s.mutable_data_ptr<float>(), m.rows, m.cols, (int)block, on.raw()),
+    Quantized r{empty_q(x, m.cols, m.rows), empty_on(x, {ceil_div(m.rows, block), m.cols}, at::kFloat)};
+    check(bi8_quantize_colwise_pitched(m.ptr, code, m.ld, r.q.mutable_data_ptr<int8_t>(), pitch16(m.rows), r.s.mutable_data_ptr<float>(), m.rows,
+                                       m.cols, (int)block, on.raw()),
           "bi8_quantize_colwise");
     return r;
 }
@@ -265,21 +247,14 @@ struct Dual {
 
 Dual quantize_dual(const Tensor& x, int64_t block) {
     need_cuda(x);
-    if (x.dim() == 2) {
-        const Tensor padded = pad16(x, block, true, true);
-        if (padded.defined()) {
-            Dual d = quantize_dual(padded, block);
-            const int64_t r = x.size(0), c = x.size(1);
-            return {{d.row.q.narrow(0, 0, r).narrow(1, 0, c), d.row.s.narrow(1, 0, r)}, {d.col.q.narrow(0, 0, c).narrow(1, 0, r), d.col.s.narrow(1, 0, c)}};
-        }
-    }
     OnDevice on(x);
     const Mat m = mat2d(x);
     const int code = dtype_code(x.scalar_type());
-    Dual d{{empty_on(x, {m.rows, m.cols}, at::kChar), empty_on(x, {ceil_div(m.cols, block), m.rows}, at::kFloat)},
-           {empty_on(x, {m.cols, m.rows}, at::kChar), empty_on(x, {ceil_div(m.rows, block), m.cols}, at::kFloat)}};
-    check(bi8_quantize_dual(m.ptr, code, m.ld, d.row.q.mutable_data_ptr<int8_t>(), d.row.s.mutable_data_ptr<float>(),
-                            d.col.q.mutable_data_ptr<int8_t>(), d.col.s.mutable_data_ptr<float>(), m.rows, m.cols, (int)block, on.raw()),
+    Dual d{{empty_q(x, m.rows, m.cols), empty_on(x, {ceil_div(m.cols, block), m.rows}, at::kFloat)},
+           {empty_q(x, m.cols, m.rows), empty_on(x, {ceil_div(m.rows, block), m.cols}, at::kFloat)}};
+    check(bi8_quantize_dual_pitched(m.ptr, code, m.ld, d.row.q.mutable_data_ptr<int8_t>(), pitch16(m.cols), d.row.s.mutable_data_ptr<float>(),
+                                    d.col.q.mutable_data_ptr<int8_t>(), pitch16(m.rows), d.col.s.mutable_data_ptr<float>(), m.rows, m.cols,
+                                    (int)block, on.raw()),
           "bi8_quantize_dual");
     return d;
 }
@@ -297,9 +272,10 @@ Tensor dequantize(const Tensor& q, const Tensor& state, int64_t block, at::Scala
     const int64_t m = q.size(0), k = q.size(1);
     check_scales(state, ceil_div(k, block), m, block, "state");
     OnDevice on(q);
-    const Tensor x = q.contiguous(), s = state.contiguous();
+    const Mat x = mat2d(q);
+    const Tensor s = state.contiguous();
     Tensor out = empty_on(q, {m, k}, out_type);
-    check(bi8_dequantize_rowwise(x.const_data_ptr<int8_t>(), s.const_data_ptr<float>(), out.data_ptr(), dtype_code(out_type), m, k, (int)block, on.raw()),
+    check(bi8_dequantize_rowwise_pitched(static_cast<const int8_t*>(x.ptr), x.ld, s.const_data_ptr<float>(), out.data_ptr(), dtype_code(out_type), m, k, (int)block, on.raw()),
           "bi8_dequantize_rowwise");
     return out;
 }
@@ -405,9 +381,9 @@ Quantized quantize_pre(int op, const Tensor& x_in, const Tensor& x2, const Tenso
     OnDevice on(x_in);
     const Pre pre(op, x_in, x2, weight);
     const int64_t m = pre.x.rows, k = pre.x.cols;
-    Quantized r{empty_on(x_in, {m, k}, at::kChar), empty_on(x_in, {ceil_div(k, block), m}, at::kFloat)};
-    check(bi8_quantize_rowwise_pre(op, pre.x.ptr, pre.x2.ptr, dtype_code(x_in.scalar_type()), pre.x.ld, pre.weight_ptr(), (float)eps,
-                                   r.q.mutable_data_ptr<int8_t>(), r.s.mutable_data_ptr<float>(), m, k, (int)block, on.raw()),
+    Quantized r{empty_q(x_in, m, k), empty_on(x_in, {ceil_div(k, block), m}, at::kFloat)};
+    check(bi8_quantize_rowwise_pre_pitched(op, pre.x.ptr, pre.x2.ptr, dtype_code(x_in.scalar_type()), pre.x.ld, pre.weight_ptr(), (float)eps,
+                                   r.q.mutable_data_ptr<int8_t>(), pitch16(k), r.s.mutable_data_ptr<float>(), m, k, (int)block, on.raw()),
           "bi8_quantize_rowwise_pre");
     return r;
 }
@@ -421,7 +397,7 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
     if (w.scalar_type() != at::kChar) value_error(std::string("weights must be int8, got ") + c10::toString(w.scalar_type()));
     OnDevice on(x_in);
     const Pre pre(op, x_in, x2, norm_weight);
-    const Mat bt = w_transposed ? mat2d_t(w) : mat2d(w);
+    Mat bt = w_transposed ? mat2d_t(w) : mat2d(w);
     const int64_t m = pre.x.rows, k = pre.x.cols, n = bt.rows, nb = ceil_div(k, block);
     check_scales(state_w, nb, n, block, "state_w");
     const Tensor sw = state_w.contiguous();
@@ -451,19 +427,30 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
     // the quantized activations live in the stream's scratch behind the GEMM's workspace
     Carve carve;
     carve.take((int64_t)ws_bytes);
-    const int64_t xq_at = carve.take(m * k), sx_at = carve.take(nb * m * 4);
+    const int64_t xq_at = carve.take(m * pitch16(k)), sx_at = carve.take(nb * m * 4);
     const Tensor ws = workspace(x_in.device(), on.stream, carve.bytes);
     char* ws_ptr = ws.defined() ? static_cast<char*>(ws.data_ptr()) : nullptr;
-    if (k % 16 != 0 && op == BI8_PRE_NONE && !res.defined() && m > 64 && target.is_same(out) && !out_in.defined() && flags == 0) {
-        // rows that are not 16-byte aligned: the quantizer and the GEMM re-pitch their operands
-        const Quantized r = quantize_rowwise(pre.x.owner.dim() == 2 ? pre.x.owner : pre.x.owner.reshape({m, k}), block);
-        return gemm(r.q, w_transposed ? w : w.t(), r.s, sw, bias_in, block, out_type, 0).view(shape);
+    int8_t* xq = reinterpret_cast<int8_t*>(ws_ptr + xq_at);
+    float* sx = reinterpret_cast<float*>(ws_ptr + sx_at);
+    void* gemm_ws = ws_bytes ? ws_ptr : nullptr;
+    const void* res_ptr = res.defined() ? res.data_ptr() : nullptr;
+    if (k % 16 != 0) {
+        // Rows that are not 16-byte aligned: the activations are quantized into rows that are, weights that have come without
+        // a pitch (a checkpoint's dense copy) are re-pitched where the GEMM is long enough to gain from it.
+        if (k >= 256 && m * n >= 128 * 128) bt = repitch(bt, x_in);
+        check(bi8_quantize_rowwise_pre_pitched(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps, xq, pitch16(k), sx, m, k,
+                                               (int)block, on.raw()),
+              "bi8_quantize_rowwise_pre");
+        check(bi8_gemm_dequant_residual(xq, pitch16(k), static_cast<const int8_t*>(bt.ptr), bt.ld, sx, sw.const_data_ptr<float>(), bias.ptr, bias.code,
+                                        res_ptr, ldr, target.data_ptr(), ldc, dtype_code(out_type), m, n, k, (int)block, gemm_ws, ws_bytes,
+                                        flags & ~BI8_GEMM_QUANT_IN_KERNEL, on.raw()),
+              "bi8_gemm_dequant_residual");
+        if (!target.is_same(out)) out.copy_(target);
+        return out;
     }
-    check(bi8_gemm_dequant_fused_pre(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps,
-                                     reinterpret_cast<int8_t*>(ws_ptr + xq_at), reinterpret_cast<float*>(ws_ptr + sx_at),
-                                     static_cast<const int8_t*>(bt.ptr), bt.ld, sw.const_data_ptr<float>(), bias.ptr, bias.code,
-                                     res.defined() ? res.data_ptr() : nullptr, ldr, target.data_ptr(), ldc, dtype_code(out_type), m, n, k,
-                                     (int)block, ws_bytes ? ws_ptr : nullptr, ws_bytes, flags, on.raw()),
+    check(bi8_gemm_dequant_fused_pre(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps, xq, sx,
+                                     static_cast<const int8_t*>(bt.ptr), bt.ld, sw.const_data_ptr<float>(), bias.ptr, bias.code, res_ptr, ldr,
+                                     target.data_ptr(), ldc, dtype_code(out_type), m, n, k, (int)block, gemm_ws, ws_bytes, flags, on.raw()),
           "bi8_gemm_dequant_fused_pre");
     if (!target.is_same(out)) out.copy_(target);
     return out;

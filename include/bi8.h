@@ -116,6 +116,28 @@ BI8_API int bi8_gemm_dequant(const int8_t* A, int64_t lda, const int8_t* Bt, int
 
 BI8_API size_t bi8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int block);
 
+/* bi8_gemm_dequant plus an addend: C = cast(cast(sum) (+ bias) + residual[m,n]), the addition in the output type as a layer's
+ * `x + proj(...)` performs it.  residual [M,N] of out_dtype, row stride ldr; it must not overlap C. */
+BI8_API int bi8_gemm_dequant_residual(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb,
+                     const float* sA, const float* sB, const void* bias, int bias_dtype, const void* residual, int64_t ldr,
+                     void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N, int64_t K, int block,
+                     void* workspace, size_t workspace_bytes, int flags, void* stream);
+
+/* The quantizers and the dequantizer with a row pitch (bytes) of the int8 tensor of their own, ldq >= its row length.  With a
+ * pitch that is a multiple of 16 every shape runs on the wide kernels and the GEMM takes the result as it is; the bytes
+ * between a row's end and its pitch are unspecified.  In bi8_quantize_colwise_pitched q is [C, ldq] with R values per row. */
+BI8_API int bi8_quantize_rowwise_pitched(const void* x, int x_dtype, int64_t ldx, int8_t* q, int64_t ldq, float* s,
+                                         int64_t M, int64_t K, int block, void* stream);
+BI8_API int bi8_quantize_colwise_pitched(const void* x, int x_dtype, int64_t ldx, int8_t* q, int64_t ldq, float* s,
+                                         int64_t R, int64_t C, int block, void* stream);
+BI8_API int bi8_quantize_dual_pitched(const void* x, int x_dtype, int64_t ldx, int8_t* q_row, int64_t ldq_row, float* s_row,
+                                      int8_t* q_col, int64_t ldq_col, float* s_col, int64_t R, int64_t C, int block, void* stream);
+BI8_API int bi8_quantize_rowwise_pre_pitched(int op, const void* x, const void* x2, int x_dtype, int64_t ldx, const void* weight,
+                                             float eps, int8_t* q, int64_t ldq, float* scales, int64_t M, int64_t K, int block,
+                                             void* stream);
+BI8_API int bi8_dequantize_rowwise_pitched(const int8_t* q, int64_t ldq, const float* s, void* out, int out_dtype,
+                                           int64_t M, int64_t K, int block, void* stream);
+
 /* bi8_gemm_dequant for callers that cannot provide a workspace because they cannot allocate device memory when
  * they call: a serving loop that must not touch cudaMalloc after start-up, a plugin whose host runtime owns the
  * allocator, a caller with a fixed memory footprint.  (No counterpart in the reference, whose wrappers allocate
