@@ -84,12 +84,12 @@ int dispatch_gemm(const GemmArgs& g, cudaStream_t st) {
     if (g.flags & BI8_GEMM_FORCE_SKINNY) {
         if (!gemm_skinny_applicable(g))
             return fail(BI8_ERR_ALIGN, "skinny tensor-core GEMM not applicable (needs M <= 64, block 32/64/128, N %% 4 == 0, 16-byte aligned "
-                                       "operand rows and weight scales, and the workspace bi8_gemm_workspace_bytes() asks for)");
+                                       "operand rows and weight scales)");
         return then_residual(launch_gemm_skinny(g, st), g, st);
     }
     const bool free_choice = !(g.flags & (BI8_GEMM_FORCE_TC | BI8_GEMM_FORCE_GENERIC)) && g.K > 0;
-    // M <= 64: one pass over the weights on the tensor cores with exchanged operand roles (needs the workspace)
-    if (free_choice && gemm_skinny_applicable(g)) return then_residual(launch_gemm_skinny(g, st), g, st);
+    // M <= 64: one pass over the weights on the tensor cores with exchanged operand roles
+    if (free_choice && gemm_skinny_preferred(g)) return then_residual(launch_gemm_skinny(g, st), g, st);
     // otherwise M <= 8 streams the weights on the CUDA cores; 9..16 would stream them twice and is faster on the
     // general tensor-core kernel
     if (free_choice && g.M <= 8 && gemm_smallm_applicable(g)) return then_residual(launch_gemm_smallm(g, st), g, st);
@@ -99,6 +99,47 @@ int dispatch_gemm(const GemmArgs& g, cudaStream_t st) {
     }
     if ((g.flags & BI8_GEMM_FORCE_GENERIC) || !tc_ok || g.K == 0) return then_residual(launch_gemm_generic(g, st), g, st);
     return launch_gemm_tc(g, st);
+}
+
+// Where a decode-sized layer quantizes its activations: inside the GEMM (one launch; every cluster repeats the work and the weights
+// wait for the predecessor) or in a kernel in front of it (weights and quantizer overlap).  Inside up to this many
+// activation values: measured on layers of a decode step, 3 x 2048: 37 us a layer against 47, 1 x 4096: 61 against 65, but 8 x
+// 4096: 78 against 71 and 16 x 2560: 54 against 49.  A plain call by itself is bound by its launches and always
+// gains up to 16 rows (16 x 4096 -> 4096: 9.8 us against 11.5).
+constexpr int64_t kQuantInKernelValues = 16384;
+constexpr int64_t kQuantInKernelRows = 16;
+
+// Decode-sized layer (the weight-streaming GEMM and what produces its activations).  `g` describes the GEMM on the
+// quantized activations g.A / g.sA, which are scratch (null: none); `alone`: a plain call, not a step with a producer or a
+// residual around it.  Sets *done to false, having launched nothing, where
+// that kernel does not take the shape.
+int launch_decode(GemmArgs g, bool alone, int op, const void* x, const void* x2, const void* norm_weight, int x_dtype, int64_t ldx, float eps, bool* done,
+                  cudaStream_t st) {
+    *done = true;
+    GemmArgs in = g;
+    in.X = x;
+    in.x_dtype = x_dtype;
+    in.ldx = ldx;
+    in.pre_op = op;
+    in.X2 = op == BI8_PRE_SILU_MUL ? x2 : op == BI8_PRE_RMSNORM ? norm_weight : nullptr;
+    in.eps = eps;
+    const bool scratch = g.A != nullptr && g.sA != nullptr;
+    const bool want_in = (g.M <= kQuantInKernelRows && (alone || g.M * g.K <= kQuantInKernelValues)) || (g.flags & BI8_GEMM_QUANT_IN_KERNEL) || !scratch;
+    if (want_in && !(op == BI8_PRE_SILU_MUL && !x2) && gemm_skinny_applicable(in)) return launch_gemm_skinny(in, st);
+    if (!scratch || g.K % 16 != 0 || !aligned(g.A, 16) || !gemm_skinny_preferred(g)) {
+        *done = false;
+        return BI8_OK;
+    }
+    // a quantizer in front; none of this library's writes weights, so the GEMM's set-up and first weight copies overlap it, and
+    // it waits for the quantizer's completion before it reads the activations
+    const bool vec = aligned(x, 16) && (ldx * dtype_size(x_dtype)) % 16 == 0 && g.K % 8 == 0;    // 8 elements per load
+    int8_t* xq = const_cast<int8_t*>(g.A);
+    float* sx = const_cast<float*>(g.sA);
+    const int rc = op == BI8_PRE_NONE && vec ? launch_skinny_quantize(x, x_dtype, ldx, xq, sx, g.M, g.K, g.block, st)
+                                             : launch_quantize_pre(op, x, x2, x_dtype, ldx, norm_weight, eps, xq, g.K, sx, g.M, g.K, g.block, st);
+    if (rc != BI8_OK) return rc;
+    g.after_own_quantizer = true;
+    return launch_gemm_skinny(g, st);
 }
 
 }  // namespace
@@ -219,8 +260,7 @@ size_t bi8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int block) {
     g.N = N;
     g.K = K;
     g.block = block;
-    const size_t a = gemm_tc_workspace_bytes(g), b = gemm_skinny_workspace_bytes(g);
-    return a > b ? a : b;
+    return gemm_tc_workspace_bytes(g);
 }
 
 int bi8_gemm_dequant(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb, const float* sA, const float* sB,
@@ -257,36 +297,14 @@ int bi8_gemm_dequant_fused_quant(const void* x, int x_dtype, int64_t ldx, int8_t
                                  const float* sW, const void* bias, int bias_dtype, void* C, int64_t ldc, int out_dtype,
                                  int64_t M, int64_t N, int64_t K, int block, void* workspace, size_t workspace_bytes, int flags,
                                  void* stream) {
-    // Decode-sized M: the skinny tensor-core GEMM.  Default: a small quantizer kernel, then the GEMM launched so that its
-    // set-up and first weight copies overlap the quantizer (programmatic dependent launch).  With BI8_GEMM_QUANT_IN_KERNEL,
-    // or without scratch, the GEMM kernel quantizes the activations itself as it loads its stages (one kernel, slower).
     if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "gemm_dequant_fused_quant: unknown dtype code %d", x_dtype);
     const bool forced = (flags & (BI8_GEMM_FORCE_GENERIC | BI8_GEMM_FORCE_TC | BI8_GEMM_FORCE_SMALLM)) != 0;
-    if (!forced && x && M > 0 && N > 0 && K > 0 && ldx >= K && aligned(x, dtype_size(x_dtype))) {
-        GemmArgs g{xq, K, Wq, ldw, sx, sW, bias, bias_dtype, C, ldc, out_dtype, nullptr, M, N, K, block, flags, workspace, workspace_bytes};
-        const bool x_vec = aligned(x, 16) && (ldx * dtype_size(x_dtype)) % 16 == 0 && K % 8 == 0;   // 8 elements per load
-        const bool chained = !(flags & BI8_GEMM_QUANT_IN_KERNEL) && x_vec && xq && sx && K % 16 == 0 && aligned(xq, 16) &&
-                             gemm_skinny_applicable(g);
-        bool in_kernel = false;
-        if (!chained) {
-            g.A = nullptr;
-            g.sA = nullptr;
-            g.X = x;
-            g.x_dtype = x_dtype;
-            g.ldx = ldx;
-            in_kernel = gemm_skinny_applicable(g);
-        }
-        if (chained || in_kernel) {
-            if (!Wq || !sW || !C) return fail(BI8_ERR_NULL, "gemm_dequant_fused_quant: null pointer");
-            if (ldw < K || ldc < N) return fail(BI8_ERR_SHAPE, "gemm_dequant_fused_quant: row pitch smaller than the row");
-            if (!dtype_ok(out_dtype) || (bias && !dtype_ok(bias_dtype))) return fail(BI8_ERR_DTYPE, "gemm_dequant_fused_quant: unknown dtype code");
-            if (!aligned(C, dtype_size(out_dtype))) return fail(BI8_ERR_ALIGN, "gemm_dequant_fused_quant: output not element aligned");
-            if (in_kernel) return launch_gemm_skinny(g, static_cast<cudaStream_t>(stream));
-            int rc = launch_skinny_quantize(x, x_dtype, ldx, xq, sx, M, K, block, static_cast<cudaStream_t>(stream));
-            if (rc != BI8_OK) return rc;
-            g.after_own_quantizer = true;
-            return launch_gemm_skinny(g, static_cast<cudaStream_t>(stream));
-        }
+    if (!forced && x && M > 0 && N > 0 && K > 0 && ldx >= K && aligned(x, dtype_size(x_dtype)) && Wq && sW && C && ldw >= K && ldc >= N &&
+        dtype_ok(out_dtype) && (!bias || dtype_ok(bias_dtype)) && aligned(C, dtype_size(out_dtype))) {
+        const GemmArgs g{xq, K, Wq, ldw, sx, sW, bias, bias_dtype, C, ldc, out_dtype, nullptr, M, N, K, block, flags, workspace, workspace_bytes};
+        bool done = false;
+        const int rc = launch_decode(g, true, BI8_PRE_NONE, x, nullptr, nullptr, x_dtype, ldx, 0.0f, &done, static_cast<cudaStream_t>(stream));
+        if (done) return rc;
     }
     // ... two kernels otherwise, through the caller's scratch
     if (M > 0 && K > 0 && (!xq || !sx))
@@ -326,7 +344,6 @@ int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtyp
     if (!dtype_ok(out_dtype)) return fail(BI8_ERR_DTYPE, "gemm_dequant_fused_pre: unknown output dtype code %d", out_dtype);
     if (residual && !aligned(residual, dtype_size(out_dtype))) return fail(BI8_ERR_ALIGN, "gemm_dequant_fused_pre: residual not element aligned");
     if (M == 0 || N == 0) return BI8_OK;
-    // C over the residual: only the decode path reads an element of the residual in the thread that then writes C
     const size_t osz = dtype_size(out_dtype);
     const char *c0 = static_cast<const char*>(C), *c1 = c0 + ((M - 1) * ldc + N) * osz;
     const char *r0 = static_cast<const char*>(residual), *r1 = residual ? r0 + ((M - 1) * ldr + N) * osz : r0;
@@ -338,33 +355,32 @@ int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtyp
                                             workspace, workspace_bytes, flags, stream);
     // the decode path: this op's quantizer in the decode quantizer's place, the GEMM overlapped with it, the residual
     // added by the kernel that writes C (through the bias operand, which gets a row pitch)
-    const bool forced = (flags & (BI8_GEMM_FORCE_GENERIC | BI8_GEMM_FORCE_TC | BI8_GEMM_FORCE_SMALLM | BI8_GEMM_QUANT_IN_KERNEL)) != 0;
+    const bool forced = (flags & (BI8_GEMM_FORCE_GENERIC | BI8_GEMM_FORCE_TC | BI8_GEMM_FORCE_SMALLM)) != 0;
     GemmArgs g{xq, K, Wq, ldw, sx, sW, bias, bias_dtype, C, ldc, out_dtype, nullptr, M, N, K, block, flags, workspace, workspace_bytes};
-    if (!forced && K > 0 && K % 16 == 0 && aligned(xq, 16) && gemm_skinny_applicable(g)) {
+    const bool x_ok = x && dtype_ok(x_dtype) && ldx >= K && aligned(x, dtype_size(x_dtype)) && (op != BI8_PRE_SILU_MUL || (x2 && aligned(x2, dtype_size(x_dtype)))) &&
+                      (!norm_weight || aligned(norm_weight, dtype_size(x_dtype))) && (op == BI8_PRE_NONE || op == BI8_PRE_RMSNORM || op == BI8_PRE_SILU_MUL);
+    const bool in_kernel_residual = residual && !bias;
+    if (!forced && K > 0 && x_ok && !(overlap && !in_kernel_residual)) {
         int rc = check_gemm(g, false);
         if (rc != BI8_OK) return rc;
-        const bool in_kernel_residual = residual && !bias;
-        if (overlap && !in_kernel_residual)
-            return fail(BI8_ERR_ALIGN, "gemm_dequant_fused_pre: C may be the residual itself only without bias");
         if (in_kernel_residual) {
             g.bias = residual;
             g.bias_dtype = out_dtype;
             g.bias_ld = ldr;
         }
-        const bool x_vec = dtype_ok(x_dtype) && x && aligned(x, 16) && (ldx * dtype_size(x_dtype)) % 16 == 0 && K % 8 == 0 && ldx >= K;
-        if (op == BI8_PRE_NONE && x_vec) rc = launch_skinny_quantize(x, x_dtype, ldx, xq, sx, M, K, block, st);
-        else rc = bi8_quantize_rowwise_pre(op, x, x2, x_dtype, ldx, norm_weight, eps, xq, sx, M, K, block, stream);
-        if (rc != BI8_OK) return rc;
-        // every quantizer of this library may be overlapped with the GEMM's set-up and first weight copies: none of them
-        // writes weights, and the GEMM waits for the quantizer's completion before it reads the activations
-        g.after_own_quantizer = true;
-        rc = launch_gemm_skinny(g, st);
-        if (rc != BI8_OK || !residual || in_kernel_residual) return rc;
-        return launch_residual_add(C, ldc, residual, ldr, out_dtype, M, N, st);
+        bool done = false;
+        rc = launch_decode(g, false, op, x, x2, norm_weight, x_dtype, ldx, eps, &done, st);
+        if (done) {
+            if (rc != BI8_OK || !residual || in_kernel_residual) return rc;
+            return launch_residual_add(C, ldc, residual, ldr, out_dtype, M, N, st);
+        }
+        g.bias_ld = 0;
     }
-    if (overlap)
-        return fail(BI8_ERR_ALIGN, "gemm_dequant_fused_pre: C may be the residual itself only on the decode path (M <= 64, N %% 4 == 0, "
-                                   "K %% 16 == 0, workspace given, no bias)");
+    // The general tensor-core kernel reads an element of the residual in the warp that then writes it, so C may be the residual.
+    const char* why = "";
+    if (overlap && ((flags & BI8_GEMM_FORCE_GENERIC) || bias || K == 0 || !gemm_tc_applicable(g, &why)))
+        return fail(BI8_ERR_ALIGN, "gemm_dequant_fused_pre: C may be the residual itself only for the tensor-core kernels, without bias");
+    if (overlap) flags |= BI8_GEMM_FORCE_TC;
     int rc = bi8_quantize_rowwise_pre(op, x, x2, x_dtype, ldx, norm_weight, eps, xq, sx, M, K, block, stream);
     if (rc != BI8_OK) return rc;
     g.flags = flags & ~BI8_GEMM_QUANT_IN_KERNEL;

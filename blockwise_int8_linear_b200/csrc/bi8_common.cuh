@@ -133,9 +133,12 @@ struct GemmArgs {
     int flags;
     void* workspace;          // optional scratch for split-K partial results
     size_t workspace_bytes;
-    const void* X = nullptr;  // non-null: activations before quantization (A and sA unused), quantized on load
+    const void* X = nullptr;  // decode kernel, non-null: activations before quantization (A and sA unused), quantized inside it
     int x_dtype = 0;
     int64_t ldx = 0;
+    int pre_op = BI8_PRE_NONE;          // ... with this step in front: X2 is the second operand of SiLU * mul (same pitch) or the RMSNorm weight
+    const void* X2 = nullptr;
+    float eps = 0.0f;
     bool after_own_quantizer = false;   // the kernel launched just before is this library's decode quantizer
     unsigned wait_limit_us = 0;         // diagnostic: limit of the general kernel's bounded waits (0 = default, about 2 s)
     int skip_stage = -1;                // diagnostic: the general kernel's producer leaves this stage of its first item out
@@ -149,8 +152,9 @@ bool gemm_tc_applicable(const GemmArgs& g, const char** why);
 size_t gemm_tc_workspace_bytes(const GemmArgs& g);
 int launch_gemm_tc(const GemmArgs& g, cudaStream_t st);
 int launch_gemm_generic(const GemmArgs& g, cudaStream_t st);
+double gemm_tc_estimate_us(const GemmArgs& g);       // few tiles: the time the general kernel takes, for a choice between kernels
 bool gemm_skinny_applicable(const GemmArgs& g);
-size_t gemm_skinny_workspace_bytes(const GemmArgs& g);
+bool gemm_skinny_preferred(const GemmArgs& g);
 int launch_gemm_skinny(const GemmArgs& g, cudaStream_t st);
 int launch_skinny_quantize(const void* x, int x_dtype, int64_t ldx, int8_t* q, float* sx, int64_t M, int64_t K, int block,
                            cudaStream_t st);

@@ -991,6 +991,13 @@ size_t gemm_tc_workspace_bytes(const GemmArgs& g) {
     return plan_split(g.M, g.N, g.K, di.sms).bytes;
 }
 
+double gemm_tc_estimate_us(const GemmArgs& g) {
+    const DeviceInfo di = device_info();
+    const SplitPlan pl = plan_split(g.M, g.N, g.K, di.sms);
+    const int64_t tiles = ((g.M + kBM - 1) / kBM) * ((g.N + tc_bn() - 1) / tc_bn()), items = tiles * pl.ksplit;
+    return 0.8 * (double)((items + di.sms - 1) / di.sms * pl.stages_per_split) + (pl.ksplit > 1 ? 10.0 : 3.0);
+}
+
 bool gemm_tc_applicable(const GemmArgs& g, const char** why) {
     auto no = [&](const char* w) {
         if (why) *why = w;

@@ -3,31 +3,32 @@
 //
 // Same contract as the reference kernel at triton_functions.py:69-139 (path inside the reference project).  With so few
 // rows of A the work is one pass over the weights Bt[N, K]: the kernel is bound by streaming them from HBM, and is
-// organised around that stream.
+// organised around that stream and around the fixed cost of a call, which is as long as the stream itself for a 4096 x 4096
+// matrix.
 //   * The weights are the M operand of the MMA: a tile is 128 weight rows, the activations (padded to 16, 32 or 64
-//     rows by the TMA's zero fill) are the N operand, so one tcgen05.mma kind::i8 (M128 N16..64 K32) covers 128 weight
-//     rows and every activation row, and the s32 accumulator of a quantisation block is only 16..64 tensor-memory columns.
-//   * All (tile, K stage) pairs form one sequence that is cut into equal contiguous ranges, one per CTA and one CTA
-//     per SM, so every SM streams the same number of bytes whatever N and K are.  A range may begin or end inside a
-//     tile: such a part of a tile goes to an fp32 workspace slot (at most two per CTA) and a second kernel adds the
-//     slots of a tile in ascending K order; tiles that lie completely inside one range are written directly.  That
-//     kernel is launched with programmatic stream serialisation: it becomes resident while this one runs and
-//     griddepcontrol.wait releases it when this grid has completed.  (Adding the parts inside the GEMM, by whichever
-//     CTA finishes a tile last, was measured slower than the second launch: the fence, the arrival count and the
-//     read-back are three dependent trips to L2 at the end of every CTA.)
+//     rows) are the N operand, so one tcgen05.mma kind::i8 (M128 N16..64 K32) covers 128 weight rows and every
+//     activation row, and the s32 accumulator of a quantisation block is only 16..64 tensor-memory columns.
+//   * Clusters of 1, 2, 4 or 8 CTAs work on a tile together, each on its share of K (split_plan: whatever lets the
+//     most SMs stream for the fewest stages), one CTA per SM; clusters walk over the tiles.  The partial sums of
+//     a tile meet in shared memory of the cluster: quarter q of the tile's rows is finished by CTA q mod cluster size,
+//     the others send theirs with st.async, which counts its bytes on the receiver's mbarrier, and the receiver
+//     adds them in ascending K order.  One kernel, no workspace, and the exchange costs about half a microsecond.  (Equal
+//     ranges of a stream-K sequence with a second kernel for the sums keep all 148 SMs streaming but need a
+//     launch more, 2.3 us of host time; sums inside the kernel through L2, by flags or by self-describing pieces, cost
+//     2 us of device time per call: a store, a poll and the cold code are one L2 trip each.)
+//   * Activations either arrive quantized (SRC 0) or are quantized by the kernel itself (SRC 1, M <= 32): every CTA takes the
+//     rows' share of K that its own stages need (with the RMSNorm or SiLU * mul step in front, if asked for) and leaves it in
+//     shared memory as the MMA's swizzled operand tiles, while the first weights are on their way.  That is one launch
+//     and one kernel boundary less per layer; the redundancy (every cluster quantizes the same rows) is hidden behind
+//     the weights' first arrival.  From 33 rows on it would not be: those come from skinny_quantize_kernel or one of
+//     the producer quantizers, launched in front so that this kernel's set-up and first weight copies overlap them.
 //   * Warp roles: promotion warps (four per 16 activation rows, or per 32 for 64 rows; one per tensor-memory lane
-//     quarter) convert and scale;
-//     one producer warp issues, per stage, three TMA copies that complete on one barrier: 128 weight rows x 128
-//     K-bytes, the activation rows of the same K range, and the stage's weight scales (a [blocks, 128] fp32 box of
-//     sB); two MMA issuer warps take the stages in turn (one accumulator range per quantisation block, one commit per
-//     stage).
-//   * With FUSED the activations arrive as bf16/fp16/fp32 and four more warps quantize, per stage, the 128 K-columns of
-//     every activation row into the stage's operand tile (same arithmetic as the standalone quantizer, written in the
-//     128-byte swizzle the MMA expects) and their block scales into the scale table: quantize-on-load in one kernel.
-//     It is the slower of the two quantize-on-load forms; the default one is skinny_quantize_kernel in front of this
-//     kernel, overlapped with its start (see the launch code at the end of the file).
+//     quarter) convert and scale; one producer warp issues, per stage, the TMA copies that complete on one
+//     barrier: 128 weight rows x 128 K-bytes, the stage's weight scales (a [blocks, 128] fp32 box of sB) and, with SRC 0,
+//     the activation rows of the same K range; two MMA issuer warps take the stages in turn (one accumulator range per
+//     quantisation block, one commit per stage); with SRC 1 five more warps help to quantize.
 //   * Promotion follows the reference's order term by term, sB*(sA*(float(P)*fl32(1/127^2))), added in ascending block
-//     order within a range, so a tile that is not divided is bit-identical to the CUDA-core kernel.
+//     order within a CTA's share of K, so a tile that is not divided is bit-identical to the CUDA-core kernel.
 #include "quant_math.cuh"
 #include "tc_common.cuh"
 #include "peer_common.cuh"
@@ -43,6 +44,7 @@ constexpr int kTileRows = 128;    // weight rows per tile (the MMA's M)
 constexpr int kSkMaxM = 64;       // beyond 64 activation rows the promotion (5 instructions per element and block, in the
                                   // reference's order) costs more than the weights take to arrive: measured slower than
                                   // the general kernel at 128 rows
+constexpr int kMostCluster = 8;   // the portable limit
 
 constexpr int pow2_at_least(int x) {
     int p = 32;
@@ -50,135 +52,376 @@ constexpr int pow2_at_least(int x) {
     return p;
 }
 
-constexpr int kQuantWarps = 4;    // FUSED: warps that quantize the activations of a stage
-constexpr int kMmaWarps = 2;      // MMA issuers, taking the stages in turn
+constexpr int kHelpWarps = 5;     // SRC 1: warps that only quantize (512 threads: 128 registers each)
 
-template <int QB, int BNS, bool FUSED = false>
+template <int QB, int BNS, int SRC>
 struct SkGeo {
-    // ring depth: the loop producer -> HBM -> MMA -> promotion -> producer takes a few thousand cycles per slot, and a
-    // stage should be re-issued every ~700 to keep up with HBM
-    static constexpr int STAGES = BNS == 16 ? 8 : 6;
-    static constexpr int BPS = kBK / QB;                  // quantisation blocks per stage
+    // A stage is SUB operand tiles of 128 K-bytes: what a stage costs beside its bytes (barrier hand-overs, a commit, the
+    // tensor-memory round trip) is about 400 cycles per role, as long as 128 x 128 bytes take to arrive.
+    static constexpr int SUB = BNS <= 32 ? 2 : 1;
+    static constexpr int KS = SUB * kBK;                  // K bytes of a stage
+    static constexpr int STAGES = BNS == 16 ? (SRC == 0 ? 5 : 4) : BNS == 32 ? (SRC == 0 ? 4 : 3) : 5;
+    static constexpr int BPS = KS / QB;                   // quantisation blocks per stage
     static constexpr int MMAS = QB / 32;                  // MMAs (K = 32) per block
-    static constexpr int CW = BNS <= 32 ? 16 : 32;        // activation rows (accumulator columns) per promotion warp
+    static constexpr int CW = BNS / 2;                    // activation rows (accumulator columns) per promotion warp
     static constexpr int CHUNKS = BNS / CW;
     static constexpr int PROMO_WARPS = 4 * CHUNKS;
-    static constexpr int VB = CW == 16 ? BPS : 1;         // blocks whose accumulators a promotion thread loads at once
-    static constexpr int THREADS = (PROMO_WARPS + 1 + kMmaWarps + (FUSED ? kQuantWarps : 0)) * 32;
+    static constexpr int VB = BPS * CW <= 32 ? BPS : 32 / CW;      // blocks whose accumulators a promotion thread loads at once
     static constexpr int ACC_STRIDE = BPS * BNS;          // tensor-memory columns of one stage's accumulators
     static constexpr int NBUF = (512 / ACC_STRIDE) < 4 ? (512 / ACC_STRIDE) : 4;
+    static constexpr int MMA_WARPS = 2;                   // MMA issuers, taking the stages in turn
+    static constexpr int THREADS = (PROMO_WARPS + 1 + MMA_WARPS + (SRC != 0 ? kHelpWarps : 0)) * 32;
     static constexpr int TMEM_COLS = pow2_at_least(NBUF * ACC_STRIDE);
-    static constexpr uint32_t W_BYTES = kTileRows * kBK;
-    static constexpr uint32_t X_BYTES = BNS * kBK;
+    static constexpr uint32_t W_BYTES = SUB * kTileRows * kBK;
+    static constexpr uint32_t XT_BYTES = BNS * kBK;                       // one operand tile of activations (128 K-bytes)
+    static constexpr uint32_t X_BYTES = SRC == 0 ? SUB * XT_BYTES : 0;    // ... inside a stage
     static constexpr uint32_t S_TX = BPS * kTileRows * 4;                 // bytes the scale copy delivers
     static constexpr uint32_t S_BYTES = S_TX < 1024 ? 1024 : S_TX;        // keeps every stage 1024-byte aligned
     static constexpr uint32_t STAGE_BYTES = W_BYTES + X_BYTES + S_BYTES;
     static constexpr uint32_t bar_off = STAGES * STAGE_BYTES;
+    static_assert(NBUF % MMA_WARPS == 0 && VB >= 1 && BPS % VB == 0, "every issuer keeps its own accumulators; whole groups of blocks");
     static constexpr int FULL_AB = 0, EMPTY_AB = STAGES, ACC_FULL = 2 * STAGES, ACC_EMPTY = 2 * STAGES + NBUF,
-                         NBARS = 2 * STAGES + 2 * NBUF;
+                         RX_FULL = 2 * STAGES + 2 * NBUF,                 // [2 buffers][promotion warps]: parts have arrived
+                         RX_FREE = RX_FULL + 2 * PROMO_WARPS,             // [2 buffers][promotion warps]: the receiver is done with ours
+                         NBARS = RX_FREE + 2 * PROMO_WARPS;
     static constexpr uint32_t misc_off = bar_off + NBARS * 8;             // tmem holder, abort flag, never-raised flag
-    static constexpr uint32_t sx_off = (misc_off + 32 + 15) & ~15u;       // activation scales [nb][BNS]
+    static constexpr uint32_t norm_off = (misc_off + 32 + 15) & ~15u;     // SRC 1, RMSNorm: sums of squares [BNS][8]
+    static constexpr uint32_t rx_off = norm_off + (SRC != 0 ? BNS * 8 * 4 : 0);   // received parts, see rx_bytes()
 };
-
-// dynamic shared memory of a launch: stage ring, barriers, activation scales [nb][BNS], alignment slack
-template <int QB, int BNS, bool FUSED>
-constexpr size_t smem_of(int nb) {
-    return (size_t)SkGeo<QB, BNS, FUSED>::sx_off + (size_t)nb * BNS * 4 + 1024;
-}
 
 struct SkParams {
     const float* sA;
-    const void* X;          // FUSED: activations before quantization, row pitch ldx elements
+    const void* X;          // SRC 1: activations before quantization, row pitch ldx elements
+    const void* X2;         // SRC 1: second operand of SiLU * mul (same pitch), or the RMSNorm weight, or null
     int64_t ldx;
-    int x_dtype;
+    float eps;
+    int x_dtype, op;
     const void* bias;
     int64_t bias_ld;        // row pitch of `bias` in elements: 0 = one row for all (a bias), else an [M, N] addend (a residual)
     void* C;
-    float* ws;
     int* status;
     int64_t ldc;
-    long long total_stages;
-    int M, N, K, nb, nks;
+    int M, N, K, nb, nks, tiles;
     int out_dtype, bias_dtype;
     int live_chunks;    // groups of CW activation rows that hold a valid row
     int early_weights;  // the weight copies of the first stages may be issued before the preceding kernel has completed
+    int rx_bufs;        // receive buffers: 2 where a cluster has more than one tile
+    int share;          // most stages of a CTA
+    uint32_t sx_off, xq_off;    // activation scales [share * BPS][BNS]; SRC 1: operand tiles [share * SUB][BNS x 128 bytes]
 };
 
-// first (tile, stage) pair of CTA c when `total` pairs are divided over `ctas` CTAs
-__host__ __device__ __forceinline__ long long range_start(long long c, long long total, long long ctas) { return c * total / ctas; }
+// Bytes of one receive buffer: for every quarter this CTA finishes and every CTA of the cluster, 32 rows x BNS sums.
+__host__ __device__ constexpr uint32_t rx_bytes(int bns, int cluster) {
+    return (uint32_t)(cluster == 1 ? 0 : cluster * (cluster < 4 ? 4 / cluster : 1) * 32 * bns * 4);
+}
 
-// C[m, n] = cast(acc) (+ cast(bias[m * bias_ld + n]) in the output type: reference lines 125-131)
-__device__ __forceinline__ void finish_store(float acc, int m, int n, const void* bias, int bias_dtype, int64_t bias_ld, void* C,
-                                             int64_t ldc, int out_dtype) {
-    float bv = 0.0f;
-    const bool hb = bias != nullptr;
-    if (hb) {
-        const int64_t bi = (int64_t)m * bias_ld + n;
-        if (bias_dtype == BI8_BF16) bv = __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[bi]);
-        else if (bias_dtype == BI8_F16) bv = __half2float(static_cast<const __half*>(bias)[bi]);
-        else bv = static_cast<const float*>(bias)[bi];
+// dynamic shared memory of a launch, and where its run-time sized parts begin
+template <int QB, int BNS, int SRC>
+size_t smem_of(int share, int cluster, int rx_bufs, uint32_t* sx_off = nullptr, uint32_t* xq_off = nullptr) {
+    using G = SkGeo<QB, BNS, SRC>;
+    const uint32_t sx = G::rx_off + (uint32_t)rx_bufs * rx_bytes(BNS, cluster);
+    uint32_t end = sx + (uint32_t)(share * G::BPS * BNS * 4);
+    if (sx_off) *sx_off = sx;
+    if (SRC != 0) {
+        end = (end + 1023u) & ~1023u;
+        if (xq_off) *xq_off = end;
+        end += (uint32_t)(share * G::SUB) * G::XT_BYTES;
     }
-    const int64_t o = (int64_t)m * ldc + n;
-    if (out_dtype == BI8_F32) {
-        static_cast<float*>(C)[o] = hb ? __fadd_rn(acc, bv) : acc;
-    } else if (out_dtype == BI8_BF16) {
-        __nv_bfloat16 c = __float2bfloat16_rn(acc);
-        if (hb) c = __float2bfloat16_rn(__fadd_rn(__bfloat162float(c), __bfloat162float(__float2bfloat16_rn(bv))));
-        static_cast<__nv_bfloat16*>(C)[o] = c;
-    } else {
-        __half c = __float2half_rn(acc);
-        if (hb) c = __float2half_rn(__fadd_rn(__half2float(c), __half2float(__float2half_rn(bv))));
-        static_cast<__half*>(C)[o] = c;
+    return (size_t)end + 1024;                            // alignment slack
+}
+
+// ---- cluster helpers ----------------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t map_to(uint32_t smem_addr, uint32_t rank) {     // the same place in another CTA of the cluster
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void remote_arrive(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+// 16 bytes into another CTA's shared memory, counted there on `cluster_bar`
+__device__ __forceinline__ void send_v4(uint32_t cluster_addr, uint32_t cluster_bar, float a, float b, float c, float d) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%2, %3, %4, %5}, [%1];" ::"r"(cluster_addr),
+                 "r"(cluster_bar), "f"(a), "f"(b), "f"(c), "f"(d)
+                 : "memory");
+}
+// mbar_wait for data that another CTA of the cluster has sent
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t abort_flag) {
+    const long long t0 = clock64();
+    while (true) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok != 0u) return true;
+        if (lds_volatile_u32(abort_flag) != 0u || clock64() - t0 > 4000000000ll) return false;
     }
 }
 
-template <int QB, int BNS, bool FUSED>
-__global__ void __launch_bounds__(SkGeo<QB, BNS, FUSED>::THREADS, 1)
+// ---- output -------------------------------------------------------------------------------------------------------------
+// C[m, n] = cast(acc) (+ cast(addend) in the output type: reference lines 125-131) for the CW rows of a chunk and one column n; the
+// addend is bias[n] (bias_ld 0) or an [M, N] residual.  All addends are requested before the first is used.
+template <typename T>
+__device__ __forceinline__ T round_as(float v);
+template <>
+__device__ __forceinline__ __nv_bfloat16 round_as<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+template <>
+__device__ __forceinline__ __half round_as<__half>(float v) { return __float2half_rn(v); }
+template <>
+__device__ __forceinline__ float round_as<float>(float v) { return v; }
+__device__ __forceinline__ float widen(__nv_bfloat16 v) { return __bfloat162float(v); }
+__device__ __forceinline__ float widen(__half v) { return __half2float(v); }
+__device__ __forceinline__ float widen(float v) { return v; }
+
+template <typename T>
+__device__ __forceinline__ void finish_rows(const float* acc, const float (&add)[8], bool has_add, int live, T* c, int64_t ldc) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (i >= live) break;
+        T v = round_as<T>(acc[i]);
+        if (has_add) v = round_as<T>(__fadd_rn(widen(v), widen(round_as<T>(add[i]))));
+        c[(int64_t)i * ldc] = v;
+    }
+}
+
+template <int CW>
+__device__ __forceinline__ void finish_chunk(const float (&acc)[CW], const SkParams& p, int m0, int n) {
+#pragma unroll
+    for (int g = 0; g < CW; g += 8) {
+        const int m = m0 + g, live = p.M - m < 8 ? p.M - m : 8;
+        if (live <= 0) break;
+        float add[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) add[i] = 0.0f;
+        const bool has_add = p.bias != nullptr;
+        if (has_add) {
+            const int64_t b0 = (int64_t)m * p.bias_ld + n;
+            if (p.bias_dtype == BI8_F32) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (i < live) add[i] = static_cast<const float*>(p.bias)[b0 + i * p.bias_ld];
+            } else {
+                unsigned short h[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) h[i] = i < live ? static_cast<const unsigned short*>(p.bias)[b0 + i * p.bias_ld] : (unsigned short)0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) add[i] = p.bias_dtype == BI8_BF16 ? bf16lo(h[i]) : __half2float(__ushort_as_half(h[i]));
+            }
+        }
+        const int64_t o = (int64_t)m * p.ldc + n;
+        if (p.out_dtype == BI8_BF16) finish_rows(acc + g, add, has_add, live, static_cast<__nv_bfloat16*>(p.C) + o, p.ldc);
+        else if (p.out_dtype == BI8_F16) finish_rows(acc + g, add, has_add, live, static_cast<__half*>(p.C) + o, p.ldc);
+        else finish_rows(acc + g, add, has_add, live, static_cast<float*>(p.C) + o, p.ldc);
+    }
+}
+
+// ---- quantization inside the kernel (SRC 1) ------------------------------------------------------------------------------
+// eight consecutive elements of a 16-byte aligned row: request, and conversion of what has arrived
+struct Raw8 {
+    uint4 a, b;           // b: the second half of eight fp32 values
+};
+__device__ __forceinline__ Raw8 request_x8(const void* base, int64_t index, int dt) {
+    Raw8 r;
+    if (dt == BI8_F32) {
+        const float* src = static_cast<const float*>(base) + index;
+        r.a = ld_nc_v4(src);
+        r.b = ld_nc_v4(src + 4);
+    } else {
+        r.a = ld_nc_v4(static_cast<const unsigned short*>(base) + index);
+        r.b = make_uint4(0u, 0u, 0u, 0u);
+    }
+    return r;
+}
+__device__ __forceinline__ void convert_x8(float (&f)[8], const Raw8& r, int dt) {
+    if (dt == BI8_F32) {
+        f[0] = __uint_as_float(r.a.x); f[1] = __uint_as_float(r.a.y); f[2] = __uint_as_float(r.a.z); f[3] = __uint_as_float(r.a.w);
+        f[4] = __uint_as_float(r.b.x); f[5] = __uint_as_float(r.b.y); f[6] = __uint_as_float(r.b.z); f[7] = __uint_as_float(r.b.w);
+    } else {
+        const uint32_t w4[4] = {r.a.x, r.a.y, r.a.z, r.a.w};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            if (dt == BI8_BF16) {
+                f[2 * h] = bf16lo(w4[h]);
+                f[2 * h + 1] = bf16hi(w4[h]);
+            } else {
+                const float2 t2 = __half22float2(*reinterpret_cast<const __half2*>(&w4[h]));
+                f[2 * h] = t2.x;
+                f[2 * h + 1] = t2.y;
+            }
+        }
+    }
+}
+
+// The activations' share [k0, k1) of 128-byte K steps, by `warps` whole warps (this one is `me`): producer step, block scales into
+// sx [block][BNS], int8 values into the MMA's operand tiles (128-byte swizzle: the 16-byte chunk index is xor-ed with the row
+// index mod 8) at shared address xq.  Values, scales and the order of RMSNorm's sum are those of the stand-alone quantizers
+// (quantize_pre.cu at 256 threads per row).  Elements from K on are not written: the weights' zero fill meets them.
+// All loads of a batch are requested before the first is used: the whole step is a few trips to L2, in front of which the
+// weights wait.
+template <int QB, int BNS>
+__device__ __forceinline__ void quantize_share(const SkParams& p, int k0, int k1, int me, int warps, int lane, float* norm, float* sx, uint32_t xq) {
+    constexpr int LPB = QB / 8;
+    const int dt = p.x_dtype;
+    if (p.op == BI8_PRE_RMSNORM) {
+        // sums of squares of whole rows: 256 virtual threads per row, a warp plays 32 of them at a time, four times at once
+        constexpr int TASKS = 4;
+        const int tasks = p.M * 8, steps = (p.K + 2047) / 2048;
+        for (int t0 = me; t0 < tasks; t0 += warps * TASKS) {
+            float ss[TASKS] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int i = 0; i < steps; ++i) {
+                Raw8 r[TASKS];
+#pragma unroll
+                for (int q = 0; q < TASKS; ++q) {
+                    const int t = t0 + q * warps, k = i * 2048 + ((t & 7) * 32 + lane) * 8;
+                    r[q].a = r[q].b = make_uint4(0u, 0u, 0u, 0u);
+                    if (t < tasks && k < p.K) r[q] = request_x8(p.X, (int64_t)(t >> 3) * p.ldx + k, dt);
+                }
+#pragma unroll
+                for (int q = 0; q < TASKS; ++q) {
+                    float f[8];
+                    convert_x8(f, r[q], dt);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) ss[q] = __fmaf_rn(f[e], f[e], ss[q]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < TASKS; ++q) {
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) ss[q] += __shfl_xor_sync(0xffffffffu, ss[q], off);
+                if (lane == 0 && t0 + q * warps < tasks) norm[t0 + q * warps] = ss[q];
+            }
+        }
+        asm volatile("bar.sync 3, %0;" ::"r"(warps * 32) : "memory");
+    }
+    const int upr = (k1 - k0) * (kBK / 8);                 // units of eight elements per row
+    const int units = p.M * upr;
+    constexpr int BATCH = 4;
+    for (int u0 = me * 32; u0 < units; u0 += warps * 32 * BATCH) {     // upr is a multiple of 16: a block's lanes stay together
+        Raw8 rx[BATCH], r2[BATCH];
+#pragma unroll
+        for (int q = 0; q < BATCH; ++q) {
+            const int u = u0 + q * warps * 32 + lane, m = u / upr, k = k0 * kBK + (u - m * upr) * 8;
+            rx[q].a = rx[q].b = r2[q].a = r2[q].b = make_uint4(0u, 0u, 0u, 0u);
+            if (u < units && k < p.K) {
+                rx[q] = request_x8(p.X, (int64_t)m * p.ldx + k, dt);
+                if (p.op == BI8_PRE_SILU_MUL) r2[q] = request_x8(p.X2, (int64_t)m * p.ldx + k, dt);
+                else if (p.op == BI8_PRE_RMSNORM && p.X2 != nullptr) r2[q] = request_x8(p.X2, k, dt);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < BATCH; ++q) {
+            if (u0 + q * warps * 32 >= units) break;
+            const int u = u0 + q * warps * 32 + lane, m = u / upr, piece = u - m * upr, k = k0 * kBK + piece * 8;
+            const bool valid = u < units && k < p.K;
+            float f[8];
+            convert_x8(f, rx[q], dt);
+            if (p.op != BI8_PRE_NONE && valid) {
+                float v[8];
+                convert_x8(v, r2[q], dt);
+                if (p.op == BI8_PRE_SILU_MUL) {
+                    silu_mul8(f, v, dt);
+                } else {
+                    float total = 0.0f;
+#pragma unroll
+                    for (int w = 0; w < 8; ++w) total += norm[m * 8 + w];
+                    const float rstd = rsqrtf(__fadd_rn(__fdiv_rn(total, (float)p.K), p.eps));
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        float y = __fmul_rn(f[e], rstd);
+                        if (p.X2) y = __fmul_rn(y, v[e]);
+                        f[e] = round_to(y, dt);
+                    }
+                }
+            }
+            float amax = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
+#pragma unroll
+            for (int off = 1; off < LPB; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+            if (!valid) continue;
+            BlockQ bq;
+            bq.set(amax, dt != BI8_F32);
+            uint32_t lo, hi;
+            quantize8(f, bq, lo, hi);
+            const int tile = piece / (kBK / 8), c16 = piece % (kBK / 8);
+            const uint32_t dst = xq + (uint32_t)(tile * BNS * kBK + m * 128 + ((((c16 >> 1) ^ (m & 7)) << 4) | ((c16 & 1) << 3)));
+            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(dst), "r"(lo), "r"(hi) : "memory");
+            if ((piece % LPB) == 0) sx[(piece / LPB) * BNS + m] = amax;
+        }
+    }
+}
+
+template <int QB, int BNS, int SRC>
+__global__ void __launch_bounds__(SkGeo<QB, BNS, SRC>::THREADS, 1)
 gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                       const __grid_constant__ CUtensorMap tmS, const SkParams p) {
-    using G = SkGeo<QB, BNS, FUSED>;
+    using G = SkGeo<QB, BNS, SRC>;
+    constexpr int CW = G::CW;
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
     const uint32_t raw = smem_u32(smem_dyn);
-    const uint32_t base = (raw + 1023u) & ~1023u;      // the swizzle atom needs 1024-byte alignment
+    const uint32_t base = (raw + 1023u) & ~1023u;      // the swizzle atom needs 1024-byte alignment (the same in every CTA)
     unsigned char* base_ptr = smem_dyn + (base - raw);
     const uint32_t bars = base + G::bar_off;
     volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(base_ptr + G::misc_off);
     const uint32_t abort_flag = base + G::misc_off + 4;
     const uint32_t never_flag = base + G::misc_off + 8;
-    float* sx = reinterpret_cast<float*>(base_ptr + G::sx_off);
-    const uint32_t sx_u32 = base + G::sx_off;
+    float* sx = reinterpret_cast<float*>(base_ptr + p.sx_off);
+    const uint32_t sx_u32 = base + p.sx_off;
     auto bar = [&](int slot) -> uint32_t { return bars + 8u * (uint32_t)slot; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int live_warps = 4 * p.live_chunks;
-    constexpr int PW = G::PROMO_WARPS, MW = G::PROMO_WARPS + 1, QW0 = G::PROMO_WARPS + 1 + kMmaWarps;
-    static_assert(G::STAGES % kMmaWarps == 0 && G::NBUF % kMmaWarps == 0, "every issuer keeps its own stages and accumulators");
+    constexpr int PW = G::PROMO_WARPS, MW = G::PROMO_WARPS + 1;
 
-    const long long s_begin = range_start(blockIdx.x, p.total_stages, gridDim.x);
-    const long long s_end = range_start((long long)blockIdx.x + 1, p.total_stages, gridDim.x);
-    // position of the CTA's first stage; every role then steps (tile, ks) by itself, without a division per stage
-    const int tile_begin = (int)(s_begin / p.nks), ks_begin = (int)(s_begin - (long long)tile_begin * p.nks);
+    // this CTA's place: rank `rank` of `CL` in its cluster, K stages [k0, k1) of every tile; the cluster takes tiles
+    // first_tile, first_tile + tile_step, ...
+    const int CL = (int)cluster_size(), rank = (int)cluster_rank();
+    const int first_tile = (int)blockIdx.x / CL, tile_step = (int)gridDim.x / CL;
+    const int k0 = rank * p.nks / CL, k1 = (rank + 1) * p.nks / CL, len = k1 - k0;
+    const int rounds = first_tile < p.tiles ? (p.tiles - first_tile + tile_step - 1) / tile_step : 0;
+    const int my_stages = rounds * len;
 
+    auto issue_x = [&](int stage, int ks) {
+#pragma unroll
+        for (int u = 0; u < G::SUB; ++u)
+            tma_load_2d(base + (uint32_t)stage * G::STAGE_BYTES + G::W_BYTES + (uint32_t)u * G::XT_BYTES, &tmX, bar(G::FULL_AB + stage),
+                        ks * G::KS + u * kBK, 0);
+    };
     // one lane; `with_x` false leaves out the activation tile, whose copy then has to follow (issue_x)
     auto issue_stage = [&](int stage, int tile, int ks, bool with_x) {
         const uint32_t dst = base + (uint32_t)stage * G::STAGE_BYTES;
-        mbar_expect_tx(bar(G::FULL_AB + stage), G::W_BYTES + (FUSED ? 0u : G::X_BYTES) + G::S_TX);
-        tma_load_2d(dst, &tmW, bar(G::FULL_AB + stage), ks * kBK, tile * kTileRows);
-        if (!FUSED && with_x) tma_load_2d(dst + G::W_BYTES, &tmX, bar(G::FULL_AB + stage), ks * kBK, 0);
+        mbar_expect_tx(bar(G::FULL_AB + stage), G::W_BYTES + G::X_BYTES + G::S_TX);
+#pragma unroll
+        for (int u = 0; u < G::SUB; ++u)
+            tma_load_2d(dst + (uint32_t)(u * kTileRows * kBK), &tmW, bar(G::FULL_AB + stage), ks * G::KS + u * kBK, tile * kTileRows);
+        if (SRC == 0 && with_x) issue_x(stage, ks);
         tma_load_2d(dst + G::W_BYTES + G::X_BYTES, &tmS, bar(G::FULL_AB + stage), tile * kTileRows, ks * G::BPS);
-    };
-    auto issue_x = [&](int stage, int ks) {
-        tma_load_2d(base + (uint32_t)stage * G::STAGE_BYTES + G::W_BYTES, &tmX, bar(G::FULL_AB + stage), ks * kBK, 0);
     };
 
     // The producer warp sets the barriers up, tells the others (named barrier 2: it arrives, they wait, so it never stands
     // still) and starts the copies of the first stages right away: the ring is empty, nothing has to be waited for.  The
     // tensor-memory allocation runs beside it.
-    int pre_tile = tile_begin, pre_ks = ks_begin, pre_count = 0;
+    int pre_tile = first_tile, pre_ks = k0, pre_count = 0;
     if (warp == PW) {
         if (lane == 0) {
             for (int s = 0; s < G::STAGES; ++s) {
-                mbar_init(bar(G::FULL_AB + s), FUSED ? 1 + kQuantWarps : 1);   // the TMA's bytes (+ the quantizer warps)
+                mbar_init(bar(G::FULL_AB + s), 1);                             // the TMA's bytes
                 // a stage is free again when every promotion warp has seen its accumulator complete (so the MMAs have
                 // read the operands) and has taken its scales
                 mbar_init(bar(G::EMPTY_AB + s), live_warps);
@@ -187,6 +430,10 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
                 mbar_init(bar(G::ACC_FULL + b), 1);
                 mbar_init(bar(G::ACC_EMPTY + b), live_warps);
             }
+            for (int b = 0; b < 2 * PW; ++b) {
+                mbar_init(bar(G::RX_FULL + b), 1);
+                mbar_init(bar(G::RX_FREE + b), 1);
+            }
             sts_u32(abort_flag, 0u);
             sts_u32(never_flag, 0u);
             mbar_fence_init();
@@ -194,24 +441,25 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
         }
         __syncwarp();
         asm volatile("bar.arrive 2, %0;" ::"n"(G::THREADS) : "memory");
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the reduction kernel may be made resident
+        cluster_arrive();                                                      // barriers are set up: see the first send
         // The kernel is always launched so that it may start before its predecessor in the stream has completed.  Behind
         // this library's own activation quantizer the weights are known to be at rest and their copies start at once;
         // behind any other kernel (which may be the one writing the weights) nothing is read before the wait.
-        if (!p.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
-        while (pre_count < G::STAGES && s_begin + pre_count < s_end) {
+        if (!p.early_weights) after_predecessor();
+        else asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        while (pre_count < G::STAGES && pre_count < my_stages) {
             if (lane == 0) issue_stage(pre_count, pre_tile, pre_ks, false);
             ++pre_count;
-            if (++pre_ks == p.nks) { pre_ks = 0; ++pre_tile; }
+            if (++pre_ks == k1) { pre_ks = k0; pre_tile += tile_step; }
         }
         // Everything above touched only the weights and their scales.  The activations come from the kernel launched just
         // before this one (a quantizer that lets its dependents start early): wait for it here.
         if (p.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
-        if (!FUSED && lane == 0) {
-            int ks = ks_begin;
+        if (SRC == 0 && lane == 0) {
+            int ks = k0;
             for (int q = 0; q < pre_count; ++q) {
                 issue_x(q, ks);
-                if (++ks == p.nks) ks = 0;
+                if (++ks == k1) ks = k0;
             }
         }
         __syncwarp();
@@ -223,9 +471,21 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     if (warp != PW) {
         tc_fence_before();
         asm volatile("bar.sync 2, %0;" ::"n"(G::THREADS) : "memory");
+        cluster_arrive();
         tc_fence_after();
+        asm volatile("griddepcontrol.wait;" ::: "memory");      // activations, their scales, and every store, after the previous kernel
     }
     const uint32_t tmem_base = (warp != PW) ? *tmem_holder : 0u;       // the producer never touches tensor memory
+    bool cluster_ready = false;                                        // this thread has waited for the cluster's set-up
+
+    if (SRC != 0 && warp != PW) {
+        // every warp but the producer quantizes; the generic stores are handed to the tensor core's proxy before the barrier
+        constexpr int QWARPS = G::THREADS / 32 - 1;
+        quantize_share<QB, BNS>(p, k0 * G::SUB, k1 * G::SUB, warp < PW ? warp : warp - 1, QWARPS, lane, reinterpret_cast<float*>(base_ptr + G::norm_off), sx,
+                                base + p.xq_off);
+        fence_proxy_async_smem();
+        asm volatile("bar.sync 3, %0;" ::"n"(QWARPS * 32) : "memory");
+    }
 
     if (warp == PW) {
         // ---------------- TMA producer ----------------
@@ -236,7 +496,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
         for (int q = 0; q < G::STAGES; ++q) last_parity[q] = q < pre_count ? 0 : -1;
         int tile = pre_tile, ks = pre_ks;
         bool ok = true;
-        for (long long s = s_begin + pre_count; s < s_end; ++s) {
+        for (int s = pre_count; s < my_stages; ++s) {
             ok = __all_sync(0xffffffffu, mbar_wait(bar(G::EMPTY_AB + stage), phase ^ 1u, abort_flag));
             if (!ok) {
                 if (lane == 0) report_timeout(p.status, abort_flag, W_EMPTY_AB);
@@ -248,7 +508,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
             for (int q = 0; q < G::STAGES; ++q)
                 if (q == stage) last_parity[q] = (int)phase;
             if (++stage == G::STAGES) { stage = 0; phase ^= 1u; }
-            if (++ks == p.nks) { ks = 0; ++tile; }
+            if (++ks == k1) { ks = k0; tile += tile_step; }
         }
         if (!ok) {
             // do not leave while our own copies may still land in this CTA's shared memory
@@ -256,17 +516,18 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
             for (int q = 0; q < G::STAGES; ++q)
                 if (last_parity[q] >= 0) (void)mbar_wait(bar(G::FULL_AB + q), (uint32_t)last_parity[q], never_flag, 200000000ll);
         }
-    } else if (warp >= MW && warp < MW + kMmaWarps) {
+        __syncwarp();
+    } else if (warp >= MW && warp < MW + G::MMA_WARPS) {
         // ---------------- MMA issuers ----------------
-        // Issuing the four K = 32 MMAs of a stage and polling its two barriers costs one thread several hundred cycles, more
-        // than the stage's bytes take to arrive, so kMmaWarps warps take the stages in turn (stage ring slots and
-        // accumulator ranges of one residue class each).
+        // Issuing the MMAs of a stage, the commit and the polls of its two barriers cost one thread several hundred cycles, so
+        // MMA_WARPS warps take the stages in turn.
+        static_assert(G::MMA_WARPS <= G::STAGES, "an issuer advances by at most one turn of the stage ring");
         constexpr uint32_t idesc = umma_idesc_i8(kTileRows, BNS);
         const int me = warp - MW;
-        int stage = me, buf = me, ks = ks_begin + me;
-        while (ks >= p.nks) ks -= p.nks;
+        int buf = me, stage = me, ks = me;                   // ks: stage inside this CTA's share
+        while (len > 0 && ks >= len) ks -= len;
         uint32_t phase = 0, accphase = 0;
-        for (long long s = s_begin + me; s < s_end; s += kMmaWarps) {
+        for (int s = me; s < my_stages; s += G::MMA_WARPS) {
             // operands landed and an accumulator range is free: one vote for both
             const bool got_ab = mbar_wait(bar(G::FULL_AB + stage), phase, abort_flag);
             const bool got_acc = got_ab && mbar_wait(bar(G::ACC_EMPTY + buf), accphase ^ 1u, abort_flag);
@@ -278,15 +539,16 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
             if (lane == 0) {
                 const uint32_t st_base = base + (uint32_t)stage * G::STAGE_BYTES;
                 const uint64_t wdesc = umma_desc_k_sw128(st_base);
-                const uint64_t xdesc = umma_desc_k_sw128(st_base + G::W_BYTES);
+                const uint64_t xdesc = umma_desc_k_sw128(SRC == 0 ? st_base + G::W_BYTES : base + p.xq_off + (uint32_t)(ks * G::SUB) * G::XT_BYTES);
 #pragma unroll
                 for (int blk = 0; blk < G::BPS; ++blk) {
-                    if (ks * G::BPS + blk < p.nb) {
+                    if ((k0 + ks) * G::BPS + blk < p.nb) {
 #pragma unroll
                         for (int i = 0; i < G::MMAS; ++i) {
-                            const uint64_t koff = (uint64_t)((blk * G::MMAS + i) * 32 / 16);
-                            mma_i8(tmem_base + (uint32_t)(buf * G::ACC_STRIDE + blk * BNS), wdesc + koff, xdesc + koff, idesc,
-                                   i > 0 ? 1u : 0u);
+                            const int kb = (blk * G::MMAS + i) * 32, sub = kb / kBK;           // K byte inside the stage, operand tile
+                            const uint64_t koff = (uint64_t)(kb % kBK / 16);
+                            mma_i8(tmem_base + (uint32_t)(buf * G::ACC_STRIDE + blk * BNS), wdesc + koff + (uint64_t)(sub * kTileRows * kBK / 16),
+                                   xdesc + koff + (uint64_t)(sub * (int)G::XT_BYTES / 16), idesc, i > 0 ? 1u : 0u);
                         }
                     }
                 }
@@ -294,123 +556,31 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
                 tc_commit(bar(G::ACC_FULL + buf));
             }
             __syncwarp();
-            stage += kMmaWarps;
+            stage += G::MMA_WARPS;
             if (stage >= G::STAGES) { stage -= G::STAGES; phase ^= 1u; }
-            buf += kMmaWarps;
+            buf += G::MMA_WARPS;
             if (buf >= G::NBUF) { buf -= G::NBUF; accphase ^= 1u; }
-            ks += kMmaWarps;
-            while (ks >= p.nks) ks -= p.nks;
-        }
-    } else if (FUSED && warp >= QW0) {
-        // ---------------- quantize-on-load: the activations of a stage, straight into the MMA's operand tile -------------
-        // A unit is 8 consecutive K elements of one activation row; a stage holds 16 units per row.  Thread t of the 128
-        // takes units t, t + 128, ...: the units of one quantisation block sit in QB/8 neighbouring lanes, whose absmax is
-        // an xor-shuffle reduction.  The raw values of the next stage are loaded before the current one is converted.
-        constexpr int UNITS = BNS / 8;                     // units per thread and stage (BNS * 16 / 128)
-        constexpr int LPB = QB / 8;                        // lanes that share a block
-        const int qt = (int)threadIdx.x - QW0 * 32;
-        const bool wide = p.x_dtype == BI8_F32;
-        const int esz = wide ? 4 : 2;
-        const unsigned char* xb = static_cast<const unsigned char*>(p.X);
-        uint4 cur[UNITS][2], nxt[UNITS][2];
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        auto load_stage = [&](int ks, uint4 (&r)[UNITS][2]) {
-#pragma unroll
-            for (int u = 0; u < UNITS; ++u) {
-                const int unit = qt + u * 128, m = unit >> 4, k = ks * kBK + (unit & 15) * 8;
-                r[u][0] = make_uint4(0u, 0u, 0u, 0u);
-                r[u][1] = make_uint4(0u, 0u, 0u, 0u);
-                if (m < p.M && k < p.K) {
-                    const unsigned char* src = xb + ((int64_t)m * p.ldx + k) * esz;
-                    r[u][0] = ld_nc_v4(src);
-                    if (wide) r[u][1] = ld_nc_v4(src + 16);
-                }
-            }
-        };
-        int stage = 0;
-        uint32_t phase = 0;
-        int ks = ks_begin;
-        if (s_begin < s_end) load_stage(ks, nxt);
-        for (long long s = s_begin; s < s_end; ++s) {
-#pragma unroll
-            for (int u = 0; u < UNITS; ++u) {
-                cur[u][0] = nxt[u][0];
-                cur[u][1] = nxt[u][1];
-            }
-            const int ks_next = (ks + 1 == p.nks) ? 0 : ks + 1;
-            if (s + 1 < s_end) load_stage(ks_next, nxt);
-            const bool ok = __all_sync(0xffffffffu, mbar_wait(bar(G::EMPTY_AB + stage), phase ^ 1u, abort_flag));
-            if (!ok) {
-                if (lane == 0) report_timeout(p.status, abort_flag, W_EMPTY_AB);
-                break;
-            }
-            const uint32_t xt = base + (uint32_t)stage * G::STAGE_BYTES + G::W_BYTES;
-#pragma unroll
-            for (int u = 0; u < UNITS; ++u) {
-                const int unit = qt + u * 128, m = unit >> 4, piece = unit & 15, k = ks * kBK + piece * 8;
-                float f[8];
-                if (wide) {
-                    f[0] = __uint_as_float(cur[u][0].x); f[1] = __uint_as_float(cur[u][0].y);
-                    f[2] = __uint_as_float(cur[u][0].z); f[3] = __uint_as_float(cur[u][0].w);
-                    f[4] = __uint_as_float(cur[u][1].x); f[5] = __uint_as_float(cur[u][1].y);
-                    f[6] = __uint_as_float(cur[u][1].z); f[7] = __uint_as_float(cur[u][1].w);
-                } else {
-                    const uint32_t w4[4] = {cur[u][0].x, cur[u][0].y, cur[u][0].z, cur[u][0].w};
-#pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        if (p.x_dtype == BI8_BF16) {
-                            f[2 * h] = bf16lo(w4[h]);
-                            f[2 * h + 1] = bf16hi(w4[h]);
-                        } else {
-                            const float2 t2 = __half22float2(*reinterpret_cast<const __half2*>(&w4[h]));
-                            f[2 * h] = t2.x;
-                            f[2 * h + 1] = t2.y;
-                        }
-                    }
-                }
-                float amax = 0.0f;
-#pragma unroll
-                for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
-#pragma unroll
-                for (int off = 1; off < LPB; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-                BlockQ bq;
-                bq.set(amax, !wide);
-                const uint32_t lo = pack4(bq.q(f[0]), bq.q(f[1]), bq.q(f[2]), bq.q(f[3]));
-                const uint32_t hi = pack4(bq.q(f[4]), bq.q(f[5]), bq.q(f[6]), bq.q(f[7]));
-                if (m < p.M) {
-                    // 128-byte swizzle of a K-major tile: the 16-byte chunk index is xor-ed with the row index mod 8
-                    const uint32_t dst = xt + (uint32_t)(m * 128 + ((((piece >> 1) ^ (m & 7)) << 4) | ((piece & 1) << 3)));
-                    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(dst), "r"(lo), "r"(hi) : "memory");
-                    const int j = k / QB;
-                    if ((piece % LPB) == 0 && j < p.nb) sx[j * BNS + m] = amax;
-                }
-            }
-            fence_proxy_async_smem();            // the MMA reads the tile through the async proxy
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar(G::FULL_AB + stage));
-            if (++stage == G::STAGES) { stage = 0; phase ^= 1u; }
-            ks = ks_next;
+            ks += G::MMA_WARPS;
+            while (ks >= len) ks -= len;
         }
     } else if (warp < PW && (warp >> 2) < p.live_chunks) {
         // ---------------- promotion + epilogue: warp = 4 * chunk + lane quarter ----------------
         const int quarter = warp & 3, chunk = warp >> 2;
         const int row = quarter * 32 + lane;                       // weight row inside the tile
-        constexpr int CW = G::CW;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * CW);
         const float div = 1.0f / (127.0f * 127.0f);
-        asm volatile("griddepcontrol.wait;" ::: "memory");      // activation scales, and every store, after the previous kernel
 
-        // activation scales of all blocks, zero beyond the valid rows: [nb][BNS] (FUSED: the quantizer warps write the
-        // entries of a stage before they arrive on its barrier; columns beyond M are never stored)
-        const int nthreads = live_warps * 32;
-        if (!FUSED) {
-            const int total = p.nb * BNS;
+        // activation scales of this CTA's blocks, zero beyond the valid rows: [blocks][BNS] (SRC 1: written by the quantizer;
+        // rows beyond M are never stored)
+        if (SRC == 0) {
+            const int nthreads = live_warps * 32, j0 = k0 * G::BPS;
+            const int total = len * G::BPS * BNS;
             for (int i0 = threadIdx.x; i0 < total; i0 += nthreads * 8) {       // eight loads in flight per thread
                 float v[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    const int i = i0 + u * nthreads, j = i / BNS, m = i % BNS;
-                    v[u] = (i < total && m < p.M) ? __ldg(p.sA + (int64_t)j * p.M + m) : 0.0f;
+                    const int i = i0 + u * nthreads, j = j0 + i / BNS, m = i % BNS;
+                    v[u] = (i < total && m < p.M && j < p.nb) ? __ldg(p.sA + (int64_t)j * p.M + m) : 0.0f;
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
@@ -419,100 +589,162 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
             asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
         }
 
-        int stage = 0, buf = 0;
-        uint32_t phase = 0, accphase = 0;
+        // exchange: CTA `owner` of the cluster finishes this warp's quarter; `slot` is the quarter's place among the owner's
+        const int owner = quarter % CL, slot = quarter / CL;
+        const int pieces = ((p.M - chunk * CW < CW ? p.M - chunk * CW : CW) + 3) / 4;         // 16-byte pieces per thread that hold live rows
+        const uint32_t rx_buf_bytes = rx_bytes(BNS, CL);
+        // [owned quarter][chunk][rank of the sender][piece][lane][4 sums]
+        auto rx_at = [&](int buf, int from) {
+            return base + G::rx_off + (uint32_t)buf * rx_buf_bytes + (uint32_t)((((slot * G::CHUNKS + chunk) * CL + from) * 32 * CW) * 4);
+        };
+
+        // Adds one block's terms to the sums, in the reference's order per term: sB * (sA * (float(P) * 1/127^2)), on packed pairs,
+        // every operation rounded on its own.  P becomes a float by integer addition onto the bits of 1.5 * 2^23 (|P| < 2^22)
+        // and an exact subtraction, which issues four times as fast as the conversion; the sum is written as fma(t, 1, acc), so
+        // that the product in front of it cannot be contracted into it.
+        uint64_t acc2[CW / 2];
+#pragma unroll
+        for (int i = 0; i < CW / 2; ++i) acc2[i] = 0ull;
+        const uint64_t one2 = pack_f32x2(1.0f, 1.0f), div2 = pack_f32x2(div, div), nmagic2 = pack_f32x2(-kMagic, -kMagic);
+        auto add_block = [&](const uint32_t (&v)[CW], float sw, int ks, int blk) {
+            if ((k0 + ks) * G::BPS + blk >= p.nb) return;
+            const uint32_t sxa = sx_u32 + (uint32_t)(((ks * G::BPS + blk) * BNS + chunk * CW) * 4);
+            const uint64_t sw2 = pack_f32x2(sw, sw);
+#pragma unroll
+            for (int q = 0; q < CW / 4; ++q) {
+                uint64_t s[2];
+                lds_2xb64(sxa + (uint32_t)(q * 16), s[0], s[1]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint64_t biased = pack_u32x2(v[q * 4 + 2 * h] + 0x4B400000u, v[q * 4 + 2 * h + 1] + 0x4B400000u);
+                    const uint64_t pf = fma_f32x2(biased, one2, nmagic2);                               // float(P), exact
+                    acc2[q * 2 + h] = fma_f32x2(f2_mul(sw2, f2_mul(s[h], f2_mul(pf, div2))), one2, acc2[q * 2 + h]);
+                }
+            }
+        };
+        auto load_block = [&](uint32_t (&v)[CW], int buf, int blk) {
+            const uint32_t ta = t_lane + (uint32_t)(buf * G::ACC_STRIDE + blk * BNS);
+            if constexpr (CW == 8) tmem_ld8(ta, v);
+            else if constexpr (CW == 16) tmem_ld16(ta, v);
+            else tmem_ld32(ta, v);
+        };
+        auto load_scales = [&](float (&sw)[G::BPS], int stage) {
+            const uint32_t sc_u32 = base + (uint32_t)stage * G::STAGE_BYTES + G::W_BYTES + G::X_BYTES + (uint32_t)(row * 4);
+#pragma unroll
+            for (int blk = 0; blk < G::BPS; ++blk) sw[blk] = lds_f32(sc_u32 + (uint32_t)(blk * kTileRows * 4));
+        };
+        // A completed accumulator also says that the stage's scales have landed: the MMA issuer had waited for them.
         bool ok = true;
-        for (long long s = s_begin; s < s_end && ok;) {
-            const int tile = (int)(s / p.nks), ks0 = (int)(s - (long long)tile * p.nks);
-            const long long left = s_end - s;
-            const int len = (long long)(p.nks - ks0) < left ? (p.nks - ks0) : (int)left;
-            const int ks1 = ks0 + len;
+        auto wait_stage = [&](int buf, uint32_t parity) {
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(G::ACC_FULL + buf), parity, abort_flag));
+            if (!ok && lane == 0) report_timeout(p.status, abort_flag, W_ACC_FULL);
+            tc_fence_after();
+        };
+        auto release_stage = [&](int stage, int buf) {       // accumulators and scales are in registers
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(bar(G::ACC_EMPTY + buf));
+                mbar_arrive(bar(G::EMPTY_AB + stage));
+            }
+        };
+        // The end of a tile's share: exchange with the cluster and output (`ok` becomes false when a wait has run out).
+        auto finish_tile = [&](int r, int tile) {
             float acc[CW];
 #pragma unroll
-            for (int i = 0; i < CW; ++i) acc[i] = 0.0f;
-
-            for (int ks = ks0; ks < ks1; ++ks) {
-                // the stage's barrier is waited on here as well: this warp reads the scales the TMA wrote
-                ok = __all_sync(0xffffffffu, mbar_wait(bar(G::FULL_AB + stage), phase, abort_flag));
-                if (!ok) {
-                    if (lane == 0) report_timeout(p.status, abort_flag, W_FULL_AB);
-                    break;
-                }
-                ok = __all_sync(0xffffffffu, mbar_wait(bar(G::ACC_FULL + buf), accphase, abort_flag));
-                if (!ok) {
-                    if (lane == 0) report_timeout(p.status, abort_flag, W_ACC_FULL);
-                    break;
-                }
-                tc_fence_after();
-                uint32_t v[G::VB][CW];
-                float sw[G::BPS];
-                const uint32_t sc_u32 = base + (uint32_t)stage * G::STAGE_BYTES + G::W_BYTES + G::X_BYTES + (uint32_t)(row * 4);
-#pragma unroll
-                for (int b0 = 0; b0 < G::BPS; b0 += G::VB) {
-#pragma unroll
-                    for (int vb = 0; vb < G::VB; ++vb) {
-                        const uint32_t ta = t_lane + (uint32_t)(buf * G::ACC_STRIDE + (b0 + vb) * BNS);
-                        if constexpr (CW == 16) tmem_ld16(ta, v[vb]);
-                        else tmem_ld32(ta, v[vb]);
+            for (int i = 0; i < CW / 2; ++i) unpack_f32x2(acc2[i], acc[2 * i], acc[2 * i + 1]);
+            if (CL > 1) {
+                const int rb = p.rx_bufs > 1 ? (r & 1) : 0;
+                const uint32_t use = (uint32_t)(p.rx_bufs > 1 ? r >> 1 : r);        // how often this buffer was used before
+                const uint32_t full = bar(G::RX_FULL + rb * PW + warp), freed = bar(G::RX_FREE + rb * PW + warp);
+                if (owner != rank) {
+                    if (!cluster_ready) {
+                        cluster_wait();
+                        cluster_ready = true;
                     }
-                    if (b0 == 0) {
-#pragma unroll
-                        for (int blk = 0; blk < G::BPS; ++blk) sw[blk] = lds_f32(sc_u32 + (uint32_t)(blk * kTileRows * 4));
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar(G::EMPTY_AB + stage));       // scales are in registers
+                    if (use > 0) ok = __all_sync(0xffffffffu, mbar_wait_cluster(freed, (use - 1) & 1u, abort_flag));
+                    if (!ok) {
+                        if (lane == 0) report_timeout(p.status, abort_flag, W_PART);
+                        return;
                     }
-                    tmem_wait_ld();
+                    const uint32_t to = map_to(rx_at(rb, rank) + (uint32_t)(lane * 16), (uint32_t)owner), to_bar = map_to(full, (uint32_t)owner);
 #pragma unroll
-                    for (int vb = 0; vb < G::VB; ++vb) {
-                        const int blk = b0 + vb, j = ks * G::BPS + blk;
-                        if (j < p.nb) {
-                            const uint32_t sxa = sx_u32 + (uint32_t)((j * BNS + chunk * CW) * 4);
-#pragma unroll
-                            for (int q = 0; q < CW / 8; ++q) {
-                                uint64_t a0, a1, a2, a3;
-                                lds_2xb64(sxa + (uint32_t)(q * 32), a0, a1);
-                                lds_2xb64(sxa + (uint32_t)(q * 32 + 16), a2, a3);
-                                float sv[8];
-                                unpack_f32x2(a0, sv[0], sv[1]);
-                                unpack_f32x2(a1, sv[2], sv[3]);
-                                unpack_f32x2(a2, sv[4], sv[5]);
-                                unpack_f32x2(a3, sv[6], sv[7]);
-#pragma unroll
-                                for (int i = 0; i < 8; ++i) {
-                                    // the reference's order for one term: sB * (sA * (float(P) * 1/127^2))
-                                    const float pf = __fmul_rn((float)(int32_t)v[vb][q * 8 + i], div);
-                                    acc[q * 8 + i] = __fadd_rn(acc[q * 8 + i], __fmul_rn(sw[blk], __fmul_rn(sv[i], pf)));
-                                }
-                            }
-                        }
-                    }
+                    for (int i = 0; i < CW / 4; ++i)
+                        if (i < pieces) send_v4(to + (uint32_t)(i * 512), to_bar, acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
+                    return;
                 }
-                tc_fence_before();
+                if (lane == 0) mbar_expect_tx(full, (uint32_t)((CL - 1) * pieces * 512));
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar(G::ACC_EMPTY + buf));
-                if (++stage == G::STAGES) { stage = 0; phase ^= 1u; }
-                if (++buf == G::NBUF) { buf = 0; accphase ^= 1u; }
-            }
-            if (!ok) break;
-
-            const int n = tile * kTileRows + row;
-            if (ks0 == 0 && ks1 == p.nks) {
-                if (n < p.N) {
-#pragma unroll
-                    for (int i = 0; i < CW; ++i) {
-                        const int m = chunk * CW + i;
-                        if (m < p.M) finish_store(acc[i], m, n, p.bias, p.bias_dtype, p.bias_ld, p.C, p.ldc, p.out_dtype);
-                    }
+                ok = __all_sync(0xffffffffu, mbar_wait_cluster(full, use & 1u, abort_flag));
+                if (!ok) {
+                    if (lane == 0) report_timeout(p.status, abort_flag, W_PART);
+                    return;
                 }
-            } else {
-                // part of a tile: slot 0 of this CTA if the part begins where the CTA's range begins, else slot 1
-                const long long slot = 2ll * blockIdx.x + (s == s_begin ? 0 : 1);
-                float* w = p.ws + (slot * BNS + chunk * CW) * kTileRows + row;
+                // parts in ascending K order, this CTA's own (from registers) among them
 #pragma unroll
-                for (int i = 0; i < CW; ++i)
-                    if (chunk * CW + i < p.M) w[i * kTileRows] = acc[i];
+                for (int i = 0; i < CW / 4; ++i) {
+                    if (i >= pieces) break;
+                    float sum[4];
+                    for (int from = 0; from < CL; ++from) {
+                        uint32_t w[4] = {__float_as_uint(acc[4 * i]), __float_as_uint(acc[4 * i + 1]), __float_as_uint(acc[4 * i + 2]),
+                                         __float_as_uint(acc[4 * i + 3])};
+                        if (from != rank) lds_v4(rx_at(rb, from) + (uint32_t)(lane * 16 + i * 512), w[0], w[1], w[2], w[3]);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) sum[u] = from == 0 ? __uint_as_float(w[u]) : __fadd_rn(sum[u], __uint_as_float(w[u]));
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) acc[4 * i + u] = sum[u];
+                }
+                // the buffer may be written again, if it is going to be: the senders wait for this before their next use of it
+                if (r + p.rx_bufs < rounds) {
+                    if (!cluster_ready) {
+                        cluster_wait();
+                        cluster_ready = true;
+                    }
+                    __syncwarp();
+                    if (lane < CL && lane != rank) remote_arrive(map_to(freed, (uint32_t)lane));
+                    __syncwarp();
+                }
             }
-            s += len;
+            const int n = tile * kTileRows + row;
+            if (n < p.N) finish_chunk<CW>(acc, p, chunk * CW, n);
+        };
+
+        // one sequence of stages over all tiles of the cluster
+        int stage = 0, buf = 0, ks = 0, r = 0, tile = first_tile;
+        uint32_t accphase = 0;
+        auto next_stage = [&] {
+            if (++stage == G::STAGES) stage = 0;
+            if (++buf == G::NBUF) { buf = 0; accphase ^= 1u; }
+        };
+        auto end_of_stage = [&] {
+            if (++ks == len) {
+                finish_tile(r, tile);
+#pragma unroll
+                for (int i = 0; i < CW / 2; ++i) acc2[i] = 0ull;
+                ks = 0;
+                ++r;
+                tile += tile_step;
+            }
+        };
+        for (int s = 0; s < my_stages; ++s) {
+            wait_stage(buf, accphase);
+            if (!ok) break;
+            float sw[G::BPS];
+            load_scales(sw, stage);
+#pragma unroll
+            for (int b0 = 0; b0 < G::BPS; b0 += G::VB) {
+                uint32_t v[G::VB][CW];
+#pragma unroll
+                for (int q = 0; q < G::VB; ++q) load_block(v[q], buf, b0 + q);
+                tmem_wait_ld();
+                if (b0 + G::VB == G::BPS) release_stage(stage, buf);
+#pragma unroll
+                for (int q = 0; q < G::VB; ++q) add_block(v[q], sw[b0 + q], ks, b0 + q);
+            }
+            next_stage();
+            end_of_stage();
+            if (!ok) break;
         }
     }
 
@@ -523,6 +755,11 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
         tc_fence_after();
         tmem_dealloc(tmem_base, G::TMEM_COLS);
     }
+    // No CTA leaves while another of its cluster may still write into its shared memory.
+    __syncwarp();
+    if (!cluster_ready) cluster_wait();
+    cluster_arrive();
+    cluster_wait();
 }
 
 // Row-wise block quantizer for the few activation rows of a decode step (same arithmetic as the standalone quantizer:
@@ -536,8 +773,7 @@ __global__ void __launch_bounds__(256) skinny_quantize_kernel(const void* __rest
     // Launched with programmatic stream serialisation itself: resident while the kernel before it (the previous layer's
     // reduction) finishes.  Its own dependent, the GEMM, is released only after that kernel has completed, so that
     // whatever the GEMM reads early (weights, weight scales) has been at rest for a full kernel boundary.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    after_predecessor();
     constexpr int LPB = QB / 8;
     const int upr = nb * LPB;                                  // units per row, padded to whole blocks
     const int64_t u = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -583,213 +819,250 @@ __global__ void __launch_bounds__(256) skinny_quantize_kernel(const void* __rest
     if ((piece % LPB) == 0) sx[(int64_t)(k / QB) * M + m] = amax;
 }
 
-// Adds the parts of divided tiles in ascending K order and writes C; tiles that one CTA covered completely were
-// already written by it.  One thread per output element (a thread per tile row with a loop over the activation rows
-// serialises the loads and is several times slower); `ctas` and `total_stages` are those of the GEMM launch, bns its BNS.
-__global__ void __launch_bounds__(256) skinny_reduce_kernel(const float* __restrict__ ws, long long total_stages, int ctas,
-                                                            int nks, int bns, const void* bias, int bias_dtype,
-                                                            int64_t bias_ld, void* C, int64_t ldc, int out_dtype, int M, int N) {
-    // Launched with programmatic stream serialisation: the blocks may become resident while the GEMM still runs and do
-    // their index arithmetic; griddepcontrol.wait returns when the GEMM grid has completed and its stores are visible.
-    // A quantizer of this library launched the same way behind this kernel (the next layer's) may become resident now.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    const bool live = i < (int64_t)M * N;
-    const int m = live ? (int)(i / N) : 0, n = live ? (int)(i % N) : 0;
-    const int tile = n / kTileRows, row = n % kTileRows;
-    const long long t0 = (long long)tile * nks, t1 = t0 + nks;
-    long long c0 = t0 * ctas / total_stages;
-    while (c0 + 1 < ctas && range_start(c0 + 1, total_stages, ctas) <= t0) ++c0;
-    while (c0 > 0 && range_start(c0, total_stages, ctas) > t0) --c0;
-    // the tile's parts belong to CTAs c0, c0 + 1, ...; a part that begins where its CTA's range begins is that CTA's
-    // slot 0, and only the first part of a tile can begin elsewhere (at the tile's first stage, inside the range of c0)
-    const long long cs0 = range_start(c0, total_stages, ctas);
-    const bool whole = cs0 <= t0 && range_start(c0 + 1, total_stages, ctas) >= t1;   // written by the GEMM itself
-    int parts = 1;
-    while (range_start(c0 + parts, total_stages, ctas) < t1) ++parts;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (!live || whole) return;
-    float acc = __ldcg(ws + ((2 * c0 + (cs0 < t0 ? 1 : 0)) * bns + m) * kTileRows + row);
-    for (int q = 1; q < parts; q += 4) {                     // four loads in flight, added in ascending order
-        float v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = (q + u < parts) ? __ldcg(ws + (2 * (c0 + q + u) * bns + m) * kTileRows + row) : 0.0f;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (q + u < parts) acc = __fadd_rn(acc, v[u]);
-    }
-    finish_store(acc, m, n, bias, bias_dtype, bias_ld, C, ldc, out_dtype);
-}
-
-// The same reduction for a row-parallel layer: the tile sums are this rank's partial result, and instead of writing them
-// out for a second kernel the CTA exchanges them with the other ranks over peer memory right away (peer_common.cuh).  A
-// thread takes four consecutive columns of a row (they lie in one tile); `part` is the fp32 [M, N] array into which the
-// GEMM wrote the tiles that one CTA covered completely.  Launched for every shape, divided tiles or not.
-__global__ void __launch_bounds__(kPeerThreads) skinny_reduce_peer_kernel(const float* __restrict__ ws, long long total_stages, int ctas,
-                                                                          int nks, int bns, const float* __restrict__ part, int M,
-                                                                          int N, const PeerArgs a, const void* bias,
-                                                                          int bias_dtype, void* out, int out_dtype,
+// Row-parallel layer: the GEMM has left this rank's partial result in `part` (fp32 [M, N]); this kernel exchanges it with the
+// other ranks over peer memory (peer_common.cuh) and writes the layer's output.  A thread takes four consecutive columns.
+// Launched as a programmatic dependent of the GEMM: resident while it runs.
+__global__ void __launch_bounds__(kPeerThreads) skinny_reduce_peer_kernel(const float* __restrict__ part, int M, int N, const PeerArgs a,
+                                                                          const void* bias, int bias_dtype, void* out, int out_dtype,
                                                                           long long limit_cycles, int* status) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");       // as in skinny_reduce_kernel
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int64_t count = (int64_t)M * N;
     const int64_t i = (int64_t)blockIdx.x * kPeerChunk + (int64_t)threadIdx.x * 4;
-    const bool live = i < count;
-    const int m = live ? (int)(i / N) : 0, n = live ? (int)(i % N) : 0;
-    const int tile = n / kTileRows, row = n % kTileRows;
-    const long long t0 = (long long)tile * nks, t1 = t0 + nks;
-    long long c0 = t0 * ctas / total_stages;
-    while (c0 + 1 < ctas && range_start(c0 + 1, total_stages, ctas) <= t0) ++c0;
-    while (c0 > 0 && range_start(c0, total_stages, ctas) > t0) --c0;
-    const long long cs0 = range_start(c0, total_stages, ctas);
-    const bool whole = cs0 <= t0 && range_start(c0 + 1, total_stages, ctas) >= t1;   // written by the GEMM itself
-    int parts = 1;
-    while (range_start(c0 + parts, total_stages, ctas) < t1) ++parts;
     const uint32_t seq = peer_sequence(a);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live) {
-        if (whole) {
-            v = __ldcg(reinterpret_cast<const float4*>(part + i));
-        } else {
-            // parts in ascending K order, like skinny_reduce_kernel (0 + first part is exact)
-            v = __ldcg(reinterpret_cast<const float4*>(ws + ((2 * c0 + (cs0 < t0 ? 1 : 0)) * bns + m) * kTileRows + row));
-            for (int q = 1; q < parts; ++q) {
-                const float4 w = __ldcg(reinterpret_cast<const float4*>(ws + (2 * (c0 + q) * bns + m) * kTileRows + row));
-                v.x = __fadd_rn(v.x, w.x);
-                v.y = __fadd_rn(v.y, w.y);
-                v.z = __fadd_rn(v.z, w.z);
-                v.w = __fadd_rn(v.w, w.w);
-            }
-        }
-    }
+    if (i < count) v = __ldcg(reinterpret_cast<const float4*>(part + i));
     peer_exchange_store(a, seq, v, count, N, bias, bias_dtype, out, out_dtype, limit_cycles, status);
 }
 
-template <int QB, int BNS, bool FUSED>
-int launch_skinny(const GemmArgs& g, const SkParams& p, int grid, cudaStream_t st) {
-    using G = SkGeo<QB, BNS, FUSED>;
+template <int QB_, int BNS_, int SRC_>
+struct Instance {
+    static constexpr int QB = QB_, BNS = BNS_, SRC = SRC_;
+};
+
+// ---- host ---------------------------------------------------------------------------------------------------------------
+// How many clusters of a size fit on the device at once (one CTA per SM): asked once per device, for one kernel of the family.
+struct ClusterSlots {
+    int n[kMostCluster + 1] = {0};
+    bool known = false;
+};
+
+template <int QB, int BNS, int SRC>
+int launch_skinny(const GemmArgs& g, const SkParams& p, int cluster, int clusters, size_t smem, cudaStream_t st) {
+    using G = SkGeo<QB, BNS, SRC>;
     CUtensorMap mw, mx, ms;
     int dev = 0;
     BI8_CUDA_TRY(cudaGetDevice(&dev));
     int rc = cached_operand_map(&mw, dev, g.Bt, g.N, g.K, g.ldb, kTileRows);
     if (rc != BI8_OK) return rc;
-    if (FUSED) {
-        mx = mw;                    // not used: the quantizer warps write the activation tile
-    } else {
+    mx = mw;                        // SRC 1: not used, the kernel writes the activation tiles itself
+    if (SRC == 0) {
         rc = cached_operand_map(&mx, dev, g.A, g.M, g.K, g.lda, BNS);
         if (rc != BI8_OK) return rc;
     }
     rc = cached_scale_map(&ms, dev, g.sB, p.nb, g.N, kTileRows, G::BPS);
     if (rc != BI8_OK) return rc;
-    const size_t smem = smem_of<QB, BNS, FUSED>(p.nb);
     static SmemOptIn opt_in;
-    rc = opt_in.ensure(gemm_tc_skinny_kernel<QB, BNS, FUSED>, smem);
+    rc = opt_in.ensure(gemm_tc_skinny_kernel<QB, BNS, SRC>, smem);
     if (rc != BI8_OK) return rc;
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)grid);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(cluster * clusters));
     cfg.blockDim = dim3(G::THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;    // what may run before the predecessor has completed: early_weights
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;      // what may run before the predecessor has completed is decided in the kernel (early_weights)
-    BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tc_skinny_kernel<QB, BNS, FUSED>, mw, mx, ms, p));
+    cfg.numAttrs = 2;
+    BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tc_skinny_kernel<QB, BNS, SRC>, mw, mx, ms, p));
     return BI8_OK;
-}
-
-int bns_for(int64_t M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
-
-// dynamic shared memory of a launch; 0 for combinations that are not built
-size_t skinny_smem(int block, int bns, bool fused, int nb);
-
-size_t skinny_smem(int block, int bns, bool fused, int nb) {
-#define BI8_SM(QB, BNS) \
-    if (block == QB && bns == BNS) return fused ? (BNS <= 32 ? smem_of<QB, (BNS <= 32 ? BNS : 16), true>(nb) : 0) : smem_of<QB, BNS, false>(nb)
-    BI8_SM(32, 16); BI8_SM(32, 32); BI8_SM(32, 64);
-    BI8_SM(64, 16); BI8_SM(64, 32); BI8_SM(64, 64);
-    BI8_SM(128, 16); BI8_SM(128, 32); BI8_SM(128, 64);
-#undef BI8_SM
-    return 0;
 }
 
 constexpr size_t kSmemLimit = 227 * 1024;
 
-// conditions that depend on the shape only (the workspace query knows nothing else)
-bool skinny_shape_ok(int64_t M, int64_t N, int64_t K, int block, bool fused = false) {
+int cluster_slots(ClusterSlots* out, int sms) {
+    static ClusterSlots table[64];
+    static std::mutex mu;
+    int dev = 0;
+    BI8_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(BI8_ERR_CUDA, "device ordinal %d out of range", dev);
+    std::lock_guard<std::mutex> lock(mu);
+    ClusterSlots& t = table[dev];
+    if (!t.known) {
+        BI8_CUDA_TRY(cudaFuncSetAttribute(gemm_tc_skinny_kernel<64, 64, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
+        t.n[1] = sms;
+        for (int c = 2; c <= kMostCluster; c *= 2) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)(c * (sms / c)));
+            cfg.blockDim = dim3(SkGeo<64, 64, 0>::THREADS);
+            cfg.dynamicSmemBytes = kSmemLimit;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)c;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            BI8_CUDA_TRY(cudaOccupancyMaxActiveClusters(&t.n[c], gemm_tc_skinny_kernel<64, 64, 0>, &cfg));
+        }
+        t.known = true;
+    }
+    *out = t;
+    return BI8_OK;
+}
+
+int bns_for(int64_t M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
+int64_t stages_of(int64_t K, int bns) {
+    const int64_t ks = bns == 16 ? SkGeo<64, 16, 0>::KS : bns == 32 ? SkGeo<64, 32, 0>::KS : SkGeo<64, 64, 0>::KS;
+    return (K + ks - 1) / ks;
+}
+
+// f(Instance<...>) for the kernel instance of (block, bns, src), or `otherwise` where none is built
+template <typename R, typename F>
+R with_instance(int block, int bns, int src, R otherwise, F f) {
+#define BI8_SK(QB, BNS)                                          \
+    if (block == QB && bns == BNS) {                             \
+        if (src == 0) return f(Instance<QB, BNS, 0>{});          \
+        if constexpr (BNS <= 32) return f(Instance<QB, BNS, 1>{}); \
+    }
+    BI8_SK(32, 16) BI8_SK(32, 32) BI8_SK(32, 64)
+    BI8_SK(64, 16) BI8_SK(64, 32) BI8_SK(64, 64)
+    BI8_SK(128, 16) BI8_SK(128, 32) BI8_SK(128, 64)
+#undef BI8_SK
+    return otherwise;
+}
+
+// The cluster size: the one with the fewest stages from the first to the last.  The exchange of partial sums, and with it the
+// wait for the slowest of the cluster, counts as kExchange stages (measured at 8, 32 and 64 rows over ten layer shapes: 1.5,
+// 2.5 and 5.5 us for 2, 4 and 8 CTAs where a stage takes 0.4 us).  It depends on the shape alone (not on where the activations come
+// from), because it decides how the sums associate.
+struct SkPlan {
+    int cluster = 1, clusters = 1;
+    int64_t cost = 0;                       // in stages
+};
+constexpr int kExchange[3][kMostCluster + 1] = {{0, 0, 4, 0, 6, 0, 0, 0, 14}, {0, 0, 2, 0, 4, 0, 0, 0, 8}, {0, 0, 3, 0, 7, 0, 0, 0, 14}};
+int split_plan(int64_t N, int64_t K, int block, int bns, int sms, SkPlan* pl) {
+    ClusterSlots slots;
+    const int rc = cluster_slots(&slots, sms);
+    if (rc != BI8_OK) return rc;
+    const int64_t tiles = (N + kTileRows - 1) / kTileRows, nks = stages_of(K, bns);
+    int64_t best = -1;
+    // sizes at which the activations' operand tiles fit as well (SRC 1), else those at which the ring does
+    for (int src = bns == 16 ? 1 : 0; src >= 0 && best < 0; --src) {
+        for (int c = 1; c <= kMostCluster && c <= nks; c *= 2) {
+            const int fit = slots.n[c];
+            if (fit < 1) continue;
+            const size_t smem = with_instance(block, bns, src, (size_t)0, [&](auto in) {
+                using I = decltype(in);
+                return smem_of<I::QB, I::BNS, I::SRC>((int)((nks + c - 1) / c), c, tiles > fit ? 2 : 1);
+            });
+            if (smem == 0 || smem > kSmemLimit) continue;
+            const int64_t cost = (tiles + fit - 1) / fit * ((nks + c - 1) / c) + kExchange[bns == 16 ? 0 : bns == 32 ? 1 : 2][c];
+            if (best < 0 || cost < best) {
+                best = pl->cost = cost;
+                pl->cluster = c;
+                pl->clusters = (int)(tiles < fit ? tiles : fit);
+            }
+        }
+    }
+    if (best < 0) pl->cluster = 0;          // no size fits
+    return BI8_OK;
+}
+
+// What a launch needs beside the operands; `smem` 0: no kernel instance, or it does not fit.
+struct SkLaunch {
+    SkPlan plan;
+    int share = 0, rx_bufs = 1;
+    uint32_t sx_off = 0, xq_off = 0;
+    size_t smem = 0;
+};
+int plan_launch(const GemmArgs& g, int sms, SkLaunch* out) {
+    const int rc = split_plan(g.N, g.K, g.block, bns_for(g.M), sms, &out->plan);
+    if (rc != BI8_OK || out->plan.cluster == 0) return rc;
+    const int64_t tiles = (g.N + kTileRows - 1) / kTileRows, nks = stages_of(g.K, bns_for(g.M));
+    const int c = out->plan.cluster;
+    out->share = (int)((nks + c - 1) / c);
+    out->rx_bufs = tiles > out->plan.clusters ? 2 : 1;
+    out->smem = with_instance(g.block, bns_for(g.M), g.X != nullptr ? 1 : 0, (size_t)0, [&](auto in) {
+        using I = decltype(in);
+        return smem_of<I::QB, I::BNS, I::SRC>(out->share, c, out->rx_bufs, &out->sx_off, &out->xq_off);
+    });
+    if (out->smem > kSmemLimit) out->smem = 0;
+    return BI8_OK;
+}
+
+// conditions that depend on the shape only
+bool skinny_shape_ok(int64_t M, int64_t N, int64_t K, int block) {
     if (M < 1 || M > kSkMaxM || N < 1 || K < 1) return false;
     if (block != 32 && block != 64 && block != 128) return false;
-    if (N % 4 != 0 || N >= (1ll << 30) || K >= (1ll << 30)) return false;
-    const int64_t nb = (K + block - 1) / block;
-    if (nb > (1 << 20)) return false;
-    const size_t smem = skinny_smem(block, bns_for(M), fused, (int)nb);
-    return smem != 0 && smem <= kSmemLimit;
+    return N % 4 == 0 && N < (1ll << 30) && K < (1ll << 30);
 }
 
 }  // namespace
-
-// two fp32 slots of 128 x BNS per CTA
-size_t gemm_skinny_workspace_bytes(const GemmArgs& g) {
-    const DeviceInfo di = device_info();
-    if (!di.ok || g.partials != nullptr || !skinny_shape_ok(g.M, g.N, g.K, g.block)) return 0;
-    return (size_t)2 * di.sms * bns_for(g.M) * kTileRows * 4;
-}
 
 int launch_skinny_quantize(const void* x, int x_dtype, int64_t ldx, int8_t* q, float* sx, int64_t M, int64_t K, int block,
                            cudaStream_t st) {
     const int nb = (int)((K + block - 1) / block);
     const int64_t units = M * nb * (block / 8);
     const unsigned blocks = (unsigned)((units + 255) / 256);
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;     // the kernel waits for its predecessor itself
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     switch (block) {
-        case 32: BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, skinny_quantize_kernel<32>, x, x_dtype, ldx, q, sx, (int)M, (int)K, nb)); break;
-        case 64: BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, skinny_quantize_kernel<64>, x, x_dtype, ldx, q, sx, (int)M, (int)K, nb)); break;
-        case 128: BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, skinny_quantize_kernel<128>, x, x_dtype, ldx, q, sx, (int)M, (int)K, nb)); break;
+        case 32: return launch_chained(skinny_quantize_kernel<32>, blocks, 256, 0, st, x, x_dtype, ldx, q, sx, (int)M, (int)K, nb);
+        case 64: return launch_chained(skinny_quantize_kernel<64>, blocks, 256, 0, st, x, x_dtype, ldx, q, sx, (int)M, (int)K, nb);
+        case 128: return launch_chained(skinny_quantize_kernel<128>, blocks, 256, 0, st, x, x_dtype, ldx, q, sx, (int)M, (int)K, nb);
         default: return fail(BI8_ERR_BLOCK, "skinny quantizer supports block 32, 64, 128 (got %d)", block);
     }
-    BI8_CUDA_TRY(cudaGetLastError());
-    return BI8_OK;
 }
 
 bool gemm_skinny_applicable(const GemmArgs& g) {
-    if (g.partials != nullptr || !skinny_shape_ok(g.M, g.N, g.K, g.block, g.X != nullptr)) return false;
-    if (!device_info().ok) return false;
+    if (g.partials != nullptr || !skinny_shape_ok(g.M, g.N, g.K, g.block)) return false;
+    const DeviceInfo di = device_info();
+    if (!di.ok) return false;
     if (!aligned(g.Bt, 16) || g.ldb % 16 != 0 || !aligned(g.sB, 16)) return false;
     if (g.X != nullptr) {
-        // quantize-on-load reads 8 elements (16 or 32 bytes) at a time
+        // quantization inside the kernel reads 8 elements (16 or 32 bytes) at a time
         const int esz = g.x_dtype == BI8_F32 ? 4 : 2;
-        if (!aligned(g.X, 16) || (g.ldx * esz) % 16 != 0 || g.K % 8 != 0) return false;
+        if (g.M > 32 || !aligned(g.X, 16) || (g.ldx * esz) % 16 != 0 || g.K % 8 != 0 || (g.X2 != nullptr && !aligned(g.X2, 16))) return false;
     } else if (!aligned(g.A, 16) || g.lda % 16 != 0) {
         return false;
     }
-    const size_t need = gemm_skinny_workspace_bytes(g);
-    return g.workspace != nullptr && g.workspace_bytes >= need && aligned(g.workspace, 16);
+    SkLaunch l;
+    return plan_launch(g, di.sms, &l) == BI8_OK && l.smem != 0;
+}
+
+// Whether this kernel is also the faster one.  Up to 32 rows it always is.  From 33 on its promotion costs as much as the weights
+// take to arrive, and the general kernel overtakes it where it fills the SMs (clearly: a small layer keeps the reference's order of
+// operations): estimates in microseconds, from a sweep at 64 rows (4096 x 22016: 29 general, 45 here; x 11008: 23, 27; x 4096: 17, 13; 11008 x 4096: 25, 23).
+bool gemm_skinny_preferred(const GemmArgs& g) {
+    if (!gemm_skinny_applicable(g)) return false;
+    if (g.M <= 32) return true;
+    SkLaunch l;
+    const char* why = "";
+    if (plan_launch(g, device_info().sms, &l) != BI8_OK || !gemm_tc_applicable(g, &why)) return true;
+    return 0.68 * (double)l.plan.cost + 4.0 <= gemm_tc_estimate_us(g) + 2.5;
 }
 
 int launch_gemm_skinny(const GemmArgs& g, cudaStream_t st) {
     const DeviceInfo di = device_info();
     if (!di.ok) return fail(BI8_ERR_CUDA, "tensor-core GEMM needs a compute capability 10.x device");
+    SkLaunch l;
+    int rc = plan_launch(g, di.sms, &l);
+    if (rc != BI8_OK) return rc;
+    if (l.smem == 0) return fail(BI8_ERR_SHAPE, "skinny tensor-core GEMM: the shape's shared memory does not fit");
     SkParams p;
     std::memset(&p, 0, sizeof(p));
     p.sA = g.sA;
     p.X = g.X;
+    p.X2 = g.X2;
     p.ldx = g.ldx;
+    p.eps = g.eps;
+    p.op = g.pre_op;
     p.x_dtype = g.x_dtype;
     p.bias = g.bias;
     p.bias_ld = g.bias_ld;
     p.C = g.C;
-    p.ws = static_cast<float*>(g.workspace);
     p.status = device_status_ptr();
     if (!p.status) return BI8_ERR_CUDA;
     p.ldc = g.ldc;
@@ -797,64 +1070,28 @@ int launch_gemm_skinny(const GemmArgs& g, cudaStream_t st) {
     p.N = (int)g.N;
     p.K = (int)g.K;
     p.nb = (int)((g.K + g.block - 1) / g.block);
-    p.nks = (int)((g.K + kBK - 1) / kBK);
+    p.nks = (int)stages_of(g.K, bns_for(g.M));
+    p.tiles = (int)((g.N + kTileRows - 1) / kTileRows);
     p.out_dtype = g.out_dtype;
     p.bias_dtype = g.bias_dtype;
-    const int bns = bns_for(g.M), cw = bns <= 32 ? 16 : 32;
+    const int bns = bns_for(g.M), cw = bns / 2;
     p.live_chunks = (int)((g.M + cw - 1) / cw);
     p.early_weights = g.after_own_quantizer ? 1 : 0;
-    const long long tiles = (g.N + kTileRows - 1) / kTileRows;
-    p.total_stages = tiles * p.nks;
-    int grid = (int)(p.total_stages < di.sms ? p.total_stages : di.sms);
-    // with at least three quarters as many tiles as SMs, one whole tile per CTA (no divided tile, no reduction kernel) is
-    // faster than an even split (measured: 112 tiles 14.8 against 15.7 us; 96 tiles and fewer lose)
-    if (tiles <= di.sms && tiles * 4 >= (long long)di.sms * 3) grid = (int)tiles;
-    const bool fused = g.X != nullptr;
-    int rc = BI8_ERR_SHAPE;
-#define BI8_SK(QB, BNS)                                                                                               \
-    if (g.block == QB && bns == BNS) {                                                                                \
-        if (fused) rc = launch_skinny<QB, (BNS <= 32 ? BNS : 16), true>(g, p, grid, st);                              \
-        else rc = launch_skinny<QB, BNS, false>(g, p, grid, st);                                                      \
-    }
-    BI8_SK(32, 16) BI8_SK(32, 32) BI8_SK(32, 64)
-    BI8_SK(64, 16) BI8_SK(64, 32) BI8_SK(64, 64)
-    BI8_SK(128, 16) BI8_SK(128, 32) BI8_SK(128, 64)
-#undef BI8_SK
-    if (rc != BI8_OK) return rc;
-    if (g.peer != nullptr) {
-        // row-parallel layer: the reduction kernel also exchanges the sums with the other ranks and writes the layer's output
-        const PeerEpilogue& pe = *g.peer;
-        const int64_t count = g.M * g.N;
-        cudaLaunchConfig_t pc;
-        std::memset(&pc, 0, sizeof(pc));
-        pc.gridDim = dim3((unsigned)((count + kPeerChunk - 1) / kPeerChunk));
-        pc.blockDim = dim3(kPeerThreads);
-        pc.stream = st;
-        cudaLaunchAttribute pa[1];
-        pa[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;     // see skinny_reduce_kernel
-        pa[0].val.programmaticStreamSerializationAllowed = 1;
-        pc.attrs = pa;
-        pc.numAttrs = 1;
-        BI8_CUDA_TRY(cudaLaunchKernelEx(&pc, skinny_reduce_peer_kernel, (const float*)p.ws, p.total_stages, grid, p.nks, bns,
-                                        (const float*)g.C, (int)g.M, (int)g.N, *static_cast<const PeerArgs*>(pe.args), pe.bias,
-                                        pe.bias_dtype, pe.out, pe.out_dtype, pe.limit_cycles, p.status));
-        return BI8_OK;
-    }
-    if (p.total_stages % grid == 0 && (p.total_stages / grid) % p.nks == 0) return BI8_OK;   // no tile is divided
-    const int64_t total = g.M * g.N;
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)((total + 255) / 256));
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;     // see skinny_reduce_kernel
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, skinny_reduce_kernel, (const float*)p.ws, p.total_stages, grid, p.nks, bns,
-                                    g.bias, g.bias_dtype, g.bias_ld, g.C, g.ldc, g.out_dtype, (int)g.M, (int)g.N));
-    return BI8_OK;
+    p.rx_bufs = l.rx_bufs;
+    p.share = l.share;
+    p.sx_off = l.sx_off;
+    p.xq_off = l.xq_off;
+    rc = with_instance(g.block, bns, g.X != nullptr ? 1 : 0, (int)BI8_ERR_SHAPE, [&](auto in) {
+        using I = decltype(in);
+        return launch_skinny<I::QB, I::BNS, I::SRC>(g, p, l.plan.cluster, l.plan.clusters, l.smem, st);
+    });
+    if (rc != BI8_OK || g.peer == nullptr) return rc;
+    // row-parallel layer: a kernel behind this one exchanges the partial results with the other ranks and writes the layer's output
+    const PeerEpilogue& pe = *g.peer;
+    const int64_t count = g.M * g.N;
+    return launch_chained(skinny_reduce_peer_kernel, (unsigned)((count + kPeerChunk - 1) / kPeerChunk), kPeerThreads, 0, st, (const float*)g.C,
+                          (int)g.M, (int)g.N, *static_cast<const PeerArgs*>(pe.args), pe.bias, pe.bias_dtype, pe.out, pe.out_dtype, pe.limit_cycles,
+                          p.status);
 }
 
 }  // namespace bi8

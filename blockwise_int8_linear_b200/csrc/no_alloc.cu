@@ -60,8 +60,7 @@ size_t bi8_gemm_static_scratch_bytes(void) { return bi8::kScratchBytes; }
 int bi8_gemm_dequant_static(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb, const float* sA, const float* sB,
                             const void* bias, int bias_dtype, void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N,
                             int64_t K, int block, int flags, void* stream) {
-    // the plan that cannot be left out: split-K of the general kernel.  (The decode kernel for M <= 64 asks for more
-    // rows of scratch as M grows; where the array does not hold that, the dispatcher simply takes the general kernel.)
+    // the plan that cannot be left out: split-K of the general kernel
     bi8::GemmArgs shape{};
     shape.M = M;
     shape.N = N;
@@ -73,10 +72,8 @@ int bi8_gemm_dequant_static(const int8_t* A, int64_t lda, const int8_t* Bt, int6
                          "gemm_dequant_static: this shape needs %zu bytes of split-K scratch, the built-in array holds %zu; "
                          "use bi8_gemm_dequant with a caller workspace",
                          need, bi8::kScratchBytes);
-    // The array is offered to the dispatcher at its full size.  That is safe because every kernel that takes scratch
-    // checks the size it is given against its own plan before using it: gemm_skinny_applicable() compares
-    // workspace_bytes with gemm_skinny_workspace_bytes() and declines when the array is too small (the general kernel
-    // then runs, whose plan was checked above), and launch_gemm_tc() runs unsplit unless workspace_bytes covers its plan.
+    // The array is offered to the dispatcher at its full size: launch_gemm_tc(), the only taker, runs unsplit unless
+    // workspace_bytes covers its plan.
     void* scratch = nullptr;
     size_t given = 0;
     if (bi8_gemm_workspace_bytes(M, N, K, block) > 0) {
@@ -84,6 +81,14 @@ int bi8_gemm_dequant_static(const int8_t* A, int64_t lda, const int8_t* Bt, int6
         if (!scratch) return BI8_ERR_CUDA;
         given = bi8::kScratchBytes;
     }
+    // 33 to 64 rows run on the general kernel here, as this entry point has always promised
+    const bool forced = (flags & (BI8_GEMM_FORCE_GENERIC | BI8_GEMM_FORCE_TC | BI8_GEMM_FORCE_SMALLM | BI8_GEMM_FORCE_SKINNY)) != 0;
+    shape.A = A;
+    shape.Bt = Bt;
+    shape.lda = lda;
+    shape.ldb = ldb;
+    const char* why = "";
+    if (M > 32 && M <= 64 && K > 0 && !forced && bi8::gemm_tc_applicable(shape, &why)) flags |= BI8_GEMM_FORCE_TC;
     return bi8_gemm_dequant(A, lda, Bt, ldb, sA, sB, bias, bias_dtype, C, ldc, out_dtype, M, N, K, block, scratch, given, flags,
                             stream);
 }

@@ -64,6 +64,61 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
     return d;
 }
 
+// the value a kernel storing `v` in the activation type would have left in memory
+__device__ __forceinline__ float round_to(float v, int dt) {
+    if (dt == BI8_BF16) return __bfloat162float(__float2bfloat16_rn(v));
+    if (dt == BI8_F16) return __half2float(__float2half_rn(v));
+    return v;
+}
+
+// silu(g) as the separate kernel stores it: one fp32 exponential, an IEEE division, one rounding to the activation type.
+__device__ __forceinline__ float silu_exact(float g, int dt) { return round_to(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), dt); }
+
+// two values rounded to a 16-bit activation type and packed; and back
+__device__ __forceinline__ uint32_t pack16(float lo, float hi, bool bf) { return bf ? pack_bf16x2(lo, hi) : pack_f16x2(lo, hi); }
+__device__ __forceinline__ float2 unpack16(uint32_t w, bool bf) {
+    return bf ? make_float2(bf16lo(w), bf16hi(w)) : __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+
+// g = cast(cast(silu(g)) * v), the gated activation as its two separate kernels would leave it, bit for bit.
+//
+// What is stored of silu(g) is its 16-bit rounding, so an approximate value decides it unless it lies next to a rounding
+// boundary: s = g * rcp(1 + ex2(-g log2 e)) with the hardware's approximations (2^-22 and 2^-23 relative) is within
+// eps = (|t| + 16) * 1.25 * 2^-24 of silu_exact's fp32 value before rounding, t = g log2 e (the rounding of t costs |t| 2^-24, the exponential
+// 4 units of 2^-24, the reciprocal 2, the sum and the product 1 each, and silu_exact's own error is at most 4), and where s (1 - eps) and
+// s (1 + eps) round to the same value, that is the value.  Elsewhere (1 in 1400 values of bf16, 1 in 180 of fp16) and for
+// |g| > 60 silu_exact is evaluated.  65 instructions per value became 20: 2048 x 11008 in 41 us was bound by issue.
+__device__ __forceinline__ void silu_mul8(float (&g)[8], const float (&v)[8], int dt) {
+    if (dt == BI8_F32) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) g[e] = __fmul_rn(silu_exact(g[e], dt), v[e]);
+        return;
+    }
+    const bool bf = dt == BI8_BF16;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        float lo[2], hi[2];
+        bool far = false;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const float x = g[2 * h + u], t = __fmul_rn(x, -1.4426950408889634f);
+            float ex, r;
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ex) : "f"(t));
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fadd_rn(1.0f, ex)));
+            const float s = __fmul_rn(x, r), eps = __fmaf_rn(fabsf(t), 1.25f * 5.9604644775390625e-8f, 20.0f * 5.9604644775390625e-8f);
+            hi[u] = __fmaf_rn(s, eps, s);
+            lo[u] = __fmaf_rn(s, -eps, s);
+            far = far || !(fabsf(x) <= 60.0f);
+        }
+        uint32_t w = pack16(lo[0], lo[1], bf);
+        if (far || w != pack16(hi[0], hi[1], bf)) w = pack16(silu_exact(g[2 * h], dt), silu_exact(g[2 * h + 1], dt), bf);
+        const float2 s = unpack16(w, bf);
+        const float2 y = unpack16(pack16(__fmul_rn(s.x, v[2 * h]), __fmul_rn(s.y, v[2 * h + 1]), bf), bf);
+        g[2 * h] = y.x;
+        g[2 * h + 1] = y.y;
+    }
+}
+
 // Quantizes eight values of one block (scale amax) on packed pairs: the same operations, each rounded on its own, as BlockQ::q.
 // Returns the bytes of values 0-3 and 4-7.
 __device__ __forceinline__ void quantize8(const float (&v)[8], const BlockQ& bq, uint32_t& lo, uint32_t& hi) {

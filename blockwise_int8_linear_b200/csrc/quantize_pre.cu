@@ -95,13 +95,6 @@ __device__ __forceinline__ void unpack8(float* f, const uint32_t* w, int dt) {
     }
 }
 
-// the value a kernel storing `v` in the activation type would have left in memory
-__device__ __forceinline__ float round_to(float v, int dt) {
-    if (dt == BI8_BF16) return __bfloat162float(__float2bfloat16_rn(v));
-    if (dt == BI8_F16) return __half2float(__float2half_rn(v));
-    return v;
-}
-
 // Quantizes the eight values of a unit whose block's other units sit in the neighbouring lanes (LPB lanes per block)
 // and stores them; all 32 lanes of the warp must call it.
 template <int QB>
@@ -240,14 +233,10 @@ __global__ void __launch_bounds__(kPreThreads) silu_mul_quantize_kernel(const vo
 #pragma unroll
     for (int e = 0; e < 8; ++e) y[e] = 0.0f;
     if (valid) {
-        float g[8], v[8];
-        load8(g, gate, (int64_t)m * ldx, k, K, dt, vec_in != 0);
+        float v[8];
+        load8(y, gate, (int64_t)m * ldx, k, K, dt, vec_in != 0);
         load8(v, up, (int64_t)m * ldx, k, K, dt, vec_in != 0);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const float s = round_to(__fdiv_rn(g[e], __fadd_rn(1.0f, expf(-g[e]))), dt);
-            y[e] = round_to(__fmul_rn(s, v[e]), dt);
-        }
+        silu_mul8(y, v, dt);
     }
     quantize_unit<QB>(y, valid, dt != BI8_F32, q, ldq, sx, m, k, M, K, vec_out != 0);
 }

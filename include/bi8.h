@@ -102,7 +102,7 @@ BI8_API int bi8_dequantize_rowwise(const int8_t* q, const float* s, void* out, i
  * transposed view Bt^T with strides (1, ldb).  sA [ceil(K/block), M], sB [ceil(K/block), N] fp32.
  * bias [N] of bias_dtype or NULL.  C [M,N] of out_dtype, row stride ldc.
  * workspace: bi8_gemm_workspace_bytes(M,N,K,block) bytes of 16-byte aligned device memory (may be NULL when that
- * is 0; without it small-M shapes run on slower kernels).  It is plain scratch: nothing has to be cleared, every
+ * is 0; without it shapes with few output tiles run slower).  It is plain scratch: nothing has to be cleared, every
  * call overwrites what it later reads; calls that may run concurrently need separate workspaces.
  * The int32 partial sums are exact.  The fp32 accumulation of the tensor-core kernel for M > 64 evaluates a term as
  * sB * fl(P * s) with s = sA/127^2 rounded to fp32 and then to 22 significant bits (relative error of s at most
@@ -147,7 +147,7 @@ BI8_API int bi8_dequantize_rowwise_pitched(const int8_t* q, int64_t ldq, const f
  * device looks up the array's device address: make it outside any stream capture.  All calls share the array
  * (nothing needs clearing between calls); calls that can overlap on one GPU race on it and must be serialised by
  * the caller.  Arguments and results are those of bi8_gemm_dequant (bit-identical where both select the same kernel;
- * for 33 <= M <= 64 this entry point's scratch is too small for the decode kernel and the general kernel runs). */
+ * for 33 <= M <= 64 this entry point always runs the general kernel). */
 BI8_API int bi8_gemm_dequant_static(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb,
                             const float* sA, const float* sB, const void* bias, int bias_dtype,
                             void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N, int64_t K, int block,
@@ -162,12 +162,12 @@ BI8_API int bi8_gemm_block_partials(const int8_t* A, int64_t lda, const int8_t* 
 /* Forward of the layer in one call (block_linear.py:78-80 / 141-143): quantize-on-load GEMM.  x [M,K] of x_dtype, row
  * stride ldx, is quantized per row and block exactly as bi8_quantize_rowwise does and multiplied with the
  * pre-quantized weights Wq [N,K] / sW; the result equals bi8_quantize_rowwise followed by bi8_gemm_dequant.
- * For M <= 64 (N a multiple of 4, K a multiple of 16, 16-byte aligned rows, workspace given) the weight-streaming
- * tensor-core GEMM runs behind a small quantizer kernel and is launched so that its set-up and first weight
- * loads overlap that kernel; with BI8_GEMM_QUANT_IN_KERNEL (or without scratch; M <= 32) the GEMM kernel itself quantizes
- * the activations as it loads its stages: one kernel, no scratch, but measured slower.  Every other shape runs the
+ * For M <= 64 (N a multiple of 4, K a multiple of 16, 16-byte aligned rows) the weight-streaming tensor-core GEMM runs: up to
+ * 16 rows it quantizes the activations itself as its first weights arrive, in one launch; above, a small quantizer kernel
+ * runs in front and the GEMM is launched so that its set-up and first weight loads overlap it.  With
+ * BI8_GEMM_QUANT_IN_KERNEL (or without scratch) the one-launch form is taken up to 32 rows.  Every other shape runs the
  * standalone quantizer and the GEMM back to back.  xq [M,K] int8 and sx [ceil(K/block),M] fp32 are scratch, which
- * may be NULL only when the M <= 32 conditions hold.  The scratch contents after the call are
+ * may be NULL only when the one-launch form applies.  The scratch contents after the call are
  * unspecified.  workspace as for bi8_gemm_dequant. */
 BI8_API int bi8_gemm_dequant_fused_quant(const void* x, int x_dtype, int64_t ldx, int8_t* xq, float* sx,
                                  const int8_t* Wq, int64_t ldw, const float* sW, const void* bias, int bias_dtype,
@@ -190,12 +190,11 @@ BI8_API int bi8_quantize_rowwise_pre(int op, const void* x, const void* x2, int 
                              float eps, int8_t* q, float* scales, int64_t M, int64_t K, int block, void* stream);
 /* bi8_gemm_dequant_fused_quant with that step in front of its quantizer and an optional residual behind its result:
  *   C = cast(acc) (+ cast(bias)) (+ residual), every addition in the output type (a layer's `x + proj(...)`).
- * residual [M,N] of out_dtype, row stride ldr, NULL for none.  For M <= 64 (N a multiple of 4, K of 16, workspace given) the
- * quantizer kernel of `op` takes the decode quantizer's place in front of the weight-streaming GEMM (same overlap), and
- * without bias the residual is added by the kernel that writes C; on that path, and only there, C may be the residual
- * itself (a residual stream updated in place; any other overlap of the two is BI8_ERR_SHAPE, the same tensor on another
- * path BI8_ERR_ALIGN).  Other shapes run quantizer, GEMM and one elementwise kernel back to back.  xq / sx are required
- * scratch. */
+ * residual [M,N] of out_dtype, row stride ldr, NULL for none.  For M <= 64 (N a multiple of 4, K of 16) the step runs inside
+ * the weight-streaming GEMM (few activation values) or in its quantizer kernel in front of it; the residual is added by
+ * the kernel that writes C, here and in the general tensor-core kernel.  Without bias C may be the residual itself (a
+ * residual stream updated in place; any other overlap of the two is BI8_ERR_SHAPE, the same tensor where neither kernel
+ * applies BI8_ERR_ALIGN).  xq / sx are required scratch. */
 BI8_API int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtype, int64_t ldx, const void* norm_weight,
                                float eps, int8_t* xq, float* sx, const int8_t* Wq, int64_t ldw, const float* sW,
                                const void* bias, int bias_dtype, const void* residual, int64_t ldr, void* C, int64_t ldc,

@@ -1,0 +1,113 @@
+"""Kernel variants at the sizes where they can go wrong: rows of any alignment, every 16-bit gate value, the cluster sizes and
+tile edges of the decode GEMM with its quantization inside, and the additions behind the general GEMM."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from oracle import blockwise_int8_oracle as O
+from tests.gpu_util import DEV, assert_clean_device, randn_bf16, set_config
+
+pytestmark = pytest.mark.gpu
+
+
+def _tf():
+    import triton_functions as tf
+    return tf
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("block", [32, 64, 128])
+@pytest.mark.parametrize("shape,offset", [((1, 1), 0), ((3, 7), 1), ((129, 131), 0), ((257, 1001), 3), ((128, 136), 5), ((70, 4101), 0)])
+def test_quantizers_take_rows_of_any_alignment(shape, offset, block, dt):
+    tf = _tf()
+    set_config(block, dt)
+    r, c = shape
+    x = randn_bf16((r, c), r + c, std=2.0).to(dt)
+    if dt == torch.float32:
+        x = x + torch.randn((r, c), generator=torch.Generator().manual_seed(c)) * 1e-3
+    buf = torch.full((r * c + 16,), float("inf"), dtype=dt, device=DEV)         # what lies around the matrix must not be taken in
+    view = buf[offset:offset + r * c].view(r, c)
+    view.copy_(x)
+    q_ref, s_ref = O.quantize(x, block)
+    qt_ref, st_ref = O.quantize(x.t().contiguous(), block)
+    for q, s in (tf.quantize_block_rowwise(view), tf.quantize_block_dual(view)[:2]):
+        assert torch.equal(q.cpu(), q_ref) and torch.equal(s.cpu(), s_ref)
+    for q, s in (tf.quantize_block_colwise(view), tf.quantize_block_dual(view)[2:]):
+        assert torch.equal(q.cpu(), qt_ref) and torch.equal(s.cpu(), st_ref)
+    q, s = tf.quantize_block_rowwise(view)
+    for pitched in (q, q.contiguous()):
+        assert torch.equal(tf.dequantize_block_rowwise(pitched, s).cpu(), O.dequantize(q_ref, s_ref, block, dt))
+    assert_clean_device()
+    set_config(64)
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_gated_activation_of_every_gate_value(dt):
+    """Every finite 16-bit value as the gate: the approximate evaluation with its exact fallback is bit-identical to
+    F.silu(gate) * up, quantized."""
+    tf = _tf()
+    set_config(64, dt)
+    bits = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(dt)
+    gate = torch.where(bits.isfinite(), bits, torch.zeros_like(bits)).view(256, 256).to(DEV)
+    up = randn_bf16((256, 256), 3).to(dt).to(DEV)
+    for u in (up, torch.ones_like(up)):
+        q, s = tf.silu_mul_quantize_block_rowwise(gate, u)
+        q_ref, s_ref = tf.quantize_block_rowwise(F.silu(gate) * u)
+        fine = s_ref.isfinite()
+        assert torch.equal(s[fine], s_ref[fine])
+        assert torch.equal(q.view(256, 4, 64)[fine.t()], q_ref.view(256, 4, 64)[fine.t()])
+    assert_clean_device()
+
+
+@pytest.mark.parametrize("block", [32, 64, 128])
+@pytest.mark.parametrize("m,k,n", [(1, 16, 4), (1, 128, 128), (7, 272, 132), (8, 1024, 4096), (9, 4096, 260), (16, 2064, 1028), (17, 528, 388),
+                                   (32, 4096, 512), (2, 8192, 22016), (5, 640, 20000)])
+def test_decode_layer_quantized_inside_the_gemm(m, k, n, block):
+    """One launch against quantizer + GEMM: bit-identical, for clusters of 1 to 8 CTAs, one and several tiles per cluster, K that
+    ends inside a block, a 128-byte step and a stage; plain, behind RMSNorm and SiLU * up, with a residual in place."""
+    tf = _tf()
+    set_config(block)
+    x = randn_bf16((m, 2 * k), 5 * m + k, std=1.5).to(DEV)
+    a, b = x[:, :k], x[:, k:]
+    wq, sw = tf.quantize_block_rowwise(randn_bf16((n, k), k + n, std=0.02).to(DEV))
+    norm = randn_bf16((k,), 9).to(DEV)
+    res = randn_bf16((m, n), 14).to(DEV)
+    steps = {"none": tf.quantize_block_rowwise(a), "rmsnorm": tf.rmsnorm_quantize_block_rowwise(a, 1e-5, norm),
+             "silu_mul": tf.silu_mul_quantize_block_rowwise(a, b)}
+    for op, (xq, sx) in steps.items():
+        want = tf.int8_matmul_block64_rowwise_dequantize(xq, wq.t(), sx, sw)
+        kw = dict(x2=b if op == "silu_mul" else None, norm_weight=norm if op == "rmsnorm" else None)
+        got = tf.pre_quantize_matmul_block_rowwise_dequantize(op, a, wq.t(), sw, flags=32, **kw)
+        assert torch.equal(got, want), op
+        out = res.clone()
+        tf.pre_quantize_matmul_block_rowwise_dequantize(op, a, wq.t(), sw, residual=out, out=out, flags=32, **kw)
+        assert torch.equal(out, want + res), op
+    q, s = (t.cpu() for t in steps["none"])
+    ref = O.gemm(q, wq.cpu().t(), s, sw.cpu(), None, block, torch.bfloat16).float()
+    got = tf.quantize_matmul_block_rowwise_dequantize(a, wq.t(), sw).cpu().float()
+    assert (got - ref).abs().max().item() <= 2.0 ** -7 * ref.abs().max().item()
+    assert_clean_device()
+    set_config(64)
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("m,k,n", [(65, 512, 160), (129, 128, 161), (100, 2048, 777), (300, 1000, 328), (2500, 256, 1000)])
+def test_bias_and_residual_behind_the_general_gemm(m, k, n, dt):
+    """Whole and divided tiles, outputs with and without aligned rows, a strided residual: each addition in the output type."""
+    tf = _tf()
+    set_config(64, dt)
+    x = randn_bf16((m, k), m + k).to(dt).to(DEV)
+    wq, sw = tf.quantize_block_rowwise(randn_bf16((n, k), k + n, std=0.02).to(DEV))
+    bias = randn_bf16((n,), 7).to(DEV)
+    wide = randn_bf16((m, n + 3), 8).to(dt).to(DEV)
+    plain = tf.quantize_matmul_block_rowwise_dequantize(x, wq.t(), sw)
+    xq, sx = tf.quantize_block_rowwise(x)
+    assert torch.equal(plain, tf.int8_matmul_block64_rowwise_dequantize(xq, wq.t(), sx, sw))
+    for b in (None, bias):
+        base = plain if b is None else plain + b.to(dt)
+        assert torch.equal(tf.quantize_matmul_block_rowwise_dequantize(x, wq.t(), sw, b), base)
+        for res in (wide[:, :n].contiguous(), wide[:, :n]):
+            got = tf.pre_quantize_matmul_block_rowwise_dequantize("none", x, wq.t(), sw, b, residual=res)
+            assert torch.equal(got, base + res)
+    assert_clean_device()
+    set_config(64)
