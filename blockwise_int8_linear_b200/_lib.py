@@ -29,7 +29,7 @@ EXPORTS = [
     "bi8_row_parallel_linear_pre", "bi8_peer_allreduce_large", "bi8_peer_allreduce_large_buffer_bytes",
     "bi8_peer_allreduce_large_partial_offset", "bi8_peer_allreduce_large_out_offset", "bi8_rope_cache_append",
     "bi8_gemm_dequant_residual", "bi8_quantize_rowwise_pitched", "bi8_quantize_colwise_pitched", "bi8_quantize_dual_pitched",
-    "bi8_quantize_rowwise_pre_pitched", "bi8_dequantize_rowwise_pitched",
+    "bi8_quantize_rowwise_pre_pitched", "bi8_dequantize_rowwise_pitched", "bi8_column_sum", "bi8_column_sum_workspace_bytes",
 ]
 ADDEND_FULL = 0x100
 PRE_NONE, PRE_RMSNORM, PRE_SILU_MUL = 0, 1, 2
@@ -64,6 +64,9 @@ def lib() -> ctypes.CDLL:
         L.bi8_quantize_colwise_pitched.argtypes = [vp, i32, i64, vp, i64, vp, i64, i64, i32, vp]
         L.bi8_quantize_dual_pitched.argtypes = [vp, i32, i64, vp, i64, vp, vp, i64, vp, i64, i64, i32, vp]
         L.bi8_quantize_rowwise_pre_pitched.argtypes = [i32, vp, vp, i32, i64, vp, c.c_float, vp, i64, vp, i64, i64, i32, vp]
+        L.bi8_column_sum.argtypes = [vp, i32, i64, vp, i64, i64, vp, sz, vp]
+        L.bi8_column_sum_workspace_bytes.argtypes = [i64, i64]
+        L.bi8_column_sum_workspace_bytes.restype = sz
         L.bi8_dequantize_rowwise_pitched.argtypes = [vp, i64, vp, vp, i32, i64, i64, i32, vp]
         L.bi8_peer_allreduce_buffer_bytes.argtypes = [i32, i64]
         L.bi8_peer_allreduce_buffer_bytes.restype = sz
@@ -95,7 +98,7 @@ def lib() -> ctypes.CDLL:
         for name in EXPORTS:
             fn = getattr(L, name)
             if name not in ("bi8_last_error_string", "bi8_gemm_workspace_bytes", "bi8_gemm_static_scratch_bytes",
-                            "bi8_peer_allreduce_buffer_bytes", "bi8_peer_allreduce_large_buffer_bytes",
+                            "bi8_peer_allreduce_buffer_bytes", "bi8_peer_allreduce_large_buffer_bytes", "bi8_column_sum_workspace_bytes",
                             "bi8_peer_allreduce_large_partial_offset", "bi8_peer_allreduce_large_out_offset"):
                 fn.restype = i32
         _lib = L

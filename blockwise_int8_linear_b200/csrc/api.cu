@@ -253,6 +253,17 @@ int bi8_dequantize_rowwise(const int8_t* q, const float* s, void* out, int out_d
     return bi8_dequantize_rowwise_pitched(q, K, s, out, out_dtype, M, K, block, stream);
 }
 
+size_t bi8_column_sum_workspace_bytes(int64_t R, int64_t C) { return column_sum_workspace_bytes(R, C); }
+
+int bi8_column_sum(const void* x, int dtype, int64_t ldx, void* out, int64_t R, int64_t C, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!dtype_ok(dtype)) return fail(BI8_ERR_DTYPE, "column_sum: unknown dtype code %d", dtype);
+    if (R < 0 || C < 0 || ldx < C) return fail(BI8_ERR_SHAPE, "column_sum: bad shape R=%lld C=%lld ldx=%lld", (long long)R, (long long)C, (long long)ldx);
+    if (C == 0) return BI8_OK;
+    if (!out || (!x && R > 0)) return fail(BI8_ERR_NULL, "column_sum: null pointer");
+    if (!aligned(x, dtype_size(dtype)) || !aligned(out, dtype_size(dtype))) return fail(BI8_ERR_ALIGN, "column_sum: pointer not element aligned");
+    return launch_column_sum(x, dtype, ldx, out, R, C, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
 size_t bi8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int block) {
     if (M <= 0 || N <= 0 || K <= 0 || (block != 32 && block != 64 && block != 128)) return 0;
     GemmArgs g{};

@@ -51,9 +51,9 @@ struct SmemOptIn {
 // writes; dependents are released only there, so that "the predecessor has completed" always means that everything before
 // it has completed too.  What it saves is the launch latency and the kernel's set-up, 1-2 us per kernel of a chain.
 template <typename... P, typename... A>
-int launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
+int launch_chained_grid(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -64,6 +64,11 @@ int launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, size_t
     cfg.numAttrs = 1;
     BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
     return BI8_OK;
+}
+
+template <typename... P, typename... A>
+int launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
+    return launch_chained_grid(kernel, dim3(grid), threads, smem, st, std::forward<A>(args)...);
 }
 
 #if defined(__CUDACC__)
@@ -101,6 +106,10 @@ int launch_peer_allreduce_large(void* const* peer_bufs, int rank, int world, int
 // rotary embedding of q and k and the append of k and v to the caches for one decode step (rope_cache.cu)
 int launch_rope_cache_append(const void* qkv, int dt, const float* cis, const long long* pos, void* q_out, void* kcache, void* vcache,
                              int64_t B, int64_t H, int64_t D, int64_t max_len, cudaStream_t st);
+// column sums in fp32 (column_sum.cu)
+size_t column_sum_workspace_bytes(int64_t R, int64_t C);
+int launch_column_sum(const void* x, int dt, int64_t ldx, void* out, int64_t R, int64_t C, void* workspace, size_t workspace_bytes,
+                      cudaStream_t st);
 int launch_dequantize_rowwise(const int8_t* q, int64_t ldq, const float* s, void* out, int dt, int64_t M, int64_t K,
                               int block, cudaStream_t st);
 

@@ -110,10 +110,11 @@ __device__ __forceinline__ void load_unit8(const T* p, const T* row_end, int val
 }
 
 // Row-wise quantize, vector path: any float type and (SHIFT) any alignment of the input rows; the int8 rows begin on 8-byte
-// boundaries (pitch ldq).  A lane takes eight elements, a CTA covers 32 rows x 256 columns; warp w handles rows w, w+8,
-// w+16, w+24 and issues their loads before any arithmetic.  Bound by memory: for 16-bit inputs that the streaming kernel
+// boundaries (pitch ldq).  A lane takes eight elements, a CTA covers 8 * RPW rows x 256 columns; warp w handles rows w, w+8,
+// ... and issues their loads before any arithmetic.  RPW is 4, or 1 where that leaves SMs without a CTA: a row is eight
+// divisions per lane in fp32, and four of them in sequence were 4.9 us of a 512 x 768 matrix's.  Bound by memory: for 16-bit inputs that the streaming kernel
 // below does not take (rows that are not 32-byte aligned) and for fp32.
-template <typename T, int B, bool SHIFT>
+template <typename T, int B, bool SHIFT, int RPW>
 __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
     const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int M, int K, int nb,
     int col_tiles) {
@@ -123,17 +124,18 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
     constexpr int BPT = WCOLS / B;          // blocks per tile row
     constexpr int NW = 2 * (int)sizeof(T);  // 32-bit words of a lane's eight elements
     static_assert(LPB >= 1 && LPB <= 32, "block must be a multiple of the lane vector");
-    __shared__ float s_scale[BPT][kTileRows];
+    constexpr int ROWS = 8 * RPW;
+    __shared__ float s_scale[BPT][ROWS];
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ct = blockIdx.x % col_tiles, rt = blockIdx.x / col_tiles;
     const int col = ct * WCOLS + lane * 8;
     const int valid = K - col < 8 ? K - col : 8;          // elements of this lane inside the row; <= 0: none
 
-    uint32_t raw[4][NW];
+    uint32_t raw[RPW][NW];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int row = rt * kTileRows + warp + 8 * i;
+    for (int i = 0; i < RPW; ++i) {
+        const int row = rt * ROWS + warp + 8 * i;
         if (valid > 0 && row < M) {
             const T* xr = x + (int64_t)row * ldx;
             load_unit8<T, SHIFT>(xr + col, xr + K, valid, raw[i]);
@@ -143,8 +145,8 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
         }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int row = rt * kTileRows + warp + 8 * i;
+    for (int i = 0; i < RPW; ++i) {
+        const int row = rt * ROWS + warp + 8 * i;
         float v[8];
         float amax = 0.0f;
         if constexpr (sizeof(T) == 4) {
@@ -167,9 +169,9 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
         if ((lane % LPB) == 0) s_scale[lane / LPB][warp + 8 * i] = amax;
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < BPT * kTileRows; t += kThreads) {
-        const int j = t / kTileRows, r = t % kTileRows;
-        const int jb = ct * BPT + j, row = rt * kTileRows + r;
+    for (int t = threadIdx.x; t < BPT * ROWS; t += kThreads) {
+        const int j = t / ROWS, r = t % ROWS;
+        const int jb = ct * BPT + j, row = rt * ROWS + r;
         if (jb < nb && row < M) s[(int64_t)jb * M + row] = s_scale[j][r];
     }
 }
@@ -620,14 +622,19 @@ int quantize_rowwise_t(const T* x, int64_t ldx, int8_t* q, int64_t ldq, float* s
         }
     }
     // Any input alignment, as long as the int8 rows are 8-byte aligned and their pitch covers a lane's last eight elements.
-    const int64_t row_tiles = (M + kTileRows - 1) / kTileRows, ctiles = (K + 255) / 256;
+    const int64_t ctiles = (K + 255) / 256;
+    const bool few = ((M + 31) / 32) * ctiles < 2ll * device_info().sms;
+    const int64_t row_tiles = few ? (M + 7) / 8 : (M + 31) / 32;
     if (small && block_ok && ldq % 8 == 0 && aligned(q, 8) && row_tiles * ctiles < (1ll << 31)) {
         const bool straight = K % 8 == 0 && aligned(x, 16) && (ldx * (int64_t)sizeof(T)) % 16 == 0;
-        const unsigned grid = (unsigned)(row_tiles * ctiles);
-#define BI8_QROW(BB)                                                                                                                                \
-    if (block == BB)                                                                                                                                \
-        return straight ? launch_chained(quantize_rowwise_vec_kernel<T, BB, false>, grid, kThreads, 0, st, x, ldx, q, ldq, s, (int)M, (int)K, (int)nb, (int)ctiles) \
-                        : launch_chained(quantize_rowwise_vec_kernel<T, BB, true>, grid, kThreads, 0, st, x, ldx, q, ldq, s, (int)M, (int)K, (int)nb, (int)ctiles);
+        auto launch = [&](auto kernel) {
+            return launch_chained(kernel, (unsigned)(row_tiles * ctiles), kThreads, 0, st, x, ldx, q, ldq, s, (int)M, (int)K, (int)nb, (int)ctiles);
+        };
+#define BI8_QROW(BB)                                                                                                              \
+    if (block == BB && few)                                                                                                       \
+        return straight ? launch(quantize_rowwise_vec_kernel<T, BB, false, 1>) : launch(quantize_rowwise_vec_kernel<T, BB, true, 1>); \
+    if (block == BB)                                                                                                              \
+        return straight ? launch(quantize_rowwise_vec_kernel<T, BB, false, 4>) : launch(quantize_rowwise_vec_kernel<T, BB, true, 4>);
         BI8_QROW(32) BI8_QROW(64) BI8_QROW(128) BI8_QROW(256)
 #undef BI8_QROW
     }

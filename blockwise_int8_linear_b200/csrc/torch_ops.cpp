@@ -481,29 +481,70 @@ at::ScalarType config_dtype() {          // with the interpreter lock
     return t;
 }
 
-// One blocking of a weight, from the cache dict under `key` or by `make` (then put into the cache, if there is one).
-template <typename Make>
-Quantized cached_weight(PyObject* cache, const char* key, Make make) {
-    if (!cache) return make();
-    {
-        pybind11::gil_scoped_acquire gil;
-        PyObject* hit = PyDict_GetItemString(cache, key);
-        if (hit && PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 2)
-            return {THPVariable_Unpack(PyTuple_GET_ITEM(hit, 0)), THPVariable_Unpack(PyTuple_GET_ITEM(hit, 1))};
+// A quantized matrix as the kernels see it: int8 rows with pitch ld, block scales [blocks, rows].
+struct QRef {
+    int8_t* q = nullptr;
+    float* s = nullptr;
+    int64_t rows = 0, cols = 0, ld = 0;
+};
+
+// Where a quantized [rows, cols] lies in one allocation of the call, and the reference to it once that exists.  The training
+// passes keep no tensor of an intermediate result: one allocation per pass instead of two per quantization.
+struct QPlan {
+    int64_t rows = 0, cols = 0, q_at = 0, s_at = 0;
+    QPlan() = default;
+    QPlan(Carve& c, int64_t rows_, int64_t cols_, int64_t block) : rows(rows_), cols(cols_) {
+        q_at = c.take(rows * pitch16(cols));
+        s_at = c.take(ceil_div(cols, block) * rows * 4);
     }
-    const Quantized r = make();
+    QRef in(void* mem) const {
+        char* m = static_cast<char*>(mem);
+        return {reinterpret_cast<int8_t*>(m + q_at), reinterpret_cast<float*>(m + s_at), rows, cols, pitch16(cols)};
+    }
+};
+
+QRef ref_of(const Quantized& r) {
+    return {static_cast<int8_t*>(r.q.data_ptr()), static_cast<float*>(r.s.data_ptr()), r.q.size(0), r.q.size(1),
+            r.q.size(0) > 1 ? r.q.stride(0) : pitch16(r.q.size(1))};
+}
+
+void rowwise_into(const Mat& m, int code, int64_t block, const QRef& r, void* stream) {
+    check(bi8_quantize_rowwise_pitched(m.ptr, code, m.ld, r.q, r.ld, r.s, m.rows, m.cols, (int)block, stream), "bi8_quantize_rowwise");
+}
+void colwise_into(const Mat& m, int code, int64_t block, const QRef& r, void* stream) {
+    check(bi8_quantize_colwise_pitched(m.ptr, code, m.ld, r.q, r.ld, r.s, m.rows, m.cols, (int)block, stream), "bi8_quantize_colwise");
+}
+void dual_into(const Mat& m, int code, int64_t block, const QRef& row, const QRef& col, void* stream) {
+    check(bi8_quantize_dual_pitched(m.ptr, code, m.ld, row.q, row.ld, row.s, col.q, col.ld, col.s, m.rows, m.cols, (int)block, stream), "bi8_quantize_dual");
+}
+// out = a b^T (+ bias); `ws` of at least bi8_gemm_workspace_bytes
+void gemm_into(const QRef& a, const QRef& b, const Bias* bias, int64_t block, const Tensor& out, void* ws, size_t ws_bytes, void* stream) {
+    check(bi8_gemm_dequant(a.q, a.ld, b.q, b.ld, a.s, b.s, bias ? bias->ptr : nullptr, bias ? bias->code : 0, out.data_ptr(), b.rows,
+                           dtype_code(out.scalar_type()), a.rows, b.rows, a.cols, (int)block, ws_bytes ? ws : nullptr, ws_bytes, 0, stream),
+          "bi8_gemm_dequant");
+}
+
+// One blocking of a weight from the cache dict under `key`, or undefined tensors.
+Quantized cache_get(PyObject* cache, const char* key) {
+    if (!cache) return {};
     pybind11::gil_scoped_acquire gil;
-    PyObject* pair = PyTuple_Pack(2, THPVariable_Wrap(r.q), THPVariable_Wrap(r.s));
+    PyObject* hit = PyDict_GetItemString(cache, key);
+    if (hit && PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 2)
+        return {THPVariable_Unpack(PyTuple_GET_ITEM(hit, 0)), THPVariable_Unpack(PyTuple_GET_ITEM(hit, 1))};
+    return {};
+}
+void cache_put(PyObject* cache, const char* key, const Quantized& r) {
+    pybind11::gil_scoped_acquire gil;
+    PyObject* pair = PyTuple_New(2);
     if (!pair) throw python_error();
-    Py_DECREF(PyTuple_GET_ITEM(pair, 0));        // the tuple holds the only references
-    Py_DECREF(PyTuple_GET_ITEM(pair, 1));
+    PyTuple_SET_ITEM(pair, 0, THPVariable_Wrap(r.q));
+    PyTuple_SET_ITEM(pair, 1, THPVariable_Wrap(r.s));
     const int rc = PyDict_SetItemString(cache, key, pair);
     Py_DECREF(pair);
     if (rc != 0) throw python_error();
-    return r;
 }
 
-Tensor rows_2d(const Tensor& t) { return t.dim() == 2 ? t : t.reshape({-1, t.size(-1)}); }
+Tensor as_bytes(const Tensor& like, int64_t bytes) { return empty_on(like, {std::max<int64_t>(bytes, 1)}, at::kByte); }
 
 using torch::autograd::Node;
 using torch::autograd::SavedVariable;
@@ -511,7 +552,7 @@ using torch::autograd::variable_list;
 
 // Backward of y = x W^T + bias with both GEMMs in blockwise int8 (block_linear.py:85-112 in the reference).
 struct LinearBackward : public Node {
-    SavedVariable x, x_state;            // x as its column-wise int8 copy and scales, or x itself (x_state then empty)
+    SavedVariable x;                     // x itself, or (x_quantized) the bytes of its column-wise int8 copy and scales
     SavedVariable weight;
     bool x_quantized = false, has_bias = false, fuse_dual = true;
     int64_t block = 0;
@@ -528,7 +569,6 @@ struct LinearBackward : public Node {
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);
         x.reset_data();
-        x_state.reset_data();
         weight.reset_data();
     }
     variable_list apply(variable_list&& grads) override;
@@ -551,30 +591,70 @@ variable_list LinearBackward::apply(variable_list&& grads) {
         auto self = getptr();
         const Tensor saved_x = x.unpack(self), w = weight.unpack(self);
         at::AutoDispatchBelowADInplaceOrView below_autograd;
-        const Tensor g = rows_2d(grads[0]);
-        const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1);
-        Quantized g_row, g_col;
-        if (need_x && need_w && fuse_dual) {
-            // G is needed blocked along N (for dX) and along the tokens (for dW): one read
-            Dual d = quantize_dual(g, b);
-            g_row = d.row;
-            g_col = d.col;
-        } else if (need_x) {
-            g_row = quantize_rowwise(g, b);
+        const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1), need_b = has_bias && task_should_compute_output(2);
+        need_cuda(grads[0]);
+        OnDevice on(grads[0]);
+        const Mat g = mat_rows(grads[0]), wm = mat2d(w);
+        const int g_code = dtype_code(grads[0].scalar_type()), w_code = dtype_code(w.scalar_type());
+        const int64_t m = g.rows, n = g.cols, k = wm.cols;
+        Mat xm;
+        if (need_w && !x_quantized) xm = mat_rows(saved_x);
+
+        // every intermediate result of this pass lies in one allocation
+        const Quantized cached = need_x ? cache_get(cache, "col") : Quantized{};
+        Quantized fresh;                                     // the weight's other blocking, where the cache is to keep it
+        const size_t ws_x = need_x ? bi8_gemm_workspace_bytes(m, k, n, (int)b) : 0, ws_w = need_w ? bi8_gemm_workspace_bytes(n, k, m, (int)b) : 0,
+                     ws_b = need_b ? bi8_column_sum_workspace_bytes(m, n) : 0;
+        Carve carve;
+        const int64_t ws_at = carve.take((int64_t)std::max({ws_x, ws_w, ws_b}));
+        QPlan g_row, g_col, w_col, x_col;
+        if (need_x) g_row = QPlan(carve, m, n, b);
+        if (need_w) g_col = QPlan(carve, n, m, b);
+        if (need_x && !cached.q.defined() && !cache) w_col = QPlan(carve, k, n, b);
+        if (need_w && x_quantized) {
+            Carve kept;
+            x_col = QPlan(kept, k, m, b);                    // the layout in which train_linear saved it
+        } else if (need_w) {
+            x_col = QPlan(carve, k, m, b);
         }
+        const Tensor mem = as_bytes(grads[0], carve.bytes);
+        void* const base = mem.data_ptr();
+        void* const ws = static_cast<char*>(base) + ws_at;
+        void* const st = on.raw();
+
+        const bool dual = need_x && need_w && fuse_dual;     // G is needed in both blockings: one read
+        if (dual) dual_into(g, g_code, b, g_row.in(base), g_col.in(base), st);
+        else if (need_x) rowwise_into(g, g_code, b, g_row.in(base), st);
         if (need_x) {
             // contraction over N, both operands blocked along N (block_linear.py:92-95).  A cached blocking is still valid:
             // unpacking the weight raised if it was modified since the forward pass.
-            const Quantized wt = cached_weight(cache, "col", [&] { return quantize_colwise(w, b); });
-            out[0] = gemm(g_row.q, wt.q.t(), g_row.s, wt.s, Tensor(), b, type, 0).view(x_sizes);
+            QRef wt;
+            if (cached.q.defined()) {
+                wt = ref_of(cached);
+            } else if (cache) {
+                fresh = Quantized{empty_q(w, k, n), empty_on(w, {ceil_div(n, b), k}, at::kFloat)};
+                wt = ref_of(fresh);
+                colwise_into(wm, w_code, b, wt, st);
+                cache_put(cache, "col", fresh);
+            } else {
+                wt = w_col.in(base);
+                colwise_into(wm, w_code, b, wt, st);
+            }
+            out[0] = empty_on(grads[0], x_sizes, type);
+            gemm_into(g_row.in(base), wt, nullptr, b, out[0], ws, ws_x, st);
         }
         if (need_w) {
             // contraction over the tokens, both operands blocked along M (block_linear.py:100-104)
-            const Quantized xt = x_quantized ? Quantized{saved_x, x_state.unpack(self)} : quantize_colwise(rows_2d(saved_x), b);
-            if (!g_col.q.defined()) g_col = quantize_colwise(g, b);
-            out[1] = gemm(g_col.q, xt.q.t(), g_col.s, xt.s, Tensor(), b, type, 0);
+            const QRef xt = x_col.in(x_quantized ? saved_x.data_ptr() : base);
+            if (!x_quantized) colwise_into(xm, dtype_code(saved_x.scalar_type()), b, xt, st);
+            if (!dual) colwise_into(g, g_code, b, g_col.in(base), st);
+            out[1] = empty_on(grads[0], {n, k}, type);
+            gemm_into(g_col.in(base), xt, nullptr, b, out[1], ws, ws_w, st);
         }
-        if (has_bias && task_should_compute_output(2)) out[2] = g.sum(0);
+        if (need_b) {
+            out[2] = empty_on(grads[0], {n}, grads[0].scalar_type());
+            check(bi8_column_sum(g.ptr, g_code, g.ld, out[2].data_ptr(), m, n, ws_b ? ws : nullptr, ws_b, st), "bi8_column_sum");
+        }
     } catch (const PyFail& e) {
         pybind11::gil_scoped_acquire gil;
         PyErr_SetString(e.type, e.text.c_str());
@@ -587,38 +667,64 @@ variable_list LinearBackward::apply(variable_list&& grads) {
 
 // y = x W^T (+ bias), every operand quantized on the fly, recorded for backward when a gradient is wanted.  With `fuse_dual`
 // a layer whose weight is trained reads x once for both of its blockings and keeps the int8 transposed copy instead of x.
-Tensor train_linear(const Tensor& x_in, const Tensor& w, const Tensor& bias, int64_t block, at::ScalarType type, bool fuse_dual, PyObject* cache) {
+Tensor train_linear(const Tensor& x_in, const Tensor& w, const Tensor& bias_in, int64_t block, at::ScalarType type, bool fuse_dual, PyObject* cache) {
     need_cuda(x_in);
     if (x_in.dim() == 0 || w.dim() != 2 || x_in.size(-1) != w.size(1)) assertion("incompatible dimensions");
-    const bool grad = at::GradMode::is_enabled() && (x_in.requires_grad() || w.requires_grad() || (bias.defined() && bias.requires_grad()));
+    const bool grad = at::GradMode::is_enabled() && (x_in.requires_grad() || w.requires_grad() || (bias_in.defined() && bias_in.requires_grad()));
     std::shared_ptr<LinearBackward> node;
     if (grad) {
         node = std::shared_ptr<LinearBackward>(new LinearBackward(), torch::autograd::deleteNode);
-        node->set_next_edges(torch::autograd::collect_next_edges(x_in, w, bias));
+        node->set_next_edges(torch::autograd::collect_next_edges(x_in, w, bias_in));
     }
     Tensor out;
     {
         at::AutoDispatchBelowADInplaceOrView below_autograd;
-        const Tensor x = rows_2d(x_in);
-        Quantized xq;
-        if (node && w.requires_grad() && fuse_dual) {
-            Dual d = quantize_dual(x, block);
-            xq = d.row;
-            node->x = SavedVariable(d.col.q, false);
-            node->x_state = SavedVariable(d.col.s, false);
+        OnDevice on(x_in);
+        const Mat x = mat_rows(x_in), wm = mat2d(w);
+        const int x_code = dtype_code(x_in.scalar_type()), w_code = dtype_code(w.scalar_type());
+        const int64_t m = x.rows, n = wm.rows, k = wm.cols;
+        const bool keep = node && w.requires_grad() && fuse_dual;
+        const Quantized cached = cache_get(cache, "row");
+        Quantized fresh;
+        const size_t ws_bytes = bi8_gemm_workspace_bytes(m, n, k, (int)block);
+        Carve carve, kept;
+        const int64_t ws_at = carve.take((int64_t)ws_bytes);
+        const QPlan x_row(carve, m, k, block), x_col = keep ? QPlan(kept, k, m, block) : QPlan();
+        const QPlan w_row = !cached.q.defined() && !cache ? QPlan(carve, n, k, block) : QPlan();
+        const Tensor mem = as_bytes(x_in, carve.bytes);
+        void* const base = mem.data_ptr();
+        void* const st = on.raw();
+        const QRef xq = x_row.in(base);
+        if (keep) {
+            const Tensor saved = as_bytes(x_in, kept.bytes);
+            dual_into(x, x_code, block, xq, x_col.in(saved.data_ptr()), st);
+            node->x = SavedVariable(saved, false);
             node->x_quantized = true;
         } else {
-            xq = quantize_rowwise(x, block);
+            rowwise_into(x, x_code, block, xq, st);
         }
-        const Quantized wq = cached_weight(cache, "row", [&] { return quantize_rowwise(w, block); });
+        QRef wq;
+        if (cached.q.defined()) {
+            wq = ref_of(cached);
+        } else if (cache) {
+            fresh = Quantized{empty_q(w, n, k), empty_on(w, {ceil_div(k, block), n}, at::kFloat)};
+            wq = ref_of(fresh);
+            rowwise_into(wm, w_code, block, wq, st);
+            cache_put(cache, "row", fresh);
+        } else {
+            wq = w_row.in(base);
+            rowwise_into(wm, w_code, block, wq, st);
+        }
+        const Bias bias(bias_in, n);
         c10::SmallVector<int64_t, 6> shape(x_in.sizes().begin(), x_in.sizes().end());
-        shape.back() = w.size(0);
-        out = gemm(xq.q, wq.q.t(), xq.s, wq.s, bias, block, type, 0).view(shape);
+        shape.back() = n;
+        out = empty_on(x_in, shape, type);
+        gemm_into(xq, wq, bias.ptr ? &bias : nullptr, block, out, static_cast<char*>(base) + ws_at, ws_bytes, st);
     }
     if (node) {
         if (!node->x_quantized) node->x = SavedVariable(x_in, false);
         node->weight = SavedVariable(w, false);
-        node->has_bias = bias.defined();
+        node->has_bias = bias_in.defined();
         node->fuse_dual = fuse_dual;
         node->block = block;
         node->x_sizes = x_in.sizes().vec();

@@ -95,6 +95,13 @@ BI8_API int bi8_quantize_dual(const void* x, int x_dtype, int64_t ldx, int8_t* q
 BI8_API int bi8_dequantize_rowwise(const int8_t* q, const float* s, void* out, int out_dtype,
                            int64_t M, int64_t K, int block, void* stream);
 
+/* Sum over the rows of x [R,C] (row stride ldx): out [C] of x's type, fp32 accumulation in a fixed order; the bias gradient of a
+ * layer (G.sum(dim=0), block_linear.py:105-106).  workspace: bi8_column_sum_workspace_bytes(R,C) bytes of scratch, may be NULL
+ * (slower). */
+BI8_API int bi8_column_sum(const void* x, int dtype, int64_t ldx, void* out, int64_t R, int64_t C, void* workspace,
+                           size_t workspace_bytes, void* stream);
+BI8_API size_t bi8_column_sum_workspace_bytes(int64_t R, int64_t C);
+
 /* Replaces int8_matmul_block64_rowwise_dequantize (triton_functions.py:142-168, kernel 69-139).
  *   C[m,n] = cast( sum_j  sB[j,n] * sA[j,m] * float(P_j[m,n]) / 127^2 )  (+ cast(bias[n]) in the output type)
  *   P_j = A[:, j*block:(j+1)*block] . Bt[:, j*block:(j+1)*block]^T   exactly, in int32.
