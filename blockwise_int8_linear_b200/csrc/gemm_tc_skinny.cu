@@ -68,7 +68,7 @@ struct SkGeo {
     static constexpr int PROMO_WARPS = 4 * CHUNKS;
     static constexpr int VB = BPS * CW <= 32 ? BPS : 32 / CW;      // blocks whose accumulators a promotion thread loads at once
     static constexpr int ACC_STRIDE = BPS * BNS;          // tensor-memory columns of one stage's accumulators
-    static constexpr int NBUF = (512 / ACC_STRIDE) < 4 ? (512 / ACC_STRIDE) : 4;
+    static constexpr int NBUF = (512 / ACC_STRIDE) < 4 || STAGES < 4 ? 2 : 4;     // no more than there are stages: see the MMA issuers
     static constexpr int MMA_WARPS = 2;                   // MMA issuers, taking the stages in turn
     static constexpr int THREADS = (PROMO_WARPS + 1 + MMA_WARPS + (SRC != 0 ? kHelpWarps : 0)) * 32;
     static constexpr int TMEM_COLS = pow2_at_least(NBUF * ACC_STRIDE);
@@ -522,17 +522,21 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
         // Issuing the MMAs of a stage, the commit and the polls of its two barriers cost one thread several hundred cycles, so
         // MMA_WARPS warps take the stages in turn.
         static_assert(G::MMA_WARPS <= G::STAGES, "an issuer advances by at most one turn of the stage ring");
+        static_assert(G::STAGES % G::MMA_WARPS == 0 || G::NBUF <= G::STAGES, "see the waits below");
         constexpr uint32_t idesc = umma_idesc_i8(kTileRows, BNS);
         const int me = warp - MW;
         int buf = me, stage = me, ks = me;                   // ks: stage inside this CTA's share
         while (len > 0 && ks >= len) ks -= len;
         uint32_t phase = 0, accphase = 0;
         for (int s = me; s < my_stages; s += G::MMA_WARPS) {
-            // operands landed and an accumulator range is free: one vote for both
-            const bool got_ab = mbar_wait(bar(G::FULL_AB + stage), phase, abort_flag);
-            const bool got_acc = got_ab && mbar_wait(bar(G::ACC_EMPTY + buf), accphase ^ 1u, abort_flag);
-            if (!__all_sync(0xffffffffu, got_acc)) {
-                if (lane == 0) report_timeout(p.status, abort_flag, got_ab ? W_ACC_EMPTY : W_FULL_AB);
+            // An accumulator range is free, then the operands have landed: one vote for both.  The order matters where the number of
+            // stages is odd and a stage's uses alternate between the issuers: a parity wait also succeeds while the use before
+            // the awaited one is still under way, and that use is known to be over only because its accumulators (at most
+            // NBUF <= STAGES uses back) have been read.
+            const bool got_acc = mbar_wait(bar(G::ACC_EMPTY + buf), accphase ^ 1u, abort_flag);
+            const bool got_ab = got_acc && mbar_wait(bar(G::FULL_AB + stage), phase, abort_flag);
+            if (!__all_sync(0xffffffffu, got_ab)) {
+                if (lane == 0) report_timeout(p.status, abort_flag, got_acc ? W_FULL_AB : W_ACC_EMPTY);
                 break;
             }
             tc_fence_after();

@@ -111,3 +111,18 @@ def test_bias_and_residual_behind_the_general_gemm(m, k, n, dt):
             assert torch.equal(got, base + res)
     assert_clean_device()
     set_config(64)
+
+
+@pytest.mark.parametrize("m", [2, 20, 40, 64])
+def test_decode_gemm_with_weights_arriving_late(m):
+    """Weights that no cache or address translation holds yet arrive out of order: the first product with them equals the later ones."""
+    tf = _tf()
+    set_config(64)
+    xq, sx = tf.quantize_block_rowwise(randn_bf16((m, 11008), m).to(DEV))
+    gen = torch.Generator(device=DEV).manual_seed(m)
+    for _ in range(12):
+        wq, sw = tf.quantize_block_rowwise(torch.randn((4096, 11008), generator=gen, device=DEV, dtype=torch.bfloat16))
+        torch.randn((1 << 26,), device=DEV)
+        first = tf.int8_matmul_block64_rowwise_dequantize(xq, wq.t(), sx, sw)
+        assert torch.equal(first, tf.int8_matmul_block64_rowwise_dequantize(xq, wq.t(), sx, sw))
+    assert_clean_device()
