@@ -2,7 +2,7 @@
 // the reference, where torch sums).
 //
 // Bound by reading x once (from L2 where the gradient's quantizer has just read it).  A CTA takes 128 columns (16 threads x 8
-// columns, one 16-byte load of a 16-bit row each; two for fp32) of a range of rows, 16 rows at a time, four steps of loads in
+// columns, one 16-byte load of a 16-bit row each; two for fp32) of a range of rows, 16 rows at a time, eight steps of loads in
 // flight; the row lanes meet in shared memory in a fixed order.  There are as many row ranges as fill the device;
 // their fp32 sums go to a workspace and a second kernel adds them in ascending order, so the result does not depend on
 // scheduling.  (torch's reduction over the leading dimension: 29 us for 8192 x 3072 bf16, 8 us of host time per call.)
@@ -69,22 +69,24 @@ __global__ void __launch_bounds__(kSumThreads) column_sum_kernel(const void* __r
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = 0.0f;
     if (live > 0) {
-        for (int r = r0 + lane; r < r1; r += kSumLanes * 4) {
-            float f[4][8];
+        constexpr int STEPS = 8;
+        int r = r0 + lane;
+        if (vec && live >= 8) {
+            for (; r + (STEPS - 1) * kSumLanes < r1; r += kSumLanes * STEPS) {      // no test between the loads
+                float f[STEPS][8];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int rr = r + u * kSumLanes;
-                if (rr < r1) {
-                    sum_load8<DT>(f[u], x, (int64_t)rr * ldx + c0, live, vec != 0);
-                } else {
+                for (int u = 0; u < STEPS; ++u) sum_load8<DT>(f[u], x, (int64_t)(r + u * kSumLanes) * ldx + c0, 8, true);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) f[u][e] = 0.0f;
-                }
+                for (int u = 0; u < STEPS; ++u)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[e] += f[u][e];
             }
+        }
+        for (; r < r1; r += kSumLanes) {
+            float f[8];
+            sum_load8<DT>(f, x, (int64_t)r * ldx + c0, live, vec != 0);
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[e] += f[u][e];
+            for (int e = 0; e < 8; ++e) acc[e] += f[e];
         }
     }
 #pragma unroll
@@ -115,11 +117,11 @@ __global__ void __launch_bounds__(128) column_sum_finish_kernel(const float* __r
     sum_store(out, dt, c, v);
 }
 
-// Row ranges: enough CTAs for four per SM, but at least 64 rows each, so that a range is a few steps of loads.
+// Row ranges: enough CTAs for four per SM, but at least 128 rows each, one batch of loads.
 int row_ranges(int64_t R, int64_t C, int sms) {
     const int64_t ctiles = (C + kSumCols - 1) / kSumCols;
     int64_t n = (4ll * sms + ctiles - 1) / ctiles;
-    if (n > (R + 63) / 64) n = (R + 63) / 64;
+    if (n > (R + 127) / 128) n = (R + 127) / 128;
     if (n > 128) n = 128;
     return n < 1 ? 1 : (int)n;
 }

@@ -126,3 +126,23 @@ def test_decode_gemm_with_weights_arriving_late(m):
         first = tf.int8_matmul_block64_rowwise_dequantize(xq, wq.t(), sx, sw)
         assert torch.equal(first, tf.int8_matmul_block64_rowwise_dequantize(xq, wq.t(), sx, sw))
     assert_clean_device()
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,n", [(1, 1), (127, 129), (128, 128), (129, 1001), (4000, 7), (2049, 520)])
+def test_bias_gradient_is_the_column_sum(rows, n, dt):
+    """Batches of loads and the rows behind them, columns of a last tile, rows of any alignment; the same bits each time."""
+    from block_linear import BlockInt8Linear
+    set_config(64, dt)
+    lin = BlockInt8Linear(64, n, True, device=DEV, dtype=dt).train()
+    x, g = randn_bf16((1, rows, 64), rows).to(dt).to(DEV), randn_bf16((1, rows, n), n, outliers=0).to(dt).to(DEV)
+    lin(x).backward(g)
+    want = g[0].double().sum(0)
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -23}[dt]
+    bound = eps * want.abs() + rows * 2.0 ** -23 * g[0].double().abs().sum(0) + 1e-12
+    assert ((lin.bias.grad.double() - want).abs() <= bound).all()
+    first = lin.bias.grad.clone()
+    lin.bias.grad = None
+    lin(x).backward(g)
+    assert torch.equal(first, lin.bias.grad)
+    set_config(64)
