@@ -233,6 +233,20 @@ __device__ __forceinline__ void fold_columns(const uint32_t (&S)[NC], uint32_t s
     }
 }
 
+// One whole 32-byte sector of a split-K part to and from L2.  As two 16-byte accesses each of a warp's 32 sectors crosses the
+// L1-L2 path twice: 1.6 us per call on the storing side, 3-5 us on the loading side.
+__device__ __forceinline__ void stg_v8(float* dst, const float (&f)[8]) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]), "f"(f[4]), "f"(f[5]),
+                 "f"(f[6]), "f"(f[7])
+                 : "memory");
+}
+__device__ __forceinline__ void ldcg_v8(float (&f)[8], const float* src) {
+    asm volatile("ld.global.cg.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7])
+                 : "l"(src)
+                 : "memory");
+}
+
 // Place of (lane quarter, column slice, group of eight columns, row of the quarter) in a workspace slot: a warp stores 1 KiB
 // runs, a thread 32 bytes of its row, and the reduction kernel reads a row's eight columns as one sector.
 template <int PW, int COLS>
@@ -287,11 +301,16 @@ __device__ __forceinline__ void add_staged(const TcParams& p, uint32_t row_addr,
     const int per = wide ? 4 : 8;                       // elements of a 16-byte piece
     const int left = p.N - col0;
     if (p.bias != nullptr) {
+        // one load per lane for the columns of the warp, handed round by shuffles: a load per column and piece was
+        // 0.7 us of latency five times (ten for fp32 outputs) per tile
+        const int lane = (int)(threadIdx.x & 31u);
+        const float b0 = lane < left ? load_as_f32(p.bias, p.bias_dtype, col0 + lane) : 0.0f;
+        const float b1 = lane + 32 < left && lane + 32 < COLS ? load_as_f32(p.bias, p.bias_dtype, col0 + lane + 32) : 0.0f;
 #pragma unroll 1
         for (int g = 0; g < COLS / 8; ++g)
             add_piece(row_addr + (uint32_t)(g * 16), wide, bf, [&](int e) {
                 const int n = g * per + e;
-                return n < left ? load_as_f32(p.bias, p.bias_dtype, col0 + n) : 0.0f;
+                return __shfl_sync(0xffffffffu, n < 32 ? b0 : b1, n & 31);
             });
     }
     if (p.residual != nullptr && m < p.M) {
@@ -664,9 +683,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     float v[8];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) unpack_f32x2(acc2[4 * g + u], v[2 * u], v[2 * u + 1]);
-                    float4* d4 = reinterpret_cast<float4*>(dst + g * 256);
-                    d4[0] = make_float4(v[0], v[1], v[2], v[3]);
-                    d4[1] = make_float4(v[4], v[5], v[6], v[7]);
+                    stg_v8(dst + g * 256, v);
                 }
             } else if (MODE == 0) {
                 // The tile leaves through the warp's staging area in shared memory: every lane writes its row's share
@@ -793,16 +810,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 // Reduction of the divided tiles: C[m,n] = cast(sum over the tile's parts) (+ cast(bias[n])) (+ residual[m,n]), the parts added
 // in ascending order, so that the result does not depend on scheduling.  A thread takes eight consecutive columns of
-// a row: one 32-byte sector of every part (eight parts in flight), one 16-byte store (two for fp32) where C allows it.
+// a row: one 32-byte sector of every part (NP parts in flight: no more registers than the parts
+// need; four neighbouring threads take the four rows of a 128-byte line), one 16-byte store (two for fp32) where C allows it.
 // The parts are at most one slot per SM (12 MB) and come from L2.  Launched as a programmatic dependent of the GEMM:
 // its CTAs are resident as the GEMM's leave.
-template <int BN, int COLS>
+template <int BN, int COLS, int NP>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const TcParams p) {
     after_predecessor();
     constexpr int GROUPS = BN / 8;                       // groups of eight columns in a tile row
     const int item = blockIdx.x * 256 + threadIdx.x;
     const int t = item / (kBM * GROUPS), rem = item - t * (kBM * GROUPS);
-    const int r = rem / GROUPS, cg = rem - r * GROUPS;   // consecutive threads: consecutive columns of a row
+    const int rb = rem / (GROUPS * 4), x = rem - rb * (GROUPS * 4);
+    const int r = rb * 4 + (x & 3), cg = x >> 2;         // four consecutive threads: the four rows of a 128-byte line of a part
     if (t >= p.tiles_m * p.tiles_n) return;
     int m0, n0;
     tile_coords<BN>(t, p.tiles_m, m0, n0);
@@ -818,21 +837,16 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const TcParams p) {
     const bool has_bias = p.bias != nullptr, has_res = p.residual != nullptr;
     if (has_bias) load8_as_f32(bias, p.bias, p.bias_dtype, n, live);
     if (has_res) load8_as_f32(res, p.residual, p.out_dtype, ro, live);
-    for (int s0 = 0; s0 < p.ksplit; s0 += 8) {
-        float4 v[8][2];
+    for (int s0 = 0; s0 < p.ksplit; s0 += NP) {
+        float v[NP][8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
+        for (int q = 0; q < NP; ++q)
+            if (s0 + q < p.ksplit) ldcg_v8(v[q], src + (int64_t)(s0 + q) * p.slot_floats);
+#pragma unroll
+        for (int q = 0; q < NP; ++q)
             if (s0 + q < p.ksplit) {
-                const float4* s4 = reinterpret_cast<const float4*>(src + (int64_t)(s0 + q) * p.slot_floats);
-                v[q][0] = __ldcg(s4);
-                v[q][1] = __ldcg(s4 + 1);
-            }
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-            if (s0 + q < p.ksplit) {
-                const float f[8] = {v[q][0].x, v[q][0].y, v[q][0].z, v[q][0].w, v[q][1].x, v[q][1].y, v[q][1].z, v[q][1].w};
-#pragma unroll
-                for (int u = 0; u < 8; ++u) acc[u] = __fadd_rn(acc[u], f[u]);
+                for (int u = 0; u < 8; ++u) acc[u] = __fadd_rn(acc[u], v[q][u]);
             }
     }
     if (p.out_dtype == BI8_F32) {
@@ -960,9 +974,11 @@ struct SplitPlan {
     int slot_floats = 0;
     size_t bytes = 0;
 };
-// A stage (128 K-bytes of a tile) takes about 0.8 us; dividing costs the second kernel and the workspace's round trip,
-// 2.5-4 us: tiles are divided only where each gets at least this many stages shorter.
-constexpr int kSplitGain = 4;
+// What a work item takes per stage (128 K-bytes of a tile), what dividing costs whatever its size (the second kernel's latency; of
+// its host time a part) and per slot (80 KB written and read again through L2): microseconds, fitted to a sweep of 1 to 32 items per
+// tile over 12 shapes of 7 to 69 tiles and 2 to 86 stages.  The number of items with the lowest sum is taken; the largest that
+// the SMs hold is often not the fastest (512 x 768 x 768: 8.4 us in 6 items, 8.1 undivided and a launch less).
+constexpr double kStageUs = 0.72, kSplitUs = 2.9, kSlotUs = 0.017;
 
 SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int sms) {
     SplitPlan pl;
@@ -971,16 +987,20 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int sms) {
     const int nks = (int)((K + kBK - 1) / kBK);
     pl.stages_per_split = nks;
     if (tiles <= 0 || nks <= 1 || tiles * 2 > sms) return pl;
-    int s = (int)(sms / tiles);
-    if (s > nks) s = nks;
-    if (s > 32) s = 32;
-    const int spp = (nks + s - 1) / s;
-    s = (nks + spp - 1) / spp;
-    if (s <= 1 || nks - spp < kSplitGain) return pl;
-    pl.ksplit = s;
-    pl.stages_per_split = spp;
+    const int most = (int)(sms / tiles) < 32 ? (int)(sms / tiles) : 32;
+    double best = kStageUs * nks;
+    for (int want = 2; want <= most && want <= nks; ++want) {
+        const int spp = (nks + want - 1) / want, s = (nks + spp - 1) / spp;
+        const double cost = kStageUs * spp + kSplitUs + kSlotUs * (double)(tiles * s);
+        if (cost < best) {
+            best = cost;
+            pl.ksplit = s;
+            pl.stages_per_split = spp;
+        }
+    }
+    if (pl.ksplit <= 1) return pl;
     pl.slot_floats = (int)((M < kBM ? (M + 31) / 32 * 32 : kBM) * bn);
-    pl.bytes = (size_t)tiles * (size_t)s * (size_t)pl.slot_floats * 4;
+    pl.bytes = (size_t)tiles * (size_t)pl.ksplit * (size_t)pl.slot_floats * 4;
     return pl;
 }
 }  // namespace
@@ -995,7 +1015,7 @@ double gemm_tc_estimate_us(const GemmArgs& g) {
     const DeviceInfo di = device_info();
     const SplitPlan pl = plan_split(g.M, g.N, g.K, di.sms);
     const int64_t tiles = ((g.M + kBM - 1) / kBM) * ((g.N + tc_bn() - 1) / tc_bn()), items = tiles * pl.ksplit;
-    return 0.8 * (double)((items + di.sms - 1) / di.sms * pl.stages_per_split) + (pl.ksplit > 1 ? 10.0 : 3.0);
+    return kStageUs * (double)((items + di.sms - 1) / di.sms * pl.stages_per_split) + 3.5 + (pl.ksplit > 1 ? kSplitUs + kSlotUs * (double)items : 0.0);
 }
 
 bool gemm_tc_applicable(const GemmArgs& g, const char** why) {
@@ -1096,7 +1116,10 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     }
     if (rc != BI8_OK || pl.ksplit == 1) return rc;
     constexpr int kTileItems = kBM * (Cfg<kPW>::BN / 8);
-    return launch_chained(splitk_reduce_kernel<Cfg<kPW>::BN, Cfg<kPW>::COLS>, (unsigned)((tiles * kTileItems + 255) / 256), 256, 0, st, p);
+    auto reduce = [&](auto kernel) { return launch_chained(kernel, (unsigned)((tiles * kTileItems + 255) / 256), 256, 0, st, p); };
+    constexpr int BN = Cfg<kPW>::BN, COLS = Cfg<kPW>::COLS;
+    if (pl.ksplit <= 2) return reduce(splitk_reduce_kernel<BN, COLS, 2>);
+    return pl.ksplit <= 4 ? reduce(splitk_reduce_kernel<BN, COLS, 4>) : reduce(splitk_reduce_kernel<BN, COLS, 8>);
 }
 
 int run_mma_peak_probe(int iters, float* ms, int* sm_count) {
