@@ -159,6 +159,7 @@ struct GemmArgs {
 
 bool gemm_tc_applicable(const GemmArgs& g, const char** why);
 size_t gemm_tc_workspace_bytes(const GemmArgs& g);
+bool gemm_tc_fills_device(const GemmArgs& g);
 int launch_gemm_tc(const GemmArgs& g, cudaStream_t st);
 int launch_gemm_generic(const GemmArgs& g, cudaStream_t st);
 double gemm_tc_estimate_us(const GemmArgs& g);       // few tiles: the time the general kernel takes, for a choice between kernels

@@ -963,10 +963,11 @@ int launch_qb(const TcMaps& tm, const TcParams& p, int grid, bool partials, bool
 
 }  // namespace
 
-// Split-K plan: when the output has at most half as many tiles as the device has SMs (small M), the K stages of every tile
-// are divided over `ksplit` work items so that all SMs work; partial results go to an fp32 workspace, one slot per
-// item, and a second kernel adds them in a fixed order.  (Dividing the tiles left over after the last full round of a larger
-// output as well would make equal rows of A give unequal bits, depending on the tile they lie in.)
+// Split-K plan: the K stages of every tile are divided over `ksplit` work items, where that lets the SMs work for a shorter time:
+// small outputs that have fewer tiles than the device SMs, and outputs whose tiles fill a last round badly (320 long tiles of a
+// weight or input gradient on 148 SMs are three rounds for 2.16 of work).  Partial results go to an fp32 workspace, one slot per
+// item, and a second kernel adds them in a fixed order.  (Dividing only the tiles left over after the last full round
+// would make equal rows of A give unequal bits, depending on the tile they lie in.)
 namespace {
 struct SplitPlan {
     int ksplit = 1;
@@ -979,6 +980,11 @@ struct SplitPlan {
 // tile over 12 shapes of 7 to 69 tiles and 2 to 86 stages.  The number of items with the lowest sum is taken; the largest that
 // the SMs hold is often not the fastest (512 x 768 x 768: 8.4 us in 6 items, 8.1 undivided and a launch less).
 constexpr double kStageUs = 0.72, kSplitUs = 2.9, kSlotUs = 0.017;
+// Where the tiles alone occupy more than half of the SMs, dividing has to save a twentieth, the workspace stays within half of L2, and from
+// kSplitRounds rounds on nothing is left to be saved.
+constexpr double kSplitWorth = 0.95;
+constexpr size_t kSplitBytes = 64u << 20;
+constexpr int kSplitRounds = 6;
 
 SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int sms) {
     SplitPlan pl;
@@ -986,12 +992,15 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int sms) {
     const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
     const int nks = (int)((K + kBK - 1) / kBK);
     pl.stages_per_split = nks;
-    if (tiles <= 0 || nks <= 1 || tiles * 2 > sms) return pl;
-    const int most = (int)(sms / tiles) < 32 ? (int)(sms / tiles) : 32;
-    double best = kStageUs * nks;
-    for (int want = 2; want <= most && want <= nks; ++want) {
+    if (tiles <= 0 || nks <= 1 || tiles > kSplitRounds * sms) return pl;
+    pl.slot_floats = (int)((M < kBM ? (M + 31) / 32 * 32 : kBM) * bn);
+    auto rounds = [&](int64_t items) { return (double)((items + sms - 1) / sms); };
+    const bool fills = tiles * 2 > sms;
+    double best = rounds(tiles) * kStageUs * nks * (fills ? kSplitWorth : 1.0);
+    for (int want = 2; want <= 32 && want <= nks; ++want) {
         const int spp = (nks + want - 1) / want, s = (nks + spp - 1) / spp;
-        const double cost = kStageUs * spp + kSplitUs + kSlotUs * (double)(tiles * s);
+        if (fills ? (size_t)tiles * (size_t)s * (size_t)pl.slot_floats * 4 > kSplitBytes : tiles * want > sms) break;
+        const double cost = rounds(tiles * s) * kStageUs * spp + kSplitUs + kSlotUs * (double)(tiles * s);
         if (cost < best) {
             best = cost;
             pl.ksplit = s;
@@ -999,11 +1008,15 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int sms) {
         }
     }
     if (pl.ksplit <= 1) return pl;
-    pl.slot_floats = (int)((M < kBM ? (M + 31) / 32 * 32 : kBM) * bn);
     pl.bytes = (size_t)tiles * (size_t)pl.ksplit * (size_t)pl.slot_floats * 4;
     return pl;
 }
 }  // namespace
+
+// Whether the undivided tiles occupy more than half of the SMs: a caller without a large workspace does without the split there.
+bool gemm_tc_fills_device(const GemmArgs& g) {
+    return ((g.M + kBM - 1) / kBM) * ((g.N + tc_bn() - 1) / tc_bn()) * 2 > device_info().sms;
+}
 
 size_t gemm_tc_workspace_bytes(const GemmArgs& g) {
     const DeviceInfo di = device_info();

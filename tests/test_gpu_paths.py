@@ -146,3 +146,26 @@ def test_bias_gradient_is_the_column_sum(rows, n, dt):
     lin(x).backward(g)
     assert torch.equal(first, lin.bias.grad)
     set_config(64)
+
+
+@pytest.mark.parametrize("m,k,n", [(1024, 11008, 4096), (2000, 8200, 2001), (8192, 20000, 768)])
+def test_outputs_of_a_few_rounds_are_divided_over_k(m, k, n):
+    """More tiles than half the SMs, a last range of K that is shorter, more parts than one batch of loads: against the undivided
+    kernel, which is what a caller with the small built-in workspace still gets."""
+    from tests.test_zz_no_alloc import _lib
+    lib, L = _lib()
+    gen = torch.Generator(device=DEV).manual_seed(k)
+    ld, nb = (k + 15) // 16 * 16, -(-k // 64)
+    a, bt = (torch.randint(-127, 128, (r, ld), generator=gen, device=DEV, dtype=torch.int8)[:, :k] for r in (m, n))
+    sa, sb = (torch.rand((nb, r), generator=gen, device=DEV) + 0.1 for r in (m, n))
+    tf = _tf()
+    set_config(64)
+    assert L.bi8_gemm_workspace_bytes(m, n, k, 64) > 8 << 20
+    got = tf.int8_matmul_block64_rowwise_dequantize(a, bt.t(), sa, sb).float()
+    c = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+    p = lib.ptr
+    lib.check(L.bi8_gemm_dequant_static(p(a), ld, p(bt), ld, p(sa), p(sb), None, 0, p(c), n, 0, m, n, k, 64, 0, lib.stream_ptr()), "static")
+    want = c.float()
+    assert ((got - want).norm() / want.norm()).item() <= 5e-3
+    assert (got - want).abs().max().item() <= 2.0 ** -7 * want.abs().max().item()
+    assert_clean_device()
