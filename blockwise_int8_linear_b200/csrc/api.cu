@@ -102,12 +102,11 @@ int dispatch_gemm(const GemmArgs& g, cudaStream_t st) {
 }
 
 // Where a decode-sized layer quantizes its activations: inside the GEMM (one launch; every cluster repeats the work and the weights
-// wait for the predecessor) or in a kernel in front of it (weights and quantizer overlap).  Inside up to this many
-// activation values: measured on layers of a decode step, 3 x 2048: 37 us a layer against 47, 1 x 4096: 61 against 65, but 8 x
-// 4096: 78 against 71 and 16 x 2560: 54 against 49.  A plain call by itself is bound by its launches and always
-// gains up to 16 rows (16 x 4096 -> 4096: 9.8 us against 11.5).
+// wait for the predecessor) or in a kernel in front of it (weights and quantizer overlap).  In a chain of steps inside up to
+// this many values: 3 x 2048: 37 us a layer against 47, 1 x 4096: 61 against 65, but 8 x 4096: 78 against 71.  A plain call by itself
+// is bound by its launches as long as a CTA's part is no longer than that: inside against in front, 16 x 4096 -> 4096 (16384
+// values a CTA) 11.4 us, 13.9; 8 x 4096 -> 11008 (32768) 19.4, 15.6; 16 x 5120 -> 13824 (81920) 33, 20.
 constexpr int64_t kQuantInKernelValues = 16384;
-constexpr int64_t kQuantInKernelRows = 16;
 
 // Decode-sized layer (the weight-streaming GEMM and what produces its activations).  `g` describes the GEMM on the
 // quantized activations g.A / g.sA, which are scratch (null: none); `alone`: a plain call, not a step with a producer or a
@@ -124,7 +123,8 @@ int launch_decode(GemmArgs g, bool alone, int op, const void* x, const void* x2,
     in.X2 = op == BI8_PRE_SILU_MUL ? x2 : op == BI8_PRE_RMSNORM ? norm_weight : nullptr;
     in.eps = eps;
     const bool scratch = g.A != nullptr && g.sA != nullptr;
-    const bool want_in = (g.M <= kQuantInKernelRows && (alone || g.M * g.K <= kQuantInKernelValues)) || (g.flags & BI8_GEMM_QUANT_IN_KERNEL) || !scratch;
+    const bool forced_in = (g.flags & BI8_GEMM_QUANT_IN_KERNEL) || !scratch;
+    const bool want_in = forced_in || (g.M <= 16 && (g.M * g.K <= kQuantInKernelValues || (alone && gemm_skinny_part(in) <= kQuantInKernelValues)));
     if (want_in && !(op == BI8_PRE_SILU_MUL && !x2) && gemm_skinny_applicable(in)) return launch_gemm_skinny(in, st);
     if (!scratch || g.K % 16 != 0 || !aligned(g.A, 16) || !gemm_skinny_preferred(g)) {
         *done = false;

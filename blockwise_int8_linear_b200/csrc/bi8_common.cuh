@@ -164,6 +164,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st);
 int launch_gemm_generic(const GemmArgs& g, cudaStream_t st);
 double gemm_tc_estimate_us(const GemmArgs& g);       // few tiles: the time the general kernel takes, for a choice between kernels
 bool gemm_skinny_applicable(const GemmArgs& g);
+int64_t gemm_skinny_part(const GemmArgs& g);
 bool gemm_skinny_preferred(const GemmArgs& g);
 int launch_gemm_skinny(const GemmArgs& g, cudaStream_t st);
 int launch_skinny_quantize(const void* x, int x_dtype, int64_t ldx, int8_t* q, float* sx, int64_t M, int64_t K, int block,

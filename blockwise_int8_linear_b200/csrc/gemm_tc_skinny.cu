@@ -1036,6 +1036,13 @@ bool gemm_skinny_applicable(const GemmArgs& g) {
     return plan_launch(g, di.sms, &l) == BI8_OK && l.smem != 0;
 }
 
+// Activation values that a CTA quantizes where the kernel does it itself.
+int64_t gemm_skinny_part(const GemmArgs& g) {
+    SkLaunch l;
+    if (!skinny_shape_ok(g.M, g.N, g.K, g.block) || plan_launch(g, device_info().sms, &l) != BI8_OK || l.plan.cluster == 0) return INT64_MAX;
+    return g.M * ((g.K + l.plan.cluster - 1) / l.plan.cluster);
+}
+
 // Whether this kernel is also the faster one.  Up to 32 rows it always is.  From 33 on its promotion costs as much as the weights
 // take to arrive, and the general kernel overtakes it where it fills the SMs (clearly: a small layer keeps the reference's order of
 // operations): estimates in microseconds, from a sweep at 64 rows (4096 x 22016: 29 general, 45 here; x 11008: 23, 27; x 4096: 17, 13; 11008 x 4096: 25, 23).
