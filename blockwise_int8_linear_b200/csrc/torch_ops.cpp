@@ -201,13 +201,15 @@ Tensor empty_q(const Tensor& like, int64_t rows, int64_t cols) {
     return ld == cols ? t : t.narrow(1, 0, cols);
 }
 
-// Copy with a 16-byte aligned row pitch of an int8 operand that has none; the bytes between K and the pitch are never read.
+// Copy with a 16-byte aligned row pitch of an int8 operand that has none; the bytes between K and the pitch are never read.  What
+// is copied is the matrix that `m` describes, at the owner's address with the pitch `ld`: the owner itself may be that matrix or
+// its transpose, which its shape does not tell where both have the same.
 Mat repitch(const Mat& m, const Tensor& like) {
     if (m.ld % 16 == 0 && reinterpret_cast<uintptr_t>(m.ptr) % 16 == 0) return m;
     Mat out = m;
     out.ld = ceil_div(m.cols, 16) * 16;
     out.owner = empty_on(like, {m.rows, out.ld}, at::kChar);
-    out.owner.narrow(1, 0, m.cols).copy_(m.owner.dim() == 2 && m.owner.size(0) == m.rows && m.owner.size(1) == m.cols ? m.owner : m.owner.t());
+    out.owner.narrow(1, 0, m.cols).copy_(m.owner.as_strided({m.rows, m.cols}, {m.ld, 1}));
     out.ptr = out.owner.data_ptr();
     return out;
 }
