@@ -142,15 +142,6 @@ def stream_ptr() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def workspace(device: torch.device, nbytes: int):
-    """GEMM workspace of at least ``nbytes`` for (device, current stream), or None for 0 bytes: scratch for the partial
-    results of divided tiles, one buffer per stream for eager launches, one per CUDA graph while a stream is captured (the
-    table is the one of ``csrc/torch_ops.cpp``, which the functional operations use)."""
-    if nbytes <= 0:
-        return None
-    return native().workspace(device.index if device.index is not None else torch.cuda.current_device(), nbytes)
-
-
 def device_status() -> int:
     """Synchronises and returns the device-side status word (0 = clean); raises on a recorded timeout."""
     detail = ctypes.c_int(0)

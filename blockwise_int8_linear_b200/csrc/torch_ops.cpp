@@ -86,16 +86,14 @@ struct Carve {
     }
 };
 
-// Scratch of the GEMMs (partial results of divided tiles, quantized activations that no caller sees), one buffer per (device, stream) for eager launches: GEMMs queued on a
-// stream run one after the other, so they share it, which saves an allocator round trip per call; a larger request replaces the
-// buffer.  While a stream is being captured the buffer's address is baked into the CUDA graph, so every capture gets
+// Scratch of one call: partial results of divided tiles, quantized activations that no caller sees.  A call is several launches, and
+// the interpreter lock is not held while they are enqueued, so two threads that share a stream may enqueue theirs
+// alternately: scratch belongs to the call, never to the stream.  The allocator gives the memory to others only behind what
+// the call has enqueued on its stream; the returned tensor is held until then.
+//
+// While a stream is being captured the buffer's address is baked into the CUDA graph, so every capture gets
 // a buffer of its own, keyed by the capture's sequence number and allocated from the capture's memory pool, which keeps it
-// reserved for the graph's lifetime; the table drops its own reference when it sees the next capture or an eager call.  At
-// most kMostStreams streams are remembered: one more empties the table (the allocator takes the buffers back in
-// stream order).  A request above kMostKept is not remembered: it is allocated for its call, which then runs for
-// far longer than the allocation takes.
-constexpr size_t kMostStreams = 64;
-constexpr int64_t kMostKept = 32 << 20;
+// reserved for the graph's lifetime; the table drops its own reference when it sees the next capture or an eager call.
 struct WsKey {
     int device;
     uint64_t id;
@@ -105,31 +103,23 @@ struct WsHash {
     size_t operator()(const WsKey& k) const { return std::hash<uint64_t>()(k.id * 0x9E3779B97F4A7C15ull + (uint64_t)k.device); }
 };
 std::mutex g_ws_mutex;
-std::unordered_map<WsKey, Tensor, WsHash>& eager_table() {
+std::unordered_map<WsKey, Tensor, WsHash>& capture_table() {
     static auto* t = new std::unordered_map<WsKey, Tensor, WsHash>();      // never destroyed: the allocator may be gone at exit
     return *t;
 }
-std::unordered_map<WsKey, Tensor, WsHash>& capture_table() {
-    static auto* t = new std::unordered_map<WsKey, Tensor, WsHash>();
-    return *t;
-}
 
-// The returned tensor keeps the buffer alive while the caller enqueues its kernels (another thread may replace the entry).
-Tensor workspace(c10::Device device, c10::cuda::CUDAStream stream, int64_t bytes) {
+Tensor scratch(c10::Device device, c10::cuda::CUDAStream stream, int64_t bytes) {
     if (bytes <= 0) return Tensor();
-    if (bytes > kMostKept) return at::detail::empty_cuda({bytes}, at::kByte, device, std::nullopt);
     unsigned long long capture = 0;
     check(bi8_stream_capture_id(stream.stream(), &capture), "bi8_stream_capture_id");
-    const WsKey key{device.index(), capture ? (uint64_t)capture : (uint64_t)reinterpret_cast<uintptr_t>(stream.stream())};
+    const WsKey key{device.index(), (uint64_t)capture};
     std::lock_guard<std::mutex> lock(g_ws_mutex);
-    auto& captures = capture_table();
-    for (auto it = captures.begin(); it != captures.end();) it = (capture && it->first == key) ? std::next(it) : captures.erase(it);
-    auto& table = capture ? captures : eager_table();
+    auto& table = capture_table();
+    for (auto it = table.begin(); it != table.end();) it = (capture && it->first == key) ? std::next(it) : table.erase(it);
+    if (!capture) return at::detail::empty_cuda({bytes}, at::kByte, device, std::nullopt);
     auto it = table.find(key);
     if (it != table.end() && it->second.numel() >= bytes) return it->second;
-    const int64_t want = std::min(std::max<int64_t>(bytes, it != table.end() ? 2 * it->second.numel() : 0), kMostKept);
-    if (it == table.end() && table.size() >= kMostStreams) table.clear();
-    Tensor t = at::detail::empty_cuda({want}, at::kByte, device, std::nullopt);
+    Tensor t = at::detail::empty_cuda({std::max<int64_t>(bytes, it != table.end() ? 2 * it->second.numel() : 0)}, at::kByte, device, std::nullopt);
     table[key] = t;
     return t;
 }
@@ -333,7 +323,7 @@ Tensor gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& state_x, const
     Tensor c = empty_on(a_in, {m, n}, out_type);
     const Bias bias(bias_in, n);
     const size_t ws_bytes = bi8_gemm_workspace_bytes(m, n, k, (int)block);
-    const Tensor ws = workspace(a_in.device(), on.stream, (int64_t)ws_bytes);
+    const Tensor ws = scratch(a_in.device(), on.stream, (int64_t)ws_bytes);
     check(bi8_gemm_dequant(static_cast<const int8_t*>(o.a.ptr), o.a.ld, static_cast<const int8_t*>(o.bt.ptr), o.bt.ld, sx.const_data_ptr<float>(),
                            sw.const_data_ptr<float>(), bias.ptr, bias.code, c.data_ptr(), n, dtype_code(out_type), m, n, k, (int)block,
                            ws.defined() ? ws.data_ptr() : nullptr, ws_bytes, flags, on.raw()),
@@ -426,11 +416,11 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
     }
     const int x_code = dtype_code(x_in.scalar_type());
     const size_t ws_bytes = bi8_gemm_workspace_bytes(m, n, k, (int)block);
-    // the quantized activations live in the stream's scratch behind the GEMM's workspace
+    // the quantized activations live in the call's scratch behind the GEMM's workspace
     Carve carve;
     carve.take((int64_t)ws_bytes);
     const int64_t xq_at = carve.take(m * pitch16(k)), sx_at = carve.take(nb * m * 4);
-    const Tensor ws = workspace(x_in.device(), on.stream, carve.bytes);
+    const Tensor ws = scratch(x_in.device(), on.stream, carve.bytes);
     char* ws_ptr = ws.defined() ? static_cast<char*>(ws.data_ptr()) : nullptr;
     int8_t* xq = reinterpret_cast<int8_t*>(ws_ptr + xq_at);
     float* sx = reinterpret_cast<float*>(ws_ptr + sx_at);
@@ -905,15 +895,6 @@ BI8_METHOD(rope_cache_append) {  // qkv, cis, pos, kcache, vcache
         return [q = g.tensor(0), c = g.tensor(1), p = g.tensor(2), k = g.tensor(3), v = g.tensor(4)] { return rope_cache_append(q, c, p, k, v); };
     });
 }
-BI8_METHOD(workspace) {          // device index, bytes (> 0)
-    return call("workspace", {a, n}, 2, [](const Args& g) {
-        return [d = (int)g.integer(0), bytes = g.integer(1)] {
-            const c10::Device device(c10::kCUDA, (c10::DeviceIndex)d);
-            c10::cuda::CUDAGuard guard(device);
-            return workspace(device, c10::cuda::getCurrentCUDAStream(device.index()), bytes);
-        };
-    });
-}
 BI8_METHOD(bind) {               // the exception class of failed library calls, the configuration module
     if (n != 2) {
         PyErr_SetString(PyExc_TypeError, "bind takes 2 arguments");
@@ -927,7 +908,7 @@ BI8_METHOD(bind) {               // the exception class of failed library calls,
 #define BI8_ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name##_py)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {BI8_ENTRY(quantize_rowwise), BI8_ENTRY(quantize_colwise), BI8_ENTRY(quantize_dual), BI8_ENTRY(quantize_pre),
                          BI8_ENTRY(dequantize), BI8_ENTRY(gemm), BI8_ENTRY(block_partials), BI8_ENTRY(matmul), BI8_ENTRY(linear),
-                         BI8_ENTRY(train_linear), BI8_ENTRY(rope_cache_append), BI8_ENTRY(workspace), BI8_ENTRY(bind),
+                         BI8_ENTRY(train_linear), BI8_ENTRY(rope_cache_append), BI8_ENTRY(bind),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Host path of the blockwise-int8 operations.", -1, methods, nullptr, nullptr, nullptr, nullptr};
 

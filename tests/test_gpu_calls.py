@@ -1,5 +1,7 @@
 """What the native host path does with its callers' operands: layouts of dense weights, threads that share a stream, branches of a
 captured graph, the layout of quantized results, and autograd features beside the plain backward pass."""
+import threading
+
 import pytest
 import torch
 
@@ -43,4 +45,41 @@ def test_dense_weights_of_unaligned_rows(m, k, n):
         for j in range(parts.shape[0]):
             cols = slice(64 * j, min(k, 64 * (j + 1)))
             assert torch.equal(parts[j].double(), xq[:, cols].double() @ q[:, cols].double().t())
+    assert_clean_device()
+
+
+@pytest.mark.parametrize("m,k,n", [(20, 1024, 1024), (128, 2048, 1536), (333, 1001, 520)])
+def test_threads_that_share_a_stream(m, k, n):
+    """Layer calls of several threads on one stream, each on its own activations: a call is a quantizer and a GEMM (with a kernel for
+    the divided tiles, and a copy of unaligned weights), which the threads enqueue alternately."""
+    from block_linear import BlockInt8Linear
+    tf = _tf()
+    set_config(64)
+    lin = BlockInt8Linear(k, n, bias=False, device=DEV, dtype=torch.bfloat16).eval()
+    xs = [randn_bf16((m, k), seed, std=1.0 + seed).to(DEV) for seed in range(4)]
+    norm = randn_bf16((k,), 9).to(DEV)
+    with torch.no_grad():
+        qs = [tf.quantize_block_rowwise(x) for x in xs]
+        w, sw = lin._quantized_weight()
+        calls = [lambda i: lin(xs[i]), lambda i: lin.infer_pre(xs[i], "rmsnorm", norm_weight=norm),
+                 lambda i: tf.int8_matmul_block64_rowwise_dequantize(qs[i][0], w.t(), qs[i][1], sw)]
+        want = [[call(i).clone() for call in calls] for i in range(len(xs))]
+    torch.cuda.synchronize()
+    bad, start = [None] * len(xs), threading.Barrier(len(xs))
+
+    def work(i):
+        wrong = 0
+        start.wait()
+        with torch.no_grad():
+            for _ in range(20):
+                outs = [[call(i) for _ in range(20)] for call in calls]
+                wrong += sum(int((torch.stack(o) != r).any(dim=-1).any(dim=-1).sum()) for o, r in zip(outs, want[i]))
+        bad[i] = wrong
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(xs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert bad == [0] * len(xs)
     assert_clean_device()
