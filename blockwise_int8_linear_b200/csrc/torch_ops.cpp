@@ -28,7 +28,6 @@
 #include <mutex>
 #include <optional>
 #include <string>
-#include <unordered_map>
 
 #include "../../include/bi8.h"
 
@@ -88,41 +87,11 @@ struct Carve {
 
 // Scratch of one call: partial results of divided tiles, quantized activations that no caller sees.  A call is several launches, and
 // the interpreter lock is not held while they are enqueued, so two threads that share a stream may enqueue theirs
-// alternately: scratch belongs to the call, never to the stream.  The allocator gives the memory to others only behind what
-// the call has enqueued on its stream; the returned tensor is held until then.
-//
-// While a stream is being captured the buffer's address is baked into the CUDA graph, so every capture gets
-// a buffer of its own, keyed by the capture's sequence number and allocated from the capture's memory pool, which keeps it
-// reserved for the graph's lifetime; the table drops its own reference when it sees the next capture or an eager call.
-struct WsKey {
-    int device;
-    uint64_t id;
-    bool operator==(const WsKey& o) const { return device == o.device && id == o.id; }
-};
-struct WsHash {
-    size_t operator()(const WsKey& k) const { return std::hash<uint64_t>()(k.id * 0x9E3779B97F4A7C15ull + (uint64_t)k.device); }
-};
-std::mutex g_ws_mutex;
-std::unordered_map<WsKey, Tensor, WsHash>& capture_table() {
-    static auto* t = new std::unordered_map<WsKey, Tensor, WsHash>();      // never destroyed: the allocator may be gone at exit
-    return *t;
-}
-
-Tensor scratch(c10::Device device, c10::cuda::CUDAStream stream, int64_t bytes) {
-    if (bytes <= 0) return Tensor();
-    unsigned long long capture = 0;
-    check(bi8_stream_capture_id(stream.stream(), &capture), "bi8_stream_capture_id");
-    const WsKey key{device.index(), (uint64_t)capture};
-    std::lock_guard<std::mutex> lock(g_ws_mutex);
-    auto& table = capture_table();
-    for (auto it = table.begin(); it != table.end();) it = (capture && it->first == key) ? std::next(it) : table.erase(it);
-    if (!capture) return at::detail::empty_cuda({bytes}, at::kByte, device, std::nullopt);
-    auto it = table.find(key);
-    if (it != table.end() && it->second.numel() >= bytes) return it->second;
-    Tensor t = at::detail::empty_cuda({std::max<int64_t>(bytes, it != table.end() ? 2 * it->second.numel() : 0)}, at::kByte, device, std::nullopt);
-    table[key] = t;
-    return t;
-}
+// alternately, and calls on forked streams of one capture become branches of a graph that may run at the same time: scratch
+// belongs to the call, not to its stream or capture.  The allocator gives the memory to others only behind what the
+// call has enqueued on its stream (the returned tensor is held until then), and while a stream is captured it takes it
+// from the capture's memory pool, which stays reserved for the graph's lifetime.
+Tensor scratch(const Tensor& like, int64_t bytes) { return bytes > 0 ? empty_on(like, {bytes}, at::kByte) : Tensor(); }
 
 // Makes the operand's device current for a call and names its current stream.
 struct OnDevice {
@@ -323,7 +292,7 @@ Tensor gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& state_x, const
     Tensor c = empty_on(a_in, {m, n}, out_type);
     const Bias bias(bias_in, n);
     const size_t ws_bytes = bi8_gemm_workspace_bytes(m, n, k, (int)block);
-    const Tensor ws = scratch(a_in.device(), on.stream, (int64_t)ws_bytes);
+    const Tensor ws = scratch(a_in, (int64_t)ws_bytes);
     check(bi8_gemm_dequant(static_cast<const int8_t*>(o.a.ptr), o.a.ld, static_cast<const int8_t*>(o.bt.ptr), o.bt.ld, sx.const_data_ptr<float>(),
                            sw.const_data_ptr<float>(), bias.ptr, bias.code, c.data_ptr(), n, dtype_code(out_type), m, n, k, (int)block,
                            ws.defined() ? ws.data_ptr() : nullptr, ws_bytes, flags, on.raw()),
@@ -420,7 +389,7 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
     Carve carve;
     carve.take((int64_t)ws_bytes);
     const int64_t xq_at = carve.take(m * pitch16(k)), sx_at = carve.take(nb * m * 4);
-    const Tensor ws = scratch(x_in.device(), on.stream, carve.bytes);
+    const Tensor ws = scratch(x_in, carve.bytes);
     char* ws_ptr = ws.defined() ? static_cast<char*>(ws.data_ptr()) : nullptr;
     int8_t* xq = reinterpret_cast<int8_t*>(ws_ptr + xq_at);
     float* sx = reinterpret_cast<float*>(ws_ptr + sx_at);

@@ -83,3 +83,32 @@ def test_threads_that_share_a_stream(m, k, n):
         t.join()
     assert bad == [0] * len(xs)
     assert_clean_device()
+
+
+@pytest.mark.parametrize("m,k,n", [(24, 2048, 4096), (128, 4096, 1536), (333, 1001, 520)])
+def test_branches_of_a_captured_graph(m, k, n):
+    """Layer calls on two forked streams of one capture: the branches may run at the same time on every replay."""
+    from block_linear import BlockInt8Linear
+    set_config(64)
+    lins = [BlockInt8Linear(k, n, bias=False, device=DEV, dtype=torch.bfloat16).eval() for _ in range(2)]
+    xs = [[randn_bf16((m, k), 10 * b + i, std=1.0 + b).to(DEV) for i in range(4)] for b in range(2)]
+    with torch.no_grad():
+        want = [[lin(x).clone() for x in x_b] for lin, x_b in zip(lins, xs)]
+        torch.cuda.synchronize()
+        graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        outs = [[], []]
+        with torch.cuda.graph(graph):
+            main = torch.cuda.current_stream()
+            side.wait_stream(main)
+            for i in range(4):
+                outs[0].append(lins[0](xs[0][i]))
+                with torch.cuda.stream(side):
+                    outs[1].append(lins[1](xs[1][i]))
+            main.wait_stream(side)
+        for _ in range(20):
+            graph.replay()
+            torch.cuda.synchronize()
+            for got_b, want_b in zip(outs, want):
+                assert all(torch.equal(g, w) for g, w in zip(got_b, want_b))
+    del outs, graph
+    assert_clean_device()
