@@ -49,17 +49,18 @@ namespace {
 bool dtype_ok(int dt) { return dt == BI8_BF16 || dt == BI8_F32 || dt == BI8_F16; }
 int dtype_size(int dt) { return dt == BI8_F32 ? 4 : 2; }
 
-int check_gemm(const GemmArgs& g, bool partials) {
+// `quantized`: the activations are there as int8 (A, sA); false where the GEMM kernel may quantize them itself.
+int check_gemm(const GemmArgs& g, bool partials, bool quantized = true) {
     if (g.M < 0 || g.N < 0 || g.K < 0) return fail(BI8_ERR_SHAPE, "gemm: negative dimension (M=%lld N=%lld K=%lld)", (long long)g.M, (long long)g.N, (long long)g.K);
     if (g.block < 1) return fail(BI8_ERR_BLOCK, "gemm: block size %d", g.block);
     if (g.M == 0 || g.N == 0) return BI8_OK;
-    if (g.K > 0 && (!g.A || !g.Bt)) return fail(BI8_ERR_NULL, "gemm: null operand");
+    if (g.K > 0 && ((quantized && !g.A) || !g.Bt)) return fail(BI8_ERR_NULL, "gemm: null operand");
     if (g.lda < g.K || g.ldb < g.K) return fail(BI8_ERR_SHAPE, "gemm: row pitch smaller than K");
     if (partials) {
         if (!g.partials && g.K > 0) return fail(BI8_ERR_NULL, "gemm_block_partials: null output");
     } else {
         if (!g.C) return fail(BI8_ERR_NULL, "gemm: null output");
-        if (g.K > 0 && (!g.sA || !g.sB)) return fail(BI8_ERR_NULL, "gemm: null scale tensor");
+        if (g.K > 0 && ((quantized && !g.sA) || !g.sB)) return fail(BI8_ERR_NULL, "gemm: null scale tensor");
         if (!dtype_ok(g.out_dtype)) return fail(BI8_ERR_DTYPE, "gemm: unknown output dtype code %d", g.out_dtype);
         if (g.bias && !dtype_ok(g.bias_dtype)) return fail(BI8_ERR_DTYPE, "gemm: unknown bias dtype code %d", g.bias_dtype);
         if (g.ldc < g.N) return fail(BI8_ERR_SHAPE, "gemm: ldc smaller than N");
@@ -106,7 +107,7 @@ int dispatch_gemm(const GemmArgs& g, cudaStream_t st) {
 // this many values: 3 x 2048: 37 us a layer against 47, 1 x 4096: 61 against 65, but 8 x 4096: 78 against 71.  A plain call by itself
 // is bound by its launches as long as a CTA's part is no longer than that: inside against in front, 16 x 4096 -> 4096 (16384
 // values a CTA) 11.4 us, 13.9; 8 x 4096 -> 11008 (32768) 19.4, 15.6; 16 x 5120 -> 13824 (81920) 33, 20.
-constexpr int64_t kQuantInKernelValues = 16384;
+constexpr int64_t kQuantInKernelValues = BI8_ONE_LAUNCH_VALUES;
 
 // Decode-sized layer (the weight-streaming GEMM and what produces its activations).  `g` describes the GEMM on the
 // quantized activations g.A / g.sA, which are scratch (null: none); `alone`: a plain call, not a step with a producer or a
@@ -350,7 +351,7 @@ int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtyp
                                const void* residual, int64_t ldr, void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N, int64_t K,
                                int block, void* workspace, size_t workspace_bytes, int flags, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (M > 0 && K > 0 && (!xq || !sx)) return fail(BI8_ERR_WORKSPACE, "gemm_dequant_fused_pre: the xq / sx scratch is required");
+    const bool scratch = xq != nullptr && sx != nullptr;
     if (residual && ldr < N) return fail(BI8_ERR_SHAPE, "gemm_dequant_fused_pre: residual row pitch smaller than the row");
     if (!dtype_ok(out_dtype)) return fail(BI8_ERR_DTYPE, "gemm_dequant_fused_pre: unknown output dtype code %d", out_dtype);
     if (residual && !aligned(residual, dtype_size(out_dtype))) return fail(BI8_ERR_ALIGN, "gemm_dequant_fused_pre: residual not element aligned");
@@ -372,7 +373,7 @@ int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtyp
                       (!norm_weight || aligned(norm_weight, dtype_size(x_dtype))) && (op == BI8_PRE_NONE || op == BI8_PRE_RMSNORM || op == BI8_PRE_SILU_MUL);
     const bool in_kernel_residual = residual && !bias;
     if (!forced && K > 0 && x_ok && !(overlap && !in_kernel_residual)) {
-        int rc = check_gemm(g, false);
+        int rc = check_gemm(g, false, scratch);
         if (rc != BI8_OK) return rc;
         if (in_kernel_residual) {
             g.bias = residual;
@@ -387,6 +388,8 @@ int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtyp
         }
         g.bias_ld = 0;
     }
+    if (K > 0 && !scratch)
+        return fail(BI8_ERR_WORKSPACE, "gemm_dequant_fused_pre: this shape runs as quantize + GEMM and needs the xq / sx scratch");
     // The general tensor-core kernel reads an element of the residual in the warp that then writes it, so C may be the residual.
     const char* why = "";
     if (overlap && ((flags & BI8_GEMM_FORCE_GENERIC) || bias || K == 0 || !gemm_tc_applicable(g, &why)))

@@ -61,6 +61,10 @@ extern "C" {
 #define BI8_GEMM_FORCE_SKINNY 16   /* weight-streaming tensor-core kernel with exchanged operand roles, M <= 64 */
 #define BI8_GEMM_QUANT_IN_KERNEL 32 /* bi8_gemm_dequant_fused_quant, M <= 32: quantize inside the GEMM kernel */
 
+/* Decode-sized layers (M <= 16) of at most this many activation values are one launch on every path: a caller without scratch
+ * gets the same kernel there. */
+#define BI8_ONE_LAUNCH_VALUES 16384
+
 BI8_API int bi8_version(void);
 
 /* Text of the last error raised on the calling thread ("" if none). */
@@ -170,7 +174,8 @@ BI8_API int bi8_gemm_block_partials(const int8_t* A, int64_t lda, const int8_t* 
  * stride ldx, is quantized per row and block exactly as bi8_quantize_rowwise does and multiplied with the
  * pre-quantized weights Wq [N,K] / sW; the result equals bi8_quantize_rowwise followed by bi8_gemm_dequant.
  * For M <= 64 (N a multiple of 4, K a multiple of 16, 16-byte aligned rows) the weight-streaming tensor-core GEMM runs: up to
- * 16 rows it quantizes the activations itself as its first weights arrive, in one launch; above, a small quantizer kernel
+ * 16 rows it quantizes the activations itself as its first weights arrive, in one launch, if there are few of them (M*K up
+ * to BI8_ONE_LAUNCH_VALUES, or as many in the share of K of one CTA); otherwise a small quantizer kernel
  * runs in front and the GEMM is launched so that its set-up and first weight loads overlap it.  With
  * BI8_GEMM_QUANT_IN_KERNEL (or without scratch) the one-launch form is taken up to 32 rows.  Every other shape runs the
  * standalone quantizer and the GEMM back to back.  xq [M,K] int8 and sx [ceil(K/block),M] fp32 are scratch, which
@@ -201,7 +206,7 @@ BI8_API int bi8_quantize_rowwise_pre(int op, const void* x, const void* x2, int 
  * the weight-streaming GEMM (few activation values) or in its quantizer kernel in front of it; the residual is added by
  * the kernel that writes C, here and in the general tensor-core kernel.  Without bias C may be the residual itself (a
  * residual stream updated in place; any other overlap of the two is BI8_ERR_SHAPE, the same tensor where neither kernel
- * applies BI8_ERR_ALIGN).  xq / sx are required scratch. */
+ * applies BI8_ERR_ALIGN).  xq / sx as in bi8_gemm_dequant_fused_quant. */
 BI8_API int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtype, int64_t ldx, const void* norm_weight,
                                float eps, int8_t* xq, float* sx, const int8_t* Wq, int64_t ldw, const float* sW,
                                const void* bias, int bias_dtype, const void* residual, int64_t ldr, void* C, int64_t ldc,

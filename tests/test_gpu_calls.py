@@ -112,3 +112,20 @@ def test_branches_of_a_captured_graph(m, k, n):
                 assert all(torch.equal(g, w) for g, w in zip(got_b, want_b))
     del outs, graph
     assert_clean_device()
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 256, 132), (1, 16384, 260), (16, 1024, 512), (4, 4096, 777), (16, 1040, 512), (17, 512, 128)])
+def test_one_launch_calls_without_scratch(m, k, n):
+    """Around BI8_ONE_LAUNCH_VALUES (and where that kernel does not take the width, 777): the layer call against quantizer + GEMM."""
+    tf = _tf()
+    set_config(64)
+    x, res, norm = randn_bf16((m, k), m + k).to(DEV), randn_bf16((m, n), 3).to(DEV), randn_bf16((k,), 4).to(DEV)
+    bias = randn_bf16((n,), 6).to(DEV)
+    w, sw = tf.quantize_block_rowwise(randn_bf16((n, k), n, std=0.02).to(DEV))
+    for op, q in (("none", tf.quantize_block_rowwise(x)), ("rmsnorm", tf.rmsnorm_quantize_block_rowwise(x, 1e-5, norm))):
+        want = tf.int8_matmul_block64_rowwise_dequantize(q[0], w.t(), q[1], sw)
+        for b, r in ((None, None), (None, res), (bias, res)):
+            got = tf.pre_quantize_matmul_block_rowwise_dequantize(op, x, w.t(), sw, b, norm_weight=norm, residual=r)
+            full = want if b is None else want + b
+            assert torch.equal(got, full if r is None else full + r)
+    assert_clean_device()

@@ -17,6 +17,12 @@ def L():
     return _lib.lib()
 
 
+def _only_without_a_gpu():
+    """A call without scratch is refused where no kernel takes it, which on a B200 would be the launch of one on these addresses."""
+    if torch.cuda.is_available():
+        pytest.skip("the addresses of this test must not reach a device")
+
+
 def test_library_exports_every_declared_symbol(L):
     header = open(os.path.join(ROOT, "include", "bi8.h")).read()
     declared = sorted(set(re.findall(r"BI8_API[^;]*?\b(bi8_\w+)\s*\(", header)))
@@ -56,6 +62,7 @@ def test_argument_validation_happens_before_cuda(L):
 
 
 def test_fused_entry_point_validates_and_flags_match_the_header(L):
+    _only_without_a_gpu()
     from blockwise_int8_linear_b200 import _lib
     header = open(os.path.join(ROOT, "include", "bi8.h")).read()
     flags = {name: int(value) for name, value in re.findall(r"#define BI8_GEMM_(\w+)\s+(\d+)", header)}
@@ -76,6 +83,7 @@ def test_fused_entry_point_validates_and_flags_match_the_header(L):
 def test_new_entry_points_validate_before_cuda(L):
     """The entry points around the layer (fused producer steps, residual, prefill-sized peer sum, rotary/cache helper):
     every argument check runs before the first CUDA call, so it can be exercised without a GPU."""
+    _only_without_a_gpu()
     from blockwise_int8_linear_b200 import _lib
     header = open(os.path.join(ROOT, "include", "bi8.h")).read()
     pre = {name: int(value) for name, value in re.findall(r"#define BI8_PRE_(\w+)\s+(\d+)", header)}
