@@ -69,6 +69,15 @@ int check_gemm(const GemmArgs& g, bool partials, bool quantized = true) {
     return BI8_OK;
 }
 
+// Whether the memory of the residual [M, N] (row pitch ldr) and of the output meet anywhere between their first and last elements.
+bool overlaps_output(const void* residual, int64_t ldr, const void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N) {
+    if (residual == nullptr || C == nullptr || M <= 0 || N <= 0) return false;
+    const int esz = dtype_size(out_dtype);
+    const char *c0 = static_cast<const char*>(C), *c1 = c0 + ((M - 1) * ldc + N) * esz;
+    const char *r0 = static_cast<const char*>(residual), *r1 = r0 + ((M - 1) * ldr + N) * esz;
+    return r0 < c1 && c0 < r1;
+}
+
 // The kernels that do not add GemmArgs::residual themselves are followed by one that does.
 int then_residual(int rc, const GemmArgs& g, cudaStream_t st) {
     if (rc != BI8_OK || g.residual == nullptr) return rc;
@@ -292,6 +301,7 @@ int bi8_gemm_dequant_residual(const int8_t* A, int64_t lda, const int8_t* Bt, in
     if (rc != BI8_OK || M == 0 || N == 0) return rc;
     if (residual && ldr < N) return fail(BI8_ERR_SHAPE, "gemm_dequant_residual: residual row pitch smaller than the row");
     if (residual && !aligned(residual, dtype_size(out_dtype))) return fail(BI8_ERR_ALIGN, "gemm_dequant_residual: residual not element aligned");
+    if (overlaps_output(residual, ldr, C, ldc, out_dtype, M, N)) return fail(BI8_ERR_SHAPE, "gemm_dequant_residual: residual and C overlap");
     g.residual = residual;
     g.ldr = ldr;
     return dispatch_gemm(g, static_cast<cudaStream_t>(stream));
@@ -356,10 +366,7 @@ int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtyp
     if (!dtype_ok(out_dtype)) return fail(BI8_ERR_DTYPE, "gemm_dequant_fused_pre: unknown output dtype code %d", out_dtype);
     if (residual && !aligned(residual, dtype_size(out_dtype))) return fail(BI8_ERR_ALIGN, "gemm_dequant_fused_pre: residual not element aligned");
     if (M == 0 || N == 0) return BI8_OK;
-    const size_t osz = dtype_size(out_dtype);
-    const char *c0 = static_cast<const char*>(C), *c1 = c0 + ((M - 1) * ldc + N) * osz;
-    const char *r0 = static_cast<const char*>(residual), *r1 = residual ? r0 + ((M - 1) * ldr + N) * osz : r0;
-    const bool overlap = residual && C && r0 < c1 && c0 < r1;
+    const bool overlap = overlaps_output(residual, ldr, C, ldc, out_dtype, M, N);
     if (overlap && (residual != C || ldr != ldc))
         return fail(BI8_ERR_SHAPE, "gemm_dequant_fused_pre: residual and C overlap without being the same tensor");
     if (op == BI8_PRE_NONE && !residual)

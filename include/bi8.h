@@ -128,7 +128,7 @@ BI8_API int bi8_gemm_dequant(const int8_t* A, int64_t lda, const int8_t* Bt, int
 BI8_API size_t bi8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int block);
 
 /* bi8_gemm_dequant plus an addend: C = cast(cast(sum) (+ bias) + residual[m,n]), the addition in the output type as a layer's
- * `x + proj(...)` performs it.  residual [M,N] of out_dtype, row stride ldr; it must not overlap C. */
+ * `x + proj(...)` performs it.  residual [M,N] of out_dtype, row stride ldr; an overlap with C is BI8_ERR_SHAPE. */
 BI8_API int bi8_gemm_dequant_residual(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb,
                      const float* sA, const float* sB, const void* bias, int bias_dtype, const void* residual, int64_t ldr,
                      void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N, int64_t K, int block,

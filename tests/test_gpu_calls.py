@@ -129,3 +129,23 @@ def test_one_launch_calls_without_scratch(m, k, n):
             full = want if b is None else want + b
             assert torch.equal(got, full if r is None else full + r)
     assert_clean_device()
+
+
+@pytest.mark.parametrize("k", [73, 1001, 64])
+def test_residual_and_output_that_overlap(k):
+    """Overlap without being the same tensor is an error for every K (with and without aligned rows); the same tensor is updated."""
+    from blockwise_int8_linear_b200._lib import Bi8Error
+    tf = _tf()
+    set_config(64)
+    m, n = 40, 64
+    x = randn_bf16((m, k), k).to(DEV)
+    w, sw = tf.quantize_block_rowwise(randn_bf16((n, k), 1, std=0.02).to(DEV))
+    buf = randn_bf16((m + 1, n), 2).to(DEV)
+    res, out, before = buf[:m], buf[1:], buf.clone()
+    with pytest.raises(Bi8Error, match="overlap"):
+        tf.pre_quantize_matmul_block_rowwise_dequantize("none", x, w.t(), sw, residual=res, out=out)
+    assert torch.equal(buf, before)
+    want = tf.pre_quantize_matmul_block_rowwise_dequantize("none", x, w.t(), sw, residual=res.clone())
+    assert tf.pre_quantize_matmul_block_rowwise_dequantize("none", x, w.t(), sw, residual=res, out=res) is not None
+    assert torch.equal(buf[:m], want) and torch.equal(buf[m:], before[m:])
+    assert_clean_device()

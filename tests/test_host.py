@@ -134,6 +134,22 @@ def test_new_entry_points_validate_before_cuda(L):
     assert r(B=0) == 0
 
 
+@pytest.mark.parametrize("dt,esz", [(0, 2), (1, 4), (2, 2)])
+def test_residual_that_overlaps_the_output_is_refused(L, dt, esz):
+    """bi8_gemm_dequant_residual, the GEMM behind layers whose K is not a multiple of 16, refuses every overlap before it launches;
+    memory that only touches the output is taken (and then stopped by the missing GPU)."""
+    _only_without_a_gpu()
+    vp = ctypes.c_void_p
+    one = vp(4096)
+    M, N, K, ld = 8, 64, 73, 80
+    out_bytes = ((M - 1) * ld + N) * esz
+    f = lambda res: L.bi8_gemm_dequant_residual(one, 80, one, 80, one, one, None, 0, vp(res), ld, vp(1 << 20), ld, dt, M, N, K, 64, None, 0, 0, None)
+    for res in ((1 << 20), (1 << 20) + esz, (1 << 20) + out_bytes - esz, (1 << 20) - out_bytes + esz):
+        assert f(res) == -4 and "overlap" in L.bi8_last_error_string().decode()
+    for res in ((1 << 20) + out_bytes, (1 << 20) - out_bytes):
+        assert f(res) == -5
+
+
 def test_python_surface_mirrors_reference_names():
     import block_linear
     import block_linear_config
