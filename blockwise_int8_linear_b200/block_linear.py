@@ -17,7 +17,7 @@ from .triton_functions import (
     quantize_block_colwise,
     quantize_block_rowwise,
 )
-from .triton_functions import _block, _pre_code
+from .triton_functions import _block, _pre_code, _scale_dtype
 
 __all__ = [
     "replace_linear_with_blockwise_int8", "fast_matmul", "blockwise_int8_linear", "BlockInt8Linear", "BlockLinear",
@@ -46,8 +46,9 @@ def replace_linear_with_blockwise_int8(model: nn.Module) -> nn.Module:
 def fast_matmul(a, b):
     """``a [M, K] @ b [K, N]`` with both operands quantized on the fly (``block_linear.py:34-40``, without its
     debug prints)."""
-    b_int8, b_state = quantize_block_colwise(b)            # == quantize(b.t().contiguous())
-    a_int8, a_state = quantize_block_rowwise(a)
+    _scale_dtype()
+    b_int8, b_state = _lib.native().quantize_colwise(b, _block(), True)            # == quantize(b.t().contiguous())
+    a_int8, a_state = _lib.native().quantize_rowwise(a, _block(), True)
     return int8_matmul_block64_rowwise_dequantize(a_int8, b_int8.t(), a_state, b_state)
 
 

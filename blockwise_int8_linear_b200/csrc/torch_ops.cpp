@@ -153,9 +153,10 @@ void need_cuda(const Tensor& t) {
 // Row pitch of a quantized matrix: the next multiple of 16 bytes, which is what the wide kernels and the tensor-core GEMM take.
 int64_t pitch16(int64_t n) { return (n + 15) / 16 * 16; }
 
-// int8 [rows, cols] whose rows begin on 16-byte boundaries: dense where cols is a multiple of 16, else a view of a wider buffer
-Tensor empty_q(const Tensor& like, int64_t rows, int64_t cols) {
-    const int64_t ld = pitch16(cols);
+// int8 [rows, cols], dense, or (`pitched`) with rows that begin on 16-byte boundaries: a view of a wider buffer where cols is not
+// a multiple of 16
+Tensor empty_q(const Tensor& like, int64_t rows, int64_t cols, bool pitched) {
+    const int64_t ld = pitched ? pitch16(cols) : cols;
     Tensor t = empty_on(like, {rows, ld}, at::kChar);
     return ld == cols ? t : t.narrow(1, 0, cols);
 }
@@ -176,28 +177,38 @@ Mat repitch(const Mat& m, const Tensor& like) {
 // ---- quantizers ---------------------------------------------------------------------------------------------------------
 struct Quantized {
     Tensor q, s;
+    int64_t ld() const { return std::max(q.stride(0), q.size(1)); }      // of what empty_q gives, a single row's too
 };
 
-Quantized quantize_rowwise(const Tensor& x, int64_t block) {
+// Whether a quantized tensor that a caller gets has a row pitch of 16 bytes.  Callers may view, save or hand on what they get, so it
+// is dense, except for large 16-bit matrices: there the re-pitching copy that the GEMM would make of it costs more than a
+// launch, and such callers have always got a view.
+bool pitched_result(const Tensor& x, int64_t block) {
+    const int64_t r = x.size(0), c = x.size(1);
+    return x.element_size() == 2 && block % 16 == 0 && r * c >= (1 << 22) && std::min(r, c) >= 256;
+}
+
+// `operand`: the result goes into a GEMM and to nobody else, so it gets the pitch that the GEMM wants
+Quantized quantize_rowwise(const Tensor& x, int64_t block, bool operand) {
     need_cuda(x);
     OnDevice on(x);
     const Mat m = mat2d(x);
     const int code = dtype_code(x.scalar_type());
-    Quantized r{empty_q(x, m.rows, m.cols), empty_on(x, {ceil_div(m.cols, block), m.rows}, at::kFloat)};
-    check(bi8_quantize_rowwise_pitched(m.ptr, code, m.ld, r.q.mutable_data_ptr<int8_t>(), pitch16(m.cols), r.s.mutable_data_ptr<float>(), m.rows,
-                                       m.cols, (int)block, on.raw()),
+    Quantized r{empty_q(x, m.rows, m.cols, operand || pitched_result(x, block)), empty_on(x, {ceil_div(m.cols, block), m.rows}, at::kFloat)};
+    check(bi8_quantize_rowwise_pitched(m.ptr, code, m.ld, r.q.mutable_data_ptr<int8_t>(), r.ld(), r.s.mutable_data_ptr<float>(), m.rows, m.cols,
+                                       (int)block, on.raw()),
           "bi8_quantize_rowwise");
     return r;
 }
 
-Quantized quantize_colwise(const Tensor& x, int64_t block) {
+Quantized quantize_colwise(const Tensor& x, int64_t block, bool operand) {
     need_cuda(x);
     OnDevice on(x);
     const Mat m = mat2d(x);
     const int code = dtype_code(x.scalar_type());
-    Quantized r{empty_q(x, m.cols, m.rows), empty_on(x, {ceil_div(m.rows, block), m.cols}, at::kFloat)};
-    check(bi8_quantize_colwise_pitched(m.ptr, code, m.ld, r.q.mutable_data_ptr<int8_t>(), pitch16(m.rows), r.s.mutable_data_ptr<float>(), m.rows,
-                                       m.cols, (int)block, on.raw()),
+    Quantized r{empty_q(x, m.cols, m.rows, operand || pitched_result(x, block)), empty_on(x, {ceil_div(m.rows, block), m.cols}, at::kFloat)};
+    check(bi8_quantize_colwise_pitched(m.ptr, code, m.ld, r.q.mutable_data_ptr<int8_t>(), r.ld(), r.s.mutable_data_ptr<float>(), m.rows, m.cols,
+                                       (int)block, on.raw()),
           "bi8_quantize_colwise");
     return r;
 }
@@ -211,10 +222,11 @@ Dual quantize_dual(const Tensor& x, int64_t block) {
     OnDevice on(x);
     const Mat m = mat2d(x);
     const int code = dtype_code(x.scalar_type());
-    Dual d{{empty_q(x, m.rows, m.cols), empty_on(x, {ceil_div(m.cols, block), m.rows}, at::kFloat)},
-           {empty_q(x, m.cols, m.rows), empty_on(x, {ceil_div(m.rows, block), m.cols}, at::kFloat)}};
-    check(bi8_quantize_dual_pitched(m.ptr, code, m.ld, d.row.q.mutable_data_ptr<int8_t>(), pitch16(m.cols), d.row.s.mutable_data_ptr<float>(),
-                                    d.col.q.mutable_data_ptr<int8_t>(), pitch16(m.rows), d.col.s.mutable_data_ptr<float>(), m.rows, m.cols,
+    const bool pitched = pitched_result(x, block);
+    Dual d{{empty_q(x, m.rows, m.cols, pitched), empty_on(x, {ceil_div(m.cols, block), m.rows}, at::kFloat)},
+           {empty_q(x, m.cols, m.rows, pitched), empty_on(x, {ceil_div(m.rows, block), m.cols}, at::kFloat)}};
+    check(bi8_quantize_dual_pitched(m.ptr, code, m.ld, d.row.q.mutable_data_ptr<int8_t>(), d.row.ld(), d.row.s.mutable_data_ptr<float>(),
+                                    d.col.q.mutable_data_ptr<int8_t>(), d.col.ld(), d.col.s.mutable_data_ptr<float>(), m.rows, m.cols,
                                     (int)block, on.raw()),
           "bi8_quantize_dual");
     return d;
@@ -342,9 +354,9 @@ Quantized quantize_pre(int op, const Tensor& x_in, const Tensor& x2, const Tenso
     OnDevice on(x_in);
     const Pre pre(op, x_in, x2, weight);
     const int64_t m = pre.x.rows, k = pre.x.cols;
-    Quantized r{empty_q(x_in, m, k), empty_on(x_in, {ceil_div(k, block), m}, at::kFloat)};
+    Quantized r{empty_q(x_in, m, k, false), empty_on(x_in, {ceil_div(k, block), m}, at::kFloat)};
     check(bi8_quantize_rowwise_pre_pitched(op, pre.x.ptr, pre.x2.ptr, dtype_code(x_in.scalar_type()), pre.x.ld, pre.weight_ptr(), (float)eps,
-                                   r.q.mutable_data_ptr<int8_t>(), pitch16(k), r.s.mutable_data_ptr<float>(), m, k, (int)block, on.raw()),
+                                   r.q.mutable_data_ptr<int8_t>(), r.ld(), r.s.mutable_data_ptr<float>(), m, k, (int)block, on.raw()),
           "bi8_quantize_rowwise_pre");
     return r;
 }
@@ -414,8 +426,8 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
     float* sx = reinterpret_cast<float*>(ws_ptr + sx_at);
     void* gemm_ws = ws_bytes ? ws_ptr : nullptr;
     if (k % 16 != 0) {
-        // Rows that are not 16-byte aligned: the activations are quantized into rows that are, weights that have come without
-        // a pitch (a checkpoint's dense copy) are re-pitched where the GEMM is long enough to gain from it.
+        // Rows that are not 16-byte aligned: the activations are quantized into rows that are, weights that have none (of
+        // a layer, a checkpoint's dense copy) are re-pitched where the GEMM is long enough to gain from it.
         if (k >= 256 && m * n >= 128 * 128) bt = repitch(bt, x_in);
         check(bi8_quantize_rowwise_pre_pitched(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps, xq, pitch16(k), sx, m, k,
                                                (int)block, on.raw()),
@@ -479,7 +491,7 @@ struct QPlan {
 
 QRef ref_of(const Quantized& r) {
     return {static_cast<int8_t*>(r.q.data_ptr()), static_cast<float*>(r.s.data_ptr()), r.q.size(0), r.q.size(1),
-            r.q.size(0) > 1 ? r.q.stride(0) : pitch16(r.q.size(1))};
+            r.ld()};
 }
 
 void rowwise_into(const Mat& m, int code, int64_t block, const QRef& r, void* stream) {
@@ -606,7 +618,7 @@ variable_list LinearBackward::apply(variable_list&& grads) {
             if (cached.q.defined()) {
                 wt = ref_of(cached);
             } else if (cache) {
-                fresh = Quantized{empty_q(w, k, n), empty_on(w, {ceil_div(n, b), k}, at::kFloat)};
+                fresh = Quantized{empty_q(w, k, n, true), empty_on(w, {ceil_div(n, b), k}, at::kFloat)};
                 wt = ref_of(fresh);
                 colwise_into(wm, w_code, b, wt, st);
                 cache_put(cache, "col", fresh);
@@ -681,7 +693,7 @@ Tensor train_linear(const Tensor& x_in, const Tensor& w, const Tensor& bias_in, 
         if (cached.q.defined()) {
             wq = ref_of(cached);
         } else if (cache) {
-            fresh = Quantized{empty_q(w, n, k), empty_on(w, {ceil_div(k, block), n}, at::kFloat)};
+            fresh = Quantized{empty_q(w, n, k, true), empty_on(w, {ceil_div(k, block), n}, at::kFloat)};
             wq = ref_of(fresh);
             rowwise_into(wm, w_code, block, wq, st);
             cache_put(cache, "row", fresh);
@@ -811,11 +823,15 @@ PyObject* call(const char* name, const Args& args, Py_ssize_t want, Body body, b
 
 #define BI8_METHOD(name) PyObject* name##_py(PyObject*, PyObject* const* a, Py_ssize_t n)
 
-BI8_METHOD(quantize_rowwise) {
-    return call("quantize_rowwise", {a, n}, 2, [](const Args& g) { return [x = g.tensor(0), b = g.block(1)] { return quantize_rowwise(x, b); }; });
+BI8_METHOD(quantize_rowwise) {   // x, block, whether the result is only a GEMM operand
+    return call("quantize_rowwise", {a, n}, 3, [](const Args& g) {
+        return [x = g.tensor(0), b = g.block(1), operand = g.integer(2) != 0] { return quantize_rowwise(x, b, operand); };
+    });
 }
-BI8_METHOD(quantize_colwise) {
-    return call("quantize_colwise", {a, n}, 2, [](const Args& g) { return [x = g.tensor(0), b = g.block(1)] { return quantize_colwise(x, b); }; });
+BI8_METHOD(quantize_colwise) {   // x, block, whether the result is only a GEMM operand
+    return call("quantize_colwise", {a, n}, 3, [](const Args& g) {
+        return [x = g.tensor(0), b = g.block(1), operand = g.integer(2) != 0] { return quantize_colwise(x, b, operand); };
+    });
 }
 BI8_METHOD(quantize_dual) {
     return call("quantize_dual", {a, n}, 2, [](const Args& g) { return [x = g.tensor(0), b = g.block(1)] { return quantize_dual(x, b); }; });

@@ -50,19 +50,19 @@ def quantize_block_rowwise(x: torch.Tensor, fblock_size=None):
 
     Returns ``(q, state)``: ``q`` int8 ``[M, K]``; ``state`` float32 ``[ceil(K/block), M]`` holding
     ``max|x|`` of each block.  ``q = rint(127 * (x / state))`` (fp32 divide, fp32 multiply, round half to
-    even); an all-zero block gives state 0 and q 0.  Where ``K`` is not a multiple of 16 the
-    returned ``q`` is a view of a buffer whose row pitch is (same values), which the wide kernels and the GEMM want;
-    call ``.contiguous()`` where a dense tensor is needed."""
+    even); an all-zero block gives state 0 and q 0.  ``q`` is dense, except for a large 16-bit ``x`` (4 M elements, 256 on
+    each side) whose ``K`` is not a multiple of 16: there it is a view of a buffer with a row pitch that is (same
+    values), which the GEMM takes without a copy; call ``.contiguous()`` where a dense tensor is needed."""
     _scale_dtype()
-    return _native().quantize_rowwise(x, _block(fblock_size))
+    return _native().quantize_rowwise(x, _block(fblock_size), False)
 
 
 def quantize_block_colwise(x: torch.Tensor, fblock_size=None):
     """``quantize_block_rowwise(x.t().contiguous())`` without materialising the transpose
     (the pattern at ``block_linear.py:93-94`` and ``100-103``).  ``x`` is ``[R, C]``; returns int8 ``[C, R]``
-    and state ``[ceil(R/block), C]``, bit-identical to the two-step form."""
+    and state ``[ceil(R/block), C]``, bit-identical to the two-step form (``q`` is laid out as there)."""
     _scale_dtype()
-    return _native().quantize_colwise(x, _block(fblock_size))
+    return _native().quantize_colwise(x, _block(fblock_size), False)
 
 
 def quantize_block_dual(x: torch.Tensor, fblock_size=None):
@@ -145,6 +145,7 @@ def int8_matmul_block_partials(a, b, fblock_size=None, *, flags: int = 0):
 
 def fast_matmulT(a, b):
     """``a [M, K] @ b[N, K]^T`` with both operands quantized on the fly (``triton_functions.py:511-514``)."""
-    a_int8, a_state = quantize_block_rowwise(a)
-    b_int8, b_state = quantize_block_rowwise(b)
+    _scale_dtype()
+    a_int8, a_state = _native().quantize_rowwise(a, _block(), True)
+    b_int8, b_state = _native().quantize_rowwise(b, _block(), True)
     return int8_matmul_block64_rowwise_dequantize(a_int8, b_int8.t(), a_state, b_state)

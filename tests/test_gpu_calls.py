@@ -149,3 +149,57 @@ def test_residual_and_output_that_overlap(k):
     assert tf.pre_quantize_matmul_block_rowwise_dequantize("none", x, w.t(), sw, residual=res, out=res) is not None
     assert torch.equal(buf[:m], want) and torch.equal(buf[m:], before[m:])
     assert_clean_device()
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("r,c", [(1, 1), (1, 1001), (1001, 1), (300, 1001), (257, 264), (250, 20001), (2047, 2047)])
+def test_quantized_results_are_dense(r, c, dt):
+    """What callers get can be viewed, saved and handed on, whatever the row length, and so can the buffers of a layer."""
+    import io
+    from block_linear import BlockInt8Linear
+    tf = _tf()
+    set_config(64, dt)
+    x = randn_bf16((r, c), r + c).to(dt).to(DEV)
+    q_ref, s_ref = O.quantize(x.cpu(), 64)
+    qt_ref, st_ref = O.quantize(x.cpu().t().contiguous(), 64)
+    row, col, dual = tf.quantize_block_rowwise(x), tf.quantize_block_colwise(x), tf.quantize_block_dual(x)
+    for q, s in (row, dual[:2]):
+        assert q.is_contiguous() and torch.equal(q.view(-1).cpu(), q_ref.view(-1)) and torch.equal(s.cpu(), s_ref)
+    for q, s in (col, dual[2:]):
+        assert q.is_contiguous() and torch.equal(q.view(-1).cpu(), qt_ref.view(-1)) and torch.equal(s.cpu(), st_ref)
+    assert tf.rmsnorm_quantize_block_rowwise(x)[0].is_contiguous() and tf.silu_mul_quantize_block_rowwise(x, x)[0].is_contiguous()
+    lin = BlockInt8Linear(c, r, bias=False, device=DEV, dtype=dt).eval()
+    lin.weight.data = x
+    with torch.no_grad():
+        y = lin(x[:1])
+    assert torch.equal(lin.W_int8.view(-1).cpu(), q_ref.view(-1)) and lin.W_int8.untyped_storage().nbytes() == r * c
+    file = io.BytesIO()
+    torch.save(lin.state_dict(), file)
+    file.seek(0)
+    other = BlockInt8Linear(c, r, bias=False, device=DEV, dtype=dt).eval()
+    other.load_state_dict(torch.load(file))
+    with torch.no_grad():
+        assert torch.equal(other(x[:1]), y)
+    set_config(64)
+
+
+@pytest.mark.parametrize("r,c", [(4099, 1031), (1031, 4100)])
+def test_large_16_bit_results_are_views_with_a_pitch(r, c):
+    """From 4 M elements on rows that are not 16-byte aligned keep the pitch that the GEMM takes without a copy, as `.contiguous()`
+    has them; a product of two such matrices quantized on the fly agrees with the one of their dense copies."""
+    tf = _tf()
+    set_config(64)
+    x = randn_bf16((r, c), r).to(DEV)
+    q, s = tf.quantize_block_rowwise(x)
+    assert q.stride() == (-(-c // 16) * 16, 1)
+    q_ref, s_ref = O.quantize(x.cpu(), 64)
+    assert torch.equal(q.contiguous().view(-1).cpu(), q_ref.view(-1)) and torch.equal(s.cpu(), s_ref)
+    b = randn_bf16((300, c), 3).to(DEV)
+    bq, bs = tf.quantize_block_rowwise(b)
+    assert bq.is_contiguous()
+    want = tf.int8_matmul_block64_rowwise_dequantize(q.contiguous(), bq.t(), s, bs)
+    assert torch.equal(tf.fast_matmulT(x, b), want)
+    assert torch.equal(tf.int8_matmul_block64_rowwise_dequantize(q, bq.t(), s, bs), want)
+    from block_linear import fast_matmul
+    assert torch.equal(fast_matmul(x, b.t().contiguous()), want)
+    assert torch.equal(tf.fast_matmulT(x[:1], b), tf.int8_matmul_block64_rowwise_dequantize(q[:1].contiguous(), bq.t(), s[:, :1], bs))
