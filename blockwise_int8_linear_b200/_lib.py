@@ -30,6 +30,7 @@ EXPORTS = [
     "bi8_peer_allreduce_large_partial_offset", "bi8_peer_allreduce_large_out_offset", "bi8_rope_cache_append",
     "bi8_gemm_dequant_residual", "bi8_quantize_rowwise_pitched", "bi8_quantize_colwise_pitched", "bi8_quantize_dual_pitched",
     "bi8_quantize_rowwise_pre_pitched", "bi8_dequantize_rowwise_pitched", "bi8_column_sum", "bi8_column_sum_workspace_bytes",
+    "bi8_copy_rows",
 ]
 ADDEND_FULL = 0x100
 PRE_NONE, PRE_RMSNORM, PRE_SILU_MUL = 0, 1, 2
@@ -64,6 +65,7 @@ def lib() -> ctypes.CDLL:
         L.bi8_quantize_colwise_pitched.argtypes = [vp, i32, i64, vp, i64, vp, i64, i64, i32, vp]
         L.bi8_quantize_dual_pitched.argtypes = [vp, i32, i64, vp, i64, vp, vp, i64, vp, i64, i64, i32, vp]
         L.bi8_quantize_rowwise_pre_pitched.argtypes = [i32, vp, vp, i32, i64, vp, c.c_float, vp, i64, vp, i64, i64, i32, vp]
+        L.bi8_copy_rows.argtypes = [vp, i64, vp, i64, i64, i64, vp]
         L.bi8_column_sum.argtypes = [vp, i32, i64, vp, i64, i64, vp, sz, vp]
         L.bi8_column_sum_workspace_bytes.argtypes = [i64, i64]
         L.bi8_column_sum_workspace_bytes.restype = sz

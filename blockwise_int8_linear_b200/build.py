@@ -21,7 +21,7 @@ OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libbi8.so")
 NATIVE = os.path.join(HERE, "_native.so")
 NATIVE_SOURCE = "torch_ops.cpp"
-SOURCES = ["api.cu", "quantize.cu", "quantize_tile.cu", "gemm_generic.cu", "gemm_tc.cu", "gemm_tc_skinny.cu", "gemm_smallm.cu", "no_alloc.cu", "peer_reduce.cu", "peer_reduce_large.cu", "quantize_pre.cu", "column_sum.cu", "rope_cache.cu"]
+SOURCES = ["api.cu", "quantize.cu", "quantize_tile.cu", "gemm_generic.cu", "gemm_tc.cu", "gemm_tc_skinny.cu", "gemm_smallm.cu", "no_alloc.cu", "peer_reduce.cu", "peer_reduce_large.cu", "quantize_pre.cu", "column_sum.cu", "rope_cache.cu", "copy_rows.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",

@@ -263,6 +263,15 @@ int bi8_dequantize_rowwise(const int8_t* q, const float* s, void* out, int out_d
     return bi8_dequantize_rowwise_pitched(q, K, s, out, out_dtype, M, K, block, stream);
 }
 
+int bi8_copy_rows(const int8_t* src, int64_t lds, int8_t* dst, int64_t ldd, int64_t rows, int64_t cols, void* stream) {
+    if (rows < 0 || cols < 0 || lds < cols || ldd < cols)
+        return fail(BI8_ERR_SHAPE, "copy_rows: bad shape rows=%lld cols=%lld pitches %lld, %lld", (long long)rows, (long long)cols, (long long)lds, (long long)ldd);
+    if (rows == 0 || cols == 0) return BI8_OK;
+    if (!src || !dst) return fail(BI8_ERR_NULL, "copy_rows: null pointer");
+    if (!aligned(dst, 16) || ldd % 16 != 0) return fail(BI8_ERR_ALIGN, "copy_rows: the copy's rows must begin on 16-byte boundaries");
+    return launch_copy_rows(src, lds, dst, ldd, rows, cols, static_cast<cudaStream_t>(stream));
+}
+
 size_t bi8_column_sum_workspace_bytes(int64_t R, int64_t C) { return column_sum_workspace_bytes(R, C); }
 
 int bi8_column_sum(const void* x, int dtype, int64_t ldx, void* out, int64_t R, int64_t C, void* workspace, size_t workspace_bytes, void* stream) {

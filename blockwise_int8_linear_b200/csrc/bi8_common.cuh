@@ -106,6 +106,8 @@ int launch_peer_allreduce_large(void* const* peer_bufs, int rank, int world, int
 // rotary embedding of q and k and the append of k and v to the caches for one decode step (rope_cache.cu)
 int launch_rope_cache_append(const void* qkv, int dt, const float* cis, const long long* pos, void* q_out, void* kcache, void* vcache,
                              int64_t B, int64_t H, int64_t D, int64_t max_len, cudaStream_t st);
+// int8 rows of any alignment to rows on 16-byte boundaries (copy_rows.cu)
+int launch_copy_rows(const int8_t* src, int64_t lds, int8_t* dst, int64_t ldd, int64_t rows, int64_t cols, cudaStream_t st);
 // column sums in fp32 (column_sum.cu)
 size_t column_sum_workspace_bytes(int64_t R, int64_t C);
 int launch_column_sum(const void* x, int dt, int64_t ldx, void* out, int64_t R, int64_t C, void* workspace, size_t workspace_bytes,

@@ -162,15 +162,16 @@ Tensor empty_q(const Tensor& like, int64_t rows, int64_t cols, bool pitched) {
 }
 
 // Copy with a 16-byte aligned row pitch of an int8 operand that has none; the bytes between K and the pitch are never read.  What
-// is copied is the matrix that `m` describes, at the owner's address with the pitch `ld`: the owner itself may be that matrix or
+// is copied is the matrix that `m` describes, at its address and with its pitch: the owner itself may be that matrix or
 // its transpose, which its shape does not tell where both have the same.
-Mat repitch(const Mat& m, const Tensor& like) {
+Mat repitch(const Mat& m, const OnDevice& on) {
     if (m.ld % 16 == 0 && reinterpret_cast<uintptr_t>(m.ptr) % 16 == 0) return m;
     Mat out = m;
-    out.ld = ceil_div(m.cols, 16) * 16;
-    out.owner = empty_on(like, {m.rows, out.ld}, at::kChar);
-    out.owner.narrow(1, 0, m.cols).copy_(m.owner.as_strided({m.rows, m.cols}, {m.ld, 1}));
+    out.ld = pitch16(m.cols);
+    out.owner = empty_on(m.owner, {m.rows, out.ld}, at::kChar);
     out.ptr = out.owner.data_ptr();
+    check(bi8_copy_rows(static_cast<const int8_t*>(m.ptr), m.ld, static_cast<int8_t*>(out.owner.data_ptr()), out.ld, m.rows, m.cols, on.raw()),
+          "bi8_copy_rows");
     return out;
 }
 
@@ -275,7 +276,7 @@ struct Operands {
 };
 
 // Brings both int8 operands to the form the library takes: a [M, K] and b^T [N, K] with contiguous rows.
-Operands gemm_operands(const Tensor& a, const Tensor& b) {
+Operands gemm_operands(const Tensor& a, const Tensor& b, const OnDevice& on) {
     need_cuda(a);
     if (a.dim() != 2 || b.dim() != 2) value_error("expected 2-D operands, got " + shape_of(a) + " and " + shape_of(b));
     if (a.size(1) != b.size(0)) assertion("incompatible dimensions");
@@ -286,8 +287,8 @@ Operands gemm_operands(const Tensor& a, const Tensor& b) {
     // operands are re-pitched once.
     const int64_t k = a.size(1);
     if (k % 16 != 0 && k >= 256 && o.a.rows * o.bt.rows >= 128 * 128) {
-        o.a = repitch(o.a, a);
-        o.bt = repitch(o.bt, a);
+        o.a = repitch(o.a, on);
+        o.bt = repitch(o.bt, on);
     }
     return o;
 }
@@ -296,7 +297,7 @@ Tensor gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& state_x, const
             at::ScalarType out_type, int flags) {
     need_cuda(a_in);
     OnDevice on(a_in);
-    const Operands o = gemm_operands(a_in, b_in);
+    const Operands o = gemm_operands(a_in, b_in, on);
     const int64_t m = o.a.rows, n = o.bt.rows, k = o.a.cols, nb = ceil_div(k, block);
     check_scales(state_x, nb, m, block, "state_x");
     check_scales(state_w, nb, n, block, "state_w");
@@ -315,7 +316,7 @@ Tensor gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& state_x, const
 Tensor block_partials(const Tensor& a, const Tensor& b, int64_t block, int flags) {
     need_cuda(a);
     OnDevice on(a);
-    const Operands o = gemm_operands(a, b);
+    const Operands o = gemm_operands(a, b, on);
     const int64_t m = o.a.rows, n = o.bt.rows, k = o.a.cols;
     Tensor out = at::zeros({ceil_div(k, block), m, n}, at::TensorOptions().dtype(at::kInt).device(a.device()));
     check(bi8_gemm_block_partials(static_cast<const int8_t*>(o.a.ptr), o.a.ld, static_cast<const int8_t*>(o.bt.ptr), o.bt.ld,
@@ -428,7 +429,7 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
     if (k % 16 != 0) {
         // Rows that are not 16-byte aligned: the activations are quantized into rows that are, weights that have none (of
         // a layer, a checkpoint's dense copy) are re-pitched where the GEMM is long enough to gain from it.
-        if (k >= 256 && m * n >= 128 * 128) bt = repitch(bt, x_in);
+        if (k >= 256 && m * n >= 128 * 128) bt = repitch(bt, on);
         check(bi8_quantize_rowwise_pre_pitched(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps, xq, pitch16(k), sx, m, k,
                                                (int)block, on.raw()),
               "bi8_quantize_rowwise_pre");

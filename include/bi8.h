@@ -149,6 +149,11 @@ BI8_API int bi8_quantize_rowwise_pre_pitched(int op, const void* x, const void* 
 BI8_API int bi8_dequantize_rowwise_pitched(const int8_t* q, int64_t ldq, const float* s, void* out, int out_dtype,
                                            int64_t M, int64_t K, int block, void* stream);
 
+/* Copies int8 rows [rows, cols] of any alignment (pitch lds bytes) to rows that begin on 16-byte boundaries (dst 16-byte aligned,
+ * pitch ldd a multiple of 16), as the tensor-core GEMM wants its operands.  The bytes between a row's end and the next
+ * multiple of 16 are unspecified. */
+BI8_API int bi8_copy_rows(const int8_t* src, int64_t lds, int8_t* dst, int64_t ldd, int64_t rows, int64_t cols, void* stream);
+
 /* bi8_gemm_dequant for callers that cannot provide a workspace because they cannot allocate device memory when
  * they call: a serving loop that must not touch cudaMalloc after start-up, a plugin whose host runtime owns the
  * allocator, a caller with a fixed memory footprint.  (No counterpart in the reference, whose wrappers allocate

@@ -203,3 +203,18 @@ def test_large_16_bit_results_are_views_with_a_pitch(r, c):
     from block_linear import fast_matmul
     assert torch.equal(fast_matmul(x, b.t().contiguous()), want)
     assert torch.equal(tf.fast_matmulT(x[:1], b), tf.int8_matmul_block64_rowwise_dequantize(q[:1].contiguous(), bq.t(), s[:, :1], bs))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 15), (5, 16), (7, 17), (33, 31), (300, 1000), (1000, 4097)])
+@pytest.mark.parametrize("offset,extra", [(0, 0), (1, 0), (7, 3), (13, 9)])
+def test_copy_of_rows_of_any_alignment(rows, cols, offset, extra):
+    """Every byte of every row, none of what lies around the matrix, nothing written outside the copy."""
+    from blockwise_int8_linear_b200 import _lib
+    L, lds, ldd = _lib.lib(), cols + extra, -(-cols // 16) * 16
+    g = torch.Generator(device=DEV).manual_seed(rows + cols)
+    buf = torch.randint(-127, 128, (offset + rows * lds + 32,), generator=g, device=DEV, dtype=torch.int8)
+    src = buf[offset:].as_strided((rows, cols), (lds, 1))
+    dst = torch.full((rows * ldd + 64,), 99, device=DEV, dtype=torch.int8)
+    _lib.check(L.bi8_copy_rows(_lib.ptr(src), lds, _lib.ptr(dst), ldd, rows, cols, _lib.stream_ptr()), "copy_rows")
+    assert torch.equal(dst[:rows * ldd].view(rows, ldd)[:, :cols], src)
+    assert bool((dst[rows * ldd:] == 99).all())
