@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
+from torch.autograd import forward_ad as _forward_ad
 
 from . import _lib
 from . import block_linear_config
@@ -15,6 +16,7 @@ from .triton_functions import (
     dequantize_block_rowwise,
     int8_matmul_block64_rowwise_dequantize,
     quantize_block_colwise,
+    quantize_block_dual,
     quantize_block_rowwise,
 )
 from .triton_functions import _block, _pre_code, _scale_dtype
@@ -81,12 +83,48 @@ class blockwise_int8_linear(torch.autograd.Function):
     row-wise quantize.  With ``FUSE_DUAL_QUANTIZE`` (default) X and G are each read once for both of their
     quantizations, and the backward pass keeps X as its transposed int8 copy; every result is unchanged.
 
-    Both passes run in the extension as a native autograd node (``csrc/torch_ops.cpp``, ``LinearBackward``): a Python
-    ``Function`` costs the engine two interpreter calls per layer, which is more than a small layer's kernels take."""
+    ``apply`` runs both passes in the extension as a native autograd node (``csrc/torch_ops.cpp``, ``LinearBackward``): a Python
+    ``Function`` costs the engine two interpreter calls per layer, which is more than a small layer's kernels take.
+    ``forward`` and ``backward`` are the same steps in Python, for what looks at a ``Function`` itself: torch's function
+    transforms, forward-mode differentiation, both of which refuse it there, and classes derived from it."""
+
+    @classmethod
+    def apply(cls, X_3D, W, bias):
+        if cls is not blockwise_int8_linear or _forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active():
+            return super().apply(X_3D, W, bias)
+        return _lib.native().train_linear(X_3D, W, bias, getattr(block_linear_config, "FUSE_DUAL_QUANTIZE", True), _weight_cache(W))
 
     @staticmethod
-    def apply(X_3D, W, bias):
-        return _lib.native().train_linear(X_3D, W, bias, getattr(block_linear_config, "FUSE_DUAL_QUANTIZE", True), _weight_cache(W))
+    def forward(ctx, X_3D, W, bias):
+        X = X_3D.reshape(-1, X_3D.size(-1))
+        ctx.has_bias, ctx.block = bias is not None, _block()
+        ctx.x_quantized = ctx.needs_input_grad[1] and getattr(block_linear_config, "FUSE_DUAL_QUANTIZE", True)
+        if ctx.x_quantized:
+            X_int8, state_X, *kept = quantize_block_dual(X)
+        else:
+            X_int8, state_X = quantize_block_rowwise(X)
+            kept = [X]
+        ctx.save_for_backward(W, *kept)
+        W_int8, state_W = quantize_block_rowwise(W)
+        return int8_matmul_block64_rowwise_dequantize(X_int8, W_int8.t(), state_X, state_W, bias).view(*X_3D.size()[:-1], -1)
+
+    @staticmethod
+    def backward(ctx, G_3D):
+        if ctx.x_quantized and ctx.block != _block():
+            raise RuntimeError("GROUP_SIZE changed between the forward and the backward pass of a BlockInt8Linear")
+        G = G_3D.reshape(-1, G_3D.size(-1))
+        W, *kept = ctx.saved_tensors
+        grad_X = grad_W = grad_bias = None
+        if ctx.needs_input_grad[0]:             # contraction over N: both operands blocked along N (block_linear.py:92-95)
+            (G_int8, state_G), (Wt_int8, state_Wt) = quantize_block_rowwise(G), quantize_block_colwise(W)
+            grad_X = int8_matmul_block64_rowwise_dequantize(G_int8, Wt_int8.t(), state_G, state_Wt).view(*G_3D.size()[:-1], -1)
+        if ctx.needs_input_grad[1]:             # contraction over the tokens: both operands blocked along M (block_linear.py:100-104)
+            Xt_int8, state_Xt = kept if ctx.x_quantized else quantize_block_colwise(*kept)
+            Gt_int8, state_Gt = quantize_block_colwise(G)
+            grad_W = int8_matmul_block64_rowwise_dequantize(Gt_int8, Xt_int8.t(), state_Gt, state_Xt)
+        if ctx.has_bias and ctx.needs_input_grad[2]:
+            grad_bias = G.sum(dim=0)
+        return grad_X, grad_W, grad_bias
 
 
 class BlockInt8Linear(nn.Linear):

@@ -564,6 +564,9 @@ struct LinearBackward : public Node {
 variable_list LinearBackward::apply(variable_list&& grads) {
     variable_list out(3);
     if (!grads[0].defined()) return out;
+    // A backward pass that is itself recorded: the bias gradient is a sum of G that can be differentiated again.  The two products
+    // of quantized operands cannot.
+    const bool want_b = has_bias && task_should_compute_output(2), recorded = at::GradMode::is_enabled() && grads[0].requires_grad();
     int64_t b = 0;
     at::ScalarType type;
     try {
@@ -578,7 +581,7 @@ variable_list LinearBackward::apply(variable_list&& grads) {
         auto self = getptr();
         const Tensor saved_x = x.unpack(self), w = weight.unpack(self);
         at::AutoDispatchBelowADInplaceOrView below_autograd;
-        const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1), need_b = has_bias && task_should_compute_output(2);
+        const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1), need_b = want_b && !recorded;
         need_cuda(grads[0]);
         OnDevice on(grads[0]);
         const Mat g = mat_rows(grads[0]), wm = mat2d(w);
@@ -649,6 +652,7 @@ variable_list LinearBackward::apply(variable_list&& grads) {
         err.persist();
         throw err;
     }
+    if (want_b && recorded) out[2] = grads[0].reshape({-1, grads[0].size(-1)}).sum(0);
     return out;
 }
 

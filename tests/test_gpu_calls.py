@@ -218,3 +218,64 @@ def test_copy_of_rows_of_any_alignment(rows, cols, offset, extra):
     _lib.check(L.bi8_copy_rows(_lib.ptr(src), lds, _lib.ptr(dst), ldd, rows, cols, _lib.stream_ptr()), "copy_rows")
     assert torch.equal(dst[:rows * ldd].view(rows, ldd)[:, :cols], src)
     assert bool((dst[rows * ldd:] == 99).all())
+
+
+def _train_case(bias=True):
+    from block_linear import BlockInt8Linear
+    set_config(64)
+    lin = BlockInt8Linear(208, 144, bias, device=DEV, dtype=torch.bfloat16).train()
+    x = randn_bf16((2, 56, 208), 1).to(DEV).requires_grad_(True)
+    return lin, x, randn_bf16((2, 56, 144), 2, outliers=0).to(DEV)
+
+
+@pytest.mark.parametrize("fuse", [True, False])
+@pytest.mark.parametrize("frozen", ["", "x", "w"])
+def test_python_form_of_the_layer_equals_the_native_one(fuse, frozen):
+    """A class derived from the autograd function runs its `forward` and `backward`: bit for bit the native passes (whose
+    operands have aligned rows for every length, as these do for multiples of 16)."""
+    import block_linear_config as cfg
+    from block_linear import blockwise_int8_linear
+
+    class Derived(blockwise_int8_linear):
+        pass
+
+    lin, x, g = _train_case()
+    x.requires_grad_(frozen != "x")
+    lin.weight.requires_grad_(frozen != "w")
+    of = [t for t in (x, lin.weight, lin.bias) if t.requires_grad]
+    results = []
+    try:
+        cfg.FUSE_DUAL_QUANTIZE = fuse
+        for fn in (blockwise_int8_linear, Derived):
+            y = fn.apply(x, lin.weight, lin.bias)
+            results.append((y.detach(), *torch.autograd.grad(y, of, g)))
+    finally:
+        cfg.FUSE_DUAL_QUANTIZE = True
+    *native, native_b = results[0]
+    *python, python_b = results[1]
+    assert all(torch.equal(a, b) for a, b in zip(native, python)) and len(native) == len(python)
+    # the bias gradients are sums of bf16 values in fp32 in two orders: one rounding apart at most
+    assert ((native_b.float() - python_b.float()).abs() <= 2.0 ** -7 * native_b.float().abs() + 112 * 2.0 ** -23 * g.float().abs().sum((0, 1))).all()
+
+
+def test_forward_mode_differentiation_is_refused():
+    import torch.autograd.forward_ad as forward_ad
+    lin, x, _ = _train_case()
+    with forward_ad.dual_level():
+        assert lin(x).shape == (2, 56, 144)                   # nothing dual about it
+        with pytest.raises(RuntimeError, match="jvp"):
+            lin(forward_ad.make_dual(x.detach(), torch.ones_like(x)))
+        with pytest.raises(RuntimeError, match="jvp"):
+            torch.func.functional_call(lin, {"weight": forward_ad.make_dual(lin.weight.detach(), torch.ones_like(lin.weight))}, (x.detach(),))
+
+
+def test_recorded_backward_pass_keeps_the_bias_gradient_differentiable():
+    lin, x, _ = _train_case()
+    y = lin(x)
+    gx, gw, gb = torch.autograd.grad((y.float() ** 2).sum(), (x, lin.weight, lin.bias), create_graph=True)
+    assert gb.requires_grad and not gx.requires_grad and not gw.requires_grad
+    # d sum(gb) / d bias = 2 per row of y
+    again = torch.autograd.grad(gb.float().sum(), lin.bias)[0]
+    assert torch.equal(again.float(), torch.full((144,), 2.0 * 112, device=DEV))
+    plain = torch.autograd.grad((lin(x).float() ** 2).sum(), lin.bias)[0]
+    assert ((plain.float() - gb.detach().float()).abs() <= 2.0 ** -7 * plain.float().abs() + 1e-2).all()

@@ -204,6 +204,18 @@ def test_cpu_tensors_are_rejected_like_the_reference():
         tf.dequantize_block_rowwise(torch.zeros(4, 64, dtype=torch.int8), torch.zeros(1, 4))
 
 
+def test_function_transforms_refuse_the_layer():
+    """torch.func transforms do not see through the native node; they say so instead of failing on a wrapper's storage, and the autograd
+    function has the two methods that its base class is about."""
+    from block_linear import blockwise_int8_linear
+    x, w = torch.randn(4, 64), torch.randn(8, 64)
+    with pytest.raises(RuntimeError, match="setup_context"):
+        torch.func.grad(lambda z: blockwise_int8_linear.apply(z, w, None).sum())(x)
+    with pytest.raises(RuntimeError, match="setup_context"):
+        torch.vmap(lambda z: blockwise_int8_linear.apply(z, w, None))(x[None])
+    assert {"forward", "backward"} <= set(vars(blockwise_int8_linear))
+
+
 def test_replace_linear_on_cpu_module_structure():
     import torch.nn as nn
     from block_linear import BlockInt8Linear, replace_linear_with_blockwise_int8
