@@ -991,18 +991,22 @@ struct SplitPlan {
     int slot_floats = 0;
     size_t bytes = 0;
 };
-// What a work item takes per stage (128 K-bytes of a tile), what dividing costs whatever its size (the second kernel's latency; of
-// its host time a part) and per slot (80 KB written and read again through L2): microseconds, fitted to a sweep of 1 to 32 items per
-// tile over 12 shapes of 7 to 69 tiles and 2 to 86 stages.  The number of items with the lowest sum is taken; the largest that
-// the SMs hold is often not the fastest (512 x 768 x 768: 8.4 us in 6 items, 8.1 undivided and a launch less).
-constexpr double kStageUs = 0.72, kSplitUs = 2.9, kSlotUs = 0.017;
+// What a work item takes per stage (128 K-bytes of a tile: four, two or one blocks to promote), what dividing costs whatever its size
+// (the second kernel's latency; of its host time a part) and per slot (80 KB written and read again through L2): microseconds.
+// Stage: from 32 to 128 stages of 148 undivided tiles, 1.48 us at block 32, 0.71 at 64, 0.45 at 128.  The others from a
+// sweep of 1 to 32 items per tile over 14 shapes of 7 to 320 tiles and 6 to 86 stages at the three blocks: with them the plan's time is
+// within 6 % of the best measured one everywhere (512 x 768 x 768: 9.2 us in six items against 12.7 at block 32, 7.9 undivided
+// against 8.2 at 64, 6.5 against 7.3 at 128; 300 x 768 x 3072: 13.0 in eight, 10.6 in eight, 9.3 in six).  The number of
+// items with the lowest sum is taken; the largest that the SMs hold is often not the fastest.
+double stage_us(int block) { return block <= 32 ? 1.48 : block <= 64 ? 0.72 : 0.45; }
+constexpr double kSplitUs = 2.9, kSlotUs = 0.017;
 // Where the tiles alone occupy more than half of the SMs, dividing has to save a twentieth, the workspace stays within half of L2, and from
 // kSplitRounds rounds on nothing is left to be saved.
 constexpr double kSplitWorth = 0.95;
 constexpr size_t kSplitBytes = 64u << 20;
 constexpr int kSplitRounds = 6;
 
-SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int sms) {
+SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, int sms) {
     SplitPlan pl;
     const int bn = tc_bn();
     const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
@@ -1012,11 +1016,12 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int sms) {
     pl.slot_floats = (int)((M < kBM ? (M + 31) / 32 * 32 : kBM) * bn);
     auto rounds = [&](int64_t items) { return (double)((items + sms - 1) / sms); };
     const bool fills = tiles * 2 > sms;
-    double best = rounds(tiles) * kStageUs * nks * (fills ? kSplitWorth : 1.0);
+    const double stage = stage_us(block);
+    double best = rounds(tiles) * stage * nks * (fills ? kSplitWorth : 1.0);
     for (int want = 2; want <= 32 && want <= nks; ++want) {
         const int spp = (nks + want - 1) / want, s = (nks + spp - 1) / spp;
         if (fills ? (size_t)tiles * (size_t)s * (size_t)pl.slot_floats * 4 > kSplitBytes : tiles * want > sms) break;
-        const double cost = rounds(tiles * s) * kStageUs * spp + kSplitUs + kSlotUs * (double)(tiles * s);
+        const double cost = rounds(tiles * s) * stage * spp + kSplitUs + kSlotUs * (double)(tiles * s);
         if (cost < best) {
             best = cost;
             pl.ksplit = s;
@@ -1037,14 +1042,14 @@ bool gemm_tc_fills_device(const GemmArgs& g) {
 size_t gemm_tc_workspace_bytes(const GemmArgs& g) {
     const DeviceInfo di = device_info();
     if (!di.ok || g.partials != nullptr) return 0;
-    return plan_split(g.M, g.N, g.K, di.sms).bytes;
+    return plan_split(g.M, g.N, g.K, g.block, di.sms).bytes;
 }
 
 double gemm_tc_estimate_us(const GemmArgs& g) {
     const DeviceInfo di = device_info();
-    const SplitPlan pl = plan_split(g.M, g.N, g.K, di.sms);
+    const SplitPlan pl = plan_split(g.M, g.N, g.K, g.block, di.sms);
     const int64_t tiles = ((g.M + kBM - 1) / kBM) * ((g.N + tc_bn() - 1) / tc_bn()), items = tiles * pl.ksplit;
-    return kStageUs * (double)((items + di.sms - 1) / di.sms * pl.stages_per_split) + 3.5 + (pl.ksplit > 1 ? kSplitUs + kSlotUs * (double)items : 0.0);
+    return stage_us(g.block) * (double)((items + di.sms - 1) / di.sms * pl.stages_per_split) + 3.5 + (pl.ksplit > 1 ? kSplitUs + kSlotUs * (double)items : 0.0);
 }
 
 bool gemm_tc_applicable(const GemmArgs& g, const char** why) {
@@ -1116,7 +1121,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     SplitPlan pl;
     pl.stages_per_split = (int)((g.K + kBK - 1) / kBK);
     if (!partials) {
-        const SplitPlan want = plan_split(g.M, g.N, g.K, di.sms);
+        const SplitPlan want = plan_split(g.M, g.N, g.K, g.block, di.sms);
         // without a large enough, 16-byte aligned workspace the GEMM simply runs unsplit
         if (want.ksplit > 1 && g.workspace != nullptr && g.workspace_bytes >= want.bytes && aligned(g.workspace, 16)) pl = want;
     }

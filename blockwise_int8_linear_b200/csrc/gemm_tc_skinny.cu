@@ -1045,14 +1045,17 @@ int64_t gemm_skinny_part(const GemmArgs& g) {
 
 // Whether this kernel is also the faster one.  Up to 32 rows it always is.  From 33 on its promotion costs as much as the weights
 // take to arrive, and the general kernel overtakes it where it fills the SMs (clearly: a small layer keeps the reference's order of
-// operations): estimates in microseconds, from a sweep at 64 rows (4096 x 22016: 29 general, 45 here; x 11008: 23, 27; x 4096: 17, 13; 11008 x 4096: 25, 23).
+// operations): estimates in microseconds, the time of a stage by the blocks it promotes, from a sweep of 10 layer shapes at 40 and
+// 64 rows.  Measured at 64 rows, general against here, at block 32 / 64 / 128: 4096 x 22016: 56, 68 / 31, 46 / 22, 37;
+// 4096 x 12288: 54, 44 / 29, 32 / 20, 28; 4096 x 4096: 19, 18 / 13, 14 / 11, 12; 11008 x 4096: 36, 34 / 22, 24 / 17, 19.
 bool gemm_skinny_preferred(const GemmArgs& g) {
     if (!gemm_skinny_applicable(g)) return false;
     if (g.M <= 32) return true;
     SkLaunch l;
     const char* why = "";
     if (plan_launch(g, device_info().sms, &l) != BI8_OK || !gemm_tc_applicable(g, &why)) return true;
-    return 0.68 * (double)l.plan.cost + 4.0 <= gemm_tc_estimate_us(g) + 2.5;
+    const double stage_us = g.block <= 32 ? 1.2 : g.block <= 64 ? 0.9 : 0.7;
+    return stage_us * (double)l.plan.cost + 2.0 <= gemm_tc_estimate_us(g) + 2.5;
 }
 
 int launch_gemm_skinny(const GemmArgs& g, cudaStream_t st) {

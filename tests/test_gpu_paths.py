@@ -148,24 +148,69 @@ def test_bias_gradient_is_the_column_sum(rows, n, dt):
     set_config(64)
 
 
+@pytest.mark.parametrize("block", [32, 64, 128])
 @pytest.mark.parametrize("m,k,n", [(1024, 11008, 4096), (2000, 8200, 2001), (8192, 20000, 768)])
-def test_outputs_of_a_few_rounds_are_divided_over_k(m, k, n):
+def test_outputs_of_a_few_rounds_are_divided_over_k(m, k, n, block):
     """More tiles than half the SMs, a last range of K that is shorter, more parts than one batch of loads: against the undivided
     kernel, which is what a caller with the small built-in workspace still gets."""
     from tests.test_zz_no_alloc import _lib
     lib, L = _lib()
     gen = torch.Generator(device=DEV).manual_seed(k)
-    ld, nb = (k + 15) // 16 * 16, -(-k // 64)
+    ld, nb = (k + 15) // 16 * 16, -(-k // block)
     a, bt = (torch.randint(-127, 128, (r, ld), generator=gen, device=DEV, dtype=torch.int8)[:, :k] for r in (m, n))
     sa, sb = (torch.rand((nb, r), generator=gen, device=DEV) + 0.1 for r in (m, n))
     tf = _tf()
-    set_config(64)
-    assert L.bi8_gemm_workspace_bytes(m, n, k, 64) > 8 << 20
+    set_config(block)
+    assert L.bi8_gemm_workspace_bytes(m, n, k, block) > 8 << 20
     got = tf.int8_matmul_block64_rowwise_dequantize(a, bt.t(), sa, sb).float()
     c = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
     p = lib.ptr
-    lib.check(L.bi8_gemm_dequant_static(p(a), ld, p(bt), ld, p(sa), p(sb), None, 0, p(c), n, 0, m, n, k, 64, 0, lib.stream_ptr()), "static")
+    lib.check(L.bi8_gemm_dequant_static(p(a), ld, p(bt), ld, p(sa), p(sb), None, 0, p(c), n, 0, m, n, k, block, 0, lib.stream_ptr()), "static")
     want = c.float()
     assert ((got - want).norm() / want.norm()).item() <= 5e-3
     assert (got - want).abs().max().item() <= 2.0 ** -7 * want.abs().max().item()
     assert_clean_device()
+    set_config(64)
+
+
+@pytest.mark.parametrize("m,k,n,divided", [(512, 768, 768, {32}), (300, 3072, 768, {32, 64, 128}), (333, 1008, 776, {32, 64}), (768, 8192, 3072, set())])
+@pytest.mark.parametrize("block", [32, 64, 128])
+def test_division_over_k_knows_the_block(m, k, n, divided, block):
+    """A stage of block 32 takes three times one of block 128, so dividing pays earlier: which blocks divide a shape, and the result
+    against the undivided kernel (no workspace), as far apart as two orders of an fp32 sum are, and against the oracle."""
+    from tests.test_zz_no_alloc import _lib
+    lib, L = _lib()
+    set_config(block)
+    assert (L.bi8_gemm_workspace_bytes(m, n, k, block) > 0) == (block in divided)
+    xq, sx = O.quantize(randn_bf16((m, k), m, std=1.5), block)
+    wq, sw = O.quantize(randn_bf16((n, k), n, std=0.02), block)
+    a, bt, sa, sb = (t.to(DEV) for t in (xq, wq, sx, sw))
+    got = _tf().int8_matmul_block64_rowwise_dequantize(a, bt.t(), sa, sb).float()
+    c = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+    p = lib.ptr
+    lib.check(L.bi8_gemm_dequant(p(a), k, p(bt), k, p(sa), p(sb), None, 0, p(c), n, 0, m, n, k, block, None, 0, 0, lib.stream_ptr()), "undivided")
+    rows = torch.arange(0, m, 37)
+    ref = O.gemm(xq[rows], wq.t(), sx[:, rows], sw, None, block, torch.bfloat16).float()
+    for want in (c.float()[rows.to(DEV)].cpu(), ref):
+        assert (got[rows.to(DEV)].cpu() - want).abs().max().item() <= 2.0 ** -7 * want.abs().max().item()
+    assert ((got - c.float()).norm() / c.float().norm()).item() <= 5e-3
+    assert_clean_device()
+    set_config(64)
+
+
+@pytest.mark.parametrize("block", [32, 64, 128])
+@pytest.mark.parametrize("m,k,n", [(33, 512, 12288), (64, 4096, 12288), (40, 768, 2304), (64, 2048, 264)])
+def test_either_side_of_the_choice_at_33_to_64_rows(m, k, n, block):
+    """Where the line between the decode and the general kernel depends on the block: both, and the choice, against the oracle."""
+    tf = _tf()
+    set_config(block)
+    xq, sx = O.quantize(randn_bf16((m, k), m, std=1.5), block)
+    wq, sw = O.quantize(randn_bf16((n, k), n, std=0.02), block)
+    ref = O.gemm(xq, wq.t(), sx, sw, None, block, torch.bfloat16).float()
+    a, b, sa, sb = xq.to(DEV), wq.to(DEV).t(), sx.to(DEV), sw.to(DEV)
+    outs = [tf.int8_matmul_block64_rowwise_dequantize(a, b, sa, sb, flags=f) for f in (0, 2, 16)]
+    for got in outs:
+        assert (got.cpu().float() - ref).abs().max().item() <= 2.0 ** -7 * ref.abs().max().item()
+    assert torch.equal(outs[0], outs[1]) or torch.equal(outs[0], outs[2])
+    assert_clean_device()
+    set_config(64)
