@@ -279,3 +279,23 @@ def test_recorded_backward_pass_keeps_the_bias_gradient_differentiable():
     assert torch.equal(again.float(), torch.full((144,), 2.0 * 112, device=DEV))
     plain = torch.autograd.grad((lin(x).float() ** 2).sum(), lin.bias)[0]
     assert ((plain.float() - gb.detach().float()).abs() <= 2.0 ** -7 * plain.float().abs() + 1e-2).all()
+
+
+@pytest.mark.parametrize("block", [32, 64, 128])
+@pytest.mark.parametrize("m,k,n", [(1, 255, 64), (1, 257, 64), (8, 1001, 1000), (64, 257, 36), (65, 1001, 40), (16, 1001, 777), (40, 2049, 132)])
+def test_dense_layers_with_unaligned_rows(m, k, n, block):
+    """Few rows times a layer's dense weights, around the K from which they are copied to aligned rows, widths that the decode kernel
+    takes and does not take: against the oracle, plain and with a residual."""
+    from block_linear import BlockInt8Linear
+    set_config(block)
+    lin = BlockInt8Linear(k, n, bias=True, device=DEV, dtype=torch.bfloat16).eval()
+    lin.weight.data = randn_bf16((n, k), n, std=0.02).to(DEV)
+    lin.bias.data = randn_bf16((n,), 2).to(DEV)
+    x, res = randn_bf16((m, k), m + k, std=1.5), randn_bf16((m, n), 4)
+    ref = O.linear_forward(x, lin.weight.detach().cpu(), lin.bias.detach().cpu(), block)
+    with torch.no_grad():
+        _close(lin(x.to(DEV)), ref)
+        _close(lin.infer_pre(x.to(DEV), residual=res.to(DEV)), ref + res)
+    assert lin.W_int8.is_contiguous()
+    assert_clean_device()
+    set_config(64)
