@@ -17,22 +17,22 @@
 //   warp 1      issues tcgen05.mma kind::i8 (M128 N=BN K32): the MMAs of one quantisation block accumulate into one of
 //               three s32 accumulators in tensor memory, then a commit hands that accumulator to the promotion warps.
 //   warps 2-3   spare (they only take part in set-up and teardown; see the register note below)
-//   warps 4..   promotion + epilogue, PW warps per tensor-memory lane quarter.  A warp owns 32 rows x BN/PW columns of
+//   warps 4-19  promotion + epilogue, four warps per tensor-memory lane quarter.  A warp owns 32 rows x 40 columns of
 //               the tile.  Per block it reads its part of the finished accumulator in two halves (the second in flight
 //               while the first is folded), re-seeds what it has read, folds the values into fp32 accumulators in
 //               registers and releases the accumulator.  After the last block of a tile it casts, adds bias and writes
-//               its 32 x BN/PW part into a staging area in shared memory, from where one TMA store (or, for
+//               its 32 x 40 part into a staging area in shared memory, from where one TMA store (or, for
 //               destinations a tensor map cannot describe, a loop of coalesced stores) moves it out.
 // What bounds the kernel: the fold costs two FMAs per element and block (t = P*s_row, acc += s_col*t), 2*128*BN FMAs per
 // block on 128 FMA lanes = 320 cycles for BN = 160, twice the 163 cycles the MMAs of a 64-deep block need.  On top of
-// that every promotion warp reads its BN/PW column scales of every block from shared memory as broadcast loads, which
+// that every promotion warp reads its 40 column scales of every block from shared memory as broadcast loads, which
 // deliver 8 bytes per wavefront: 16 warps x ~21 wavefronts, plus the 144 wavefronts in which the tensor core reads the
 // block's operands, is ~520 shared-memory wavefronts per block on a pipe that serves one per cycle.  Measured (block 64)
 // the kernel needs ~790 cycles per block with the instruction issue slots 57 % and the shared-memory pipe 65 % busy.
 //
 // Registers: a scheduler (SM sub-partition) owns a quarter of the register file and every fourth warp, and setmaxnreg can
 // only move registers between warps of the same scheduler.  Each scheduler has exactly one of warps 0-3, which shrinks,
-// and PW promotion warps, which grow: PW = 4: 96 at launch -> 32 / 112; PW = 3: 128 -> 32 / 160; PW = 2: 168 -> 40 / 232.
+// and four promotion warps, which grow: 96 at launch -> 32 and 112.
 //
 // Seeded conversion (default): the promotion warps refill a drained accumulator with the bit pattern of 1.5*2^23 and
 // every MMA accumulates on top of it.  Integer addition on that pattern is exact float arithmetic while |P| < 2^22
@@ -66,27 +66,27 @@ constexpr uint32_t kABytes = kBM * kBK;  // 16 KiB
 constexpr uint32_t kSeedBits = 0x4B400000u;   // float 1.5 * 2^23
 constexpr float kSeedF = 12582912.0f;
 
-// Geometry that depends on the number of promotion warps per lane quarter.
-template <int PW>
+// Promotion warps per tensor-memory lane quarter, and what follows from it: a thread owns COLS columns of its row.  (Two or three
+// warps with 80 or 48 columns each were 7-18 % slower.)
+constexpr int kPW = 4;
 struct Cfg {
-    static_assert(PW == 2 || PW == 3 || PW == 4, "2, 3 or 4 promotion warps per lane quarter");
-    static constexpr int BN = PW == 3 ? 144 : 160;        // tile columns: kAccBufs * BN <= 512 tensor-memory columns
-    static constexpr int COLS = BN / PW;                  // columns owned by one promotion thread: 80, 48, 40
-    static constexpr int H0 = PW == 2 ? 40 : 24;          // the accumulator is read as columns [0, H0) and [H0, COLS)
-    static constexpr int H1 = COLS - H0;                  // 40, 24, 16
-    static constexpr int EPI_WARPS = 4 * PW;
+    static constexpr int BN = 160;                        // tile columns: kAccBufs * BN <= 512 tensor-memory columns
+    static constexpr int COLS = BN / kPW;                 // columns owned by one promotion thread
+    static constexpr int H0 = 24;                         // the accumulator is read as columns [0, H0) and [H0, COLS)
+    static constexpr int H1 = COLS - H0;
+    static constexpr int EPI_WARPS = 4 * kPW;
     static constexpr int THREADS = (kRoleWarps + EPI_WARPS) * 32;
-    static constexpr int LAUNCH_REGS = PW == 2 ? 168 : PW == 3 ? 128 : 96;     // 65536 / THREADS, rounded down to a multiple of 8
-    static constexpr int ROLE_REGS = PW == 2 ? 40 : 32;
-    static constexpr int EPI_REGS = PW == 2 ? 232 : PW == 3 ? 160 : 112;
+    static constexpr int LAUNCH_REGS = 96;                // 65536 / THREADS, rounded down to a multiple of 8
+    static constexpr int ROLE_REGS = 32;
+    static constexpr int EPI_REGS = 112;
     static constexpr uint32_t B_BYTES = BN * kBK;
     static constexpr uint32_t STAGE_BYTES = kABytes + B_BYTES;
     static constexpr uint32_t scale_off = kStages * STAGE_BYTES;
     // setmaxnreg moves registers inside a scheduler's share of the CTA's launch-time allocation: the total after the
     // moves must not exceed it, or setmaxnreg.inc blocks forever.  (The launcher also checks the register count the
     // compiler really chose for the kernel.)
-    static_assert(ROLE_REGS + PW * EPI_REGS <= (1 + PW) * LAUNCH_REGS, "register budget of a scheduler exceeds its launch allocation");
-    static_assert((1 + PW) * 32 * LAUNCH_REGS <= 16384, "launch allocation exceeds a scheduler's register file");
+    static_assert(ROLE_REGS + kPW * EPI_REGS <= (1 + kPW) * LAUNCH_REGS, "register budget of a scheduler exceeds its launch allocation");
+    static_assert((1 + kPW) * 32 * LAUNCH_REGS <= 16384, "launch allocation exceeds a scheduler's register file");
     static_assert(kAccBufs * BN <= 512 && COLS % 8 == 0 && H0 % 8 == 0 && H1 % 8 == 0 && BN % 16 == 0, "tile geometry");
     __host__ __device__ static constexpr uint32_t a_off(int s) { return (uint32_t)s * STAGE_BYTES; }
     __host__ __device__ static constexpr uint32_t b_off(int s) { return a_off(s) + kABytes; }
@@ -117,9 +117,9 @@ struct TcParams {
     int skip_stage;     // >= 0: diagnostic, the producer leaves this stage of its first work item out
 };
 
-template <int QB, int PW>
+template <int QB>
 struct Geo {
-    using C = Cfg<PW>;
+    using C = Cfg;
     static constexpr int BPS = kBK / QB;                        // quantisation blocks per stage
     static constexpr int MMAS = QB / 32;                        // MMAs (K = 32) per block
     static constexpr int SC_FLOATS = (BPS * (kBM + C::BN) + 31) / 32 * 32;   // scale floats per stage, [BPS][128] of sA then [BPS][BN] of sB, padded to 128 bytes
@@ -169,23 +169,12 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, uint32_
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, limit));
 }
 
-// NC (a multiple of 8, at most 40) consecutive accumulator columns of this thread's lane -> registers.
+// NC consecutive accumulator columns of this thread's lane -> registers.
 template <int NC>
 __device__ __forceinline__ void tmem_load_cols(uint32_t taddr, uint32_t (&S)[NC]) {
-    static_assert(NC == 40 || NC == 32 || NC == 24 || NC == 16 || NC == 8, "supported part widths");
-    if constexpr (NC == 32) {
-        tmem_ld32(taddr, S);
-    } else if constexpr (NC == 8) {
-        tmem_ld8(taddr, S);
-    } else if constexpr (NC == 40) {
-        tmem_ld32(taddr, reinterpret_cast<uint32_t(&)[32]>(S[0]));
-        tmem_ld8(taddr + 32u, reinterpret_cast<uint32_t(&)[8]>(S[32]));
-    } else if constexpr (NC == 24) {
-        tmem_ld16(taddr, reinterpret_cast<uint32_t(&)[16]>(S[0]));
-        tmem_ld8(taddr + 16u, reinterpret_cast<uint32_t(&)[8]>(S[16]));
-    } else {
-        tmem_ld16(taddr, reinterpret_cast<uint32_t(&)[16]>(S[0]));
-    }
+    static_assert(NC == 24 || NC == 16, "the two parts of a thread's columns");
+    tmem_ld16(taddr, reinterpret_cast<uint32_t(&)[16]>(S[0]));
+    if constexpr (NC == 24) tmem_ld8(taddr + 16u, reinterpret_cast<uint32_t(&)[8]>(S[16]));
 }
 
 // Blocks go round the kAccBufs = 3 accumulators and every stage has BPS blocks, so block `blk` of the stage at position
@@ -205,26 +194,22 @@ __device__ __forceinline__ uint32_t keep(uint32_t v) {
 }
 
 // Folds NC s32 words a thread has read from an accumulator (its row, columns C0 .. C0+NC-1 of its COLS, one quantisation
-// block) into its fp32 accumulators: acc[n] += sB[n] * (P[n] * s), both products as packed FMAs on column pairs (PACK1
-// false: the first one as scalar FMAs).  `sw` is the shared address of the block's column scales of this thread (16-byte
+// block) into its fp32 accumulators: acc[n] += sB[n] * (P[n] * s), both products as packed FMAs on column pairs.  `sw` is the shared address of the block's column scales of this thread (16-byte
 // aligned).
-template <bool SEED, bool PACK1, int C0, int NC, int COLS>
+template <bool SEED, int C0, int NC, int COLS>
 __device__ __forceinline__ void fold_columns(const uint32_t (&S)[NC], uint32_t sw, float sxd, float negc, uint64_t (&acc2)[COLS / 2]) {
     const uint64_t sxd2 = pack_f32x2(sxd, sxd), negc2 = pack_f32x2(negc, negc);
 #pragma unroll
     for (int q = 0; q < NC / 4; ++q) {
         uint64_t w0, w1, t0, t1;
         lds_2xb64(sw + (uint32_t)((C0 / 4 + q) * 16), w0, w1);
-        if (SEED && PACK1) {
+        if (SEED) {
             t0 = fma_f32x2(pack_u32x2(S[4 * q], S[4 * q + 1]), sxd2, negc2);
             t1 = fma_f32x2(pack_u32x2(S[4 * q + 2], S[4 * q + 3]), sxd2, negc2);
         } else {
             float t[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (SEED) t[u] = __fmaf_rn(__uint_as_float(S[4 * q + u]), sxd, negc);
-                else t[u] = __fmul_rn((float)(int32_t)S[4 * q + u], sxd);
-            }
+            for (int u = 0; u < 4; ++u) t[u] = __fmul_rn((float)(int32_t)S[4 * q + u], sxd);
             t0 = pack_f32x2(t[0], t[1]);
             t1 = pack_f32x2(t[2], t[3]);
         }
@@ -249,9 +234,9 @@ __device__ __forceinline__ void ldcg_v8(float (&f)[8], const float* src) {
 
 // Place of (lane quarter, column slice, group of eight columns, row of the quarter) in a workspace slot: a warp stores 1 KiB
 // runs, a thread 32 bytes of its row, and the reduction kernel reads a row's eight columns as one sector.
-template <int PW, int COLS>
+template <int COLS>
 __host__ __device__ constexpr int ws_index(int quarter, int slice, int group, int row) {
-    return (((quarter * PW + slice) * (COLS / 8) + group) * 32 + row) * 8;
+    return (((quarter * kPW + slice) * (COLS / 8) + group) * 32 + row) * 8;
 }
 
 // element n of a vector of type `dt`
@@ -363,13 +348,13 @@ __device__ __forceinline__ void add_staged(const TcParams& p, uint32_t row_addr,
     }
 }
 
-template <int QB, int MODE, bool SEED, int PW>
-__global__ void __launch_bounds__(Cfg<PW>::THREADS, 1)
+template <int QB, int MODE, bool SEED>
+__global__ void __launch_bounds__(Cfg::THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmSA, const __grid_constant__ CUtensorMap tmSB,
                const __grid_constant__ CUtensorMap tmC, const TcParams p) {
-    using C = Cfg<PW>;
-    using G = Geo<QB, PW>;
+    using C = Cfg;
+    using G = Geo<QB>;
     constexpr int BN = C::BN, COLS = C::COLS, H0 = C::H0, H1 = C::H1;
     constexpr bool kScales = (MODE == 0);           // the partial-sum dump uses no scales
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
@@ -566,7 +551,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int row = quarter * 32 + lane;
         const uint32_t t_lane = keep(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(slice * COLS));
         // eight spare tensor-memory columns of this warp's lanes keep the seed pattern
-        static_assert(kAccBufs * BN + 8 * PW <= 512, "no spare tensor-memory columns for the seed pattern");
+        static_assert(kAccBufs * BN + 8 * kPW <= 512, "no spare tensor-memory columns for the seed pattern");
         const uint32_t t_seed = keep(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(kAccBufs * BN + 8 * slice));
         // shared addresses of this thread's row scale and of its first column scale in scale stage 0, block 0
         const uint32_t sa_addr = keep(sc_ring_u32 + (uint32_t)(row * 4));
@@ -661,10 +646,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     tmem_wait_ld();
                     tmem_load_cols<H1>(t_acc + (uint32_t)H0, S1);    // second half, in flight during the fold of the first
                     reseed(t_acc, 0, H0);
-                    fold_columns<SEED, true, 0, H0, COLS>(S0, sw, sxd, negc, acc2);
+                    fold_columns<SEED, 0, H0, COLS>(S0, sw, sxd, negc, acc2);
                     tmem_wait_ld();
                     reseed(t_acc, H0, H1);
-                    fold_columns<SEED, true, H0, H1, COLS>(S1, sw, sxd, negc, acc2);
+                    fold_columns<SEED, H0, H1, COLS>(S1, sw, sxd, negc, acc2);
                 }
                 if (SEED) tmem_wait_st();
                 tc_fence_before();
@@ -697,7 +682,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (MODE == 0 && slot >= 0) {
                 // Part of a divided tile: straight from the registers to the item's workspace slot, in the order in which
                 // the reduction kernel reads it (ws_index: 32 bytes of one row per thread and step).
-                float* dst = p.ws + (int64_t)slot * p.slot_floats + ws_index<PW, COLS>(quarter, slice, 0, lane);
+                float* dst = p.ws + (int64_t)slot * p.slot_floats + ws_index<COLS>(quarter, slice, 0, lane);
                 const bool live = quarter * 32 * BN < p.slot_floats;
 #pragma unroll
                 for (int g = 0; g < COLS / 8; ++g) {
@@ -844,7 +829,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const TcParams p) {
     const int m = m0 + r, n = n0 + cg * 8;
     if (m >= p.M || n >= p.N) return;
     const int slice = cg / (COLS / 8), group = cg - slice * (COLS / 8);
-    const float* src = p.ws + (int64_t)t * p.ksplit * p.slot_floats + ws_index<BN / COLS, COLS>(r / 32, slice, group, r & 31);
+    const float* src = p.ws + (int64_t)t * p.ksplit * p.slot_floats + ws_index<COLS>(r / 32, slice, group, r & 31);
     const int live = p.N - n < 8 ? p.N - n : 8;
     const int64_t o = (int64_t)m * p.ldc + n, ro = (int64_t)m * p.ldr + n;
     float acc[8], bias[8], res[8];
@@ -948,33 +933,30 @@ struct TcMaps {
     CUtensorMap a, b, sa, sb, c;
 };
 
-template <int QB, int MODE, bool SEED, int PW>
+template <int QB, int MODE, bool SEED>
 int launch_one(const TcMaps& tm, const TcParams& p, int grid, cudaStream_t st) {
-    using C = Cfg<PW>;
-    constexpr size_t smem = Geo<QB, PW>::total + 1024;
+    constexpr size_t smem = Geo<QB>::total + 1024;
     static SmemOptIn opt_in;
-    const int rc = opt_in.ensure(gemm_tc_kernel<QB, MODE, SEED, PW>, smem);
+    const int rc = opt_in.ensure(gemm_tc_kernel<QB, MODE, SEED>, smem);
     if (rc != BI8_OK) return rc;
     // setmaxnreg.inc waits for registers that the role warps of the same scheduler give up: if the compiler gave the
     // kernel fewer registers per thread than the budget was written for, the wait would never end.  Checked once.
     static int regs_ok = 0;       // 0 unknown, 1 fine, -1 refused
     if (regs_ok == 0) {
         cudaFuncAttributes fa;
-        BI8_CUDA_TRY(cudaFuncGetAttributes(&fa, gemm_tc_kernel<QB, MODE, SEED, PW>));
-        regs_ok = ((1 + PW) * fa.numRegs >= C::ROLE_REGS + PW * C::EPI_REGS && (1 + PW) * 32 * fa.numRegs <= 16384) ? 1 : -1;
+        BI8_CUDA_TRY(cudaFuncGetAttributes(&fa, gemm_tc_kernel<QB, MODE, SEED>));
+        regs_ok = ((1 + kPW) * fa.numRegs >= Cfg::ROLE_REGS + kPW * Cfg::EPI_REGS && (1 + kPW) * 32 * fa.numRegs <= 16384) ? 1 : -1;
     }
     if (regs_ok < 0) return fail(BI8_ERR_CUDA, "tensor-core GEMM: the kernel was compiled with a register count its register moves do not fit");
-    return launch_chained(gemm_tc_kernel<QB, MODE, SEED, PW>, grid, C::THREADS, smem, st, tm.a, tm.b, tm.sa, tm.sb, tm.c, p);
+    return launch_chained(gemm_tc_kernel<QB, MODE, SEED>, grid, Cfg::THREADS, smem, st, tm.a, tm.b, tm.sa, tm.sb, tm.c, p);
 }
 
-// Promotion warps per lane quarter (and with it the tile width) of the kernel that runs.
-constexpr int kPW = 4;
-int tc_bn() { return Cfg<kPW>::BN; }
+int tc_bn() { return Cfg::BN; }
 
 template <int QB>
 int launch_qb(const TcMaps& tm, const TcParams& p, int grid, bool partials, bool seed, cudaStream_t st) {
-    if (partials) return seed ? launch_one<QB, 1, true, kPW>(tm, p, grid, st) : launch_one<QB, 1, false, kPW>(tm, p, grid, st);
-    return seed ? launch_one<QB, 0, true, kPW>(tm, p, grid, st) : launch_one<QB, 0, false, kPW>(tm, p, grid, st);
+    if (partials) return seed ? launch_one<QB, 1, true>(tm, p, grid, st) : launch_one<QB, 1, false>(tm, p, grid, st);
+    return seed ? launch_one<QB, 0, true>(tm, p, grid, st) : launch_one<QB, 0, false>(tm, p, grid, st);
 }
 
 }  // namespace
@@ -1149,9 +1131,9 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
         default: return fail(BI8_ERR_BLOCK, "tensor-core GEMM supports block 32, 64, 128 (got %d)", g.block);
     }
     if (rc != BI8_OK || pl.ksplit == 1) return rc;
-    constexpr int kTileItems = kBM * (Cfg<kPW>::BN / 8);
+    constexpr int kTileItems = kBM * (Cfg::BN / 8);
     auto reduce = [&](auto kernel) { return launch_chained(kernel, (unsigned)((tiles * kTileItems + 255) / 256), 256, 0, st, p); };
-    constexpr int BN = Cfg<kPW>::BN, COLS = Cfg<kPW>::COLS;
+    constexpr int BN = Cfg::BN, COLS = Cfg::COLS;
     if (pl.ksplit <= 2) return reduce(splitk_reduce_kernel<BN, COLS, 2>);
     return pl.ksplit <= 4 ? reduce(splitk_reduce_kernel<BN, COLS, 4>) : reduce(splitk_reduce_kernel<BN, COLS, 8>);
 }

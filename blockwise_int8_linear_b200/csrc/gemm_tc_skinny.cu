@@ -20,8 +20,9 @@
 //     rows' share of K that its own stages need (with the RMSNorm or SiLU * mul step in front, if asked for) and leaves it in
 //     shared memory as the MMA's swizzled operand tiles, while the first weights are on their way.  That is one launch
 //     and one kernel boundary less per layer; the redundancy (every cluster quantizes the same rows) is hidden behind
-//     the weights' first arrival.  From 33 rows on it would not be: those come from skinny_quantize_kernel or one of
-//     the producer quantizers, launched in front so that this kernel's set-up and first weight copies overlap them.
+//     the weights' first arrival only where a CTA's part is short.  Where it is not (kQuantInKernelValues in api.cu has the line
+//     and both sides) and above 16 rows they come from skinny_quantize_kernel or one of the producer
+//     quantizers, launched in front so that this kernel's set-up and first weight copies overlap them.
 //   * Warp roles: promotion warps (four per 16 activation rows, or per 32 for 64 rows; one per tensor-memory lane
 //     quarter) convert and scale; one producer warp issues, per stage, the TMA copies that complete on one
 //     barrier: 128 weight rows x 128 K-bytes, the stage's weight scales (a [blocks, 128] fp32 box of sB) and, with SRC 0,
@@ -924,7 +925,8 @@ int64_t stages_of(int64_t K, int bns) {
     return (K + ks - 1) / ks;
 }
 
-// f(Instance<...>) for the kernel instance of (block, bns, src), or `otherwise` where none is built
+// f(Instance<...>) for the kernel instance of (block, bns, src), or `otherwise` where none is built.  The dispatcher quantizes inside the
+// kernel up to 16 rows; the instances with 32 serve callers that ask for it or have no scratch (BI8_GEMM_QUANT_IN_KERNEL).
 template <typename R, typename F>
 R with_instance(int block, int bns, int src, R otherwise, F f) {
 #define BI8_SK(QB, BNS)                                          \

@@ -101,17 +101,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
     }
 }
 
-// The same for a whole converged warp: every lane polls; the result is made uniform with one vote, so that
-// a warp-aligned instruction after the wait is never reached by only some of the lanes.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint32_t abort_flag_smem) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag_smem));
-}
-
-// Asynchronous 16-byte / 4-byte copies global -> shared (no registers, no waiting in the issuing thread).
-// src_bytes < copy size zero-fills the remainder; with src_bytes == 0 nothing is read from `src`.
-__device__ __forceinline__ void cp_async_16(uint32_t dst_smem, const void* src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(src_bytes) : "memory");
-}
+// Asynchronous 4-byte copy global -> shared (no registers, no waiting in the issuing thread).
+// src_bytes 0 zero-fills the destination and reads nothing from `src`.
 __device__ __forceinline__ void cp_async_4(uint32_t dst_smem, const void* src, uint32_t src_bytes) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst_smem), "l"(src), "r"(src_bytes) : "memory");
 }
@@ -196,14 +187,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr)
         : "memory");
 }
-// Writes the same 32-bit value to 32 lanes x 16 consecutive columns.
-__device__ __forceinline__ void tmem_fill16(uint32_t taddr, uint32_t v) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr),
-        "r"(v)
-        : "memory");
-}
 // 32 lanes x 8 consecutive 32-bit columns.
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -215,13 +198,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
                  "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
-}
-// A register holding `bits` that the compiler cannot rematerialise (so a vector of them stays resident
-// instead of being rebuilt with moves before every store).
-__device__ __forceinline__ uint32_t opaque_u32(uint32_t bits) {
-    uint32_t r;
-    asm volatile("mov.b32 %0, %1;" : "=r"(r) : "r"(bits));
-    return r;
 }
 // packed fp32 pairs (one instruction, two lanes of data): d = a * b + c
 __device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
@@ -242,16 +218,6 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-// Writes the same 32-bit value to 32 lanes x 32 consecutive columns.
-__device__ __forceinline__ void tmem_fill32(uint32_t taddr, uint32_t v) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
-        "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr),
-        "r"(v)
-        : "memory");
-}
-
 template <int N>
 __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
