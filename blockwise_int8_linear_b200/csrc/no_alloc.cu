@@ -9,7 +9,7 @@
 // from a fixed array that lives inside the library.
 //
 // The array is a file-scope __device__ array of kScratchBytes: every GPU that loads the library holds that much
-// memory until the process exits.  A problem whose split-K plan needs more is rejected with BI8_ERR_LIMIT.
+// memory until the process exits.  A problem of few tiles whose split-K plan needs more is rejected with BI8_ERR_LIMIT.
 // Nothing here (or below it) calls cudaMalloc, cudaFree or an allocating library routine.
 //
 // In host code the array's name is only a handle; the kernels need its device address, which
@@ -60,12 +60,13 @@ size_t bi8_gemm_static_scratch_bytes(void) { return bi8::kScratchBytes; }
 int bi8_gemm_dequant_static(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb, const float* sA, const float* sB,
                             const void* bias, int bias_dtype, void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N,
                             int64_t K, int block, int flags, void* stream) {
-    // the plan that cannot be left out: split-K of the general kernel
+    // The plan that cannot be left out: split-K of the general kernel, at block 64 whatever the block, so that a shape is taken or
+    // refused for every block alike.  Another block's plan that does not fit the array runs undivided.
     bi8::GemmArgs shape{};
     shape.M = M;
     shape.N = N;
     shape.K = K;
-    shape.block = block;
+    shape.block = 64;
     const size_t need = (M > 0 && N > 0 && K > 0 && (block == 32 || block == 64 || block == 128)) ? bi8::gemm_tc_workspace_bytes(shape) : 0;
     if (need > bi8::kScratchBytes && !bi8::gemm_tc_fills_device(shape))
         return bi8::fail(BI8_ERR_LIMIT,
@@ -83,6 +84,7 @@ int bi8_gemm_dequant_static(const int8_t* A, int64_t lda, const int8_t* Bt, int6
     }
     // 33 to 64 rows run on the general kernel here, as this entry point has always promised
     const bool forced = (flags & (BI8_GEMM_FORCE_GENERIC | BI8_GEMM_FORCE_TC | BI8_GEMM_FORCE_SMALLM | BI8_GEMM_FORCE_SKINNY)) != 0;
+    shape.block = block;
     shape.A = A;
     shape.Bt = Bt;
     shape.lda = lda;

@@ -158,8 +158,8 @@ BI8_API int bi8_copy_rows(const int8_t* src, int64_t lds, int8_t* dst, int64_t l
  * they call: a serving loop that must not touch cudaMalloc after start-up, a plugin whose host runtime owns the
  * allocator, a caller with a fixed memory footprint.  (No counterpart in the reference, whose wrappers allocate
  * with torch on every call.)  The split-K scratch comes from a fixed 8 MiB array inside the library (reported by
- * bi8_gemm_static_scratch_bytes; every GPU that loads the library holds it until exit); a shape whose plan needs
- * more returns BI8_ERR_LIMIT.  No cudaMalloc/cudaFree or allocating library call is made.  The first call on a
+ * bi8_gemm_static_scratch_bytes; every GPU that loads the library holds it until exit); a shape of few tiles whose plan
+ * at block 64 needs more returns BI8_ERR_LIMIT (other plans that need more run undivided).  No cudaMalloc/cudaFree or allocating library call is made.  The first call on a
  * device looks up the array's device address: make it outside any stream capture.  All calls share the array
  * (nothing needs clearing between calls); calls that can overlap on one GPU race on it and must be serialised by
  * the caller.  Arguments and results are those of bi8_gemm_dequant (bit-identical where both select the same kernel;

@@ -99,3 +99,21 @@ def test_static_scratch_rejects_oversized_plans():
     p = lib.ptr
     rc = L.bi8_gemm_dequant_static(p(a), k, p(bt), k, p(sa), p(sb), p(bias), 0, p(c), n, 0, m, n, k, 64, 0, lib.stream_ptr())
     assert rc == -9 and b"built-in array" in L.bi8_last_error_string()
+
+
+@pytest.mark.parametrize("block", [32, 64, 128])
+@pytest.mark.parametrize("m,k,n,rc", [(512, 768, 768, 0), (300, 3072, 768, -9), (128, 1024, 1024, 0)])
+def test_static_scratch_takes_the_same_shapes_for_every_block(m, k, n, rc, block):
+    """At block 32 a GEMM is divided into more parts than at block 64 (512 x 768 x 768: six, 9.8 MB; not at all at 64): what does not
+    fit the array runs undivided, as without a workspace."""
+    lib, L = _lib()
+    a, bt, _, _, _ = _operands(m, k, n, seed=m)
+    sa, sb = (torch.rand((k // block, r), device="cuda") + 0.5 for r in (m, n))
+    c, want = (torch.zeros((m, n), dtype=torch.float32, device="cuda") for _ in range(2))
+    p = lib.ptr
+    got = L.bi8_gemm_dequant_static(p(a), k, p(bt), k, p(sa), p(sb), None, 0, p(c), n, 1, m, n, k, block, 0, lib.stream_ptr())
+    assert got == rc
+    if rc == 0:
+        lib.check(L.bi8_gemm_dequant(p(a), k, p(bt), k, p(sa), p(sb), None, 0, p(want), n, 1, m, n, k, block, None, 0, 0, lib.stream_ptr()), "undivided")
+        assert ((c - want).norm() / want.norm()).item() <= 1e-5
+    assert lib.device_status() == 0
