@@ -103,6 +103,11 @@ def test_bias_and_residual_behind_the_general_gemm(m, k, n, dt):
     plain = tf.quantize_matmul_block_rowwise_dequantize(x, wq.t(), sw)
     xq, sx = tf.quantize_block_rowwise(x)
     assert torch.equal(plain, tf.int8_matmul_block64_rowwise_dequantize(xq, wq.t(), sx, sw))
+    # 12 * 2^-24 of the terms' absolute sum and half a step of the output type
+    acc = O.gemm_acc(xq.cpu(), wq.cpu().t(), sx.cpu(), sw.cpu(), 64)
+    mag = O.gemm_term_abs_sum(xq.cpu(), wq.cpu().t(), sx.cpu(), sw.cpu(), 64)
+    step = {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12, torch.float32: 0.0}[dt]
+    assert ((plain.cpu().float() - acc).abs() <= 12 * 2.0 ** -24 * mag + 2 * step * acc.abs() + (6e-8 if dt == torch.float16 else 0.0)).all()
     for b in (None, bias):
         base = plain if b is None else plain + b.to(dt)
         assert torch.equal(tf.quantize_matmul_block_rowwise_dequantize(x, wq.t(), sw, b), base)
@@ -152,7 +157,7 @@ def test_bias_gradient_is_the_column_sum(rows, n, dt):
 @pytest.mark.parametrize("m,k,n", [(1024, 11008, 4096), (2000, 8200, 2001), (8192, 20000, 768)])
 def test_outputs_of_a_few_rounds_are_divided_over_k(m, k, n, block):
     """More tiles than half the SMs, a last range of K that is shorter, more parts than one batch of loads: against the undivided
-    kernel, which is what a caller with the small built-in workspace still gets."""
+    kernel, which is what a caller with the small built-in workspace still gets, and sampled rows against the oracle."""
     from tests.test_zz_no_alloc import _lib
     lib, L = _lib()
     gen = torch.Generator(device=DEV).manual_seed(k)
@@ -169,6 +174,9 @@ def test_outputs_of_a_few_rounds_are_divided_over_k(m, k, n, block):
     want = c.float()
     assert ((got - want).norm() / want.norm()).item() <= 5e-3
     assert (got - want).abs().max().item() <= 2.0 ** -7 * want.abs().max().item()
+    rows = torch.arange(0, m, m // 5)
+    ref = O.gemm(a[rows].cpu(), bt.cpu().t(), sa[:, rows].cpu(), sb.cpu(), None, block, torch.bfloat16).float()
+    assert (got[rows].cpu() - ref).abs().max().item() <= 2.0 ** -7 * ref.abs().max().item()
     assert_clean_device()
     set_config(64)
 

@@ -244,9 +244,9 @@ def test_colwise_block128_on_second_device(shape):
 
 @pytest.mark.parametrize("shape", [(4099, 1031), (1031, 4099), (4112, 1031)])
 def test_large_unaligned_tensors_are_padded_not_slowed(shape):
-    """Large 16-bit tensors whose row or column count is not a multiple of 16 (GPT-2's 50257-wide logits) are copied once
-    into a zero-padded buffer and go through the fast kernels; the results (returned as views of the padded outputs)
-    must equal the oracle's on the unpadded tensor, bit for bit."""
+    """Large 16-bit tensors whose row or column count is not a multiple of 16 (GPT-2's 50257-wide logits) go through the fast
+    kernels as they lie, into int8 rows with a padded pitch; the results (views of the padded outputs) must equal the
+    oracle's, bit for bit."""
     from triton_functions import quantize_block_colwise, quantize_block_dual, quantize_block_rowwise
     x = randn_bf16(shape, 11 * shape[0] + shape[1], outliers=0.01)
     xd = x.to(DEV)

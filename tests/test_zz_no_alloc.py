@@ -70,8 +70,8 @@ def test_static_scratch_entry_point_matches_workspace_entry_point():
 
 
 def test_static_scratch_too_small_for_the_decode_kernel_takes_the_general_kernel():
-    """33 <= M <= 64: the decode kernel's plan does not fit the built-in array, so the dispatcher declines it and the
-    general kernel runs with the array as its split-K scratch: same result as bi8_gemm_dequant forced onto that kernel."""
+    """33 <= M <= 64: this entry point takes the general kernel, with the array as its split-K scratch: same result as
+    bi8_gemm_dequant forced onto that kernel."""
     lib, L = _lib()
     m, k, n = 48, 4096, 4096
     a, bt, sa, sb, bias = _operands(m, k, n, seed=11)
