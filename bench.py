@@ -681,7 +681,7 @@ def tp_bench(dev, rank, world, hbm_gbs):
             tot.sort()
             t = torch.tensor([tot[len(tot) // 2]], device=dev, dtype=torch.float64)
             dist.all_reduce(t, op=dist.ReduceOp.MAX)
-            out[tag]["peer_reduce_fused"] = {"kernel": "bi8_row_parallel_linear (the decode GEMM's reduction kernel sums tile parts and ranks)",
+            out[tag]["peer_reduce_fused"] = {"kernel": "bi8_row_parallel_linear (a kernel chained behind the decode GEMM sums the ranks)",
                                              "ms_per_pair": t[0].item()}
             from blockwise_int8_linear_b200 import _lib
             _lib.device_status()

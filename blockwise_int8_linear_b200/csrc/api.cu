@@ -456,7 +456,7 @@ int bi8_row_parallel_linear_pre(int op, const void* x, const void* x2, int x_dty
     const bool forced = (flags & (BI8_GEMM_FORCE_GENERIC | BI8_GEMM_FORCE_TC | BI8_GEMM_FORCE_SMALLM | BI8_GEMM_QUANT_IN_KERNEL)) != 0;
     const bool x_vec = aligned(x, 16) && (ldx * dtype_size(x_dtype)) % 16 == 0;
     if (!forced && (x_vec || op != BI8_PRE_NONE) && K % 16 == 0 && aligned(xq, 16)) {
-        // decode-sized M: quantizer, weight-streaming GEMM, and a reduction kernel that sums the tile parts AND the ranks
+        // decode-sized M: quantizer, weight-streaming GEMM into `partial`, and a kernel behind it that sums the ranks
         GemmArgs g{xq, K, Wq, ldw, sx, sW, nullptr, 0, partial, N, BI8_F32, nullptr, M, N, K, block, flags, workspace, workspace_bytes};
         if (gemm_skinny_applicable(g)) {
             PeerEpilogue pe{&pa, bias, bias_dtype, out, out_dtype, peer_wait_limit_cycles(wait_limit_us)};

@@ -115,8 +115,8 @@ int launch_column_sum(const void* x, int dt, int64_t ldx, void* out, int64_t R, 
 int launch_dequantize_rowwise(const int8_t* q, int64_t ldq, const float* s, void* out, int dt, int64_t M, int64_t K,
                               int block, cudaStream_t st);
 
-// Row-parallel layers: the fp32 result in C is this rank's partial result; where the kernel that finishes the GEMM can, it
-// hands its values straight to the peer-memory reduction (peer_common.cuh) instead of leaving that to a second kernel.
+// Row-parallel layers: the fp32 result in C is this rank's partial result, which a kernel launched behind the decode GEMM (resident
+// as it ends) exchanges over peer memory (peer_common.cuh).
 struct PeerEpilogue {
     const void* args;         // const PeerArgs*
     const void* bias;
@@ -153,7 +153,7 @@ struct GemmArgs {
     bool after_own_quantizer = false;   // the kernel launched just before is this library's decode quantizer
     unsigned wait_limit_us = 0;         // diagnostic: limit of the general kernel's bounded waits (0 = default, about 2 s)
     int skip_stage = -1;                // diagnostic: the general kernel's producer leaves this stage of its first item out
-    const PeerEpilogue* peer = nullptr; // decode kernel only: reduce over the ranks inside its reduction kernel
+    const PeerEpilogue* peer = nullptr; // decode kernel only: sum C over the ranks in a kernel behind it
     const void* residual = nullptr;     // general tensor-core kernel only: [M, N] addend of the output type, added after the bias
     int64_t ldr = 0;                    // its row pitch in elements
     int64_t bias_ld = 0;                // decode kernel only: row pitch of `bias` in elements; non-zero makes it an [M, N] addend

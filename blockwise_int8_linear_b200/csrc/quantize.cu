@@ -300,8 +300,7 @@ __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
     }
 }
 
-// Row-wise quantize, any type / block / alignment: one warp per (row, block).
-// Row-wise quantize for rows that are not 16-byte aligned (row length not a multiple of 8, e.g. a 50257-wide vocabulary),
+// Row-wise quantize to int8 rows that are not 8-byte aligned (a dense result whose row length is not a multiple of 8),
 // block <= 64.  A warp takes kRagGroup consecutive blocks of one row; lane l handles elements l and l + 32 of every block, so
 // all loads of the group (2-byte, coalesced) are in flight before the first absmax reduction, and the stores are runs of 32
 // consecutive bytes.  Same arithmetic as every other quantizer (BlockQ).
@@ -344,6 +343,7 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_ragged_kernel(
     }
 }
 
+// Row-wise quantize, any type / block / alignment: one warp per (row, block).
 template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_rowwise_generic_kernel(
     const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int64_t M, int64_t K, int B,

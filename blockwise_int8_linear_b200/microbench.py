@@ -5,6 +5,7 @@
     python -m blockwise_int8_linear_b200.microbench colwise 8192 8192
     python -m blockwise_int8_linear_b200.microbench rmsnorm 4096 4096             # normalise + quantize in one kernel
     python -m blockwise_int8_linear_b200.microbench silu_mul 4096 11008           # silu(gate) * up + quantize in one kernel
+    python -m blockwise_int8_linear_b200.microbench column_sum 8192 12288         # the bias gradient
     python -m blockwise_int8_linear_b200.microbench gemm 4096 4096 11008          # M K N, int8 operands given
     python -m blockwise_int8_linear_b200.microbench gemm 16 4096 4096 --block 64
 
@@ -25,7 +26,7 @@ if ROOT not in sys.path:
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("op", choices=["quantize", "dequantize", "colwise", "dual", "rmsnorm", "silu_mul", "gemm"])
+    ap.add_argument("op", choices=["quantize", "dequantize", "colwise", "dual", "rmsnorm", "silu_mul", "column_sum", "gemm"])
     ap.add_argument("dims", type=int, nargs="+")
     ap.add_argument("--block", type=int, default=64)
     ap.add_argument("--reps", type=int, default=7)
@@ -49,6 +50,16 @@ def main():
         fn = lambda: F.int8_matmul_block64_rowwise_dequantize(xq, wq.t(), xs, ws, flags=a.flags)
         work = 2.0 * m * n * k
         nbytes = m * k + n * k + 4 * (m + n) * nb + 2 * m * n
+    elif a.op == "column_sum":
+        from blockwise_int8_linear_b200 import _lib
+        (m, k), work = a.dims, 0.0
+        x = torch.randn((m, k), device=dev, generator=g).to(torch.bfloat16)
+        out = torch.empty(k, device=dev, dtype=torch.bfloat16)
+        ws_bytes = _lib.lib().bi8_column_sum_workspace_bytes(m, k)
+        ws = torch.empty(max(ws_bytes, 1), device=dev, dtype=torch.uint8)
+        fn = lambda: _lib.check(_lib.lib().bi8_column_sum(_lib.ptr(x), _lib.BI8_BF16, k, _lib.ptr(out), m, k, _lib.ptr(ws), ws_bytes,
+                                                          _lib.stream_ptr()), "bi8_column_sum")
+        nbytes = 2 * m * k
     else:
         m, k = a.dims
         x = torch.randn((m, k), device=dev, generator=g).to(torch.bfloat16)

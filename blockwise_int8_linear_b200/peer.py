@@ -161,9 +161,9 @@ class PeerAllReduce:
         ``cast(sum over ranks of pre(x_r) @ W_r^T) + bias`` (or ``+ residual``, a tensor of the output's shape and type).
         ``op`` / ``x2`` / ``norm_weight`` / ``eps``: the producer step fused into the quantizer, as in
         ``pre_quantize_matmul_block_rowwise_dequantize`` ('silu_mul' for a gated MLP's down projection; 'rmsnorm' would
-        normalise over this rank's slice only and is rejected).  For decode-sized batches (at most 64 rows) the kernel that
-        finishes the weight-streaming GEMM exchanges its sums with the other ranks itself; the result equals
-        ``self(partial)`` on the fp32 output of ``quantize_matmul_block_rowwise_dequantize``."""
+        normalise over this rank's slice only and is rejected).  For decode-sized batches (at most 64 rows) that is three
+        chained launches: quantizer, weight-streaming GEMM into an fp32 partial result, and the exchange behind it; the result
+        equals ``self(partial)`` on the fp32 output of ``quantize_matmul_block_rowwise_dequantize``."""
         from .triton_functions import _block, ceil_div
         if op == "rmsnorm" and self.world > 1:
             raise ValueError("a row-parallel layer holds a slice of the features: normalise before the slice is taken")

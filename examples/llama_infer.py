@@ -131,7 +131,7 @@ class Int8Linear(nn.Module):
     def summed(self, x, op="none", x2=None, residual=None):
         """``residual + sum over the group of this row-parallel layer applied to pre(x)``, cast to the activation type: for
         decode-sized inputs with the peer-memory reduction installed, one library call whose first kernel applies `op` and
-        quantizes and whose last kernel adds the GEMM's tile parts, the ranks and the residual."""
+        quantizes and whose last kernel adds the ranks' partial results and the residual."""
         peer = self.world > 1 and self.mode == "row" and PEER is not None and self.lin is not None
         if peer:
             rows = x.numel() // x.shape[-1]

@@ -114,7 +114,8 @@ BI8_API size_t bi8_column_sum_workspace_bytes(int64_t R, int64_t C);
  * bias [N] of bias_dtype or NULL.  C [M,N] of out_dtype, row stride ldc.
  * workspace: bi8_gemm_workspace_bytes(M,N,K,block) bytes of 16-byte aligned device memory (may be NULL when that
  * is 0; without it shapes with few output tiles run slower).  It is plain scratch: nothing has to be cleared, every
- * call overwrites what it later reads; calls that may run concurrently need separate workspaces.
+ * call overwrites what it later reads; calls that may run concurrently, or that several threads enqueue on one stream (a call
+ * is more than one launch), need separate workspaces.
  * The int32 partial sums are exact.  The fp32 accumulation of the tensor-core kernel for M > 64 evaluates a term as
  * sB * fl(P * s) with s = sA/127^2 rounded to fp32 and then to 22 significant bits (relative error of s at most
  * 2^-24 + 2^-22), one rounding for P*s and one for the fused multiply-add into the sum, where the reference rounds
@@ -288,8 +289,8 @@ BI8_API int bi8_peer_allreduce_large(void* const* peer_bufs, int rank, int world
 
 /* A whole row-parallel layer in one call: quantize x [M,K] (this rank's slice of the input features), multiply with this
  * rank's weight slice Wq [N,K] / sW, and sum the ranks' fp32 partial results as bi8_peer_allreduce does.  For M <= 64
- * (decode) the kernel that adds the weight-streaming GEMM's tile parts hands its sums straight to the exchange, so the layer
- * is three launches (quantizer, GEMM, reduction over parts and ranks) with no fp32 round trip in between; other shapes run
+ * (decode) the layer is three chained launches: quantizer, weight-streaming GEMM into `partial`, and the exchange, whose CTAs
+ * are resident as the GEMM ends; other shapes run
  * bi8_gemm_dequant_fused_quant into `partial` followed by bi8_peer_allreduce.  Same results as those two calls.
  * xq [M,K] int8 and sx [ceil(K/block), M] fp32 are scratch as in bi8_gemm_dequant_fused_quant; partial [M,N] fp32 is scratch
  * (16-byte aligned); workspace as in bi8_gemm_dequant; peer_bufs .. capacity, bias, out, wait_limit_us as in
