@@ -164,10 +164,6 @@ Tensor empty_q(const Tensor& like, int64_t rows, int64_t cols, bool pitched) {
 // Copy with a 16-byte aligned row pitch of an int8 operand that has none; the bytes between K and the pitch are never read.  What
 // is copied is the matrix that `m` describes, at its address and with its pitch: the owner itself may be that matrix or
 // its transpose, which its shape does not tell where both have the same.
-// Without it the GEMM is the CUDA-core kernel's, whose time grows with K: against copy and tensor cores 4.5 and 5 us at K = 65
-// (1 to 40 rows, 64 to 4000 columns), 7 and 5 at 129, 11 and 6 at 257, 20 and 7 at 513, 36 and 8 at 1001.  A launch is 2.5 us of
-// host time, so the line is where the copies of both operands are paid for.
-constexpr int64_t kRepitchK = 256;
 Mat repitch(const Mat& m, const OnDevice& on) {
     if (m.ld % 16 == 0 && reinterpret_cast<uintptr_t>(m.ptr) % 16 == 0) return m;
     Mat out = m;
@@ -178,6 +174,12 @@ Mat repitch(const Mat& m, const OnDevice& on) {
           "bi8_copy_rows");
     return out;
 }
+
+// Whether that is worth its launches.  Without it the GEMM is the CUDA-core kernel's, whose time grows with K for any output: against copy
+// and tensor cores 4.5 and 5 us at K = 65 (1 to 40 rows, 64 to 4000 columns), 7 and 5 at 129, 11 and 6 at 257, 20 and 7 at 513, 36
+// and 8 at 1001; and with the output for any K: 1024 x 2000 takes 11 and 7 us at K = 17, 19 and 7 at 65, 29 and 8 at 129, 8192 x 4096
+// takes 126 and 24, 260 and 28, 407 and 35.  A launch is 2.5 us of host time: the lines are where it is paid for.
+bool worth_repitch(int64_t m, int64_t n, int64_t k) { return k % 16 != 0 && (k >= 256 || m * n >= (1ll << 27) / (k + 64)); }
 
 // ---- quantizers ---------------------------------------------------------------------------------------------------------
 struct Quantized {
@@ -287,11 +289,11 @@ Operands gemm_operands(const Tensor& a, const Tensor& b, const OnDevice& on) {
     if (a.scalar_type() != at::kChar || b.scalar_type() != at::kChar)
         value_error(std::string("operands must be int8, got ") + c10::toString(a.scalar_type()) + " and " + c10::toString(b.scalar_type()));
     Operands o{mat2d(a), mat2d_t(b)};
-    // The tensor-core kernels need 16-byte aligned operand rows: for a long contraction that is not a multiple of 16 both
-    // operands are re-pitched once (kRepitchK).  Not for a narrow output of more rows than the decode kernel takes: callers
-    // get the reference's order of operations there, from the CUDA cores.
-    const int64_t k = a.size(1);
-    if (k % 16 != 0 && k >= kRepitchK && (o.a.rows <= 64 || o.a.rows * o.bt.rows >= 128 * 128)) {
+    // The tensor-core kernels need 16-byte aligned operand rows: where it is worth it both operands are re-pitched once.  Not for
+    // a narrow output of more rows than the decode kernel takes: callers get the reference's order of operations there,
+    // from the CUDA cores.
+    const int64_t m = o.a.rows, n = o.bt.rows;
+    if (worth_repitch(m, n, a.size(1)) && (m <= 64 || m * n >= 128 * 128)) {
         o.a = repitch(o.a, on);
         o.bt = repitch(o.bt, on);
     }
@@ -434,7 +436,7 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
     if (k % 16 != 0) {
         // Rows that are not 16-byte aligned: the activations are quantized into rows that are, weights that have none (of
         // a layer, a checkpoint's dense copy) are re-pitched where the GEMM is long enough to gain from it.
-        if (k >= kRepitchK) bt = repitch(bt, on);
+        if (worth_repitch(m, n, k)) bt = repitch(bt, on);
         check(bi8_quantize_rowwise_pre_pitched(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps, xq, pitch16(k), sx, m, k,
                                                (int)block, on.raw()),
               "bi8_quantize_rowwise_pre");

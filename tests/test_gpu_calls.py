@@ -282,9 +282,10 @@ def test_recorded_backward_pass_keeps_the_bias_gradient_differentiable():
 
 
 @pytest.mark.parametrize("block", [32, 64, 128])
-@pytest.mark.parametrize("m,k,n", [(1, 255, 64), (1, 257, 64), (8, 1001, 1000), (64, 257, 36), (65, 1001, 40), (16, 1001, 777), (40, 2049, 132)])
+@pytest.mark.parametrize("m,k,n", [(1, 255, 64), (1, 257, 64), (8, 1001, 1000), (64, 257, 36), (65, 1001, 40), (16, 1001, 777), (40, 2049, 132),
+                                   (300, 17, 5600), (2048, 65, 500), (2048, 65, 520)])
 def test_dense_layers_with_unaligned_rows(m, k, n, block):
-    """Few rows times a layer's dense weights, around the K from which they are copied to aligned rows, widths that the decode kernel
+    """A layer's dense weights around the K and the outputs from which they are copied to aligned rows, widths that the decode kernel
     takes and does not take: against the oracle, plain and with a residual."""
     from block_linear import BlockInt8Linear
     set_config(block)
