@@ -1113,7 +1113,8 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     p.residual = g.residual;
     p.ldr = g.ldr;
     p.res_vec = (g.residual != nullptr && aligned(g.residual, 16) && (g.ldr * esz) % 16 == 0) ? 1 : 0;
-    if (!partials && pl.ksplit == 1 && p.vec_store) {
+    // (a tensor map clips at 16 bytes: where rows end inside such a piece, the bytes behind them would be written)
+    if (!partials && pl.ksplit == 1 && p.vec_store && (g.N * esz) % 16 == 0) {
         // one box = what a promotion warp stages per pass: 32 rows x (its columns, or half of them for 4-byte elements)
         const int cols = bn / kPW;
         rc = cached_output_map(&tm.c, dev, g.C, esz, g.M, g.N, g.ldc, 32, esz == 2 ? cols : cols / 2);

@@ -280,6 +280,46 @@ def test_bounded_wait_gives_up_cleanly():
     set_config(64)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [
+    # (M, N, row pitch of C beyond N, elements between a 16-byte boundary and C)
+    (1, 160, 0, 0), (128, 161, 0, 0), (129, 163, 0, 1), (33, 7, 2, 3), (300, 330, 5, 7), (257, 240, 3, 2), (130, 1, 0, 5), (64, 488, 8, 0),
+])
+def test_tile_store_paths(shape, dtype):
+    """Undivided tiles reach C by tensor map or, where none describes it, from the promotion warps: the same bits at every alignment,
+    and nothing written outside the M x N elements (a pitch of whole 16-byte pieces with rows that end inside one)."""
+    from blockwise_int8_linear_b200 import _lib
+    L = _lib.lib()
+    set_config(64, dtype)
+    m, n, more, lead = shape
+    k = 128                                            # one stage: no plan divides it
+    xq, xs, wq, ws = quantized_pair(m, k, n, 64, seed=m * 7 + n)
+    a, bt, sa, sb = xq.to(DEV), wq.to(DEV), xs.to(DEV), ws.to(DEV)
+    bias = torch.randn(n, generator=torch.Generator().manual_seed(n)).to(dtype).to(DEV)
+    code = {torch.bfloat16: _lib.BI8_BF16, torch.float16: _lib.BI8_F16, torch.float32: _lib.BI8_F32}[dtype]
+    for b in (None, bias):
+        outs = []
+        for pitch, off in (((n + 7) // 8 * 8, 0), (n + more, lead)):
+            buf = torch.full((off + m * pitch + 64,), 77.0, dtype=dtype, device=DEV)
+            c = buf[off:off + m * pitch].view(m, pitch)
+            rc = L.bi8_gemm_dequant(_lib.ptr(a), k, _lib.ptr(bt), k, _lib.ptr(sa), _lib.ptr(sb), None if b is None else _lib.ptr(b), code,
+                                    c.data_ptr(), pitch, code, m, n, k, 64, None, 0, TC, _lib.stream_ptr())
+            _lib.check(rc, "bi8_gemm_dequant")
+            outs.append(c[:, :n].clone())
+            c[:, :n] = 77.0
+            assert bool((buf == 77.0).all())
+        assert torch.equal(outs[0], outs[1])
+        acc = O.gemm_acc(xq, wq.t(), xs, ws, 64)
+        ref = acc.to(dtype) if b is None else acc.to(dtype) + b.cpu()
+        mag = O.gemm_term_abs_sum(xq, wq.t(), xs, ws, 64)
+        # one rounding of the sum to the output type, a second one where a bias follows
+        step = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -24}[dtype]
+        bound = FP32_TOL * mag + 2 * step * (acc.abs() + ref.float().abs()) + 1e-30
+        assert bool(((outs[1].float().cpu() - ref.float()).abs() <= bound).all())
+    assert_clean_device()
+    set_config(64)
+
+
 def test_unaligned_long_contraction_is_repitched_onto_the_tensor_cores():
     """K = 1000 + 17: not a multiple of 16.  The shim re-pitches the operands; results equal the CUDA-core kernel's
     within the tensor-core tolerance and the int32 partial sums stay exact."""
