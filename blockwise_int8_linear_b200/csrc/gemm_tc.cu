@@ -7,38 +7,42 @@
 //
 // One persistent CTA per SM works on 128 x BN output tiles.  Warp roles:
 //   warp 0      producer.  Per stage two TMA copies of 128-byte-swizzled K-major operand tiles (A: 128 rows, Bt: BN
-//               rows, 128 K-bytes) into a ring of kStages slots, and two TMA copies of the stage's block scales (an
-//               fp32 box [blocks, 128] of sA and [blocks, BN] of sB) into a ring of kScaleStages slots, all four on the
-//               stage's one "full" barrier.  Scale tensors that a tensor map cannot describe (base or row length not
-//               16-byte aligned) are copied with cp.async by the warp's 32 lanes instead, arriving on the same barrier.
-//               The scale ring needs no barriers of its own: the promotion warps read a stage's scales only after
-//               they have seen one of its accumulators complete (the MMAs were issued after the stage's barrier), and
-//               the ring is deep enough that a slot is never rewritten while in use (see kScaleStages).
+//               rows, 128 K-bytes) into a ring of kStages slots, and two TMA copies of the stage's block scales (fp32
+//               boxes [blocks, BN] of sA and of sB) into rings of SC_STAGES slots, all four on the stage's one "full"
+//               barrier.  Scale tensors that a tensor map cannot describe (base or row length not 16-byte aligned) are
+//               copied with cp.async by the warp's 32 lanes instead, arriving on the same barrier.  The scale rings need
+//               no barriers of their own: the promotion warps read a stage's scales only after they have seen one of
+//               its accumulators complete (the MMAs were issued after the stage's barrier), and the rings are deep
+//               enough that a slot is never rewritten while in use (SC_STAGES).
 //   warp 1      issues tcgen05.mma kind::i8 (M128 N=BN K32): the MMAs of one quantisation block accumulate into one of
 //               three s32 accumulators in tensor memory, then a commit hands that accumulator to the promotion warps.
-//   warps 2-3   spare (they only take part in set-up and teardown; see the register note below)
-//   warps 4-19  promotion + epilogue, four warps per tensor-memory lane quarter.  A warp owns 32 rows x 40 columns of
-//               the tile.  Per block it reads its part of the finished accumulator in two halves (the second in flight
-//               while the first is folded), re-seeds what it has read, folds the values into fp32 accumulators in
-//               registers and releases the accumulator.  After the last block of a tile it casts, adds bias and writes
-//               its 32 x 40 part into a staging area in shared memory, from where one TMA store (or, for
-//               destinations a tensor map cannot describe, a loop of coalesced stores) moves it out.
-// What bounds the kernel: the fold costs two FMAs per element and block (t = P*s_row, acc += s_col*t), 2*128*BN FMAs per
-// block on 128 FMA lanes = 320 cycles for BN = 160, twice the 163 cycles the MMAs of a 64-deep block need.  On top of
-// that every promotion warp reads its 40 column scales of every block from shared memory as broadcast loads, which
-// deliver 8 bytes per wavefront: 16 warps x ~21 wavefronts, plus the 144 wavefronts in which the tensor core reads the
-// block's operands, is ~520 shared-memory wavefronts per block on a pipe that serves one per cycle.  Measured (block 64)
-// the kernel needs ~790 cycles per block with the instruction issue slots 57 % and the shared-memory pipe 65 % busy.
+//   warp 2      seeder: puts the seed pattern (below) into every accumulator that the promotion warps have released.
+//   warp 3      storer: moves finished tiles from shared memory to C by TMA stores.
+//   warps 4-19  promotion, four warps per tensor-memory lane quarter.  A warp owns 32 rows x 40 columns of the tile.  Per
+//               block it reads its part of the finished accumulator eight columns at a time (the next eight in flight
+//               while eight are folded), folds the values into fp32 accumulators in registers, and releases the
+//               accumulator as soon as the last columns are in registers.  After the last block of a tile it casts,
+//               stages its 32 x 40 part in shared memory, adds bias and residual there and goes on with the next tile.
+// What bounds the kernel: the fold, t = P*s_row and acc += s_col*t for two columns per FFMA2.  The first has one operand that changes, the
+// second three, and a packed FMA with three 64-bit operands of its own issues every 3.2 to 3.5 cycles, not every 2 (measured in
+// isolation; two scalar FMAs are no faster): 430 cycles per 128 x 160 block for the FMAs alone, against 163 for the MMAs of a
+// 64-deep block.  With the tensor-memory reads, the column scales (broadcast loads, 8 bytes per shared-memory wavefront, in
+// competition with the tensor core's operand reads) and the hand-over of accumulators the loop takes 600-640 cycles per block of
+// 32 or 64 and 720-750 at 128.  8192 x 4096 x 11008: 716 -> 681 us at block 64, 449 -> 423 at 128, 1470 -> 1370 at 32.
 //
 // Registers: a scheduler (SM sub-partition) owns a quarter of the register file and every fourth warp, and setmaxnreg can
 // only move registers between warps of the same scheduler.  Each scheduler has exactly one of warps 0-3, which shrinks,
 // and four promotion warps, which grow: 96 at launch -> 32 and 112.
 //
-// Seeded conversion (default): the promotion warps refill a drained accumulator with the bit pattern of 1.5*2^23 and
-// every MMA accumulates on top of it.  Integer addition on that pattern is exact float arithmetic while |P| < 2^22
-// (127^2 * 128 < 2^22), so the word read back is the float 1.5*2^23 + P and
+// Seeded conversion (default): every accumulator starts as the bit pattern of 1.5*2^23 and the MMAs accumulate on top
+// of it.  Integer addition on that pattern is exact float arithmetic while |P| < 2^22 (127^2 * 128 < 2^22), so the word
+// read back is the float 1.5*2^23 + P and
 //   t = fma(word, s, -1.5*2^23 * s) = fl(P * s)
 // needs no int->float conversion.  s = sA[j,m]/127^2 rounded to 22 significant bits makes 1.5*2^23*s exact.
+// The pattern is written by an fp16 MMA of constants (every row 2048, 2048, 2048, 0 ...: 3 * 2048^2 = 1.5*2^23, exact in any
+// order) that overwrites the accumulator, issued by the seeder and complete (commit, barrier) before the block's int8 MMAs are
+// issued.  As tensor-memory stores of the promotion warps it cost them 100 of 590 cycles per block in isolation and held
+// every accumulator until the last of its columns was folded.
 #include "bi8_common.cuh"
 #include "tc_common.cuh"
 
@@ -55,13 +59,7 @@ constexpr int kBM = 128;                 // tile rows
 constexpr int kAccBufs = 3;              // s32 accumulators in tensor memory
 constexpr int kProbeN = 256;             // N of the issue-rate probe's MMAs
 constexpr int kStages = 4;               // operand stages of 128 K-bytes in flight
-// Scale ring depth.  The producer fills the slot of stage s after the MMA warp has committed stage s - kStages, whose last
-// block was issued into an accumulator that the promotion warps had released three blocks earlier: with 2 blocks per
-// stage they are then done with every stage up to s - kStages - 2, with 1 block per stage up to s - kStages - 3, with 4
-// up to s - kStages - 1.  A ring of kStages + 3 slots is therefore never overwritten while a promotion warp reads it.
-constexpr int kScaleStages = 8;
-static_assert(kScaleStages >= kStages + 3, "scale ring too shallow for the lag of the promotion warps");
-constexpr int kRoleWarps = 4;            // producer, MMA issuer, two spare: one warp per scheduler gives its registers away
+constexpr int kRoleWarps = 4;            // producer, MMA issuer, seeder, storer: one warp per scheduler gives its registers away
 constexpr uint32_t kABytes = kBM * kBK;  // 16 KiB
 constexpr uint32_t kSeedBits = 0x4B400000u;   // float 1.5 * 2^23
 constexpr float kSeedF = 12582912.0f;
@@ -72,8 +70,7 @@ constexpr int kPW = 4;
 struct Cfg {
     static constexpr int BN = 160;                        // tile columns: kAccBufs * BN <= 512 tensor-memory columns
     static constexpr int COLS = BN / kPW;                 // columns owned by one promotion thread
-    static constexpr int H0 = 24;                         // the accumulator is read as columns [0, H0) and [H0, COLS)
-    static constexpr int H1 = COLS - H0;
+    static constexpr int CH = 8;                          // columns read from the accumulator at a time
     static constexpr int EPI_WARPS = 4 * kPW;
     static constexpr int THREADS = (kRoleWarps + EPI_WARPS) * 32;
     static constexpr int LAUNCH_REGS = 96;                // 65536 / THREADS, rounded down to a multiple of 8
@@ -87,10 +84,18 @@ struct Cfg {
     // compiler really chose for the kernel.)
     static_assert(ROLE_REGS + kPW * EPI_REGS <= (1 + kPW) * LAUNCH_REGS, "register budget of a scheduler exceeds its launch allocation");
     static_assert((1 + kPW) * 32 * LAUNCH_REGS <= 16384, "launch allocation exceeds a scheduler's register file");
-    static_assert(kAccBufs * BN <= 512 && COLS % 8 == 0 && H0 % 8 == 0 && H1 % 8 == 0 && BN % 16 == 0, "tile geometry");
+    static_assert(kAccBufs * BN <= 512 && COLS % CH == 0 && COLS % 8 == 0 && BN % 32 == 0, "tile geometry");
     __host__ __device__ static constexpr uint32_t a_off(int s) { return (uint32_t)s * STAGE_BYTES; }
     __host__ __device__ static constexpr uint32_t b_off(int s) { return a_off(s) + kABytes; }
 };
+
+// How a finished tile leaves: kTma, through the tensor map tmC (16-bit outputs by the storer warp, fp32 ones in two passes by the promotion
+// warps: handing the halves over was 2 us slower where there is one round of tiles); kOwn, by the promotion warps, to
+// outputs that a tensor map cannot describe.
+enum StoreMode { kTma = 0, kOwn = 1 };
+// Instances of the kernel by the way its tiles leave: code for the other ways, even where it is not executed, costs the K loop up to
+// 10 % through its registers (8192 x 4096 x 11008 at block 64).
+enum OutKind { kAnyOut = 0, kSplit, kTma16, kTma16Add, kOwn16, kWide };
 
 struct TcParams {
     const float* sA;
@@ -104,7 +109,9 @@ struct TcParams {
     int tiles_m, tiles_n;
     int out_dtype, bias_dtype;
     int vec_store;      // C base and row pitch allow 16-byte stores
-    int tma_store;      // the output is described by the tensor map tmC: staged tiles leave by TMA stores
+    int store;          // how undivided tiles leave (StoreMode)
+    unsigned tm_mul;    // division by tiles_m: (umulhi(t, tm_mul) + t) >> tm_shift
+    int tm_shift;
     int tma_scales;     // bit 0: sA is described by the tensor map tmSA, bit 1: sB by tmSB
     int ksplit;         // > 1: the K stages are divided over ksplit work items per tile (split-K)
     int stages_per_split;
@@ -122,19 +129,30 @@ struct Geo {
     using C = Cfg;
     static constexpr int BPS = kBK / QB;                        // quantisation blocks per stage
     static constexpr int MMAS = QB / 32;                        // MMAs (K = 32) per block
-    static constexpr int SC_FLOATS = (BPS * (kBM + C::BN) + 31) / 32 * 32;   // scale floats per stage, [BPS][128] of sA then [BPS][BN] of sB, padded to 128 bytes
-    static constexpr int SB_OFF = BPS * kBM;                    // first sB float of a stage
-    static constexpr uint32_t bar_off = C::scale_off + kScaleStages * SC_FLOATS * 4;
+    // Scale rings, one record of BN floats per block for sA (128 of them used) and one for sB, so that one offset serves both.
+    // Depth: the producer fills the slot of stage s after the MMA warp has committed stage s - kStages, whose last block was
+    // issued into an accumulator that the promotion warps had released kAccBufs blocks earlier, having read everything but some
+    // of that block's scales: stages up to s - kStages - ceil((kAccBufs + 1) / BPS) may still be read.
+    static constexpr int SC_STAGES = kStages + (kAccBufs + 1 + BPS - 1) / BPS;
+    static constexpr uint32_t SC_REC = C::BN * 4;               // bytes of a record
+    static constexpr uint32_t SC_RING = SC_STAGES * BPS * SC_REC;
+    static constexpr uint32_t sb_off = C::scale_off + SC_RING;
+    static constexpr uint32_t bar_off = sb_off + SC_RING;
     // barrier slots (8 bytes each)
     static constexpr int FULL_AB = 0, EMPTY_AB = kStages, ACC_FULL = 2 * kStages, ACC_EMPTY = 2 * kStages + kAccBufs,
-                         NBARS = 2 * kStages + 2 * kAccBufs;
+                         ACC_SEEDED = 2 * kStages + 2 * kAccBufs, OUT_FULL = 2 * kStages + 3 * kAccBufs, OUT_EMPTY = OUT_FULL + 1,
+                         NBARS = OUT_EMPTY + 1;
     static constexpr uint32_t misc_off = bar_off + NBARS * 8;   // tmem holder (4 B) + abort flag (4 B) + never-raised flag (4 B)
-    // outputs leave through shared memory: every promotion warp stages 32 rows x COLS*2 bytes per pass
-    static constexpr uint32_t OUT_WARP_BYTES = 32 * C::COLS * 2;
+    // Finished tiles are staged as one part of 32 rows of 80 bytes per promotion warp; a tile of fp32 takes two passes of half its columns.
+    static constexpr uint32_t PART_ROW = C::COLS * 2, PART_BYTES = 32 * PART_ROW;
+    static constexpr uint32_t OUT_BYTES = C::EPI_WARPS * PART_BYTES;
     static constexpr uint32_t out_off = (misc_off + 16 + 127) & ~127u;
-    static constexpr uint32_t total = out_off + C::EPI_WARPS * OUT_WARP_BYTES;
-    static_assert(OUT_WARP_BYTES % 128 == 0, "TMA store sources are 128-byte aligned");
-    static_assert((SC_FLOATS * 4) % 128 == 0 && (SB_OFF * 4) % 128 == 0 && C::scale_off % 1024 == 0, "TMA destinations of the scale boxes are 128-byte aligned");
+    // operand of the seeding MMAs (both A and B): 16 fp16 values per row as 8-row core matrices
+    static constexpr uint32_t seed_off = out_off + OUT_BYTES;
+    static constexpr uint32_t SEED_BYTES = C::BN * 32;
+    static constexpr uint32_t total = seed_off + SEED_BYTES;
+    static_assert(PART_BYTES % 128 == 0, "TMA store sources are 128-byte aligned");
+    static_assert(SC_REC % 128 == 0 && C::scale_off % 1024 == 0, "TMA destinations of the scale boxes are 128-byte aligned");
 };
 
 // Work item -> tile and K-stage range.  Items of one split are consecutive, so CTAs that run together work on different
@@ -155,10 +173,12 @@ __device__ __forceinline__ void item_range(int item, const TcParams& p, int nks,
 }
 
 template <int BN>
-__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int& m0, int& n0) {
+__device__ __forceinline__ void tile_coords(int tile, const TcParams& p, int& m0, int& n0) {
+    // (a division by a product with host-made constants, exact below 2^31)
     // consecutive tiles (CTAs that run together) share a column panel of Bt and sweep the rows of A
-    m0 = (tile % tiles_m) * kBM;
-    n0 = (tile / tiles_m) * BN;
+    const int tn = (int)((__umulhi((unsigned)tile, p.tm_mul) + (unsigned)tile) >> p.tm_shift);
+    m0 = (tile - tn * p.tiles_m) * kBM;
+    n0 = tn * BN;
 }
 
 // Bounded wait of a converged warp: one poll by every lane, then (phase not complete yet, or the lanes disagree) the
@@ -167,14 +187,6 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int& m0, int&
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, uint32_t abort_flag, long long limit) {
     if (__builtin_expect(__all_sync(0xffffffffu, mbar_test(bar, parity)), 1)) return true;
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, limit));
-}
-
-// NC consecutive accumulator columns of this thread's lane -> registers.
-template <int NC>
-__device__ __forceinline__ void tmem_load_cols(uint32_t taddr, uint32_t (&S)[NC]) {
-    static_assert(NC == 24 || NC == 16, "the two parts of a thread's columns");
-    tmem_ld16(taddr, reinterpret_cast<uint32_t(&)[16]>(S[0]));
-    if constexpr (NC == 24) tmem_ld8(taddr + 16u, reinterpret_cast<uint32_t(&)[8]>(S[16]));
 }
 
 // Blocks go round the kAccBufs = 3 accumulators and every stage has BPS blocks, so block `blk` of the stage at position
@@ -194,10 +206,10 @@ __device__ __forceinline__ uint32_t keep(uint32_t v) {
 }
 
 // Folds NC s32 words a thread has read from an accumulator (its row, columns C0 .. C0+NC-1 of its COLS, one quantisation
-// block) into its fp32 accumulators: acc[n] += sB[n] * (P[n] * s), both products as packed FMAs on column pairs.  `sw` is the shared address of the block's column scales of this thread (16-byte
-// aligned).
-template <bool SEED, int C0, int NC, int COLS>
-__device__ __forceinline__ void fold_columns(const uint32_t (&S)[NC], uint32_t sw, float sxd, float negc, uint64_t (&acc2)[COLS / 2]) {
+// block) into its fp32 accumulators: acc[n] += sB[n] * (P[n] * s), both products as packed FMAs on column pairs.  `sw` is the
+// shared address of the block's column scales of this thread (16-byte aligned).
+template <bool SEED, int NC, int COLS>
+__device__ __forceinline__ void fold_columns(int C0, const uint32_t (&S)[NC], uint32_t sw, float sxd, float negc, uint64_t (&acc2)[COLS / 2]) {
     const uint64_t sxd2 = pack_f32x2(sxd, sxd), negc2 = pack_f32x2(negc, negc);
 #pragma unroll
     for (int q = 0; q < NC / 4; ++q) {
@@ -282,7 +294,7 @@ __device__ __forceinline__ void add_piece(uint32_t addr, bool wide, bool bf, Add
 // several rows at once; running addresses, because a division and a product per element were more instructions than the
 // promotion has (8192 x 50257, K 768: 1040 -> 902 us).  Not inlined: the registers of the K loop are to stay as they are.
 template <int ROWB>
-__device__ __noinline__ void store_elements(unsigned char* dst, int64_t pitch, uint32_t stage, int lane, int rows, int cols) {
+__device__ __forceinline__ void store_elements(unsigned char* dst, int64_t pitch, uint32_t stage, int lane, int rows, int cols) {
     constexpr int REST = ROWB / 2 - 32, ROWS = 32 / REST;
     static_assert(REST > 0 && 32 % REST == 0, "whole rows of remaining columns per step");
     auto column = [&](int r, int c, int step, int count) {
@@ -298,6 +310,31 @@ __device__ __noinline__ void store_elements(unsigned char* dst, int64_t pitch, u
     };
     column(0, lane, 1, 32);
     column(lane / REST, 32 + lane % REST, ROWS, 32 / ROWS);
+}
+
+// A promotion warp's 32 staged rows of ROWB bytes to an output of any alignment: consecutive lanes store consecutive 4-byte words of a
+// row, or 2-byte elements where the rows of a 16-bit output are not all 4-byte aligned.
+template <int ROWB>
+__device__ __noinline__ void store_own(unsigned char* dst, int64_t pitch, uint32_t stage, int rows_valid, int cols_left, bool wide, int lane) {
+    const int cols_pass = ROWB / (wide ? 4 : 2);
+    const int cols_valid = cols_left < cols_pass ? cols_left : cols_pass;      // rows_valid may exceed 32, both may be negative
+    if (wide || (((reinterpret_cast<uintptr_t>(dst) | (uintptr_t)pitch) & 3u) == 0)) {
+        constexpr int WPR = ROWB / 4;                          // words per staged row
+        const int words = wide ? cols_valid : (cols_valid >> 1);
+        const bool odd_tail = !wide && (cols_valid & 1) && cols_valid > 0;
+#pragma unroll 4
+        for (int idx = lane; idx < 32 * WPR; idx += 32) {
+            const int r = idx / WPR, w = idx - r * WPR;
+            if (r < rows_valid) {
+                const uint32_t v = lds_u32(stage + (uint32_t)(idx * 4));
+                unsigned char* d = dst + (int64_t)r * pitch + w * 4;
+                if (w < words) *reinterpret_cast<uint32_t*>(d) = v;
+                else if (odd_tail && w == words) *reinterpret_cast<uint16_t*>(d) = (uint16_t)(v & 0xffffu);
+            }
+        }
+    } else {
+        store_elements<ROWB>(dst, pitch, stage, lane, rows_valid, cols_valid);
+    }
 }
 
 // Adds bias[n] and then residual[m, n], each in the output type, to a thread's staged row (COLS 16-bit or COLS/2 fp32 values at
@@ -348,22 +385,23 @@ __device__ __forceinline__ void add_staged(const TcParams& p, uint32_t row_addr,
     }
 }
 
-template <int QB, int MODE, bool SEED>
+template <int QB, int MODE, bool SEED, int OUT>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmSA, const __grid_constant__ CUtensorMap tmSB,
                const __grid_constant__ CUtensorMap tmC, const TcParams p) {
     using C = Cfg;
     using G = Geo<QB>;
-    constexpr int BN = C::BN, COLS = C::COLS, H0 = C::H0, H1 = C::H1;
+    constexpr int BN = C::BN, COLS = C::COLS, CH = C::CH;
     constexpr bool kScales = (MODE == 0);           // the partial-sum dump uses no scales
+    const int store = OUT == kTma16 || OUT == kTma16Add ? kTma : OUT == kOwn16 ? kOwn : p.store;
+    const bool wide = OUT == kWide || (OUT == kAnyOut && p.out_dtype == BI8_F32);
+    const bool addends = OUT != kTma16 && (OUT == kTma16Add || p.bias != nullptr || p.residual != nullptr);
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
     // dynamic shared memory is only guaranteed 16-byte aligned: round up to the swizzle atom
     const uint32_t raw = smem_u32(smem_dyn);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* base_ptr = smem_dyn + (base - raw);
-    const float* sc_ring = reinterpret_cast<const float*>(base_ptr + C::scale_off);
-    const uint32_t sc_ring_u32 = base + C::scale_off;
     const uint32_t bars = base + G::bar_off;
     volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(base_ptr + G::misc_off);
     const uint32_t abort_flag = base + G::misc_off + 4;
@@ -390,7 +428,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int b = 0; b < kAccBufs; ++b) {
             mbar_init(bar(G::ACC_FULL + b), 1);
             mbar_init(bar(G::ACC_EMPTY + b), C::EPI_WARPS);
+            mbar_init(bar(G::ACC_SEEDED + b), 1);
         }
+        mbar_init(bar(G::OUT_FULL), C::EPI_WARPS);
+        mbar_init(bar(G::OUT_EMPTY), 1);
         sts_u32(abort_flag, 0u);
         sts_u32(never_flag, 0u);                     // a flag nobody raises, for waits that must not be cut short
         mbar_fence_init();
@@ -399,6 +440,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (warp == 1) {
         tmem_alloc(smem_u32((const void*)tmem_holder), 512);
         tmem_relinquish();
+    }
+    if (SEED) {
+        // a row is 2048, 2048, 2048, 0 ... 0: its product with another is 3 * 2^22 = 1.5 * 2^23
+        for (uint32_t i = threadIdx.x; i < G::SEED_BYTES / 16; i += C::THREADS)
+            sts_v4(base + G::seed_off + i * 16u, (i & 8u) ? 0u : 0x68006800u, (i & 8u) ? 0u : 0x00006800u, 0u, 0u);
+        fence_proxy_async_smem();
     }
     tc_fence_before();
     __syncthreads();
@@ -421,12 +468,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int s = 0; s < kStages; ++s) last_parity[s] = -1;
             bool ok = true;
             bool first_item = true;
-            constexpr uint32_t kSaBytes = (uint32_t)(G::BPS * kBM * 4), kSbBytes = (uint32_t)(G::BPS * BN * 4);
+            constexpr uint32_t kScBytes = (uint32_t)(G::BPS * BN * 4);
             const bool tma_sa = kScales && (p.tma_scales & 1), tma_sb = kScales && (p.tma_scales & 2);
             for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
                 int tile, slot, ks0, ks1, m0, n0;
                 item_range(item, p, nks, tile, slot, ks0, ks1);
-                tile_coords<BN>(tile, p.tiles_m, m0, n0);
+                tile_coords<BN>(tile, p, m0, n0);
                 for (int ks = ks0; ks < ks1; ++ks) {
                     ok = warp_wait(bar(G::EMPTY_AB + stage), phase ^ 1u, abort_flag, wait_limit);
                     if (!ok) {
@@ -435,14 +482,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                     const bool skip = first_item && p.skip_stage >= 0 && ks - ks0 == p.skip_stage;   // diagnostic only
                     const uint32_t fb = bar(G::FULL_AB + stage);
-                    const uint32_t sdst = sc_ring_u32 + (uint32_t)(sslot * G::SC_FLOATS * 4);
+                    const uint32_t sadst = base + C::scale_off + (uint32_t)sslot * kScBytes, sbdst = sadst + G::SC_RING;
                     if (lane == 0 && !skip) {
-                        mbar_expect_tx(fb, C::STAGE_BYTES + (tma_sa ? kSaBytes : 0u) + (tma_sb ? kSbBytes : 0u));
+                        mbar_expect_tx(fb, C::STAGE_BYTES + (tma_sa ? kScBytes : 0u) + (tma_sb ? kScBytes : 0u));
                         tma_load_2d(base + C::a_off(stage), &tmA, fb, ks * kBK, m0);
                         tma_load_2d(base + C::b_off(stage), &tmB, fb, ks * kBK, n0);
-                        // boxes [BPS, 128] of sA and [BPS, BN] of sB; rows and blocks outside the tensors read as zero
-                        if (tma_sa) tma_load_2d(sdst, &tmSA, fb, m0, ks * G::BPS);
-                        if (tma_sb) tma_load_2d(sdst + (uint32_t)(G::SB_OFF * 4), &tmSB, fb, n0, ks * G::BPS);
+                        // boxes [BPS, BN]; rows and blocks outside the tensors read as zero
+                        if (tma_sa) tma_load_2d(sadst, &tmSA, fb, m0, ks * G::BPS);
+                        if (tma_sb) tma_load_2d(sbdst, &tmSB, fb, n0, ks * G::BPS);
                     }
                     if (kScales && !(tma_sa && tma_sb) && !skip) {
                         // A scale tensor whose rows are not 16-byte aligned: asynchronous 4-byte copies by the 32 lanes (the
@@ -456,7 +503,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                                 for (int c = lane; c < kBM; c += 32) {
                                     const bool live = j < p.nb && m0 + c < p.M;
-                                    cp_async_4(sdst + (uint32_t)((blk * kBM + c) * 4), live ? row + c : p.sA, live ? 4u : 0u);
+                                    cp_async_4(sadst + (uint32_t)((blk * BN + c) * 4), live ? row + c : p.sA, live ? 4u : 0u);
                                 }
                             }
                             if (!tma_sb) {
@@ -464,7 +511,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                                 for (int c = lane; c < BN; c += 32) {
                                     const bool live = j < p.nb && n0 + c < p.N;
-                                    cp_async_4(sdst + (uint32_t)((G::SB_OFF + blk * BN + c) * 4), live ? row + c : p.sB, live ? 4u : 0u);
+                                    cp_async_4(sbdst + (uint32_t)((blk * BN + c) * 4), live ? row + c : p.sB, live ? 4u : 0u);
                                 }
                             }
                         }
@@ -477,7 +524,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             if (s == stage) last_parity[s] = (int)phase;
                     }
                     if (++stage == kStages) { stage = 0; phase ^= 1u; }
-                    if (++sslot == kScaleStages) sslot = 0;
+                    if (++sslot == G::SC_STAGES) sslot = 0;
                 }
                 first_item = false;
             }
@@ -512,7 +559,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                 for (int blk = 0; blk < G::BPS; ++blk) {
                     const int buf = RotInfo<G::BPS>::buf(ROT, blk);
-                    ok = warp_wait(bar(G::ACC_EMPTY + buf), accpar[buf], abort_flag, wait_limit_mma);
+                    ok = warp_wait(bar((SEED ? G::ACC_SEEDED : G::ACC_EMPTY) + buf), accpar[buf], abort_flag, wait_limit_mma);
                     if (!ok) {
                         if (lane == 0) report_timeout(p.status, abort_flag, W_ACC_EMPTY);
                         return;
@@ -542,6 +589,66 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     if (ks + 2 < ks1 && ok) issue_stage(std::integral_constant<int, 2>{});
                 }
             }
+        } else if (warp == 2 && SEED) {
+            // ---------------- seeder ----------------
+            // follows the accumulators in the order of the MMA issuer, which waits for its commits instead of the promotion warps
+            constexpr uint32_t idesc = umma_idesc_f16_f32(kBM, BN);
+            const uint64_t desc = umma_desc_k_none(base + G::seed_off, 128, 256);
+            uint32_t accpar[kAccBufs] = {0u, 0u, 0u};
+            bool ok = true;
+            auto seed_acc = [&](int buf) {
+                ok = warp_wait(bar(G::ACC_EMPTY + buf), accpar[buf], abort_flag, wait_limit);
+                if (!ok) {
+                    if (lane == 0) report_timeout(p.status, abort_flag, W_ACC_EMPTY);
+                    return;
+                }
+                accpar[buf] ^= 1u;
+                tc_fence_after();
+                if (lane == 0) {
+                    mma_f16(tmem_base + (uint32_t)(buf * BN), desc, desc, idesc, 0u);
+                    tc_commit(bar(G::ACC_SEEDED + buf));
+                }
+                __syncwarp();
+            };
+            for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+                int tile, slot, ks0, ks1;
+                item_range(item, p, nks, tile, slot, ks0, ks1);
+                const int blocks = (ks1 - ks0) * G::BPS;
+                for (int j = 0; j < blocks && ok; j += kAccBufs)
+#pragma unroll
+                    for (int b = 0; b < kAccBufs; ++b)
+                        if (j + b < blocks && ok) seed_acc(b);
+            }
+        } else if (warp == 3 && MODE == 0 && OUT != kSplit && p.ksplit == 1 && store == kTma && !wide) {
+            // ---------------- storer ----------------
+            uint32_t par = 0;
+            bool ok = true;
+            for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+                int m0, n0;
+                tile_coords<BN>(item, p, m0, n0);
+                // this wait spans the K loop of a tile: one limit for each of its stages
+                ok = false;
+                for (int t = 0; t <= nks && !ok; ++t) {
+                    ok = warp_wait(bar(G::OUT_FULL), par, abort_flag, wait_limit);
+                    if (!ok && __any_sync(0xffffffffu, lds_volatile_u32(abort_flag) != 0u)) break;
+                }
+                if (!ok) {
+                    if (lane == 0) report_timeout(p.status, abort_flag, W_OUT_FULL);
+                    break;
+                }
+                // the promotion warps' writes (ordered by the barrier) before the copies below
+                fence_proxy_async_smem();
+                // rows and columns of the boxes that lie outside the tensor are not written
+                if (lane < C::EPI_WARPS) {
+                    const int col0 = n0 + (lane >> 2) * COLS, row0 = m0 + (lane & 3) * 32;
+                    if (col0 < p.N && row0 < p.M) tma_store_2d(&tmC, base + G::out_off + (uint32_t)lane * G::PART_BYTES, col0, row0);
+                }
+                tma_store_commit();
+                tma_store_wait_read();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(G::OUT_EMPTY));
+                par ^= 1u;
+            }
         }
     } else {
         // ---------------- promotion + epilogue ----------------
@@ -550,136 +657,105 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int slice = (warp - kRoleWarps) >> 2;       // columns COLS*slice .. of the tile
         const int row = quarter * 32 + lane;
         const uint32_t t_lane = keep(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(slice * COLS));
-        // eight spare tensor-memory columns of this warp's lanes keep the seed pattern
-        static_assert(kAccBufs * BN + 8 * kPW <= 512, "no spare tensor-memory columns for the seed pattern");
-        const uint32_t t_seed = keep(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(kAccBufs * BN + 8 * slice));
         // shared addresses of this thread's row scale and of its first column scale in scale stage 0, block 0
-        const uint32_t sa_addr = keep(sc_ring_u32 + (uint32_t)(row * 4));
-        const uint32_t sw_addr = keep(sc_ring_u32 + (uint32_t)((G::SB_OFF + slice * COLS) * 4));
+        const uint32_t sa_addr = keep(base + C::scale_off + (uint32_t)(row * 4));
+        const uint32_t sw_addr = keep(base + G::sb_off + (uint32_t)(slice * COLS * 4));
         const uint32_t bar0 = keep(bars);
         const uint32_t leader = keep(lane == 0 ? 1u : 0u);
         const float div = 1.0f / (127.0f * 127.0f);
-        uint32_t seedv[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) seedv[i] = kSeedBits;
-
-        if (SEED) {
-#pragma unroll
-            for (int b = 0; b < kAccBufs; ++b)
-#pragma unroll
-                for (int c = 0; c < COLS / 8; ++c) tmem_st8(t_lane + (uint32_t)(b * BN + c * 8), seedv);
-            tmem_wait_st();
-            // The promotion loop re-reads the seed pattern from the spare columns in every block: the result of a load is
-            // a tuple of consecutive registers, which is what the stores want, and it is live for half a block only.
-            // Eight constants would be rebuilt with eight moves in front of every store; a tuple kept across the loop
-            // costs eight registers that the loop does not have, and the compiler then copies it around.
-            tmem_st8(t_seed, seedv);
-            tmem_wait_st();
-        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
 #pragma unroll
             for (int b = 0; b < kAccBufs; ++b) mbar_arrive(bar(G::ACC_EMPTY + b));
         }
-        auto reseed = [&](uint32_t taddr, int c0, int nc) {
-            if (SEED) {
-#pragma unroll
-                for (int c = 0; c < nc / 8; ++c) tmem_st8(taddr + (uint32_t)(c0 + c * 8), seedv);
-            }
-        };
-
-        int sstage = 0;
         uint32_t accpar[kAccBufs] = {0u, 0u, 0u};   // barrier parities of the three accumulators, flipped with every use
-        uint32_t sc_off = 0;                      // byte offset of scale stage `sstage`
+        uint32_t sc_off = 0;                      // byte offset of the block's records in the scale rings
         bool ok = true;
+        uint32_t out_par = 1u;                    // staging area: parity of the release before the tile
         int fail_code = 0;
 
         // the tile's COLS fp32 accumulators of this thread, kept as packed pairs for fma.rn.f32x2
         uint64_t acc2[COLS / 2];
         int m = 0, nbase = 0;
-        uint32_t S0[H0], S1[H1];
 
-        // One stage of the promotion: BPS blocks.  `rot_tag` is the stage's position in a cycle of three stages, which
-        // fixes the accumulator of each of its blocks (RotInfo); `ks` is the stage's index along K.
-        auto promote_stage = [&](auto rot_tag, int ks) {
-            constexpr int ROT = decltype(rot_tag)::value;
-            using R = RotInfo<G::BPS>;
+        // Promotion of block j, which lies in accumulator `buf_tag`.
+        auto promote_block = [&](auto buf_tag, int j) {
+            constexpr int buf = decltype(buf_tag)::value;
+            const uint32_t t_acc = t_lane + (uint32_t)(buf * BN);
+            ok = warp_wait(bar0 + 8u * (uint32_t)(G::ACC_FULL + buf), accpar[buf], abort_flag, wait_limit);
+            if (!ok) {
+                fail_code = W_ACC_FULL;
+                return;
+            }
+            accpar[buf] ^= 1u;
+            tc_fence_after();
+            if (MODE == 1) {
 #pragma unroll
-            for (int blk = 0; blk < G::BPS; ++blk) {
-                const int buf = R::buf(ROT, blk);
-                const uint32_t t_acc = t_lane + (uint32_t)(buf * BN);
-                ok = warp_wait(bar0 + 8u * (uint32_t)(G::ACC_FULL + buf), accpar[buf], abort_flag, wait_limit);
-                if (!ok) {
-                    fail_code = W_ACC_FULL;
-                    return;
-                }
-                accpar[buf] ^= 1u;
-                tc_fence_after();
-                if (MODE == 1) {
-                    const int j = ks * G::BPS + blk;
-#pragma unroll
-                    for (int c = 0; c < COLS / 8; ++c) {
-                        uint32_t pv[8];
-                        tmem_ld8(t_acc + (uint32_t)(c * 8), pv);
-                        tmem_wait_ld();
-                        reseed(t_acc, c * 8, 8);
-                        if (m < p.M && j < p.nb) {
-                            int32_t* dst = p.partials + ((int64_t)j * p.M + m) * p.N + nbase + c * 8;
-#pragma unroll
-                            for (int i = 0; i < 8; ++i)
-                                if (nbase + c * 8 + i < p.N)
-                                    dst[i] = SEED ? (int32_t)(pv[i] - kSeedBits) : (int32_t)pv[i];
-                        }
-                    }
-                } else {
-                    tmem_load_cols<H0>(t_acc, S0);
-                    if (SEED) tmem_ld8(t_seed, seedv);      // the seed tuple for this block's stores
-                    // the row's scale, while the read of the first half is in flight
-                    float sxd = __fmul_rn(lds_f32(sa_addr + sc_off + (uint32_t)(blk * kBM * 4)), div);
-                    float negc = 0.0f;
-                    if (SEED) {
-                        sxd = __uint_as_float((__float_as_uint(sxd) + 2u) & 0xFFFFFFFCu);   // 22 significant bits
-                        negc = -__fmul_rn(kSeedF, sxd);                                      // exact
-                    }
-                    const uint32_t sw = sw_addr + sc_off + (uint32_t)(blk * BN * 4);
+                for (int c = 0; c < COLS / 8; ++c) {
+                    uint32_t pv[8];
+                    tmem_ld8(t_acc + (uint32_t)(c * 8), pv);
                     tmem_wait_ld();
-                    tmem_load_cols<H1>(t_acc + (uint32_t)H0, S1);    // second half, in flight during the fold of the first
-                    reseed(t_acc, 0, H0);
-                    fold_columns<SEED, 0, H0, COLS>(S0, sw, sxd, negc, acc2);
-                    tmem_wait_ld();
-                    reseed(t_acc, H0, H1);
-                    fold_columns<SEED, H0, H1, COLS>(S1, sw, sxd, negc, acc2);
+                    if (m < p.M && j < p.nb) {
+                        int32_t* dst = p.partials + ((int64_t)j * p.M + m) * p.N + nbase + c * 8;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (nbase + c * 8 + i < p.N)
+                                dst[i] = SEED ? (int32_t)(pv[i] - kSeedBits) : (int32_t)pv[i];
+                    }
                 }
-                if (SEED) tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
                 if (leader) mbar_arrive(bar0 + 8u * (uint32_t)(G::ACC_EMPTY + buf));
-            }
-            if (kScales) {
-                sc_off += (uint32_t)(G::SC_FLOATS * 4);
-                if (++sstage == kScaleStages) { sstage = 0; sc_off = 0; }
+            } else {
+                uint32_t S[2][CH];
+                tmem_ld8(t_acc, S[0]);
+                // the row's scale, while the read of the first columns is in flight
+                float sxd = __fmul_rn(lds_f32(sa_addr + sc_off), div);
+                float negc = 0.0f;
+                if (SEED) {
+                    sxd = __uint_as_float((__float_as_uint(sxd) + 2u) & 0xFFFFFFFCu);   // 22 significant bits
+                    negc = -__fmul_rn(kSeedF, sxd);                                      // exact
+                }
+                const uint32_t sw = sw_addr + sc_off;
+#pragma unroll
+                for (int c = 0; c < COLS / CH; ++c) {
+                    tmem_wait_ld();
+                    if (c + 1 < COLS / CH) {
+                        tmem_ld8(t_acc + (uint32_t)((c + 1) * CH), S[(c + 1) & 1]);
+                    } else {
+                        // all of the accumulator is in registers
+                        tc_fence_before();
+                        __syncwarp();
+                        if (leader) mbar_arrive(bar0 + 8u * (uint32_t)(G::ACC_EMPTY + buf));
+                    }
+                    fold_columns<SEED, CH, COLS>(c * CH, S[c & 1], sw, sxd, negc, acc2);
+                }
+                sc_off += G::SC_REC;
+                if (sc_off == G::SC_RING) sc_off = 0;
             }
         };
 
         for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
             int tile, slot, ks0, ks1, m0, n0;
             item_range(item, p, nks, tile, slot, ks0, ks1);
-            tile_coords<BN>(tile, p.tiles_m, m0, n0);
+            tile_coords<BN>(tile, p, m0, n0);
             m = m0 + row;
             nbase = n0 + slice * COLS;
 #pragma unroll
             for (int i = 0; i < COLS / 2; ++i) acc2[i] = 0ull;
 
-            // cycles of three stages; every tile starts on accumulator 0, like the MMA issuer
-            for (int ks = ks0; ks < ks1 && ok; ks += 3) {
-                promote_stage(std::integral_constant<int, 0>{}, ks);
-                if (ks + 1 < ks1 && ok) promote_stage(std::integral_constant<int, 1>{}, ks + 1);
-                if (ks + 2 < ks1 && ok) promote_stage(std::integral_constant<int, 2>{}, ks + 2);
+            // the blocks go round the accumulators; every tile starts on accumulator 0, like the MMA issuer
+            const int j1 = ks1 * G::BPS;
+#pragma unroll 1
+            for (int j = ks0 * G::BPS; j < j1 && ok; j += kAccBufs) {
+                promote_block(std::integral_constant<int, 0>{}, j);
+                if (j + 1 < j1 && ok) promote_block(std::integral_constant<int, 1>{}, j + 1);
+                if (j + 2 < j1 && ok) promote_block(std::integral_constant<int, 2>{}, j + 2);
             }
             if (!ok) break;
 
-            if (MODE == 0 && slot >= 0) {
+            if (MODE == 0 && (OUT == kSplit || (OUT == kAnyOut && slot >= 0))) {
                 // Part of a divided tile: straight from the registers to the item's workspace slot, in the order in which
                 // the reduction kernel reads it (ws_index: 32 bytes of one row per thread and step).
                 float* dst = p.ws + (int64_t)slot * p.slot_floats + ws_index<COLS>(quarter, slice, 0, lane);
@@ -693,28 +769,61 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     stg_v8(dst + g * 256, v);
                 }
             } else if (MODE == 0) {
-                // The tile leaves through the warp's staging area in shared memory: every lane writes its row's share
-                // (ROWB bytes), then either one TMA store or a loop of coalesced stores moves the 32 x ROWB bytes out.
-                // 2-byte outputs take one pass of COLS columns, 4-byte outputs two passes of COLS / 2.  Addresses are
-                // derived here from the thread index rather than kept in registers through the K loop, whose register
-                // budget is full.  Bias and residual are added to the staged row by a loop of its own: with their code
-                // unrolled between the casts the epilogue was 1.1 us per tile (instruction fetch), a third of a K = 512 tile.
-                constexpr uint32_t ROWB = (uint32_t)(COLS * 2);
+                // The tile leaves through shared memory: the promotion warps write their shares, the storer warp moves them out while
+                // the promotion warps go on with the next tile.  Fencing, issuing and waiting for the copies here cost 800 of
+                // a K = 512 tile's 7500 cycles (8192 x 512 x 11840: 134 -> 112 us with this and the fast division of tile_coords).  Addresses are derived here from the thread index rather than kept in
+                // registers through the K loop, whose register budget is full.  Bias and residual are added to the staged row
+                // by a loop of its own: with their code unrolled between the casts the epilogue was 1.1 us per tile
+                // (instruction fetch).
                 uint32_t tid_now;
                 asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid_now));
-                const uint32_t ln = tid_now & 31u;
-                const uint32_t out_stage = base + G::out_off + ((tid_now >> 5) - (uint32_t)kRoleWarps) * G::OUT_WARP_BYTES;
-                const uint32_t my_row = out_stage + ln * ROWB;
-                const bool wide = p.out_dtype == BI8_F32;
-                const int row0 = m - (int)ln;                         // first row of the warp's part
-                const int passes = wide ? 2 : 1;
-#pragma unroll 1
-                for (int ps = 0; ps < passes; ++ps) {
-                    const int col0 = nbase + ps * (COLS / 2);
-                    // the previous TMA store must have read the staging area before it is written again
-                    if (p.tma_store && ln == 0) tma_store_wait_read();
+                const uint32_t ln = tid_now & 31u, w = (tid_now >> 5) - (uint32_t)kRoleWarps, qt = w & 3u, sl = w >> 2;
+                const uint32_t out = base + G::out_off;
+                if (store == kTma && !wide) {
+                    // the copies of the tile before must have read the staging area
+                    ok = warp_wait(bar0 + 8u * (uint32_t)G::OUT_EMPTY, out_par, abort_flag, wait_limit);
+                    if (!ok) {
+                        fail_code = W_OUT_EMPTY;
+                        break;
+                    }
+                    out_par ^= 1u;
+                }
+                const uint32_t part = out + w * G::PART_BYTES, my_row = part + ln * G::PART_ROW;
+                if (!wide) {
+                    uint32_t e[COLS / 2];
+                    if (p.out_dtype == BI8_BF16) {
+#pragma unroll
+                        for (int i = 0; i < COLS / 2; ++i) {
+                            float lo, hi;
+                            unpack_f32x2(acc2[i], lo, hi);
+                            e[i] = pack_bf16x2(lo, hi);
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < COLS / 2; ++i) {
+                            float lo, hi;
+                            unpack_f32x2(acc2[i], lo, hi);
+                            e[i] = pack_f16x2(lo, hi);
+                        }
+                    }
+#pragma unroll
+                    for (int g = 0; g < COLS / 8; ++g) sts_v4(my_row + (uint32_t)(g * 16), e[4 * g], e[4 * g + 1], e[4 * g + 2], e[4 * g + 3]);
+                    if (addends) add_staged<COLS>(p, my_row, m, nbase, wide);
                     __syncwarp();
-                    if (wide) {
+                    if (store == kTma) {
+                        if (ln == 0) mbar_arrive(bar0 + 8u * (uint32_t)G::OUT_FULL);
+                    } else {
+                        store_own<(int)G::PART_ROW>(static_cast<unsigned char*>(p.C) + ((int64_t)(m - (int)ln) * p.ldc + nbase) * 2, p.ldc * 2, part,
+                                                    p.M - m + (int)ln, p.N - nbase, wide, (int)ln);
+                        __syncwarp();
+                    }
+                } else {
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+                        const int col0 = nbase + h * (COLS / 2), row0 = m - (int)ln;
+                        // the previous TMA store must have read the part before it is written again
+                        if (store == kTma && ln == 0) tma_store_wait_read();
+                        __syncwarp();
 #pragma unroll
                         for (int g = 0; g < COLS / 8; ++g) {
                             float v[4];
@@ -723,78 +832,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             sts_v4(my_row + (uint32_t)(g * 16), __float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]),
                                    __float_as_uint(v[3]));
                         }
-                        // the second pass finds its columns where the first found its own
+                        // the second half finds its columns where the first found its own
 #pragma unroll
                         for (int i = 0; i < COLS / 4; ++i) acc2[i] = acc2[i + COLS / 4];
-                    } else if (p.out_dtype == BI8_BF16) {
-#pragma unroll
-                        for (int g = 0; g < COLS / 8; ++g) {
-                            uint32_t w[4];
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                float lo, hi;
-                                unpack_f32x2(acc2[g * 4 + u], lo, hi);
-                                w[u] = pack_bf16x2(lo, hi);
-                            }
-                            sts_v4(my_row + (uint32_t)(g * 16), w[0], w[1], w[2], w[3]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int g = 0; g < COLS / 8; ++g) {
-                            uint32_t w[4];
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                float lo, hi;
-                                unpack_f32x2(acc2[g * 4 + u], lo, hi);
-                                w[u] = pack_f16x2(lo, hi);
-                            }
-                            sts_v4(my_row + (uint32_t)(g * 16), w[0], w[1], w[2], w[3]);
-                        }
-                    }
-                    if (p.bias != nullptr || p.residual != nullptr) add_staged<COLS>(p, my_row, m, col0, wide);
-                    if (p.tma_store) {
-                        // rows and columns of the box that lie outside the tensor are not written
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (ln == 0 && col0 < p.N && row0 < p.M) {
-                            tma_store_2d(&tmC, out_stage, col0, row0);
-                            tma_store_commit();
-                        }
-                    } else {
-                        // Destinations that a tensor map cannot describe (base or row pitch not 16-byte aligned):
-                        // consecutive lanes store consecutive 4-byte words of a row, or 2-byte elements where the rows of
-                        // a 16-bit output are not all 4-byte aligned.
-                        __syncwarp();
-                        const int esz = wide ? 4 : 2;
-                        const int64_t pitch = p.ldc * esz;
-                        unsigned char* dst = static_cast<unsigned char*>(p.C) + (int64_t)row0 * pitch + (int64_t)col0 * esz;
-                        const int rows_valid = p.M - row0;                         // may exceed 32 or be negative
-                        const int cols_left = p.N - col0;
-                        const int cols_pass = wide ? COLS / 2 : COLS;
-                        const int cols_valid = cols_left < cols_pass ? cols_left : cols_pass;
-                        if (wide || (((reinterpret_cast<uintptr_t>(dst) | (uintptr_t)pitch) & 3u) == 0)) {
-                            constexpr int WPR = (int)ROWB / 4;                     // words per staged row
-                            const int words = wide ? cols_valid : (cols_valid >> 1);
-                            const bool odd_tail = !wide && (cols_valid & 1) && cols_valid > 0;
-#pragma unroll 4
-                            for (int idx = (int)ln; idx < 32 * WPR; idx += 32) {
-                                const int r = idx / WPR, w = idx - r * WPR;
-                                if (r < rows_valid) {
-                                    const uint32_t v = lds_u32(out_stage + (uint32_t)(idx * 4));
-                                    unsigned char* d = dst + (int64_t)r * pitch + w * 4;
-                                    if (w < words) *reinterpret_cast<uint32_t*>(d) = v;
-                                    else if (odd_tail && w == words) *reinterpret_cast<uint16_t*>(d) = (uint16_t)(v & 0xffffu);
-                                }
+                        if (addends) add_staged<COLS>(p, my_row, m, col0, wide);
+                        if (store == kTma) {
+                            fence_proxy_async_smem();
+                            __syncwarp();
+                            if (ln == 0 && col0 < p.N && row0 < p.M) {
+                                tma_store_2d(&tmC, part, col0, row0);
+                                tma_store_commit();
                             }
                         } else {
-                            store_elements<(int)ROWB>(dst, pitch, out_stage, (int)ln, rows_valid, cols_valid);
+                            __syncwarp();
+                            store_own<(int)G::PART_ROW>(static_cast<unsigned char*>(p.C) + ((int64_t)row0 * p.ldc + col0) * 4, p.ldc * 4, part,
+                                                        p.M - row0, p.N - col0, wide, (int)ln);
+                            __syncwarp();
                         }
                     }
                 }
             }
         }
         // shared memory stays valid until the last store has read it
-        if (lane == 0) tma_store_wait_read();
+        if (wide && lane == 0) tma_store_wait_read();
         if (!ok) {
             if (lane == 0) report_timeout(p.status, abort_flag, fail_code);
         }
@@ -825,7 +885,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const TcParams p) {
     const int r = rb * 4 + (x & 3), cg = x >> 2;         // four consecutive threads: the four rows of a 128-byte line of a part
     if (t >= p.tiles_m * p.tiles_n) return;
     int m0, n0;
-    tile_coords<BN>(t, p.tiles_m, m0, n0);
+    tile_coords<BN>(t, p, m0, n0);
     const int m = m0 + r, n = n0 + cg * 8;
     if (m >= p.M || n >= p.N) return;
     const int slice = cg / (COLS / 8), group = cg - slice * (COLS / 8);
@@ -933,30 +993,34 @@ struct TcMaps {
     CUtensorMap a, b, sa, sb, c;
 };
 
-template <int QB, int MODE, bool SEED>
+template <int QB, int MODE, bool SEED, int OUT>
 int launch_one(const TcMaps& tm, const TcParams& p, int grid, cudaStream_t st) {
     constexpr size_t smem = Geo<QB>::total + 1024;
     static SmemOptIn opt_in;
-    const int rc = opt_in.ensure(gemm_tc_kernel<QB, MODE, SEED>, smem);
+    const int rc = opt_in.ensure(gemm_tc_kernel<QB, MODE, SEED, OUT>, smem);
     if (rc != BI8_OK) return rc;
     // setmaxnreg.inc waits for registers that the role warps of the same scheduler give up: if the compiler gave the
     // kernel fewer registers per thread than the budget was written for, the wait would never end.  Checked once.
     static int regs_ok = 0;       // 0 unknown, 1 fine, -1 refused
     if (regs_ok == 0) {
         cudaFuncAttributes fa;
-        BI8_CUDA_TRY(cudaFuncGetAttributes(&fa, gemm_tc_kernel<QB, MODE, SEED>));
+        BI8_CUDA_TRY(cudaFuncGetAttributes(&fa, gemm_tc_kernel<QB, MODE, SEED, OUT>));
         regs_ok = ((1 + kPW) * fa.numRegs >= Cfg::ROLE_REGS + kPW * Cfg::EPI_REGS && (1 + kPW) * 32 * fa.numRegs <= 16384) ? 1 : -1;
     }
     if (regs_ok < 0) return fail(BI8_ERR_CUDA, "tensor-core GEMM: the kernel was compiled with a register count its register moves do not fit");
-    return launch_chained(gemm_tc_kernel<QB, MODE, SEED>, grid, Cfg::THREADS, smem, st, tm.a, tm.b, tm.sa, tm.sb, tm.c, p);
+    return launch_chained(gemm_tc_kernel<QB, MODE, SEED, OUT>, grid, Cfg::THREADS, smem, st, tm.a, tm.b, tm.sa, tm.sb, tm.c, p);
 }
 
 int tc_bn() { return Cfg::BN; }
 
 template <int QB>
 int launch_qb(const TcMaps& tm, const TcParams& p, int grid, bool partials, bool seed, cudaStream_t st) {
-    if (partials) return seed ? launch_one<QB, 1, true>(tm, p, grid, st) : launch_one<QB, 1, false>(tm, p, grid, st);
-    return seed ? launch_one<QB, 0, true>(tm, p, grid, st) : launch_one<QB, 0, false>(tm, p, grid, st);
+    if (partials) return seed ? launch_one<QB, 1, true, kAnyOut>(tm, p, grid, st) : launch_one<QB, 1, false, kAnyOut>(tm, p, grid, st);
+    if (!seed) return launch_one<QB, 0, false, kAnyOut>(tm, p, grid, st);
+    if (p.ksplit > 1) return launch_one<QB, 0, true, kSplit>(tm, p, grid, st);
+    if (p.out_dtype == BI8_F32) return launch_one<QB, 0, true, kWide>(tm, p, grid, st);
+    if (p.store == kOwn) return launch_one<QB, 0, true, kOwn16>(tm, p, grid, st);
+    return p.bias || p.residual ? launch_one<QB, 0, true, kTma16Add>(tm, p, grid, st) : launch_one<QB, 0, true, kTma16>(tm, p, grid, st);
 }
 
 }  // namespace
@@ -1070,7 +1134,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     tm.sa = tm.a;          // stand-ins that are never dereferenced
     tm.sb = tm.b;
     if (tma_sa) {
-        rc = cached_scale_map(&tm.sa, dev, g.sA, nb, g.M, kBM, bps);
+        rc = cached_scale_map(&tm.sa, dev, g.sA, nb, g.M, bn, bps);
         if (rc != BI8_OK) return rc;
     }
     if (tma_sb) {
@@ -1097,7 +1161,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     p.vec_store = (g.C != nullptr && aligned(g.C, 16) && (g.ldc * esz) % 16 == 0) ? 1 : 0;
     p.wait_limit_us = g.wait_limit_us;
     p.skip_stage = g.skip_stage;
-    tm.c = tm.a;           // stand-in, never dereferenced without tma_store
+    tm.c = tm.a;           // stand-in, never dereferenced unless the store mode is kTma
     const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
     if (tiles >= (1ll << 31) / 32) return fail(BI8_ERR_SHAPE, "too many output tiles");
     SplitPlan pl;
@@ -1113,15 +1177,18 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     p.residual = g.residual;
     p.ldr = g.ldr;
     p.res_vec = (g.residual != nullptr && aligned(g.residual, 16) && (g.ldr * esz) % 16 == 0) ? 1 : 0;
-    // (a tensor map clips at 16 bytes: where rows end inside such a piece, the bytes behind them would be written)
+    p.store = kOwn;
+    // (a tensor map clips at 16 bytes: a last piece that is not whole would be written whole)
     if (!partials && pl.ksplit == 1 && p.vec_store && (g.N * esz) % 16 == 0) {
         // one box = what a promotion warp stages per pass: 32 rows x (its columns, or half of them for 4-byte elements)
         const int cols = bn / kPW;
         rc = cached_output_map(&tm.c, dev, g.C, esz, g.M, g.N, g.ldc, 32, esz == 2 ? cols : cols / 2);
         if (rc != BI8_OK) return rc;
-        p.tma_store = 1;
+        p.store = kTma;
     }
     p.ws = static_cast<float*>(g.workspace);
+    while ((1ll << p.tm_shift) < p.tiles_m) ++p.tm_shift;
+    p.tm_mul = (unsigned)((((1ull << p.tm_shift) - (unsigned)p.tiles_m) << 32) / (unsigned)p.tiles_m + 1);
     const int64_t items = tiles * pl.ksplit;
     const int grid = (int)(items < di.sms ? items : di.sms);
     const bool seed = (g.flags & BI8_GEMM_NO_SEED) == 0;

@@ -14,7 +14,7 @@ namespace bi8 {
 constexpr int kBK = 128;   // K bytes per pipeline stage (one 128-byte swizzle row)
 
 // codes stored in the status word's detail when a bounded wait gives up
-enum WaitCode { W_EMPTY_AB = 1, W_FULL_AB = 2, W_ACC_EMPTY = 3, W_ACC_FULL = 4, W_SC_EMPTY = 5, W_SC_FULL = 6, W_PROBE = 7, W_PART = 8 };
+enum WaitCode { W_EMPTY_AB = 1, W_FULL_AB = 2, W_ACC_EMPTY = 3, W_ACC_FULL = 4, W_SC_EMPTY = 5, W_SC_FULL = 6, W_PROBE = 7, W_PART = 8, W_OUT_FULL = 9, W_OUT_EMPTY = 10 };
 
 // Raises the CTA's abort flag (a word in shared memory) and records the first failing wait in the device's
 // status word.
