@@ -1039,17 +1039,18 @@ struct SplitPlan {
 };
 // What a work item takes per stage (128 K-bytes of a tile: four, two or one blocks to promote), what dividing costs whatever its size
 // (the second kernel's latency; of its host time a part) and per slot (80 KB written and read again through L2): microseconds.
-// Stage: from 32 to 128 stages of 148 undivided tiles, 1.48 us at block 32, 0.71 at 64, 0.45 at 128.  The others from a
+// Stage: slope over 4 to 32 stages of 4736 undivided tiles, 1.38 us at block 32, 0.68 at 64, 0.43 at 128.  The others from a
 // sweep of 1 to 32 items per tile over 14 shapes of 7 to 320 tiles and 6 to 86 stages at the three blocks: with them the plan's time is
 // within 6 % of the best measured one everywhere (512 x 768 x 768: 9.2 us in six items against 12.7 at block 32, 7.9 undivided
 // against 8.2 at 64, 6.5 against 7.3 at 128; 300 x 768 x 3072: 13.0 in eight, 10.6 in eight, 9.3 in six).  The number of
 // items with the lowest sum is taken; the largest that the SMs hold is often not the fastest.
-double stage_us(int block) { return block <= 32 ? 1.48 : block <= 64 ? 0.72 : 0.45; }
+double stage_us(int block) { return block <= 32 ? 1.38 : block <= 64 ? 0.68 : 0.43; }
 constexpr double kSplitUs = 2.9, kSlotUs = 0.017;
-// Where the tiles alone occupy more than half of the SMs, dividing has to save a twentieth, the workspace stays within half of L2, and from
-// kSplitRounds rounds on nothing is left to be saved.
+// Where the tiles alone occupy more than half of the SMs, dividing has to save a twentieth, the workspace stays within L2 (8192 x 50257 x
+// 768: 320 tiles in two parts, 52 MB and five rounds of 197 stages, 732 us; in four, 105 MB and nine rounds of 99, 685), and
+// from kSplitRounds rounds on nothing is left to be saved.
 constexpr double kSplitWorth = 0.95;
-constexpr size_t kSplitBytes = 64u << 20;
+constexpr size_t kSplitBytes = 112u << 20;
 constexpr int kSplitRounds = 6;
 
 SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, int sms) {
