@@ -90,12 +90,13 @@ struct Cfg {
 };
 
 // How a finished tile leaves: kTma, through the tensor map tmC (16-bit outputs by the storer warp, fp32 ones in two passes by the promotion
-// warps: handing the halves over was 2 us slower where there is one round of tiles); kOwn, by the promotion warps, to
-// outputs that a tensor map cannot describe.
-enum StoreMode { kTma = 0, kOwn = 1 };
+// warps: handing the halves over was 2 us slower where there is one round of tiles); kRows, by the storer warp to 16-bit
+// outputs whose rows no tensor map can describe, but every eighth of which one can (store_rows); kOwn, by the promotion warps,
+// to all others.
+enum StoreMode { kTma = 0, kRows = 1, kOwn = 2 };
 // Instances of the kernel by the way its tiles leave: code for the other ways, even where it is not executed, costs the K loop up to
 // 10 % through its registers (8192 x 4096 x 11008 at block 64).
-enum OutKind { kAnyOut = 0, kSplit, kTma16, kTma16Add, kOwn16, kWide };
+enum OutKind { kAnyOut = 0, kSplit, kTma16, kTma16Add, kRows16, kOwn16, kWide };
 
 struct TcParams {
     const float* sA;
@@ -145,13 +146,15 @@ struct Geo {
     static constexpr uint32_t misc_off = bar_off + NBARS * 8;   // tmem holder (4 B) + abort flag (4 B) + never-raised flag (4 B)
     // Finished tiles are staged as one part of 32 rows of 80 bytes per promotion warp; a tile of fp32 takes two passes of half its columns.
     static constexpr uint32_t PART_ROW = C::COLS * 2, PART_BYTES = 32 * PART_ROW;
-    static constexpr uint32_t OUT_BYTES = C::EPI_WARPS * PART_BYTES;
+    // kRows: [8 rows modulo 8][16] bodies of 304 bytes, then per row the first and the last eight elements
+    static constexpr uint32_t BODY = C::BN * 2 - 16, CLASS_BYTES = kBM / 8 * BODY, EDGES = 8 * CLASS_BYTES;
+    static constexpr uint32_t OUT_BYTES = EDGES + kBM * 32;
     static constexpr uint32_t out_off = (misc_off + 16 + 127) & ~127u;
     // operand of the seeding MMAs (both A and B): 16 fp16 values per row as 8-row core matrices
     static constexpr uint32_t seed_off = out_off + OUT_BYTES;
     static constexpr uint32_t SEED_BYTES = C::BN * 32;
     static constexpr uint32_t total = seed_off + SEED_BYTES;
-    static_assert(PART_BYTES % 128 == 0, "TMA store sources are 128-byte aligned");
+    static_assert(PART_BYTES % 128 == 0 && CLASS_BYTES % 128 == 0 && OUT_BYTES >= C::EPI_WARPS * PART_BYTES && OUT_BYTES % 128 == 0, "TMA store sources are 128-byte aligned");
     static_assert(SC_REC % 128 == 0 && C::scale_off % 1024 == 0, "TMA destinations of the scale boxes are 128-byte aligned");
 };
 
@@ -337,6 +340,59 @@ __device__ __noinline__ void store_own(unsigned char* dst, int64_t pitch, uint32
     }
 }
 
+// 16-bit outputs with rows of any even alignment (kRows).  Rows that are eight apart have the same alignment, so a tensor map whose
+// "rows" are eight rows long describes them: with h the elements of a tile row before its first 16-byte boundary, elements h .. h+151
+// of the 16 rows of a tile that are equal modulo 8 leave by one TMA store, the first h and last 8-h one by one; a last, partial column of tiles is kOwn's.  8192 x 50257, K 768:
+// 848 us by the promotion warps, 694 this way (604 with aligned rows); one bulk copy per row took 110 cycles a row, 16-byte pieces moved by the storer
+// 190 (1430 and 1870 us).
+__device__ __forceinline__ uint32_t rows_head(const TcParams& p, uint32_t row_class, int n0) {
+    return (0u - (row_class * (uint32_t)p.ldc + (uint32_t)n0)) & 7u;
+}
+// A thread's 40 results (pairs, in `e`) of slice `sl` of a row whose class has head `h` to the row's body and edges.
+template <uint32_t BODY, int PAIRS>
+__device__ __forceinline__ void stage_row(uint32_t body, uint32_t edges, uint32_t sl, uint32_t h, const uint32_t (&e)[PAIRS]) {
+    if (sl == 0) sts_v4(edges, e[0], e[1], e[2], e[3]);
+    if (sl == 3) sts_v4(edges + 16u, e[PAIRS - 4], e[PAIRS - 3], e[PAIRS - 2], e[PAIRS - 1]);
+    // words of the body: at odd heads they hold the second half of one pair and the first of the next
+    const uint32_t sh = (h & 1u) * 16u;
+    const int at = (int)(sl * 4u * PAIRS) - 2 * (int)((h + 1u) & ~1u);        // byte of word 0 in the body
+    const uint32_t dst = body + (uint32_t)at;
+    if (sl != 0) {
+        if (sh) sts_h(dst + 2u, e[0]);
+        else sts_w(dst, e[0]);
+        if (sh && sl != 3) sts_h(dst + 4u * PAIRS, e[PAIRS - 1] >> 16);
+    } else {
+        if (sh) sts_h(dst + 4u * PAIRS, e[PAIRS - 1] >> 16);
+        if (at == 0) sts_w(dst, e[0]);
+    }
+#pragma unroll
+    for (int k = 1; k < PAIRS; ++k) {
+        const uint32_t v = __funnelshift_l(e[k - 1], e[k], sh);
+        if (k < 4) {
+            if (at + 4 * k >= 0) sts_w(dst + (uint32_t)(4 * k), v);
+        } else if (k >= PAIRS - 4) {
+            if (at + 4 * k < (int)BODY) sts_w(dst + (uint32_t)(4 * k), v);
+        } else {
+            sts_w(dst + (uint32_t)(4 * k), v);
+        }
+    }
+}
+template <uint32_t BODY>
+__device__ __forceinline__ void store_rows(const TcParams& p, const void* tmC, uint32_t out, int m0, int n0, int lane) {
+    constexpr uint32_t CLASS = kBM / 8 * BODY, EDGES = 8 * CLASS;
+    constexpr int LAST = BODY / 2;                           // column of the tile's last eight
+    const int rows = p.M - m0 < kBM ? p.M - m0 : kBM;
+    uint16_t* const c0 = static_cast<uint16_t*>(p.C) + (int64_t)m0 * p.ldc + n0;
+    if (lane < 8) tma_store_2d(tmC, out + (uint32_t)lane * CLASS, lane * (int)p.ldc + n0 + (int)rows_head(p, (uint32_t)lane, n0), m0 / 8);
+    const uint32_t j = (uint32_t)lane & 7u;
+    const bool first0 = j < rows_head(p, (uint32_t)lane >> 3, n0), first1 = j < rows_head(p, ((uint32_t)lane >> 3) + 4u, n0);
+#pragma unroll 4
+    for (int r = lane >> 3; r < kBM; r += 4) {
+        const bool first = (r & 4) ? first1 : first0;
+        if (r < rows) c0[(int64_t)r * p.ldc + (first ? 0 : LAST) + j] = lds_u16(out + EDGES + (uint32_t)r * 32u + (first ? 0u : 16u) + 2u * j);
+    }
+}
+
 // Adds bias[n] and then residual[m, n], each in the output type, to a thread's staged row (COLS 16-bit or COLS/2 fp32 values at
 // shared address `row_addr`, columns from col0).  Columns and rows outside the output get no addend; they are not stored.
 template <int COLS>
@@ -394,9 +450,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     using G = Geo<QB>;
     constexpr int BN = C::BN, COLS = C::COLS, CH = C::CH;
     constexpr bool kScales = (MODE == 0);           // the partial-sum dump uses no scales
-    const int store = OUT == kTma16 || OUT == kTma16Add ? kTma : OUT == kOwn16 ? kOwn : p.store;
+    const int store = OUT == kTma16 || OUT == kTma16Add ? kTma : OUT == kRows16 ? kRows : OUT == kOwn16 ? kOwn : p.store;
     const bool wide = OUT == kWide || (OUT == kAnyOut && p.out_dtype == BI8_F32);
-    const bool addends = OUT != kTma16 && (OUT == kTma16Add || p.bias != nullptr || p.residual != nullptr);
+    const bool addends = OUT != kTma16 && OUT != kRows16 && (OUT == kTma16Add || p.bias != nullptr || p.residual != nullptr);
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
     // dynamic shared memory is only guaranteed 16-byte aligned: round up to the swizzle atom
     const uint32_t raw = smem_u32(smem_dyn);
@@ -619,7 +675,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     for (int b = 0; b < kAccBufs; ++b)
                         if (j + b < blocks && ok) seed_acc(b);
             }
-        } else if (warp == 3 && MODE == 0 && OUT != kSplit && p.ksplit == 1 && store == kTma && !wide) {
+        } else if (warp == 3 && MODE == 0 && OUT != kSplit && p.ksplit == 1 && store != kOwn && !wide) {
             // ---------------- storer ----------------
             uint32_t par = 0;
             bool ok = true;
@@ -639,7 +695,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 // the promotion warps' writes (ordered by the barrier) before the copies below
                 fence_proxy_async_smem();
                 // rows and columns of the boxes that lie outside the tensor are not written
-                if (lane < C::EPI_WARPS) {
+                if (OUT == kRows16) {
+                    // (a last, partial column of tiles has been stored by the promotion warps)
+                    if (n0 + BN <= p.N) store_rows<G::BODY>(p, &tmC, base + G::out_off, m0, n0, lane);
+                } else if (lane < C::EPI_WARPS) {
                     const int col0 = n0 + (lane >> 2) * COLS, row0 = m0 + (lane & 3) * 32;
                     if (col0 < p.N && row0 < p.M) tma_store_2d(&tmC, base + G::out_off + (uint32_t)lane * G::PART_BYTES, col0, row0);
                 }
@@ -779,7 +838,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid_now));
                 const uint32_t ln = tid_now & 31u, w = (tid_now >> 5) - (uint32_t)kRoleWarps, qt = w & 3u, sl = w >> 2;
                 const uint32_t out = base + G::out_off;
-                if (store == kTma && !wide) {
+                if (store != kOwn && !wide) {
                     // the copies of the tile before must have read the staging area
                     ok = warp_wait(bar0 + 8u * (uint32_t)G::OUT_EMPTY, out_par, abort_flag, wait_limit);
                     if (!ok) {
@@ -806,17 +865,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             e[i] = pack_f16x2(lo, hi);
                         }
                     }
-#pragma unroll
-                    for (int g = 0; g < COLS / 8; ++g) sts_v4(my_row + (uint32_t)(g * 16), e[4 * g], e[4 * g + 1], e[4 * g + 2], e[4 * g + 3]);
-                    if (addends) add_staged<COLS>(p, my_row, m, nbase, wide);
-                    __syncwarp();
-                    if (store == kTma) {
-                        if (ln == 0) mbar_arrive(bar0 + 8u * (uint32_t)G::OUT_FULL);
+                    const bool own = store == kOwn || (OUT == kRows16 && nbase - (int)sl * COLS + BN > p.N);
+                    if (OUT == kRows16 && !own) {
+                        stage_row<G::BODY>(out + (ln & 7u) * G::CLASS_BYTES + (qt * 4u + (ln >> 3)) * G::BODY, out + G::EDGES + (qt * 32u + ln) * 32u, sl,
+                                           rows_head(p, ln & 7u, nbase - (int)sl * COLS), e);
                     } else {
+#pragma unroll
+                        for (int g = 0; g < COLS / 8; ++g) sts_v4(my_row + (uint32_t)(g * 16), e[4 * g], e[4 * g + 1], e[4 * g + 2], e[4 * g + 3]);
+                        if (addends) add_staged<COLS>(p, my_row, m, nbase, wide);
+                    }
+                    __syncwarp();
+                    if (own) {
                         store_own<(int)G::PART_ROW>(static_cast<unsigned char*>(p.C) + ((int64_t)(m - (int)ln) * p.ldc + nbase) * 2, p.ldc * 2, part,
                                                     p.M - m + (int)ln, p.N - nbase, wide, (int)ln);
                         __syncwarp();
                     }
+                    if (store != kOwn && ln == 0) mbar_arrive(bar0 + 8u * (uint32_t)G::OUT_FULL);
                 } else {
 #pragma unroll 1
                     for (int h = 0; h < 2; ++h) {
@@ -1019,6 +1083,7 @@ int launch_qb(const TcMaps& tm, const TcParams& p, int grid, bool partials, bool
     if (!seed) return launch_one<QB, 0, false, kAnyOut>(tm, p, grid, st);
     if (p.ksplit > 1) return launch_one<QB, 0, true, kSplit>(tm, p, grid, st);
     if (p.out_dtype == BI8_F32) return launch_one<QB, 0, true, kWide>(tm, p, grid, st);
+    if (p.store == kRows) return launch_one<QB, 0, true, kRows16>(tm, p, grid, st);
     if (p.store == kOwn) return launch_one<QB, 0, true, kOwn16>(tm, p, grid, st);
     return p.bias || p.residual ? launch_one<QB, 0, true, kTma16Add>(tm, p, grid, st) : launch_one<QB, 0, true, kTma16>(tm, p, grid, st);
 }
@@ -1179,6 +1244,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     p.ldr = g.ldr;
     p.res_vec = (g.residual != nullptr && aligned(g.residual, 16) && (g.ldr * esz) % 16 == 0) ? 1 : 0;
     p.store = kOwn;
+    const bool seed = (g.flags & BI8_GEMM_NO_SEED) == 0;
     // (a tensor map clips at 16 bytes: a last piece that is not whole would be written whole)
     if (!partials && pl.ksplit == 1 && p.vec_store && (g.N * esz) % 16 == 0) {
         // one box = what a promotion warp stages per pass: 32 rows x (its columns, or half of them for 4-byte elements)
@@ -1186,13 +1252,16 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
         rc = cached_output_map(&tm.c, dev, g.C, esz, g.M, g.N, g.ldc, 32, esz == 2 ? cols : cols / 2);
         if (rc != BI8_OK) return rc;
         p.store = kTma;
+    } else if (!partials && seed && pl.ksplit == 1 && esz == 2 && !g.bias && !g.residual && g.M % 8 == 0 && aligned(g.C, 16) && g.ldc < (1ll << 28) && g.N >= bn) {
+        rc = cached_output_map(&tm.c, dev, g.C, 2, g.M / 8, 7 * g.ldc + g.N, 8 * g.ldc, kBM / 8, bn - 8);
+        if (rc != BI8_OK) return rc;
+        p.store = kRows;
     }
     p.ws = static_cast<float*>(g.workspace);
     while ((1ll << p.tm_shift) < p.tiles_m) ++p.tm_shift;
     p.tm_mul = (unsigned)((((1ull << p.tm_shift) - (unsigned)p.tiles_m) << 32) / (unsigned)p.tiles_m + 1);
     const int64_t items = tiles * pl.ksplit;
     const int grid = (int)(items < di.sms ? items : di.sms);
-    const bool seed = (g.flags & BI8_GEMM_NO_SEED) == 0;
     switch (g.block) {
         case 32: rc = launch_qb<32>(tm, p, grid, partials, seed, st); break;
         case 64: rc = launch_qb<64>(tm, p, grid, partials, seed, st); break;

@@ -283,11 +283,13 @@ def test_bounded_wait_gives_up_cleanly():
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("shape", [
     # (M, N, row pitch of C beyond N, elements between a 16-byte boundary and C)
+    # the third row: rows of any even alignment by every eighth row (M a multiple of 8, more than one tile column, C aligned)
     (1, 160, 0, 0), (128, 161, 0, 0), (129, 163, 0, 1), (33, 7, 2, 3), (300, 330, 5, 7), (257, 240, 3, 2), (130, 1, 0, 5), (64, 488, 8, 0),
+    (256, 325, 0, 0), (136, 479, 3, 0), (8, 321, 1, 0), (264, 778, 0, 0), (128, 327, 2, 0), (16, 1604, 0, 0),
 ])
 def test_tile_store_paths(shape, dtype):
-    """Undivided tiles reach C by tensor map or, where none describes it, from the promotion warps: the same bits at every alignment,
-    and nothing written outside the M x N elements (a pitch of whole 16-byte pieces with rows that end inside one)."""
+    """Undivided tiles reach C by tensor map or, where none describes it, by every eighth row or from the promotion warps: the same bits at
+    every alignment, and nothing written outside the M x N elements (a pitch of whole 16-byte pieces with rows that end inside one)."""
     from blockwise_int8_linear_b200 import _lib
     L = _lib.lib()
     set_config(64, dtype)
