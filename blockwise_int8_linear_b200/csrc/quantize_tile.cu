@@ -8,12 +8,17 @@
 //
 // Persistent CTAs walk over tiles of 128 rows x 128 columns of a 16-bit input:
 //   * one elected thread fetches the tile with two TMA loads (64 columns = 128 bytes wide each, 128-byte swizzle) that
-//     complete on an mbarrier; rows and columns outside the tensor arrive as zeros.  Inputs whose rows are not 16-byte
-//     aligned, which a tensor map cannot describe (a 50257-wide vocabulary), are fetched by all threads instead (SHIFT): a
-//     half-warp reads a tile row as aligned 16-byte pieces, shifts the bytes into place between neighbouring lanes and
-//     stores them where the TMA would have put them.  The loads of the next tile are in flight, in registers, while the
-//     current one is quantized.  (A zero-padded copy in front of the kernel cost one more pass: 0.9 ms for a
-//     8192 x 50257 matrix.);
+//     complete on an mbarrier; rows and columns outside the tensor arrive as zeros.
+//   * Inputs whose rows are not 16-byte aligned, which a tensor map cannot describe (a 50257-wide vocabulary): rows eight
+//     apart share an alignment, so a tensor map whose "rows" are eight rows long describes them.  Eight TMA loads (kOct) fetch
+//     the 16 rows of a tile that are equal modulo 8, 136 columns from the 16-byte boundary at or before the tile's first.
+//     The threads shift what they read by the class's offset, which is a constant for the column-wise role's unrolled
+//     rows and, with a warp per class, for a whole warp of the row-wise role.  8192 x 50257: dual 494 -> 399 us (345 with aligned
+//     rows), column-wise 488 -> 224 (225).
+//     Where the number of rows is not a multiple of 8 (kShift) all threads fetch: a half-warp reads a tile row as aligned
+//     16-byte pieces, shifts the bytes into place between neighbouring lanes and stores them where the TMA would have put
+//     them.  The loads of the next tile are in flight, in registers, while the current one is quantized.  (A zero-padded
+//     copy in front of the kernel cost one more pass: 0.9 ms for a 8192 x 50257 matrix.);
 //   * column-wise: a thread owns a pair of adjacent columns and 32 rows.  It reads them as 32 four-byte words (all lanes
 //     of a warp read one row: conflict free under the swizzle), takes the absmax of both columns with packed 16-bit
 //     max instructions, exchanges it with the other row groups of its block through shared memory, and quantizes
@@ -44,11 +49,15 @@ constexpr int kQThreads = 256;
 enum { QW_LOAD = 1, QW_EMPTY = 2 };
 
 // shared memory layout (offsets from a 1024-byte aligned base) for NST input stages
+enum InputKind { kTiled = 0, kShift = 1, kOct = 2 };   // how a tile is fetched
 constexpr uint32_t kInStage = 2 * kQT * 128;          // two sub-tiles [128 rows][128 bytes]
-template <int NST>
+constexpr int kOctCols = kQT + 8;                     // kOct: columns fetched
+constexpr uint32_t kOctRow = kOctCols * 2, kOctClass = kQT / 8 * kOctRow, kOctStage = 8 * kOctClass;   // [8 classes][16 rows][272 bytes]
+static_assert(kOctClass % 128 == 0 && kOctStage % 1024 == 0, "TMA destinations");
+template <int NST, int IN>
 struct QLayout {
-    static constexpr uint32_t in_off = 0;
-    static constexpr uint32_t outc_off = NST * kInStage;              // [128 columns][128 row bytes]
+    static constexpr uint32_t in_off = 0, in_stage = IN == kOct ? kOctStage : kInStage;
+    static constexpr uint32_t outc_off = NST * in_stage;              // [128 columns][128 row bytes]
     static constexpr uint32_t ex_off = outc_off + kQT * 128;          // absmax exchange [4 row groups][128 columns] fp32
     static constexpr uint32_t bar_off = ex_off + 4 * kQT * 4;         // 2 * NST barriers and the abort flag
     static constexpr uint32_t outr_off = bar_off + 1024;              // [128 rows][128 column bytes]   (dual only)
@@ -225,7 +234,7 @@ struct ShiftLoader {
     }
 };
 
-template <typename T, int B, bool DUAL, bool SHIFT>
+template <typename T, int B, bool DUAL, int IN>
 __global__ void __launch_bounds__(DUAL ? 2 * kQThreads : kQThreads, DUAL ? 1 : 2)
 quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmQc,
                      const __grid_constant__ CUtensorMap tmQr, const void* __restrict__ x, int64_t ldx, float* __restrict__ s_col,
@@ -233,7 +242,8 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     static_assert(B == 32 || B == 64 || B == 128, "block sizes of the tile quantizer");
     constexpr int NT = DUAL ? 2 * kQThreads : kQThreads;
     constexpr int NST = DUAL ? 3 : 2;                      // input stages: the loads of the next NST - 1 tiles are in flight
-    using L = QLayout<NST>;
+    using L = QLayout<NST, IN>;
+    constexpr bool SHIFT = IN == kShift, OCT = IN == kOct;
     constexpr long long kLimit = 2000000000ll;            // about a second at the boost clock
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
     const uint32_t raw = smem_u32(smem_dyn);
@@ -246,10 +256,16 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
 
     auto issue = [&](int t, int stage) {
         const int c0 = (t % col_tiles) * kQT, r0 = (t / col_tiles) * kQT;
-        const uint32_t dst = base + L::in_off + (uint32_t)stage * kInStage;
-        mbar_expect_tx(full(stage), kInStage);
-        tma_load_2d(dst, &tmX, full(stage), c0, r0);
-        tma_load_2d(dst + kQT * 128, &tmX, full(stage), c0 + 64, r0);
+        const uint32_t dst = base + L::in_off + (uint32_t)stage * L::in_stage;
+        mbar_expect_tx(full(stage), L::in_stage);
+        if constexpr (OCT) {
+#pragma unroll 1
+            for (int k = 0; k < 8; ++k)
+                tma_load_2d(dst + (uint32_t)k * kOctClass, &tmX, full(stage), (int)(((int64_t)k * ldx + c0) & ~7ll), r0 / 8);
+        } else {
+            tma_load_2d(dst, &tmX, full(stage), c0, r0);
+            tma_load_2d(dst + kQT * 128, &tmX, full(stage), c0 + 64, r0);
+        }
     };
     if (tid == 0) {
         for (int s = 0; s < NST; ++s) {
@@ -308,7 +324,9 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             if (!ok) fail_code = QW_LOAD;
         }
         const int c0 = (int)(t % col_tiles) * kQT, r0 = (int)(t / col_tiles) * kQT;
-        const uint32_t in_tile = base + L::in_off + (uint32_t)cur * kInStage;
+        const uint32_t in_tile = base + L::in_off + (uint32_t)cur * L::in_stage;
+        // kOct: elements between the class's first fetched column and the tile's
+        auto oct_shift = [&](int k) { return ((uint32_t)k * (uint32_t)ldx + (uint32_t)c0) & 7u; };
         const int this_stage = cur;
         if (++cur == NST) { cur = 0; par ^= 1u; }
         // SHIFT: the next tile goes into stage `cur`, last read NST - 1 iterations ago
@@ -337,11 +355,32 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             uint32_t v[32];
             uint32_t m2 = 0u;
             if (ok) {
+                if constexpr (OCT) {
+                    const int valid = C - (c0 + 2 * p);    // columns of the pair inside the tensor
+                    const uint32_t keep = valid >= 2 ? 0xffffffffu : valid == 1 ? 0xffffu : 0u;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int r = g * 32 + i;
-                    v[i] = lds_u32(in + swz(r, w >> 2));
-                    m2 = Pk<T>::absmax(v[i], m2);
+                    for (int k = 0; k < 8; ++k) {
+                        const uint32_t sh = oct_shift(k);
+                        const uint32_t at = in_tile + (uint32_t)k * kOctClass + (uint32_t)(g * 4) * kOctRow + (sh >> 1) * 4u + (uint32_t)p * 4u;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) v[8 * j + k] = lds_u32(at + (uint32_t)j * kOctRow);
+                        if (sh & 1u) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) v[8 * j + k] = __funnelshift_r(v[8 * j + k], lds_u32(at + (uint32_t)j * kOctRow + 4u), 16);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        v[i] &= keep;
+                        m2 = Pk<T>::absmax(v[i], m2);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        const int r = g * 32 + i;
+                        v[i] = lds_u32(in + swz(r, w >> 2));
+                        m2 = Pk<T>::absmax(v[i], m2);
+                    }
                 }
                 mbar_arrive(empty(this_stage));            // this thread's part of the stage is in registers
             }
@@ -413,14 +452,39 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
         } else {
             // ---------------- row-wise ----------------
             const int rwarp = rtid >> 5;
-            const int row = rwarp * 16 + (lane & 7) + 8 * (lane >> 4), half = (lane >> 3) & 1;
+            // kOct: warp w has the rows equal to w modulo 8, in the order of their place in the staged class
+            const int row = OCT ? (lane & 15) * 8 + rwarp : rwarp * 16 + (lane & 7) + 8 * (lane >> 4), half = OCT ? lane >> 4 : (lane >> 3) & 1;
+            const int srow = OCT ? rwarp * 16 + (lane & 15) : row;        // row of the staged output
             const uint32_t in = in_tile + (uint32_t)(half * kQT * 128);
             uint32_t v[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0u;
             if (ok) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) lds_v4(in + swz(row, k), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                for (int k = 0; k < 8; ++k) {
+                    const uint32_t at = OCT ? in_tile + (uint32_t)rwarp * kOctClass + (uint32_t)(lane & 15) * kOctRow + (uint32_t)(half * 128 + 16 * k) : in + swz(row, k);
+                    lds_v4(at, v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                }
+                if constexpr (OCT) {
+                    uint32_t t[4];
+                    lds_v4(in_tile + (uint32_t)rwarp * kOctClass + (uint32_t)(lane & 15) * kOctRow + (uint32_t)(half * 128 + 128), t[0], t[1], t[2], t[3]);
+                    const uint32_t sh = oct_shift(rwarp), bits = (sh & 1u) * 16u;
+                    auto shifted = [&](auto words) {       // the columns begin `WS` words and `bits` bits into what was read
+                        constexpr int WS = decltype(words)::value;
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            v[i] = __funnelshift_r(i + WS < 32 ? v[(i + WS) & 31] : t[(i + WS) & 3], i + WS + 1 < 32 ? v[(i + WS + 1) & 31] : t[(i + WS + 1) & 3], bits);
+                    };
+                    if ((sh >> 1) == 0) shifted(std::integral_constant<int, 0>{});
+                    else if ((sh >> 1) == 1) shifted(std::integral_constant<int, 1>{});
+                    else if ((sh >> 1) == 2) shifted(std::integral_constant<int, 2>{});
+                    else shifted(std::integral_constant<int, 3>{});
+                    const int valid = C - (c0 + half * 64);
+                    if (valid < 64) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = 2 * i >= valid ? 0u : 2 * i + 1 >= valid ? v[i] & 0xffffu : v[i];
+                    }
+                }
                 mbar_arrive(empty(this_stage));
             }
             constexpr int NBT = B == 32 ? 2 : 1;           // blocks inside the thread's 64 columns
@@ -434,7 +498,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                 Pk<T>::unpack(m2, lo, hi);
                 amax[b] = fmaxf(lo, hi);
             }
-            if (B == 128) amax[0] = fmaxf(amax[0], __shfl_xor_sync(0xffffffffu, amax[0], 8));   // the row's other half
+            if (B == 128) amax[0] = fmaxf(amax[0], __shfl_xor_sync(0xffffffffu, amax[0], OCT ? 16 : 8));   // the row's other half
             if (rtid == 0) tma_store_wait_read();
             ok = role_barrier_all(rt_id, kQThreads, ok);
             if (!ok) break;
@@ -459,7 +523,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                             pq.template q<FAST>(x2, x3, b2, b3);
                             wd[u] = pack4(b0, b1, b2, b3);
                         }
-                        sts_v4(outr + swz(row, half * 4 + b * (4 / NBT) + k), wd[0], wd[1], wd[2], wd[3]);
+                        sts_v4(outr + swz(srow, half * 4 + b * (4 / NBT) + k), wd[0], wd[1], wd[2], wd[3]);
                     }
                 };
                 if (pq.fast) quantize_row(std::true_type{});
@@ -476,7 +540,8 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             fence_proxy_async_smem();
             role_barrier(rt_id, kQThreads);
             if (rtid == 0) {
-                tma_store_2d(&tmQr, outr, c0, r0);
+                if constexpr (OCT) tma_store_3d(&tmQr, outr, c0, r0 / 8, 0);
+                else tma_store_2d(&tmQr, outr, c0, r0);
                 tma_store_commit();
             }
             store_next();
@@ -502,6 +567,38 @@ int make_q_map(CUtensorMap* map, int8_t* ptr, int64_t rows, int64_t cols, int64_
     return BI8_OK;
 }
 
+// The same tensor as [8 rows modulo 8][rows / 8][cols] -> boxes of 8 x 16 rows x 128 bytes (rows a multiple of 8)
+int make_q_oct_map(CUtensorMap* map, int8_t* ptr, int64_t rows, int64_t cols, int64_t ld) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return fail(BI8_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    ensure_current_context();
+    cuuint64_t gdim[3] = {(cuuint64_t)cols, (cuuint64_t)(rows / 8), 8};
+    cuuint64_t gstride[2] = {(cuuint64_t)ld * 8, (cuuint64_t)ld};
+    cuuint32_t box[3] = {128, kQT / 8, 8};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, ptr, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(BI8_ERR_CUDA, "cuTensorMapEncodeTiled (int8 rows modulo 8) failed with CUresult %d", (int)r);
+    return BI8_OK;
+}
+
+// 16-bit [rows, cols] with rows of any even alignment and row pitch ld elements, rows a multiple of 8 and a 16-byte aligned base, as
+// "rows" of eight rows -> boxes of 136 columns x 16 of them, no swizzle.  Columns behind a row are the next row's.
+int make_x_oct_map(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return fail(BI8_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    ensure_current_context();
+    cuuint64_t gdim[2] = {(cuuint64_t)(7 * ld + cols), (cuuint64_t)(rows / 8)};
+    cuuint64_t gstride[1] = {(cuuint64_t)ld * 16};
+    cuuint32_t box[2] = {kOctCols, kQT / 8};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(BI8_ERR_CUDA, "cuTensorMapEncodeTiled (input rows modulo 8) failed with CUresult %d", (int)r);
+    return BI8_OK;
+}
+
 // 16-bit [rows, cols] row-major with row pitch ld elements -> boxes of 64 columns x 128 rows, 128-byte swizzle
 int make_x_map(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld) {
     EncodeTiledFn fn = encode_fn();
@@ -520,29 +617,29 @@ int make_x_map(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, in
 
 // Encoded maps are looked up in the library's map table first (kinds 5 and 6 there): a training step quantizes tensors of
 // the same few shapes at addresses the allocator keeps handing back, and an encode is a driver call of a few microseconds.
-int cached_x_map(CUtensorMap* map, int dev, const void* ptr, int64_t rows, int64_t cols, int64_t ld) {
-    const MapKey key{dev, 5, ptr, rows, cols, ld, 128, 64};
+int cached_x_map(CUtensorMap* map, int dev, const void* ptr, int64_t rows, int64_t cols, int64_t ld, bool oct) {
+    const MapKey key{dev, oct ? 7 : 5, ptr, rows, cols, ld, 128, 64};
     if (map_cache().find(key, map)) return BI8_OK;
-    const int rc = make_x_map(map, ptr, rows, cols, ld);
+    const int rc = oct ? make_x_oct_map(map, ptr, rows, cols, ld) : make_x_map(map, ptr, rows, cols, ld);
     if (rc == BI8_OK) map_cache().put(key, *map);
     return rc;
 }
-int cached_q_map(CUtensorMap* map, int dev, int8_t* ptr, int64_t rows, int64_t cols, int64_t ld) {
-    const MapKey key{dev, 6, ptr, rows, cols, ld, 128, 128};
+int cached_q_map(CUtensorMap* map, int dev, int8_t* ptr, int64_t rows, int64_t cols, int64_t ld, bool oct) {
+    const MapKey key{dev, oct ? 8 : 6, ptr, rows, cols, ld, 128, 128};
     if (map_cache().find(key, map)) return BI8_OK;
-    const int rc = make_q_map(map, ptr, rows, cols, ld);
+    const int rc = oct ? make_q_oct_map(map, ptr, rows, cols, ld) : make_q_map(map, ptr, rows, cols, ld);
     if (rc == BI8_OK) map_cache().put(key, *map);
     return rc;
 }
 
-template <typename T, int B, bool DUAL, bool SHIFT>
+template <typename T, int B, bool DUAL, int IN>
 int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap& tqr, const void* x, int64_t ldx, float* s_col, float* s_row,
                 int64_t R, int64_t C, cudaStream_t st) {
     const int64_t ctiles = (C + kQT - 1) / kQT, rtiles = (R + kQT - 1) / kQT;
     if (ctiles * rtiles >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "quantize: grid too large");
-    constexpr size_t smem = (DUAL ? QLayout<3>::bytes_dual : QLayout<2>::bytes_col) + 1024;
+    constexpr size_t smem = (DUAL ? QLayout<3, IN>::bytes_dual : QLayout<2, IN>::bytes_col) + 1024;
     static SmemOptIn opt_in;
-    const int rc = opt_in.ensure(quantize_tile_kernel<T, B, DUAL, SHIFT>, smem);
+    const int rc = opt_in.ensure(quantize_tile_kernel<T, B, DUAL, IN>, smem);
     if (rc != BI8_OK) return rc;
     int* status = device_status_ptr();
     if (!status) return BI8_ERR_CUDA;
@@ -550,7 +647,7 @@ int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap
     const int64_t tiles = ctiles * rtiles;
     const int64_t resident = (int64_t)(DUAL ? 1 : 2) * di.sms;                 // CTAs that fit at once
     const int grid = (int)(tiles < resident ? tiles : resident);
-    return launch_chained(quantize_tile_kernel<T, B, DUAL, SHIFT>, grid, DUAL ? 2 * kQThreads : kQThreads, smem, st, tx, tqc, tqr, x, ldx, s_col, s_row, (int)R, (int)C, (int)ctiles, (int)tiles, status);
+    return launch_chained(quantize_tile_kernel<T, B, DUAL, IN>, grid, DUAL ? 2 * kQThreads : kQThreads, smem, st, tx, tqc, tqr, x, ldx, s_col, s_row, (int)R, (int)C, (int)ctiles, (int)tiles, status);
 }
 
 template <typename T>
@@ -559,22 +656,24 @@ int tile_dispatch(const void* x, int64_t ldx, int8_t* q_col, int64_t ldqc, float
     CUtensorMap tx, tqc, tqr;
     int dev = 0;
     BI8_CUDA_TRY(cudaGetDevice(&dev));
-    int rc = cached_q_map(&tqc, dev, q_col, C, R, ldqc);
+    int rc = cached_q_map(&tqc, dev, q_col, C, R, ldqc, false);
     if (rc != BI8_OK) return rc;
     tx = tqr = tqc;
-    const bool shift = !aligned(x, 16) || (ldx * 2) % 16 != 0;        // no tensor map can describe the input
-    if (!shift) {
-        rc = cached_x_map(&tx, dev, x, R, C, ldx);
+    const bool tiled = aligned(x, 16) && (ldx * 2) % 16 == 0;         // a tensor map can describe the input
+    const bool oct = !tiled && aligned(x, 16) && R % 8 == 0 && ldx < (1ll << 28);   // ... or every eighth row of it
+    if (tiled || oct) {
+        rc = cached_x_map(&tx, dev, x, R, C, ldx, oct);
         if (rc != BI8_OK) return rc;
     }
     const bool dual = q_row != nullptr;
     if (dual) {
-        rc = cached_q_map(&tqr, dev, q_row, R, C, ldqr);
+        rc = cached_q_map(&tqr, dev, q_row, R, C, ldqr, oct);
         if (rc != BI8_OK) return rc;
     }
 #define BI8_TILE_D(BB, DUAL)                                                                                \
-    shift ? launch_tile<T, BB, DUAL, true>(tx, tqc, tqr, x, ldx, s_col, s_row, R, C, st)                    \
-          : launch_tile<T, BB, DUAL, false>(tx, tqc, tqr, x, ldx, s_col, s_row, R, C, st)
+    tiled ? launch_tile<T, BB, DUAL, kTiled>(tx, tqc, tqr, x, ldx, s_col, s_row, R, C, st)                  \
+    : oct ? launch_tile<T, BB, DUAL, kOct>(tx, tqc, tqr, x, ldx, s_col, s_row, R, C, st)                    \
+          : launch_tile<T, BB, DUAL, kShift>(tx, tqc, tqr, x, ldx, s_col, s_row, R, C, st)
 #define BI8_TILE(BB) \
     if (block == BB) return dual ? (BI8_TILE_D(BB, true)) : (BI8_TILE_D(BB, false));
     BI8_TILE(32) BI8_TILE(64) BI8_TILE(128)

@@ -122,7 +122,9 @@ def test_row_strided_input():
 
 
 @pytest.mark.parametrize("block", [32, 64, 128, 256, 48])
-@pytest.mark.parametrize("shape", [(128, 128), (200, 136), (64, 1000), (1000, 64), (70, 33), (8192, 768), (130, 50257), (50257, 40)])
+@pytest.mark.parametrize("shape", [(128, 128), (200, 136), (64, 1000), (1000, 64), (70, 33), (8192, 768), (130, 50257), (50257, 40),
+                                   # rows of any even alignment, a multiple of 8 of them: fetched by every eighth row
+                                   (8, 3), (72, 33), (136, 127), (256, 129), (200, 257), (64, 1003), (1032, 386), (8, 50257)])
 def test_colwise_equals_transpose_then_rowwise(shape, block):
     from triton_functions import quantize_block_colwise
     x = randn_bf16(shape, shape[0] + 7 * shape[1], outliers=0.01)
@@ -135,7 +137,8 @@ def test_colwise_equals_transpose_then_rowwise(shape, block):
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("block", [32, 64, 128, 48])
 @pytest.mark.parametrize("shape", [(128, 128), (256, 384), (208, 144), (48, 1008), (1008, 48), (8192, 768), (4096, 4096),
-                                   (70, 33), (200, 136), (130, 50257)])
+                                   (70, 33), (200, 136), (130, 50257),
+                                   (8, 3), (72, 33), (136, 127), (256, 129), (200, 257), (64, 1003), (1032, 386), (8, 50257)])
 def test_dual_equals_both_single_quantizers(shape, block, dt):
     """One read, both quantizations: each output must be bit-identical to its single-purpose function and to the
     oracle (zero columns, NaN-free outliers and ragged tile edges included; shapes the one-pass kernel does not take go
