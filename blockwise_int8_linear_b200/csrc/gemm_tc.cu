@@ -41,7 +41,7 @@
 // needs no int->float conversion.  s = sA[j,m]/127^2 rounded to 22 significant bits makes 1.5*2^23*s exact.
 // The pattern is written by an fp16 MMA of constants (every row 2048, 2048, 2048, 0 ...: 3 * 2048^2 = 1.5*2^23, exact in any
 // order) that overwrites the accumulator, issued by the seeder and complete (commit, barrier) before the block's int8 MMAs are
-// issued.  As tensor-memory stores of the promotion warps it cost them 100 of 590 cycles per block in isolation and held
+// issued; its A lies in tensor memory, so that it reads only B from shared memory (1.3 % at block 64).  As tensor-memory stores of the promotion warps it cost them 100 of 590 cycles per block in isolation and held
 // every accumulator until the last of its columns was folded.
 #include "bi8_common.cuh"
 #include "tc_common.cuh"
@@ -150,7 +150,7 @@ struct Geo {
     static constexpr uint32_t BODY = C::BN * 2 - 16, CLASS_BYTES = kBM / 8 * BODY, EDGES = 8 * CLASS_BYTES;
     static constexpr uint32_t OUT_BYTES = EDGES + kBM * 32;
     static constexpr uint32_t out_off = (misc_off + 16 + 127) & ~127u;
-    // operand of the seeding MMAs (both A and B): 16 fp16 values per row as 8-row core matrices
+    // operand B of the seeding MMAs: 16 fp16 values per row as 8-row core matrices
     static constexpr uint32_t seed_off = out_off + OUT_BYTES;
     static constexpr uint32_t SEED_BYTES = C::BN * 32;
     static constexpr uint32_t total = seed_off + SEED_BYTES;
@@ -661,7 +661,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 accpar[buf] ^= 1u;
                 tc_fence_after();
                 if (lane == 0) {
-                    mma_f16(tmem_base + (uint32_t)(buf * BN), desc, desc, idesc, 0u);
+                    mma_f16_ta(tmem_base + (uint32_t)(buf * BN), tmem_base + (uint32_t)(kAccBufs * BN), desc, idesc, 0u);
                     tc_commit(bar(G::ACC_SEEDED + buf));
                 }
                 __syncwarp();
@@ -722,6 +722,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const uint32_t bar0 = keep(bars);
         const uint32_t leader = keep(lane == 0 ? 1u : 0u);
         const float div = 1.0f / (127.0f * 127.0f);
+        if (SEED && slice == 0) {
+            // A of the seeding MMAs: the same rows as B's, in eight spare tensor-memory columns
+            static_assert(kAccBufs * BN + 8 <= 512, "no spare tensor-memory columns");
+            const uint32_t row_words[8] = {0x68006800u, 0x00006800u, 0u, 0u, 0u, 0u, 0u, 0u};
+            tmem_st8(t_lane + (uint32_t)(kAccBufs * BN), row_words);
+            tmem_wait_st();
+        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
