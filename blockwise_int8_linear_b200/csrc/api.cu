@@ -283,15 +283,20 @@ int bi8_column_sum(const void* x, int dtype, int64_t ldx, void* out, int64_t R, 
     return launch_column_sum(x, dtype, ldx, out, R, C, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
-size_t bi8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int block) {
+namespace {
+size_t gemm_scratch(int64_t M, int64_t N, int64_t K, int block, bool used) {
     if (M <= 0 || N <= 0 || K <= 0 || (block != 32 && block != 64 && block != 128)) return 0;
     GemmArgs g{};
     g.M = M;
     g.N = N;
     g.K = K;
     g.block = block;
-    return gemm_tc_workspace_bytes(g);
+    return gemm_tc_workspace_bytes(g, used);
 }
+}  // namespace
+
+size_t bi8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int block) { return gemm_scratch(M, N, K, block, false); }
+size_t bi8_gemm_workspace_used(int64_t M, int64_t N, int64_t K, int block) { return gemm_scratch(M, N, K, block, true); }
 
 int bi8_gemm_dequant(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb, const float* sA, const float* sB,
                      const void* bias, int bias_dtype, void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N, int64_t K,

@@ -160,7 +160,8 @@ struct GemmArgs {
 };
 
 bool gemm_tc_applicable(const GemmArgs& g, const char** why);
-size_t gemm_tc_workspace_bytes(const GemmArgs& g);
+size_t gemm_tc_workspace_bytes(const GemmArgs& g, bool used);   // `used`: nothing where clusters add the parts
+size_t gemm_tc_static_bytes(int64_t M, int64_t N, int64_t K);
 bool gemm_tc_fills_device(const GemmArgs& g);
 int launch_gemm_tc(const GemmArgs& g, cudaStream_t st);
 int launch_gemm_generic(const GemmArgs& g, cudaStream_t st);

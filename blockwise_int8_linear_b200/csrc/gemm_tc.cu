@@ -47,6 +47,7 @@
 #include "tc_common.cuh"
 
 #include <cstring>
+#include <mutex>
 #include <type_traits>
 
 
@@ -96,7 +97,7 @@ struct Cfg {
 enum StoreMode { kTma = 0, kRows = 1, kOwn = 2 };
 // Instances of the kernel by the way its tiles leave: code for the other ways, even where it is not executed, costs the K loop up to
 // 10 % through its registers (8192 x 4096 x 11008 at block 64).
-enum OutKind { kAnyOut = 0, kSplit, kTma16, kTma16Add, kRows16, kOwn16, kWide };
+enum OutKind { kAnyOut = 0, kSplit, kCluster, kTma16, kTma16Add, kRows16, kOwn16, kWide };
 
 struct TcParams {
     const float* sA;
@@ -142,26 +143,40 @@ struct Geo {
     // barrier slots (8 bytes each)
     static constexpr int FULL_AB = 0, EMPTY_AB = kStages, ACC_FULL = 2 * kStages, ACC_EMPTY = 2 * kStages + kAccBufs,
                          ACC_SEEDED = 2 * kStages + 2 * kAccBufs, OUT_FULL = 2 * kStages + 3 * kAccBufs, OUT_EMPTY = OUT_FULL + 1,
-                         NBARS = OUT_EMPTY + 1;
+                         RX_FULL = OUT_EMPTY + 1, NBARS = RX_FULL + 8;
     static constexpr uint32_t misc_off = bar_off + NBARS * 8;   // tmem holder (4 B) + abort flag (4 B) + never-raised flag (4 B)
     // Finished tiles are staged as one part of 32 rows of 80 bytes per promotion warp; a tile of fp32 takes two passes of half its columns.
     static constexpr uint32_t PART_ROW = C::COLS * 2, PART_BYTES = 32 * PART_ROW;
     // kRows: [8 rows modulo 8][16] bodies of 304 bytes, then per row the first and the last eight elements
     static constexpr uint32_t BODY = C::BN * 2 - 16, CLASS_BYTES = kBM / 8 * BODY, EDGES = 8 * CLASS_BYTES;
     static constexpr uint32_t OUT_BYTES = EDGES + kBM * 32;
-    static constexpr uint32_t out_off = (misc_off + 16 + 127) & ~127u;
     // operand B of the seeding MMAs: 16 fp16 values per row as 8-row core matrices
-    static constexpr uint32_t seed_off = out_off + OUT_BYTES;
+    static constexpr uint32_t seed_off = (misc_off + 16 + 127) & ~127u;
     static constexpr uint32_t SEED_BYTES = C::BN * 32;
-    static constexpr uint32_t total = seed_off + SEED_BYTES;
+    // kCluster: what a warp has of a tile, in fp32; a warp that finishes its part receives one from every other CTA, and stages there
+    static constexpr uint32_t RX_BYTES = 32 * C::COLS * 4;
+    static constexpr uint32_t out_off = seed_off + SEED_BYTES;
+    static constexpr uint32_t total = out_off + OUT_BYTES;
+    static constexpr size_t cluster_total(int n) {
+        const uint32_t rx = (uint32_t)((C::EPI_WARPS + n - 1) / n) * (uint32_t)(n - 1) * RX_BYTES;
+        return out_off + (rx > OUT_BYTES ? rx : OUT_BYTES);
+    }
     static_assert(PART_BYTES % 128 == 0 && CLASS_BYTES % 128 == 0 && OUT_BYTES >= C::EPI_WARPS * PART_BYTES && OUT_BYTES % 128 == 0, "TMA store sources are 128-byte aligned");
     static_assert(SC_REC % 128 == 0 && C::scale_off % 1024 == 0, "TMA destinations of the scale boxes are 128-byte aligned");
 };
 
 // Work item -> tile and K-stage range.  Items of one split are consecutive, so CTAs that run together work on different
-// tiles of the same K range.  `slot` is the item's place in the workspace, -1 where tiles are not divided.
+// tiles of the same K range; the parts of a tile that a cluster shares are its CTAs.  `slot` is the item's place in the
+// workspace, -1 where there is none.
+template <int OUT>
 __device__ __forceinline__ void item_range(int item, const TcParams& p, int nks, int& tile, int& slot, int& ks0, int& ks1) {
-    if (p.ksplit == 1) {
+    if (OUT == kCluster) {
+        tile = item / p.ksplit;
+        const int split = item - tile * p.ksplit;
+        slot = -1;
+        ks0 = split * nks / p.ksplit;
+        ks1 = (split + 1) * nks / p.ksplit;
+    } else if (p.ksplit == 1) {
         tile = item;
         slot = -1;
         ks0 = 0;
@@ -451,7 +466,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     constexpr int BN = C::BN, COLS = C::COLS, CH = C::CH;
     constexpr bool kScales = (MODE == 0);           // the partial-sum dump uses no scales
     const int store = OUT == kTma16 || OUT == kTma16Add ? kTma : OUT == kRows16 ? kRows : OUT == kOwn16 ? kOwn : p.store;
-    const bool wide = OUT == kWide || (OUT == kAnyOut && p.out_dtype == BI8_F32);
+    const bool wide = OUT == kWide || ((OUT == kAnyOut || OUT == kCluster) && p.out_dtype == BI8_F32);
     const bool addends = OUT != kTma16 && OUT != kRows16 && (OUT == kTma16Add || p.bias != nullptr || p.residual != nullptr);
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
     // dynamic shared memory is only guaranteed 16-byte aligned: round up to the swizzle atom
@@ -488,10 +503,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         mbar_init(bar(G::OUT_FULL), C::EPI_WARPS);
         mbar_init(bar(G::OUT_EMPTY), 1);
+        if (OUT == kCluster)
+            for (int w = 0; w < 8; ++w) mbar_init(bar(G::RX_FULL + w), 1);
         sts_u32(abort_flag, 0u);
         sts_u32(never_flag, 0u);                     // a flag nobody raises, for waits that must not be cut short
         mbar_fence_init();
         fence_proxy_async_smem();
+        if (OUT == kCluster) {
+            // the places of the parts that this CTA finishes: one part from every other CTA
+            const int rank = (int)cluster_rank();
+            for (int w = rank; w < C::EPI_WARPS; w += p.ksplit) mbar_expect_tx(bar(G::RX_FULL + w / p.ksplit), (uint32_t)(p.ksplit - 1) * G::RX_BYTES);
+        }
     }
     if (warp == 1) {
         tmem_alloc(smem_u32((const void*)tmem_holder), 512);
@@ -507,6 +529,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    if (OUT == kCluster) cluster_arrive();          // the barriers are set up: waited for before the first send
     // Launched so that all of the above may run while the preceding kernel finishes; no global memory is touched before this
     // wait.  Dependents become resident as this kernel's CTAs leave.
     after_predecessor();
@@ -528,7 +551,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const bool tma_sa = kScales && (p.tma_scales & 1), tma_sb = kScales && (p.tma_scales & 2);
             for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
                 int tile, slot, ks0, ks1, m0, n0;
-                item_range(item, p, nks, tile, slot, ks0, ks1);
+                item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
                 tile_coords<BN>(tile, p, m0, n0);
                 for (int ks = ks0; ks < ks1; ++ks) {
                     ok = warp_wait(bar(G::EMPTY_AB + stage), phase ^ 1u, abort_flag, wait_limit);
@@ -638,7 +661,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             };
             for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
                 int tile, slot, ks0, ks1;
-                item_range(item, p, nks, tile, slot, ks0, ks1);
+                item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
                 for (int ks = ks0; ks < ks1 && ok; ks += 3) {
                     issue_stage(std::integral_constant<int, 0>{});
                     if (ks + 1 < ks1 && ok) issue_stage(std::integral_constant<int, 1>{});
@@ -668,14 +691,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             };
             for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
                 int tile, slot, ks0, ks1;
-                item_range(item, p, nks, tile, slot, ks0, ks1);
+                item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
                 const int blocks = (ks1 - ks0) * G::BPS;
                 for (int j = 0; j < blocks && ok; j += kAccBufs)
 #pragma unroll
                     for (int b = 0; b < kAccBufs; ++b)
                         if (j + b < blocks && ok) seed_acc(b);
             }
-        } else if (warp == 3 && MODE == 0 && OUT != kSplit && p.ksplit == 1 && store != kOwn && !wide) {
+        } else if (warp == 3 && MODE == 0 && OUT != kSplit && OUT != kCluster && p.ksplit == 1 && store != kOwn && !wide) {
             // ---------------- storer ----------------
             uint32_t par = 0;
             bool ok = true;
@@ -708,6 +731,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (lane == 0) mbar_arrive(bar(G::OUT_EMPTY));
                 par ^= 1u;
             }
+        }
+        if (OUT == kCluster) {
+            // the cluster's barriers: set-up and, below, teardown (see the promotion warps)
+            __syncwarp();
+            cluster_wait();
         }
     } else {
         // ---------------- promotion + epilogue ----------------
@@ -804,7 +832,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
         for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
             int tile, slot, ks0, ks1, m0, n0;
-            item_range(item, p, nks, tile, slot, ks0, ks1);
+            item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
             tile_coords<BN>(tile, p, m0, n0);
             m = m0 + row;
             nbase = n0 + slice * COLS;
@@ -819,7 +847,58 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (j + 1 < j1 && ok) promote_block(std::integral_constant<int, 1>{}, j + 1);
                 if (j + 2 < j1 && ok) promote_block(std::integral_constant<int, 2>{}, j + 2);
             }
+            bool mine = true;
+            if (OUT == kCluster) {
+                // The cluster's CTAs hold sums over their shares of K (one tile each; this loop runs once).  Part w of the tile,
+                // what warp w of every CTA has, is finished by CTA w mod their number: the others write theirs into its
+                // shared memory and it adds them in ascending K order.  (After a wait that ran out a part is sent all the
+                // same, so that nobody waits for it.)
+                const uint32_t n = (uint32_t)p.ksplit, rank = cluster_rank(), w = (uint32_t)warp - (uint32_t)kRoleWarps;
+                const uint32_t owner = w % n, place = base + G::out_off + (w / n) * (n - 1u) * G::RX_BYTES;
+                const uint32_t full = bars + 8u * ((uint32_t)G::RX_FULL + w / n);
+                mine = owner == rank;
+                __syncwarp();
+                cluster_wait();
+                if (!mine) {
+                    // by way of the operand ring: this CTA's MMAs have read their last operands
+                    const uint32_t src = base + w * G::RX_BYTES;
+#pragma unroll
+                    for (int g = 0; g < COLS / 4; ++g) {
+                        float v[4];
+                        unpack_f32x2(acc2[2 * g], v[0], v[1]);
+                        unpack_f32x2(acc2[2 * g + 1], v[2], v[3]);
+                        sts_v4(src + (uint32_t)(lane * 16 + g * 512), __float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0)
+                        bulk_send(map_to(place + (rank < owner ? rank : rank - 1u) * G::RX_BYTES, owner), src, G::RX_BYTES, map_to(full, owner));
+                } else if (ok) {
+                    ok = __all_sync(0xffffffffu, mbar_wait_cluster(full, 0u, abort_flag));
+                    if (!ok) fail_code = W_PART;
+#pragma unroll
+                    for (int g = 0; g < COLS / 4; ++g) {
+                        float own[4], sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                        unpack_f32x2(acc2[2 * g], own[0], own[1]);
+                        unpack_f32x2(acc2[2 * g + 1], own[2], own[3]);
+#pragma unroll 1
+                        for (uint32_t r = 0; r < n; ++r) {
+                            uint32_t v[4] = {__float_as_uint(own[0]), __float_as_uint(own[1]), __float_as_uint(own[2]), __float_as_uint(own[3])};
+                            if (r != rank) lds_v4(place + (r < rank ? r : r - 1u) * G::RX_BYTES + (uint32_t)(lane * 16 + g * 512), v[0], v[1], v[2], v[3]);
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) sum[u] = __fadd_rn(sum[u], __uint_as_float(v[u]));
+                        }
+                        acc2[2 * g] = pack_f32x2(sum[0], sum[1]);
+                        acc2[2 * g + 1] = pack_f32x2(sum[2], sum[3]);
+                    }
+                    __syncwarp();                   // all of the place is read: it may be staged into
+                } else {
+                    // not gone before the others' copies have landed
+                    (void)mbar_wait_cluster(full, 0u, never_flag);
+                }
+            }
             if (!ok) break;
+            if (!mine) continue;
 
             if (MODE == 0 && (OUT == kSplit || (OUT == kAnyOut && slot >= 0))) {
                 // Part of a divided tile: straight from the registers to the item's workspace slot, in the order in which
@@ -845,7 +924,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid_now));
                 const uint32_t ln = tid_now & 31u, w = (tid_now >> 5) - (uint32_t)kRoleWarps, qt = w & 3u, sl = w >> 2;
                 const uint32_t out = base + G::out_off;
-                if (store != kOwn && !wide) {
+                if (OUT != kCluster && store != kOwn && !wide) {
                     // the copies of the tile before must have read the staging area
                     ok = warp_wait(bar0 + 8u * (uint32_t)G::OUT_EMPTY, out_par, abort_flag, wait_limit);
                     if (!ok) {
@@ -854,7 +933,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                     out_par ^= 1u;
                 }
-                const uint32_t part = out + w * G::PART_BYTES, my_row = part + ln * G::PART_ROW;
+                const uint32_t part = OUT == kCluster ? out + (w / (uint32_t)p.ksplit) * ((uint32_t)p.ksplit - 1u) * G::RX_BYTES : out + w * G::PART_BYTES, my_row = part + ln * G::PART_ROW;
                 if (!wide) {
                     uint32_t e[COLS / 2];
                     if (p.out_dtype == BI8_BF16) {
@@ -887,7 +966,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                                     p.M - m + (int)ln, p.N - nbase, wide, (int)ln);
                         __syncwarp();
                     }
-                    if (store != kOwn && ln == 0) mbar_arrive(bar0 + 8u * (uint32_t)G::OUT_FULL);
+                    if (OUT == kCluster) {
+                        if (store == kTma) {
+                            fence_proxy_async_smem();
+                            __syncwarp();
+                            if (ln == 0 && nbase < p.N && m < p.M) {
+                                tma_store_2d(&tmC, part, nbase, m);
+                                tma_store_commit();
+                            }
+                        }
+                    } else if (store != kOwn && ln == 0) {
+                        mbar_arrive(bar0 + 8u * (uint32_t)G::OUT_FULL);
+                    }
                 } else {
 #pragma unroll 1
                     for (int h = 0; h < 2; ++h) {
@@ -925,13 +1015,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
         }
         // shared memory stays valid until the last store has read it
-        if (wide && lane == 0) tma_store_wait_read();
+        if ((wide || OUT == kCluster) && lane == 0) tma_store_wait_read();
         if (!ok) {
             if (lane == 0) report_timeout(p.status, abort_flag, fail_code);
         }
     }
 
     // ---------------- teardown ----------------
+    if (OUT == kCluster) {
+        // no CTA leaves while another may still write into its shared memory
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -1066,7 +1162,7 @@ struct TcMaps {
 
 template <int QB, int MODE, bool SEED, int OUT>
 int launch_one(const TcMaps& tm, const TcParams& p, int grid, cudaStream_t st) {
-    constexpr size_t smem = Geo<QB>::total + 1024;
+    const size_t smem = (OUT == kCluster ? Geo<QB>::cluster_total(p.ksplit) : (size_t)Geo<QB>::total) + 1024;
     static SmemOptIn opt_in;
     const int rc = opt_in.ensure(gemm_tc_kernel<QB, MODE, SEED, OUT>, smem);
     if (rc != BI8_OK) return rc;
@@ -1079,15 +1175,33 @@ int launch_one(const TcMaps& tm, const TcParams& p, int grid, cudaStream_t st) {
         regs_ok = ((1 + kPW) * fa.numRegs >= Cfg::ROLE_REGS + kPW * Cfg::EPI_REGS && (1 + kPW) * 32 * fa.numRegs <= 16384) ? 1 : -1;
     }
     if (regs_ok < 0) return fail(BI8_ERR_CUDA, "tensor-core GEMM: the kernel was compiled with a register count its register moves do not fit");
+    if (OUT == kCluster) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(Cfg::THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = (unsigned)p.ksplit;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        BI8_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<QB, MODE, SEED, OUT>, tm.a, tm.b, tm.sa, tm.sb, tm.c, p));
+        return BI8_OK;
+    }
     return launch_chained(gemm_tc_kernel<QB, MODE, SEED, OUT>, grid, Cfg::THREADS, smem, st, tm.a, tm.b, tm.sa, tm.sb, tm.c, p);
 }
 
 int tc_bn() { return Cfg::BN; }
 
 template <int QB>
-int launch_qb(const TcMaps& tm, const TcParams& p, int grid, bool partials, bool seed, cudaStream_t st) {
+int launch_qb(const TcMaps& tm, const TcParams& p, int grid, bool partials, bool seed, bool cluster, cudaStream_t st) {
     if (partials) return seed ? launch_one<QB, 1, true, kAnyOut>(tm, p, grid, st) : launch_one<QB, 1, false, kAnyOut>(tm, p, grid, st);
     if (!seed) return launch_one<QB, 0, false, kAnyOut>(tm, p, grid, st);
+    if (cluster) return launch_one<QB, 0, true, kCluster>(tm, p, grid, st);
     if (p.ksplit > 1) return launch_one<QB, 0, true, kSplit>(tm, p, grid, st);
     if (p.out_dtype == BI8_F32) return launch_one<QB, 0, true, kWide>(tm, p, grid, st);
     if (p.store == kRows) return launch_one<QB, 0, true, kRows16>(tm, p, grid, st);
@@ -1108,6 +1222,8 @@ struct SplitPlan {
     int stages_per_split = 0;
     int slot_floats = 0;
     size_t bytes = 0;
+    double us = 0.0;
+    bool cluster = false;      // the parts of a tile are the CTAs of a cluster, which add them through shared memory
 };
 // What a work item takes per stage (128 K-bytes of a tile: four, two or one blocks to promote), what dividing costs whatever its size
 // (the second kernel's latency; of its host time a part) and per slot (80 KB written and read again through L2): microseconds.
@@ -1125,7 +1241,23 @@ constexpr double kSplitWorth = 0.95;
 constexpr size_t kSplitBytes = 112u << 20;
 constexpr int kSplitRounds = 6;
 
-SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, int sms) {
+// The parts of a tile as the CTAs of a cluster: one launch and no workspace, but the exchange, and the later start of a cluster behind a
+// kernel that fills the SMs, come to 0.2 + 1.2 us per CTA.  Layer calls, eager / in a graph, against the workspace: 128 x 4096 x
+// 11008 in two 22.7 / 24.0 us against 24.5 / 25.4, 300 x 768 x 3072 at block 32 in two 14.3 / 13.5 against 15.9 / 15.6 (undivided),
+// 384 x 2048 x 2048 in three 15.3 / 14.4 against 15.8 / 15.0; beyond the line 128 x 4096 x 4096 in four 18.0 / 17.7 against
+// 17.3 / 16.6, 256 x 1024 x 1024 in three 11.7 / 10.9 against 11.7 / 10.1.
+constexpr double kMeetUs = 0.2, kMeetPartUs = 1.2;
+constexpr int kMostCluster = 4;          // what the shared memory has places for
+constexpr size_t kSmemLimit = 227 * 1024;
+size_t cluster_smem(int block, int n) {
+    return 1024 + (block == 32 ? Geo<32>::cluster_total(n) : block == 64 ? Geo<64>::cluster_total(n) : Geo<128>::cluster_total(n));
+}
+struct ClusterSlots {
+    bool known = false;
+    int n[kMostCluster + 1] = {0};
+};
+
+SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, double stage, int sms, const ClusterSlots* slots) {
     SplitPlan pl;
     const int bn = tc_bn();
     const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
@@ -1135,7 +1267,6 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, int sms) {
     pl.slot_floats = (int)((M < kBM ? (M + 31) / 32 * 32 : kBM) * bn);
     auto rounds = [&](int64_t items) { return (double)((items + sms - 1) / sms); };
     const bool fills = tiles * 2 > sms;
-    const double stage = stage_us(block);
     double best = rounds(tiles) * stage * nks * (fills ? kSplitWorth : 1.0);
     for (int want = 2; want <= 32 && want <= nks; ++want) {
         const int spp = (nks + want - 1) / want, s = (nks + spp - 1) / spp;
@@ -1147,9 +1278,53 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, int sms) {
             pl.stages_per_split = spp;
         }
     }
-    if (pl.ksplit <= 1) return pl;
-    pl.bytes = (size_t)tiles * (size_t)pl.ksplit * (size_t)pl.slot_floats * 4;
+    for (int c = 2; slots != nullptr && c <= kMostCluster && c <= nks; ++c) {
+        const double cost = stage * ((nks + c - 1) / c) + kMeetUs + kMeetPartUs * c;
+        if (tiles <= slots->n[c] && cluster_smem(block, c) <= kSmemLimit && cost < best) {
+            best = cost;
+            pl.ksplit = c;
+            pl.stages_per_split = (nks + c - 1) / c;
+            pl.cluster = true;
+        }
+    }
+    pl.us = best;
+    if (pl.ksplit > 1 && !pl.cluster) pl.bytes = (size_t)tiles * (size_t)pl.ksplit * (size_t)pl.slot_floats * 4;
     return pl;
+}
+
+// Clusters of 2 to 8 CTAs of the general kernel that the device holds at once (asked once per device).
+const ClusterSlots* cluster_slots() {
+    static ClusterSlots table[64];
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    ClusterSlots& t = table[dev];
+    if (!t.known) {
+        auto kernel = gemm_tc_kernel<64, 0, true, kCluster>;
+        constexpr size_t smem = kSmemLimit;
+        static_assert(Geo<32>::total > kSmemLimit / 2 && Geo<64>::total > kSmemLimit / 2 && Geo<128>::total > kSmemLimit / 2, "one CTA per SM at every block size");
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return nullptr;
+        const int sms = device_info().sms;
+        for (int c = 2; c <= kMostCluster; ++c) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)(c * (sms / c)));
+            cfg.blockDim = dim3(Cfg::THREADS);
+            cfg.dynamicSmemBytes = smem;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)c;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&t.n[c], kernel, &cfg) != cudaSuccess) {
+                (void)cudaGetLastError();
+                t.n[c] = 0;
+            }
+        }
+        t.known = true;
+    }
+    return &t;
 }
 }  // namespace
 
@@ -1158,17 +1333,24 @@ bool gemm_tc_fills_device(const GemmArgs& g) {
     return ((g.M + kBM - 1) / kBM) * ((g.N + tc_bn() - 1) / tc_bn()) * 2 > device_info().sms;
 }
 
-size_t gemm_tc_workspace_bytes(const GemmArgs& g) {
+size_t gemm_tc_workspace_bytes(const GemmArgs& g, bool used) {
     const DeviceInfo di = device_info();
     if (!di.ok || g.partials != nullptr) return 0;
-    return plan_split(g.M, g.N, g.K, g.block, di.sms).bytes;
+    return plan_split(g.M, g.N, g.K, g.block, stage_us(g.block), di.sms, used ? cluster_slots() : nullptr).bytes;
+}
+
+// Scratch of the division through the workspace at block 64, with the stage time that the refusals of bi8_gemm_dequant_static are
+// defined by: which shapes that entry point takes does not move with this kernel's speed.
+size_t gemm_tc_static_bytes(int64_t M, int64_t N, int64_t K) {
+    const DeviceInfo di = device_info();
+    return di.ok ? plan_split(M, N, K, 64, 0.72, di.sms, nullptr).bytes : 0;
 }
 
 double gemm_tc_estimate_us(const GemmArgs& g) {
     const DeviceInfo di = device_info();
-    const SplitPlan pl = plan_split(g.M, g.N, g.K, g.block, di.sms);
-    const int64_t tiles = ((g.M + kBM - 1) / kBM) * ((g.N + tc_bn() - 1) / tc_bn()), items = tiles * pl.ksplit;
-    return stage_us(g.block) * (double)((items + di.sms - 1) / di.sms * pl.stages_per_split) + 3.5 + (pl.ksplit > 1 ? kSplitUs + kSlotUs * (double)items : 0.0);
+    const SplitPlan pl = plan_split(g.M, g.N, g.K, g.block, stage_us(g.block), di.sms, cluster_slots());
+    const int64_t tiles = ((g.M + kBM - 1) / kBM) * ((g.N + tc_bn() - 1) / tc_bn());
+    return 3.5 + (pl.ksplit > 1 ? pl.us : stage_us(g.block) * (double)((tiles + di.sms - 1) / di.sms * pl.stages_per_split));
 }
 
 bool gemm_tc_applicable(const GemmArgs& g, const char** why) {
@@ -1200,7 +1382,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     if (rc != BI8_OK) return rc;
     TcParams p;
     std::memset(&p, 0, sizeof(p));
-    const bool partials = g.partials != nullptr;
+    const bool partials = g.partials != nullptr, seed = (g.flags & BI8_GEMM_NO_SEED) == 0;
     // a scale tensor goes through TMA when a tensor map can describe it: 16-byte aligned base and row length
     const bool tma_sa = !partials && aligned(g.sA, 16) && g.M % 4 == 0, tma_sb = !partials && aligned(g.sB, 16) && g.N % 4 == 0;
     p.tma_scales = (tma_sa ? 1 : 0) | (tma_sb ? 2 : 0);
@@ -1240,9 +1422,10 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     SplitPlan pl;
     pl.stages_per_split = (int)((g.K + kBK - 1) / kBK);
     if (!partials) {
-        const SplitPlan want = plan_split(g.M, g.N, g.K, g.block, di.sms);
+        const SplitPlan want = plan_split(g.M, g.N, g.K, g.block, stage_us(g.block), di.sms, seed && g.wait_limit_us == 0 ? cluster_slots() : nullptr);
         // without a large enough, 16-byte aligned workspace the GEMM simply runs unsplit
-        if (want.ksplit > 1 && g.workspace != nullptr && g.workspace_bytes >= want.bytes && aligned(g.workspace, 16)) pl = want;
+        if (want.cluster) pl = want;
+        else if (want.ksplit > 1 && g.workspace != nullptr && g.workspace_bytes >= want.bytes && aligned(g.workspace, 16)) pl = want;
     }
     p.ksplit = pl.ksplit;
     p.stages_per_split = pl.stages_per_split;
@@ -1251,9 +1434,8 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     p.ldr = g.ldr;
     p.res_vec = (g.residual != nullptr && aligned(g.residual, 16) && (g.ldr * esz) % 16 == 0) ? 1 : 0;
     p.store = kOwn;
-    const bool seed = (g.flags & BI8_GEMM_NO_SEED) == 0;
     // (a tensor map clips at 16 bytes: a last piece that is not whole would be written whole)
-    if (!partials && pl.ksplit == 1 && p.vec_store && (g.N * esz) % 16 == 0) {
+    if (!partials && (pl.ksplit == 1 || pl.cluster) && p.vec_store && (g.N * esz) % 16 == 0) {
         // one box = what a promotion warp stages per pass: 32 rows x (its columns, or half of them for 4-byte elements)
         const int cols = bn / kPW;
         rc = cached_output_map(&tm.c, dev, g.C, esz, g.M, g.N, g.ldc, 32, esz == 2 ? cols : cols / 2);
@@ -1270,12 +1452,12 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     const int64_t items = tiles * pl.ksplit;
     const int grid = (int)(items < di.sms ? items : di.sms);
     switch (g.block) {
-        case 32: rc = launch_qb<32>(tm, p, grid, partials, seed, st); break;
-        case 64: rc = launch_qb<64>(tm, p, grid, partials, seed, st); break;
-        case 128: rc = launch_qb<128>(tm, p, grid, partials, seed, st); break;
+        case 32: rc = launch_qb<32>(tm, p, grid, partials, seed, pl.cluster, st); break;
+        case 64: rc = launch_qb<64>(tm, p, grid, partials, seed, pl.cluster, st); break;
+        case 128: rc = launch_qb<128>(tm, p, grid, partials, seed, pl.cluster, st); break;
         default: return fail(BI8_ERR_BLOCK, "tensor-core GEMM supports block 32, 64, 128 (got %d)", g.block);
     }
-    if (rc != BI8_OK || pl.ksplit == 1) return rc;
+    if (rc != BI8_OK || pl.ksplit == 1 || pl.cluster) return rc;
     constexpr int kTileItems = kBM * (Cfg::BN / 8);
     auto reduce = [&](auto kernel) { return launch_chained(kernel, (unsigned)((tiles * kTileItems + 255) / 256), 256, 0, st, p); };
     constexpr int BN = Cfg::BN, COLS = Cfg::COLS;

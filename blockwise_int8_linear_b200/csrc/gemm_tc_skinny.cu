@@ -132,49 +132,12 @@ size_t smem_of(int share, int cluster, int rx_bufs, uint32_t* sx_off = nullptr, 
 }
 
 // ---- cluster helpers ----------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t map_to(uint32_t smem_addr, uint32_t rank) {     // the same place in another CTA of the cluster
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void remote_arrive(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
 // 16 bytes into another CTA's shared memory, counted there on `cluster_bar`
 __device__ __forceinline__ void send_v4(uint32_t cluster_addr, uint32_t cluster_bar, float a, float b, float c, float d) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%2, %3, %4, %5}, [%1];" ::"r"(cluster_addr),
                  "r"(cluster_bar), "f"(a), "f"(b), "f"(c), "f"(d)
                  : "memory");
 }
-// mbar_wait for data that another CTA of the cluster has sent
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t abort_flag) {
-    const long long t0 = clock64();
-    while (true) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok != 0u) return true;
-        if (lds_volatile_u32(abort_flag) != 0u || clock64() - t0 > 4000000000ll) return false;
-    }
-}
-
 // ---- output -------------------------------------------------------------------------------------------------------------
 // C[m, n] = cast(acc) (+ cast(addend) in the output type: reference lines 125-131) for the CW rows of a chunk and one column n; the
 // addend is bias[n] (bias_ld 0) or an [M, N] residual.  All addends are requested before the first is used.

@@ -67,7 +67,7 @@ int bi8_gemm_dequant_static(const int8_t* A, int64_t lda, const int8_t* Bt, int6
     shape.N = N;
     shape.K = K;
     shape.block = 64;
-    const size_t need = (M > 0 && N > 0 && K > 0 && (block == 32 || block == 64 || block == 128)) ? bi8::gemm_tc_workspace_bytes(shape) : 0;
+    const size_t need = (M > 0 && N > 0 && K > 0 && (block == 32 || block == 64 || block == 128)) ? bi8::gemm_tc_static_bytes(M, N, K) : 0;
     if (need > bi8::kScratchBytes && !bi8::gemm_tc_fills_device(shape))
         return bi8::fail(BI8_ERR_LIMIT,
                          "gemm_dequant_static: this shape needs %zu bytes of split-K scratch, the built-in array holds %zu; "

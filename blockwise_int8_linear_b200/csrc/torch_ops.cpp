@@ -311,7 +311,7 @@ Tensor gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& state_x, const
     const Tensor sx = state_x.contiguous(), sw = state_w.contiguous();
     Tensor c = empty_on(a_in, {m, n}, out_type);
     const Bias bias(bias_in, n);
-    const size_t ws_bytes = bi8_gemm_workspace_bytes(m, n, k, (int)block);
+    const size_t ws_bytes = flags ? bi8_gemm_workspace_bytes(m, n, k, (int)block) : bi8_gemm_workspace_used(m, n, k, (int)block);
     const Tensor ws = scratch(a_in, (int64_t)ws_bytes);
     check(bi8_gemm_dequant(static_cast<const int8_t*>(o.a.ptr), o.a.ld, static_cast<const int8_t*>(o.bt.ptr), o.bt.ld, sx.const_data_ptr<float>(),
                            sw.const_data_ptr<float>(), bias.ptr, bias.code, c.data_ptr(), n, dtype_code(out_type), m, n, k, (int)block,
@@ -423,7 +423,7 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
             return finish();
         }
     }
-    const size_t ws_bytes = bi8_gemm_workspace_bytes(m, n, k, (int)block);
+    const size_t ws_bytes = bi8_gemm_workspace_used(m, n, k, (int)block);
     // the quantized activations live in the call's scratch behind the GEMM's workspace
     Carve carve;
     carve.take((int64_t)ws_bytes);
@@ -511,7 +511,7 @@ void colwise_into(const Mat& m, int code, int64_t block, const QRef& r, void* st
 void dual_into(const Mat& m, int code, int64_t block, const QRef& row, const QRef& col, void* stream) {
     check(bi8_quantize_dual_pitched(m.ptr, code, m.ld, row.q, row.ld, row.s, col.q, col.ld, col.s, m.rows, m.cols, (int)block, stream), "bi8_quantize_dual");
 }
-// out = a b^T (+ bias); `ws` of at least bi8_gemm_workspace_bytes
+// out = a b^T (+ bias); `ws` of at least bi8_gemm_workspace_used
 void gemm_into(const QRef& a, const QRef& b, const Bias* bias, int64_t block, const Tensor& out, void* ws, size_t ws_bytes, void* stream) {
     check(bi8_gemm_dequant(a.q, a.ld, b.q, b.ld, a.s, b.s, bias ? bias->ptr : nullptr, bias ? bias->code : 0, out.data_ptr(), b.rows,
                            dtype_code(out.scalar_type()), a.rows, b.rows, a.cols, (int)block, ws_bytes ? ws : nullptr, ws_bytes, 0, stream),
@@ -600,7 +600,7 @@ variable_list LinearBackward::apply(variable_list&& grads) {
         // every intermediate result of this pass lies in one allocation
         const Quantized cached = need_x ? cache_get(cache, "col") : Quantized{};
         Quantized fresh;                                     // the weight's other blocking, where the cache is to keep it
-        const size_t ws_x = need_x ? bi8_gemm_workspace_bytes(m, k, n, (int)b) : 0, ws_w = need_w ? bi8_gemm_workspace_bytes(n, k, m, (int)b) : 0,
+        const size_t ws_x = need_x ? bi8_gemm_workspace_used(m, k, n, (int)b) : 0, ws_w = need_w ? bi8_gemm_workspace_used(n, k, m, (int)b) : 0,
                      ws_b = need_b ? bi8_column_sum_workspace_bytes(m, n) : 0;
         Carve carve;
         const int64_t ws_at = carve.take((int64_t)std::max({ws_x, ws_w, ws_b}));
@@ -684,7 +684,7 @@ Tensor train_linear(const Tensor& x_in, const Tensor& w, const Tensor& bias_in, 
         const bool keep = node && w.requires_grad() && fuse_dual;
         const Quantized cached = cache_get(cache, "row");
         Quantized fresh;
-        const size_t ws_bytes = bi8_gemm_workspace_bytes(m, n, k, (int)block);
+        const size_t ws_bytes = bi8_gemm_workspace_used(m, n, k, (int)block);
         Carve carve, kept;
         const int64_t ws_at = carve.take((int64_t)ws_bytes);
         const QPlan x_row(carve, m, k, block), x_col = keep ? QPlan(kept, k, m, block) : QPlan();

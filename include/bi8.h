@@ -128,6 +128,9 @@ BI8_API int bi8_gemm_dequant(const int8_t* A, int64_t lda, const int8_t* Bt, int
 
 BI8_API size_t bi8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int block);
 
+/* How much of that a call without flags uses: nothing where the parts of a tile are added inside clusters. */
+BI8_API size_t bi8_gemm_workspace_used(int64_t M, int64_t N, int64_t K, int block);
+
 /* bi8_gemm_dequant plus an addend: C = cast(cast(sum) (+ bias) + residual[m,n]), the addition in the output type as a layer's
  * `x + proj(...)` performs it.  residual [M,N] of out_dtype, row stride ldr; an overlap with C is BI8_ERR_SHAPE. */
 BI8_API int bi8_gemm_dequant_residual(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb,

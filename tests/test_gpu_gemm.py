@@ -322,6 +322,32 @@ def test_tile_store_paths(shape, dtype):
     set_config(64)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [
+    # (M, K, N, block): tiles whose parts are the CTAs of a cluster (of two, three; the last one's plan needs the workspace)
+    (128, 4096, 11008, 64), (70, 4096, 11001, 64), (300, 768, 3072, 32), (384, 2048, 2048, 64), (130, 2000, 5000, 64), (128, 4096, 11008, 128),
+    (128, 4096, 4096, 64),
+])
+def test_divided_tiles_in_clusters(shape, dtype):
+    """Without a workspace only clusters divide a tile: within the tolerance of the oracle on sampled rows, with bias, the same bits
+    call for call, and equal rows give equal bits."""
+    m, k, n, block = shape
+    set_config(block, dtype)
+    xq, xs, wq, ws = quantized_pair(m, k, n, block, seed=m + k)
+    xq[m - 1], xs[:, m - 1] = xq[0], xs[:, 0]
+    bias = torch.randn(n, generator=torch.Generator().manual_seed(n)).to(dtype)
+    c = _gemm(xq, wq, xs, ws, bias)
+    assert torch.equal(c[0], c[m - 1]) and torch.equal(c, _gemm(xq, wq, xs, ws, bias))
+    rows = [0, 1, 31, 32, 63, m // 2, m - 2]
+    args = (c[rows], xq[rows], wq, xs[:, rows].contiguous(), ws, block)
+    if dtype == torch.float32:
+        _check_fp32(*args, bias)
+    else:
+        _check_bf16(*args, bias)
+    assert_clean_device()
+    set_config(64)
+
+
 def test_unaligned_long_contraction_is_repitched_onto_the_tensor_cores():
     """K = 1000 + 17: not a multiple of 16.  The shim re-pitches the operands; results equal the CUDA-core kernel's
     within the tensor-core tolerance and the int32 partial sums stay exact."""
