@@ -27,7 +27,7 @@ int* device_status_ptr() {
     static int* ptrs[64] = {nullptr};
     static std::mutex mu;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    if (current_device(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
         fail(BI8_ERR_CUDA, "cudaGetDevice failed");
         return nullptr;
     }
@@ -181,6 +181,7 @@ int bi8_device_status(int* detail) {
 
 int bi8_quantize_rowwise_pitched(const void* x, int x_dtype, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t M, int64_t K, int block,
                                  void* stream) {
+    DeviceOfCall call;
     if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "quantize_rowwise: unknown dtype code %d", x_dtype);
     if (block < 1) return fail(BI8_ERR_BLOCK, "quantize_rowwise: block size %d", block);
     if (M < 0 || K < 0 || ldx < K || ldq < K) return fail(BI8_ERR_SHAPE, "quantize_rowwise: bad shape M=%lld K=%lld ldx=%lld ldq=%lld", (long long)M, (long long)K, (long long)ldx, (long long)ldq);
@@ -197,6 +198,7 @@ int bi8_quantize_rowwise(const void* x, int x_dtype, int64_t ldx, int8_t* q, flo
 
 int bi8_quantize_colwise_pitched(const void* x, int x_dtype, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t R, int64_t C, int block,
                                  void* stream) {
+    DeviceOfCall call;
     if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "quantize_colwise: unknown dtype code %d", x_dtype);
     if (block < 1) return fail(BI8_ERR_BLOCK, "quantize_colwise: block size %d", block);
     if (R < 0 || C < 0 || ldx < C || ldq < R) return fail(BI8_ERR_SHAPE, "quantize_colwise: bad shape R=%lld C=%lld ldx=%lld ldq=%lld", (long long)R, (long long)C, (long long)ldx, (long long)ldq);
@@ -213,6 +215,7 @@ int bi8_quantize_colwise(const void* x, int x_dtype, int64_t ldx, int8_t* q, flo
 
 int bi8_quantize_dual_pitched(const void* x, int x_dtype, int64_t ldx, int8_t* q_row, int64_t ldq_row, float* s_row, int8_t* q_col, int64_t ldq_col,
                               float* s_col, int64_t R, int64_t C, int block, void* stream) {
+    DeviceOfCall call;
     if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "quantize_dual: unknown dtype code %d", x_dtype);
     if (block < 1) return fail(BI8_ERR_BLOCK, "quantize_dual: block size %d", block);
     if (R < 0 || C < 0 || ldx < C || ldq_row < C || ldq_col < R)
@@ -234,6 +237,45 @@ int bi8_quantize_dual(const void* x, int x_dtype, int64_t ldx, int8_t* q_row, fl
     return bi8_quantize_dual_pitched(x, x_dtype, ldx, q_row, C, s_row, q_col, R, s_col, R, C, block, stream);
 }
 
+int bi8_quantize_many_fits(const bi8_quantize_task* tasks, int n, int block) {
+    return tasks && n > 0 && quantize_jobs_fit(tasks, n, block) ? 1 : 0;
+}
+
+int bi8_quantize_many(const bi8_quantize_task* tasks, int n, int block, void* stream) {
+    DeviceOfCall call;
+    if (n < 0 || (n > 0 && !tasks)) return fail(BI8_ERR_NULL, "quantize_many: null pointer");
+    if (block < 1) return fail(BI8_ERR_BLOCK, "quantize_many: block size %d", block);
+    const bool fits = n > 0 && quantize_jobs_fit(tasks, n, block);
+    for (int i = 0; i < n; ++i) {
+        const bi8_quantize_task& t = tasks[i];
+        const bool copy = t.x_dtype == BI8_I8;
+        if (!copy && !dtype_ok(t.x_dtype)) return fail(BI8_ERR_DTYPE, "quantize_many: unknown dtype code %d", t.x_dtype);
+        if (t.rows < 0 || t.cols < 0 || t.ldx < t.cols || (t.q_row && t.ldq_row < t.cols) || (t.q_col && t.ldq_col < t.rows))
+            return fail(BI8_ERR_SHAPE, "quantize_many: bad shape of task %d", i);
+        if (copy && (!t.q_row || !aligned(t.q_row, 16) || t.ldq_row % 16 != 0 || t.ldq_row < (t.cols + 15) / 16 * 16))
+            return fail(BI8_ERR_ALIGN, "quantize_many: rows of task %d do not begin on 16-byte boundaries", i);
+        if (t.rows == 0 || t.cols == 0) continue;
+        if (!t.x || (!copy && ((t.q_row && !t.s_row) || (t.q_col && !t.s_col)))) return fail(BI8_ERR_NULL, "quantize_many: null pointer in task %d", i);
+        if (!copy && (!aligned(t.x, dtype_size(t.x_dtype)) || (t.q_row && !aligned(t.s_row, 4)) || (t.q_col && !aligned(t.s_col, 4)) ||
+                      (t.sum && !aligned(t.sum, dtype_size(t.x_dtype)))))
+            return fail(BI8_ERR_ALIGN, "quantize_many: pointer of task %d not element aligned", i);
+        if (t.sum && !fits) return fail(BI8_ERR_LIMIT, "quantize_many: column sums only where the tasks fit one launch");
+    }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (fits) return launch_quantize_jobs(tasks, n, block, st);
+    for (int i = 0; i < n; ++i) {
+        const bi8_quantize_task& t = tasks[i];
+        int rc = BI8_OK;
+        if (t.x_dtype == BI8_I8) rc = bi8_copy_rows(static_cast<const int8_t*>(t.x), t.ldx, t.q_row, t.ldq_row, t.rows, t.cols, stream);
+        else if (t.q_row && t.q_col)
+            rc = bi8_quantize_dual_pitched(t.x, t.x_dtype, t.ldx, t.q_row, t.ldq_row, t.s_row, t.q_col, t.ldq_col, t.s_col, t.rows, t.cols, block, stream);
+        else if (t.q_row) rc = bi8_quantize_rowwise_pitched(t.x, t.x_dtype, t.ldx, t.q_row, t.ldq_row, t.s_row, t.rows, t.cols, block, stream);
+        else if (t.q_col) rc = bi8_quantize_colwise_pitched(t.x, t.x_dtype, t.ldx, t.q_col, t.ldq_col, t.s_col, t.rows, t.cols, block, stream);
+        if (rc != BI8_OK) return rc;
+    }
+    return BI8_OK;
+}
+
 size_t bi8_peer_allreduce_buffer_bytes(int world, int64_t capacity) {
     if (world < 1 || world > 8 || capacity <= 0 || capacity % 1024 != 0) return 0;
     return peer_allreduce_buffer_bytes(world, capacity);
@@ -249,6 +291,7 @@ int bi8_peer_allreduce(void* const* peer_bufs, int rank, int world, int64_t capa
 
 int bi8_dequantize_rowwise_pitched(const int8_t* q, int64_t ldq, const float* s, void* out, int out_dtype, int64_t M, int64_t K, int block,
                                    void* stream) {
+    DeviceOfCall call;
     if (!dtype_ok(out_dtype)) return fail(BI8_ERR_DTYPE, "dequantize: unknown dtype code %d", out_dtype);
     if (block < 1) return fail(BI8_ERR_BLOCK, "dequantize: block size %d", block);
     if (M < 0 || K < 0 || ldq < K) return fail(BI8_ERR_SHAPE, "dequantize: bad shape M=%lld K=%lld ldq=%lld", (long long)M, (long long)K, (long long)ldq);
@@ -275,6 +318,7 @@ int bi8_copy_rows(const int8_t* src, int64_t lds, int8_t* dst, int64_t ldd, int6
 size_t bi8_column_sum_workspace_bytes(int64_t R, int64_t C) { return column_sum_workspace_bytes(R, C); }
 
 int bi8_column_sum(const void* x, int dtype, int64_t ldx, void* out, int64_t R, int64_t C, void* workspace, size_t workspace_bytes, void* stream) {
+    DeviceOfCall call;
     if (!dtype_ok(dtype)) return fail(BI8_ERR_DTYPE, "column_sum: unknown dtype code %d", dtype);
     if (R < 0 || C < 0 || ldx < C) return fail(BI8_ERR_SHAPE, "column_sum: bad shape R=%lld C=%lld ldx=%lld", (long long)R, (long long)C, (long long)ldx);
     if (C == 0) return BI8_OK;
@@ -285,6 +329,7 @@ int bi8_column_sum(const void* x, int dtype, int64_t ldx, void* out, int64_t R, 
 
 namespace {
 size_t gemm_scratch(int64_t M, int64_t N, int64_t K, int block, bool used) {
+    DeviceOfCall call;
     if (M <= 0 || N <= 0 || K <= 0 || (block != 32 && block != 64 && block != 128)) return 0;
     GemmArgs g{};
     g.M = M;
@@ -301,6 +346,7 @@ size_t bi8_gemm_workspace_used(int64_t M, int64_t N, int64_t K, int block) { ret
 int bi8_gemm_dequant(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb, const float* sA, const float* sB,
                      const void* bias, int bias_dtype, void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N, int64_t K,
                      int block, void* workspace, size_t workspace_bytes, int flags, void* stream) {
+    DeviceOfCall call;
     GemmArgs g{A, lda, Bt, ldb, sA, sB, bias, bias_dtype, C, ldc, out_dtype, nullptr, M, N, K, block, flags, workspace, workspace_bytes};
     int rc = check_gemm(g, false);
     if (rc != BI8_OK || M == 0 || N == 0) return rc;
@@ -310,6 +356,7 @@ int bi8_gemm_dequant(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb
 int bi8_gemm_dequant_residual(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb, const float* sA, const float* sB, const void* bias,
                               int bias_dtype, const void* residual, int64_t ldr, void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N,
                               int64_t K, int block, void* workspace, size_t workspace_bytes, int flags, void* stream) {
+    DeviceOfCall call;
     GemmArgs g{A, lda, Bt, ldb, sA, sB, bias, bias_dtype, C, ldc, out_dtype, nullptr, M, N, K, block, flags, workspace, workspace_bytes};
     int rc = check_gemm(g, false);
     if (rc != BI8_OK || M == 0 || N == 0) return rc;
@@ -333,6 +380,7 @@ int bi8_gemm_dequant_fused_quant(const void* x, int x_dtype, int64_t ldx, int8_t
                                  const float* sW, const void* bias, int bias_dtype, void* C, int64_t ldc, int out_dtype,
                                  int64_t M, int64_t N, int64_t K, int block, void* workspace, size_t workspace_bytes, int flags,
                                  void* stream) {
+    DeviceOfCall call;
     if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "gemm_dequant_fused_quant: unknown dtype code %d", x_dtype);
     const bool forced = (flags & (BI8_GEMM_FORCE_GENERIC | BI8_GEMM_FORCE_TC | BI8_GEMM_FORCE_SMALLM)) != 0;
     if (!forced && x && M > 0 && N > 0 && K > 0 && ldx >= K && aligned(x, dtype_size(x_dtype)) && Wq && sW && C && ldw >= K && ldc >= N &&
@@ -353,6 +401,7 @@ int bi8_gemm_dequant_fused_quant(const void* x, int x_dtype, int64_t ldx, int8_t
 
 int bi8_quantize_rowwise_pre_pitched(int op, const void* x, const void* x2, int x_dtype, int64_t ldx, const void* weight, float eps, int8_t* q,
                                      int64_t ldq, float* scales, int64_t M, int64_t K, int block, void* stream) {
+    DeviceOfCall call;
     if (!dtype_ok(x_dtype)) return fail(BI8_ERR_DTYPE, "quantize_rowwise_pre: unknown dtype code %d", x_dtype);
     if (op != BI8_PRE_NONE && op != BI8_PRE_RMSNORM && op != BI8_PRE_SILU_MUL)
         return fail(BI8_ERR_SHAPE, "quantize_rowwise_pre: unknown operation code %d", op);
@@ -374,6 +423,7 @@ int bi8_gemm_dequant_fused_pre(int op, const void* x, const void* x2, int x_dtyp
                                int8_t* xq, float* sx, const int8_t* Wq, int64_t ldw, const float* sW, const void* bias, int bias_dtype,
                                const void* residual, int64_t ldr, void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N, int64_t K,
                                int block, void* workspace, size_t workspace_bytes, int flags, void* stream) {
+    DeviceOfCall call;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool scratch = xq != nullptr && sx != nullptr;
     if (residual && ldr < N) return fail(BI8_ERR_SHAPE, "gemm_dequant_fused_pre: residual row pitch smaller than the row");

@@ -27,6 +27,28 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
         if (e__ != cudaSuccess) return ::bi8::fail(BI8_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e__)); \
     } while (0)
 
+// The current device, asked for once per call of the C API: an entry point holds a DeviceOfCall while it works (nothing below it changes
+// the device), and the launchers, plans and tables that are keyed by device find the answer there.  cudaGetDevice costs 0.1 to
+// 0.2 us and a GEMM call asked five times.
+struct DeviceOfCall {
+    static inline thread_local int depth = 0, dev = -1;
+    DeviceOfCall() {
+        if (depth++ == 0) dev = -1;
+    }
+    ~DeviceOfCall() { --depth; }
+    DeviceOfCall(const DeviceOfCall&) = delete;
+    DeviceOfCall& operator=(const DeviceOfCall&) = delete;
+};
+inline cudaError_t current_device(int* dev) {
+    if (DeviceOfCall::depth > 0 && DeviceOfCall::dev >= 0) {
+        *dev = DeviceOfCall::dev;
+        return cudaSuccess;
+    }
+    const cudaError_t e = cudaGetDevice(dev);
+    if (e == cudaSuccess && DeviceOfCall::depth > 0) DeviceOfCall::dev = *dev;
+    return e;
+}
+
 // The opt-in to more than 48 KiB of dynamic shared memory is an attribute of a kernel ON A DEVICE.  A launcher keeps
 // one SmemOptIn per kernel instance (a function-local static) and calls ensure() before every launch: the attribute
 // is set the first time the instance is used on each device, under a mutex (launchers run on several host threads).
@@ -36,7 +58,7 @@ struct SmemOptIn {
     template <typename Kern>
     int ensure(Kern kern, size_t want) {
         int dev = 0;
-        BI8_CUDA_TRY(cudaGetDevice(&dev));
+        BI8_CUDA_TRY(current_device(&dev));
         if (dev < 0 || dev >= 64) return fail(BI8_ERR_CUDA, "device ordinal %d out of range", dev);
         std::lock_guard<std::mutex> lock(mu);
         if (bytes[dev] >= want) return BI8_OK;
@@ -88,6 +110,9 @@ int launch_quantize_colwise(const void* x, int dt, int64_t ldx, int8_t* q, int64
 bool quantize_tile_applicable(int dt, const void* q_col, int64_t ldqc, const void* q_row, int64_t ldqr, int64_t R, int64_t C, int block);
 int launch_quantize_tile(const void* x, int dt, int64_t ldx, int8_t* q_col, int64_t ldqc, float* s_col, int8_t* q_row, int64_t ldqr,
                          float* s_row, int64_t R, int64_t C, int block, cudaStream_t st);
+// several small quantizations, column sums and row copies in one launch (quantize.cu)
+bool quantize_jobs_fit(const bi8_quantize_task* tasks, int n, int block);
+int launch_quantize_jobs(const bi8_quantize_task* tasks, int n, int block, cudaStream_t st);
 // sum of the ranks' fp32 partial results over peer memory (peer_reduce.cu)
 size_t peer_allreduce_buffer_bytes(int world, int64_t capacity);
 int launch_peer_allreduce(void* const* peer_bufs, int rank, int world, int64_t capacity, const float* partial, int64_t M, int64_t N,

@@ -3,11 +3,10 @@
 // The tensor-core GEMM reads its operands by TMA, which takes rows on 16-byte boundaries only.  The library's own intermediate results
 // have them; a dense int8 matrix whose rows are not a multiple of 16 long (the weight buffer of such a layer, a checkpoint's
 // copy, a caller's own tensor) is copied once per call.  Bound by memory, and for the matrices of a few hundred KB that occur by the
-// latency of a launch: 777 x 1000 takes 2 us, 9 us with the three tensor operations that it replaces.  A thread makes 16 bytes of
-// a row from the two aligned pieces that hold them; its neighbour reads the second one too, from L1.
+// latency of a launch: 777 x 1000 takes 2 us, 9 us with the three tensor operations that it replaces.  (copy_rows.cuh has
+// what a thread does; beside a layer's activations it shares their quantizer's launch: quantize_jobs_kernel in quantize.cu.)
 #include "bi8_common.cuh"
-
-#include <type_traits>
+#include "copy_rows.cuh"
 
 namespace bi8 {
 namespace {
@@ -18,27 +17,7 @@ __global__ void __launch_bounds__(kCopyThreads) copy_rows_kernel(const int8_t* _
                                                                  int64_t pieces, int per_row, int64_t cols) {
     after_predecessor();
     const int64_t i = (int64_t)blockIdx.x * kCopyThreads + threadIdx.x;
-    if (i >= pieces) return;
-    const int64_t row = i / per_row, c = (i - row * per_row) * 16;
-    const uintptr_t a = reinterpret_cast<uintptr_t>(src + row * lds + c), end = reinterpret_cast<uintptr_t>(src + row * lds + cols);
-    const uintptr_t base = a & ~(uintptr_t)15;
-    // a piece is read only where it holds a byte of the row: no access leaves the matrix's 16-byte granules
-    const uint4 lo = __ldg(reinterpret_cast<const uint4*>(base));
-    uint4 hi = make_uint4(0u, 0u, 0u, 0u);
-    if (base + 16 < end) hi = __ldg(reinterpret_cast<const uint4*>(base + 16));
-    const uint32_t r[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-    const uint32_t off = (uint32_t)(a & 15u), bits = (off & 3u) * 8u;
-    uint32_t w[4];
-    auto shifted = [&](auto words) {
-        constexpr int WS = decltype(words)::value;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) w[k] = __funnelshift_r(r[k + WS], r[k + WS + 1], bits);
-    };
-    if (off < 4u) shifted(std::integral_constant<int, 0>{});
-    else if (off < 8u) shifted(std::integral_constant<int, 1>{});
-    else if (off < 12u) shifted(std::integral_constant<int, 2>{});
-    else shifted(std::integral_constant<int, 3>{});
-    *reinterpret_cast<uint4*>(dst + row * ldd + c) = make_uint4(w[0], w[1], w[2], w[3]);
+    copy_rows_piece(i, src, lds, dst, ldd, pieces, per_row, cols);
 }
 
 }  // namespace

@@ -223,7 +223,7 @@ bool gemm_smallm_applicable(const GemmArgs& g) {
 
 int launch_gemm_smallm(const GemmArgs& g, cudaStream_t st) {
     int dev = 0, sms = 0;
-    BI8_CUDA_TRY(cudaGetDevice(&dev));
+    BI8_CUDA_TRY(current_device(&dev));
     BI8_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int nb = (int)((g.K + g.block - 1) / g.block);
     const int chunks = (int)((g.K + kChunk - 1) / kChunk);

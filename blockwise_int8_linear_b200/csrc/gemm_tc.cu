@@ -1222,7 +1222,6 @@ struct SplitPlan {
     int stages_per_split = 0;
     int slot_floats = 0;
     size_t bytes = 0;
-    double us = 0.0;
     bool cluster = false;      // the parts of a tile are the CTAs of a cluster, which add them through shared memory
 };
 // What a work item takes per stage (128 K-bytes of a tile: four, two or one blocks to promote), what dividing costs whatever its size
@@ -1242,11 +1241,11 @@ constexpr size_t kSplitBytes = 112u << 20;
 constexpr int kSplitRounds = 6;
 
 // The parts of a tile as the CTAs of a cluster: one launch and no workspace, but the exchange, and the later start of a cluster behind a
-// kernel that fills the SMs, come to 0.2 + 1.2 us per CTA.  Layer calls, eager / in a graph, against the workspace: 128 x 4096 x
+// kernel that fills the SMs, come to 0.2 + 1.25 us per CTA.  Layer calls, eager / in a graph, against the workspace: 128 x 4096 x
 // 11008 in two 22.7 / 24.0 us against 24.5 / 25.4, 300 x 768 x 3072 at block 32 in two 14.3 / 13.5 against 15.9 / 15.6 (undivided),
 // 384 x 2048 x 2048 in three 15.3 / 14.4 against 15.8 / 15.0; beyond the line 128 x 4096 x 4096 in four 18.0 / 17.7 against
 // 17.3 / 16.6, 256 x 1024 x 1024 in three 11.7 / 10.9 against 11.7 / 10.1.
-constexpr double kMeetUs = 0.2, kMeetPartUs = 1.2;
+constexpr double kMeetUs = 0.2, kMeetPartUs = 1.25;
 constexpr int kMostCluster = 4;          // what the shared memory has places for
 constexpr size_t kSmemLimit = 227 * 1024;
 size_t cluster_smem(int block, int n) {
@@ -1278,6 +1277,9 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, double stage, i
             pl.stages_per_split = spp;
         }
     }
+    // (slots of fewer than 128 rows are smaller than what kSlotUs was measured with; a cluster exchanges whole parts: 40 x 3000 x 5000 takes
+    // 14.0 us in four through the workspace and 16.0 in a cluster of four)
+    if (pl.ksplit > 1) best -= kSlotUs * (double)(tiles * pl.ksplit) * (1.0 - (double)pl.slot_floats / (kBM * bn));
     for (int c = 2; slots != nullptr && c <= kMostCluster && c <= nks; ++c) {
         const double cost = stage * ((nks + c - 1) / c) + kMeetUs + kMeetPartUs * c;
         if (tiles <= slots->n[c] && cluster_smem(block, c) <= kSmemLimit && cost < best) {
@@ -1287,7 +1289,6 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, double stage, i
             pl.cluster = true;
         }
     }
-    pl.us = best;
     if (pl.ksplit > 1 && !pl.cluster) pl.bytes = (size_t)tiles * (size_t)pl.ksplit * (size_t)pl.slot_floats * 4;
     return pl;
 }
@@ -1297,7 +1298,7 @@ const ClusterSlots* cluster_slots() {
     static ClusterSlots table[64];
     static std::mutex mu;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    if (current_device(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
     ClusterSlots& t = table[dev];
     if (!t.known) {
@@ -1326,6 +1327,32 @@ const ClusterSlots* cluster_slots() {
     }
     return &t;
 }
+
+// The plan of a shape on the current device, with or without clusters.  A call asks for it two or three times (scratch, choice of kernel,
+// launch) at 0.2 to 0.4 us each; each thread keeps the last few (a plan depends on nothing but its key).
+SplitPlan plan_of(const GemmArgs& g, bool clusters) {
+    struct Entry {
+        int64_t M = -1, N = 0, K = 0;
+        int block = 0, dev = 0;
+        bool clusters = false;
+        SplitPlan plan;
+    };
+    static thread_local Entry memo[8];
+    int dev = 0;
+    if (current_device(&dev) != cudaSuccess) dev = 0;
+    Entry& e = memo[((uint64_t)(g.M * 31 + g.N * 7 + g.K * 3 + g.block + (clusters ? 1 : 0)) * 0x9E3779B97F4A7C15ull) >> 61];
+    if (e.M != g.M || e.N != g.N || e.K != g.K || e.block != g.block || e.dev != dev || e.clusters != clusters) {
+        const SplitPlan plan = plan_split(g.M, g.N, g.K, g.block, stage_us(g.block), device_info().sms, clusters ? cluster_slots() : nullptr);
+        e.M = g.M;
+        e.N = g.N;
+        e.K = g.K;
+        e.block = g.block;
+        e.dev = dev;
+        e.clusters = clusters;
+        e.plan = plan;
+    }
+    return e.plan;
+}
 }  // namespace
 
 // Whether the undivided tiles occupy more than half of the SMs: a caller without a large workspace does without the split there.
@@ -1336,7 +1363,7 @@ bool gemm_tc_fills_device(const GemmArgs& g) {
 size_t gemm_tc_workspace_bytes(const GemmArgs& g, bool used) {
     const DeviceInfo di = device_info();
     if (!di.ok || g.partials != nullptr) return 0;
-    return plan_split(g.M, g.N, g.K, g.block, stage_us(g.block), di.sms, used ? cluster_slots() : nullptr).bytes;
+    return plan_of(g, used).bytes;
 }
 
 // Scratch of the division through the workspace at block 64, with the stage time that the refusals of bi8_gemm_dequant_static are
@@ -1346,11 +1373,15 @@ size_t gemm_tc_static_bytes(int64_t M, int64_t N, int64_t K) {
     return di.ok ? plan_split(M, N, K, 64, 0.72, di.sms, nullptr).bytes : 0;
 }
 
+// For the choice between this kernel and the decode kernel at 33 to 64 rows: the model that the choice was measured with (stages of the
+// kernel as it was then, division through the workspace).  With the present stage times and clusters in it 40 x 3000 x 5000
+// moved here and took 16.0 us instead of 14.0.
 double gemm_tc_estimate_us(const GemmArgs& g) {
     const DeviceInfo di = device_info();
-    const SplitPlan pl = plan_split(g.M, g.N, g.K, g.block, stage_us(g.block), di.sms, cluster_slots());
-    const int64_t tiles = ((g.M + kBM - 1) / kBM) * ((g.N + tc_bn() - 1) / tc_bn());
-    return 3.5 + (pl.ksplit > 1 ? pl.us : stage_us(g.block) * (double)((tiles + di.sms - 1) / di.sms * pl.stages_per_split));
+    const double stage = g.block <= 32 ? 1.48 : g.block <= 64 ? 0.72 : 0.45;
+    const SplitPlan pl = plan_split(g.M, g.N, g.K, g.block, stage, di.sms, nullptr);
+    const int64_t tiles = ((g.M + kBM - 1) / kBM) * ((g.N + tc_bn() - 1) / tc_bn()), items = tiles * pl.ksplit;
+    return stage * (double)((items + di.sms - 1) / di.sms * pl.stages_per_split) + 3.5 + (pl.ksplit > 1 ? kSplitUs + kSlotUs * (double)items : 0.0);
 }
 
 bool gemm_tc_applicable(const GemmArgs& g, const char** why) {
@@ -1370,7 +1401,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     const DeviceInfo di = device_info();
     if (!di.ok) return fail(BI8_ERR_CUDA, "tensor-core GEMM needs a compute capability 10.x device");
     int dev = 0;
-    BI8_CUDA_TRY(cudaGetDevice(&dev));
+    BI8_CUDA_TRY(current_device(&dev));
     if (dev < 0 || dev >= 64) return fail(BI8_ERR_CUDA, "device ordinal %d out of range", dev);
     const int bps = kBK / g.block;
     const int nb = (int)((g.K + g.block - 1) / g.block);
@@ -1422,7 +1453,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     SplitPlan pl;
     pl.stages_per_split = (int)((g.K + kBK - 1) / kBK);
     if (!partials) {
-        const SplitPlan want = plan_split(g.M, g.N, g.K, g.block, stage_us(g.block), di.sms, seed && g.wait_limit_us == 0 ? cluster_slots() : nullptr);
+        const SplitPlan want = plan_of(g, seed && g.wait_limit_us == 0);
         // without a large enough, 16-byte aligned workspace the GEMM simply runs unsplit
         if (want.cluster) pl = want;
         else if (want.ksplit > 1 && g.workspace != nullptr && g.workspace_bytes >= want.bytes && aligned(g.workspace, 16)) pl = want;

@@ -820,7 +820,7 @@ int launch_skinny(const GemmArgs& g, const SkParams& p, int cluster, int cluster
     using G = SkGeo<QB, BNS, SRC>;
     CUtensorMap mw, mx, ms;
     int dev = 0;
-    BI8_CUDA_TRY(cudaGetDevice(&dev));
+    BI8_CUDA_TRY(current_device(&dev));
     int rc = cached_operand_map(&mw, dev, g.Bt, g.N, g.K, g.ldb, kTileRows);
     if (rc != BI8_OK) return rc;
     mx = mw;                        // SRC 1: not used, the kernel writes the activation tiles itself
@@ -856,7 +856,7 @@ int cluster_slots(ClusterSlots* out, int sms) {
     static ClusterSlots table[64];
     static std::mutex mu;
     int dev = 0;
-    BI8_CUDA_TRY(cudaGetDevice(&dev));
+    BI8_CUDA_TRY(current_device(&dev));
     if (dev < 0 || dev >= 64) return fail(BI8_ERR_CUDA, "device ordinal %d out of range", dev);
     std::lock_guard<std::mutex> lock(mu);
     ClusterSlots& t = table[dev];

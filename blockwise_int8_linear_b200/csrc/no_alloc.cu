@@ -33,7 +33,7 @@ void* scratch_ptr() {
     static void* ptrs[64] = {nullptr};
     static std::mutex mu;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    if (current_device(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
         fail(BI8_ERR_CUDA, "gemm_dequant_static: cudaGetDevice failed");
         return nullptr;
     }

@@ -201,7 +201,7 @@ int launch_peer_allreduce_large(void* const* peer_bufs, int rank, int world, int
     int* status = device_status_ptr();
     if (!status) return BI8_ERR_CUDA;
     int dev = 0, sms = 0;
-    BI8_CUDA_TRY(cudaGetDevice(&dev));
+    BI8_CUDA_TRY(current_device(&dev));
     BI8_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t my_chunks = ((count + kPeerChunk - 1) / kPeerChunk + world - 1) / world;
     const long long limit = peer_wait_limit_cycles(wait_limit_us);

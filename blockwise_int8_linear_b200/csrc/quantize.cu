@@ -12,6 +12,7 @@
 // block) by the streaming quantizer, and staged through shared memory by the tile kernels so that its
 // stores (and, for dequantize, its loads) are contiguous along the row index.
 #include "bi8_common.cuh"
+#include "copy_rows.cuh"
 #include "quant_math.cuh"
 #include "tc_common.cuh"
 
@@ -54,6 +55,15 @@ template <>
 __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
 template <>
 __device__ __forceinline__ float to_f32<float>(float v) { return v; }
+
+template <typename TO>
+__device__ __forceinline__ TO from_f32(float v);
+template <>
+__device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+template <>
+__device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
+template <>
+__device__ __forceinline__ float from_f32<float>(float v) { return v; }
 
 // two packed 16-bit floats -> two fp32
 template <typename T>
@@ -126,10 +136,8 @@ __device__ __forceinline__ void load_unit8(const T* p, const T* row_end, int val
 // divisions per lane in fp32, and four of them in sequence were 4.9 us of a 512 x 768 matrix's.  Bound by memory: for 16-bit inputs that the streaming kernel
 // below does not take (rows that are not 32-byte aligned) and for fp32.
 template <typename T, int B, bool SHIFT, int RPW>
-__global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
-    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int M, int K, int nb,
-    int col_tiles) {
-    after_predecessor();
+__device__ __forceinline__ void quantize_rowwise_tile(int tile, const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq,
+                                                      float* __restrict__ s, int M, int K, int nb, int col_tiles) {
     constexpr int WCOLS = 256;              // columns per warp pass
     constexpr int LPB = B / 8;              // lanes sharing one block
     constexpr int BPT = WCOLS / B;          // blocks per tile row
@@ -139,7 +147,7 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
     __shared__ float s_scale[BPT][ROWS];
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ct = blockIdx.x % col_tiles, rt = blockIdx.x / col_tiles;
+    const int ct = tile % col_tiles, rt = tile / col_tiles;
     const int col = ct * WCOLS + lane * 8;
     const int valid = K - col < 8 ? K - col : 8;          // elements of this lane inside the row; <= 0: none
 
@@ -185,6 +193,14 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
         const int jb = ct * BPT + j, row = rt * ROWS + r;
         if (jb < nb && row < M) s[(int64_t)jb * M + row] = s_scale[j][r];
     }
+}
+
+template <typename T, int B, bool SHIFT, int RPW>
+__global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
+    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int M, int K, int nb,
+    int col_tiles) {
+    after_predecessor();
+    quantize_rowwise_tile<T, B, SHIFT, RPW>((int)blockIdx.x, x, ldx, q, ldq, s, M, K, nb, col_tiles);
 }
 
 // Row-wise quantize, streaming path (16-bit inputs, K % 16 == 0, 32-byte aligned rows).
@@ -386,14 +402,13 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_generic_kernel(
 // transposed tile, and each column's B bytes leave as 16-byte pieces (bytes where the output is not aligned).  With one thread per column
 // and a loop down the block (the kernel below) a 300 x 256 matrix took 9 us of serial loads.
 template <typename T, int B>
-__global__ void __launch_bounds__(kThreads) quantize_colwise_cols_kernel(
-    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int R, int C, int col_tiles) {
-    after_predecessor();
+__device__ __forceinline__ void quantize_colwise_tile(int tile_index, const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq,
+                                                      float* __restrict__ s, int R, int C, int col_tiles) {
     constexpr int TC = 64, GROUPS = kThreads / TC, RPT = B / GROUPS;     // columns, row groups, rows per thread
     constexpr int PITCH = B + 16;                                        // bytes; rows 16-byte aligned
     __shared__ float s_max[GROUPS][TC];
     __shared__ __align__(16) unsigned char tile[TC * PITCH];
-    const int j = blockIdx.x / col_tiles, c0 = (blockIdx.x % col_tiles) * TC;
+    const int j = tile_index / col_tiles, c0 = (tile_index % col_tiles) * TC;
     const int c = threadIdx.x % TC, g = threadIdx.x / TC;
     const int r0 = j * B + g * RPT;
     const bool col_ok = c0 + c < C;
@@ -428,6 +443,13 @@ __global__ void __launch_bounds__(kThreads) quantize_colwise_cols_kernel(
             for (int b = 0; b < 16 && b < left; ++b) dst[b] = (int8_t)src[b];
         }
     }
+}
+
+template <typename T, int B>
+__global__ void __launch_bounds__(kThreads) quantize_colwise_cols_kernel(
+    const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int R, int C, int col_tiles) {
+    after_predecessor();
+    quantize_colwise_tile<T, B>((int)blockIdx.x, x, ldx, q, ldq, s, R, C, col_tiles);
 }
 
 // Column-wise quantize for the other block sizes, rows of any alignment.  A CTA takes
@@ -549,15 +571,6 @@ __global__ void __launch_bounds__(kThreads) dequantize_rowwise_vec_kernel(
     }
 }
 
-template <typename TO>
-__device__ __forceinline__ TO from_f32(float v);
-template <>
-__device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-template <>
-__device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
-template <>
-__device__ __forceinline__ float from_f32<float>(float v) { return v; }
-
 // Dequantize to rows that are not 32-byte aligned (K not a multiple of 16), or any block size and alignment.  A warp takes a
 // run of 256 columns of a row; a lane's four stores are aligned 4-byte words (two 16-bit results, or one fp32), 32 lanes
 // next to each other, whatever the row's alignment: for a 16-bit row that begins between two words, the words hold elements
@@ -605,6 +618,66 @@ __global__ void __launch_bounds__(kThreads) dequantize_rowwise_words_kernel(
                 if (k + e >= 0 && k + e < K) row[k + e] = v[e];
         }
     }
+}
+
+// Several small jobs of one pass in one launch: row-wise and column-wise quantizations, column sums, copies of int8 rows to aligned
+// ones.  For matrices of a few hundred KB each of them is a launch (2 to 3 us of host time and as much latency on the device) around
+// well under a microsecond of work.  A CTA finds its job by its index; the tiles are those of the single-purpose kernels.
+enum JobKind { kJobRow = 0, kJobRowShift, kJobCol, kJobSum, kJobCopy };
+struct Job {
+    const void* x;
+    void* q;            // int8 result; kJobSum: the sums
+    float* s;
+    int64_t ldx, ldq;
+    int M, K, nb, tiles, kind, end;       // `end`: first CTA of the next job
+};
+constexpr int kMostJobs = 8;
+struct Jobs {
+    Job job[kMostJobs];
+};
+
+// Sums of 32 columns over all rows by eight groups of rows, added in the groups' order (fp32).
+template <typename T>
+__device__ __forceinline__ void column_sum_tile(int tile, const T* __restrict__ x, int64_t ldx, T* __restrict__ out, int R, int C) {
+    __shared__ float part[8][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, c = tile * 32 + lane;
+    const int per = (R + 7) / 8, r1 = (g + 1) * per < R ? (g + 1) * per : R;
+    float acc = 0.0f;
+    if (c < C) {
+        int r = g * per;
+        for (; r + 8 <= r1; r += 8) {
+            float f[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) f[u] = to_f32<T>(x[(int64_t)(r + u) * ldx + c]);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) acc += f[u];
+        }
+        for (; r < r1; ++r) acc += to_f32<T>(x[(int64_t)r * ldx + c]);
+    }
+    part[g][lane] = acc;
+    __syncthreads();
+    if (g == 0 && c < C) {
+        float v = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v += part[k][lane];
+        out[c] = from_f32<T>(v);
+    }
+}
+
+template <typename T, int B>
+__global__ void __launch_bounds__(kThreads) quantize_jobs_kernel(const __grid_constant__ Jobs jobs) {
+    after_predecessor();
+    int k = 0;
+    while ((int)blockIdx.x >= jobs.job[k].end) ++k;
+    const Job& j = jobs.job[k];
+    const int tile = (int)blockIdx.x - (k ? jobs.job[k - 1].end : 0);
+    const T* x = static_cast<const T*>(j.x);
+    int8_t* q = static_cast<int8_t*>(j.q);
+    if (j.kind == kJobRow) quantize_rowwise_tile<T, B, false, 1>(tile, x, j.ldx, q, j.ldq, j.s, j.M, j.K, j.nb, j.tiles);
+    else if (j.kind == kJobRowShift) quantize_rowwise_tile<T, B, true, 1>(tile, x, j.ldx, q, j.ldq, j.s, j.M, j.K, j.nb, j.tiles);
+    else if (j.kind == kJobCol) quantize_colwise_tile<T, B>(tile, x, j.ldx, q, j.ldq, j.s, j.M, j.K, j.tiles);
+    else if (j.kind == kJobSum) column_sum_tile<T>(tile, x, j.ldx, static_cast<T*>(j.q), j.M, j.K);
+    else copy_rows_piece((int64_t)tile * kThreads + threadIdx.x, static_cast<const int8_t*>(j.x), j.ldx, q, j.ldq, (int64_t)j.M * j.tiles, j.tiles, j.K);
 }
 
 // From here on a tensor and what is computed from it do not both stay in L2 (126 MB).
@@ -751,6 +824,79 @@ int launch_dequantize_rowwise(const int8_t* q, int64_t ldq, const float* s, void
         case BI8_F32: return dequantize_t(q, ldq, s, static_cast<float*>(out), M, K, block, st);
     }
     return fail(BI8_ERR_DTYPE, "dequantize: unknown dtype code %d", dt);
+}
+
+// The most values that a launch of several jobs quantizes (row-wise and column-wise counted each), and the most int8 values that it copies
+// beside them: up to there it takes no longer on the device than the single-purpose kernels one after another (a training step's
+// quantizers at 2048 x 768 x 768, 4.3 M in the forward pass with separate kernels 16.9 us, at 1024 x 512 x 512 15.6 -> 8.8) and is two
+// or three launches of 2 to 3 us of host time less: 300 x 256 x 384 in fp32 99 -> 82 us a step, 11 launches -> 5, 512 x 1024 x
+// 1024 bf16 91 -> 81; a layer of 333 x 1000 x 777 with unaligned weights 13.6 -> 12.3 us.  Column sums of more than kJobSumRows
+// rows want more CTAs than a job gives them.
+namespace {
+constexpr int64_t kJobValues = 4 << 20, kJobCopied = 1 << 20;
+constexpr int kJobSumRows = 512;
+
+// One launch's worth of jobs, or a negative number where some task needs a kernel of its own.
+int collect_jobs(const bi8_quantize_task* t, int n, int block, Jobs* jobs) {
+    if (block != 32 && block != 64 && block != 128) return -1;
+    int count = 0, dt = -1;
+    int64_t values = 0, ctas = 0;
+    for (int i = 0; i < n; ++i) {
+        const bi8_quantize_task& a = t[i];
+        if (a.rows <= 0 || a.cols <= 0 || a.rows >= (1 << 30) || a.cols >= (1 << 30)) return -1;
+        auto add = [&](int kind, const void* x, void* q, int64_t ldq, float* s, int nb, int tiles, int64_t blocks) {
+            if (count == kMostJobs) return false;
+            ctas += blocks;
+            if (ctas >= (1ll << 30)) return false;
+            if (jobs) jobs->job[count] = Job{x, q, s, a.ldx, ldq, (int)a.rows, (int)a.cols, nb, tiles, kind, (int)ctas};
+            ++count;
+            return true;
+        };
+        if (a.x_dtype == BI8_I8) {
+            const int64_t per_row = (a.cols + 15) / 16;
+            if (a.rows * a.cols > kJobCopied || a.q_col || a.sum || !add(kJobCopy, a.x, a.q_row, a.ldq_row, nullptr, 0, (int)per_row, (a.rows * per_row + kThreads - 1) / kThreads)) return -1;
+            continue;
+        }
+        if (dt >= 0 && dt != a.x_dtype) return -1;
+        dt = a.x_dtype;
+        values += a.rows * a.cols * ((a.q_row ? 1 : 0) + (a.q_col ? 1 : 0));
+        const int esz = dt == BI8_F32 ? 4 : 2;
+        if (a.q_row) {
+            if (a.ldq_row % 8 != 0 || !aligned(a.q_row, 8)) return -1;
+            const int64_t ctiles = (a.cols + 255) / 256;
+            const bool straight = a.cols % 8 == 0 && aligned(a.x, 16) && a.ldx * esz % 16 == 0;
+            if (!add(straight ? kJobRow : kJobRowShift, a.x, a.q_row, a.ldq_row, a.s_row, (int)((a.cols + block - 1) / block), (int)ctiles, (a.rows + 7) / 8 * ctiles)) return -1;
+        }
+        if (a.q_col) {
+            const int64_t ctiles = (a.cols + 63) / 64;
+            if (!add(kJobCol, a.x, a.q_col, a.ldq_col, a.s_col, 0, (int)ctiles, (a.rows + block - 1) / block * ctiles)) return -1;
+        }
+        if (a.sum) {
+            if (a.rows > kJobSumRows || !add(kJobSum, a.x, a.sum, 0, nullptr, 0, 0, (a.cols + 31) / 32)) return -1;
+        }
+    }
+    return dt >= 0 && values <= kJobValues ? count : -1;
+}
+
+template <typename T>
+int launch_jobs(const Jobs& jobs, int count, int block, cudaStream_t st) {
+    const unsigned ctas = (unsigned)jobs.job[count - 1].end;
+    return block == 32   ? launch_chained(quantize_jobs_kernel<T, 32>, ctas, kThreads, 0, st, jobs)
+           : block == 64 ? launch_chained(quantize_jobs_kernel<T, 64>, ctas, kThreads, 0, st, jobs)
+                         : launch_chained(quantize_jobs_kernel<T, 128>, ctas, kThreads, 0, st, jobs);
+}
+}  // namespace
+
+bool quantize_jobs_fit(const bi8_quantize_task* tasks, int n, int block) { return collect_jobs(tasks, n, block, nullptr) > 1; }
+
+int launch_quantize_jobs(const bi8_quantize_task* tasks, int n, int block, cudaStream_t st) {
+    Jobs jobs{};
+    const int count = collect_jobs(tasks, n, block, &jobs);
+    if (count < 1) return fail(BI8_ERR_LIMIT, "quantize_many: the tasks do not fit one launch");
+    int dt = BI8_I8;
+    for (int i = 0; i < n; ++i)
+        if (tasks[i].x_dtype != BI8_I8) dt = tasks[i].x_dtype;
+    return dt == BI8_BF16 ? launch_jobs<__nv_bfloat16>(jobs, count, block, st) : dt == BI8_F16 ? launch_jobs<__half>(jobs, count, block, st) : launch_jobs<float>(jobs, count, block, st);
 }
 
 }  // namespace bi8

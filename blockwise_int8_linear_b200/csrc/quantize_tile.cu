@@ -655,7 +655,7 @@ int tile_dispatch(const void* x, int64_t ldx, int8_t* q_col, int64_t ldqc, float
                   int64_t C, int block, cudaStream_t st) {
     CUtensorMap tx, tqc, tqr;
     int dev = 0;
-    BI8_CUDA_TRY(cudaGetDevice(&dev));
+    BI8_CUDA_TRY(current_device(&dev));
     int rc = cached_q_map(&tqc, dev, q_col, C, R, ldqc, false);
     if (rc != BI8_OK) return rc;
     tx = tqr = tqc;

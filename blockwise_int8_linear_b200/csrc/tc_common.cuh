@@ -200,7 +200,7 @@ struct DeviceInfo {
 inline DeviceInfo device_info() {
     static DeviceInfo cache[64];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return DeviceInfo{};
+    if (current_device(&dev) != cudaSuccess || dev < 0 || dev >= 64) return DeviceInfo{};
     if (!cache[dev].ok) {
         int sms = 0, major = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return DeviceInfo{};

@@ -164,8 +164,9 @@ Tensor empty_q(const Tensor& like, int64_t rows, int64_t cols, bool pitched) {
 // Copy with a 16-byte aligned row pitch of an int8 operand that has none; the bytes between K and the pitch are never read.  What
 // is copied is the matrix that `m` describes, at its address and with its pitch: the owner itself may be that matrix or
 // its transpose, which its shape does not tell where both have the same.
+bool on_boundaries(const Mat& m) { return m.ld % 16 == 0 && reinterpret_cast<uintptr_t>(m.ptr) % 16 == 0; }
 Mat repitch(const Mat& m, const OnDevice& on) {
-    if (m.ld % 16 == 0 && reinterpret_cast<uintptr_t>(m.ptr) % 16 == 0) return m;
+    if (on_boundaries(m)) return m;
     Mat out = m;
     out.ld = pitch16(m.cols);
     out.owner = empty_on(m.owner, {m.rows, out.ld}, at::kChar);
@@ -428,18 +429,47 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
     Carve carve;
     carve.take((int64_t)ws_bytes);
     const int64_t xq_at = carve.take(m * pitch16(k)), sx_at = carve.take(nb * m * 4);
+    // Weights whose rows are not 16-byte aligned (of a layer, a checkpoint's dense copy) are copied to rows that are where the GEMM is
+    // long enough to gain from it.
+    const bool copy_w = k % 16 != 0 && worth_repitch(m, n, k) && !on_boundaries(bt);
+    const int64_t w_at = copy_w ? carve.take(n * pitch16(k)) : 0;
     const Tensor ws = scratch(x_in, carve.bytes);
     char* ws_ptr = ws.defined() ? static_cast<char*>(ws.data_ptr()) : nullptr;
     int8_t* xq = reinterpret_cast<int8_t*>(ws_ptr + xq_at);
     float* sx = reinterpret_cast<float*>(ws_ptr + sx_at);
     void* gemm_ws = ws_bytes ? ws_ptr : nullptr;
     if (k % 16 != 0) {
-        // Rows that are not 16-byte aligned: the activations are quantized into rows that are, weights that have none (of
-        // a layer, a checkpoint's dense copy) are re-pitched where the GEMM is long enough to gain from it.
-        if (worth_repitch(m, n, k)) bt = repitch(bt, on);
-        check(bi8_quantize_rowwise_pre_pitched(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps, xq, pitch16(k), sx, m, k,
-                                               (int)block, on.raw()),
-              "bi8_quantize_rowwise_pre");
+        // rows that are not 16-byte aligned: the activations are quantized into rows that are, with the copy in one launch if they are few
+        // (one after another it is the copy first: the GEMM starts early behind the short quantizer)
+        bi8_quantize_task tasks[2] = {};
+        bi8_quantize_task &tw = tasks[0], &tx = tasks[1];
+        if (copy_w) {
+            tw.x = bt.ptr;
+            tw.x_dtype = BI8_I8;
+            tw.ldx = bt.ld;
+            tw.rows = n;
+            tw.cols = k;
+            tw.q_row = reinterpret_cast<int8_t*>(ws_ptr + w_at);
+            tw.ldq_row = pitch16(k);
+            bt.ptr = tw.q_row;
+            bt.ld = tw.ldq_row;
+        }
+        if (op == BI8_PRE_NONE) {
+            tx.x = pre.x.ptr;
+            tx.x_dtype = x_code;
+            tx.ldx = pre.x.ld;
+            tx.rows = m;
+            tx.cols = k;
+            tx.q_row = xq;
+            tx.ldq_row = pitch16(k);
+            tx.s_row = sx;
+            check(bi8_quantize_many(copy_w ? tasks : &tx, copy_w ? 2 : 1, (int)block, on.raw()), "bi8_quantize_many");
+        } else {
+            if (copy_w) check(bi8_quantize_many(&tw, 1, (int)block, on.raw()), "bi8_quantize_many");
+            check(bi8_quantize_rowwise_pre_pitched(op, pre.x.ptr, pre.x2.ptr, x_code, pre.x.ld, pre.weight_ptr(), (float)eps, xq, pitch16(k), sx, m, k,
+                                                   (int)block, on.raw()),
+                  "bi8_quantize_rowwise_pre");
+        }
         check(bi8_gemm_dequant_residual(xq, pitch16(k), static_cast<const int8_t*>(bt.ptr), bt.ld, sx, sw.const_data_ptr<float>(), bias.ptr, bias.code,
                                         res_ptr, ldr, target.data_ptr(), ldc, dtype_code(out_type), m, n, k, (int)block, gemm_ws, ws_bytes,
                                         flags & ~BI8_GEMM_QUANT_IN_KERNEL, on.raw()),
@@ -502,15 +532,35 @@ QRef ref_of(const Quantized& r) {
             r.ld()};
 }
 
-void rowwise_into(const Mat& m, int code, int64_t block, const QRef& r, void* stream) {
-    check(bi8_quantize_rowwise_pitched(m.ptr, code, m.ld, r.q, r.ld, r.s, m.rows, m.cols, (int)block, stream), "bi8_quantize_rowwise");
-}
-void colwise_into(const Mat& m, int code, int64_t block, const QRef& r, void* stream) {
-    check(bi8_quantize_colwise_pitched(m.ptr, code, m.ld, r.q, r.ld, r.s, m.rows, m.cols, (int)block, stream), "bi8_quantize_colwise");
-}
-void dual_into(const Mat& m, int code, int64_t block, const QRef& row, const QRef& col, void* stream) {
-    check(bi8_quantize_dual_pitched(m.ptr, code, m.ld, row.q, row.ld, row.s, col.q, col.ld, col.s, m.rows, m.cols, (int)block, stream), "bi8_quantize_dual");
-}
+// The quantizations of a pass, which share a launch where they are small.
+struct Tasks {
+    bi8_quantize_task list[4];
+    int n = 0;
+    // x row-wise and / or column-wise
+    void add(const Mat& m, int code, const QRef* row, const QRef* col) {
+        bi8_quantize_task t{};
+        t.x = m.ptr;
+        t.x_dtype = code;
+        t.ldx = m.ld;
+        t.rows = m.rows;
+        t.cols = m.cols;
+        if (row) {
+            t.q_row = row->q;
+            t.ldq_row = row->ld;
+            t.s_row = row->s;
+        }
+        if (col) {
+            t.q_col = col->q;
+            t.ldq_col = col->ld;
+            t.s_col = col->s;
+        }
+        list[n++] = t;
+    }
+    bool fits(int64_t block) const { return n > 0 && bi8_quantize_many_fits(list, n, (int)block) != 0; }
+    void run(int64_t block, void* stream) const {
+        if (n > 0) check(bi8_quantize_many(list, n, (int)block, stream), "bi8_quantize_many");
+    }
+};
 // out = a b^T (+ bias); `ws` of at least bi8_gemm_workspace_used
 void gemm_into(const QRef& a, const QRef& b, const Bias* bias, int64_t block, const Tensor& out, void* ws, size_t ws_bytes, void* stream) {
     check(bi8_gemm_dequant(a.q, a.ld, b.q, b.ld, a.s, b.s, bias ? bias->ptr : nullptr, bias ? bias->code : 0, out.data_ptr(), b.rows,
@@ -619,37 +669,56 @@ variable_list LinearBackward::apply(variable_list&& grads) {
         void* const ws = static_cast<char*>(base) + ws_at;
         void* const st = on.raw();
 
-        const bool dual = need_x && need_w && fuse_dual;     // G is needed in both blockings: one read
-        if (dual) dual_into(g, g_code, b, g_row.in(base), g_col.in(base), st);
-        else if (need_x) rowwise_into(g, g_code, b, g_row.in(base), st);
+        // All operands first: G (in both blockings with one read, where the layer fuses them), the weight along N and the tokens of x.
+        const QRef gr = need_x ? g_row.in(base) : QRef{}, gc = need_w ? g_col.in(base) : QRef{};
+        Tasks tasks;
+        if (need_x && need_w && fuse_dual) {
+            tasks.add(g, g_code, &gr, &gc);
+        } else {
+            if (need_x) tasks.add(g, g_code, &gr, nullptr);
+            if (need_w) tasks.add(g, g_code, nullptr, &gc);
+        }
+        QRef wt, xt;
         if (need_x) {
-            // contraction over N, both operands blocked along N (block_linear.py:92-95).  A cached blocking is still valid:
-            // unpacking the weight raised if it was modified since the forward pass.
-            QRef wt;
-            if (cached.q.defined()) {
-                wt = ref_of(cached);
-            } else if (cache) {
-                fresh = Quantized{empty_q(w, k, n, true), empty_on(w, {ceil_div(n, b), k}, at::kFloat)};
-                wt = ref_of(fresh);
-                colwise_into(wm, w_code, b, wt, st);
-                cache_put(cache, "col", fresh);
-            } else {
-                wt = w_col.in(base);
-                colwise_into(wm, w_code, b, wt, st);
+            // A cached blocking is still valid: unpacking the weight raised if it was modified since the forward pass.
+            if (cached.q.defined()) wt = ref_of(cached);
+            else {
+                if (cache) {
+                    fresh = Quantized{empty_q(w, k, n, true), empty_on(w, {ceil_div(n, b), k}, at::kFloat)};
+                    wt = ref_of(fresh);
+                } else {
+                    wt = w_col.in(base);
+                }
+                tasks.add(wm, w_code, nullptr, &wt);
             }
+        }
+        if (need_w) {
+            xt = x_col.in(x_quantized ? saved_x.data_ptr() : base);
+            if (!x_quantized) tasks.add(xm, dtype_code(saved_x.scalar_type()), nullptr, &xt);
+        }
+        // small passes: the bias gradient rides in the same launch
+        bool summed = false;
+        if (need_b) {
+            out[2] = empty_on(grads[0], {n}, grads[0].scalar_type());
+            if (tasks.n > 0 && tasks.list[0].x == g.ptr) {
+                tasks.list[0].sum = out[2].data_ptr();
+                summed = tasks.fits(b);
+                if (!summed) tasks.list[0].sum = nullptr;
+            }
+        }
+        tasks.run(b, st);
+        if (fresh.q.defined()) cache_put(cache, "col", fresh);
+        if (need_x) {
+            // contraction over N, both operands blocked along N (block_linear.py:92-95)
             out[0] = empty_on(grads[0], x_sizes, type);
-            gemm_into(g_row.in(base), wt, nullptr, b, out[0], ws, ws_x, st);
+            gemm_into(gr, wt, nullptr, b, out[0], ws, ws_x, st);
         }
         if (need_w) {
             // contraction over the tokens, both operands blocked along M (block_linear.py:100-104)
-            const QRef xt = x_col.in(x_quantized ? saved_x.data_ptr() : base);
-            if (!x_quantized) colwise_into(xm, dtype_code(saved_x.scalar_type()), b, xt, st);
-            if (!dual) colwise_into(g, g_code, b, g_col.in(base), st);
             out[1] = empty_on(grads[0], {n, k}, type);
-            gemm_into(g_col.in(base), xt, nullptr, b, out[1], ws, ws_w, st);
+            gemm_into(gc, xt, nullptr, b, out[1], ws, ws_w, st);
         }
-        if (need_b) {
-            out[2] = empty_on(grads[0], {n}, grads[0].scalar_type());
+        if (need_b && !summed) {
             check(bi8_column_sum(g.ptr, g_code, g.ld, out[2].data_ptr(), m, n, ws_b ? ws : nullptr, ws_b, st), "bi8_column_sum");
         }
     } catch (const PyFail& e) {
@@ -693,13 +762,15 @@ Tensor train_linear(const Tensor& x_in, const Tensor& w, const Tensor& bias_in, 
         void* const base = mem.data_ptr();
         void* const st = on.raw();
         const QRef xq = x_row.in(base);
+        Tasks tasks;
         if (keep) {
             const Tensor saved = as_bytes(x_in, kept.bytes);
-            dual_into(x, x_code, block, xq, x_col.in(saved.data_ptr()), st);
+            const QRef xt = x_col.in(saved.data_ptr());
+            tasks.add(x, x_code, &xq, &xt);
             node->x = SavedVariable(saved, false);
             node->x_quantized = true;
         } else {
-            rowwise_into(x, x_code, block, xq, st);
+            tasks.add(x, x_code, &xq, nullptr);
         }
         QRef wq;
         if (cached.q.defined()) {
@@ -707,12 +778,13 @@ Tensor train_linear(const Tensor& x_in, const Tensor& w, const Tensor& bias_in, 
         } else if (cache) {
             fresh = Quantized{empty_q(w, n, k, true), empty_on(w, {ceil_div(k, block), n}, at::kFloat)};
             wq = ref_of(fresh);
-            rowwise_into(wm, w_code, block, wq, st);
-            cache_put(cache, "row", fresh);
+            tasks.add(wm, w_code, &wq, nullptr);
         } else {
             wq = w_row.in(base);
-            rowwise_into(wm, w_code, block, wq, st);
+            tasks.add(wm, w_code, &wq, nullptr);
         }
+        tasks.run(block, st);
+        if (fresh.q.defined()) cache_put(cache, "row", fresh);
         const Bias bias(bias_in, n);
         c10::SmallVector<int64_t, 6> shape(x_in.sizes().begin(), x_in.sizes().end());
         shape.back() = n;

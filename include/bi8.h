@@ -51,6 +51,7 @@ extern "C" {
 #define BI8_BF16 0
 #define BI8_F32 1
 #define BI8_F16 2
+#define BI8_I8 3                 /* bi8_quantize_task only: rows of int8 values to be copied */
 
 /* flags for bi8_gemm_dequant */
 #define BI8_GEMM_DEFAULT 0
@@ -152,6 +153,26 @@ BI8_API int bi8_quantize_rowwise_pre_pitched(int op, const void* x, const void* 
                                              void* stream);
 BI8_API int bi8_dequantize_rowwise_pitched(const int8_t* q, int64_t ldq, const float* s, void* out, int out_dtype,
                                            int64_t M, int64_t K, int block, void* stream);
+
+/* Several quantizations of one pass.  A task quantizes x [rows, cols] row-wise (q_row not NULL), column-wise (q_col), or both, sums its
+ * columns into `sum` (cols values of x_dtype, accumulated in fp32 in a fixed order), or (x_dtype BI8_I8) copies int8 rows to
+ * q_row as bi8_copy_rows does.  The quantized results are those of the single-purpose functions.  Small tasks share one launch;
+ * bi8_quantize_many_fits says whether these do (1), else they run one after another and `sum` must be NULL. */
+typedef struct {
+    const void* x;
+    int64_t ldx;
+    int64_t rows, cols;
+    int8_t* q_row;
+    int64_t ldq_row;
+    float* s_row;
+    int8_t* q_col;
+    int64_t ldq_col;
+    float* s_col;
+    void* sum;
+    int x_dtype;
+} bi8_quantize_task;
+BI8_API int bi8_quantize_many_fits(const bi8_quantize_task* tasks, int n, int block);
+BI8_API int bi8_quantize_many(const bi8_quantize_task* tasks, int n, int block, void* stream);
 
 /* Copies int8 rows [rows, cols] of any alignment (pitch lds bytes) to rows that begin on 16-byte boundaries (dst 16-byte aligned,
  * pitch ldd a multiple of 16), as the tensor-core GEMM wants its operands.  The bytes between a row's end and the next
