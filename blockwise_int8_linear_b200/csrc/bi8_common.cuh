@@ -100,6 +100,21 @@ __device__ __forceinline__ void after_predecessor() {
 }
 #endif
 
+// Division by a number that the host knows, as a product and a shift: exact for dividends below 2^31.  (A division by a variable is 20
+// instructions in 32 bits and 70 to 100 in 64.)
+struct FastDiv {
+    unsigned mul = 1, d = 1;
+    int shift = 0;
+    FastDiv() = default;
+    explicit FastDiv(int64_t divisor) : d((unsigned)divisor) {
+        while ((1ll << shift) < divisor) ++shift;
+        mul = (unsigned)((((1ull << shift) - d) << 32) / d + 1);
+    }
+#if defined(__CUDACC__)
+    __device__ __forceinline__ unsigned div(unsigned t) const { return (__umulhi(t, mul) + t) >> shift; }
+#endif
+};
+
 // ---- launchers implemented in the other translation units -------------------------------------
 // (ldq: row pitch of the int8 result in bytes)
 int launch_quantize_rowwise(const void* x, int dt, int64_t ldx, int8_t* q, int64_t ldq, float* s, int64_t M, int64_t K,

@@ -112,8 +112,7 @@ struct TcParams {
     int out_dtype, bias_dtype;
     int vec_store;      // C base and row pitch allow 16-byte stores
     int store;          // how undivided tiles leave (StoreMode)
-    unsigned tm_mul;    // division by tiles_m: (umulhi(t, tm_mul) + t) >> tm_shift
-    int tm_shift;
+    FastDiv by_tiles_m;
     int tma_scales;     // bit 0: sA is described by the tensor map tmSA, bit 1: sB by tmSB
     int ksplit;         // > 1: the K stages are divided over ksplit work items per tile (split-K)
     int stages_per_split;
@@ -192,9 +191,8 @@ __device__ __forceinline__ void item_range(int item, const TcParams& p, int nks,
 
 template <int BN>
 __device__ __forceinline__ void tile_coords(int tile, const TcParams& p, int& m0, int& n0) {
-    // (a division by a product with host-made constants, exact below 2^31)
     // consecutive tiles (CTAs that run together) share a column panel of Bt and sweep the rows of A
-    const int tn = (int)((__umulhi((unsigned)tile, p.tm_mul) + (unsigned)tile) >> p.tm_shift);
+    const int tn = (int)p.by_tiles_m.div((unsigned)tile);
     m0 = (tile - tn * p.tiles_m) * kBM;
     n0 = tn * BN;
 }
@@ -1411,8 +1409,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     const int bn = tc_bn();
     rc = cached_operand_map(&tm.b, dev, g.Bt, g.N, g.K, g.ldb, bn);
     if (rc != BI8_OK) return rc;
-    TcParams p;
-    std::memset(&p, 0, sizeof(p));
+    TcParams p{};
     const bool partials = g.partials != nullptr, seed = (g.flags & BI8_GEMM_NO_SEED) == 0;
     // a scale tensor goes through TMA when a tensor map can describe it: 16-byte aligned base and row length
     const bool tma_sa = !partials && aligned(g.sA, 16) && g.M % 4 == 0, tma_sb = !partials && aligned(g.sB, 16) && g.N % 4 == 0;
@@ -1478,8 +1475,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
         p.store = kRows;
     }
     p.ws = static_cast<float*>(g.workspace);
-    while ((1ll << p.tm_shift) < p.tiles_m) ++p.tm_shift;
-    p.tm_mul = (unsigned)((((1ull << p.tm_shift) - (unsigned)p.tiles_m) << 32) / (unsigned)p.tiles_m + 1);
+    p.by_tiles_m = FastDiv(p.tiles_m);
     const int64_t items = tiles * pl.ksplit;
     const int grid = (int)(items < di.sms ? items : di.sms);
     switch (g.block) {

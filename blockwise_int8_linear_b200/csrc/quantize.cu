@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_vec_kernel(
 template <typename T, int B, bool FAR>
 __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
     const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ q, int64_t ldq, float* __restrict__ s, int M, int K, int nb,
-    int col_units, int64_t total_units) {
+    FastDiv col_units, int64_t total_units) {
     after_predecessor();
     constexpr int LPB = B / 16;             // lanes sharing one block
     const int lane = threadIdx.x & 31;
@@ -230,8 +230,9 @@ __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
         f2_bits(f2_fma(z, cone, cmagic), b0, b1);
     };
 
+    auto row_group = [&](int64_t u) { return u < (1ll << 31) ? (int)col_units.div((unsigned)u) : (int)(u / col_units.d); };
     auto load_unit = [&](int64_t u, uint32_t (&buf)[4][8]) {
-        const int rg = (int)(u / col_units), ct = (int)(u % col_units);
+        const int rg = row_group(u), ct = (int)(u - (int64_t)rg * col_units.d);
         const int col = ct * 512 + lane * 16;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
         }
     };
     auto process_unit = [&](int64_t u, const uint32_t (&buf)[4][8]) {
-        const int rg = (int)(u / col_units), ct = (int)(u % col_units);
+        const int rg = row_group(u), ct = (int)(u - (int64_t)rg * col_units.d);
         const int col = ct * 512 + lane * 16;
         float sc[4];
 #pragma unroll
@@ -701,7 +702,7 @@ int quantize_rowwise_t(const T* x, int64_t ldx, int8_t* q, int64_t ldq, float* s
             int64_t ctas = (total + kThreads / 32 - 1) / (kThreads / 32);   // one unit per warp at least
             if (ctas > 2ll * di.sms) ctas = 2ll * di.sms;                   // two resident CTAs per SM, persistent beyond that
             auto launch = [&](auto kernel) {
-                return launch_chained(kernel, (unsigned)ctas, kThreads, 0, st, x, ldx, q, ldq, s, (int)M, (int)K, (int)nb, col_units, total);
+                return launch_chained(kernel, (unsigned)ctas, kThreads, 0, st, x, ldx, q, ldq, s, (int)M, (int)K, (int)nb, FastDiv(col_units), total);
             };
             const bool far = M * K * (int64_t)sizeof(T) > kFarBytes;
 #define BI8_QSTREAM(BB) \

@@ -220,14 +220,12 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quan
 template <int QB, int DT>
 __global__ void __launch_bounds__(kPreThreads) silu_mul_quantize_kernel(const void* __restrict__ gate, const void* __restrict__ up,
                                                                         int64_t ldx, int8_t* __restrict__ q, int64_t ldq,
-                                                                        float* __restrict__ sx, int M, int K, int nb, int vec_in,
+                                                                        float* __restrict__ sx, int M, int K, FastDiv upr, int vec_in,
                                                                         int vec_out) {
     after_predecessor();
-    constexpr int LPB = QB / 8;
     constexpr int dt = DT;
-    const int upr = nb * LPB;
     const int64_t u = (int64_t)blockIdx.x * kPreThreads + threadIdx.x;
-    const int m = (int)(u / upr), k = (int)(u % upr) * 8;
+    const int m = u < (1ll << 31) ? (int)upr.div((unsigned)u) : (int)(u / upr.d), k = (int)(u - (int64_t)m * upr.d) * 8;
     const bool valid = m < M && k < K;
     float y[8];
 #pragma unroll
@@ -304,11 +302,12 @@ int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t l
         if (!x2) return fail(BI8_ERR_NULL, "quantize_pre: the gated activation needs its second operand");
         const int64_t units = M * nb * (block / 8);
         const unsigned grid = (unsigned)((units + kPreThreads - 1) / kPreThreads);
+        const FastDiv upr((int64_t)nb * (block / 8));
 #define BI8_PRE_SILU(QB)                                                                                                             \
     do {                                                                                                                             \
-        if (dt == BI8_BF16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_BF16>, grid, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
-        else if (dt == BI8_F16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_F16>, grid, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
-        else return launch_chained(silu_mul_quantize_kernel<QB, BI8_F32>, grid, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
+        if (dt == BI8_BF16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_BF16>, grid, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, upr, vec_in, vec_out); \
+        else if (dt == BI8_F16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_F16>, grid, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, upr, vec_in, vec_out); \
+        else return launch_chained(silu_mul_quantize_kernel<QB, BI8_F32>, grid, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, upr, vec_in, vec_out); \
     } while (0)
         switch (block) {
             case 32: BI8_PRE_SILU(32); break;
