@@ -23,7 +23,7 @@ _DTYPE_CODE = {torch.bfloat16: BI8_BF16, torch.float32: BI8_F32, torch.float16: 
 
 EXPORTS = [
     "bi8_version", "bi8_last_error_string", "bi8_device_status", "bi8_quantize_rowwise", "bi8_quantize_colwise", "bi8_quantize_dual", "bi8_peer_allreduce", "bi8_peer_allreduce_buffer_bytes", "bi8_row_parallel_linear",
-    "bi8_dequantize_rowwise", "bi8_gemm_dequant", "bi8_gemm_workspace_bytes", "bi8_gemm_workspace_used", "bi8_quantize_many", "bi8_quantize_many_fits", "bi8_gemm_block_partials",
+    "bi8_dequantize_rowwise", "bi8_gemm_dequant", "bi8_gemm_workspace_bytes", "bi8_gemm_workspace_used", "bi8_quantize_many", "bi8_quantize_many_fits", "bi8_quantize_dual_sum", "bi8_quantize_dual_sum_workspace_bytes", "bi8_gemm_block_partials",
     "bi8_gemm_dequant_fused_quant", "bi8_mma_peak_probe", "bi8_gemm_dequant_static", "bi8_gemm_static_scratch_bytes",
     "bi8_gemm_wait_selftest", "bi8_stream_capture_id", "bi8_quantize_rowwise_pre", "bi8_gemm_dequant_fused_pre",
     "bi8_row_parallel_linear_pre", "bi8_peer_allreduce_large", "bi8_peer_allreduce_large_buffer_bytes",
@@ -90,6 +90,9 @@ def lib() -> ctypes.CDLL:
         L.bi8_gemm_workspace_bytes.restype = sz
         L.bi8_gemm_workspace_used.argtypes = [i64, i64, i64, i32]
         L.bi8_gemm_workspace_used.restype = sz
+        L.bi8_quantize_dual_sum.argtypes = [vp, i32, i64, vp, i64, vp, vp, i64, vp, vp, i64, i64, i32, vp, sz, vp]
+        L.bi8_quantize_dual_sum_workspace_bytes.argtypes = [i32, i64, i64, i32]
+        L.bi8_quantize_dual_sum_workspace_bytes.restype = sz
         L.bi8_quantize_many.argtypes = [vp, i32, i32, vp]
         L.bi8_quantize_many_fits.argtypes = [vp, i32, i32]
         L.bi8_gemm_block_partials.argtypes = [vp, i64, vp, i64, vp, i64, i64, i64, i32, i32, vp]
@@ -103,7 +106,7 @@ def lib() -> ctypes.CDLL:
         L.bi8_mma_peak_probe.argtypes = [i32, c.POINTER(c.c_float), c.POINTER(i32)]
         for name in EXPORTS:
             fn = getattr(L, name)
-            if name not in ("bi8_last_error_string", "bi8_gemm_workspace_bytes", "bi8_gemm_workspace_used", "bi8_gemm_static_scratch_bytes",
+            if name not in ("bi8_last_error_string", "bi8_gemm_workspace_bytes", "bi8_gemm_workspace_used", "bi8_quantize_dual_sum_workspace_bytes", "bi8_gemm_static_scratch_bytes",
                             "bi8_peer_allreduce_buffer_bytes", "bi8_peer_allreduce_large_buffer_bytes", "bi8_column_sum_workspace_bytes",
                             "bi8_peer_allreduce_large_partial_offset", "bi8_peer_allreduce_large_out_offset"):
                 fn.restype = i32

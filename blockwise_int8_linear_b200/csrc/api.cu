@@ -232,6 +232,29 @@ int bi8_quantize_dual_pitched(const void* x, int x_dtype, int64_t ldx, int8_t* q
     return launch_quantize_colwise(x, x_dtype, ldx, q_col, ldq_col, s_col, R, C, block, st);
 }
 
+size_t bi8_quantize_dual_sum_workspace_bytes(int x_dtype, int64_t R, int64_t C, int block) {
+    if (x_dtype == BI8_F32 || !dtype_ok(x_dtype) || R < 0 || C < 0 || R >= (1ll << 31) - 256 || C >= (1ll << 31) - 65536) return 0;
+    if (block != 32 && block != 64 && block != 128) return 0;
+    return (size_t)((R + kTileSumRows - 1) / kTileSumRows) * (size_t)C * 4;
+}
+
+int bi8_quantize_dual_sum(const void* x, int x_dtype, int64_t ldx, int8_t* q_row, int64_t ldq_row, float* s_row, int8_t* q_col, int64_t ldq_col,
+                          float* s_col, void* sum, int64_t R, int64_t C, int block, void* workspace, size_t workspace_bytes, void* stream) {
+    DeviceOfCall call;
+    if (R <= 0 || C <= 0 || ldx < C || ldq_row < C || ldq_col < R) return fail(BI8_ERR_SHAPE, "quantize_dual_sum: bad shape R=%lld C=%lld ldx=%lld", (long long)R, (long long)C, (long long)ldx);
+    const size_t need = bi8_quantize_dual_sum_workspace_bytes(x_dtype, R, C, block);
+    if (need == 0) return fail(BI8_ERR_LIMIT, "quantize_dual_sum: 16-bit inputs and blocks of 32, 64 or 128");
+    if (!x || !q_row || !s_row || !q_col || !s_col || !sum) return fail(BI8_ERR_NULL, "quantize_dual_sum: null pointer");
+    if (!workspace || workspace_bytes < need || !aligned(workspace, 4)) return fail(BI8_ERR_WORKSPACE, "quantize_dual_sum: workspace missing or too small");
+    if (!aligned(x, 2) || !aligned(sum, 2) || !aligned(s_row, 4) || !aligned(s_col, 4)) return fail(BI8_ERR_ALIGN, "quantize_dual_sum: pointer not element aligned");
+    if (!quantize_tile_applicable(x_dtype, q_col, ldq_col, q_row, ldq_row, R, C, block))
+        return fail(BI8_ERR_ALIGN, "quantize_dual_sum: int8 rows do not begin on 16-byte boundaries");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    float* partial = static_cast<float*>(workspace);
+    const int rc = launch_quantize_tile(x, x_dtype, ldx, q_col, ldq_col, s_col, q_row, ldq_row, s_row, R, C, block, st, partial);
+    return rc != BI8_OK ? rc : launch_column_sum_finish(partial, sum, x_dtype, C, (R + kTileSumRows - 1) / kTileSumRows, st);
+}
+
 int bi8_quantize_dual(const void* x, int x_dtype, int64_t ldx, int8_t* q_row, float* s_row, int8_t* q_col, float* s_col, int64_t R,
                       int64_t C, int block, void* stream) {
     return bi8_quantize_dual_pitched(x, x_dtype, ldx, q_row, C, s_row, q_col, R, s_col, R, C, block, stream);

@@ -124,7 +124,9 @@ int launch_quantize_colwise(const void* x, int dt, int64_t ldx, int8_t* q, int64
 // tile quantizer (quantize_tile.cu): column-wise result, and with q_row != nullptr the row-wise result of the same input
 bool quantize_tile_applicable(int dt, const void* q_col, int64_t ldqc, const void* q_row, int64_t ldqr, int64_t R, int64_t C, int block);
 int launch_quantize_tile(const void* x, int dt, int64_t ldx, int8_t* q_col, int64_t ldqc, float* s_col, int8_t* q_row, int64_t ldqr,
-                         float* s_row, int64_t R, int64_t C, int block, cudaStream_t st);
+                         float* s_row, int64_t R, int64_t C, int block, cudaStream_t st, float* sums = nullptr);   // sums [ceil(R / 128), C]: column sums of the tile rows (both results only)
+constexpr int kTileSumRows = 128;
+int launch_column_sum_finish(const float* partial, void* out, int dt, int64_t C, int64_t ranges, cudaStream_t st);
 // several small quantizations, column sums and row copies in one launch (quantize.cu)
 bool quantize_jobs_fit(const bi8_quantize_task* tasks, int n, int block);
 int launch_quantize_jobs(const bi8_quantize_task* tasks, int n, int block, cudaStream_t st);

@@ -117,6 +117,33 @@ __global__ void __launch_bounds__(128) column_sum_finish_kernel(const float* __r
     sum_store(out, dt, c, v);
 }
 
+// The same for many partial rows (one per 128 rows of the matrix): 32 columns by eight groups of consecutive partial rows, each in
+// ascending order with eight loads in flight, then the groups in ascending order.
+__global__ void __launch_bounds__(256) column_sum_groups_kernel(const float* __restrict__ partial, void* __restrict__ out, int dt, int C, int ranges) {
+    after_predecessor();
+    __shared__ float s_part[8][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+    const int per = (ranges + 7) / 8, r0 = g * per, r1 = r0 + per < ranges ? r0 + per : ranges;
+    float v = 0.0f;
+    if (c < C) {
+        for (int r = r0; r < r1; r += 8) {
+            float f[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) f[u] = r + u < r1 ? __ldcg(partial + (int64_t)(r + u) * C + c) : 0.0f;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v += f[u];
+        }
+    }
+    s_part[g][lane] = v;
+    __syncthreads();
+    if (g == 0 && c < C) {
+        v = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v += s_part[k][lane];
+        sum_store(out, dt, c, v);
+    }
+}
+
 // Row ranges: enough CTAs for four per SM, but at least 128 rows each, one batch of loads.
 int row_ranges(int64_t R, int64_t C, int sms) {
     const int64_t ctiles = (C + kSumCols - 1) / kSumCols;
@@ -151,6 +178,12 @@ int launch_column_sum(const void* x, int dt, int64_t ldx, void* out, int64_t R, 
     const int rc = dt == BI8_BF16 ? launch(column_sum_kernel<BI8_BF16>) : dt == BI8_F16 ? launch(column_sum_kernel<BI8_F16>) : launch(column_sum_kernel<BI8_F32>);
     if (rc != BI8_OK || ranges == 1) return rc;
     return launch_chained(column_sum_finish_kernel, (unsigned)((C + 127) / 128), 128, 0, st, partial, out, dt, (int)C, ranges);
+}
+
+// Column sums of `ranges` partial rows [ranges, C].
+int launch_column_sum_finish(const float* partial, void* out, int dt, int64_t C, int64_t ranges, cudaStream_t st) {
+    if (C >= (1ll << 31) - 65536 || ranges >= (1ll << 31)) return fail(BI8_ERR_LIMIT, "column_sum: too many columns or partial sums");
+    return launch_chained(column_sum_groups_kernel, (unsigned)((C + 31) / 32), 256, 0, st, partial, out, dt, (int)C, (int)ranges);
 }
 
 }  // namespace bi8

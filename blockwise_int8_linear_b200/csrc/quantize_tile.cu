@@ -59,7 +59,8 @@ struct QLayout {
     static constexpr uint32_t in_off = 0, in_stage = IN == kOct ? kOctStage : kInStage;
     static constexpr uint32_t outc_off = NST * in_stage;              // [128 columns][128 row bytes]
     static constexpr uint32_t ex_off = outc_off + kQT * 128;          // absmax exchange [4 row groups][128 columns] fp32
-    static constexpr uint32_t bar_off = ex_off + 4 * kQT * 4;         // 2 * NST barriers and the abort flag
+    static constexpr uint32_t sum_off = ex_off + 4 * kQT * 4;         // column sums of the row groups (dual only)
+    static constexpr uint32_t bar_off = sum_off + 4 * kQT * 4;        // 2 * NST barriers and the abort flag
     static constexpr uint32_t outr_off = bar_off + 1024;              // [128 rows][128 column bytes]   (dual only)
     static constexpr uint32_t bytes_col = outr_off, bytes_dual = outr_off + kQT * 128;
     static_assert(outr_off % 1024 == 0 && outc_off % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
@@ -234,11 +235,11 @@ struct ShiftLoader {
     }
 };
 
-template <typename T, int B, bool DUAL, int IN>
+template <typename T, int B, bool DUAL, int IN, bool SUM>
 __global__ void __launch_bounds__(DUAL ? 2 * kQThreads : kQThreads, DUAL ? 1 : 2)
 quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmQc,
                      const __grid_constant__ CUtensorMap tmQr, const void* __restrict__ x, int64_t ldx, float* __restrict__ s_col,
-                     float* __restrict__ s_row, int R, int C, int col_tiles, int num_tiles, int* status) {
+                     float* __restrict__ s_row, float* __restrict__ sums, int R, int C, int col_tiles, int num_tiles, int* status) {
     static_assert(B == 32 || B == 64 || B == 128, "block sizes of the tile quantizer");
     constexpr int NT = DUAL ? 2 * kQThreads : kQThreads;
     constexpr int NST = DUAL ? 3 : 2;                      // input stages: the loads of the next NST - 1 tiles are in flight
@@ -405,6 +406,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             PairQ pq;
             pq.set(alo, ahi);
             const int c = 2 * p;
+            float sum_lo = 0.0f, sum_hi = 0.0f;            // SUM: this thread's 32 rows of both columns
             const uint32_t outc = base + L::outc_off;
             auto quantize_cols = [&](auto fast_tag) {
                 constexpr bool FAST = decltype(fast_tag)::value;
@@ -418,6 +420,10 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                         for (int u = 0; u < 4; ++u) {
                             float xlo, xhi;
                             Pk<T>::unpack(v[part * 16 + k * 4 + u], xlo, xhi);
+                            if (SUM) {
+                                sum_lo += xlo;
+                                sum_hi += xhi;
+                            }
                             pq.template q<FAST>(xlo, xhi, bl[u], bh[u]);
                         }
                         wl[k] = pack4(bl[0], bl[1], bl[2], bl[3]);
@@ -442,11 +448,17 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                     }
                 }
             }
+            if (SUM) reinterpret_cast<float2*>(base_ptr + L::sum_off)[g * 64 + p] = make_float2(sum_lo, sum_hi);
             fence_proxy_async_smem();
             role_barrier(rt_id, kQThreads);
             if (rtid == 0) {
                 tma_store_2d(&tmQc, outc, r0, c0);
                 tma_store_commit();
+            }
+            if (SUM && rtid < kQT && c0 + rtid < C) {
+                // the tile's row groups in ascending order; the next tile writes them behind another barrier of the role
+                const float* part = reinterpret_cast<const float*>(base_ptr + L::sum_off) + rtid;
+                sums[(int64_t)(r0 / kQT) * C + c0 + rtid] = ((part[0] + part[kQT]) + part[2 * kQT]) + part[3 * kQT];
             }
             store_next();
         } else {
@@ -632,14 +644,14 @@ int cached_q_map(CUtensorMap* map, int dev, int8_t* ptr, int64_t rows, int64_t c
     return rc;
 }
 
-template <typename T, int B, bool DUAL, int IN>
-int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap& tqr, const void* x, int64_t ldx, float* s_col, float* s_row,
+template <typename T, int B, bool DUAL, int IN, bool SUM>
+int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap& tqr, const void* x, int64_t ldx, float* s_col, float* s_row, float* sums,
                 int64_t R, int64_t C, cudaStream_t st) {
     const int64_t ctiles = (C + kQT - 1) / kQT, rtiles = (R + kQT - 1) / kQT;
     if (ctiles * rtiles >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "quantize: grid too large");
     constexpr size_t smem = (DUAL ? QLayout<3, IN>::bytes_dual : QLayout<2, IN>::bytes_col) + 1024;
     static SmemOptIn opt_in;
-    const int rc = opt_in.ensure(quantize_tile_kernel<T, B, DUAL, IN>, smem);
+    const int rc = opt_in.ensure(quantize_tile_kernel<T, B, DUAL, IN, SUM>, smem);
     if (rc != BI8_OK) return rc;
     int* status = device_status_ptr();
     if (!status) return BI8_ERR_CUDA;
@@ -647,11 +659,11 @@ int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap
     const int64_t tiles = ctiles * rtiles;
     const int64_t resident = (int64_t)(DUAL ? 1 : 2) * di.sms;                 // CTAs that fit at once
     const int grid = (int)(tiles < resident ? tiles : resident);
-    return launch_chained(quantize_tile_kernel<T, B, DUAL, IN>, grid, DUAL ? 2 * kQThreads : kQThreads, smem, st, tx, tqc, tqr, x, ldx, s_col, s_row, (int)R, (int)C, (int)ctiles, (int)tiles, status);
+    return launch_chained(quantize_tile_kernel<T, B, DUAL, IN, SUM>, grid, DUAL ? 2 * kQThreads : kQThreads, smem, st, tx, tqc, tqr, x, ldx, s_col, s_row, sums, (int)R, (int)C, (int)ctiles, (int)tiles, status);
 }
 
 template <typename T>
-int tile_dispatch(const void* x, int64_t ldx, int8_t* q_col, int64_t ldqc, float* s_col, int8_t* q_row, int64_t ldqr, float* s_row, int64_t R,
+int tile_dispatch(const void* x, int64_t ldx, int8_t* q_col, int64_t ldqc, float* s_col, int8_t* q_row, int64_t ldqr, float* s_row, float* sums, int64_t R,
                   int64_t C, int block, cudaStream_t st) {
     CUtensorMap tx, tqc, tqr;
     int dev = 0;
@@ -670,12 +682,12 @@ int tile_dispatch(const void* x, int64_t ldx, int8_t* q_col, int64_t ldqc, float
         rc = cached_q_map(&tqr, dev, q_row, R, C, ldqr, oct);
         if (rc != BI8_OK) return rc;
     }
-#define BI8_TILE_D(BB, DUAL)                                                                                \
-    tiled ? launch_tile<T, BB, DUAL, kTiled>(tx, tqc, tqr, x, ldx, s_col, s_row, R, C, st)                  \
-    : oct ? launch_tile<T, BB, DUAL, kOct>(tx, tqc, tqr, x, ldx, s_col, s_row, R, C, st)                    \
-          : launch_tile<T, BB, DUAL, kShift>(tx, tqc, tqr, x, ldx, s_col, s_row, R, C, st)
+#define BI8_TILE_D(BB, DUAL, SUM)                                                                                \
+    tiled ? launch_tile<T, BB, DUAL, kTiled, SUM>(tx, tqc, tqr, x, ldx, s_col, s_row, sums, R, C, st)           \
+    : oct ? launch_tile<T, BB, DUAL, kOct, SUM>(tx, tqc, tqr, x, ldx, s_col, s_row, sums, R, C, st)             \
+          : launch_tile<T, BB, DUAL, kShift, SUM>(tx, tqc, tqr, x, ldx, s_col, s_row, sums, R, C, st)
 #define BI8_TILE(BB) \
-    if (block == BB) return dual ? (BI8_TILE_D(BB, true)) : (BI8_TILE_D(BB, false));
+    if (block == BB) return !dual ? (BI8_TILE_D(BB, false, false)) : sums ? (BI8_TILE_D(BB, true, true)) : (BI8_TILE_D(BB, true, false));
     BI8_TILE(32) BI8_TILE(64) BI8_TILE(128)
 #undef BI8_TILE
 #undef BI8_TILE_D
@@ -696,9 +708,9 @@ bool quantize_tile_applicable(int dt, const void* q_col, int64_t ldqc, const voi
 }
 
 int launch_quantize_tile(const void* x, int dt, int64_t ldx, int8_t* q_col, int64_t ldqc, float* s_col, int8_t* q_row, int64_t ldqr,
-                         float* s_row, int64_t R, int64_t C, int block, cudaStream_t st) {
-    if (dt == BI8_BF16) return tile_dispatch<__nv_bfloat16>(x, ldx, q_col, ldqc, s_col, q_row, ldqr, s_row, R, C, block, st);
-    if (dt == BI8_F16) return tile_dispatch<__half>(x, ldx, q_col, ldqc, s_col, q_row, ldqr, s_row, R, C, block, st);
+                         float* s_row, int64_t R, int64_t C, int block, cudaStream_t st, float* sums) {
+    if (dt == BI8_BF16) return tile_dispatch<__nv_bfloat16>(x, ldx, q_col, ldqc, s_col, q_row, ldqr, s_row, sums, R, C, block, st);
+    if (dt == BI8_F16) return tile_dispatch<__half>(x, ldx, q_col, ldqc, s_col, q_row, ldqr, s_row, sums, R, C, block, st);
     return fail(BI8_ERR_DTYPE, "tile quantizer takes bf16 or fp16 input");
 }
 

@@ -651,9 +651,10 @@ variable_list LinearBackward::apply(variable_list&& grads) {
         const Quantized cached = need_x ? cache_get(cache, "col") : Quantized{};
         Quantized fresh;                                     // the weight's other blocking, where the cache is to keep it
         const size_t ws_x = need_x ? bi8_gemm_workspace_used(m, k, n, (int)b) : 0, ws_w = need_w ? bi8_gemm_workspace_used(n, k, m, (int)b) : 0,
-                     ws_b = need_b ? bi8_column_sum_workspace_bytes(m, n) : 0;
+                     ws_b = need_b ? bi8_column_sum_workspace_bytes(m, n) : 0,
+                     ws_d = need_b && need_x && need_w && fuse_dual ? bi8_quantize_dual_sum_workspace_bytes(g_code, m, n, (int)b) : 0;
         Carve carve;
-        const int64_t ws_at = carve.take((int64_t)std::max({ws_x, ws_w, ws_b}));
+        const int64_t ws_at = carve.take((int64_t)std::max({ws_x, ws_w, ws_b, ws_d}));
         QPlan g_row, g_col, w_col, x_col;
         if (need_x) g_row = QPlan(carve, m, n, b);
         if (need_w) g_col = QPlan(carve, n, m, b);
@@ -704,6 +705,14 @@ variable_list LinearBackward::apply(variable_list&& grads) {
                 tasks.list[0].sum = out[2].data_ptr();
                 summed = tasks.fits(b);
                 if (!summed) tasks.list[0].sum = nullptr;
+            }
+            if (!summed && ws_d && m > 0 && n > 0) {
+                // larger ones: from the read that makes both blockings
+                check(bi8_quantize_dual_sum(g.ptr, g_code, g.ld, gr.q, gr.ld, gr.s, gc.q, gc.ld, gc.s, out[2].data_ptr(), m, n, (int)b, ws, ws_d, st),
+                      "bi8_quantize_dual_sum");
+                for (int i = 1; i < tasks.n; ++i) tasks.list[i - 1] = tasks.list[i];
+                --tasks.n;
+                summed = true;
             }
         }
         tasks.run(b, st);

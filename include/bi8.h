@@ -154,6 +154,14 @@ BI8_API int bi8_quantize_rowwise_pre_pitched(int op, const void* x, const void* 
 BI8_API int bi8_dequantize_rowwise_pitched(const int8_t* q, int64_t ldq, const float* s, void* out, int out_dtype,
                                            int64_t M, int64_t K, int block, void* stream);
 
+/* bi8_quantize_dual_pitched of a 16-bit x that also sums its columns (C values of x_dtype, accumulated in fp32 in a fixed order) from the
+ * same read: a gradient's two blockings and the bias gradient.  workspace: bi8_quantize_dual_sum_workspace_bytes, which is 0 for
+ * what it does not take (fp32, other blocks); the int8 rows begin on 16-byte boundaries. */
+BI8_API size_t bi8_quantize_dual_sum_workspace_bytes(int x_dtype, int64_t R, int64_t C, int block);
+BI8_API int bi8_quantize_dual_sum(const void* x, int x_dtype, int64_t ldx, int8_t* q_row, int64_t ldq_row, float* s_row, int8_t* q_col,
+                                  int64_t ldq_col, float* s_col, void* sum, int64_t R, int64_t C, int block, void* workspace,
+                                  size_t workspace_bytes, void* stream);
+
 /* Several quantizations of one pass.  A task quantizes x [rows, cols] row-wise (q_row not NULL), column-wise (q_col), or both, sums its
  * columns into `sum` (cols values of x_dtype, accumulated in fp32 in a fixed order), or (x_dtype BI8_I8) copies int8 rows to
  * q_row as bi8_copy_rows does.  The quantized results are those of the single-purpose functions.  Small tasks share one launch;

@@ -161,6 +161,37 @@ def test_dual_equals_both_single_quantizers(shape, block, dt):
     assert_clean_device()
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("block", [32, 64, 128])
+@pytest.mark.parametrize("shape", [(128, 128), (1, 3), (8, 33), (200, 257), (129, 64), (1031, 386), (8192, 768), (72, 50257)])
+def test_dual_with_column_sums(shape, block, dt):
+    """The column sums of the dual quantizer's tiles: the quantized results stay what they are; each sum is fp32 over R terms, so within
+    R * 2^-24 * sum |x| of the exact one before it is rounded to the input's type."""
+    from blockwise_int8_linear_b200 import _lib
+    from triton_functions import quantize_block_dual
+    L = _lib.lib()
+    r, c = shape
+    x = randn_bf16(shape, r + c, outliers=0.01).to(dt).to(DEV)
+    code = _lib.BI8_BF16 if dt == torch.bfloat16 else _lib.BI8_F16
+    pr, pc = (c + 15) // 16 * 16, (r + 15) // 16 * 16
+    q_row, q_col = (torch.zeros(s, dtype=torch.int8, device=DEV) for s in ((r, pr), (c, pc)))
+    s_row, s_col = torch.zeros((-(-c // block), r), device=DEV), torch.zeros((-(-r // block), c), device=DEV)
+    out = torch.zeros(c, dtype=dt, device=DEV)
+    need = L.bi8_quantize_dual_sum_workspace_bytes(code, r, c, block)
+    ws = torch.empty(need, dtype=torch.uint8, device=DEV)
+    p = _lib.ptr
+    _lib.check(L.bi8_quantize_dual_sum(p(x), code, c, p(q_row), pr, p(s_row), p(q_col), pc, p(s_col), p(out), r, c, block, p(ws), need, _lib.stream_ptr()),
+               "bi8_quantize_dual_sum")
+    want = quantize_block_dual(x, block)
+    for got, ref in zip((q_row[:, :c], s_row, q_col[:, :r], s_col), want):
+        assert torch.equal(got, ref)
+    exact, mag = x.double().sum(0), x.double().abs().sum(0)
+    step = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+    assert bool(((out.double() - exact).abs() <= r * 2.0 ** -24 * mag * (1 + step) + step * exact.abs()).all())
+    assert L.bi8_quantize_dual_sum_workspace_bytes(_lib.BI8_F32, r, c, block) == 0
+    assert_clean_device()
+
+
 def test_dual_strided_rows_and_extremes():
     """Row pitch larger than the row, values at the ends of the bf16 range, and a block whose only nonzero is subnormal in
     fp32 terms (the exact-division shortcut must hand over to the IEEE division there)."""
