@@ -41,15 +41,15 @@
 // needs no int->float conversion.  s = sA[j,m]/127^2 rounded to 22 significant bits makes 1.5*2^23*s exact.
 // The pattern is written by an fp16 MMA of constants (every row 2048, 2048, 2048, 0 ...: 3 * 2048^2 = 1.5*2^23, exact in any
 // order) that overwrites the accumulator, issued by the seeder and complete (commit, barrier) before the block's int8 MMAs are
-// issued; its A lies in tensor memory, so that it reads only B from shared memory (1.3 % at block 64).  As tensor-memory stores of the promotion warps it cost them 100 of 590 cycles per block in isolation and held
-// every accumulator until the last of its columns was folded.
+// issued; its A lies in tensor memory, so that it reads only B from shared memory (1.3 % at block 64: 678 -> 668 us).  As
+// tensor-memory stores of the promotion warps it cost them 100 of 590 cycles per block in isolation and held every accumulator
+// until the last of its columns was folded.
 #include "bi8_common.cuh"
 #include "tc_common.cuh"
 
 #include <cstring>
 #include <mutex>
 #include <type_traits>
-
 
 namespace bi8 {
 namespace {

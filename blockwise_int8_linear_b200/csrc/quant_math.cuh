@@ -53,6 +53,7 @@ __device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
     return d;
 }
 __device__ __forceinline__ void f2_bits(uint64_t v, uint32_t& lo, uint32_t& hi) { asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v)); }
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -87,7 +88,8 @@ __device__ __forceinline__ float2 unpack16(uint32_t w, bool bf) {
 // eps = (|t| + 16) * 1.25 * 2^-24 of silu_exact's fp32 value before rounding, t = g log2 e (the rounding of t costs |t| 2^-24, the exponential
 // 4 units of 2^-24, the reciprocal 2, the sum and the product 1 each, and silu_exact's own error is at most 4), and where s (1 - eps) and
 // s (1 + eps) round to the same value, that is the value.  Elsewhere (1 in 1400 values of bf16, 1 in 180 of fp16) and for
-// |g| > 60 silu_exact is evaluated.  65 instructions per value became 20: 2048 x 11008 in 41 us was bound by issue.
+// |g| > 60 (in any of the eight) silu_exact is evaluated.  65 instructions per value became 20; the products and sums run on packed
+// pairs, each rounded on its own (4096 x 11008: 62.3 -> 60.4 us).
 __device__ __forceinline__ void silu_mul8(float (&g)[8], const float (&v)[8], int dt) {
     if (dt == BI8_F32) {
 #pragma unroll
@@ -95,27 +97,34 @@ __device__ __forceinline__ void silu_mul8(float (&g)[8], const float (&v)[8], in
         return;
     }
     const bool bf = dt == BI8_BF16;
+    float most = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) most = fmaxf(most, fabsf(g[e]));
+    const bool far = !(most <= 60.0f);
+    const uint64_t log2e = f2_pack(-1.4426950408889634f, -1.4426950408889634f), one = f2_pack(1.0f, 1.0f);
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
-        float lo[2], hi[2];
-        bool far = false;
+        const uint64_t x = f2_pack(g[2 * h], g[2 * h + 1]);
+        float t[2], ex[2], sum[2], r[2], eps[2], lo[2], hi[2], y[2];
+        f2_unpack(f2_mul(x, log2e), t[0], t[1]);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-            const float x = g[2 * h + u], t = __fmul_rn(x, -1.4426950408889634f);
-            float ex, r;
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ex) : "f"(t));
-            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fadd_rn(1.0f, ex)));
-            const float s = __fmul_rn(x, r), eps = __fmaf_rn(fabsf(t), 1.25f * 5.9604644775390625e-8f, 20.0f * 5.9604644775390625e-8f);
-            hi[u] = __fmaf_rn(s, eps, s);
-            lo[u] = __fmaf_rn(s, -eps, s);
-            far = far || !(fabsf(x) <= 60.0f);
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ex[u]) : "f"(t[u]));
+            eps[u] = __fmaf_rn(fabsf(t[u]), 1.25f * 5.9604644775390625e-8f, 20.0f * 5.9604644775390625e-8f);
         }
+        f2_unpack(f2_fma(f2_pack(ex[0], ex[1]), one, one), sum[0], sum[1]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r[u]) : "f"(sum[u]));
+        const uint64_t s = f2_mul(x, f2_pack(r[0], r[1]));
+        f2_unpack(f2_fma(s, f2_pack(eps[0], eps[1]), s), hi[0], hi[1]);
+        f2_unpack(f2_fma(s, f2_pack(-eps[0], -eps[1]), s), lo[0], lo[1]);
         uint32_t w = pack16(lo[0], lo[1], bf);
         if (far || w != pack16(hi[0], hi[1], bf)) w = pack16(silu_exact(g[2 * h], dt), silu_exact(g[2 * h + 1], dt), bf);
-        const float2 s = unpack16(w, bf);
-        const float2 y = unpack16(pack16(__fmul_rn(s.x, v[2 * h]), __fmul_rn(s.y, v[2 * h + 1]), bf), bf);
-        g[2 * h] = y.x;
-        g[2 * h + 1] = y.y;
+        const float2 silu = unpack16(w, bf);
+        f2_unpack(f2_mul(f2_pack(silu.x, silu.y), f2_pack(v[2 * h], v[2 * h + 1])), y[0], y[1]);
+        const float2 z = unpack16(pack16(y[0], y[1], bf), bf);
+        g[2 * h] = z.x;
+        g[2 * h + 1] = z.y;
     }
 }
 

@@ -18,6 +18,7 @@
 // they are resident before that kernel has finished.
 #include "bi8_common.cuh"
 #include "quant_math.cuh"
+#include "tc_common.cuh"
 
 #include <cstring>
 
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quan
     }
 }
 
-// One thread per unit of eight elements, as in the decode quantizer.
+// One thread per unit of eight elements, as in the decode quantizer: few rows, fp32, operands off 16-byte boundaries.
 template <int QB, int DT>
 __global__ void __launch_bounds__(kPreThreads) silu_mul_quantize_kernel(const void* __restrict__ gate, const void* __restrict__ up,
                                                                         int64_t ldx, int8_t* __restrict__ q, int64_t ldq,
@@ -251,6 +252,89 @@ __global__ void __launch_bounds__(kPreThreads) silu_mul_quantize_kernel(const vo
         silu_mul8(y, v, dt);
     }
     quantize_unit<QB>(y, valid, dt != BI8_F32, q, ldq, sx, m, k, M, K, vec_out != 0);
+}
+
+// The same for many rows of 16-bit operands on 16-byte boundaries: persistent warps walk over units of four rows x 256 columns, a row
+// at a time with the next row's two loads in flight while one is computed.  The lane that leads a block keeps the four rows' scales
+// and writes them as one piece of the transposed scales.  In the kernel above a thread loads, computes 20 instructions per value and
+// stores, one after another.  Behind a flushed L2, with silu_mul8 on packed pairs: 4096 x 11008 72.7 -> 60.4 us, 2048 x 11008 41.9 ->
+// 35.3, 512 x 11008 16.4 -> 15.4.  Five CTAs per SM (48 registers, 12 bytes spilled) against four: 62.5 -> 60.4; the exact silu out of
+// line: 62.5 -> 64.5.  kSiluWide: from as many units as the resident warps can take (five CTAs x eight warps x 148 SMs = 5920) two
+// thirds on; with fewer, threads of the kernel above are more in flight (1376 units of 128 x 11008: no difference).
+constexpr int kSiluCtas = 5;
+constexpr int64_t kSiluWide = 4096;
+template <int QB, int DT>
+__global__ void __launch_bounds__(kPreThreads, kSiluCtas) silu_mul_quantize_stream_kernel(const void* __restrict__ gate, const void* __restrict__ up,
+                                                                               int64_t ldx, int8_t* __restrict__ q, int64_t ldq,
+                                                                               float* __restrict__ sx, int M, int K, FastDiv col_units, unsigned units,
+                                                                               int vec_s) {
+    after_predecessor();
+    constexpr int LPB = QB / 8;
+    const int lane = threadIdx.x & 31;
+    const unsigned warps = gridDim.x * (kPreThreads / 32);
+    unsigned u = blockIdx.x * (kPreThreads / 32) + (threadIdx.x >> 5);
+    if (u >= units) return;
+    uint4 g, v;
+    unsigned rg = col_units.div(u);
+    int m = (int)rg * 4, k = (int)(u - rg * (unsigned)col_units.d) * 256 + lane * 8;
+    auto fetch = [&](int row, int col) {
+        g = v = make_uint4(0u, 0u, 0u, 0u);
+        if (row < M && col < K) {
+            const int64_t at = ((int64_t)row * ldx + col) * 2;
+            g = ld_nc_v4(static_cast<const unsigned char*>(gate) + at);
+            v = ld_nc_v4(static_cast<const unsigned char*>(up) + at);
+        }
+    };
+    fetch(m, k);
+    while (true) {
+        const unsigned un = u + warps;
+        int mn = M, kn = 0;
+        if (un < units) {
+            rg = col_units.div(un);
+            mn = (int)rg * 4;
+            kn = (int)(un - rg * (unsigned)col_units.d) * 256 + lane * 8;
+        }
+        float scale[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            float y[8], w[8];
+            {
+                const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, vw[4] = {v.x, v.y, v.z, v.w};
+                unpack8(y, gw, DT);
+                unpack8(w, vw, DT);
+            }
+            if (r < 3) fetch(m + r + 1, k);
+            else fetch(mn, kn);
+            silu_mul8(y, w, DT);
+            float amax = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(y[e]));
+#pragma unroll
+            for (int off = 1; off < LPB; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+            scale[r] = amax;
+            BlockQ bq;
+            bq.set(amax, true);
+            if (m + r < M && k < K) {
+                uint32_t lo, hi;
+                quantize8(y, bq, lo, hi);
+                *reinterpret_cast<uint2*>(q + (int64_t)(m + r) * ldq + k) = make_uint2(lo, hi);
+            }
+        }
+        if (lane % LPB == 0 && k < K) {
+            float* dst = sx + (int64_t)(k / QB) * M + m;
+            if (vec_s) {
+                *reinterpret_cast<float4*>(dst) = make_float4(scale[0], scale[1], scale[2], scale[3]);
+            } else {
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    if (m + r < M) dst[r] = scale[r];
+            }
+        }
+        if (un >= units) return;
+        u = un;
+        m = mn;
+        k = kn;
+    }
 }
 
 // C[m, n] = cast(C[m, n] + R[m, n]): the addition a layer's `x + proj(...)` performs in the activation type
@@ -317,6 +401,18 @@ int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t l
         const int64_t units = M * nb * (block / 8);
         const unsigned grid = (unsigned)((units + kPreThreads - 1) / kPreThreads);
         const FastDiv upr((int64_t)nb * (block / 8));
+        const int64_t col_units = (K + 255) / 256, wide = (M + 3) / 4 * col_units;
+        if (dt != BI8_F32 && vec_in && vec_out && M >= 4 && wide >= kSiluWide && wide < (1ll << 30)) {
+            const FastDiv cu(col_units);
+            const int vec_s = M % 4 == 0 && aligned(sx, 16);
+            const int64_t want = (wide + kPreThreads / 32 - 1) / (kPreThreads / 32), fit = (int64_t)device_info().sms * kSiluCtas;
+            const unsigned ctas = (unsigned)(want < fit || fit <= 0 ? want : fit);
+#define BI8_PRE_SILU_STREAM(QB)                                                                                                      \
+    if (block == QB) return dt == BI8_BF16 ? launch_chained(silu_mul_quantize_stream_kernel<QB, BI8_BF16>, ctas, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, cu, (unsigned)wide, vec_s) \
+                                           : launch_chained(silu_mul_quantize_stream_kernel<QB, BI8_F16>, ctas, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, cu, (unsigned)wide, vec_s);
+            BI8_PRE_SILU_STREAM(32) BI8_PRE_SILU_STREAM(64) BI8_PRE_SILU_STREAM(128)
+#undef BI8_PRE_SILU_STREAM
+        }
 #define BI8_PRE_SILU(QB)                                                                                                             \
     do {                                                                                                                             \
         if (dt == BI8_BF16) return launch_chained(silu_mul_quantize_kernel<QB, BI8_BF16>, grid, kPreThreads, 0, st, x, x2, ldx, q, ldq, sx, Mi, Ki, upr, vec_in, vec_out); \

@@ -94,6 +94,27 @@ def test_silu_mul_quantize_bit_exact(shape, dt, block):
     assert_clean_device()
 
 
+@pytest.mark.parametrize("shape", [(1030, 4104), (4099, 1000), (513, 8192), (512, 8192)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("block", [32, 64, 128])
+def test_silu_mul_quantize_many_rows_bit_exact(shape, dt, block):
+    """The persistent kernel of many rows, at its smallest size and with rows and columns left over: the same values as the separate
+    steps give, gates beyond the range of the approximation and blocks of zeros among them."""
+    set_config(block)
+    tf = _tf()
+    m, k = shape
+    gu = randn_bf16((m, 2 * k), m + k, std=2.0).to(dt).to(DEV)
+    gate, up = gu[:, :k], gu[:, k:]
+    gate[::7, 5::97] *= 40
+    gate[m // 2, :block] = 0
+    up[m - 1, k - 8:] = 0
+    q, s = tf.silu_mul_quantize_block_rowwise(gate, up)
+    want_q, want_s = tf.quantize_block_rowwise(F.silu(gate) * up)
+    assert torch.equal(s, want_s)
+    assert torch.equal(q, want_q)
+    assert_clean_device()
+
+
 def test_pre_quantizers_empty_and_errors():
     set_config(64)
     tf = _tf()
