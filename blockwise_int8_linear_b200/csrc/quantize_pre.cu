@@ -254,15 +254,16 @@ __global__ void __launch_bounds__(kPreThreads) silu_mul_quantize_kernel(const vo
     quantize_unit<QB>(y, valid, dt != BI8_F32, q, ldq, sx, m, k, M, K, vec_out != 0);
 }
 
-// The same for many rows of 16-bit operands on 16-byte boundaries: persistent warps walk over units of four rows x 256 columns, a row
-// at a time with the next row's two loads in flight while one is computed.  The lane that leads a block keeps the four rows' scales
-// and writes them as one piece of the transposed scales.  In the kernel above a thread loads, computes 20 instructions per value and
-// stores, one after another.  Behind a flushed L2, with silu_mul8 on packed pairs: 4096 x 11008 72.7 -> 60.4 us, 2048 x 11008 41.9 ->
-// 35.3, 512 x 11008 16.4 -> 15.4.  Five CTAs per SM (48 registers, 12 bytes spilled) against four: 62.5 -> 60.4; the exact silu out of
-// line: 62.5 -> 64.5.  kSiluWide: from as many units as the resident warps can take (five CTAs x eight warps x 148 SMs = 5920) two
-// thirds on; with fewer, threads of the kernel above are more in flight (1376 units of 128 x 11008: no difference).
-constexpr int kSiluCtas = 5;
-constexpr int64_t kSiluWide = 4096;
+// The same for many rows of 16-bit operands on 16-byte boundaries: persistent warps walk over units of two rows x 256 columns, a row
+// at a time with the next row's two loads in flight while one is computed; in the kernel above a thread loads, computes 20
+// instructions per value and stores, one after another.  The lane that leads a block writes both rows' scales at once.  Cold
+// operands, bf16, block 64, 11008 columns, kernel above against this one: 4096 rows 68.9 -> 54.7 us, 2048 36.5 -> 28.9, 1024 18.9 ->
+// 15.7, 512 10.8 -> 9.0, 384 8.6 -> 8.6, 256 6.2 -> 5.4, 128 (2752 units) 4.05 -> 3.9, 64 (1376) 3.15 -> 3.2: kSiluWide lies between the
+// last two.  Units of four rows: 2048 rows 30.4 us, 768 15.4 (the last round is emptier; 12.7 with two); of one row: 31.1 and 12.8.
+// Four CTAs per SM instead of five (48 registers): 62.5 us against 60.4 with units of four; the exact silu out of line: 64.5 against 62.5.
+constexpr int kSiluCtas = 5, kSiluRows = 2;
+constexpr int64_t kSiluWide = 2500;
+
 template <int QB, int DT>
 __global__ void __launch_bounds__(kPreThreads, kSiluCtas) silu_mul_quantize_stream_kernel(const void* __restrict__ gate, const void* __restrict__ up,
                                                                                int64_t ldx, int8_t* __restrict__ q, int64_t ldq,
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(kPreThreads, kSiluCtas) silu_mul_quantize_stre
     if (u >= units) return;
     uint4 g, v;
     unsigned rg = col_units.div(u);
-    int m = (int)rg * 4, k = (int)(u - rg * (unsigned)col_units.d) * 256 + lane * 8;
+    int m = (int)rg * kSiluRows, k = (int)(u - rg * (unsigned)col_units.d) * 256 + lane * 8;
     auto fetch = [&](int row, int col) {
         g = v = make_uint4(0u, 0u, 0u, 0u);
         if (row < M && col < K) {
@@ -291,19 +292,19 @@ __global__ void __launch_bounds__(kPreThreads, kSiluCtas) silu_mul_quantize_stre
         int mn = M, kn = 0;
         if (un < units) {
             rg = col_units.div(un);
-            mn = (int)rg * 4;
+            mn = (int)rg * kSiluRows;
             kn = (int)(un - rg * (unsigned)col_units.d) * 256 + lane * 8;
         }
-        float scale[4];
+        float scale[kSiluRows];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+        for (int r = 0; r < kSiluRows; ++r) {
             float y[8], w[8];
             {
                 const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, vw[4] = {v.x, v.y, v.z, v.w};
                 unpack8(y, gw, DT);
                 unpack8(w, vw, DT);
             }
-            if (r < 3) fetch(m + r + 1, k);
+            if (r + 1 < kSiluRows) fetch(m + r + 1, k);
             else fetch(mn, kn);
             silu_mul8(y, w, DT);
             float amax = 0.0f;
@@ -323,10 +324,10 @@ __global__ void __launch_bounds__(kPreThreads, kSiluCtas) silu_mul_quantize_stre
         if (lane % LPB == 0 && k < K) {
             float* dst = sx + (int64_t)(k / QB) * M + m;
             if (vec_s) {
-                *reinterpret_cast<float4*>(dst) = make_float4(scale[0], scale[1], scale[2], scale[3]);
+                *reinterpret_cast<float2*>(dst) = make_float2(scale[0], scale[kSiluRows - 1]);
             } else {
 #pragma unroll
-                for (int r = 0; r < 4; ++r)
+                for (int r = 0; r < kSiluRows; ++r)
                     if (m + r < M) dst[r] = scale[r];
             }
         }
@@ -401,10 +402,10 @@ int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t l
         const int64_t units = M * nb * (block / 8);
         const unsigned grid = (unsigned)((units + kPreThreads - 1) / kPreThreads);
         const FastDiv upr((int64_t)nb * (block / 8));
-        const int64_t col_units = (K + 255) / 256, wide = (M + 3) / 4 * col_units;
-        if (dt != BI8_F32 && vec_in && vec_out && M >= 4 && wide >= kSiluWide && wide < (1ll << 30)) {
+        const int64_t col_units = (K + 255) / 256, wide = (M + kSiluRows - 1) / kSiluRows * col_units;
+        if (dt != BI8_F32 && vec_in && vec_out && wide >= kSiluWide && wide < (1ll << 30)) {
             const FastDiv cu(col_units);
-            const int vec_s = M % 4 == 0 && aligned(sx, 16);
+            const int vec_s = M % 2 == 0 && aligned(sx, 8);
             const int64_t want = (wide + kPreThreads / 32 - 1) / (kPreThreads / 32), fit = (int64_t)device_info().sms * kSiluCtas;
             const unsigned ctas = (unsigned)(want < fit || fit <= 0 ? want : fit);
 #define BI8_PRE_SILU_STREAM(QB)                                                                                                      \

@@ -94,11 +94,11 @@ def test_silu_mul_quantize_bit_exact(shape, dt, block):
     assert_clean_device()
 
 
-@pytest.mark.parametrize("shape", [(1030, 4104), (4099, 1000), (513, 8192), (512, 8192)])
+@pytest.mark.parametrize("shape", [(1030, 4104), (4099, 1000), (513, 8192), (512, 8192), (157, 8192), (156, 8192)])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("block", [32, 64, 128])
 def test_silu_mul_quantize_many_rows_bit_exact(shape, dt, block):
-    """The persistent kernel of many rows, at its smallest size and with rows and columns left over: the same values as the separate
+    """The persistent kernel of many rows, at its smallest size (157 x 8192; 156 rows are the other kernel's) and with rows and columns left over: the same values as the separate
     steps give, gates beyond the range of the approximation and blocks of zeros among them."""
     set_config(block)
     tf = _tf()
