@@ -871,9 +871,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     __syncwarp();
                     if (lane == 0)
                         bulk_send(map_to(place + (rank < owner ? rank : rank - 1u) * G::RX_BYTES, owner), src, G::RX_BYTES, map_to(full, owner));
-                } else if (ok) {
-                    ok = __all_sync(0xffffffffu, mbar_wait_cluster(full, 0u, abort_flag));
-                    if (!ok) fail_code = W_PART;
+                } else {
+                    if (ok) {
+                        ok = __all_sync(0xffffffffu, mbar_wait_cluster(full, 0u, abort_flag, wait_limit));
+                        if (!ok) fail_code = W_PART;
+                    }
+                    // Given up, here or before: the others send all the same, at the latest when a wait of theirs runs out, and
+                    // neither end of such a copy may be gone before it has landed.
+                    if (!ok) (void)mbar_wait_cluster(full, 0u, never_flag, 2 * wait_limit);
 #pragma unroll
                     for (int g = 0; g < COLS / 4; ++g) {
                         float own[4], sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -890,9 +895,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         acc2[2 * g + 1] = pack_f32x2(sum[2], sum[3]);
                     }
                     __syncwarp();                   // all of the place is read: it may be staged into
-                } else {
-                    // not gone before the others' copies have landed
-                    (void)mbar_wait_cluster(full, 0u, never_flag);
                 }
             }
             if (!ok) break;
@@ -1450,7 +1452,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     SplitPlan pl;
     pl.stages_per_split = (int)((g.K + kBK - 1) / kBK);
     if (!partials) {
-        const SplitPlan want = plan_of(g, seed && g.wait_limit_us == 0);
+        const SplitPlan want = plan_of(g, seed);
         // without a large enough, 16-byte aligned workspace the GEMM simply runs unsplit
         if (want.cluster) pl = want;
         else if (want.ksplit > 1 && g.workspace != nullptr && g.workspace_bytes >= want.bytes && aligned(g.workspace, 16)) pl = want;

@@ -167,7 +167,7 @@ __device__ __forceinline__ void remote_arrive(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 // mbar_wait for data that another CTA of the cluster has sent
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t abort_flag) {
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t abort_flag, long long limit_cycles = 4000000000ll) {
     const long long t0 = clock64();
     while (true) {
         uint32_t ok;
@@ -179,7 +179,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
             : "r"(bar), "r"(parity)
             : "memory");
         if (ok != 0u) return true;
-        if (lds_volatile_u32(abort_flag) != 0u || clock64() - t0 > 4000000000ll) return false;
+        if (lds_volatile_u32(abort_flag) != 0u || clock64() - t0 > limit_cycles) return false;
     }
 }
 // Bulk copy to another CTA of the cluster (16-byte aligned, a multiple of 16 bytes), counted there on `cluster_bar`.

@@ -280,6 +280,33 @@ def test_bounded_wait_gives_up_cleanly():
     set_config(64)
 
 
+@pytest.mark.parametrize("block", [32, 64, 128])
+def test_bounded_wait_gives_up_cleanly_in_a_cluster(block):
+    """The same where the parts of a tile are the CTAs of a cluster: a stage that every CTA misses, and (33 stages for two CTAs) one that only
+    the second has, whose part the first waits for.  All leave, the status says why, and the next call is right."""
+    import ctypes
+    from blockwise_int8_linear_b200 import _lib
+    L = _lib.lib()
+    set_config(block, torch.float32)
+    m, k, n = 128, 33 * 128, 11008
+    assert L.bi8_gemm_workspace_bytes(m, n, k, block) > 0 == L.bi8_gemm_workspace_used(m, n, k, block), "the plan is a cluster"
+    xq, xs, wq, ws = quantized_pair(m, k, n, block, seed=block)
+    a, bt, sa, sb = xq.to(DEV), wq.to(DEV), xs.to(DEV), ws.to(DEV)
+    c = torch.empty((m, n), dtype=torch.float32, device=DEV)
+    assert _lib.device_status() == 0
+    rows = [0, 31, 64, 127]
+    for skip in (0, 15, 16):
+        rc = L.bi8_gemm_wait_selftest(_lib.ptr(a), k, _lib.ptr(bt), k, _lib.ptr(sa), _lib.ptr(sb), _lib.ptr(c), n, _lib.BI8_F32,
+                                      m, n, k, block, 200, skip, _lib.stream_ptr())
+        _lib.check(rc, "bi8_gemm_wait_selftest")
+        torch.cuda.synchronize()
+        detail = ctypes.c_int(0)
+        assert L.bi8_device_status(ctypes.byref(detail)) == -6 and detail.value == 2
+        _check_fp32(_gemm(xq, wq, xs, ws)[rows], xq[rows], wq, xs[:, rows].contiguous(), ws, block)
+    assert_clean_device()
+    set_config(64)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("shape", [
     # (M, N, row pitch of C beyond N, elements between a 16-byte boundary and C)
