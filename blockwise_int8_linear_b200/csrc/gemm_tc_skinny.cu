@@ -719,6 +719,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     // ---------------- teardown ----------------
     tc_fence_before();
     __syncthreads();
+    const bool gave_up = lds_volatile_u32(abort_flag) != 0u;
     if (warp == MW) {
         tc_fence_after();
         tmem_dealloc(tmem_base, G::TMEM_COLS);
@@ -728,6 +729,12 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     if (!cluster_ready) cluster_wait();
     cluster_arrive();
     cluster_wait();
+    // A CTA that gave up has not waited for everything that was sent to it, and the barrier orders the sending of an asynchronous
+    // store, not its arrival: it stays for 0.2 ms, where such a store takes a microsecond.
+    if (gave_up) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 400000ll) __nanosleep(1000);
+    }
 }
 
 // Row-wise block quantizer for the few activation rows of a decode step (same arithmetic as the standalone quantizer:
