@@ -47,6 +47,7 @@
 #include "bi8_common.cuh"
 #include "tc_common.cuh"
 
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -1256,7 +1257,8 @@ struct ClusterSlots {
     int n[kMostCluster + 1] = {0};
 };
 
-SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, double stage, int sms, const ClusterSlots* slots) {
+// `limit`: bytes of workspace that a plan may use.
+SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, double stage, int sms, const ClusterSlots* slots, size_t limit = SIZE_MAX) {
     SplitPlan pl;
     const int bn = tc_bn();
     const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
@@ -1269,7 +1271,8 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, double stage, i
     double best = rounds(tiles) * stage * nks * (fills ? kSplitWorth : 1.0);
     for (int want = 2; want <= 32 && want <= nks; ++want) {
         const int spp = (nks + want - 1) / want, s = (nks + spp - 1) / spp;
-        if (fills ? (size_t)tiles * (size_t)s * (size_t)pl.slot_floats * 4 > kSplitBytes : tiles * want > sms) break;
+        const size_t bytes = (size_t)tiles * (size_t)s * (size_t)pl.slot_floats * 4;
+        if (bytes > limit || (fills ? bytes > kSplitBytes : tiles * want > sms)) break;
         const double cost = rounds(tiles * s) * stage * spp + kSplitUs + kSlotUs * (double)(tiles * s);
         if (cost < best) {
             best = cost;
@@ -1328,11 +1331,13 @@ const ClusterSlots* cluster_slots() {
     return &t;
 }
 
-// The plan of a shape on the current device, with or without clusters.  A call asks for it two or three times (scratch, choice of kernel,
-// launch) at 0.2 to 0.4 us each; each thread keeps the last few (a plan depends on nothing but its key).
-SplitPlan plan_of(const GemmArgs& g, bool clusters) {
+// The plan of a shape on the current device, with or without clusters, in a workspace of at most `limit` bytes.  A call asks for it two or
+// three times (scratch, choice of kernel, launch) at 0.2 to 0.4 us each; each thread keeps the last few (a plan depends on
+// nothing but its key).
+SplitPlan plan_of(const GemmArgs& g, bool clusters, size_t limit = SIZE_MAX) {
     struct Entry {
         int64_t M = -1, N = 0, K = 0;
+        size_t limit = 0;
         int block = 0, dev = 0;
         bool clusters = false;
         SplitPlan plan;
@@ -1340,15 +1345,16 @@ SplitPlan plan_of(const GemmArgs& g, bool clusters) {
     static thread_local Entry memo[8];
     int dev = 0;
     if (current_device(&dev) != cudaSuccess) dev = 0;
-    Entry& e = memo[((uint64_t)(g.M * 31 + g.N * 7 + g.K * 3 + g.block + (clusters ? 1 : 0)) * 0x9E3779B97F4A7C15ull) >> 61];
-    if (e.M != g.M || e.N != g.N || e.K != g.K || e.block != g.block || e.dev != dev || e.clusters != clusters) {
-        const SplitPlan plan = plan_split(g.M, g.N, g.K, g.block, stage_us(g.block), device_info().sms, clusters ? cluster_slots() : nullptr);
+    Entry& e = memo[((uint64_t)(g.M * 31 + g.N * 7 + g.K * 3 + g.block + (int64_t)(limit >> 8) * 5 + (clusters ? 1 : 0)) * 0x9E3779B97F4A7C15ull) >> 61];
+    if (e.M != g.M || e.N != g.N || e.K != g.K || e.block != g.block || e.dev != dev || e.clusters != clusters || e.limit != limit) {
+        const SplitPlan plan = plan_split(g.M, g.N, g.K, g.block, stage_us(g.block), device_info().sms, clusters ? cluster_slots() : nullptr, limit);
         e.M = g.M;
         e.N = g.N;
         e.K = g.K;
         e.block = g.block;
         e.dev = dev;
         e.clusters = clusters;
+        e.limit = limit;
         e.plan = plan;
     }
     return e.plan;
@@ -1452,10 +1458,10 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     SplitPlan pl;
     pl.stages_per_split = (int)((g.K + kBK - 1) / kBK);
     if (!partials) {
-        const SplitPlan want = plan_of(g, seed);
-        // without a large enough, 16-byte aligned workspace the GEMM simply runs unsplit
-        if (want.cluster) pl = want;
-        else if (want.ksplit > 1 && g.workspace != nullptr && g.workspace_bytes >= want.bytes && aligned(g.workspace, 16)) pl = want;
+        pl = plan_of(g, seed);
+        // the best plan that a smaller workspace has room for (one that is not 16-byte aligned is none): fewer parts, a cluster or no division
+        const size_t given = g.workspace != nullptr && aligned(g.workspace, 16) ? g.workspace_bytes : 0;
+        if (pl.bytes > given) pl = plan_of(g, seed, given);
     }
     p.ksplit = pl.ksplit;
     p.stages_per_split = pl.stages_per_split;

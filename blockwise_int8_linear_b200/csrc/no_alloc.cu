@@ -61,7 +61,8 @@ int bi8_gemm_dequant_static(const int8_t* A, int64_t lda, const int8_t* Bt, int6
                             const void* bias, int bias_dtype, void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N,
                             int64_t K, int block, int flags, void* stream) {
     // The plan that cannot be left out: split-K of the general kernel, at block 64 whatever the block, so that a shape is taken or
-    // refused for every block alike.  Another block's plan that does not fit the array runs undivided.
+    // refused for every block alike.  Another block's plan that does not fit the array
+    // gives way to the best one that does.
     bi8::GemmArgs shape{};
     shape.M = M;
     shape.N = N;
@@ -73,8 +74,8 @@ int bi8_gemm_dequant_static(const int8_t* A, int64_t lda, const int8_t* Bt, int6
                          "gemm_dequant_static: this shape needs %zu bytes of split-K scratch, the built-in array holds %zu; "
                          "use bi8_gemm_dequant with a caller workspace",
                          need, bi8::kScratchBytes);
-    // The array is offered to the dispatcher at its full size: launch_gemm_tc(), the only taker, runs unsplit unless
-    // workspace_bytes covers its plan.
+    // The array is offered to the dispatcher at its full size: launch_gemm_tc(), the only taker, plans with what it
+    // has room for.
     void* scratch = nullptr;
     size_t given = 0;
     if (bi8_gemm_workspace_bytes(M, N, K, block) > 0) {

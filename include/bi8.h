@@ -113,8 +113,9 @@ BI8_API size_t bi8_column_sum_workspace_bytes(int64_t R, int64_t C);
  * A  [M,K] int8, row stride lda.  Bt [N,K] int8, row stride ldb — the reference's `b` operand is the
  * transposed view Bt^T with strides (1, ldb).  sA [ceil(K/block), M], sB [ceil(K/block), N] fp32.
  * bias [N] of bias_dtype or NULL.  C [M,N] of out_dtype, row stride ldc.
- * workspace: bi8_gemm_workspace_bytes(M,N,K,block) bytes of 16-byte aligned device memory (may be NULL when that
- * is 0; without it shapes with few output tiles run slower).  It is plain scratch: nothing has to be cleared, every
+ * workspace: bi8_gemm_workspace_bytes(M,N,K,block) bytes of 16-byte aligned device memory, at most 112 MiB (may be NULL when
+ * that is 0).  In a smaller one, or none, the call runs the fastest way that it has room for: K divided into fewer parts, into parts
+ * that meet without a workspace, or not at all.  It is plain scratch: nothing has to be cleared, every
  * call overwrites what it later reads; calls that may run concurrently, or that several threads enqueue on one stream (a call
  * is more than one launch), need separate workspaces.
  * The int32 partial sums are exact.  The fp32 accumulation of the tensor-core kernel for M > 64 evaluates a term as
@@ -192,7 +193,8 @@ BI8_API int bi8_copy_rows(const int8_t* src, int64_t lds, int8_t* dst, int64_t l
  * allocator, a caller with a fixed memory footprint.  (No counterpart in the reference, whose wrappers allocate
  * with torch on every call.)  The split-K scratch comes from a fixed 8 MiB array inside the library (reported by
  * bi8_gemm_static_scratch_bytes; every GPU that loads the library holds it until exit); a shape of few tiles whose plan
- * at block 64 needs more returns BI8_ERR_LIMIT (other plans that need more run undivided).  No cudaMalloc/cudaFree or allocating library call is made.  The first call on a
+ * at block 64 needs more returns BI8_ERR_LIMIT (other plans that need more
+ * give way to the best one that fits).  No cudaMalloc/cudaFree or allocating library call is made.  The first call on a
  * device looks up the array's device address: make it outside any stream capture.  All calls share the array
  * (nothing needs clearing between calls); calls that can overlap on one GPU race on it and must be serialised by
  * the caller.  Arguments and results are those of bi8_gemm_dequant (bit-identical where both select the same kernel;

@@ -185,7 +185,8 @@ def test_outputs_of_a_few_rounds_are_divided_over_k(m, k, n, block):
 @pytest.mark.parametrize("block", [32, 64, 128])
 def test_division_over_k_knows_the_block(m, k, n, divided, block):
     """A stage of block 32 takes three times one of block 128, so dividing pays earlier: which blocks divide a shape, and the result
-    against the undivided kernel (no workspace), as far apart as two orders of an fp32 sum are, and against the oracle."""
+    against the undivided kernel (no workspace; without seeds no clusters either), as far apart as two orders of an fp32 sum and another
+    conversion are, and against the oracle."""
     from tests.test_zz_no_alloc import _lib
     lib, L = _lib()
     set_config(block)
@@ -196,7 +197,7 @@ def test_division_over_k_knows_the_block(m, k, n, divided, block):
     got = _tf().int8_matmul_block64_rowwise_dequantize(a, bt.t(), sa, sb).float()
     c = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
     p = lib.ptr
-    lib.check(L.bi8_gemm_dequant(p(a), k, p(bt), k, p(sa), p(sb), None, 0, p(c), n, 0, m, n, k, block, None, 0, 0, lib.stream_ptr()), "undivided")
+    lib.check(L.bi8_gemm_dequant(p(a), k, p(bt), k, p(sa), p(sb), None, 0, p(c), n, 0, m, n, k, block, None, 0, lib.GEMM_NO_SEED, lib.stream_ptr()), "undivided")
     rows = torch.arange(0, m, 37)
     ref = O.gemm(xq[rows], wq.t(), sx[:, rows], sw, None, block, torch.bfloat16).float()
     for want in (c.float()[rows.to(DEV)].cpu(), ref):
@@ -204,6 +205,39 @@ def test_division_over_k_knows_the_block(m, k, n, divided, block):
     assert ((got - c.float()).norm() / c.float().norm()).item() <= 5e-3
     assert_clean_device()
     set_config(64)
+
+
+@pytest.mark.parametrize("flags", [2, 2 | 4])
+@pytest.mark.parametrize("m,k,n,block", [(300, 3072, 768, 64), (128, 4096, 4096, 32), (96, 5120, 640, 128), (1000, 40960, 1600, 64)])
+def test_smaller_workspace_takes_a_smaller_plan(m, k, n, block, flags):
+    """What a call's plan needs, a byte less, two parts, a byte less, none: divided through whatever workspace holds a plan that pays (few
+    tiles without clusters: two parts), written only there, and within the tolerance of the oracle on sampled rows."""
+    from blockwise_int8_linear_b200 import _lib as lib
+    L = lib.lib()
+    need = L.bi8_gemm_workspace_bytes(m, n, k, block)
+    tiles = -(-m // 128) * -(-n // 160)
+    part = tiles * min(128, -(-m // 32) * 32) * 160 * 4
+    assert need >= 3 * part, "the plan has three parts or more"
+    gen = torch.Generator(device=DEV).manual_seed(k)
+    nb = -(-k // block)
+    a, bt = (torch.randint(-127, 128, (r, k), generator=gen, device=DEV, dtype=torch.int8) for r in (m, n))
+    sa, sb = (torch.rand((nb, r), generator=gen, device=DEV) + 0.1 for r in (m, n))
+    rows = torch.tensor([0, 31, m // 2, m - 1])
+    host = (a[rows].cpu(), bt.cpu().t(), sa[:, rows].cpu(), sb.cpu(), block)
+    acc, mag = O.gemm_acc(*host), O.gemm_term_abs_sum(*host)
+    p = lib.ptr
+    few = tiles * 2 <= torch.cuda.get_device_properties(0).multi_processor_count
+    for given in (need, need - 1, 2 * part, 2 * part - 1, 0):
+        ws = torch.full((need + 4096,), 0x5A, dtype=torch.uint8, device=DEV)
+        c = torch.empty((m, n), dtype=torch.float32, device=DEV)
+        lib.check(L.bi8_gemm_dequant(p(a), k, p(bt), k, p(sa), p(sb), None, 0, p(c), n, lib.BI8_F32, m, n, k, block, p(ws), given, flags,
+                                     lib.stream_ptr()), "bi8_gemm_dequant")
+        written = bool((ws[:given] != 0x5A).any())
+        assert bool((ws[given:] == 0x5A).all())
+        if given >= need - 1 or given < 2 * part or (few and flags & lib.GEMM_NO_SEED):
+            assert written == (given >= 2 * part)
+        assert bool(((c[rows].cpu() - acc).abs() <= 12 * 2.0 ** -24 * mag).all())
+    assert_clean_device()
 
 
 @pytest.mark.parametrize("block", [32, 64, 128])

@@ -105,7 +105,7 @@ def test_static_scratch_rejects_oversized_plans():
 @pytest.mark.parametrize("m,k,n,rc", [(512, 768, 768, 0), (300, 3072, 768, -9), (128, 1024, 1024, 0)])
 def test_static_scratch_takes_the_same_shapes_for_every_block(m, k, n, rc, block):
     """At block 32 a GEMM is divided into more parts than at block 64 (512 x 768 x 768: six, 9.8 MB; not at all at 64): what does not
-    fit the array runs undivided, as without a workspace."""
+    fit the array runs by a plan that does, near the result without a workspace."""
     lib, L = _lib()
     a, bt, _, _, _ = _operands(m, k, n, seed=m)
     sa, sb = (torch.rand((k // block, r), device="cuda") + 0.5 for r in (m, n))
