@@ -278,6 +278,11 @@ struct Bias {
     }
 };
 
+// Workspace of a GEMM call: without seeds no parts of a tile meet in a cluster, and those that would have take one.
+size_t gemm_workspace(int64_t m, int64_t n, int64_t k, int64_t block, int flags) {
+    return flags & BI8_GEMM_NO_SEED ? bi8_gemm_workspace_bytes(m, n, k, (int)block) : bi8_gemm_workspace_used(m, n, k, (int)block);
+}
+
 struct Operands {
     Mat a, bt;
 };
@@ -312,7 +317,7 @@ Tensor gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& state_x, const
     const Tensor sx = state_x.contiguous(), sw = state_w.contiguous();
     Tensor c = empty_on(a_in, {m, n}, out_type);
     const Bias bias(bias_in, n);
-    const size_t ws_bytes = flags ? bi8_gemm_workspace_bytes(m, n, k, (int)block) : bi8_gemm_workspace_used(m, n, k, (int)block);
+    const size_t ws_bytes = gemm_workspace(m, n, k, block, flags);
     const Tensor ws = scratch(a_in, (int64_t)ws_bytes);
     check(bi8_gemm_dequant(static_cast<const int8_t*>(o.a.ptr), o.a.ld, static_cast<const int8_t*>(o.bt.ptr), o.bt.ld, sx.const_data_ptr<float>(),
                            sw.const_data_ptr<float>(), bias.ptr, bias.code, c.data_ptr(), n, dtype_code(out_type), m, n, k, (int)block,
@@ -424,7 +429,7 @@ Tensor linear(int op, const Tensor& x_in, const Tensor& w, bool w_transposed, co
             return finish();
         }
     }
-    const size_t ws_bytes = bi8_gemm_workspace_used(m, n, k, (int)block);
+    const size_t ws_bytes = gemm_workspace(m, n, k, block, flags);
     // the quantized activations live in the call's scratch behind the GEMM's workspace
     Carve carve;
     carve.take((int64_t)ws_bytes);

@@ -130,7 +130,7 @@ BI8_API int bi8_gemm_dequant(const int8_t* A, int64_t lda, const int8_t* Bt, int
 
 BI8_API size_t bi8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int block);
 
-/* How much of that a call without flags uses: nothing where the parts of a tile are added inside clusters. */
+/* How much of that a call without BI8_GEMM_NO_SEED uses: nothing where the parts of a tile are added inside clusters. */
 BI8_API size_t bi8_gemm_workspace_used(int64_t M, int64_t N, int64_t K, int block);
 
 /* bi8_gemm_dequant plus an addend: C = cast(cast(sum) (+ bias) + residual[m,n]), the addition in the output type as a layer's

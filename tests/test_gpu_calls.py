@@ -300,3 +300,23 @@ def test_dense_layers_with_unaligned_rows(m, k, n, block):
     assert lin.W_int8.is_contiguous()
     assert_clean_device()
     set_config(64)
+
+
+@pytest.mark.parametrize("k", [4096, 4095])
+def test_layer_call_without_seeds_has_the_workspace_of_its_plan(k):
+    """BI8_GEMM_NO_SEED takes no clusters, so K is divided through a workspace: the layer's call as the two-step one, bit for bit (undivided
+    sums would differ in their last bits), for weights on 16-byte rows and off them."""
+    from blockwise_int8_linear_b200 import _lib
+    tf = _tf()
+    set_config(64, torch.float32)
+    m, n = 128, 11008
+    assert _lib.lib().bi8_gemm_workspace_bytes(m, n, k, 64) > 0 == _lib.lib().bi8_gemm_workspace_used(m, n, k, 64)
+    x = randn_bf16((m, k), 1, std=1.5).to(DEV)
+    q, s = O.quantize(randn_bf16((n, k), 2, std=0.02), 64)
+    w, sw = q.to(DEV), s.to(DEV)
+    xq, sx = tf.quantize_block_rowwise(x)
+    two = tf.int8_matmul_block64_rowwise_dequantize(xq, w.t(), sx, sw, flags=_lib.GEMM_NO_SEED)
+    assert torch.equal(tf.quantize_matmul_block_rowwise_dequantize(x, w.t(), sw, flags=_lib.GEMM_NO_SEED), two)
+    assert torch.equal(tf.pre_quantize_matmul_block_rowwise_dequantize("none", x, w.t(), sw, flags=_lib.GEMM_NO_SEED), two)
+    assert_clean_device()
+    set_config(64)
