@@ -190,7 +190,7 @@ class PeerAllReduce:
             wait_limit_us = self.wait_limit_us
         L = _lib.lib()
         with torch.cuda.device(dev):
-            ws_bytes = L.bi8_gemm_workspace_bytes(m, n, k, block)
+            ws_bytes = L.bi8_gemm_workspace_used(m, n, k, block)
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev) if ws_bytes else None
             rc = L.bi8_row_parallel_linear_pre(code, _lib.ptr(x2d), _lib.ptr(x2_2d), _lib.dtype_code(x2d.dtype), _pitch(x2d),
                                                _lib.ptr(norm_weight), float(eps), _lib.ptr(xq), _lib.ptr(sx), _lib.ptr(w_int8),

@@ -248,6 +248,19 @@ def test_peer_allreduce_one_rank_and_bounded_wait():
         want = res + quantize_matmul_block_rowwise_dequantize(torch.nn.functional.silu(gu[:, :1024]) * gu[:, 1024:], wq.t(), sw)
         assert torch.equal(big.row_parallel_linear(gu[:, :1024], wq, sw, op="silu_mul", x2=gu[:, 1024:], residual=res), want)
     assert _lib.device_status() == 0
+    # no workspace where the parts of a tile meet in clusters: outputs, quantized activations and the allocator's granules are all
+    m, k, n = 128, 4096, 11008
+    assert _lib.lib().bi8_gemm_workspace_bytes(m, n, k, 64) > 4 << 20 and _lib.lib().bi8_gemm_workspace_used(m, n, k, 64) == 0
+    wide = PeerAllReduce(m * n, DEV)
+    wq, sw = quantize_block_rowwise((torch.randn((n, k), device=DEV) * 0.02).to(torch.bfloat16))
+    x = torch.randn((m, k), device=DEV).to(torch.bfloat16)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    y = wide.row_parallel_linear(x, wq, sw)
+    assert torch.cuda.max_memory_allocated() - before < m * n * (2 + 4) + m * k + (k // 64) * m * 4 + (1 << 20)
+    assert torch.equal(y, quantize_matmul_block_rowwise_dequantize(x, wq.t(), sw))
+    assert _lib.device_status() == 0
     # the prefill-sized kernel with one rank, and its bounded waits with a second rank that never runs
     from blockwise_int8_linear_b200.peer import PeerAllReduceLarge
     big1 = PeerAllReduceLarge(300 * 4096, DEV)
