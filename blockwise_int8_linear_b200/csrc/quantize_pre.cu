@@ -127,8 +127,14 @@ __device__ __forceinline__ void quantize_unit(const float (&y)[8], bool valid, b
 // ascending order: the same bits on every launch with the same THREADS, which the launcher picks from M and K).  Pass 2: normalise, round, quantize.  Rows of up
 // to kPreHold * THREADS * 8 elements stay in registers between the passes; longer rows are read again.  THREADS = 128
 // for rows of up to 4096 elements: a row is in flight for a load latency plus a reduction, so what bounds a large
-// batch is the number of rows resident per SM (ten CTAs of 128 threads against four of 256).
-template <int QB, int THREADS, int DT>
+// batch is the number of rows resident per SM (ten CTAs of 128 threads against five of 256).
+//
+// EARLY: the weight is requested with the row, not behind the reduction, for 56 registers instead of 46 and four resident CTAs instead
+// of five.  Back to back, bf16, block 64, without / with: 8 x 4096 2.7 / 2.45 us, 256 x 4096 3.5 / 3.15, 512 x 4096 5.1 / 4.4, 760 x 4096
+// 6.8 / 6.45, 1024 x 4096 7.65 / 7.35, 2048 x 8192 21.2 / 20.0, 2048 x 5120 15.2 / 15.2 (cold, in a decode layer of 8 sequences, 69.7 /
+// 68.6 a layer).  Not where five CTAs per SM take all rows at once and four do not (600 to 740 x 4096: 5.3-5.5 / 5.7-6.3), and
+// not for rows that do not stay in registers, which have no use for it (2048 x 11008: 39.0 / 45.7, 2048 x 16384: 53.8 / 64.0).
+template <int QB, int THREADS, int DT, bool EARLY>
 __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quantize_kernel(const void* __restrict__ x, int64_t ldx,
                                                                        const void* __restrict__ weight, float eps,
                                                                        int8_t* __restrict__ q, int64_t ldq, float* __restrict__ sx, int M, int K,
@@ -143,11 +149,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quan
     const bool hold = dt != BI8_F32 && upr <= kPreHold * THREADS;
     const int64_t row_off = (int64_t)m * ldx;
     uint32_t raw[kPreHold][4];
-    // 256 threads: the weight is requested with the row, not behind the reduction (in a decode step it comes from DRAM: a layer of
-    // 8 sequences 69.7 -> 68.6 us).
-    // Where rows are many it stays in L1 and ten CTAs per SM have no registers for it.
-    constexpr bool kEarly = THREADS == 256;
-    uint32_t wraw[kEarly ? kPreHold : 1][4];
+    uint32_t wraw[EARLY ? kPreHold : 1][4];
     float ss = 0.0f;
     if (hold) {
 #pragma unroll
@@ -156,7 +158,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quan
             if (k < K) load_raw8(raw[i], x, row_off, k, K, vec_in != 0);
             else raw[i][0] = raw[i][1] = raw[i][2] = raw[i][3] = 0u;
         }
-        if constexpr (kEarly) {
+        if constexpr (EARLY) {
 #pragma unroll
             for (int i = 0; i < kPreHold; ++i) {
                 const int k = (i * THREADS + tid) * 8;
@@ -212,7 +214,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 10 : 4) rmsnorm_quan
                 const int u = i * THREADS + tid, k = u * 8;
                 float y[8];
                 unpack8(y, raw[i], dt);
-                finish_unit(y, k, u < upr && k < K, kEarly ? wraw[kEarly ? i : 0] : nullptr);
+                finish_unit(y, k, u < upr && k < K, EARLY ? wraw[EARLY ? i : 0] : nullptr);
             }
         }
     } else {
@@ -380,15 +382,18 @@ int launch_quantize_pre(int op, const void* x, const void* x2, int dt, int64_t l
         // 128 threads per row where the row fits their registers and there are rows enough to fill the SMs ten deep; a
         // handful of decode rows finish sooner with 256 threads each
         const bool narrow = (int64_t)nb * (block / 8) <= kPreHold * 128 && M > 1024;
-#define BI8_PRE_RMS_T(QB, T)                                                                                                          \
+        const int sms = device_info().sms;
+        const bool early = !narrow && (int64_t)nb * (block / 8) <= kPreHold * 256 && (M <= 4 * sms || M > 5 * sms);
+#define BI8_PRE_RMS_T(QB, T, EARLY)                                                                                                   \
     do {                                                                                                                             \
-        if (dt == BI8_BF16) return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_BF16>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
-        else if (dt == BI8_F16) return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_F16>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
-        else return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_F32>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
+        if (dt == BI8_BF16) return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_BF16, EARLY>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
+        else if (dt == BI8_F16) return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_F16, EARLY>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
+        else return launch_chained(rmsnorm_quantize_kernel<QB, T, BI8_F32, false>, (unsigned)M, T, 0, st, x, ldx, weight, eps, q, ldq, sx, Mi, Ki, nb, vec_in, vec_out); \
     } while (0)
 #define BI8_PRE_RMS(QB)                                                                                                              \
-    if (narrow) BI8_PRE_RMS_T(QB, 128);                                                                                              \
-    else BI8_PRE_RMS_T(QB, 256)
+    if (narrow) BI8_PRE_RMS_T(QB, 128, false);                                                                                       \
+    else if (early) BI8_PRE_RMS_T(QB, 256, true);                                                                                    \
+    else BI8_PRE_RMS_T(QB, 256, false)
         switch (block) {
             case 32: BI8_PRE_RMS(32); break;
             case 64: BI8_PRE_RMS(64); break;

@@ -47,6 +47,23 @@ def test_rmsnorm_quantize_integer_rows_bit_exact(shape, block):
     assert_clean_device()
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("k", [4096, 8192, 8200])
+@pytest.mark.parametrize("m", [592, 593, 740, 741])
+def test_rmsnorm_quantize_does_not_depend_on_the_number_of_rows(m, k, dt):
+    """When the weight is requested depends on the rows against what the SMs hold at once (four and five CTAs each, 148 SMs) and on their
+    length (8192 stay in registers): the same bits as in calls of 100 rows, with and without a weight."""
+    set_config(64)
+    tf = _tf()
+    gen = torch.Generator(device=DEV).manual_seed(m + k)
+    x = torch.randn((m, k), generator=gen, device=DEV).to(dt)
+    for weight in (None, (torch.rand(k, generator=gen, device=DEV) + 0.5).to(dt)):
+        q, s = tf.rmsnorm_quantize_block_rowwise(x, EPS, weight)
+        parts = [tf.rmsnorm_quantize_block_rowwise(x[i:i + 100], EPS, weight) for i in range(0, m, 100)]
+        assert torch.equal(q, torch.cat([p[0] for p in parts])) and torch.equal(s, torch.cat([p[1] for p in parts], 1))
+    assert_clean_device()
+
+
 @pytest.mark.parametrize("shape", [(8, 4096), (40, 11008), (7, 1000), (3, 150), (2, 9000)])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
 def test_rmsnorm_quantize_against_oracle(shape, dt):
