@@ -375,6 +375,47 @@ def test_divided_tiles_in_clusters(shape, dtype):
     set_config(64)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [
+    # (M, K, N, block): clusters of two and three; whole tiles, rows and columns left over, rows no tensor map describes
+    (128, 4096, 11008, 64), (70, 4096, 11001, 64), (300, 768, 3072, 32), (384, 2048, 2048, 64), (130, 2000, 5002, 64), (100, 4096, 11004, 128),
+])
+def test_addends_behind_tiles_divided_in_clusters(shape, dtype):
+    """Residual, bias and both behind a cluster's sum, in every output type: what the additions in that type make of the plain result, bit for
+    bit; and the residual updated in place."""
+    from blockwise_int8_linear_b200 import _lib
+    import triton_functions as tf
+    L = _lib.lib()
+    m, k, n, block = shape
+    set_config(block, dtype)
+    assert L.bi8_gemm_workspace_used(m, n, k, block) == 0, "the plan is a cluster"
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    x = torch.randn((m, k), generator=gen, device=DEV).to(torch.bfloat16)
+    wq = torch.randint(-127, 128, (n, k), generator=gen, device=DEV, dtype=torch.int8)
+    sw = torch.rand((-(-k // block), n), generator=gen, device=DEV) * 0.02 + 0.01
+    res, bias = torch.randn((m, n), generator=gen, device=DEV).to(dtype), torch.randn(n, generator=gen, device=DEV).to(dtype)
+    plain = tf.quantize_matmul_block_rowwise_dequantize(x, wq.t(), sw)
+    rows = [0, 31, 32, m // 2, m - 1]
+    xq, sx = tf.quantize_block_rowwise(x)
+    host = (xq[rows].cpu(), wq.t().cpu(), sx[:, rows].cpu(), sw.cpu(), block)
+    acc, mag = O.gemm_acc(*host), O.gemm_term_abs_sum(*host)
+    step = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -24}[dtype]
+    assert bool(((plain[rows].cpu().float() - acc).abs() <= FP32_TOL * mag + step * (1 + 2.0 ** -7) * acc.abs()).all())
+    for b, r in ((None, res), (bias, None), (bias, res)):
+        want = plain if b is None else plain + b
+        want = want if r is None else want + r
+        assert torch.equal(tf.pre_quantize_matmul_block_rowwise_dequantize("none", x, wq.t(), sw, b, residual=r), want)
+    if k % 16 == 0:
+        xq, sx = torch.empty((m, k), dtype=torch.int8, device=DEV), torch.empty((-(-k // block), m), device=DEV)
+        code, c = _lib.dtype_code(dtype), res.clone()
+        p = _lib.ptr
+        _lib.check(L.bi8_gemm_dequant_fused_pre(_lib.PRE_NONE, p(x), None, _lib.BI8_BF16, k, None, 0.0, p(xq), p(sx), p(wq), k, p(sw), None, 0,
+                                                p(c), n, p(c), n, code, m, n, k, block, None, 0, 0, _lib.stream_ptr()), "in place")
+        assert torch.equal(c, plain + res)
+    assert_clean_device()
+    set_config(64)
+
+
 def test_unaligned_long_contraction_is_repitched_onto_the_tensor_cores():
     """K = 1000 + 17: not a multiple of 16.  The shim re-pitches the operands; results equal the CUDA-core kernel's
     within the tensor-core tolerance and the int32 partial sums stay exact."""
