@@ -96,8 +96,10 @@ struct Cfg {
 // outputs whose rows no tensor map can describe, but every eighth of which one can (store_rows); kOwn, by the promotion warps,
 // to all others.
 enum StoreMode { kTma = 0, kRows = 1, kOwn = 2 };
-// Instances of the kernel by the way its tiles leave: code for the other ways, even where it is not executed, costs the K loop up to
-// 10 % through its registers (8192 x 4096 x 11008 at block 64).
+// Instances of the kernel by the way its tiles leave: code for the other ways, even where it is not executed, costs the K loop
+// registers.  kAnyOut in the instance's place at block 32 / 64 / 128: kTma16 8192 x 4096 x 11008 +2.1 / 2.0 / 0 %, 4096 x 512 x 4096 +4.7 / 6.3 /
+// 6.2 %; kTma16Add 2048 x 768 x 3072 +5.1 / 3.3 / 2.0 %; kOwn16 8192 x 4096 x 11005 +5.1 / 5.0 / 1.2 %; kWide 8192 x 4096 x 11008 +1.8 / 1.9 /
+// 0 %, 4096 x 512 x 4096 +3.8 / 3.9 / 0 %.
 enum OutKind { kAnyOut = 0, kSplit, kCluster, kTma16, kTma16Add, kRows16, kOwn16, kWide };
 
 struct TcParams {
@@ -1041,7 +1043,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // in ascending order, so that the result does not depend on scheduling.  A thread takes eight consecutive columns of
 // a row: one 32-byte sector of every part (NP parts in flight: no more registers than the parts
 // need; four neighbouring threads take the four rows of a 128-byte line), one 16-byte store (two for fp32) where C allows it.
-// The parts are at most one slot per SM (12 MB) and come from L2.  Launched as a programmatic dependent of the GEMM:
+// The parts come from L2 where they are few (one slot per SM, 12 MB, for outputs of few tiles) and in part from DRAM where they are
+// kSplitBytes.  Launched as a programmatic dependent of the GEMM:
 // its CTAs are resident as the GEMM's leave.
 template <int BN, int COLS, int NP>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const TcParams p) {
@@ -1227,16 +1230,20 @@ struct SplitPlan {
 };
 // What a work item takes per stage (128 K-bytes of a tile: four, two or one blocks to promote), what dividing costs whatever its size
 // (the second kernel's latency; of its host time a part) and per slot (80 KB written and read again through L2): microseconds.
-// Stage: slope over 4 to 32 stages of 4736 undivided tiles, 1.38 us at block 32, 0.68 at 64, 0.43 at 128.  The others from a
-// sweep of 1 to 32 items per tile over 14 shapes of 7 to 320 tiles and 6 to 86 stages at the three blocks: with them the plan's time is
-// within 6 % of the best measured one everywhere (512 x 768 x 768: 9.2 us in six items against 12.7 at block 32, 7.9 undivided
-// against 8.2 at 64, 6.5 against 7.3 at 128; 300 x 768 x 3072: 13.0 in eight, 10.6 in eight, 9.3 in six).  The number of
-// items with the lowest sum is taken; the largest that the SMs hold is often not the fastest.
+// Stage: slope over 4 to 32 stages of 4736 undivided tiles, 1.38 us at block 32, 0.68 at 64, 0.43 at 128.  Checked on a sweep of 1 to 32
+// items per tile and clusters of two to four over 23 shapes of 4 to 320 tiles and 6 to 86 stages at the three blocks (GEMM alone in a
+// graph): the plan is within 5 % of the best one everywhere and within 2 % in 62 of 69 (block 32 / 64 / 128, the plan's time
+// and the undivided one's: 512 x 768 x 768 8.9, 12.0 / 8.0, 8.0 / 6.5, 6.5; 300 x 3072 x 768 12.1, 36.9 / 10.1, 20.4 / 9.3, 13.8; furthest off
+// 100 x 2048 x 2048 at 64, 9.4 in four items against 9.0 in six).  The number of items with the lowest sum is taken; the
+// largest that the SMs hold is often not the fastest.
 double stage_us(int block) { return block <= 32 ? 1.38 : block <= 64 ? 0.68 : 0.43; }
 constexpr double kSplitUs = 2.9, kSlotUs = 0.017;
-// Where the tiles alone occupy more than half of the SMs, dividing has to save a twentieth, the workspace stays within L2 (8192 x 50257 x
-// 768: 320 tiles in two parts, 52 MB and five rounds of 197 stages, 732 us; in four, 105 MB and nine rounds of 99, 685), and
-// from kSplitRounds rounds on nothing is left to be saved.
+// Where the tiles alone occupy more than half of the SMs, dividing has to save a twentieth, the parts stay below kSplitBytes, and from
+// kSplitRounds rounds on nothing is left to be saved.  The parts go to DRAM and back in part (they share 126 MB of L2 with the
+// operands) but behind other tiles' loops.  MiB of parts and us, block 64, cold L2: 8192 x 50257 x 768 0 840, 50 724, 75 697, 100 683, 125 677,
+// 150 673, 200 704; 768 x 50257 x 8192 0 828, 49 718, 73 683, 97 665, 121 656, 195 659; 4096 x 50257 x 1024 0 568, 52 512, 87 497, 105 515;
+// 6144 x 30000 x 1024 0 525, 52 458, 78 447, 105 482; at blocks 32 and 128 the same order.  Beyond the limit 1 to 2 % are left for half as
+// much memory again.
 constexpr double kSplitWorth = 0.95;
 constexpr size_t kSplitBytes = 112u << 20;
 constexpr int kSplitRounds = 6;
@@ -1296,7 +1303,7 @@ SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int block, double stage, i
     return pl;
 }
 
-// Clusters of 2 to 8 CTAs of the general kernel that the device holds at once (asked once per device).
+// Clusters of two to kMostCluster CTAs of the general kernel that the device holds at once (asked once per device).
 const ClusterSlots* cluster_slots() {
     static ClusterSlots table[64];
     static std::mutex mu;
@@ -1379,9 +1386,9 @@ size_t gemm_tc_static_bytes(int64_t M, int64_t N, int64_t K) {
     return di.ok ? plan_split(M, N, K, 64, 0.72, di.sms, nullptr).bytes : 0;
 }
 
-// For the choice between this kernel and the decode kernel at 33 to 64 rows: the model that the choice was measured with (stages of the
-// kernel as it was then, division through the workspace).  With the present stage times and clusters in it 40 x 3000 x 5000
-// moved here and took 16.0 us instead of 14.0.
+// For the choice between this kernel and the decode kernel at 33 to 64 rows: a model of this kernel that does not move with its speed (stage
+// times of an earlier form, division through the workspace).  What it decides is for which shapes a caller gets the reference's order
+// of operations, not only how fast: see gemm_skinny_preferred.
 double gemm_tc_estimate_us(const GemmArgs& g) {
     const DeviceInfo di = device_info();
     const double stage = g.block <= 32 ? 1.48 : g.block <= 64 ? 0.72 : 0.45;

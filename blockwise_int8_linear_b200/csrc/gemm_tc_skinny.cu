@@ -1015,11 +1015,15 @@ int64_t gemm_skinny_part(const GemmArgs& g) {
     return g.M * ((g.K + l.plan.cluster - 1) / l.plan.cluster);
 }
 
-// Whether this kernel is also the faster one.  Up to 32 rows it always is.  From 33 on its promotion costs as much as the weights
-// take to arrive, and the general kernel overtakes it where it fills the SMs (clearly: a small layer keeps the reference's order of
-// operations): estimates in microseconds, the time of a stage by the blocks it promotes, from a sweep of 10 layer shapes at 40 and
-// 64 rows.  Measured at 64 rows, general against here, at block 32 / 64 / 128: 4096 x 22016: 56, 68 / 31, 46 / 22, 37;
-// 4096 x 12288: 54, 44 / 29, 32 / 20, 28; 4096 x 4096: 19, 18 / 13, 14 / 11, 12; 11008 x 4096: 36, 34 / 22, 24 / 17, 19.
+// Whether this kernel is taken.  Up to 32 rows it always is.  From 33 on its promotion costs as much as the weights take to arrive, and the
+// general kernel, whose terms are rounded differently, overtakes it where it fills the SMs: it is taken where a model says that
+// it gains 2.5 us (estimates in microseconds, the time of a stage by the blocks it promotes).  The present general kernel is faster than
+// that model: at 64 rows, general against here, block 32 / 64 / 128: taken there 4096 x 11008 31.8, 42.8 / 20.9, 31.7 / 16.7, 26.4; 5120 x
+// 5120 22.3, 30.3 / 15.1, 20.3 / 12.5, 16.0; kept here 8192 x 8192 55.4, 46.7 / 32.5, 30.7 / 23.8, 23.9; 11008 x 4096 34.8, 34.3 / (taken) 21.8,
+// 23.6 / 16.7, 18.9; 4096 x 4096 17.9, 17.6 / 12.8, 13.7 / 11.0, 12.1; 1024 x 1024 6.9, 10.0 / 6.2, 8.3 / 6.5, 7.6; 2048 x 2048 at 64 8.8, 11.3.
+// In 48 shapes of 33, 40 and 64 rows the general kernel is nowhere taken and more than 3 % slower; in a third this one is kept and 5 % or more
+// slower, by 3.1 us at most.  The line does not follow the general kernel's speed, because its error is the larger one: against 64
+// bits, fp32 results, 1.1-1.5e-7 where this kernel has 0.5-1.2e-7 (K up to 4096; 11008: 1.4-1.9e-7 and 1.0-1.8e-7).
 bool gemm_skinny_preferred(const GemmArgs& g) {
     if (!gemm_skinny_applicable(g)) return false;
     if (g.M <= 32) return true;

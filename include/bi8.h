@@ -118,11 +118,12 @@ BI8_API size_t bi8_column_sum_workspace_bytes(int64_t R, int64_t C);
  * that meet without a workspace, or not at all.  It is plain scratch: nothing has to be cleared, every
  * call overwrites what it later reads; calls that may run concurrently, or that several threads enqueue on one stream (a call
  * is more than one launch), need separate workspaces.
- * The int32 partial sums are exact.  The fp32 accumulation of the tensor-core kernel for M > 64 evaluates a term as
+ * The int32 partial sums are exact.  The fp32 accumulation of the general tensor-core kernel (M > 64, and large layers from M = 33 on)
+ * evaluates a term as
  * sB * fl(P * s) with s = sA/127^2 rounded to fp32 and then to 22 significant bits (relative error of s at most
  * 2^-24 + 2^-22), one rounding for P*s and one for the fused multiply-add into the sum, where the reference rounds
- * three times per term; the result stays within 12 * 2^-24 * sum_j |term_j| of the reference's.  The kernels for
- * M <= 64 and the CUDA-core kernel evaluate every term in the reference's order. */
+ * three times per term; the result stays within 12 * 2^-24 * sum_j |term_j| of the reference's.  The decode
+ * kernels and the CUDA-core kernel evaluate every term in the reference's order. */
 BI8_API int bi8_gemm_dequant(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb,
                      const float* sA, const float* sB, const void* bias, int bias_dtype,
                      void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N, int64_t K, int block,
