@@ -198,8 +198,8 @@ BI8_API int bi8_copy_rows(const int8_t* src, int64_t lds, int8_t* dst, int64_t l
  * give way to the best one that fits).  No cudaMalloc/cudaFree or allocating library call is made.  The first call on a
  * device looks up the array's device address: make it outside any stream capture.  All calls share the array
  * (nothing needs clearing between calls); calls that can overlap on one GPU race on it and must be serialised by
- * the caller.  Arguments and results are those of bi8_gemm_dequant (bit-identical where both select the same kernel;
- * for 33 <= M <= 64 this entry point always runs the general kernel). */
+ * the caller.  Arguments and results are those of bi8_gemm_dequant (bit-identical to a call with a
+ * workspace of the array's size where both select the same kernel; for 33 <= M <= 64 this entry point always runs the general kernel). */
 BI8_API int bi8_gemm_dequant_static(const int8_t* A, int64_t lda, const int8_t* Bt, int64_t ldb,
                             const float* sA, const float* sB, const void* bias, int bias_dtype,
                             void* C, int64_t ldc, int out_dtype, int64_t M, int64_t N, int64_t K, int block,

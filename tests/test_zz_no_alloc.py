@@ -117,3 +117,19 @@ def test_static_scratch_takes_the_same_shapes_for_every_block(m, k, n, rc, block
         lib.check(L.bi8_gemm_dequant(p(a), k, p(bt), k, p(sa), p(sb), None, 0, p(want), n, 1, m, n, k, block, None, 0, 0, lib.stream_ptr()), "undivided")
         assert ((c - want).norm() / want.norm()).item() <= 1e-5
     assert lib.device_status() == 0
+
+
+@pytest.mark.parametrize("m,k,n,block", [(512, 768, 768, 32), (600, 768, 640, 32), (384, 768, 960, 32)])
+def test_static_scratch_plans_like_a_workspace_of_its_size(m, k, n, block):
+    """Plans that want more than the array: the same division, and so the same bits, as in a workspace of 8 MiB."""
+    lib, L = _lib()
+    assert L.bi8_gemm_workspace_bytes(m, n, k, block) > L.bi8_gemm_static_scratch_bytes()
+    a, bt, _, _, _ = _operands(m, k, n, seed=m)
+    sa, sb = (torch.rand((k // block, r), device="cuda") + 0.5 for r in (m, n))
+    ws = torch.empty(L.bi8_gemm_static_scratch_bytes(), dtype=torch.uint8, device="cuda")
+    got, want = (torch.zeros((m, n), dtype=torch.float32, device="cuda") for _ in range(2))
+    p = lib.ptr
+    rc = L.bi8_gemm_dequant_static(p(a), k, p(bt), k, p(sa), p(sb), None, 0, p(got), n, 1, m, n, k, block, 0, lib.stream_ptr())
+    lib.check(L.bi8_gemm_dequant(p(a), k, p(bt), k, p(sa), p(sb), None, 0, p(want), n, 1, m, n, k, block, p(ws), ws.numel(), 0, lib.stream_ptr()), "workspace")
+    assert rc == 0 and torch.equal(got, want)
+    assert lib.device_status() == 0
