@@ -94,9 +94,11 @@ int launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, size_t
 }
 
 #if defined(__CUDACC__)
+__device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void after_predecessor() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    wait_predecessor();
+    release_dependents();
 }
 #endif
 

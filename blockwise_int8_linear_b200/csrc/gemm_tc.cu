@@ -532,13 +532,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t tmem_base = *tmem_holder;
     if (OUT == kCluster) cluster_arrive();          // the barriers are set up: waited for before the first send
     // Launched so that all of the above may run while the preceding kernel finishes; no global memory is touched before this
-    // wait.  Dependents become resident as this kernel's CTAs leave.
-    after_predecessor();
+    // wait.  The dependents are released by the producer when its last copies are under way: with a small kernel pending from the start (the next
+    // quantizer) every block of the K loop was slower (2048 x 4096 x 22016 at block 128 behind a quantizer: 218 us, 199 with the late release).
+    wait_predecessor();
 
     if (warp < kRoleWarps) {
         setmaxnreg_dec<C::ROLE_REGS>();
-        // Whole warps run the producer and MMA loops convergently and one lane issues: lanes parked at the final
-        // barrier while a sibling lane loops make that loop crawl.
         if (warp == 0) {
             // ---------------- producer: operand tiles and block scales ----------------
             int stage = 0, sslot = 0;
@@ -563,7 +562,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     const bool skip = first_item && p.skip_stage >= 0 && ks - ks0 == p.skip_stage;   // diagnostic only
                     const uint32_t fb = bar(G::FULL_AB + stage);
                     const uint32_t sadst = base + C::scale_off + (uint32_t)sslot * kScBytes, sbdst = sadst + G::SC_RING;
-                    if (lane == 0 && !skip) {
+                    if (!skip && elect_one()) {
                         mbar_expect_tx(fb, C::STAGE_BYTES + (tma_sa ? kScBytes : 0u) + (tma_sb ? kScBytes : 0u));
                         tma_load_2d(base + C::a_off(stage), &tmA, fb, ks * kBK, m0);
                         tma_load_2d(base + C::b_off(stage), &tmB, fb, ks * kBK, n0);
@@ -608,6 +607,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 first_item = false;
             }
+            release_dependents();
             if (!ok) {
                 // do not leave while our own copies may still land in this CTA's shared memory
 #pragma unroll
@@ -621,32 +621,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             // depends only on the stage's position in a cycle of three stages: the K loop runs in such cycles, with the
             // stage body in three copies that have the accumulator as a constant (RotInfo) and no dispatch between
             // them.  The barrier parity of each accumulator flips with every use.
-            constexpr uint32_t idesc = umma_idesc_i8(kBM, BN);
-            int stage = 0;
-            uint32_t phase = 0;
-            uint32_t accpar[kAccBufs] = {0u, 0u, 0u};
-            bool ok = true;
-            auto issue_stage = [&](auto rot_tag) {
-                constexpr int ROT = decltype(rot_tag)::value;
-                ok = warp_wait(bar(G::FULL_AB + stage), phase, abort_flag, wait_limit_mma);
-                if (!ok) {
-                    if (lane == 0) report_timeout(p.status, abort_flag, W_FULL_AB);
-                    return;
-                }
-                tc_fence_after();
-                const uint64_t adesc = umma_desc_k_sw128(base + C::a_off(stage));
-                const uint64_t bdesc = umma_desc_k_sw128(base + C::b_off(stage));
-#pragma unroll
-                for (int blk = 0; blk < G::BPS; ++blk) {
-                    const int buf = RotInfo<G::BPS>::buf(ROT, blk);
-                    ok = warp_wait(bar((SEED ? G::ACC_SEEDED : G::ACC_EMPTY) + buf), accpar[buf], abort_flag, wait_limit_mma);
+            // One elected thread runs the whole loop: its chain of waits, MMAs and commits per block is what paced the kernel.  As a loop
+            // of the warp in which a lane that a comparison picked issued, a block took 640 cycles whatever its width (four columns of
+            // promotion work instead of 40 changed nothing); with elect.sync per issue 475, this way 445.
+            if (elect_one()) {
+                constexpr uint32_t idesc = umma_idesc_i8(kBM, BN);
+                int stage = 0;
+                uint32_t phase = 0;
+                uint32_t accpar[kAccBufs] = {0u, 0u, 0u};
+                bool ok = true;
+                auto issue_stage = [&](auto rot_tag) {
+                    constexpr int ROT = decltype(rot_tag)::value;
+                    ok = mbar_wait(bar(G::FULL_AB + stage), phase, abort_flag, wait_limit_mma);
                     if (!ok) {
-                        if (lane == 0) report_timeout(p.status, abort_flag, W_ACC_EMPTY);
+                        report_timeout(p.status, abort_flag, W_FULL_AB);
                         return;
                     }
-                    accpar[buf] ^= 1u;
-                    tc_fence_after();
-                    if (lane == 0) {
+                    const uint64_t adesc = umma_desc_k_sw128(base + C::a_off(stage));
+                    const uint64_t bdesc = umma_desc_k_sw128(base + C::b_off(stage));
+#pragma unroll
+                    for (int blk = 0; blk < G::BPS; ++blk) {
+                        const int buf = RotInfo<G::BPS>::buf(ROT, blk);
+                        ok = mbar_wait(bar((SEED ? G::ACC_SEEDED : G::ACC_EMPTY) + buf), accpar[buf], abort_flag, wait_limit_mma);
+                        if (!ok) {
+                            report_timeout(p.status, abort_flag, W_ACC_EMPTY);
+                            return;
+                        }
+                        accpar[buf] ^= 1u;
+                        tc_fence_after();
 #pragma unroll
                         for (int i = 0; i < G::MMAS; ++i) {
                             const uint64_t koff = (uint64_t)((blk * G::MMAS + i) * 32 / 16);
@@ -654,51 +656,50 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                         tc_commit(bar(G::ACC_FULL + buf));
                     }
-                    __syncwarp();
-                }
-                if (lane == 0) tc_commit(bar(G::EMPTY_AB + stage));
-                __syncwarp();
-                if (++stage == kStages) { stage = 0; phase ^= 1u; }
-            };
-            for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-                int tile, slot, ks0, ks1;
-                item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
-                for (int ks = ks0; ks < ks1 && ok; ks += 3) {
-                    issue_stage(std::integral_constant<int, 0>{});
-                    if (ks + 1 < ks1 && ok) issue_stage(std::integral_constant<int, 1>{});
-                    if (ks + 2 < ks1 && ok) issue_stage(std::integral_constant<int, 2>{});
+                    tc_commit(bar(G::EMPTY_AB + stage));
+                    if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                };
+                for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+                    int tile, slot, ks0, ks1;
+                    item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
+                    for (int ks = ks0; ks < ks1 && ok; ks += 3) {
+                        issue_stage(std::integral_constant<int, 0>{});
+                        if (ks + 1 < ks1 && ok) issue_stage(std::integral_constant<int, 1>{});
+                        if (ks + 2 < ks1 && ok) issue_stage(std::integral_constant<int, 2>{});
+                    }
                 }
             }
+            __syncwarp();
         } else if (warp == 2 && SEED) {
             // ---------------- seeder ----------------
             // follows the accumulators in the order of the MMA issuer, which waits for its commits instead of the promotion warps
-            constexpr uint32_t idesc = umma_idesc_f16_f32(kBM, BN);
-            const uint64_t desc = umma_desc_k_none(base + G::seed_off, 128, 256);
-            uint32_t accpar[kAccBufs] = {0u, 0u, 0u};
-            bool ok = true;
-            auto seed_acc = [&](int buf) {
-                ok = warp_wait(bar(G::ACC_EMPTY + buf), accpar[buf], abort_flag, wait_limit);
-                if (!ok) {
-                    if (lane == 0) report_timeout(p.status, abort_flag, W_ACC_EMPTY);
-                    return;
-                }
-                accpar[buf] ^= 1u;
-                tc_fence_after();
-                if (lane == 0) {
+            if (elect_one()) {
+                constexpr uint32_t idesc = umma_idesc_f16_f32(kBM, BN);
+                const uint64_t desc = umma_desc_k_none(base + G::seed_off, 128, 256);
+                uint32_t accpar[kAccBufs] = {0u, 0u, 0u};
+                bool ok = true;
+                auto seed_acc = [&](int buf) {
+                    ok = mbar_wait(bar(G::ACC_EMPTY + buf), accpar[buf], abort_flag, wait_limit);
+                    if (!ok) {
+                        report_timeout(p.status, abort_flag, W_ACC_EMPTY);
+                        return;
+                    }
+                    accpar[buf] ^= 1u;
+                    tc_fence_after();
                     mma_f16_ta(tmem_base + (uint32_t)(buf * BN), tmem_base + (uint32_t)(kAccBufs * BN), desc, idesc, 0u);
                     tc_commit(bar(G::ACC_SEEDED + buf));
-                }
-                __syncwarp();
-            };
-            for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-                int tile, slot, ks0, ks1;
-                item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
-                const int blocks = (ks1 - ks0) * G::BPS;
-                for (int j = 0; j < blocks && ok; j += kAccBufs)
+                };
+                for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+                    int tile, slot, ks0, ks1;
+                    item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
+                    const int blocks = (ks1 - ks0) * G::BPS;
+                    for (int j = 0; j < blocks && ok; j += kAccBufs)
 #pragma unroll
-                    for (int b = 0; b < kAccBufs; ++b)
-                        if (j + b < blocks && ok) seed_acc(b);
+                        for (int b = 0; b < kAccBufs; ++b)
+                            if (j + b < blocks && ok) seed_acc(b);
+                }
             }
+            __syncwarp();
         } else if (warp == 3 && MODE == 0 && OUT != kSplit && OUT != kCluster && p.ksplit == 1 && store != kOwn && !wide) {
             // ---------------- storer ----------------
             uint32_t par = 0;
