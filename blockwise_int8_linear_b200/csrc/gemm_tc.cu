@@ -16,19 +16,23 @@
 //               enough that a slot is never rewritten while in use (SC_STAGES).
 //   warp 1      issues tcgen05.mma kind::i8 (M128 N=BN K32): the MMAs of one quantisation block accumulate into one of
 //               three s32 accumulators in tensor memory, then a commit hands that accumulator to the promotion warps.
-//   warp 2      seeder: puts the seed pattern (below) into every accumulator that the promotion warps have released.
+//   warp 2      seeder: puts the seed pattern (below) into every accumulator that the promotion warps have released, and makes the row
+//               records of every stage: per row and block (s, -1.5*2^23*s), s the row scale as the fold takes it.
 //   warp 3      storer: moves finished tiles from shared memory to C by TMA stores.
 //   warps 4-19  promotion, four warps per tensor-memory lane quarter.  A warp owns 32 rows x 40 columns of the tile.  Per
-//               block it reads its part of the finished accumulator eight columns at a time (the next eight in flight
-//               while eight are folded), folds the values into fp32 accumulators in registers, and releases the
-//               accumulator as soon as the last columns are in registers.  After the last block of a tile it casts,
-//               stages its 32 x 40 part in shared memory, adds bias and residual there and goes on with the next tile.
-// What bounds the kernel: the fold, t = P*s_row and acc += s_col*t for two columns per FFMA2.  The first has one operand that changes, the
-// second three, and a packed FMA with three 64-bit operands of its own issues every 3.2 to 3.5 cycles, not every 2 (measured in
-// isolation; two scalar FMAs are no faster): 430 cycles per 128 x 160 block for the FMAs alone, against 163 for the MMAs of a
-// 64-deep block.  With the tensor-memory reads, the column scales (broadcast loads, 8 bytes per shared-memory wavefront, in
-// competition with the tensor core's operand reads) and the hand-over of accumulators the loop takes 600-640 cycles per block of
-// 32 or 64 and 720-750 at 128.  8192 x 4096 x 11008: 716 -> 681 us at block 64, 449 -> 423 at 128, 1470 -> 1370 at 32.
+//               block it reads its part of the finished accumulator, folds the values into fp32 accumulators in registers, and
+//               releases the accumulator as soon as the last columns are in registers.  After the last block of a tile it casts, adds
+//               the bias, stages its 32 x 40 part in shared memory, adds the residual there and goes on with the next tile.
+// What bounds the kernel: at blocks of 32 and 64 the promotion, t = P*s_row and acc += s_col*t for two columns per FFMA2 (the second
+// has three 64-bit operands that change and issues every 3.2 to 3.5 cycles where its scale pair is not reused) next to what the scales
+// cost: every register that a shared-memory load fills takes its time on that pipe, broadcast or not.  As a thread with one row and 40
+// columns (32x32b reads) a warp loaded 41 scales per block and thread; with four rows and ten columns (16x256b) 4 records and 10 scales,
+// each scale pair of the columns used for four rows in turn.  Row scales are prepared once per CTA by the seeder, not by every
+// thread for its four rows.  At 128 the operands' way from L2 (64 bytes per cycle and SM, 576 cycles per 128 x 160 x 128) bounds as well.
+// 8192 x 4096 x 11008, cold: 666 -> 593 us at block 64, 416 -> 380 at 128, 1323 -> 1189 at 32 (with the row-wise reads and the
+// issuer as a loop of its warp, the same box); a lab loop without epilogue 683 -> 535, 731 -> 569 and 611 -> 535 cycles a block.
+// Reading 8 + 32 columns at a time, the accumulator is free early and the first fold hides the second read: in that loop 527 cycles
+// against 548 for all at once, 536 for 16 + 24, 636 for five times eight.
 //
 // Registers: a scheduler (SM sub-partition) owns a quarter of the register file and every fourth warp, and setmaxnreg can
 // only move registers between warps of the same scheduler.  Each scheduler has exactly one of warps 0-3, which shrinks,
@@ -72,7 +76,6 @@ constexpr int kPW = 4;
 struct Cfg {
     static constexpr int BN = 160;                        // tile columns: kAccBufs * BN <= 512 tensor-memory columns
     static constexpr int COLS = BN / kPW;                 // columns owned by one promotion thread
-    static constexpr int CH = 8;                          // columns read from the accumulator at a time
     static constexpr int EPI_WARPS = 4 * kPW;
     static constexpr int THREADS = (kRoleWarps + EPI_WARPS) * 32;
     static constexpr int LAUNCH_REGS = 96;                // 65536 / THREADS, rounded down to a multiple of 8
@@ -86,10 +89,25 @@ struct Cfg {
     // compiler really chose for the kernel.)
     static_assert(ROLE_REGS + kPW * EPI_REGS <= (1 + kPW) * LAUNCH_REGS, "register budget of a scheduler exceeds its launch allocation");
     static_assert((1 + kPW) * 32 * LAUNCH_REGS <= 16384, "launch allocation exceeds a scheduler's register file");
-    static_assert(kAccBufs * BN <= 512 && COLS % CH == 0 && COLS % 8 == 0 && BN % 32 == 0, "tile geometry");
+    static_assert(kAccBufs * BN <= 512 && COLS % 8 == 0 && BN % 32 == 0, "tile geometry");
     __host__ __device__ static constexpr uint32_t a_off(int s) { return (uint32_t)s * STAGE_BYTES; }
     __host__ __device__ static constexpr uint32_t b_off(int s) { return a_off(s) + kABytes; }
 };
+
+// Transposes a 4 x 4 matrix whose rows are the arrays of four neighbouring lanes (c the lane's place among them).
+template <typename T>
+__device__ __forceinline__ void transpose4(T (&v)[4], uint32_t c) {
+#pragma unroll
+    for (int d = 1; d <= 2; d <<= 1)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i & d) continue;
+            const bool up = (c & (uint32_t)d) != 0u;
+            const T got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + d], d);
+            if (up) v[i] = got;
+            else v[i + d] = got;
+        }
+}
 
 // How a finished tile leaves: kTma, through the tensor map tmC (16-bit outputs by the storer warp, fp32 ones in two passes by the promotion
 // warps: handing the halves over was 2 us slower where there is one round of tiles); kRows, by the storer warp to 16-bit
@@ -133,15 +151,23 @@ struct Geo {
     using C = Cfg;
     static constexpr int BPS = kBK / QB;                        // quantisation blocks per stage
     static constexpr int MMAS = QB / 32;                        // MMAs (K = 32) per block
-    // Scale rings, one record of BN floats per block for sA (128 of them used) and one for sB, so that one offset serves both.
-    // Depth: the producer fills the slot of stage s after the MMA warp has committed stage s - kStages, whose last block was
-    // issued into an accumulator that the promotion warps had released kAccBufs blocks earlier, having read everything but some
-    // of that block's scales: stages up to s - kStages - ceil((kAccBufs + 1) / BPS) may still be read.
+    // Column scales: a ring of records of BN floats, one per block.  The producer fills the slot of stage s after the MMA warp has
+    // committed stage s - kStages, whose last block was issued into an accumulator that the promotion warps had released kAccBufs
+    // blocks earlier, having read everything but some of that block's scales: stages up to s - kStages - ceil((kAccBufs + 1) / BPS)
+    // may still be read.
     static constexpr int SC_STAGES = kStages + (kAccBufs + 1 + BPS - 1) / BPS;
     static constexpr uint32_t SC_REC = C::BN * 4;               // bytes of a record
     static constexpr uint32_t SC_RING = SC_STAGES * BPS * SC_REC;
-    static constexpr uint32_t sb_off = C::scale_off + SC_RING;
-    static constexpr uint32_t bar_off = sb_off + SC_RING;
+    static constexpr uint32_t sb_off = C::scale_off;
+    // Row scales as they come, with the operand stage, and as the promotion warps read them: one (s, -1.5*2^23*s) per row and block,
+    // made by the seeder warp.  That warp has seen the accumulator of the block before a stage released, and with it the records up to
+    // kAccBufs blocks before that one read, when it writes a stage's.
+    static constexpr uint32_t SA_STAGE = BPS * kBM * 4;
+    static constexpr uint32_t sa_off = sb_off + SC_RING;
+    static constexpr uint32_t ROW_REC = kBM * 8;
+    static constexpr uint32_t ROW_RING = (BPS + kAccBufs) * ROW_REC;
+    static constexpr uint32_t row_off = sa_off + kStages * SA_STAGE;
+    static constexpr uint32_t bar_off = row_off + ROW_RING;
     // barrier slots (8 bytes each)
     static constexpr int FULL_AB = 0, EMPTY_AB = kStages, ACC_FULL = 2 * kStages, ACC_EMPTY = 2 * kStages + kAccBufs,
                          ACC_SEEDED = 2 * kStages + 2 * kAccBufs, OUT_FULL = 2 * kStages + 3 * kAccBufs, OUT_EMPTY = OUT_FULL + 1,
@@ -164,7 +190,7 @@ struct Geo {
         return out_off + (rx > OUT_BYTES ? rx : OUT_BYTES);
     }
     static_assert(PART_BYTES % 128 == 0 && CLASS_BYTES % 128 == 0 && OUT_BYTES >= C::EPI_WARPS * PART_BYTES && OUT_BYTES % 128 == 0, "TMA store sources are 128-byte aligned");
-    static_assert(SC_REC % 128 == 0 && C::scale_off % 1024 == 0, "TMA destinations of the scale boxes are 128-byte aligned");
+    static_assert(SC_REC % 128 == 0 && SA_STAGE % 128 == 0 && C::scale_off % 1024 == 0, "TMA destinations of the scale boxes are 128-byte aligned");
 };
 
 // Work item -> tile and K-stage range.  Items of one split are consecutive, so CTAs that run together work on different
@@ -224,28 +250,28 @@ __device__ __forceinline__ uint32_t keep(uint32_t v) {
     return v;
 }
 
-// Folds NC s32 words a thread has read from an accumulator (its row, columns C0 .. C0+NC-1 of its COLS, one quantisation
-// block) into its fp32 accumulators: acc[n] += sB[n] * (P[n] * s), both products as packed FMAs on column pairs.  `sw` is the
-// shared address of the block's column scales of this thread (16-byte aligned).
-template <bool SEED, int NC, int COLS>
-__device__ __forceinline__ void fold_columns(int C0, const uint32_t (&S)[NC], uint32_t sw, float sxd, float negc, uint64_t (&acc2)[COLS / 2]) {
-    const uint64_t sxd2 = pack_f32x2(sxd, sxd), negc2 = pack_f32x2(negc, negc);
+// Folds the s32 words that a thread has read of NC columns from C0 on (one quantisation block; NC / 8 groups of four words for each half of
+// 16 rows) into its fp32 accumulators: acc += sB[n] * (P * s), both products as packed FMAs on column pairs.  `sw` is the shared address
+// of the block's first pair of column scales of this thread, s2 and n2 the scales of its four rows and their seed terms.
+template <bool SEED, int NC, int C0, int COLS>
+__device__ __forceinline__ void fold_columns(const uint32_t (&W)[NC], uint32_t sw, const uint64_t (&s2)[4], const uint64_t (&n2)[4], uint64_t (&acc2)[COLS / 2]) {
 #pragma unroll
-    for (int q = 0; q < NC / 4; ++q) {
-        uint64_t w0, w1, t0, t1;
-        lds_2xb64(sw + (uint32_t)((C0 / 4 + q) * 16), w0, w1);
-        if (SEED) {
-            t0 = fma_f32x2(pack_u32x2(S[4 * q], S[4 * q + 1]), sxd2, negc2);
-            t1 = fma_f32x2(pack_u32x2(S[4 * q + 2], S[4 * q + 3]), sxd2, negc2);
-        } else {
-            float t[4];
+    for (int q = 0; q < NC / 8; ++q) {
+        const uint64_t w = lds_b64(sw + (uint32_t)((C0 / 8 + q) * 32));
+        uint64_t t[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) t[u] = __fmul_rn((float)(int32_t)S[4 * q + u], sxd);
-            t0 = pack_f32x2(t[0], t[1]);
-            t1 = pack_f32x2(t[2], t[3]);
+        for (int r = 0; r < 4; ++r) {
+            const uint32_t* const S = W + (r >> 1) * (NC / 2) + 4 * q + 2 * (r & 1);
+            if (SEED) {
+                t[r] = fma_f32x2(pack_u32x2(S[0], S[1]), s2[r], n2[r]);
+            } else {
+                float sr, dup;
+                unpack_f32x2(s2[r], sr, dup);
+                t[r] = pack_f32x2(__fmul_rn((float)(int32_t)S[0], sr), __fmul_rn((float)(int32_t)S[1], sr));
+            }
         }
-        acc2[C0 / 2 + 2 * q] = fma_f32x2(w0, t0, acc2[C0 / 2 + 2 * q]);
-        acc2[C0 / 2 + 2 * q + 1] = fma_f32x2(w1, t1, acc2[C0 / 2 + 2 * q + 1]);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc2[C0 / 2 + 4 * q + r] = fma_f32x2(w, t[r], acc2[C0 / 2 + 4 * q + r]);
     }
 }
 
@@ -263,11 +289,11 @@ __device__ __forceinline__ void ldcg_v8(float (&f)[8], const float* src) {
                  : "memory");
 }
 
-// Place of (lane quarter, column slice, group of eight columns, row of the quarter) in a workspace slot: a warp stores 1 KiB
-// runs, a thread 32 bytes of its row, and the reduction kernel reads a row's eight columns as one sector.
+// Place of (lane quarter, column slice, group of eight columns, lane) in a workspace slot: a warp stores 1 KiB runs, a thread as one
+// sector its two columns of four rows.
 template <int COLS>
-__host__ __device__ constexpr int ws_index(int quarter, int slice, int group, int row) {
-    return (((quarter * kPW + slice) * (COLS / 8) + group) * 32 + row) * 8;
+__host__ __device__ constexpr int ws_index(int quarter, int slice, int group, int lane) {
+    return (((quarter * kPW + slice) * (COLS / 8) + group) * 32 + lane) * 8;
 }
 
 // element n of a vector of type `dt`
@@ -409,51 +435,57 @@ __device__ __forceinline__ void store_rows(const TcParams& p, const void* tmC, u
     }
 }
 
-// Adds bias[n] and then residual[m, n], each in the output type, to a thread's staged row (COLS 16-bit or COLS/2 fp32 values at
-// shared address `row_addr`, columns from col0).  Columns and rows outside the output get no addend; they are not stored.
+// Asks for a bias value without using it.
+__device__ __forceinline__ void touch_bias(const TcParams& p, int n) {
+    const char* const a = static_cast<const char*>(p.bias) + (int64_t)(n < p.N ? n : p.N - 1) * (p.bias_dtype == BI8_F32 ? 4 : 2);
+    asm volatile("{\n\t.reg .u16 v;\n\tld.global.u16 v, [%0];\n\t}" ::"l"(a) : "memory");
+}
+// The bias of columns n and n + 1, zero outside the output.
+__device__ __forceinline__ void bias_pair(const TcParams& p, int n, float& lo, float& hi) {
+    lo = n < p.N ? load_as_f32(p.bias, p.bias_dtype, n) : 0.0f;
+    hi = n + 1 < p.N ? load_as_f32(p.bias, p.bias_dtype, n + 1) : 0.0f;
+}
+// The sum of two pairs of a 16-bit type, each rounded once.
+__device__ __forceinline__ uint32_t add_pair(uint32_t a, uint32_t b, bool bf) {
+    if (bf) {
+        const __nv_bfloat162 v = __hadd2_rn(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+        return *reinterpret_cast<const uint32_t*>(&v);
+    }
+    const __half2 v = __hadd2_rn(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// Adds residual[m, n] in the output type to a staged row (COLS 16-bit or COLS/2 fp32 values at shared address `row_addr`, columns from
+// col0).  Columns and rows outside the output get no addend; they are not stored.
 template <int COLS>
-__device__ __forceinline__ void add_staged(const TcParams& p, uint32_t row_addr, int m, int col0, bool wide) {
+__device__ __forceinline__ void add_residual(const TcParams& p, uint32_t row_addr, int m, int col0, bool wide) {
     const bool bf = p.out_dtype == BI8_BF16;
     const int per = wide ? 4 : 8;                       // elements of a 16-byte piece
     const int left = p.N - col0;
-    if (p.bias != nullptr) {
-        // one load per lane for the columns of the warp, handed round by shuffles: a load per column and piece was
-        // 0.7 us of latency five times (ten for fp32 outputs) per tile
-        const int lane = (int)(threadIdx.x & 31u);
-        const float b0 = lane < left ? load_as_f32(p.bias, p.bias_dtype, col0 + lane) : 0.0f;
-        const float b1 = lane + 32 < left && lane + 32 < COLS ? load_as_f32(p.bias, p.bias_dtype, col0 + lane + 32) : 0.0f;
+    if (m >= p.M) return;
+    const int64_t r0 = (int64_t)m * p.ldr + col0;
+    if (p.res_vec && COLS / 8 * per <= left) {
+        // the row's pieces are all requested before the first is added
+        uint4 res[COLS / 8];
+#pragma unroll
+        for (int g = 0; g < COLS / 8; ++g)
+            res[g] = __ldcg(reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(p.residual) + (r0 + g * per) * (wide ? 4 : 2)));
+#pragma unroll
+        for (int g = 0; g < COLS / 8; ++g) {
+            const uint32_t rw[4] = {res[g].x, res[g].y, res[g].z, res[g].w};
+            uint32_t w[4];
+            lds_v4(row_addr + (uint32_t)(g * 16), w[0], w[1], w[2], w[3]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) w[u] = wide ? __float_as_uint(__fadd_rn(__uint_as_float(w[u]), __uint_as_float(rw[u]))) : add_pair(w[u], rw[u], bf);
+            sts_v4(row_addr + (uint32_t)(g * 16), w[0], w[1], w[2], w[3]);
+        }
+    } else {
 #pragma unroll 1
         for (int g = 0; g < COLS / 8; ++g)
             add_piece(row_addr + (uint32_t)(g * 16), wide, bf, [&](int e) {
                 const int n = g * per + e;
-                return __shfl_sync(0xffffffffu, n < 32 ? b0 : b1, n & 31);
+                return n < left ? load_as_f32(p.residual, p.out_dtype, r0 + n) : 0.0f;
             });
-    }
-    if (p.residual != nullptr && m < p.M) {
-        const int64_t r0 = (int64_t)m * p.ldr + col0;
-        if (p.res_vec && COLS / 8 * per <= left) {
-            // the row's pieces are all requested before the first is added
-            uint4 res[COLS / 8];
-#pragma unroll
-            for (int g = 0; g < COLS / 8; ++g)
-                res[g] = __ldcg(reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(p.residual) + (r0 + g * per) * (wide ? 4 : 2)));
-#pragma unroll
-            for (int g = 0; g < COLS / 8; ++g) {
-                const uint32_t rw[4] = {res[g].x, res[g].y, res[g].z, res[g].w};
-                add_piece(row_addr + (uint32_t)(g * 16), wide, bf, [&](int e) {
-                    if (wide) return __uint_as_float(rw[e & 3]);
-                    const uint32_t h = (rw[(e >> 1) & 3] >> (16 * (e & 1))) & 0xffffu;
-                    return bf ? bf16lo(h) : __half2float(__ushort_as_half((unsigned short)h));
-                });
-            }
-        } else {
-#pragma unroll 1
-            for (int g = 0; g < COLS / 8; ++g)
-                add_piece(row_addr + (uint32_t)(g * 16), wide, bf, [&](int e) {
-                    const int n = g * per + e;
-                    return n < left ? load_as_f32(p.residual, p.out_dtype, r0 + n) : 0.0f;
-                });
-        }
     }
 }
 
@@ -464,7 +496,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                const __grid_constant__ CUtensorMap tmC, const TcParams p) {
     using C = Cfg;
     using G = Geo<QB>;
-    constexpr int BN = C::BN, COLS = C::COLS, CH = C::CH;
+    constexpr int BN = C::BN, COLS = C::COLS;
     constexpr bool kScales = (MODE == 0);           // the partial-sum dump uses no scales
     const int store = OUT == kTma16 || OUT == kTma16Add ? kTma : OUT == kRows16 ? kRows : OUT == kOwn16 ? kOwn : p.store;
     const bool wide = OUT == kWide || ((OUT == kAnyOut || OUT == kCluster) && p.out_dtype == BI8_F32);
@@ -495,10 +527,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int s = 0; s < kStages; ++s) {
             // the lane that issues the TMA copies; with scales copied by cp.async, every lane of the producer warp as well
             mbar_init(bar(G::FULL_AB + s), (kScales && p.tma_scales != 3) ? 33 : 1);
-            mbar_init(bar(G::EMPTY_AB + s), 1);
+            mbar_init(bar(G::EMPTY_AB + s), kScales ? 2 : 1);     // the MMAs have read the stage, the seeder its row scales
         }
         for (int b = 0; b < kAccBufs; ++b) {
-            mbar_init(bar(G::ACC_FULL + b), 1);
+            mbar_init(bar(G::ACC_FULL + b), kScales ? 2 : 1);     // the block's MMAs and its row records are complete
             mbar_init(bar(G::ACC_EMPTY + b), C::EPI_WARPS);
             mbar_init(bar(G::ACC_SEEDED + b), 1);
         }
@@ -547,7 +579,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int s = 0; s < kStages; ++s) last_parity[s] = -1;
             bool ok = true;
             bool first_item = true;
-            constexpr uint32_t kScBytes = (uint32_t)(G::BPS * BN * 4);
+            constexpr uint32_t kSbBytes = (uint32_t)(G::BPS * BN * 4);
             const bool tma_sa = kScales && (p.tma_scales & 1), tma_sb = kScales && (p.tma_scales & 2);
             for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
                 int tile, slot, ks0, ks1, m0, n0;
@@ -561,12 +593,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                     const bool skip = first_item && p.skip_stage >= 0 && ks - ks0 == p.skip_stage;   // diagnostic only
                     const uint32_t fb = bar(G::FULL_AB + stage);
-                    const uint32_t sadst = base + C::scale_off + (uint32_t)sslot * kScBytes, sbdst = sadst + G::SC_RING;
+                    const uint32_t sadst = base + G::sa_off + (uint32_t)stage * G::SA_STAGE, sbdst = base + G::sb_off + (uint32_t)sslot * kSbBytes;
                     if (!skip && elect_one()) {
-                        mbar_expect_tx(fb, C::STAGE_BYTES + (tma_sa ? kScBytes : 0u) + (tma_sb ? kScBytes : 0u));
+                        mbar_expect_tx(fb, C::STAGE_BYTES + (tma_sa ? G::SA_STAGE : 0u) + (tma_sb ? kSbBytes : 0u));
                         tma_load_2d(base + C::a_off(stage), &tmA, fb, ks * kBK, m0);
                         tma_load_2d(base + C::b_off(stage), &tmB, fb, ks * kBK, n0);
-                        // boxes [BPS, BN]; rows and blocks outside the tensors read as zero
+                        // boxes [BPS, 128] and [BPS, BN]; rows and blocks outside the tensors read as zero
                         if (tma_sa) tma_load_2d(sadst, &tmSA, fb, m0, ks * G::BPS);
                         if (tma_sb) tma_load_2d(sbdst, &tmSB, fb, n0, ks * G::BPS);
                     }
@@ -582,7 +614,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                                 for (int c = lane; c < kBM; c += 32) {
                                     const bool live = j < p.nb && m0 + c < p.M;
-                                    cp_async_4(sadst + (uint32_t)((blk * BN + c) * 4), live ? row + c : p.sA, live ? 4u : 0u);
+                                    cp_async_4(sadst + (uint32_t)((blk * kBM + c) * 4), live ? row + c : p.sA, live ? 4u : 0u);
                                 }
                             }
                             if (!tma_sb) {
@@ -670,36 +702,78 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
             }
             __syncwarp();
-        } else if (warp == 2 && SEED) {
-            // ---------------- seeder ----------------
-            // follows the accumulators in the order of the MMA issuer, which waits for its commits instead of the promotion warps
-            if (elect_one()) {
-                constexpr uint32_t idesc = umma_idesc_f16_f32(kBM, BN);
-                const uint64_t desc = umma_desc_k_none(base + G::seed_off, 128, 256);
-                uint32_t accpar[kAccBufs] = {0u, 0u, 0u};
-                bool ok = true;
-                auto seed_acc = [&](int buf) {
-                    ok = mbar_wait(bar(G::ACC_EMPTY + buf), accpar[buf], abort_flag, wait_limit);
-                    if (!ok) {
-                        report_timeout(p.status, abort_flag, W_ACC_EMPTY);
-                        return;
-                    }
-                    accpar[buf] ^= 1u;
+        } else if (warp == 2 && (SEED || kScales)) {
+            // ---------------- seeder and row records ----------------
+            // Follows the accumulators in the order of the MMA issuer, which waits for the seeds' commits instead of the promotion warps;
+            // turns a stage's row scales into the records that those read (they wait for both).
+            constexpr uint32_t idesc = umma_idesc_f16_f32(kBM, BN);
+            const uint64_t desc = umma_desc_k_none(base + G::seed_off, 128, 256);
+            int stage = 0;
+            uint32_t phase = 0, accpar = 0, rec_off = 0;
+            bool ok = true;
+            auto seed_acc = [&](int buf) {
+                ok = warp_wait(bar(G::ACC_EMPTY + buf), (accpar >> buf) & 1u, abort_flag, wait_limit);
+                if (!ok) {
+                    if (lane == 0) report_timeout(p.status, abort_flag, W_ACC_EMPTY);
+                    return;
+                }
+                accpar ^= 1u << buf;
+                if (SEED) {
                     tc_fence_after();
-                    mma_f16_ta(tmem_base + (uint32_t)(buf * BN), tmem_base + (uint32_t)(kAccBufs * BN), desc, idesc, 0u);
-                    tc_commit(bar(G::ACC_SEEDED + buf));
-                };
-                for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-                    int tile, slot, ks0, ks1;
-                    item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
+                    if (elect_one()) {
+                        mma_f16_ta(tmem_base + (uint32_t)(buf * BN), tmem_base + (uint32_t)(kAccBufs * BN), desc, idesc, 0u);
+                        tc_commit(bar(G::ACC_SEEDED + buf));
+                    }
+                    __syncwarp();
+                }
+            };
+            int ahead = 0;                    // blocks whose accumulators are seeded already
+            for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+                int tile, slot, ks0, ks1;
+                item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
+                if (item == (int)blockIdx.x) {
+                    // all accumulators are free: seeded while the first operands are on their way
                     const int blocks = (ks1 - ks0) * G::BPS;
-                    for (int j = 0; j < blocks && ok; j += kAccBufs)
+                    for (; ahead < kAccBufs && ahead < blocks && ok; ++ahead) seed_acc(ahead);
+                }
+                int buf = 0;
+                for (int ks = ks0; ks < ks1 && ok; ++ks) {
+                    if (kScales) {
+                        ok = warp_wait(bar(G::FULL_AB + stage), phase, abort_flag, wait_limit);
+                        if (!ok) {
+                            if (lane == 0) report_timeout(p.status, abort_flag, W_FULL_AB);
+                            break;
+                        }
 #pragma unroll
-                        for (int b = 0; b < kAccBufs; ++b)
-                            if (j + b < blocks && ok) seed_acc(b);
+                        for (int blk = 0; blk < G::BPS; ++blk) {
+                            uint32_t v[4], r[8];
+                            lds_v4(base + G::sa_off + (uint32_t)stage * G::SA_STAGE + (uint32_t)(blk * kBM * 4 + lane * 16), v[0], v[1], v[2], v[3]);
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                float sxd = __fmul_rn(__uint_as_float(v[u]), 1.0f / (127.0f * 127.0f));
+                                if (SEED) sxd = __uint_as_float((__float_as_uint(sxd) + 2u) & 0xFFFFFFFCu);     // 22 significant bits
+                                r[2 * u] = __float_as_uint(sxd);
+                                r[2 * u + 1] = __float_as_uint(-__fmul_rn(kSeedF, sxd));                         // exact
+                            }
+                            const uint32_t dst = base + G::row_off + rec_off + (uint32_t)lane * 32u;
+                            sts_v4(dst, r[0], r[1], r[2], r[3]);
+                            sts_v4(dst + 16u, r[4], r[5], r[6], r[7]);
+                            rec_off += G::ROW_REC;
+                            if (rec_off == G::ROW_RING) rec_off = 0;
+                        }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar(G::EMPTY_AB + stage));
+                        if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                    }
+#pragma unroll 1
+                    for (int blk = 0; blk < G::BPS && ok; ++blk) {
+                        if (ahead > 0) --ahead;
+                        else seed_acc(buf);
+                        if (kScales && ok && lane == 0) mbar_arrive(bar(G::ACC_FULL + buf));
+                        if (++buf == kAccBufs) buf = 0;
+                    }
                 }
             }
-            __syncwarp();
         } else if (warp == 3 && MODE == 0 && OUT != kSplit && OUT != kCluster && p.ksplit == 1 && store != kOwn && !wide) {
             // ---------------- storer ----------------
             uint32_t par = 0;
@@ -744,14 +818,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         setmaxnreg_inc<C::EPI_REGS>();
         const int quarter = warp & 3;                     // tensor-memory lanes 32*quarter .. +31 belong to this warp
         const int slice = (warp - kRoleWarps) >> 2;       // columns COLS*slice .. of the tile
-        const int row = quarter * 32 + lane;
+        // A warp reads its 32 x 40 part of an accumulator in two halves of 16 rows, in the shape in which a thread gets the columns 2*c4 and
+        // 2*c4 + 1 of every eight and the rows g and g + 8 of each half: rows 8*r + g, r 0 .. 3.  One scale pair then serves four rows.
+        const uint32_t g = (uint32_t)lane >> 2, c4 = (uint32_t)lane & 3u;
         const uint32_t t_lane = keep(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(slice * COLS));
-        // shared addresses of this thread's row scale and of its first column scale in scale stage 0, block 0
-        const uint32_t sa_addr = keep(base + C::scale_off + (uint32_t)(row * 4));
-        const uint32_t sw_addr = keep(base + G::sb_off + (uint32_t)(slice * COLS * 4));
+        // shared addresses of this thread's first row record and of its first pair of column scales in the rings
+        const uint32_t row_addr = keep(base + G::row_off + ((uint32_t)(quarter * 32) + g) * 8u);
+        const uint32_t sw_addr = keep(base + G::sb_off + (uint32_t)(slice * COLS * 4) + c4 * 8u);
         const uint32_t bar0 = keep(bars);
         const uint32_t leader = keep(lane == 0 ? 1u : 0u);
-        const float div = 1.0f / (127.0f * 127.0f);
         if (SEED && slice == 0) {
             // A of the seeding MMAs: the same rows as B's, in eight spare tensor-memory columns
             static_assert(kAccBufs * BN + 8 <= 512, "no spare tensor-memory columns");
@@ -766,14 +841,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int b = 0; b < kAccBufs; ++b) mbar_arrive(bar(G::ACC_EMPTY + b));
         }
         uint32_t accpar[kAccBufs] = {0u, 0u, 0u};   // barrier parities of the three accumulators, flipped with every use
-        uint32_t sc_off = 0;                      // byte offset of the block's records in the scale rings
+        uint32_t sc_off = 0, rec_off = 0;         // byte offsets of the block's records in the rings
         bool ok = true;
         uint32_t out_par = 1u;                    // staging area: parity of the release before the tile
         int fail_code = 0;
 
-        // the tile's COLS fp32 accumulators of this thread, kept as packed pairs for fma.rn.f32x2
+        // the tile's COLS fp32 accumulators of this thread, kept as packed pairs for fma.rn.f32x2: pair 4*k + r has the columns 8*k + 2*c4, + 1
+        // of row 8*r + g
         uint64_t acc2[COLS / 2];
-        int m = 0, nbase = 0;
+        int m = 0, nbase = 0;                     // first row of the quarter, first column of the slice
 
         // Promotion of block j, which lies in accumulator `buf_tag`.
         auto promote_block = [&](auto buf_tag, int j) {
@@ -792,8 +868,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     uint32_t pv[8];
                     tmem_ld8(t_acc + (uint32_t)(c * 8), pv);
                     tmem_wait_ld();
-                    if (m < p.M && j < p.nb) {
-                        int32_t* dst = p.partials + ((int64_t)j * p.M + m) * p.N + nbase + c * 8;
+                    if (m + lane < p.M && j < p.nb) {
+                        int32_t* dst = p.partials + ((int64_t)j * p.M + m + lane) * p.N + nbase + c * 8;
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
                             if (nbase + c * 8 + i < p.N)
@@ -804,29 +880,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 __syncwarp();
                 if (leader) mbar_arrive(bar0 + 8u * (uint32_t)(G::ACC_EMPTY + buf));
             } else {
-                uint32_t S[2][CH];
-                tmem_ld8(t_acc, S[0]);
-                // the row's scale, while the read of the first columns is in flight
-                float sxd = __fmul_rn(lds_f32(sa_addr + sc_off), div);
-                float negc = 0.0f;
-                if (SEED) {
-                    sxd = __uint_as_float((__float_as_uint(sxd) + 2u) & 0xFFFFFFFCu);   // 22 significant bits
-                    negc = -__fmul_rn(kSeedF, sxd);                                      // exact
+                // the first eight columns, then the other 32 while those are folded; the accumulator is free when all are in registers
+                uint32_t W0[8], W1[4 * COLS / 4 - 8];
+                tmem_ld_16x256<8>(t_acc, W0);
+                // the rows' records, while the read is in flight
+                uint64_t s2[4], n2[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    float sr, nr;
+                    lds_pair(row_addr + rec_off + (uint32_t)(r * 64), sr, nr);
+                    s2[r] = pack_f32x2(sr, sr);
+                    n2[r] = pack_f32x2(nr, nr);
                 }
                 const uint32_t sw = sw_addr + sc_off;
-#pragma unroll
-                for (int c = 0; c < COLS / CH; ++c) {
-                    tmem_wait_ld();
-                    if (c + 1 < COLS / CH) {
-                        tmem_ld8(t_acc + (uint32_t)((c + 1) * CH), S[(c + 1) & 1]);
-                    } else {
-                        // all of the accumulator is in registers
-                        tc_fence_before();
-                        __syncwarp();
-                        if (leader) mbar_arrive(bar0 + 8u * (uint32_t)(G::ACC_EMPTY + buf));
-                    }
-                    fold_columns<SEED, CH, COLS>(c * CH, S[c & 1], sw, sxd, negc, acc2);
-                }
+                tmem_wait_ld();
+                tmem_ld_16x256<COLS - 8>(t_acc + 8u, W1);
+                fold_columns<SEED, 8, 0, COLS>(W0, sw, s2, n2, acc2);
+                tmem_wait_ld();
+                tc_fence_before();
+                __syncwarp();
+                if (leader) mbar_arrive(bar0 + 8u * (uint32_t)(G::ACC_EMPTY + buf));
+                fold_columns<SEED, COLS - 8, 8, COLS>(W1, sw, s2, n2, acc2);
+                rec_off += G::ROW_REC;
+                if (rec_off == G::ROW_RING) rec_off = 0;
                 sc_off += G::SC_REC;
                 if (sc_off == G::SC_RING) sc_off = 0;
             }
@@ -836,8 +912,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int tile, slot, ks0, ks1, m0, n0;
             item_range<OUT>(item, p, nks, tile, slot, ks0, ks1);
             tile_coords<BN>(tile, p, m0, n0);
-            m = m0 + row;
+            m = m0 + quarter * 32;
             nbase = n0 + slice * COLS;
+            if (addends && p.bias != nullptr) {
+                // into L1, where the epilogue finds it (40 cycles instead of 700)
+                touch_bias(p, nbase + lane);
+                touch_bias(p, nbase + lane + 32 < nbase + COLS ? nbase + lane + 32 : nbase + lane);
+            }
 #pragma unroll
             for (int i = 0; i < COLS / 2; ++i) acc2[i] = 0ull;
 
@@ -938,9 +1019,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     out_par ^= 1u;
                 }
                 const uint32_t part = OUT == kCluster ? out + (w / (uint32_t)p.ksplit) * ((uint32_t)p.ksplit - 1u) * G::RX_BYTES : out + w * G::PART_BYTES, my_row = part + ln * G::PART_ROW;
+                const uint32_t gg = ln >> 2, cc = ln & 3u;
                 if (!wide) {
+                    const bool bf = p.out_dtype == BI8_BF16;
                     uint32_t e[COLS / 2];
-                    if (p.out_dtype == BI8_BF16) {
+                    if (bf) {
 #pragma unroll
                         for (int i = 0; i < COLS / 2; ++i) {
                             float lo, hi;
@@ -955,19 +1038,42 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             e[i] = pack_f16x2(lo, hi);
                         }
                     }
+                    if (addends && p.bias != nullptr) {
+                        uint32_t b[COLS / 8];
+#pragma unroll
+                        for (int k = 0; k < COLS / 8; ++k) {
+                            float lo, hi;
+                            bias_pair(p, nbase + 8 * k + 2 * (int)cc, lo, hi);
+                            b[k] = bf ? pack_bf16x2(lo, hi) : pack_f16x2(lo, hi);
+                        }
+#pragma unroll
+                        for (int i = 0; i < COLS / 2; ++i) e[i] = add_pair(e[i], b[i / 4], bf);
+                    }
                     const bool own = store == kOwn || (OUT == kRows16 && nbase - (int)sl * COLS + BN > p.N);
                     if (OUT == kRows16 && !own) {
-                        stage_row<G::BODY>(out + (ln & 7u) * G::CLASS_BYTES + (qt * 4u + (ln >> 3)) * G::BODY, out + G::EDGES + (qt * 32u + ln) * 32u, sl,
-                                           rows_head(p, ln & 7u, nbase - (int)sl * COLS), e);
+                        // four neighbouring lanes exchange: lane cc gets row 8*cc + gg, all columns
+                        uint32_t rowwise[COLS / 2];
+#pragma unroll
+                        for (int k = 0; k < COLS / 8; ++k) {
+                            uint32_t v[4] = {e[4 * k], e[4 * k + 1], e[4 * k + 2], e[4 * k + 3]};
+                            transpose4(v, cc);
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) rowwise[4 * k + u] = v[u];
+                        }
+                        stage_row<G::BODY>(out + gg * G::CLASS_BYTES + (qt * 4u + cc) * G::BODY, out + G::EDGES + (qt * 32u + 8u * cc + gg) * 32u, sl,
+                                           rows_head(p, gg, nbase - (int)sl * COLS), rowwise);
                     } else {
 #pragma unroll
-                        for (int g = 0; g < COLS / 8; ++g) sts_v4(my_row + (uint32_t)(g * 16), e[4 * g], e[4 * g + 1], e[4 * g + 2], e[4 * g + 3]);
-                        if (addends) add_staged<COLS>(p, my_row, m, nbase, wide);
+                        for (int i = 0; i < COLS / 2; ++i) sts_w(part + (8u * (i & 3) + gg) * G::PART_ROW + (uint32_t)(i / 4) * 16u + cc * 4u, e[i]);
+                        if (addends && p.residual != nullptr) {
+                            __syncwarp();
+                            add_residual<COLS>(p, my_row, m + (int)ln, nbase, wide);
+                        }
                     }
                     __syncwarp();
                     if (own) {
-                        store_own<(int)G::PART_ROW>(static_cast<unsigned char*>(p.C) + ((int64_t)(m - (int)ln) * p.ldc + nbase) * 2, p.ldc * 2, part,
-                                                    p.M - m + (int)ln, p.N - nbase, wide, (int)ln);
+                        store_own<(int)G::PART_ROW>(static_cast<unsigned char*>(p.C) + ((int64_t)m * p.ldc + nbase) * 2, p.ldc * 2, part,
+                                                    p.M - m, p.N - nbase, wide, (int)ln);
                         __syncwarp();
                     }
                     if (OUT == kCluster) {
@@ -983,24 +1089,42 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         mbar_arrive(bar0 + 8u * (uint32_t)G::OUT_FULL);
                     }
                 } else {
+                    if (p.bias != nullptr) {
+#pragma unroll
+                        for (int k = 0; k < COLS / 8; ++k) {
+                            float b0, b1;
+                            bias_pair(p, nbase + 8 * k + 2 * (int)cc, b0, b1);
+#pragma unroll
+                            for (int r = 0; r < 4; ++r) {
+                                float lo, hi;
+                                unpack_f32x2(acc2[4 * k + r], lo, hi);
+                                acc2[4 * k + r] = pack_f32x2(__fadd_rn(lo, b0), __fadd_rn(hi, b1));
+                            }
+                        }
+                    }
 #pragma unroll 1
                     for (int h = 0; h < 2; ++h) {
-                        const int col0 = nbase + h * (COLS / 2), row0 = m - (int)ln;
+                        const int col0 = nbase + h * (COLS / 2), row0 = m;
                         // the previous TMA store must have read the part before it is written again
                         if (store == kTma && ln == 0) tma_store_wait_read();
                         __syncwarp();
+                        // groups of eight columns 0 .. 2, then 2 .. 4; the third has columns of both halves
+                        static_assert(COLS == 40, "two halves of two and a half groups of eight columns");
 #pragma unroll
-                        for (int g = 0; g < COLS / 8; ++g) {
-                            float v[4];
-                            unpack_f32x2(acc2[2 * g], v[0], v[1]);
-                            unpack_f32x2(acc2[2 * g + 1], v[2], v[3]);
-                            sts_v4(my_row + (uint32_t)(g * 16), __float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]),
-                                   __float_as_uint(v[3]));
+                        for (int k = 0; k < 3; ++k) {
+                            const int c = 8 * k + 2 * (int)cc - 4 * h;
+                            if (c >= 0 && c < COLS / 2) {
+#pragma unroll
+                                for (int r = 0; r < 4; ++r) sts_b64(part + (8u * r + gg) * G::PART_ROW + (uint32_t)c * 4u, acc2[4 * k + r]);
+                            }
                         }
-                        // the second half finds its columns where the first found its own
+                        // the second half finds its groups where the first found its own
 #pragma unroll
-                        for (int i = 0; i < COLS / 4; ++i) acc2[i] = acc2[i + COLS / 4];
-                        if (addends) add_staged<COLS>(p, my_row, m, col0, wide);
+                        for (int i = 0; i < 12; ++i) acc2[i] = acc2[i + 8];
+                        if (p.residual != nullptr) {
+                            __syncwarp();
+                            add_residual<COLS>(p, my_row, m + (int)ln, col0, wide);
+                        }
                         if (store == kTma) {
                             fence_proxy_async_smem();
                             __syncwarp();
@@ -1041,9 +1165,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 }
 
 // Reduction of the divided tiles: C[m,n] = cast(sum over the tile's parts) (+ cast(bias[n])) (+ residual[m,n]), the parts added
-// in ascending order, so that the result does not depend on scheduling.  A thread takes eight consecutive columns of
-// a row: one 32-byte sector of every part (NP parts in flight: no more registers than the parts
-// need; four neighbouring threads take the four rows of a 128-byte line), one 16-byte store (two for fp32) where C allows it.
+// in ascending order, so that the result does not depend on scheduling.  A thread adds what one thread of the GEMM has left, one 32-byte
+// sector of every part (NP parts in flight: no more registers than the parts need): two columns of four rows.  Four neighbouring threads
+// exchange their sums, so that each has eight consecutive columns of a row: one 16-byte store (two for fp32) where C allows it.
 // The parts come from L2 where they are few (one slot per SM, 12 MB, for outputs of few tiles) and in part from DRAM where they are
 // kSplitBytes.  Launched as a programmatic dependent of the GEMM:
 // its CTAs are resident as the GEMM's leave.
@@ -1052,36 +1176,48 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const TcParams p) {
     after_predecessor();
     constexpr int GROUPS = BN / 8;                       // groups of eight columns in a tile row
     const int item = blockIdx.x * 256 + threadIdx.x;
+    static_assert(kBM * GROUPS % 32 == 0, "a warp works on one tile");
     const int t = item / (kBM * GROUPS), rem = item - t * (kBM * GROUPS);
     const int rb = rem / (GROUPS * 4), x = rem - rb * (GROUPS * 4);
-    const int r = rb * 4 + (x & 3), cg = x >> 2;         // four consecutive threads: the four rows of a 128-byte line of a part
+    const int quarter = rb >> 3, g = rb & 7, c = x & 3, cg = x >> 2;         // four neighbouring threads: c 0 .. 3
     if (t >= p.tiles_m * p.tiles_n) return;
     int m0, n0;
     tile_coords<BN>(t, p, m0, n0);
-    const int m = m0 + r, n = n0 + cg * 8;
-    if (m >= p.M || n >= p.N) return;
+    const int m = m0 + quarter * 32 + 8 * c + g, n = n0 + cg * 8;            // after the exchange
     const int slice = cg / (COLS / 8), group = cg - slice * (COLS / 8);
-    const float* src = p.ws + (int64_t)t * p.ksplit * p.slot_floats + ws_index<COLS>(r / 32, slice, group, r & 31);
+    const float* src = p.ws + (int64_t)t * p.ksplit * p.slot_floats + ws_index<COLS>(quarter, slice, group, 4 * g + c);
+    // (a quarter without rows has no place in the slots; the same for all four)
+    const bool there = quarter * 32 * BN < p.slot_floats && n < p.N, mine = there && m < p.M;
     const int live = p.N - n < 8 ? p.N - n : 8;
     const int64_t o = (int64_t)m * p.ldc + n, ro = (int64_t)m * p.ldr + n;
     float acc[8], bias[8], res[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) acc[u] = bias[u] = res[u] = 0.0f;
     const bool has_bias = p.bias != nullptr, has_res = p.residual != nullptr;
-    if (has_bias) load8_as_f32(bias, p.bias, p.bias_dtype, n, live);
-    if (has_res) load8_as_f32(res, p.residual, p.out_dtype, ro, live);
-    for (int s0 = 0; s0 < p.ksplit; s0 += NP) {
-        float v[NP][8];
+    if (has_bias && mine) load8_as_f32(bias, p.bias, p.bias_dtype, n, live);
+    if (has_res && mine) load8_as_f32(res, p.residual, p.out_dtype, ro, live);
+    if (there) {
+        for (int s0 = 0; s0 < p.ksplit; s0 += NP) {
+            float v[NP][8];
 #pragma unroll
-        for (int q = 0; q < NP; ++q)
-            if (s0 + q < p.ksplit) ldcg_v8(v[q], src + (int64_t)(s0 + q) * p.slot_floats);
+            for (int q = 0; q < NP; ++q)
+                if (s0 + q < p.ksplit) ldcg_v8(v[q], src + (int64_t)(s0 + q) * p.slot_floats);
 #pragma unroll
-        for (int q = 0; q < NP; ++q)
-            if (s0 + q < p.ksplit) {
+            for (int q = 0; q < NP; ++q)
+                if (s0 + q < p.ksplit) {
 #pragma unroll
-                for (int u = 0; u < 8; ++u) acc[u] = __fadd_rn(acc[u], v[q][u]);
-            }
+                    for (int u = 0; u < 8; ++u) acc[u] = __fadd_rn(acc[u], v[q][u]);
+                }
+        }
     }
+    __syncwarp();
+    uint64_t pairs[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) pairs[u] = pack_f32x2(acc[2 * u], acc[2 * u + 1]);
+    transpose4(pairs, (uint32_t)c);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) unpack_f32x2(pairs[u], acc[2 * u], acc[2 * u + 1]);
+    if (!mine) return;
     if (p.out_dtype == BI8_F32) {
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -1433,7 +1569,7 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
     tm.sa = tm.a;          // stand-ins that are never dereferenced
     tm.sb = tm.b;
     if (tma_sa) {
-        rc = cached_scale_map(&tm.sa, dev, g.sA, nb, g.M, bn, bps);
+        rc = cached_scale_map(&tm.sa, dev, g.sA, nb, g.M, kBM, bps);
         if (rc != BI8_OK) return rc;
     }
     if (tma_sb) {

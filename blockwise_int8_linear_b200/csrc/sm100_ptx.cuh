@@ -43,6 +43,15 @@ __device__ __forceinline__ float lds_f32(uint32_t addr) {
 __device__ __forceinline__ void lds_2xb64(uint32_t addr, uint64_t& a, uint64_t& b) {
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
 }
+__device__ __forceinline__ uint64_t lds_b64(uint32_t addr) {
+    uint64_t v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void lds_pair(uint32_t addr, float& a, float& b) {
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(addr));
+}
+__device__ __forceinline__ void sts_b64(uint32_t addr, uint64_t v) { asm volatile("st.shared.b64 [%0], %1;" ::"r"(addr), "l"(v) : "memory"); }
 __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
@@ -265,6 +274,27 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr)
                  : "memory");
+}
+// 32 lanes x N consecutive columns, half by half of 16 lanes: thread t gets the lanes t/4 and t/4 + 8 of a half and the columns
+// 2*(t%4), + 1 of every eight, as N/8 groups of four words (first lane's pair, second lane's pair) per half.
+template <int N, int OFF = 0, int TOTAL = N>
+__device__ __forceinline__ void tmem_ld_16x256(uint32_t taddr, uint32_t (&r)[TOTAL]) {
+    static_assert(N == 8 || N % 16 == 0, "pieces of 16 columns, or eight");
+    constexpr int P = N == 8 ? 8 : 16;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t* const d = r + h * (TOTAL / 2) + OFF / 2;
+        const uint32_t a = taddr + (uint32_t)(h * (16 << 16)) + (uint32_t)OFF;
+        if constexpr (P == 8) {
+            asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];" : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a) : "memory");
+        } else {
+            asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
+                         : "r"(a)
+                         : "memory");
+        }
+    }
+    if constexpr (N > 16) tmem_ld_16x256<N - 16, OFF + 16, TOTAL>(taddr, r);
 }
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
