@@ -23,9 +23,12 @@
 //               block it reads its part of the finished accumulator, folds the values into fp32 accumulators in registers, and
 //               releases the accumulator as soon as the last columns are in registers.  After the last block of a tile it casts, adds
 //               the bias, stages its 32 x 40 part in shared memory, adds the residual there and goes on with the next tile.
-// What bounds the kernel: at blocks of 32 and 64 the promotion, t = P*s_row and acc += s_col*t for two columns per FFMA2 (the second
-// has three 64-bit operands that change and issues every 3.2 to 3.5 cycles where its scale pair is not reused) next to what the scales
-// cost: every register that a shared-memory load fills takes its time on that pipe, broadcast or not.  As a thread with one row and 40
+// What bounds the kernel: the promotion, t = P*s_row and acc += s_col*t for two columns per FFMA2, and what its warps issue beside it.  A
+// scheduler takes two cycles per FFMA2 and one per other instruction, and its four warps have 80 and about 60 of them per block: 520 cycles
+// (the promotion alone, without MMAs; 372 without the barriers).  MMAs beside it cost another 60 to 70 cycles each: one of M128 N160 K32 reads
+// 9.2 KB of operands in 80 cycles, 90 % of the shared memory's bandwidth, and the loads of the scales wait (552, 602 and 733 cycles a block
+// of 32, 64 and 128; without the loads of scales 604 at 128).  The MMAs and seeds alone take 162, 242 and 402.  Every register that a
+// shared-memory load fills takes its time on that pipe, broadcast or not.  As a thread with one row and 40
 // columns (32x32b reads) a warp loaded 41 scales per block and thread; with four rows and ten columns (16x256b) 4 records and 10 scales,
 // each scale pair of the columns used for four rows in turn.  Row scales are prepared once per CTA by the seeder, not by every
 // thread for its four rows.  At 128 the operands' way from L2 (64 bytes per cycle and SM, 576 cycles per 128 x 160 x 128) bounds as well.
@@ -33,6 +36,11 @@
 // issuer as a loop of its warp, the same box); a lab loop without epilogue 683 -> 535, 731 -> 569 and 611 -> 535 cycles a block.
 // Reading 8 + 32 columns at a time, the accumulator is free early and the first fold hides the second read: in that loop 527 cycles
 // against 548 for all at once, 536 for 16 + 24, 636 for five times eight.
+// The release of an accumulator is one predicated arrival (a branch around it: 577 cycles a block, 538 so), and the issuer tests a stage and its first
+// accumulator at once: sustained 681 -> 672 us at block 64, 1182 -> 1160 at 32, 240 = 240 for 2048 x 4096 x 22016 at 128.
+// Slower: the next block's words, or words and scales, requested behind this block's folds (649 us cold at block 64 against 614); records of 16 bytes
+// that need no moves (655 cycles against 561) or of 4 bytes (591); two wide warps per quarter with everything requested a block ahead (660 cycles
+// against 602); row records by the storer or the producer (613 to 900 us against 601).
 //
 // Registers: a scheduler (SM sub-partition) owns a quarter of the register file and every fourth warp, and setmaxnreg can
 // only move registers between warps of the same scheduler.  Each scheduler has exactly one of warps 0-3, which shrinks,
@@ -178,9 +186,9 @@ struct Geo {
     // kRows: [8 rows modulo 8][16] bodies of 304 bytes, then per row the first and the last eight elements
     static constexpr uint32_t BODY = C::BN * 2 - 16, CLASS_BYTES = kBM / 8 * BODY, EDGES = 8 * CLASS_BYTES;
     static constexpr uint32_t OUT_BYTES = EDGES + kBM * 32;
-    // operand B of the seeding MMAs: 16 fp16 values per row as 8-row core matrices
+    // operand B of the seeding MMAs: 16 fp16 values per row, the same eight rows (two core matrices) for all of them
     static constexpr uint32_t seed_off = (misc_off + 16 + 127) & ~127u;
-    static constexpr uint32_t SEED_BYTES = C::BN * 32;
+    static constexpr uint32_t SEED_BYTES = 256;
     // kCluster: what a warp has of a tile, in fp32; a warp that finishes its part receives one from every other CTA, and stages there
     static constexpr uint32_t RX_BYTES = 32 * C::COLS * 4;
     static constexpr uint32_t out_off = seed_off + SEED_BYTES;
@@ -664,17 +672,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 bool ok = true;
                 auto issue_stage = [&](auto rot_tag) {
                     constexpr int ROT = decltype(rot_tag)::value;
-                    ok = mbar_wait(bar(G::FULL_AB + stage), phase, abort_flag, wait_limit_mma);
-                    if (!ok) {
-                        report_timeout(p.status, abort_flag, W_FULL_AB);
-                        return;
+                    // a test takes about 80 cycles: those of the stage and of its first accumulator go out together
+                    constexpr int buf0 = RotInfo<G::BPS>::buf(ROT, 0), acc_bar = SEED ? G::ACC_SEEDED : G::ACC_EMPTY;
+                    const bool full = mbar_test(bar(G::FULL_AB + stage), phase), acc0 = mbar_test(bar(acc_bar + buf0), accpar[buf0]);
+                    if (!full) {
+                        ok = mbar_wait(bar(G::FULL_AB + stage), phase, abort_flag, wait_limit_mma);
+                        if (!ok) {
+                            report_timeout(p.status, abort_flag, W_FULL_AB);
+                            return;
+                        }
                     }
                     const uint64_t adesc = umma_desc_k_sw128(base + C::a_off(stage));
                     const uint64_t bdesc = umma_desc_k_sw128(base + C::b_off(stage));
 #pragma unroll
                     for (int blk = 0; blk < G::BPS; ++blk) {
                         const int buf = RotInfo<G::BPS>::buf(ROT, blk);
-                        ok = mbar_wait(bar((SEED ? G::ACC_SEEDED : G::ACC_EMPTY) + buf), accpar[buf], abort_flag, wait_limit_mma);
+                        if (blk > 0 || !acc0) ok = mbar_wait(bar(acc_bar + buf), accpar[buf], abort_flag, wait_limit_mma);
                         if (!ok) {
                             report_timeout(p.status, abort_flag, W_ACC_EMPTY);
                             return;
@@ -707,7 +720,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             // Follows the accumulators in the order of the MMA issuer, which waits for the seeds' commits instead of the promotion warps;
             // turns a stage's row scales into the records that those read (they wait for both).
             constexpr uint32_t idesc = umma_idesc_f16_f32(kBM, BN);
-            const uint64_t desc = umma_desc_k_none(base + G::seed_off, 128, 256);
+            const uint64_t desc = umma_desc_k_none(base + G::seed_off, 128, 0);
             int stage = 0;
             uint32_t phase = 0, accpar = 0, rec_off = 0;
             bool ok = true;
@@ -878,7 +891,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (leader) mbar_arrive(bar0 + 8u * (uint32_t)(G::ACC_EMPTY + buf));
+                mbar_arrive_if(bar0 + 8u * (uint32_t)(G::ACC_EMPTY + buf), leader);
             } else {
                 // the first eight columns, then the other 32 while those are folded; the accumulator is free when all are in registers
                 uint32_t W0[8], W1[4 * COLS / 4 - 8];
@@ -899,7 +912,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 tmem_wait_ld();
                 tc_fence_before();
                 __syncwarp();
-                if (leader) mbar_arrive(bar0 + 8u * (uint32_t)(G::ACC_EMPTY + buf));
+                mbar_arrive_if(bar0 + 8u * (uint32_t)(G::ACC_EMPTY + buf), leader);
                 fold_columns<SEED, COLS - 8, 8, COLS>(W1, sw, s2, n2, acc2);
                 rec_off += G::ROW_REC;
                 if (rec_off == G::ROW_RING) rec_off = 0;
