@@ -24,7 +24,7 @@
 //               releases the accumulator as soon as the last columns are in registers.  After the last block of a tile it casts, adds
 //               the bias, stages its 32 x 40 part in shared memory, adds the residual there and goes on with the next tile.
 // What bounds the kernel: the promotion, t = P*s_row and acc += s_col*t for two columns per FFMA2, and what its warps issue beside it.  A
-// scheduler takes two cycles per FFMA2 and one per other instruction, and its four warps have 80 and about 60 of them per block: 520 cycles
+// scheduler takes two cycles per FFMA2 and one per other instruction, and each of its four warps has 40 and about 60 of them per block: 520 cycles
 // (the promotion alone, without MMAs; 372 without the barriers).  MMAs beside it cost another 60 to 70 cycles each: one of M128 N160 K32 reads
 // 9.2 KB of operands in 80 cycles, 90 % of the shared memory's bandwidth, and the loads of the scales wait (552, 602 and 733 cycles a block
 // of 32, 64 and 128; without the loads of scales 604 at 128).  The MMAs and seeds alone take 162, 242 and 402.  Every register that a
@@ -38,7 +38,8 @@
 // against 548 for all at once, 536 for 16 + 24, 636 for five times eight.
 // The release of an accumulator is one predicated arrival (a branch around it: 577 cycles a block, 538 so), and the issuer tests a stage and its first
 // accumulator at once: sustained 681 -> 672 us at block 64, 1182 -> 1160 at 32, 240 = 240 for 2048 x 4096 x 22016 at 128.
-// Slower: the next block's words, or words and scales, requested behind this block's folds (649 us cold at block 64 against 614); records of 16 bytes
+// One read for 32 columns of a half instead of two: 672.8 -> 670.5 us, 1175 -> 1168; 8192 x 768 x 50257 779.5 -> 772.5.
+// Slower: a loop of whole cycles of three blocks with the rest behind it (8192 x 768 x 50257 777 -> 804, though fp32 4096^3 146 -> 141); the next block's words, or words and scales, requested behind this block's folds (649 us cold at block 64 against 614); records of 16 bytes
 // that need no moves (655 cycles against 561) or of 4 bytes (591); two wide warps per quarter with everything requested a block ahead (660 cycles
 // against 602); row records by the storer or the producer (613 to 900 us against 601).
 //

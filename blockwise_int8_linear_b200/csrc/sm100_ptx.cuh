@@ -281,24 +281,23 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
 }
 // 32 lanes x N consecutive columns, half by half of 16 lanes: thread t gets the lanes t/4 and t/4 + 8 of a half and the columns
 // 2*(t%4), + 1 of every eight, as N/8 groups of four words (first lane's pair, second lane's pair) per half.
-template <int N, int OFF = 0, int TOTAL = N>
-__device__ __forceinline__ void tmem_ld_16x256(uint32_t taddr, uint32_t (&r)[TOTAL]) {
-    static_assert(N == 8 || N % 16 == 0, "pieces of 16 columns, or eight");
-    constexpr int P = N == 8 ? 8 : 16;
+template <int N>
+__device__ __forceinline__ void tmem_ld_16x256(uint32_t taddr, uint32_t (&r)[N]) {
+    static_assert(N == 8 || N == 32, "one read per half");
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        uint32_t* const d = r + h * (TOTAL / 2) + OFF / 2;
-        const uint32_t a = taddr + (uint32_t)(h * (16 << 16)) + (uint32_t)OFF;
-        if constexpr (P == 8) {
+        uint32_t* const d = r + h * (N / 2);
+        const uint32_t a = taddr + (uint32_t)(h * (16 << 16));
+        if constexpr (N == 8) {
             asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];" : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a) : "memory");
         } else {
-            asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
+            asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]), "=r"(d[9]), "=r"(d[10]),
+                           "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
                          : "r"(a)
                          : "memory");
         }
     }
-    if constexpr (N > 16) tmem_ld_16x256<N - 16, OFF + 16, TOTAL>(taddr, r);
 }
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
