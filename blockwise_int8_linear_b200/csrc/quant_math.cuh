@@ -15,14 +15,31 @@ constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to intege
 // e is exact, q0 + e/b is the exact quotient, and the quotient of two such short operands is either
 // representable or at least 2^-13 ulp away from a rounding boundary, far more than the error of e*r.
 // For fp32 operands, and for scales outside [2^-100, 2^100], the IEEE division is used directly.
+//
+// `once`: the byte needs no quotient.  With X and S the significands of x and the scale as integers below 2^11 and 2^k the ratio of their
+// units, 127 x / s lies at least 2^-19 of its value away from every n + 1/2 that it does not equal: |254 X 2^k - (2n + 1) S| is an integer, or
+// one divided by 2^-k, and 254 X < 2^19.  Both fl(127 fl(x / s)) (off by less than 2^-23 of its value) and x * r, r within 2^-21 above 127 / s,
+// then round to the same integer.  Equality, 254 X 2^k = (2n + 1) S, asks for a factor of 127 on the right.  In 2n + 1: n = 63 and
+// x = s / 2, where the quotient is exact and 63.5 goes to 64, as does x * r, which is 63.5 or more.  Or in S, the scale's 11 significant bits a
+// multiple of 127: there fl(127 fl(x / s)) goes to the even neighbour (all pairs of 11-bit numbers tried), and x * r does too where 127 / s is a
+// power of two and r exactly that (S = 2032, the only such bf16 scale); the other seven fp16 ones have no `once`.  One fused operation replaces
+// five, which at two issue cycles a packed pair were most of the tile quantizer; taken there and in the streaming row-wise kernel, not where
+// fp16 would need the code of both (rows of any alignment, 8192 x 12289: 98.4 us without, 100.4 with) or few values are quantized.
 struct BlockQ {
     float scale;
     float rcp;
-    bool fast;
+    bool fast, once;
     __device__ __forceinline__ void set(float amax, bool short_mantissa) {
         scale = amax;
         fast = short_mantissa && amax > 7.8886090522101181e-31f && amax < 1.2676506002282294e30f;
         rcp = fast ? __frcp_rn(amax) : 0.0f;
+        const uint32_t sig = significand();
+        once = fast && (sig == 2032u || sig % 127u != 0u);
+    }
+    __device__ __forceinline__ uint32_t significand() const { return ((__float_as_uint(scale) >> 13) & 0x3ffu) | 0x400u; }
+    // 127 / scale, too large by less than 2^-21 of it and never too small, or exact (computed where it is used: not kept beside rcp)
+    __device__ __forceinline__ float r127() const {
+        return significand() == 2032u ? __fmul_rn(127.0f, rcp) : __fmul_ru(__fmul_ru(127.0f, rcp), 1.00000011920928955f);
     }
     // returns fl32(127 * fl32(x / scale)) + magic, whose low byte is the int8 result
     __device__ __forceinline__ uint32_t q(float x) const {

@@ -268,7 +268,19 @@ __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
             BlockQ bq;
             bq.set(amax, true);
             uint32_t out[4];
-            if (bq.fast) {
+            // bf16: `once` is `fast`; fp16 keeps the five operations
+            constexpr bool ONCE = std::is_same_v<T, __nv_bfloat16>;
+            if (ONCE && bq.once) {
+                const float r = bq.r127();
+                const uint64_t r2 = f2_pack(r, r);
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    uint32_t b0, b1, b2, b3;
+                    f2_bits(f2_fma(v2[2 * w], r2, cmagic), b0, b1);
+                    f2_bits(f2_fma(v2[2 * w + 1], r2, cmagic), b2, b3);
+                    out[w] = pack4(b0, b1, b2, b3);
+                }
+            } else if (!ONCE && bq.fast) {
                 const uint64_t r2 = f2_pack(bq.rcp, bq.rcp), ns2 = f2_pack(-amax, -amax);
 #pragma unroll
                 for (int w = 0; w < 4; ++w) {

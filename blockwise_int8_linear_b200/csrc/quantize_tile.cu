@@ -14,7 +14,9 @@
 //     the 16 rows of a tile that are equal modulo 8, 136 columns from the 16-byte boundary at or before the tile's first.
 //     The threads shift what they read by the class's offset, which is a constant for the column-wise role's unrolled
 //     rows and, with a warp per class, for a whole warp of the row-wise role.  8192 x 50257: dual 494 -> 399 us (345 with aligned
-//     rows), column-wise 488 -> 224 (225).
+//     rows), column-wise 488 -> 224 (225); with one operation per pair (quant_math.cuh) dual 358, and 8192 x 8192, aligned, 63.5 -> 57.3,
+//     8192 x 3072 30.7 -> 26.6.  What is left is the rest of the instructions: with twice the threads and half the words for each (64 registers, no
+//     spills) every one of those times was a tenth longer.
 //     Where the number of rows is not a multiple of 8 (kShift) all threads fetch: a half-warp reads a tile row as aligned
 //     16-byte pieces, shifts the bytes into place between neighbouring lanes and stores them where the TMA would have put
 //     them.  The loads of the next tile are in flight, in registers, while the current one is quantized.  (A zero-padded
@@ -102,25 +104,26 @@ struct Pk<__half> {
 };
 
 // Quantizer of a pair of values with (possibly different) block scales, on packed fp32 pairs.  The same operations, in
-// the same order and each rounded on its own, as BlockQ::q: q0 = x*r, e = fma(-s, q0, x), y = fma(e, r, q0),
+// the same order and each rounded on its own, as BlockQ::q: kOnce fma(x, r127, magic); kFast q0 = x*r, e = fma(-s, q0, x), y = fma(e, r, q0),
 // z = 127*y, z + magic (written as fma(z, 1, magic) so that the multiply cannot be contracted into the addition).
+enum QuantWay { kOnce = 0, kFast = 1, kDivide = 2 };
 struct PairQ {
     BlockQ lo, hi;
-    uint64_t r2, ns2;
-    bool fast;
+    bool fast, once;
     __device__ __forceinline__ void set(float amax_lo, float amax_hi) {
         lo.set(amax_lo, true);
         hi.set(amax_hi, true);
         fast = lo.fast && hi.fast;
-        r2 = f2_pack(lo.rcp, hi.rcp);
-        ns2 = f2_pack(-amax_lo, -amax_hi);
+        once = lo.once && hi.once;
     }
-    // FAST is this->fast, tested once by the caller around its whole loop rather than once per pair
-    template <bool FAST>
+    // The way is chosen by the caller around its whole loop (choose) rather than per pair.
+    template <int WAY>
     __device__ __forceinline__ void q(float xlo, float xhi, uint32_t& blo, uint32_t& bhi) const {
-        if (FAST) {
+        if (WAY == kOnce) {
+            f2_bits(f2_fma(f2_pack(xlo, xhi), f2_pack(lo.r127(), hi.r127()), f2_pack(kMagic, kMagic)), blo, bhi);
+        } else if (WAY == kFast) {
             const uint64_t c127 = f2_pack(127.0f, 127.0f), cmagic = f2_pack(kMagic, kMagic), cone = f2_pack(1.0f, 1.0f);
-            const uint64_t v2 = f2_pack(xlo, xhi);
+            const uint64_t v2 = f2_pack(xlo, xhi), r2 = f2_pack(lo.rcp, hi.rcp), ns2 = f2_pack(-lo.scale, -hi.scale);
             const uint64_t q0 = f2_mul(v2, r2);
             const uint64_t e = f2_fma(ns2, q0, v2);
             const uint64_t y = f2_fma(e, r2, q0);
@@ -128,6 +131,20 @@ struct PairQ {
         } else {
             blo = lo.q(xlo);
             bhi = hi.q(xhi);
+        }
+    }
+    // f(the way of this thread's pairs).  bf16: one operation or the division (`once` is `fast`).  fp16: with ONCE one operation where that
+    // holds for the whole warp, because a warp that is divided would do both; the third way's code costs registers, which kShift does not
+    // have (dual, 8190 x 3071: 49 us without, 56 with) and kOct and the column-wise kernel gain nothing from (26.6, 28.7; dual tiles 30.7, 28.7).
+    template <typename T, bool ONCE, typename F>
+    __device__ __forceinline__ void choose(F f) const {
+        if constexpr (std::is_same_v<T, __nv_bfloat16>) {
+            if (once) f(std::integral_constant<int, kOnce>{});
+            else f(std::integral_constant<int, kDivide>{});
+        } else {
+            if (ONCE && __all_sync(0xffffffffu, once)) f(std::integral_constant<int, kOnce>{});
+            else if (fast) f(std::integral_constant<int, kFast>{});
+            else f(std::integral_constant<int, kDivide>{});
         }
     }
 };
@@ -413,8 +430,8 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             const int c = 2 * p;
             float sum_lo = 0.0f, sum_hi = 0.0f;            // SUM: this thread's 32 rows of both columns
             const uint32_t outc = base + L::outc_off;
-            auto quantize_cols = [&](auto fast_tag) {
-                constexpr bool FAST = decltype(fast_tag)::value;
+            auto quantize_cols = [&](auto way_tag) {
+                constexpr int WAY = decltype(way_tag)::value;
 #pragma unroll
                 for (int part = 0; part < 2; ++part) {     // 16 rows = one 16-byte piece of each column's output row
                     uint32_t wl[4], wh[4];
@@ -429,7 +446,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                                 sum_lo += xlo;
                                 sum_hi += xhi;
                             }
-                            pq.template q<FAST>(xlo, xhi, bl[u], bh[u]);
+                            pq.template q<WAY>(xlo, xhi, bl[u], bh[u]);
                         }
                         wl[k] = pack4(bl[0], bl[1], bl[2], bl[3]);
                         wh[k] = pack4(bh[0], bh[1], bh[2], bh[3]);
@@ -438,8 +455,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                     sts_v4(outc + swz(c + 1, g * 2 + part), wh[0], wh[1], wh[2], wh[3]);
                 }
             };
-            if (pq.fast) quantize_cols(std::true_type{});
-            else quantize_cols(std::false_type{});
+            pq.template choose<T, DUAL && IN == kTiled>(quantize_cols);
             // scales [ceil(R/B), C]: the first row group of each block writes the pair
             if ((g % (B / 32)) == 0) {
                 const int rb = r0 + g * 32;
@@ -524,8 +540,8 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             for (int b = 0; b < NBT; ++b) {
                 PairQ pq;
                 pq.set(amax[b], amax[b]);
-                auto quantize_row = [&](auto fast_tag) {
-                    constexpr bool FAST = decltype(fast_tag)::value;
+                auto quantize_row = [&](auto way_tag) {
+                    constexpr int WAY = decltype(way_tag)::value;
 #pragma unroll
                     for (int k = 0; k < 4 / NBT; ++k) {
                         uint32_t wd[4];
@@ -536,15 +552,14 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                             uint32_t b0, b1, b2, b3;
                             Pk<T>::unpack(v[i], x0, x1);
                             Pk<T>::unpack(v[i + 1], x2, x3);
-                            pq.template q<FAST>(x0, x1, b0, b1);
-                            pq.template q<FAST>(x2, x3, b2, b3);
+                            pq.template q<WAY>(x0, x1, b0, b1);
+                            pq.template q<WAY>(x2, x3, b2, b3);
                             wd[u] = pack4(b0, b1, b2, b3);
                         }
                         sts_v4(outr + swz(srow, half * 4 + b * (4 / NBT) + k), wd[0], wd[1], wd[2], wd[3]);
                     }
                 };
-                if (pq.fast) quantize_row(std::true_type{});
-                else quantize_row(std::false_type{});
+                pq.template choose<T, DUAL && IN == kTiled>(quantize_row);
             }
             // scales [ceil(C/B), R] (transposed): eight consecutive rows per quarter-warp
             if (r0 + row < R) {

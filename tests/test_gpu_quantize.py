@@ -325,3 +325,37 @@ def test_tensor_map_kernels_from_a_fresh_thread():
     for a, b in zip(want[0], got[0][0]):
         assert torch.equal(a, b)
     assert torch.equal(want[1][0], got[0][1][0]) and torch.equal(want[2], got[0][2])
+
+
+def _all_ratios(dt, scales, shifts):
+    """Rows of blocks of 64: a block holds a scale (significand `scales`, as integer) and values that are all significands times 2**shift, both signs."""
+    bits = 8 if dt == torch.bfloat16 else 11
+    sig = torch.arange(1 << (bits - 1), 1 << bits, dtype=torch.float64)
+    rows = []
+    for s in scales:
+        x = torch.cat([sig * 2.0 ** k for k in shifts])
+        x = x[x <= s]
+        x = torch.where(torch.arange(x.numel()) % 2 == 1, -x, x)
+        x = torch.cat([x, x.new_zeros(-x.numel() % 63)]).reshape(-1, 63)
+        rows.append(torch.cat([x.new_full((x.shape[0], 1), float(s)), x], 1))
+    m = torch.cat(rows) * 2.0 ** (-5 if dt == torch.float16 else -9)
+    out = m.to(dt)
+    assert torch.equal(out.double(), m)
+    return out
+
+
+@pytest.mark.parametrize("dt,scales", [(torch.bfloat16, range(128, 256)), (torch.float16, [127 * m for m in range(9, 17)] + [1024, 1025, 1271, 1600, 2046, 2047])])
+def test_every_ratio_of_short_significands(dt, scales):
+    # quotients that lie on a tie, next to one, and scales that are multiples of 127, through the kernels with ways of their own
+    from triton_functions import quantize_block_dual
+    x = _all_ratios(dt, scales, range(-3, 1))
+    set_config(64, dt)
+    _check_quant(x, 64)                                                     # rows of one block
+    wide = x[: x.shape[0] // 8 * 8].reshape(-1, 512)
+    wide = wide[: wide.shape[0] // 8 * 8].contiguous()
+    _check_quant(wide, 64)
+    for m in (wide, wide.t().contiguous()):
+        qr, sr, qc, sc = quantize_block_dual(m.to(DEV))
+        for got_q, got_s, ref in ((qr, sr, m), (qc, sc, m.t().contiguous())):
+            q_ref, s_ref = O.quantize(ref, 64)
+            assert torch.equal(got_q.cpu(), q_ref) and torch.equal(got_s.cpu(), s_ref)

@@ -1,5 +1,6 @@
 """The CPU restatements against the golden vectors produced by the reference's own kernels
 (tests/golden/make_golden.py), and against each other.  No GPU needed."""
+import numpy as np
 import pytest
 import torch
 
@@ -118,3 +119,27 @@ def test_producer_step_restatements_equal_torch_cpu(dt):
     q, s = O.silu_mul_quantize(x, u, 64)
     q2, s2 = O.quantize(O.silu_mul(x, u), 64)
     assert torch.equal(q, q2) and torch.equal(s, s2)
+
+
+@pytest.mark.parametrize("bits", [8, 11])
+def test_one_fused_operation_gives_the_quotients_byte(bits):
+    """The quantizers' shortcut for bf16 (8 significant bits) and fp16 (11): rint(x * r), r = 127 / s rounded up (exact for the scale 2032), is
+    rint(fl(127 * fl(x / s))) for every pair of significands and every ratio of units down to 2**-10 (below, both are 0), but for scales that are
+    multiples of 127.  127 / s is a product in fp32 as the device computes it; x * r is exact in fp64."""
+    f = np.float32
+    sig = np.arange(1 << (bits - 1), 1 << bits)
+    x = (sig[None, :] * 2.0 ** np.arange(-10, 1)[:, None]).ravel()
+
+    def mul_up(a, b):
+        e = float(a) * float(b)
+        r = f(e)
+        return np.nextafter(r, f(np.inf)) if float(r) < e else r
+
+    for s in sig:
+        s11 = int(s) << (11 - bits)
+        if s11 % 127 == 0 and s11 != 2032:
+            continue
+        rcp = f(1.0) / f(s)
+        r = f(127.0) * rcp if s11 == 2032 else mul_up(mul_up(f(127.0), rcp), f(1.00000011920928955))
+        v = x[x <= s]
+        assert np.array_equal(np.rint(f(127.0) * (v.astype(f) / f(s))), np.rint(v * np.float64(r)))
