@@ -346,7 +346,8 @@ __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
 // Row-wise quantize to int8 rows that are not 8-byte aligned (a dense result whose row length is not a multiple of 8),
 // block <= 64.  A warp takes kRagGroup consecutive blocks of one row; lane l handles elements l and l + 32 of every block, so
 // all loads of the group (2-byte, coalesced) are in flight before the first absmax reduction, and the stores are runs of 32
-// consecutive bytes.  Same arithmetic as every other quantizer (BlockQ).
+// consecutive bytes.  Same arithmetic as every other quantizer (BlockQ).  What bounds it is a warp's chain of reductions: side by side
+// instead of block after block 512 x 4100 takes 9.2 us (11.6), 4001 x 1001 13.9 (17.5), 300 x 777 4.6 (5.8); at block 32, with half the lanes idle, 13.0 (13.9).
 constexpr int kRagGroup = 8;
 template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_rowwise_ragged_kernel(
@@ -358,31 +359,34 @@ __global__ void __launch_bounds__(kThreads) quantize_rowwise_ragged_kernel(
     if (task >= M * groups_per_row) return;
     const int64_t row = task / groups_per_row, j0 = (task % groups_per_row) * kRagGroup;
     const T* xr = x + row * ldx;
-    float v[kRagGroup][2];
+    float v[kRagGroup][2], amax[kRagGroup];
 #pragma unroll
     for (int b = 0; b < kRagGroup; ++b) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int64_t k = (j0 + b) * B + lane + 32 * e;
-            const bool valid = (j0 + b) < nb && lane + 32 * e < B && k < K;
-            v[b][e] = valid ? to_f32<T>(xr[k]) : 0.0f;
+            v[b][e] = (j0 + b < nb && lane + 32 * e < B && k < K) ? to_f32<T>(xr[k]) : 0.0f;
         }
     }
 #pragma unroll
-    for (int b = 0; b < kRagGroup; ++b) {
-        float amax = fmaxf(fabsf(v[b][0]), fabsf(v[b][1]));
+    for (int b = 0; b < kRagGroup; ++b) amax[b] = fmaxf(fabsf(v[b][0]), fabsf(v[b][1]));
+    // the blocks' reductions side by side
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+        for (int b = 0; b < kRagGroup; ++b) amax[b] = fmaxf(amax[b], __shfl_xor_sync(0xffffffffu, amax[b], off));
+#pragma unroll
+    for (int b = 0; b < kRagGroup; ++b) {
         const int64_t j = j0 + b;
-        if (j >= nb) continue;
+        if (j >= nb) break;
         BlockQ bq;
-        bq.set(amax, sizeof(T) == 2);
+        bq.set(amax[b], sizeof(T) == 2);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int64_t k = j * B + lane + 32 * e;
             if (lane + 32 * e < B && k < K) q[row * ldq + k] = (int8_t)(bq.q(v[b][e]) & 0xffu);
         }
-        if (lane == 0) s[j * M + row] = amax;
+        if (lane == 0) s[j * M + row] = amax[b];
     }
 }
 
