@@ -268,9 +268,13 @@ __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
             BlockQ bq;
             bq.set(amax, true);
             uint32_t out[4];
-            // bf16: `once` is `fast`; fp16 keeps the five operations
+            // bf16: `once` is `fast`; fp16 keeps the five operations.  Lanes behind the row's end have a scale of zero in every unit there: they
+            // must not drag the warp through the divisions (3907 x 2688: 19.5 us for quantize and dequantize, 13.9 this way).
             constexpr bool ONCE = std::is_same_v<T, __nv_bfloat16>;
-            if (ONCE && bq.once) {
+            if (ONCE && amax == 0.0f) {
+#pragma unroll
+                for (int w = 0; w < 4; ++w) out[w] = 0u;
+            } else if (ONCE && bq.once) {
                 const float r = bq.r127();
                 const uint64_t r2 = f2_pack(r, r);
 #pragma unroll
@@ -300,6 +304,7 @@ __global__ void __launch_bounds__(kThreads, 2) quantize_rowwise_stream_kernel(
                     out[w] = pack4(b0, b1, b2, b3);
                 }
             } else {
+                if (ONCE) bq.fast = false;            // what is left are divisions
 #pragma unroll
                 for (int w = 0; w < 4; ++w) {
                     uint32_t a0, a1, a2, a3;
