@@ -1381,7 +1381,8 @@ struct SplitPlan {
 };
 // What a work item takes per stage (128 K-bytes of a tile: four, two or one blocks to promote), what dividing costs whatever its size
 // (the second kernel's latency; of its host time a part) and per slot (80 KB written and read again through L2): microseconds.
-// Stage: slope over 4 to 32 stages of 4736 undivided tiles, 1.38 us at block 32, 0.68 at 64, 0.43 at 128.  Checked on a sweep of 1 to 32
+// Stage: slope over 4 to 32 stages of 4736 undivided tiles, 1.38 us at block 32, 0.68 at 64, 0.43 at 128, of the form that the sweep below was made with
+// (8192 x 4096 x 11008 now takes 1.24, 0.62 and 0.41 a stage: the parts of a tile, and with them the association of its sums, stay as they were).  Checked on a sweep of 1 to 32
 // items per tile and clusters of two to four over 23 shapes of 4 to 320 tiles and 6 to 86 stages at the three blocks (GEMM alone in a
 // graph): the plan is within 5 % of the best one everywhere and within 2 % in 62 of 69 (block 32 / 64 / 128, the plan's time
 // and the undivided one's: 512 x 768 x 768 8.9, 12.0 / 8.0, 8.0 / 6.5, 6.5; 300 x 3072 x 768 12.1, 36.9 / 10.1, 20.4 / 9.3, 13.8; furthest off
