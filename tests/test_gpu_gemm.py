@@ -548,3 +548,50 @@ def test_zero_sized():
     b = torch.zeros((256, 128), dtype=torch.int8, device=DEV)
     c = mm(a, b.t(), torch.empty((2, 0), device=DEV), torch.ones((2, 256), device=DEV))
     assert tuple(c.shape) == (0, 256)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("block,stages", [(128, 1), (128, 2), (128, 4), (128, 5), (64, 1), (64, 2), (64, 3), (32, 1), (32, 2)])
+@pytest.mark.parametrize("shape", [
+    # (M, N), 315 tiles on 148 SMs: C by tensor map with scales by tensor map; sA by cp.async; odd rows of C by every eighth row, sB by
+    # cp.async; own stores, both by cp.async
+    (1920, 3360), (1918, 3352), (1920, 3355), (1917, 3355),
+])
+def test_short_items_over_several_rounds(shape, block, stages, dtype):
+    """A CTA goes from tile to tile while the rings of operands, scales, row records and accumulators run on: two or three undivided tiles per CTA
+    of one to five stages (one to ten blocks: fewer than there are accumulators, and numbers that are no multiple of them).  Every row is, bit for bit, that
+    of calls in which no CTA has a second tile; sampled rows are within the tolerance of the oracle; bias and residual are what additions in the output
+    type make of the plain result."""
+    from blockwise_int8_linear_b200 import _lib
+    L = _lib.lib()
+    (m, n), k = shape, 128 * stages
+    chunk = 7 * 128                                    # times 21 tiles of 160 columns: 147 tiles
+    code, p = _lib.dtype_code(dtype), _lib.ptr
+    gen = torch.Generator(device=DEV).manual_seed(m * n + k)
+    a, bt = (torch.randint(-127, 128, (r, k), generator=gen, device=DEV, dtype=torch.int8) for r in (m, n))
+    sa, sb = (torch.rand((k // block, r), generator=gen, device=DEV) * c + c for r, c in ((m, 0.5), (n, 0.01)))
+    res, bias = torch.randn((m, n), generator=gen, device=DEV).to(dtype), torch.randn(n, generator=gen, device=DEV).to(dtype)
+
+    def call(r0, r1, flags, b=None, r=None):
+        c = torch.full((r1 - r0, n), 77.0, dtype=dtype, device=DEV)
+        s = sa[:, r0:r1].contiguous()
+        args = (p(a[r0:r1]), k, p(bt), k, p(s), p(sb), None if b is None else p(b), code)
+        tail = (p(c), n, code, r1 - r0, n, k, block, None, 0, flags, _lib.stream_ptr())      # no workspace: undivided
+        _lib.check(L.bi8_gemm_dequant(*args, *tail) if r is None else L.bi8_gemm_dequant_residual(*args, p(r), n, *tail), "gemm")
+        return c
+
+    rows = [0, 31, 127, 128, m // 2, m - 1]
+    host = (a[rows].cpu(), bt.t().cpu(), sa[:, rows].cpu(), sb.cpu(), block)
+    acc, mag = O.gemm_acc(*host), O.gemm_term_abs_sum(*host)
+    # one rounding to the output type (2^-25: half a step of fp16's subnormals)
+    step = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -24}[dtype]
+    bound = FP32_TOL * mag + step * (1 + 2.0 ** -7) * acc.abs() + 2.0 ** -25 * (dtype == torch.float16)
+    for flags in (TC, TC | NO_SEED):
+        plain = call(0, m, flags)
+        apart = torch.cat([call(r0, min(m, r0 + chunk), flags) for r0 in range(0, m, chunk)])
+        assert torch.equal(plain, apart)
+        assert bool(((plain[rows].cpu().float() - acc).abs() <= bound).all())
+        assert torch.equal(call(0, m, flags, bias), plain + bias)
+        assert torch.equal(call(0, m, flags, None, res), plain + res)
+        assert torch.equal(call(0, m, flags, bias, res), (plain + bias) + res)
+    assert_clean_device()
