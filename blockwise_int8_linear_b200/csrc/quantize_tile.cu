@@ -133,13 +133,14 @@ struct PairQ {
             bhi = hi.q(xhi);
         }
     }
-    // f(the way of this thread's pairs).  bf16: one operation or the division (`once` is `fast`).  fp16: with ONCE one operation where that
+    // f(the way of this thread's pairs).  bf16: one operation or the division; `once` is `fast` there, and it is `fast` that is asked, because that is what
+    // keeps the five operations out of the division's code (of zero blocks, rows behind the last, a last tile of few columns).  fp16: with ONCE one operation where that
     // holds for the whole warp, because a warp that is divided would do both; the third way's code costs registers, which kShift does not
     // have (dual, 8190 x 3071: 49 us without, 56 with) and kOct and the column-wise kernel gain nothing from (26.6, 28.7; dual tiles 30.7, 28.7).
     template <typename T, bool ONCE, typename F>
     __device__ __forceinline__ void choose(F f) const {
         if constexpr (std::is_same_v<T, __nv_bfloat16>) {
-            if (once) f(std::integral_constant<int, kOnce>{});
+            if (fast) f(std::integral_constant<int, kOnce>{});
             else f(std::integral_constant<int, kDivide>{});
         } else {
             if (ONCE && __all_sync(0xffffffffu, once)) f(std::integral_constant<int, kOnce>{});

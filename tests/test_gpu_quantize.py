@@ -359,3 +359,32 @@ def test_every_ratio_of_short_significands(dt, scales):
         for got_q, got_s, ref in ((qr, sr, m), (qc, sc, m.t().contiguous())):
             q_ref, s_ref = O.quantize(ref, 64)
             assert torch.equal(got_q.cpu(), q_ref) and torch.equal(got_s.cpu(), s_ref)
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("block", [32, 64, 128])
+@pytest.mark.parametrize("shape", [
+    # by tensor map (a last tile of 64 and of 8 columns, rows behind the last), by every eighth row, by the threads
+    (256, 192), (200, 136), (264, 181), (136, 321), (261, 181), (131, 192 + 3),
+])
+def test_scales_of_every_kind_side_by_side(shape, block, dt):
+    """Blocks whose scale is ordinary, zero and beyond the shortcuts' range lie side by side, in a pair of columns, a warp and a tile, whole zero blocks
+    and rows among them: every way of the tile quantizer next to every other."""
+    from triton_functions import quantize_block_colwise, quantize_block_dual
+    r, c = shape
+    x = randn_bf16(shape, r * c + block, outliers=0.01).float()
+    far, near = (2.0 ** 110, 2.0 ** -110) if dt == torch.bfloat16 else (2.0 ** 9, 2.0 ** -18)
+    rows, cols = torch.arange(r)[:, None] // 32, torch.arange(c)[None, :]
+    kind = (rows * 7 + cols * 5 + cols // 32) % 11
+    x = torch.where(kind == 1, x * far, torch.where(kind == 2, x * near, torch.where((kind == 3) | (kind == 4), torch.zeros(()), x)))
+    x[:, 40:52] = 0
+    x[32:64, 50:120] = 0                            # zero rows in the middle of a tile
+    x[:, -1] = 0
+    x[-3:] = 0
+    x = x.to(dt)
+    got = quantize_block_dual(x.to(DEV), block)
+    col = quantize_block_colwise(x.to(DEV), block)
+    want = (*O.quantize(x.float(), block), *O.quantize(x.float().t().contiguous(), block))
+    for a, b in zip((*got, *col), (*want, *want[2:])):
+        assert torch.equal(a.cpu(), b)
+    assert_clean_device()
