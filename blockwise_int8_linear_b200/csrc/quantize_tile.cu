@@ -109,12 +109,15 @@ struct Pk<__half> {
 enum QuantWay { kOnce = 0, kFast = 1, kDivide = 2 };
 struct PairQ {
     BlockQ lo, hi;
+    uint64_t r2, ns2;             // kFast; packed in its loop they cost fp16 up to 12 bytes of spills more
     bool fast, once;
     __device__ __forceinline__ void set(float amax_lo, float amax_hi) {
         lo.set(amax_lo, true);
         hi.set(amax_hi, true);
         fast = lo.fast && hi.fast;
         once = lo.once && hi.once;
+        r2 = f2_pack(lo.rcp, hi.rcp);
+        ns2 = f2_pack(-amax_lo, -amax_hi);
     }
     // The way is chosen by the caller around its whole loop (choose) rather than per pair.
     template <int WAY>
@@ -123,7 +126,7 @@ struct PairQ {
             f2_bits(f2_fma(f2_pack(xlo, xhi), f2_pack(lo.r127(), hi.r127()), f2_pack(kMagic, kMagic)), blo, bhi);
         } else if (WAY == kFast) {
             const uint64_t c127 = f2_pack(127.0f, 127.0f), cmagic = f2_pack(kMagic, kMagic), cone = f2_pack(1.0f, 1.0f);
-            const uint64_t v2 = f2_pack(xlo, xhi), r2 = f2_pack(lo.rcp, hi.rcp), ns2 = f2_pack(-lo.scale, -hi.scale);
+            const uint64_t v2 = f2_pack(xlo, xhi);
             const uint64_t q0 = f2_mul(v2, r2);
             const uint64_t e = f2_fma(ns2, q0, v2);
             const uint64_t y = f2_fma(e, r2, q0);

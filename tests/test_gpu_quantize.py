@@ -388,3 +388,22 @@ def test_scales_of_every_kind_side_by_side(shape, block, dt):
     for a, b in zip((*got, *col), (*want, *want[2:])):
         assert torch.equal(a.cpu(), b)
     assert_clean_device()
+
+
+@pytest.mark.parametrize("dt,scales", [(torch.bfloat16, range(128, 256)), (torch.float16, [127 * m for m in range(9, 17)] + [1024, 1025, 1271, 1600, 2046, 2047])])
+def test_every_ratio_in_wide_rows_and_both_dual_layouts(dt, scales):
+    """All blocks of the ratios' list, filled up with its first ones instead of cut to whole rows: the last scales (254, whose ties are real, 255, 2047)
+    reach the wide row-wise kernels and both roles of the tile quantizer as well."""
+    from triton_functions import quantize_block_dual
+    x = _all_ratios(dt, scales, range(-3, 1))
+    x = torch.cat([x, x[: -x.shape[0] % 64]])
+    wide = x.reshape(-1, 512)
+    assert wide.shape[0] % 8 == 0
+    set_config(64, dt)
+    _check_quant(wide, 64)
+    for m in (wide, wide.t().contiguous()):
+        qr, sr, qc, sc = quantize_block_dual(m.to(DEV), 64)
+        for got_q, got_s, ref in ((qr, sr, m), (qc, sc, m.t().contiguous())):
+            q_ref, s_ref = O.quantize(ref, 64)
+            assert torch.equal(got_q.cpu(), q_ref) and torch.equal(got_s.cpu(), s_ref)
+    set_config(64)
