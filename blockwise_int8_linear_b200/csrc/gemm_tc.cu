@@ -104,15 +104,14 @@ struct Cfg {
 };
 
 // Transposes a 4 x 4 matrix whose rows are the arrays of four neighbouring lanes (c the lane's place among them).
-template <typename T>
-__device__ __forceinline__ void transpose4(T (&v)[4], uint32_t c) {
+__device__ __forceinline__ void transpose4(uint32_t (&v)[4], uint32_t c) {
 #pragma unroll
     for (int d = 1; d <= 2; d <<= 1)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             if (i & d) continue;
             const bool up = (c & (uint32_t)d) != 0u;
-            const T got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + d], d);
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + d], d);
             if (up) v[i] = got;
             else v[i + d] = got;
         }
@@ -310,19 +309,6 @@ __device__ __forceinline__ float load_as_f32(const void* v, int dt, int64_t n) {
     if (dt == BI8_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(v)[n]);
     if (dt == BI8_F16) return __half2float(static_cast<const __half*>(v)[n]);
     return static_cast<const float*>(v)[n];
-}
-// elements n .. n + live - 1 (at most eight), all requested before the first is used; the rest reads as zero
-__device__ __forceinline__ void load8_as_f32(float (&f)[8], const void* v, int dt, int64_t n, int live) {
-    if (dt == BI8_F32) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) f[u] = u < live ? __ldcg(static_cast<const float*>(v) + n + u) : 0.0f;
-    } else {
-        uint16_t h[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) h[u] = u < live ? __ldcg(static_cast<const unsigned short*>(v) + n + u) : (unsigned short)0;
-#pragma unroll
-        for (int u = 0; u < 8; ++u) f[u] = dt == BI8_BF16 ? bf16lo(h[u]) : __half2float(__ushort_as_half(h[u]));
-    }
 }
 // a + b where both have (a) or are first rounded to (b) the 16-bit type: the sum rounded once more (reference lines 127-131)
 __device__ __forceinline__ uint32_t add_rounded(uint32_t a16, float b, bool bf) {
@@ -1180,8 +1166,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 // Reduction of the divided tiles: C[m,n] = cast(sum over the tile's parts) (+ cast(bias[n])) (+ residual[m,n]), the parts added
 // in ascending order, so that the result does not depend on scheduling.  A thread adds what one thread of the GEMM has left, one 32-byte
-// sector of every part (NP parts in flight: no more registers than the parts need): two columns of four rows.  Four neighbouring threads
-// exchange their sums, so that each has eight consecutive columns of a row: one 16-byte store (two for fp32) where C allows it.
+// sector of every part (NP parts in flight: no more registers than the parts need), and stores that: two columns of four rows, a warp 64
+// consecutive columns of a row at a time.  (Exchanged between four threads, so that each had eight columns of a row, it was 64-bit shuffles
+// and, with eight parts, spills, for wider stores that odd rows could not use.  Layer calls in a graph: 256 x 4096 x 1024 fp32 at block 64, eight
+// parts, 15.4 -> 14.2 us, 300 x 3072 x 768 at 32 14.4 -> 14.1, 333 x 1000 x 777 fp16, odd rows of C, 12.5 -> 10.2.)
 // The parts come from L2 where they are few (one slot per SM, 12 MB, for outputs of few tiles) and in part from DRAM where they are
 // kSplitBytes.  Launched as a programmatic dependent of the GEMM:
 // its CTAs are resident as the GEMM's leave.
@@ -1190,79 +1178,84 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const TcParams p) {
     after_predecessor();
     constexpr int GROUPS = BN / 8;                       // groups of eight columns in a tile row
     const int item = blockIdx.x * 256 + threadIdx.x;
-    static_assert(kBM * GROUPS % 32 == 0, "a warp works on one tile");
     const int t = item / (kBM * GROUPS), rem = item - t * (kBM * GROUPS);
     const int rb = rem / (GROUPS * 4), x = rem - rb * (GROUPS * 4);
-    const int quarter = rb >> 3, g = rb & 7, c = x & 3, cg = x >> 2;         // four neighbouring threads: c 0 .. 3
+    const int quarter = rb >> 3, g = rb & 7, c = x & 3, cg = x >> 2;
     if (t >= p.tiles_m * p.tiles_n) return;
     int m0, n0;
     tile_coords<BN>(t, p, m0, n0);
-    const int m = m0 + quarter * 32 + 8 * c + g, n = n0 + cg * 8;            // after the exchange
+    const int m = m0 + quarter * 32 + g, n = n0 + cg * 8 + 2 * c;            // the first of rows 8 apart, the first column
+    if (m >= p.M || n >= p.N) return;
     const int slice = cg / (COLS / 8), group = cg - slice * (COLS / 8);
     const float* src = p.ws + (int64_t)t * p.ksplit * p.slot_floats + ws_index<COLS>(quarter, slice, group, 4 * g + c);
-    // (a quarter without rows has no place in the slots; the same for all four)
-    const bool there = quarter * 32 * BN < p.slot_floats && n < p.N, mine = there && m < p.M;
-    const int live = p.N - n < 8 ? p.N - n : 8;
-    const int64_t o = (int64_t)m * p.ldc + n, ro = (int64_t)m * p.ldr + n;
-    float acc[8], bias[8], res[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) acc[u] = bias[u] = res[u] = 0.0f;
+    const bool both = n + 1 < p.N, wide = p.out_dtype == BI8_F32, bf = p.out_dtype == BI8_BF16;
     const bool has_bias = p.bias != nullptr, has_res = p.residual != nullptr;
-    if (has_bias && mine) load8_as_f32(bias, p.bias, p.bias_dtype, n, live);
-    if (has_res && mine) load8_as_f32(res, p.residual, p.out_dtype, ro, live);
-    if (there) {
-        for (int s0 = 0; s0 < p.ksplit; s0 += NP) {
-            float v[NP][8];
+    float b0 = 0.0f, b1 = 0.0f;
+    uint32_t res[8];                                     // per row its two values, or one word of two 16-bit ones
+    if (has_bias) bias_pair(p, n, b0, b1);
+    if (has_res) {
 #pragma unroll
-            for (int q = 0; q < NP; ++q)
-                if (s0 + q < p.ksplit) ldcg_v8(v[q], src + (int64_t)(s0 + q) * p.slot_floats);
-#pragma unroll
-            for (int q = 0; q < NP; ++q)
-                if (s0 + q < p.ksplit) {
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) acc[u] = __fadd_rn(acc[u], v[q][u]);
+        for (int r = 0; r < 4; ++r) {
+            const int64_t at = (int64_t)(m + 8 * r) * p.ldr + n;
+            const bool live = m + 8 * r < p.M;
+            res[2 * r] = res[2 * r + 1] = 0u;
+            if (wide) {
+                const unsigned* const v = static_cast<const unsigned*>(p.residual) + at;
+                if (live) res[2 * r] = __ldcg(v);
+                if (live && both) res[2 * r + 1] = __ldcg(v + 1);
+            } else {
+                const unsigned short* const v = static_cast<const unsigned short*>(p.residual) + at;
+                if (live && both && p.res_vec) {
+                    res[2 * r] = __ldcg(reinterpret_cast<const unsigned*>(v));
+                } else if (live) {
+                    res[2 * r] = __ldcg(v);
+                    if (both) res[2 * r] |= (uint32_t)__ldcg(v + 1) << 16;
                 }
+            }
         }
     }
-    __syncwarp();
-    uint64_t pairs[4];
+    float acc[8];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) pairs[u] = pack_f32x2(acc[2 * u], acc[2 * u + 1]);
-    transpose4(pairs, (uint32_t)c);
+    for (int u = 0; u < 8; ++u) acc[u] = 0.0f;
+    for (int s0 = 0; s0 < p.ksplit; s0 += NP) {
+        float v[NP][8];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) unpack_f32x2(pairs[u], acc[2 * u], acc[2 * u + 1]);
-    if (!mine) return;
-    if (p.out_dtype == BI8_F32) {
+        for (int q = 0; q < NP; ++q)
+            if (s0 + q < p.ksplit) ldcg_v8(v[q], src + (int64_t)(s0 + q) * p.slot_floats);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            if (has_bias) acc[u] = __fadd_rn(acc[u], bias[u]);
-            if (has_res) acc[u] = __fadd_rn(acc[u], res[u]);
-        }
-        float* c = static_cast<float*>(p.C) + o;
-        if (live == 8 && p.vec_store) {
-            reinterpret_cast<float4*>(c)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-            reinterpret_cast<float4*>(c)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        for (int q = 0; q < NP; ++q)
+            if (s0 + q < p.ksplit) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) acc[u] = __fadd_rn(acc[u], v[q][u]);
+            }
+    }
+    const bool vec = both && p.vec_store;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        if (m + 8 * r >= p.M) return;
+        const int64_t o = (int64_t)(m + 8 * r) * p.ldc + n;
+        float lo = acc[2 * r], hi = acc[2 * r + 1];
+        if (wide) {
+            if (has_bias) lo = __fadd_rn(lo, b0), hi = __fadd_rn(hi, b1);
+            if (has_res) lo = __fadd_rn(lo, __uint_as_float(res[2 * r])), hi = __fadd_rn(hi, __uint_as_float(res[2 * r + 1]));
+            float* const d = static_cast<float*>(p.C) + o;
+            if (vec) {
+                *reinterpret_cast<float2*>(d) = make_float2(lo, hi);
+            } else {
+                d[0] = lo;
+                if (both) d[1] = hi;
+            }
         } else {
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (u < live) c[u] = acc[u];
-        }
-    } else {
-        const bool bf = p.out_dtype == BI8_BF16;
-        uint32_t h[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            h[u] = (bf ? pack_bf16x2(acc[u], 0.0f) : pack_f16x2(acc[u], 0.0f)) & 0xffffu;
-            if (has_bias) h[u] = add_rounded(h[u], bias[u], bf);
-            if (has_res) h[u] = add_rounded(h[u], res[u], bf);
-        }
-        uint16_t* c = static_cast<uint16_t*>(p.C) + o;
-        if (live == 8 && p.vec_store) {
-            *reinterpret_cast<uint4*>(c) = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
-        } else {
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (u < live) c[u] = (uint16_t)h[u];
+            uint32_t w = bf ? pack_bf16x2(lo, hi) : pack_f16x2(lo, hi);
+            if (has_bias) w = add_pair(w, bf ? pack_bf16x2(b0, b1) : pack_f16x2(b0, b1), bf);
+            if (has_res) w = add_pair(w, res[2 * r], bf);
+            uint16_t* const d = static_cast<uint16_t*>(p.C) + o;
+            if (vec) {
+                *reinterpret_cast<uint32_t*>(d) = w;
+            } else {
+                d[0] = (uint16_t)w;
+                if (both) d[1] = (uint16_t)(w >> 16);
+            }
         }
     }
 }

@@ -595,3 +595,63 @@ def test_short_items_over_several_rounds(shape, block, stages, dtype):
         assert torch.equal(call(0, m, flags, None, res), plain + res)
         assert torch.equal(call(0, m, flags, bias, res), (plain + bias) + res)
     assert_clean_device()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [
+    # (M, N, K, block), in 4, 8, 8, 16, 16, 32, 11, 6, 2 and 4 parts: a quarter of a tile's rows, one column, the last tile of either edge
+    (333, 777, 1008, 64), (256, 1024, 4096, 64), (100, 2047, 2048, 64), (70, 1001, 4096, 64), (129, 163, 4096, 64), (65, 7, 8192, 64),
+    (193, 325, 4096, 128), (257, 1003, 768, 32), (760, 5919, 4096, 32), (2047, 3100, 5504, 32),
+])
+def test_reduction_of_divided_tiles(shape, dtype):
+    """Parts added from the workspace, to outputs and residuals of every alignment: sampled rows within the tolerance of the oracle, equal rows
+    give equal bits, bias and residual (in place too) are what additions in the output type make of the plain result, and nothing outside the
+    M x N elements is written."""
+    from blockwise_int8_linear_b200 import _lib
+    import triton_functions as tf
+    L, p = _lib.lib(), _lib.ptr
+    m, n, k, block = shape
+    set_config(block, dtype)
+    need = L.bi8_gemm_workspace_used(m, n, k, block)
+    assert need > 0, "the plan divides the tiles through the workspace"
+    gen = torch.Generator(device=DEV).manual_seed(m * n)
+    x = torch.randn((m, k), generator=gen, device=DEV).to(torch.bfloat16)
+    x[m - 1] = x[0]
+    a, sa = tf.quantize_block_rowwise(x)
+    bt = torch.randint(-127, 128, (n, k), generator=gen, device=DEV, dtype=torch.int8)
+    sb = torch.rand((-(-k // block), n), generator=gen, device=DEV) * 0.02 + 0.01
+    bias = torch.randn(n, generator=gen, device=DEV).to(dtype)
+    work = torch.empty(need, dtype=torch.uint8, device=DEV)
+    code, plain = _lib.dtype_code(dtype), None
+    rows = sorted({0, 31, m // 2, m - 1})
+    host = (a[rows].cpu(), bt.t().cpu(), sa[:, rows].cpu(), sb.cpu(), block)
+    acc, mag = O.gemm_acc(*host), O.gemm_term_abs_sum(*host)
+    step = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -24}[dtype]
+    for pitch, lead in (((n + 7) // 8 * 8, 0), (n + 3, 1)):
+        buf = torch.full((lead + m * pitch + 64,), 77.0, dtype=dtype, device=DEV)
+        c = buf[lead:lead + m * pitch].view(m, pitch)
+        res_buf = torch.randn(lead + m * pitch, generator=gen, device=DEV).to(dtype)
+        res = res_buf[lead:].view(m, pitch)
+        for b, r in ((None, None), (bias, None), (None, res), (bias, res)):
+            args = (p(a), k, p(bt), k, p(sa), p(sb), None if b is None else p(b), code)
+            tail = (c.data_ptr(), pitch, code, m, n, k, block, p(work), need, 0, _lib.stream_ptr())
+            _lib.check(L.bi8_gemm_dequant(*args, *tail) if r is None else L.bi8_gemm_dequant_residual(*args, r.data_ptr(), pitch, *tail), "gemm")
+            got = c[:, :n].clone()
+            c[:, :n] = 77.0
+            assert bool((buf == 77.0).all())
+            if plain is None:
+                plain = got
+                assert torch.equal(plain[0], plain[m - 1])
+                err = (plain[rows].cpu().float() - acc).abs()
+                assert bool((err <= FP32_TOL * mag + step * (1 + 2.0 ** -7) * acc.abs() + 2.0 ** -25 * (dtype == torch.float16)).all())
+            want = plain if b is None else plain + b
+            assert torch.equal(got, want if r is None else want + r[:, :n])
+        c[:, :n] = res[:, :n]
+        xq, sx = torch.empty_like(a), torch.empty_like(sa)
+        _lib.check(L.bi8_gemm_dequant_fused_pre(_lib.PRE_NONE, p(x), None, _lib.BI8_BF16, k, None, 0.0, p(xq), p(sx), p(bt), k, p(sb), None, 0,
+                                                c.data_ptr(), pitch, c.data_ptr(), pitch, code, m, n, k, block, p(work), need, 0, _lib.stream_ptr()), "in place")
+        assert torch.equal(c[:, :n], plain + res[:, :n])
+        c[:, :n] = 77.0
+        assert bool((buf == 77.0).all())
+    assert_clean_device()
+    set_config(64)
