@@ -1352,7 +1352,9 @@ int launch_qb(const TcMaps& tm, const TcParams& p, int grid, bool partials, bool
     if (cluster) return launch_one<QB, 0, true, kCluster>(tm, p, grid, st);
     if (p.ksplit > 1) return launch_one<QB, 0, true, kSplit>(tm, p, grid, st);
     if (p.out_dtype == BI8_F32) return launch_one<QB, 0, true, kWide>(tm, p, grid, st);
-    if (p.store == kRows) return launch_one<QB, 0, true, kRows16>(tm, p, grid, st);
+    if constexpr (QB != 32) {
+        if (p.store == kRows) return launch_one<QB, 0, true, kRows16>(tm, p, grid, st);
+    }
     if (p.store == kOwn) return launch_one<QB, 0, true, kOwn16>(tm, p, grid, st);
     return p.bias || p.residual ? launch_one<QB, 0, true, kTma16Add>(tm, p, grid, st) : launch_one<QB, 0, true, kTma16>(tm, p, grid, st);
 }
@@ -1629,7 +1631,10 @@ int launch_gemm_tc(const GemmArgs& g, cudaStream_t st) {
         rc = cached_output_map(&tm.c, dev, g.C, esz, g.M, g.N, g.ldc, 32, esz == 2 ? cols : cols / 2);
         if (rc != BI8_OK) return rc;
         p.store = kTma;
-    } else if (!partials && seed && pl.ksplit == 1 && esz == 2 && !g.bias && !g.residual && g.M % 8 == 0 && aligned(g.C, 16) && g.ldc < (1ll << 28) && g.N >= bn) {
+    } else if (!partials && seed && pl.ksplit == 1 && esz == 2 && !g.bias && !g.residual && g.block != 32 && g.M % 8 == 0 && aligned(g.C, 16) &&
+               g.ldc < (1ll << 28) && g.N >= bn) {
+        // (at block 32 the K loop of that instance is half as long again: 8192 x 4096 x 11005 1835 us, 1230 by own stores, 8192 x 768 x 50257 1670,
+        // 1320; at 64 666, 649 and 682, 800; at 128 441, 456 and 531, 611)
         rc = cached_output_map(&tm.c, dev, g.C, 2, g.M / 8, 7 * g.ldc + g.N, 8 * g.ldc, kBM / 8, bn - 8);
         if (rc != BI8_OK) return rc;
         p.store = kRows;
