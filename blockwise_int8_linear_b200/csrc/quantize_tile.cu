@@ -14,8 +14,8 @@
 //     the 16 rows of a tile that are equal modulo 8, 136 columns from the 16-byte boundary at or before the tile's first.
 //     The threads shift what they read by the class's offset, which is a constant for the column-wise role's unrolled
 //     rows and, with a warp per class, for a whole warp of the row-wise role.  8192 x 50257: dual 494 -> 399 us (345 with aligned
-//     rows), column-wise 488 -> 224 (225); with one operation per pair (quant_math.cuh) dual 358, and 8192 x 8192, aligned, 63.5 -> 57.3,
-//     8192 x 3072 30.7 -> 26.6.  What is left is the rest of the instructions: with twice the threads and half the words for each (64 registers, no
+//     rows), column-wise 488 -> 224 (225); with one operation per pair (quant_math.cuh) dual 338 (288), and 8192 x 8192, aligned, 63.5 -> 54.4,
+//     8192 x 3072 30.8 -> 26.6.  What is left is the rest of the instructions: with twice the threads and half the words for each (64 registers, no
 //     spills) every one of those times was a tenth longer.
 //     Where the number of rows is not a multiple of 8 (kShift) all threads fetch: a half-warp reads a tile row as aligned
 //     16-byte pieces, shifts the bytes into place between neighbouring lanes and stores them where the TMA would have put
@@ -30,8 +30,8 @@
 //   * SUM (dual): the column-wise role has every value in a register when it quantizes, so the column sums of the tile (the bias
 //     gradient, out of a gradient) cost its 32 additions per column and no read of their own: 8192 x 768 x 3072 forward and
 //     backward 226 -> 213 us.  fp32, rows ascending, one partial row per tile; column_sum.cu adds those.  Where the threads fetch
-//     the input themselves (kShift) the sums spill a few registers, and still cost less than a read of their own: with sums / with a separate
-//     column sum / without, block 64: 8190 x 3071 54 / 75 / 48 us, 8190 x 50257 597 / 750 / 500, 1001 x 3109 21.5 / 29.7 / 18.5.
+//     the input themselves (kShift) the sums of fp16 spill a few registers, and still cost less than a read of their own: with sums / with a separate
+//     column sum / without, block 64: 8190 x 3071 bf16 48 / 71 / 44 us, fp16 56 / 75 / 48, 8190 x 50257 472 / 716 / 466 and 601 / 759 / 509.
 //   * the two int8 tiles leave with one TMA store each (128-byte swizzle again, so that the transposed writes do not
 //     pile up on a few banks); tile parts outside the tensors are clipped by the store.
 // The input tile has three stages (two in the column-wise kernel), so the next loads are in flight while a tile is quantized;
@@ -140,9 +140,10 @@ struct PairQ {
     // keeps the five operations out of the division's code (of zero blocks, rows behind the last, a last tile of few columns).  fp16: with ONCE one operation where that
     // holds for the whole warp, because a warp that is divided would do both; the third way's code costs registers, which kShift does not
     // have (dual, 8190 x 3071: 49 us without, 56 with) and kOct and the column-wise kernel gain nothing from (26.6, 28.7; dual tiles 30.7, 28.7).
-    template <typename T, bool ONCE, typename F>
+    // FIVE: bf16 by the five operations (see five_operations).
+    template <typename T, bool ONCE, bool FIVE, typename F>
     __device__ __forceinline__ void choose(F f) const {
-        if constexpr (std::is_same_v<T, __nv_bfloat16>) {
+        if constexpr (std::is_same_v<T, __nv_bfloat16> && !FIVE) {
             if (fast) f(std::integral_constant<int, kOnce>{});
             else f(std::integral_constant<int, kDivide>{});
         } else {
@@ -261,7 +262,7 @@ struct ShiftLoader {
     }
 };
 
-template <typename T, int B, bool DUAL, int IN, bool SUM>
+template <typename T, int B, bool DUAL, int IN, bool SUM, bool FIVE>
 __global__ void __launch_bounds__(DUAL ? 2 * kQThreads : kQThreads, DUAL ? 1 : 2)
 quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmQc,
                      const __grid_constant__ CUtensorMap tmQr, const void* __restrict__ x, int64_t ldx, float* __restrict__ s_col,
@@ -459,7 +460,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                     sts_v4(outc + swz(c + 1, g * 2 + part), wh[0], wh[1], wh[2], wh[3]);
                 }
             };
-            pq.template choose<T, DUAL && IN == kTiled>(quantize_cols);
+            pq.template choose<T, DUAL && IN == kTiled, FIVE>(quantize_cols);
             // scales [ceil(R/B), C]: the first row group of each block writes the pair
             if ((g % (B / 32)) == 0) {
                 const int rb = r0 + g * 32;
@@ -563,7 +564,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                         sts_v4(outr + swz(srow, half * 4 + b * (4 / NBT) + k), wd[0], wd[1], wd[2], wd[3]);
                     }
                 };
-                pq.template choose<T, DUAL && IN == kTiled>(quantize_row);
+                pq.template choose<T, DUAL && IN == kTiled, FIVE>(quantize_row);
             }
             // scales [ceil(C/B), R] (transposed): eight consecutive rows per quarter-warp
             if (r0 + row < R) {
@@ -668,14 +669,14 @@ int cached_q_map(CUtensorMap* map, int dev, int8_t* ptr, int64_t rows, int64_t c
     return rc;
 }
 
-template <typename T, int B, bool DUAL, int IN, bool SUM>
+template <typename T, int B, bool DUAL, int IN, bool SUM, bool FIVE = false>
 int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap& tqr, const void* x, int64_t ldx, float* s_col, float* s_row, float* sums,
                 int64_t R, int64_t C, cudaStream_t st) {
     const int64_t ctiles = (C + kQT - 1) / kQT, rtiles = (R + kQT - 1) / kQT;
     if (ctiles * rtiles >= (1ll << 31)) return fail(BI8_ERR_SHAPE, "quantize: grid too large");
     constexpr size_t smem = (DUAL ? QLayout<3, IN>::bytes_dual : QLayout<2, IN>::bytes_col) + 1024;
     static SmemOptIn opt_in;
-    const int rc = opt_in.ensure(quantize_tile_kernel<T, B, DUAL, IN, SUM>, smem);
+    const int rc = opt_in.ensure(quantize_tile_kernel<T, B, DUAL, IN, SUM, FIVE>, smem);
     if (rc != BI8_OK) return rc;
     int* status = device_status_ptr();
     if (!status) return BI8_ERR_CUDA;
@@ -683,7 +684,17 @@ int launch_tile(const CUtensorMap& tx, const CUtensorMap& tqc, const CUtensorMap
     const int64_t tiles = ctiles * rtiles;
     const int64_t resident = (int64_t)(DUAL ? 1 : 2) * di.sms;                 // CTAs that fit at once
     const int grid = (int)(tiles < resident ? tiles : resident);
-    return launch_chained(quantize_tile_kernel<T, B, DUAL, IN, SUM>, grid, DUAL ? 2 * kQThreads : kQThreads, smem, st, tx, tqc, tqr, x, ldx, s_col, s_row, sums, (int)R, (int)C, (int)ctiles, (int)tiles, status);
+    return launch_chained(quantize_tile_kernel<T, B, DUAL, IN, SUM, FIVE>, grid, DUAL ? 2 * kQThreads : kQThreads, smem, st, tx, tqc, tqr, x, ldx, s_col, s_row, sums, (int)R, (int)C, (int)ctiles, (int)tiles, status);
+}
+
+// The column-wise kernel's way with bf16.  One operation per pair is faster until the memory is what bounds it; there warps that ask for it in shorter
+// bursts get less of it (both ways in a graph, one / five, block 64, blocks 32 and 128 alike).  Tiles by tensor map: 8192 x 8192 35.5 / 36.3 us, 8192 x
+// 10240 43.7 / 43.4, 8192 x 12288 51.8 / 51.7, 8192 x 14336 61.9 / 59.8, 16384 x 16384 154.5 / 144.4.  By every eighth row: 8192 x 30001 129 / 136, 8192 x
+// 35001 148-153 / 157, 32768 x 10001 167 / 180, 16384 x 20001 170-190 / 179, 8192 x 40001 184 / 177, 65536 x 6001 238 / 215, 8192 x 50257 240 / 221.
+constexpr int64_t kFiveTiled = 160ll << 20, kFiveOct = 624ll << 20;         // bytes of the input
+template <typename T>
+bool five_operations(int64_t R, int64_t C, bool tiled) {
+    return std::is_same_v<T, __nv_bfloat16> && R * C * 2 >= (tiled ? kFiveTiled : kFiveOct);
 }
 
 template <typename T>
@@ -706,14 +717,21 @@ int tile_dispatch(const void* x, int64_t ldx, int8_t* q_col, int64_t ldqc, float
         rc = cached_q_map(&tqr, dev, q_row, R, C, ldqr, oct);
         if (rc != BI8_OK) return rc;
     }
+    constexpr bool BF = std::is_same_v<T, __nv_bfloat16>;
+    const bool five = five_operations<T>(R, C, tiled);
+#define BI8_TILE_C(BB)                                                                                           \
+    five && tiled ? launch_tile<T, BB, false, kTiled, false, BF>(tx, tqc, tqr, x, ldx, s_col, s_row, sums, R, C, st) \
+    : five && oct ? launch_tile<T, BB, false, kOct, false, BF>(tx, tqc, tqr, x, ldx, s_col, s_row, sums, R, C, st)   \
+                  : BI8_TILE_D(BB, false, false)
 #define BI8_TILE_D(BB, DUAL, SUM)                                                                                \
     tiled ? launch_tile<T, BB, DUAL, kTiled, SUM>(tx, tqc, tqr, x, ldx, s_col, s_row, sums, R, C, st)           \
     : oct ? launch_tile<T, BB, DUAL, kOct, SUM>(tx, tqc, tqr, x, ldx, s_col, s_row, sums, R, C, st)             \
           : launch_tile<T, BB, DUAL, kShift, SUM>(tx, tqc, tqr, x, ldx, s_col, s_row, sums, R, C, st)
 #define BI8_TILE(BB) \
-    if (block == BB) return !dual ? (BI8_TILE_D(BB, false, false)) : sums ? (BI8_TILE_D(BB, true, true)) : (BI8_TILE_D(BB, true, false));
+    if (block == BB) return !dual ? (BI8_TILE_C(BB)) : sums ? (BI8_TILE_D(BB, true, true)) : (BI8_TILE_D(BB, true, false));
     BI8_TILE(32) BI8_TILE(64) BI8_TILE(128)
 #undef BI8_TILE
+#undef BI8_TILE_C
 #undef BI8_TILE_D
     return fail(BI8_ERR_BLOCK, "tile quantizer supports block 32, 64, 128 (got %d)", block);
 }

@@ -407,3 +407,23 @@ def test_every_ratio_in_wide_rows_and_both_dual_layouts(dt, scales):
             q_ref, s_ref = O.quantize(ref, 64)
             assert torch.equal(got_q.cpu(), q_ref) and torch.equal(got_s.cpu(), s_ref)
     set_config(64)
+
+
+@pytest.mark.parametrize("block", [32, 64, 128])
+@pytest.mark.parametrize("shape", [(10485, 8000), (10486, 8000), (32768, 9983), (32768, 9985)])
+def test_colwise_either_side_of_the_two_ways(shape, block):
+    """bf16 inputs below and above the sizes from which the column-wise kernel takes five operations a pair instead of one: the row-wise
+    kernel's result for the transposed matrix, bit for bit, with zero blocks and scales beyond the shortcuts' range among them."""
+    from triton_functions import quantize_block_colwise, quantize_block_rowwise
+    set_config(block)
+    gen = torch.Generator(device=DEV).manual_seed(shape[0] + block)
+    x = torch.randn(shape, generator=gen, device=DEV).to(torch.bfloat16)
+    x[: shape[0] // 3, 5::97] = 0
+    x[shape[0] // 2:, 7::89] *= 2.0 ** 110
+    x[shape[0] // 2:, 8::89] *= 2.0 ** -110
+    x[-3:] = 0
+    q, s = quantize_block_colwise(x, block)
+    q2, s2 = quantize_block_rowwise(x.t().contiguous(), block)
+    assert torch.equal(s, s2) and torch.equal(q, q2)
+    assert_clean_device()
+    set_config(64)
