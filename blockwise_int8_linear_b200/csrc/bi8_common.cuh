@@ -69,9 +69,15 @@ struct SmemOptIn {
 };
 
 // Launch that may start before its predecessor in the stream has completed (programmatic stream serialisation).  Every kernel
-// launched this way executes after_predecessor() in every thread, before it touches memory that an earlier kernel reads or
-// writes; dependents are released only there, so that "the predecessor has completed" always means that everything before
-// it has completed too.  What it saves is the launch latency and the kernel's set-up, 1-2 us per kernel of a chain.
+// launched this way waits for its predecessor (wait_predecessor) in every thread that touches memory which an earlier kernel reads or writes,
+// and before it ends, so that "the predecessor has completed" always means that everything before it has completed too.  What a kernel
+// reads before its wait is memory that no incomplete earlier kernel writes.  Most kernels release their dependents right after the wait
+// (after_predecessor), so that behind them only they themselves are incomplete.  The general GEMM releases later, from its producer warp alone: still
+// after the wait, which is for the whole preceding grid.  Two kernels release before their wait: the decode GEMM with early weights, which runs
+// only behind this library's own quantizer (that one releases after its wait and writes neither weights nor their scales), and the
+// reduction over peers behind such a GEMM, which reads nothing early but its own sequence number.  What follows either may start while two or three
+// kernels are incomplete, and waits first thing.  What all this saves is the launch latency and the kernel's set-up, 1-2 us per
+// kernel of a chain.
 template <typename... P, typename... A>
 int launch_chained_grid(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchConfig_t cfg{};

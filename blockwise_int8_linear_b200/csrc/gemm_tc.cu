@@ -8,11 +8,12 @@
 // One persistent CTA per SM works on 128 x BN output tiles.  Warp roles:
 //   warp 0      producer.  Per stage two TMA copies of 128-byte-swizzled K-major operand tiles (A: 128 rows, Bt: BN
 //               rows, 128 K-bytes) into a ring of kStages slots, and two TMA copies of the stage's block scales (fp32
-//               boxes [blocks, BN] of sA and of sB) into rings of SC_STAGES slots, all four on the stage's one "full"
-//               barrier.  Scale tensors that a tensor map cannot describe (base or row length not 16-byte aligned) are
-//               copied with cp.async by the warp's 32 lanes instead, arriving on the same barrier.  The scale rings need
-//               no barriers of their own: the promotion warps read a stage's scales only after they have seen one of
-//               its accumulators complete (the MMAs were issued after the stage's barrier), and the rings are deep
+//               boxes [blocks, 128] of sA and [blocks, BN] of sB), all four on the stage's one "full" barrier.  Scale tensors that a
+//               tensor map cannot describe (base or row length not 16-byte aligned) are
+//               copied with cp.async by the warp's 32 lanes instead, arriving on the same barrier.  sA lies in the operand stage's slot:
+//               only the seeder reads it, and the slot is free when the stage's MMAs are complete and the seeder has
+//               arrived (EMPTY_AB).  sB lies in a ring of its own without barriers: the promotion warps read a stage's column scales after they
+//               have seen one of its accumulators complete (the MMAs were issued after the stage's barrier), and the ring is deep
 //               enough that a slot is never rewritten while in use (SC_STAGES).
 //   warp 1      issues tcgen05.mma kind::i8 (M128 N=BN K32): the MMAs of one quantisation block accumulate into one of
 //               three s32 accumulators in tensor memory, then a commit hands that accumulator to the promotion warps.
@@ -24,7 +25,8 @@
 //               releases the accumulator as soon as the last columns are in registers.  After the last block of a tile it casts, adds
 //               the bias, stages its 32 x 40 part in shared memory, adds the residual there and goes on with the next tile.
 // What bounds the kernel: the promotion, t = P*s_row and acc += s_col*t for two columns per FFMA2, and what its warps issue beside it.  A
-// scheduler takes two cycles per FFMA2 and one per other instruction, and each of its four warps has 40 and about 60 of them per block: 520 cycles
+// scheduler takes two cycles per FFMA2 and one per other instruction, and each of its four warps has 40 and about 50 of them per block (92
+// instructions a block and promotion warp in all, epilogue and role warps included): 520 cycles
 // (the promotion alone, without MMAs; 372 without the barriers).  MMAs beside it cost another 60 to 70 cycles each: one of M128 N160 K32 reads
 // 9.2 KB of operands in 80 cycles, 90 % of the shared memory's bandwidth, and the loads of the scales wait (552, 602 and 733 cycles a block
 // of 32, 64 and 128; without the loads of scales 604 at 128).  The MMAs and seeds alone take 162, 242 and 402.  Every register that a
@@ -32,8 +34,8 @@
 // columns (32x32b reads) a warp loaded 41 scales per block and thread; with four rows and ten columns (16x256b) 4 records and 10 scales,
 // each scale pair of the columns used for four rows in turn.  Row scales are prepared once per CTA by the seeder, not by every
 // thread for its four rows.  At 128 the operands' way from L2 (64 bytes per cycle and SM, 576 cycles per 128 x 160 x 128) bounds as well.
-// 8192 x 4096 x 11008, cold: 666 -> 593 us at block 64, 416 -> 380 at 128, 1323 -> 1189 at 32 (with the row-wise reads and the
-// issuer as a loop of its warp, the same box); a lab loop without epilogue 683 -> 535, 731 -> 569 and 611 -> 535 cycles a block.
+// 8192 x 4096 x 11008, cold: 672 -> 591 us at block 64, 425 -> 383 at 128, 1327 -> 1177 at 32 (with the row-wise reads and the
+// issuer as a loop of its warp, the same GPU; others take 1 to 2 % more on either side); a lab loop without epilogue 683 -> 535, 731 -> 569 and 611 -> 535 cycles a block.
 // Reading 8 + 32 columns at a time, the accumulator is free early and the first fold hides the second read: in that loop 527 cycles
 // against 548 for all at once, 536 for 16 + 24, 636 for five times eight.
 // The release of an accumulator is one predicated arrival (a branch around it: 577 cycles a block, 538 so), and the issuer tests a stage and its first
@@ -79,12 +81,13 @@ constexpr uint32_t kABytes = kBM * kBK;  // 16 KiB
 constexpr uint32_t kSeedBits = 0x4B400000u;   // float 1.5 * 2^23
 constexpr float kSeedF = 12582912.0f;
 
-// Promotion warps per tensor-memory lane quarter, and what follows from it: a thread owns COLS columns of its row.  (Two or three
+// Promotion warps per tensor-memory lane quarter, and what follows from it: a warp owns COLS columns of its 32 rows, a thread COLS results
+// (a quarter of those columns in four rows).  (Two or three
 // warps with 80 or 48 columns each were 7-18 % slower.)
 constexpr int kPW = 4;
 struct Cfg {
     static constexpr int BN = 160;                        // tile columns: kAccBufs * BN <= 512 tensor-memory columns
-    static constexpr int COLS = BN / kPW;                 // columns owned by one promotion thread
+    static constexpr int COLS = BN / kPW;                 // columns owned by one promotion warp
     static constexpr int EPI_WARPS = 4 * kPW;
     static constexpr int THREADS = (kRoleWarps + EPI_WARPS) * 32;
     static constexpr int LAUNCH_REGS = 96;                // 65536 / THREADS, rounded down to a multiple of 8
@@ -123,9 +126,9 @@ __device__ __forceinline__ void transpose4(uint32_t (&v)[4], uint32_t c) {
 // to all others.
 enum StoreMode { kTma = 0, kRows = 1, kOwn = 2 };
 // Instances of the kernel by the way its tiles leave: code for the other ways, even where it is not executed, costs the K loop
-// registers.  kAnyOut in the instance's place at block 32 / 64 / 128: kTma16 8192 x 4096 x 11008 +2.1 / 2.0 / 0 %, 4096 x 512 x 4096 +4.7 / 6.3 /
-// 6.2 %; kTma16Add 2048 x 768 x 3072 +5.1 / 3.3 / 2.0 %; kOwn16 8192 x 4096 x 11005 +5.1 / 5.0 / 1.2 %; kWide 8192 x 4096 x 11008 +1.8 / 1.9 /
-// 0 %, 4096 x 512 x 4096 +3.8 / 3.9 / 0 %.
+// registers.  kAnyOut in the instance's place at block 32 / 64 / 128: kTma16 8192 x 4096 x 11008 +1.4 / 0.9 / 0.8 %, 4096 x 512 x 4096 +4.9 / 7.9 /
+// 0 %; kTma16Add 2048 x 768 x 3072 +1.1 / 2.6 / 0 %; kOwn16 8192 x 4096 x 11005 with bias 0 / 0.6 / 0 %; kWide 8192 x 4096 x 11008 0 / 1.7 /
+// 0.4 %, 4096 x 512 x 4096 +1.7 / 1.3 / 3 %.
 enum OutKind { kAnyOut = 0, kSplit, kCluster, kTma16, kTma16Add, kRows16, kOwn16, kWide };
 
 struct TcParams {
@@ -160,9 +163,10 @@ struct Geo {
     static constexpr int BPS = kBK / QB;                        // quantisation blocks per stage
     static constexpr int MMAS = QB / 32;                        // MMAs (K = 32) per block
     // Column scales: a ring of records of BN floats, one per block.  The producer fills the slot of stage s after the MMA warp has
-    // committed stage s - kStages, whose last block was issued into an accumulator that the promotion warps had released kAccBufs
-    // blocks earlier, having read everything but some of that block's scales: stages up to s - kStages - ceil((kAccBufs + 1) / BPS)
-    // may still be read.
+    // committed stage s - kStages.  By then every promotion warp had released a block at most kAccBufs before that stage's last one (a tile
+    // restarts on accumulator 0, so the use before may be up to five blocks back, but then a later block's release has been
+    // seen), having read everything but some of the released block's scales: the oldest stage that may still be read is
+    // s - kStages + 1 - ceil((kAccBufs + 1) / BPS) = s - SC_STAGES + 1, and the slot held s - SC_STAGES.
     static constexpr int SC_STAGES = kStages + (kAccBufs + 1 + BPS - 1) / BPS;
     static constexpr uint32_t SC_REC = C::BN * 4;               // bytes of a record
     static constexpr uint32_t SC_RING = SC_STAGES * BPS * SC_REC;
@@ -380,8 +384,9 @@ __device__ __noinline__ void store_own(unsigned char* dst, int64_t pitch, uint32
 // 16-bit outputs with rows of any even alignment (kRows).  Rows that are eight apart have the same alignment, so a tensor map whose
 // "rows" are eight rows long describes them: with h the elements of a tile row before its first 16-byte boundary, elements h .. h+151
 // of the 16 rows of a tile that are equal modulo 8 leave by one TMA store, the first h and last 8-h one by one; a last, partial column of tiles is kOwn's.  8192 x 50257, K 768:
-// 848 us by the promotion warps, 694 this way (604 with aligned rows); one bulk copy per row took 110 cycles a row, 16-byte pieces moved by the storer
-// 190 (1430 and 1870 us).
+// 800 us by the promotion warps at block 64, 682 this way (545 with aligned rows); one bulk copy per row took 110 cycles a row, 16-byte pieces moved by
+// the storer 190 (twice and nearly three times as long).  A thread's values are exchanged by shuffles first, so that a lane stages one row; words joined with the
+// neighbouring lane's instead take 834 us, two-byte stores 953, an exchange through shared memory by stmatrix 703.
 __device__ __forceinline__ uint32_t rows_head(const TcParams& p, uint32_t row_class, int n0) {
     return (0u - (row_class * (uint32_t)p.ldc + (uint32_t)n0)) & 7u;
 }
@@ -987,7 +992,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
             if (MODE == 0 && (OUT == kSplit || (OUT == kAnyOut && slot >= 0))) {
                 // Part of a divided tile: straight from the registers to the item's workspace slot, in the order in which
-                // the reduction kernel reads it (ws_index: 32 bytes of one row per thread and step).
+                // the reduction kernel reads it (ws_index: 32 bytes per thread and step, two columns of its four rows).
                 float* dst = p.ws + (int64_t)slot * p.slot_floats + ws_index<COLS>(quarter, slice, 0, lane);
                 const bool live = quarter * 32 * BN < p.slot_floats;
 #pragma unroll
@@ -1002,9 +1007,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 // The tile leaves through shared memory: the promotion warps write their shares, the storer warp moves them out while
                 // the promotion warps go on with the next tile.  Fencing, issuing and waiting for the copies here cost 800 of
                 // a K = 512 tile's 7500 cycles (8192 x 512 x 11840: 134 -> 112 us with this and the fast division of tile_coords).  Addresses are derived here from the thread index rather than kept in
-                // registers through the K loop, whose register budget is full.  Bias and residual are added to the staged row
-                // by a loop of its own: with their code unrolled between the casts the epilogue was 1.1 us per tile
-                // (instruction fetch).
+                // registers through the K loop, whose register budget is full.  The bias is added to the packed pairs behind the casts (a pair
+                // of columns serves four rows), the residual to the staged row.
                 uint32_t tid_now;
                 asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid_now));
                 const uint32_t ln = tid_now & 31u, w = (tid_now >> 5) - (uint32_t)kRoleWarps, qt = w & 3u, sl = w >> 2;
@@ -1376,10 +1380,12 @@ struct SplitPlan {
 };
 // What a work item takes per stage (128 K-bytes of a tile: four, two or one blocks to promote), what dividing costs whatever its size
 // (the second kernel's latency; of its host time a part) and per slot (80 KB written and read again through L2): microseconds.
-// Stage: slope over 4 to 32 stages of 4736 undivided tiles, 1.38 us at block 32, 0.68 at 64, 0.43 at 128, of the form that the sweep below was made with
-// (8192 x 4096 x 11008 now takes 1.24, 0.62 and 0.41 a stage: the parts of a tile, and with them the association of its sums, stay as they were).  Checked on a sweep of 1 to 32
+// Stage: slope over 4 to 32 stages of 4736 undivided tiles, 1.38 us at block 32, 0.68 at 64, 0.43 at 128, of an earlier form of the kernel (8192 x
+// 4096 x 11008 now takes 1.22, 0.61 and 0.40 a stage), as is kSplitUs of a reduction that now takes up to a microsecond less.  The parts of a
+// tile, and with them the association of its sums, stay as they were; how far the plans are from the best ones of the present
+// form is not measured.  The earlier form was checked on a sweep of 1 to 32
 // items per tile and clusters of two to four over 23 shapes of 4 to 320 tiles and 6 to 86 stages at the three blocks (GEMM alone in a
-// graph): the plan is within 5 % of the best one everywhere and within 2 % in 62 of 69 (block 32 / 64 / 128, the plan's time
+// graph): the plan was within 5 % of the best one everywhere and within 2 % in 62 of 69 (block 32 / 64 / 128, the plan's time
 // and the undivided one's: 512 x 768 x 768 8.9, 12.0 / 8.0, 8.0 / 6.5, 6.5; 300 x 3072 x 768 12.1, 36.9 / 10.1, 20.4 / 9.3, 13.8; furthest off
 // 100 x 2048 x 2048 at 64, 9.4 in four items against 9.0 in six).  The number of items with the lowest sum is taken; the
 // largest that the SMs hold is often not the fastest.
